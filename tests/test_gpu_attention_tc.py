@@ -1,0 +1,98 @@
+"""CACHED_ATTENTION with many rows (the tensor-core form: f32 operands split into half-precision pairs) in two-op programs against float64:
+key dimensions and value widths around the 64-wide chunks, partial row and key tiles, every mask, ring wrap-around and a second state slot, caps, score
+tables, sinks, sigmoid weights, several maps, key ranges dealt to several CTAs, magnitudes far from 1, and rows that hold a NaN or an infinity.
+
+Tolerance: a split operand keeps its value to 2^-23 of itself or 2^-39 of its row's (tile's) largest, and f32 sums of up to a thousand terms add a few
+2^-24 of the largest partial sum: 1e-5 of the output's scale is ten times what scores up to about 10 make of that."""
+import numpy as np
+import pytest
+
+from test_gpu_recops import ctl_words, run
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(q, keys, vals, seen, scale, cap=0.0, table=None, dist=None, sink=None, sigmoid=False):
+    """One head: q [T, dk], keys [n, dk], vals [n, dv], seen [T, n]."""
+    s = q @ keys.T * scale
+    if cap:
+        s = cap * np.tanh(s / cap)
+    if table is not None:
+        s = s + table[np.clip(dist, 0, len(table) - 1)]
+    if sigmoid:
+        return np.where(seen, 1.0 / (1.0 + np.exp(-s)), 0.0) @ vals
+    s = np.where(seen, s, -np.inf)
+    m = s.max(1, keepdims=True)
+    e = np.exp(s - m)
+    return e @ vals / (e.sum(1, keepdims=True) + (np.exp(sink - m) if sink is not None else 0.0))
+
+
+def case(be, T, pos, H, G, dk, dv, maps=1, mask="causal", size=0, R=None, slot=0, cap=0.0, table=False, sink=False, sigmoid=False, out_scale=None, gain=1.0, seed=0, poison=None, block=0):
+    from zgml_b200 import DeviceBuffer, DeviceOp, ExternBuffer, abi
+    r = np.random.default_rng(seed)
+    kw, vw = G * maps * dk, G * dv
+    R = R or pos + T
+    kc, vc = (gain * r.standard_normal((2, R, kw))).astype(np.float32), r.standard_normal((2, R, vw)).astype(np.float32) * np.float32(gain)
+    if poison:
+        poison(kc[slot], vc[slot])
+    q = (r.standard_normal((T, H * maps * dk)) * 2.0 / gain).astype(np.float32)
+    bk, bv = DeviceBuffer(be, kc.nbytes, zero=False), DeviceBuffer(be, vc.nbytes, zero=False)
+    bk.upload(kc)
+    bv.upload(vc)
+    sizes, ext, io, kwargs = [T * H * maps * dv, q.size, bk.elems, bv.elems, 8 + T], [ExternBuffer(2, bk), ExternBuffer(3, bv)], [(1, q), (4, ctl_words(pos, slot))], {}
+    tab = (r.standard_normal((H * maps, R)) * 0.5).astype(np.float32) if table else None
+    if table:
+        sizes.append(tab.size)
+        io.append((len(sizes) - 1, tab))
+        kwargs.update(score_table=len(sizes) - 1, table_len=R)
+    sk = r.standard_normal(H * maps).astype(np.float32) if sink else None
+    if sink:
+        sizes.append(sk.size)
+        io.append((len(sizes) - 1, sk))
+        kwargs.update(sink=len(sizes) - 1, sink_wdt=abi.W_F32)
+    op = DeviceOp.cached_attention(0, 1, 2, 3, 4, 0, 0, 0, T, H, G, maps, dk, dv, H * maps * dk, kw, vw, R, dk ** -0.5, mask=mask, mask_size=size, softcap=cap,
+                                   weights="sigmoid" if sigmoid else "softmax", out_scale=out_scale, **kwargs)
+    got = run(be, [op], sizes, io, 0, (T, H, maps, dv), ext)
+    bk.free()
+    bv.free()
+    p = np.arange(pos, pos + T)
+    lo = {"causal": 0 * p, "window": np.maximum(p + 1 - size, 0), "block": p - p % max(size, 1)}[mask]
+    j = np.arange(lo[0], pos + T)
+    seen, dist = (j <= p[:, None]) & (j >= lo[:, None]), p[:, None] - j
+    want = np.empty((T, H, maps, dv))
+    for h in range(H):
+        g = h // (H // G)
+        for m in range(maps):
+            keys, vals = kc[slot][j % R][:, (g * maps + m) * dk:(g * maps + m + 1) * dk].astype(np.float64), vc[slot][j % R][:, g * dv:(g + 1) * dv].astype(np.float64)
+            with np.errstate(invalid="ignore"):
+                want[:, h, m] = reference(q[:, (h * maps + m) * dk:(h * maps + m + 1) * dk].astype(np.float64), keys, vals, seen, dk ** -0.5, cap, tab[h * maps + m] if table else None,
+                                          dist, sk[h * maps + m] if sink else None, sigmoid) * (out_scale or 1.0)
+    return got, want, seen, j
+
+
+def close(got, want):
+    return np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("shape", [
+    dict(T=257, pos=0, H=8, G=8, dk=64, dv=64), dict(T=200, pos=131, H=8, G=2, dk=128, dv=128, sink=True), dict(T=130, pos=300, H=16, G=4, dk=36, dv=100),
+    dict(T=129, pos=127, H=12, G=4, dk=160, dv=128, out_scale=0.5), dict(T=96, pos=500, H=8, G=1, dk=192, dv=128), dict(T=64, pos=900, H=8, G=2, dk=256, dv=200, sink=True),
+    dict(T=16, pos=4000, H=8, G=8, dk=128, dv=128), dict(T=385, pos=77, H=8, G=4, dk=96, dv=64, mask="window", size=190, R=600), dict(T=300, pos=1000, H=8, G=8, dk=64, dv=32, mask="window", size=333, R=640),
+    dict(T=300, pos=650, H=8, G=4, dk=64, dv=64, mask="block", size=400, R=800, slot=1), dict(T=150, pos=100, H=8, G=4, dk=64, dv=128, maps=2, cap=3.0, table=True),
+    dict(T=260, pos=60, H=8, G=4, dk=128, dv=64, table=True, sigmoid=True), dict(T=200, pos=333, H=8, G=4, dk=192, dv=64, cap=2.0, sink=True, slot=1),
+    dict(T=200, pos=100, H=8, G=4, dk=128, dv=128, gain=1e-12), dict(T=200, pos=100, H=8, G=4, dk=128, dv=128, gain=1e15)])
+def test_many_rows(cuda_backend, shape):
+    got, want, _, _ = case(cuda_backend, **shape)
+    assert close(got, want)
+
+
+@pytest.mark.parametrize("what", ["nan key", "nan value", "infinite value"])
+def test_rows_that_see_nothing_non_finite_are_exact(cuda_backend, what):
+    """Position 150 of every key head or value head is poisoned: the queries before it are as they were, and those that see it are not finite."""
+    def poison(k, v):
+        (k if what == "nan key" else v)[150] = np.inf if what == "infinite value" else np.nan
+    got, _, seen, j = case(cuda_backend, T=200, pos=60, H=8, G=4, dk=128, dv=128, poison=poison, seed=3)
+    clean, want, _, _ = case(cuda_backend, T=200, pos=60, H=8, G=4, dk=128, dv=128, seed=3)
+    sees = seen[:, j == 150][:, 0]
+    assert close(clean, want) and close(got[~sees], want[~sees])
+    assert not np.isfinite(got[sees]).any()

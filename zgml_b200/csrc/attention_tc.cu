@@ -1,0 +1,740 @@
+// Attention of many query rows over f32 keys and values on the 5th-generation tensor cores, with f32 accuracy.
+//
+// Every f32 operand x is split into two half-precision values, x = hi + lo: hi = f16(x s), lo = f16(x s - hi), with s a power of
+// two that brings the largest magnitude of its tile (keys, values) or row (queries) to [2^14, 2^15).  hi and lo together keep 22
+// to 24 significant bits of everything within 2^-17 of that maximum (what is smaller loses bits below 2^-39 of the maximum), so
+// the split costs about one f32 rounding per operand.  A product is three MMAs, hi lo + lo hi + hi hi, accumulated in f32 in TMEM: the
+// small cross terms first, so that only the dk / 16 steps of hi hi add to a large accumulator.  The probabilities (at most 1) are
+// scaled by 2^14 and split the same way.  Outputs of different key tiles are added in registers, in f32.
+//
+//   * k_atc_prep: 128 keys (or 128 columns of 128 values) per CTA, held in registers: maximum, split, store.  Keys as rows [hi dims | lo
+//     dims], values transposed, rows of one value column over all keys [hi | lo]: both are K-major operands that TMA brings as they lie (128-byte
+//     swizzle).  The cache is read and split once per step instead of once per query tile that meets it.
+//   * k_attention_tc: one CTA per 128 query rows.  Warp 16 loads 16 KB pieces through a ring of 12, warp 17 issues
+//     tcgen05.mma.cta_group::1.kind::f16, warps 0 - 15 are the softmax: four threads share a query row, each with a quarter of the tile's keys
+//     and a quarter of the output columns.  Queries lie split in TMEM (A operand), scores of two key tiles alternate between two TMEM buffers, and
+//     the probabilities replace the scores they came from, in place, as the A operand of the product with the values: no operand but keys and values
+//     passes through shared memory, whose bandwidth (128 B per clock) a 128 x 128 tile with both operands in it would saturate.  MMA order:
+//     scores of tile i + 1 before values of tile i, so the softmax of one tile runs beside the products of its neighbours.
+//   * Measured per 128 x 128 tile of 128 dims (its 48 MMAs execute in 3072 clocks): 9400 clocks with one thread per query row and the MMAs issued
+//     inside a single lane's branch, 9100 with four threads per row, 4700 once the whole MMA warp walks the tiles (below).
+//   * Every wait is bounded; a CTA whose wait ran out stops issuing, leaves its rows and frees its TMEM.
+//
+// Non-finite inputs: a key or value tile that holds one is marked by a NaN scale; the rows of a CTA that met such a tile are evaluated one
+// by one in plain f32 (atc_slow_row), as the SIMT kernels would.
+#include "attention_tc.cuh"
+
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+namespace {
+
+constexpr uint32_t kAtcThreads = 576, kAtcRing = 12, kAtcPiece = 16384;
+constexpr uint32_t kAtcShare = 2 * 4 * 128 * 4;                   // row maxima of the four quarters, two tiles
+constexpr uint32_t kAtcTiles = 512;                               // key tiles whose class and scales a CTA keeps at hand
+constexpr uint32_t kAtcSmem = kAtcRing * kAtcPiece + kAtcShare + kAtcTiles * 12 + 1024 + 256;
+constexpr uint32_t kAtcSpin = 1u << 22;
+constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+constexpr float kPScale = 16384.0f, kPInv = 1.0f / 16384.0f;      // probabilities are held times 2^14
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < kAtcSpin; i++) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap* map, uint32_t c0, uint32_t c1, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+// Shared-memory operand: K-major, 128-byte swizzle, 8-row groups 1024 B apart.  The low word holds the address, the high word never changes.
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_low(uint32_t addr) { return ((addr & 0x3FFFF) >> 4) | (1u << 16); }
+// D[tmem d] (+)= A[tmem a] B[shared]
+template <bool ACCUMULATE>
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint32_t b_low, uint32_t idesc) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tmov.b64 b, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+                 ::"r"(d), "r"(a), "r"(b_low), "n"(kDescHigh), "r"(idesc), "n"(ACCUMULATE ? 1 : 0) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// TMEM rows of a warp's lanes, N columns.  The loaded registers pass through the wait, so that nothing that reads them moves above it.
+__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
+}
+__device__ __forceinline__ void tmem_st(uint32_t addr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&v)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])::"memory");
+}
+__device__ __forceinline__ void tmem_st(uint32_t addr, const uint32_t (&v)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
+}
+__device__ __forceinline__ void tmem_st(uint32_t addr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void bar_sync(uint32_t id, uint32_t threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+
+// power of two that brings magnitudes up to `amax` below 2^15, and its inverse (NaN for a non-finite maximum)
+__device__ __forceinline__ void split_scale(float amax, float& scale, float& inv) {
+    const uint32_t bits = __float_as_uint(amax);
+    if (bits >= 0x7f800000u) { scale = 1.0f; inv = __uint_as_float(0x7fffffffu); return; }
+    int e = (int)(bits >> 23) - 127;
+    if (e < -112) e = -112;
+    scale = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
+    inv = __uint_as_float((uint32_t)(127 - 14 + e) << 23);
+}
+// two values -> packed hi, packed lo
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ float abs_or_inf(float m, float x) { const float a = fabsf(x); return a <= 3.4028234e38f ? fmaxf(m, a) : INFINITY; }   // NaN counts as infinite
+
+// ── where keys, values and queries come from ─────────────────────────────────────────────────────────────────────
+// A SOURCE names the keys of a step (for k_atc_prep) and, for the attention kernel, a CTA's items and range of key tiles, the class of a tile
+// (0: no row sees it, 1: every row sees all of it, 2: some), a row's query and what becomes of its scores.  Keys are counted from the first one
+// that any row of the step can see.
+
+// CACHED_ATTENTION: rows are (token, head of the key group) pairs
+template <bool EXTRA>      // score caps, score tables, sigmoid weights, pooled blocks
+struct AtcCached {
+    CaArgs a;
+    uint32_t rh, row_tiles, n_vs, vslice, splits, tiles;      // tiles: of 128 keys, that the planes have room for
+    float* part;
+    struct Step { uint32_t pos0, slot, k_lo, n_pool, n_keys; };
+    __device__ __forceinline__ Step step() const {
+        Step s;
+        s.pos0 = (uint32_t)ctl_word(a.ctl, ZG_CTL_POS); s.slot = ca_slot(a);
+        s.k_lo = mask_low(s.pos0, a.kind, a.size);
+        const uint32_t last = s.pos0 + a.T - 1;
+        s.n_pool = EXTRA && a.pool ? min(pooled_seen(last, a.size, a.pool), a.pool_rows) : 0u;
+        s.n_keys = min(s.n_pool + last - s.k_lo + 1, tiles * 128);
+        return s;
+    }
+    // row `u` of a key item or a value head; u < n_keys
+    __device__ __forceinline__ const float* row(const Step& s, bool value, uint32_t item, uint32_t u) const {
+        const uint32_t col = item * (value ? a.dv : a.dk), w = value ? a.vw : a.kw;
+        if (EXTRA && u < s.n_pool) return (value ? a.vp : a.kp) + (size_t)s.slot * a.pool_rows * a.kw + (size_t)u * a.kw + col;
+        return (value ? a.vc + a.v_off : a.kc + a.k_off) + ((size_t)s.slot * a.R + (s.k_lo + u - s.n_pool) % a.R) * w + col;
+    }
+    __device__ __forceinline__ uint32_t prep_keys(uint32_t) const { return step().n_keys; }
+    struct Cta { Step s; uint32_t r0, nq, p_min, p_max, lo_min, lo_max, nb_min, nb_max, gm, g, m, vs, split, t0, t1; };
+    __device__ __forceinline__ Cta cta(uint32_t bk) const {
+        Cta c;
+        c.s = step();
+        const uint32_t items = a.G * a.maps * n_vs, item = blockIdx.x % items;
+        c.gm = item / n_vs; c.vs = item % n_vs; c.g = c.gm / a.maps; c.m = c.gm % a.maps; c.split = blockIdx.y;
+        c.r0 = (row_tiles - 1 - blockIdx.x / items) * 128;            // later rows meet more keys: heaviest first
+        c.nq = min(128u, a.T * rh - c.r0);
+        c.p_min = c.s.pos0 + c.r0 / rh; c.p_max = c.s.pos0 + (c.r0 + c.nq - 1) / rh;
+        c.lo_min = mask_low(c.p_min, a.kind, a.size); c.lo_max = mask_low(c.p_max, a.kind, a.size);
+        c.nb_min = c.nb_max = 0;
+        if (EXTRA && a.pool) { c.nb_min = pooled_seen(c.p_min, a.size, a.pool); c.nb_max = pooled_seen(c.p_max, a.size, a.pool); }
+        const uint32_t first = c.s.n_pool ? 0u : (c.lo_min - c.s.k_lo) / bk, end = (min(c.s.n_keys, c.s.n_pool + c.p_max - c.s.k_lo + 1) + bk - 1) / bk;
+        const uint32_t per = (end - min(end, first) + splits - 1) / splits;
+        c.t0 = min(end, first + c.split * per); c.t1 = min(end, c.t0 + per);
+        return c;
+    }
+    __device__ __forceinline__ uint32_t k_item(const Cta& c) const { return c.gm; }
+    __device__ __forceinline__ uint32_t v_item(const Cta& c) const { return c.g * n_vs + c.vs; }
+    __device__ __forceinline__ uint32_t classify(const Cta& c, uint32_t t, uint32_t bk) const {
+        const uint32_t u0 = t * bk, u1 = u0 + bk - 1;
+        if (EXTRA && u0 < c.s.n_pool) {
+            if (u1 >= c.s.n_pool) return 2;
+            return u0 >= c.nb_max ? 0 : u1 < c.nb_min ? 1 : 2;
+        }
+        const uint32_t j0 = c.s.k_lo + u0 - c.s.n_pool, j1 = j0 + bk - 1;
+        if (j0 > c.p_max || j1 < c.lo_min) return 0;
+        return j1 <= c.p_min && j0 >= c.lo_max && u1 < c.s.n_keys ? 1 : 2;
+    }
+    struct Row { bool on; uint32_t r, p, lo, nb, hm; const float* q; const float* tab; };
+    __device__ __forceinline__ Row query(const Cta& c, uint32_t i) const {
+        Row w;
+        w.on = i < c.nq;
+        w.r = c.r0 + (w.on ? i : 0);
+        const uint32_t t = w.r / rh, h = c.g * rh + w.r % rh;
+        w.hm = h * a.maps + c.m;
+        w.p = c.s.pos0 + t; w.lo = mask_low(w.p, a.kind, a.size);
+        w.nb = EXTRA && a.pool ? pooled_seen(w.p, a.size, a.pool) : 0u;
+        w.q = a.q + (size_t)t * a.q_rs + a.q_off + (size_t)w.hm * a.dk;
+        w.tab = EXTRA && a.tab ? a.tab + (size_t)w.hm * a.tab_rs : nullptr;
+        return w;
+    }
+    __device__ __forceinline__ uint32_t dk() const { return a.dk; }
+    __device__ __forceinline__ uint32_t dv(const Cta& c) const { return min(vslice, a.dv - c.vs * vslice); }
+    __device__ __forceinline__ float scale(const Cta&) const { return a.scale; }
+    __device__ __forceinline__ bool sigmoid() const { return EXTRA && a.wkind; }
+    __device__ __forceinline__ bool plain_tile() const { return !EXTRA; }
+    // scores in units of log2 of keys u0 .. u0 + N - 1, from the scaled products times log2(e); -inf where the row does not see the key
+    template <int N>
+    __device__ __forceinline__ void scores(const Cta& c, const Row& w, uint32_t u0, float (&x)[N]) const {
+        if (EXTRA && a.cap > 0.0f) {
+#pragma unroll
+            for (int i = 0; i < N; i++) x[i] = a.cap * tanhf(x[i] * kLn2 / a.cap) * kLog2e;
+        }
+        if (EXTRA && w.tab) {                                         // no pooled blocks here: positions ascend with u
+            const uint32_t j0 = c.s.k_lo + u0;
+#pragma unroll
+            for (int i = 0; i < N; i++) if (j0 + i <= w.p && j0 + i >= w.lo) x[i] = fmaf(w.tab[w.p - j0 - i], kLog2e, x[i]);
+        }
+        const uint32_t base = c.s.k_lo - c.s.n_pool;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const uint32_t u = u0 + i, j = base + u;
+            const bool seen = EXTRA && u < c.s.n_pool ? u < w.nb : u < c.s.n_keys && j <= w.p && j >= w.lo;
+            if (!seen) x[i] = -INFINITY;
+        }
+    }
+    // natural units, from the plain product
+    __device__ __forceinline__ float slow_score(const Cta& c, const Row& w, uint32_t u, float dot) const {
+        const bool pooled = EXTRA && u < c.s.n_pool;
+        const uint32_t j = c.s.k_lo + u - c.s.n_pool;
+        if (pooled ? u >= w.nb : (u >= c.s.n_keys || j > w.p || j < w.lo)) return -INFINITY;
+        float s = ca_score(a, dot);
+        if (EXTRA && w.tab && !pooled) s += w.tab[w.p - j];
+        return s;
+    }
+    // columns col .. col + N - 1 of the CTA's value slice; `m` in natural or log2 units as m2 says; sums and outputs carry the factor 1 / unit
+    template <int N>
+    __device__ __forceinline__ void store(const Cta& c, const Row& w, uint32_t col, const float (&o)[N], float m, bool m2, float l, float unit) const {
+        const uint32_t n = dv(c) > col ? dv(c) - col : 0u, t = w.r / rh;
+        float* out;
+        float f;
+        if (splits == 1) {
+            out = a.dst + (size_t)t * a.dst_rs + (size_t)w.hm * a.dv + (size_t)c.vs * vslice + col;
+            float sum = l * unit;
+            if (!sigmoid() && a.sink) sum += m2 ? exp2f(fmaf(ca_sink(a, w.hm), kLog2e, -m)) : expf(ca_sink(a, w.hm) - m);
+            f = unit * a.out_scale * (sigmoid() ? 1.0f : 1.0f / sum);
+        } else {
+            float* mine = part + (((size_t)t * a.H * a.maps + w.hm) * splits + c.split) * (4 + a.dv);
+            if (c.vs == 0 && col == 0) { mine[0] = m2 ? m * kLn2 : m; mine[1] = l * unit; }
+            out = mine + 4 + (size_t)c.vs * vslice + col;
+            f = unit;
+        }
+        if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+#pragma unroll
+            for (int i = 0; i < N; i += 4)
+                if ((uint32_t)i + 4 <= n) *reinterpret_cast<float4*>(out + i) = make_float4(o[i] * f, o[i + 1] * f, o[i + 2] * f, o[i + 3] * f);
+        } else {
+#pragma unroll
+            for (int i = 0; i < N; i++) if ((uint32_t)i < n) out[i] = o[i] * f;
+        }
+    }
+};
+template <bool EXTRA>
+__device__ __forceinline__ const float* src_row(const AtcCached<EXTRA>& s, bool value, uint32_t head, uint32_t u) { return s.row(s.step(), value, head, u); }
+template <bool EXTRA>
+__device__ __forceinline__ const float* src_key(const AtcCached<EXTRA>& s, const typename AtcCached<EXTRA>::Cta& c, uint32_t u) { return s.row(c.s, false, c.gm, u); }
+template <bool EXTRA>
+__device__ __forceinline__ const float* src_value(const AtcCached<EXTRA>& s, const typename AtcCached<EXTRA>::Cta& c, uint32_t u) { return s.row(c.s, true, c.g, u) + c.vs * s.vslice; }
+
+struct AtcPlanes {
+    __half* k;           // [key items][tiles * 128][2 dkp]: hi | lo of a key
+    __half* v;           // [value items][vslice][2 tiles * 128]: hi | lo of a value column; an item is a slice of a value head's columns
+    float* k_inv;        // [key items][tiles]: 1 / scale of a tile, NaN where it holds something non-finite
+    float* v_inv;
+    uint32_t dkp, vslice, dk, dv, k_items, v_items, n_vs, tiles;
+};
+
+// CTA (tile, item): 128 keys of key item y, or 128 values of value item y - k_items.  C: 64-wide chunks of the widest item, all of which lie in
+// registers: every load is in flight at once.  (Reading twice, once for the maximum, took 17.5 us where this takes 9.5: 2048 keys and values of
+// 4 heads of 128, cold.)
+constexpr uint32_t kPrepThreads = 512;
+template <class Src, int C>
+__global__ void __launch_bounds__(kPrepThreads) k_atc_prep(const Src src, const AtcPlanes pl) {
+    pdl_enter();
+    __shared__ float red[kPrepThreads / 32];
+    __shared__ uint32_t t_hi[64][65], t_lo[64][65];      // a 64-column chunk of 128 values, transposed: pairs of keys per word
+    const bool value = blockIdx.y >= pl.k_items;
+    const uint32_t item = value ? blockIdx.y - pl.k_items : blockIdx.y, head = value ? item / pl.n_vs : item, u0 = blockIdx.x * 128, n_keys = src.prep_keys(head);
+    if (u0 >= n_keys) return;
+    const uint32_t first = value ? item % pl.n_vs * pl.vslice : 0, dim = value ? min(pl.vslice, pl.dv - first) : pl.dk, padded = value ? pl.vslice : pl.dkp;
+    const uint32_t tid = threadIdx.x, c4 = 4 * (tid & 15), k0 = 4 * (tid >> 4);      // columns c4 .. + 3 of every chunk, keys k0 .. + 3
+    float4 x[C][4];
+    float mx = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t u = u0 + k0 + k;
+        const float* row = u < n_keys ? src_row(src, value, head, u) + first : nullptr;
+#pragma unroll
+        for (int c = 0; c < C; c++) x[c][k] = row && 64 * c + c4 < dim ? *reinterpret_cast<const float4*>(row + 64 * c + c4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int c = 0; c < C; c++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) mx = abs_or_inf(abs_or_inf(abs_or_inf(abs_or_inf(mx, x[c][k].x), x[c][k].y), x[c][k].z), x[c][k].w);
+    mx = warp_max(mx);
+    if ((tid & 31) == 0) red[tid >> 5] = mx;
+    __syncthreads();
+    mx = warp_max(red[tid & 15]);
+    float scale, inv;
+    split_scale(mx, scale, inv);
+    if (tid == 0) (value ? pl.v_inv : pl.k_inv)[(size_t)item * pl.tiles + blockIdx.x] = inv;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        if (64 * c >= padded) break;
+        if (!value) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                uint32_t h[2], l[2];
+                split2(x[c][k].x * scale, x[c][k].y * scale, h[0], l[0]);
+                split2(x[c][k].z * scale, x[c][k].w * scale, h[1], l[1]);
+                __half* out = pl.k + ((size_t)item * pl.tiles * 128 + u0 + k0 + k) * 2 * pl.dkp + 64 * c + c4;
+                *reinterpret_cast<uint2*>(out) = make_uint2(h[0], h[1]);
+                *reinterpret_cast<uint2*>(out + pl.dkp) = make_uint2(l[0], l[1]);
+            }
+            continue;
+        }
+        if (c) __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; k += 2) {
+            const float* a = &x[c][k].x;
+            const float* b = &x[c][k + 1].x;
+#pragma unroll
+            for (int e = 0; e < 4; e++) split2(a[e] * scale, b[e] * scale, t_hi[c4 + e][(k0 + k) / 2], t_lo[c4 + e][(k0 + k) / 2]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t i = tid; i < 64 * 64; i += kPrepThreads) {
+            const uint32_t col = i >> 6, w = i & 63;
+            uint32_t* out = reinterpret_cast<uint32_t*>(pl.v + ((size_t)item * pl.vslice + 64 * c + col) * 2 * pl.tiles * 128 + u0);
+            out[w] = t_hi[col][w];
+            out[pl.tiles * 64 + w] = t_lo[col][w];
+        }
+    }
+}
+
+// one row in plain f32 over the keys of the CTA's tiles, output columns col .. col + N - 1
+template <int N, class Src>
+__device__ __noinline__ void atc_slow_row(const Src& src, const typename Src::Cta& c, const typename Src::Row& w, uint32_t col, uint32_t bk) {
+    float acc[N], m = -INFINITY, l = 0.0f;
+    for (int i = 0; i < N; i++) acc[i] = 0.0f;
+    const uint32_t dk = src.dk(), n = src.dv(c) > col ? min((uint32_t)N, src.dv(c) - col) : 0u;
+    for (uint32_t t = c.t0; t < c.t1; t++) {
+        if (!src.classify(c, t, bk)) continue;
+        for (uint32_t u = t * bk; u < (t + 1) * bk; u++) {
+            if (src.slow_score(c, w, u, 0.0f) == -INFINITY) continue;          // not seen
+            const float* k = src_key(src, c, u);
+            float d = 0.0f;
+            for (uint32_t i = 0; i < dk; i++) d = fmaf(w.q[i], k[i], d);
+            const float s = src.slow_score(c, w, u, d);
+            float e;
+            if (src.sigmoid()) e = s == -INFINITY ? 0.0f : ca_sigmoid(s);
+            else {
+                if (s == -INFINITY) continue;
+                const float mn = fmaxf(m, s), al = m == -INFINITY ? 0.0f : expf(m - mn);
+                e = expf(s - mn);
+                l = fmaf(l, al, e);
+                m = mn;
+                for (uint32_t i = 0; i < n; i++) acc[i] *= al;
+            }
+            const float* v = src_value(src, c, u) + col;
+            for (uint32_t i = 0; i < n; i++) acc[i] = fmaf(e, v[i], acc[i]);
+        }
+    }
+    src.template store<N>(c, w, col, acc, m, false, l, 1.0f);
+}
+
+// NC: 64-wide chunks of the key dimension; DV: value columns of the CTA (64 or 128)
+template <class Src, int NC, int DV>
+__global__ void __launch_bounds__(kAtcThreads, 1)
+k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Src src, const AtcPlanes pl) {
+    constexpr uint32_t BK = NC <= 2 ? 128 : 64, KC = BK / 64;       // keys per tile: scores twice, outputs and queries share the 512 columns of TMEM
+    constexpr uint32_t kS = 0, kO = 2 * BK, kQ = kO + DV;           // TMEM columns; the CTA owns all 512, so their addresses are constants
+    static_assert(kQ + 64 * NC <= 512, "TMEM columns");
+    constexpr uint32_t kPieceK = BK * 128, kPieceV = DV * 128;
+    extern __shared__ uint8_t dsm_raw[];
+    const uint32_t base = (smem_u32(dsm_raw) + 1023u) & ~1023u, bars = base + kAtcRing * kAtcPiece + kAtcShare + kAtcTiles * 12;
+    const uint32_t full = bars, empty = full + 8 * kAtcRing, s_full = empty + 8 * kAtcRing, p_full = s_full + 16, o_full = p_full + 8, q_full = o_full + 8, tmem_slot = q_full + 8;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < kAtcRing; i++) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 1); }
+        mbar_init(s_full, 1); mbar_init(s_full + 8, 1); mbar_init(p_full, 16); mbar_init(o_full, 1); mbar_init(q_full, 16);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 17) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tmem_slot) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const typename Src::Cta c = src.cta(BK);
+    // class and scales of the first tiles: read from global memory inside the loop they cost every tile an L2 round trip
+    float* const share = reinterpret_cast<float*>(dsm_raw + (base - smem_u32(dsm_raw)) + kAtcRing * kAtcPiece);
+    float2* const tile_inv = reinterpret_cast<float2*>(share + kAtcShare / 4);
+    uint32_t* const tile_class = reinterpret_cast<uint32_t*>(tile_inv + kAtcTiles);
+    const float* k_inv = pl.k_inv + (size_t)src.k_item(c) * pl.tiles;
+    const float* v_inv = pl.v_inv + (size_t)src.v_item(c) * pl.tiles;
+    for (uint32_t i = threadIdx.x; i < min(c.t1 - c.t0, kAtcTiles); i += kAtcThreads) {
+        const uint32_t t = c.t0 + i;
+        tile_class[i] = src.classify(c, t, BK);
+        tile_inv[i] = make_float2(k_inv[t * BK / 128], v_inv[t * BK / 128]);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    auto class_of = [&](uint32_t t) { return t - c.t0 < kAtcTiles ? tile_class[t - c.t0] : src.classify(c, t, BK); };
+
+    if (warp == 16) {
+        if (lane == 0) {
+            uint32_t slot = 0, phase = 1;                            // ring position
+            bool ok = true;
+            auto piece = [&](const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bytes) {
+                if (ok) ok = mbar_wait(empty + 8 * slot, phase);
+                if (!ok) return;
+                mbar_expect_tx(full + 8 * slot, bytes);
+                tma_2d(base + slot * kAtcPiece, map, x, y, full + 8 * slot);
+                if (++slot == kAtcRing) { slot = 0; phase ^= 1; }
+            };
+            const uint32_t ky = src.k_item(c) * pl.tiles * 128, vy = src.v_item(c) * pl.vslice;
+            auto values = [&](uint32_t t) {
+                for (int part = 1; part >= 0; part--)                // lo first: the cross terms come first
+                    for (uint32_t k = 0; k < KC; k++) piece(&map_v, part * pl.tiles * 128 + t * BK + 64 * k, vy, kPieceV);
+            };
+            uint32_t prev = 0;
+            bool have = false;
+            for (uint32_t t = c.t0; t < c.t1 && ok; t++) {
+                if (!class_of(t)) continue;
+                for (int part = 1; part >= 0; part--)
+                    for (uint32_t k = 0; k < NC; k++) piece(&map_k, part * pl.dkp + 64 * k, ky + t * BK, kPieceK);
+                if (have) values(prev);
+                prev = t; have = true;
+            }
+            if (have) values(prev);
+        }
+        __syncwarp();
+    } else if (warp == 17) {
+        // The whole warp walks the tiles and waits; one elected lane issues.  Addresses stay warp-uniform that way: with the loop inside a
+        // single lane's branch every MMA took 130 clocks to issue, twice what it takes to execute.
+        constexpr uint32_t idesc_s = (1u << 4) | ((BK >> 3) << 17) | ((128u >> 4) << 24), idesc_o = (1u << 4) | ((DV >> 3) << 17) | ((128u >> 4) << 24);   // f16 x f16 -> f32
+        const bool leader = elect_one();
+        const uint32_t b0 = desc_low(base);
+        uint32_t n_tiles = 0, slot = 0, phase = 0;                    // ring position
+        for (uint32_t t = c.t0; t < c.t1; t++) n_tiles += class_of(t) ? 1 : 0;
+        bool ok = mbar_wait(q_full, 0);
+        fence_after();
+        uint32_t held[4];                                             // ring slots of the hi pieces, which serve two products
+        auto next = [&]() {                                           // the next piece has arrived
+            const uint32_t s = slot;
+            if (ok) ok = mbar_wait(full + 8 * s, phase);
+            if (++slot == kAtcRing) { slot = 0; phase ^= 1; }
+            return s;
+        };
+        // D += A B over the 64 keys or dims of ring slot s: A at TMEM column a, STEP columns from one 16 to the next
+        auto product = [&](uint32_t d, uint32_t a, auto step, uint32_t s, uint32_t idesc, auto first) {
+            const uint32_t b = b0 + s * (kAtcPiece >> 4);
+            mma_ts<!decltype(first)::value>(d, a, b, idesc);
+#pragma unroll
+            for (uint32_t k = 1; k < 4; k++) mma_ts<true>(d, a + decltype(step)::value * k, b + 2 * k, idesc);
+        };
+        // three products of A (hi at a, lo at a + lo_at, `chunk` columns per piece) with N pieces of B: hi lo, lo hi, hi hi
+        auto triple = [&](uint32_t d, uint32_t a, uint32_t lo_at, uint32_t chunk, auto step, auto count, uint32_t idesc) {
+            constexpr uint32_t N = decltype(count)::value;
+#pragma unroll
+            for (uint32_t k = 0; k < N; k++) {
+                const uint32_t s = next();
+                fence_after();
+                if (leader && ok) {
+                    if (k == 0) product(d, a, step, s, idesc, std::true_type{}); else product(d, a + chunk * k, step, s, idesc, std::false_type{});
+                    mma_commit(empty + 8 * s);
+                }
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < N; k++) {
+                held[k] = next();
+                fence_after();
+                if (leader && ok) product(d, a + lo_at + chunk * k, step, held[k], idesc, std::false_type{});
+            }
+            if (leader && ok) {
+#pragma unroll
+                for (uint32_t k = 0; k < N; k++) {
+                    product(d, a + chunk * k, step, held[k], idesc, std::false_type{});
+                    mma_commit(empty + 8 * held[k]);
+                }
+            }
+        };
+        auto scores = [&](uint32_t i) {
+            triple(kS + (i & 1) * BK, kQ, 32 * NC, 32, std::integral_constant<uint32_t, 8>{}, std::integral_constant<uint32_t, NC>{}, idesc_s);
+            if (leader && ok) mma_commit(s_full + 8 * (i & 1));
+        };
+        // probabilities of 16 keys lie in 16 columns: 8 with their hi pairs, 8 with their lo pairs
+        auto values = [&](uint32_t i) {
+            if (ok) ok = mbar_wait(p_full, i & 1);
+            fence_after();
+            triple(kO, kS + (i & 1) * BK, 8, 64, std::integral_constant<uint32_t, 16>{}, std::integral_constant<uint32_t, KC>{}, idesc_o);
+            if (leader && ok) mma_commit(o_full);
+        };
+        for (uint32_t i = 0; i < n_tiles && ok; i++) {
+            scores(i);
+            if (i) values(i - 1);
+        }
+        if (n_tiles && ok) values(n_tiles - 1);
+        __syncwarp();
+    } else {
+        // ── four threads per query row: quarter `part` of a tile's keys, of the output columns and of the query's dims ──
+        constexpr int KW = BK / 4, OW = DV / 4;
+        const uint32_t part = warp >> 2, row = (warp & 3) * 32 + lane, lanes = ((warp & 3) * 32) << 16;
+        const typename Src::Row w = src.query(c, row);
+        uint32_t n_share = 0;
+        auto row_max = [&](float x) {                                // over the row's four threads; two buffers in turns, so one barrier is enough
+            float* s = share + (n_share++ & 1) * 512;
+            s[part * 128 + row] = x;
+            bar_sync(1 + (warp & 3), 128);
+            return fmaxf(fmaxf(s[row], s[128 + row]), fmaxf(s[256 + row], s[384 + row]));
+        };
+        float q_inv, q_scale;
+        {
+            const uint32_t dk = src.dk();
+            float4 x[4 * NC];                                        // 16 NC dims from 16 NC part on
+            float mx = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4 * NC; i++) {
+                const uint32_t d = 16 * NC * part + 4 * i;
+                x[i] = d < dk ? *reinterpret_cast<const float4*>(w.q + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int i = 0; i < 4 * NC; i++) mx = abs_or_inf(abs_or_inf(abs_or_inf(abs_or_inf(mx, x[i].x), x[i].y), x[i].z), x[i].w);
+            split_scale(row_max(mx), q_scale, q_inv);
+#pragma unroll
+            for (int i = 0; i < NC; i++) {                           // 16 dims: 8 columns of pairs
+                uint32_t hi[8], lo[8];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    split2(x[4 * i + j].x * q_scale, x[4 * i + j].y * q_scale, hi[2 * j], lo[2 * j]);
+                    split2(x[4 * i + j].z * q_scale, x[4 * i + j].w * q_scale, hi[2 * j + 1], lo[2 * j + 1]);
+                }
+                tmem_st(lanes + kQ + 8 * (NC * part + i), hi);
+                tmem_st(lanes + kQ + 32 * NC + 8 * (NC * part + i), lo);
+            }
+            tmem_wait_st();
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(q_full);
+        }
+        const float unit = src.scale(c) * kLog2e;
+        const bool sigmoid = src.sigmoid();
+        float o[OW];
+#pragma unroll
+        for (int i = 0; i < OW; i++) o[i] = 0.0f;
+        float m = -INFINITY, l = 0.0f, alpha_prev = 1.0f, f_prev = 0.0f;
+        bool ok = true, slow = !(q_inv == q_inv);
+        uint32_t it = 0;
+        auto add_output = [&](uint32_t i) {                          // outputs of tile i join the running ones
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(o_full, i & 1));
+            fence_after();
+            uint32_t v[OW];
+            tmem_ld(lanes + kO + OW * part, v);
+            tmem_wait_ld(v);
+#pragma unroll
+            for (int j = 0; j < OW; j += 2) {
+                const float2 r = __ffma2_rn(make_float2(o[j], o[j + 1]), make_float2(alpha_prev, alpha_prev),
+                                            __fmul2_rn(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), make_float2(f_prev, f_prev)));
+                o[j] = r.x; o[j + 1] = r.y;
+            }
+        };
+        for (uint32_t t = c.t0; t < c.t1; t++) {
+            const uint32_t cls = class_of(t);
+            if (!cls) continue;
+            const float2 inv = t - c.t0 < kAtcTiles ? tile_inv[t - c.t0] : make_float2(k_inv[t * BK / 128], v_inv[t * BK / 128]);
+            slow = slow || !(inv.x + inv.y == inv.x + inv.y);
+            const float f = q_inv * inv.x * unit;
+            const bool plain = src.plain_tile() && cls == 1;
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(s_full + 8 * (it & 1), (it >> 1) & 1));
+            fence_after();
+            const uint32_t s = lanes + kS + (it & 1) * BK + KW * part, u0 = t * BK + KW * part;
+            uint32_t v[KW];
+            tmem_ld(s, v);
+            tmem_wait_ld(v);
+            float x[KW], alpha = 1.0f, shift = 14.0f;                // scores in units of log2; probabilities times 2^14
+#pragma unroll
+            for (int j = 0; j < KW; j++) x[j] = __uint_as_float(v[j]) * f;
+            if (!plain) src.scores(c, w, u0, x);
+            if (!sigmoid) {
+                float m0 = x[0], m1 = x[1];
+#pragma unroll
+                for (int j = 2; j < KW; j += 2) { m0 = fmaxf(m0, x[j]); m1 = fmaxf(m1, x[j + 1]); }
+                const float mx = row_max(fmaxf(m0, m1)), m_new = fmaxf(m, mx);
+                slow = slow || mx == INFINITY;
+                alpha = m == -INFINITY ? 0.0f : ex2(m - m_new);
+                m = m_new;
+                if (m_new != -INFINITY) shift -= m_new;
+#pragma unroll
+                for (int j = 0; j < KW; j++) x[j] = ex2(x[j] + shift);
+            } else {
+#pragma unroll
+                for (int j = 0; j < KW; j++) x[j] = x[j] == -INFINITY ? 0.0f : kPScale * ca_sigmoid(x[j] * kLn2);
+            }
+            float l0 = 0.0f, l1 = 0.0f;
+#pragma unroll
+            for (int j = 0; j < KW; j += 2) {
+                l0 += x[j]; l1 += x[j + 1];
+                split2(x[j], x[j + 1], v[(j / 16) * 16 + (j % 16) / 2], v[(j / 16) * 16 + 8 + (j % 16) / 2]);
+            }
+            tmem_st(s, v);
+            l = fmaf(l, alpha, l0 + l1);
+            tmem_wait_st();
+            if (it) add_output(it - 1);
+            alpha_prev = alpha; f_prev = inv.y;
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full);
+            it++;
+        }
+        if (it) add_output(it - 1);
+        {
+            float* s = share + (n_share & 1) * 512;                  // the row's sum
+            s[part * 128 + row] = l;
+            bar_sync(1 + (warp & 3), 128);
+            l = (s[row] + s[128 + row]) + (s[256 + row] + s[384 + row]);
+        }
+        if (ok && w.on) {
+            if (slow) atc_slow_row<OW>(src, c, w, OW * part, BK);
+            else src.template store<OW>(c, w, OW * part, o, m, true, l, kPInv);
+        }
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __syncwarp();
+    fence_before();
+    __syncthreads();
+    if (warp == 17) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(0u) : "memory");
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_tiled() {
+    static const EncodeTiledFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess ? (EncodeTiledFn)f : (EncodeTiledFn)nullptr;
+    }();
+    return fn;
+}
+bool encode_plane(CUtensorMap* map, void* p, uint64_t width, uint64_t rows, uint32_t box_rows) {
+    const cuuint64_t dims[2] = {width, rows}, stride[1] = {width * 2};
+    const cuuint32_t box[2] = {64, box_rows}, one[2] = {1, 1};
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) { zg_set_error("cuTensorMapEncodeTiled entry point not available"); return false; }
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p, dims, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { zg_set_error("cuTensorMapEncodeTiled(attention planes) failed (%d)", (int)r); return false; }
+    return true;
+}
+size_t up64(size_t n) { return (n + 63) & ~(size_t)63; }
+// scratch: planes, then scales, then whatever the caller adds; offsets in f32 slots
+struct AtcLayout { size_t k, v, k_inv, v_inv, total; };
+AtcLayout layout(const AtcPlanes& p) {
+    AtcLayout L;
+    size_t o = 0;
+    L.k = o; o += up64((size_t)p.k_items * p.tiles * 128 * p.dkp);
+    L.v = o; o += up64((size_t)p.v_items * p.vslice * p.tiles * 128);
+    L.k_inv = o; o += up64((size_t)p.k_items * p.tiles);
+    L.v_inv = o; o += up64((size_t)p.v_items * p.tiles);
+    L.total = o;
+    return L;
+}
+void place(AtcPlanes& p, float* scratch) {
+    const AtcLayout L = layout(p);
+    p.k = reinterpret_cast<__half*>(scratch + L.k); p.v = reinterpret_cast<__half*>(scratch + L.v);
+    p.k_inv = scratch + L.k_inv; p.v_inv = scratch + L.v_inv;
+}
+template <class Src, int NC, int DV>
+bool launch(const Src& src, const AtcPlanes& pl, dim3 grid, cudaStream_t st) {
+    constexpr uint32_t BK = NC <= 2 ? 128 : 64;
+    constexpr int C = NC > DV / 64 ? NC : DV / 64;
+    CUtensorMap mk, mv;
+    if (!encode_plane(&mk, pl.k, 2 * pl.dkp, (uint64_t)pl.k_items * pl.tiles * 128, BK) || !encode_plane(&mv, pl.v, (uint64_t)2 * pl.tiles * 128, (uint64_t)pl.v_items * pl.vslice, DV)) return false;
+    static const cudaError_t set = cudaFuncSetAttribute(k_attention_tc<Src, NC, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAtcSmem);
+    if (set != cudaSuccess) { zg_set_error("cudaFuncSetAttribute(attention) failed: %s", cudaGetErrorString(set)); return false; }
+    launch_pdl(k_atc_prep<Src, C>, dim3(pl.tiles, pl.k_items + pl.v_items), dim3(kPrepThreads), 0, st, src, pl);
+    ZG_COUNT_LAUNCH();
+    launch_pdl(k_attention_tc<Src, NC, DV>, grid, dim3(kAtcThreads), kAtcSmem, st, mk, mv, src, pl);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { zg_set_error("attention launch failed: %s", cudaGetErrorString(e)); return false; }
+    ZG_COUNT_LAUNCH();
+    return true;
+}
+template <class Src>
+bool launch_dims(const Src& src, const AtcPlanes& pl, dim3 grid, cudaStream_t st) {
+    const uint32_t nc = pl.dkp / 64;
+#define ZG_ATC(NC_) (pl.vslice == 64 ? launch<Src, NC_, 64>(src, pl, grid, st) : launch<Src, NC_, 128>(src, pl, grid, st))
+    return nc == 1 ? ZG_ATC(1) : nc == 2 ? ZG_ATC(2) : nc == 3 ? ZG_ATC(3) : ZG_ATC(4);
+#undef ZG_ATC
+}
+struct CachedPlan { AtcPlanes pl; uint32_t rh, row_tiles, splits; };
+CachedPlan cached_plan(const ZgAtcShape& s, int n_sm) {
+    CachedPlan P = {};
+    P.pl.vslice = s.dv <= 64 ? 64 : 128; P.pl.n_vs = (s.dv + P.pl.vslice - 1) / P.pl.vslice;
+    P.pl.dk = s.dk; P.pl.dv = s.dv; P.pl.dkp = (s.dk + 63) / 64 * 64;
+    P.pl.k_items = s.G * s.maps; P.pl.v_items = s.G * P.pl.n_vs; P.pl.tiles = (s.reach + 127) / 128;
+    P.rh = s.H / s.G; P.row_tiles = (s.T * P.rh + 127) / 128;
+    // few row tiles over many keys: key ranges of at least two tiles of 128 go to CTAs of their own until the SMs are covered
+    const uint32_t ctas = P.row_tiles * P.pl.k_items * P.pl.n_vs;
+    uint32_t S = (uint32_t)n_sm / (ctas ? ctas : 1), most = P.pl.tiles / 2;
+    if (S > most) S = most;
+    P.splits = S < 2 ? 1 : S > 64 ? 64 : S;
+    return P;
+}
+}  // namespace
+
+// Measured against the SIMT kernels over 32 shapes (16 to 1024 tokens, 1 to 16 heads of 32 to 160, windows of 71 to 749 and whole caches): with
+// tokens x heads x keys x (dk + dv) of 60 M and more this form was 1.0 to 2.7 times as fast, 11.9 times at 1024 tokens x 16 heads x 2048 keys of
+// 128; between 5 M and 36 M it took 0.8 to 1.1 times as long: the split of the cache and the start of the pipeline cost about 10 us.
+bool zg_attention_tc_usable(const ZgAtcShape& s) {
+    return s.dk >= 32 && s.dk <= 256 && s.dv >= 32 && s.T >= 16 && (uint64_t)s.T * s.H * s.maps * s.keys * (s.dk + s.dv) >= 48000000ull;
+}
+size_t zg_attention_tc_scratch_elems(const ZgAtcShape& s, int n_sm) {
+    const CachedPlan P = cached_plan(s, n_sm);
+    return layout(P.pl).total + (P.splits > 1 ? (size_t)s.T * s.H * s.maps * P.splits * (4 + s.dv) : 0);
+}
+bool zg_attention_tc_launch(const ZgAtcShape& s, const void* args, float* scratch, int n_sm, cudaStream_t st, uint32_t* splits, float** part) {
+    const CaArgs& a = *static_cast<const CaArgs*>(args);
+    CachedPlan P = cached_plan(s, n_sm);
+    place(P.pl, scratch);
+    *splits = P.splits;
+    *part = P.splits > 1 ? scratch + layout(P.pl).total : nullptr;
+    const dim3 grid(P.row_tiles * P.pl.k_items * P.pl.n_vs, P.splits);
+    if (a.cap > 0.0f || a.tab || a.wkind || a.pool) {
+        AtcCached<true> src = {a, P.rh, P.row_tiles, P.pl.n_vs, P.pl.vslice, P.splits, P.pl.tiles, *part};
+        return launch_dims(src, P.pl, grid, st);
+    }
+    AtcCached<false> src = {a, P.rh, P.row_tiles, P.pl.n_vs, P.pl.vslice, P.splits, P.pl.tiles, *part};
+    return launch_dims(src, P.pl, grid, st);
+}

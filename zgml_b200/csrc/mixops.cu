@@ -4,7 +4,7 @@
 // the cache with grouped heads / several score maps per head / causal, sliding and block masks, the differential
 // combination of two maps, sigmoid gates, block-diagonal (per-head) products and the PolyNorm activation.
 // Everything here is f32: positions and angles, scores and softmax weights, norms, gates and the sums.
-#include "seq_common.cuh"
+#include "attention_tc.cuh"
 
 #include <math.h>
 #include <stdlib.h>
@@ -205,69 +205,6 @@ __global__ void k_cache_append(float* __restrict__ cache, const float* __restric
 }
 
 // ── CACHED_ATTENTION ─────────────────────────────────────────────────────────────────────────────────────────────
-// first position a query at p can see
-__device__ __forceinline__ uint32_t mask_low(uint32_t p, uint32_t kind, uint32_t size) {
-    if (kind == 1 || kind == 3) return p + 1 >= size ? p + 1 - size : 0;
-    if (kind == 2) return p - p % size;
-    return 0;
-}
-// mask 3: beside its window a query at p sees the mean row of every block of `pool` positions that lies wholly before the window
-__device__ __forceinline__ uint32_t pooled_seen(uint32_t p, uint32_t size, uint32_t pool) { return p + 1 > size ? (p + 1 - size) / pool : 0; }
-struct CaArgs {
-    float* dst; const float* q; const float* kc; const float* vc; const float* ctl;
-    uint32_t T, H, G, maps, dk, dv, q_rs, q_off, kw, k_off, vw, v_off, R, kind, size;
-    float scale;
-    const float* tab;      // score table [H * maps, tab_rs] by distance, or null
-    uint32_t tab_rs, wkind;   // weights: 0 softmax over the visible keys, 1 sigmoid of every visible key (not normalised)
-    float cap;             // > 0: the scaled score passes cap * tanh(s / cap)
-    const void* sink;      // a learned score per (head, map) that joins the softmax's denominator only, or null
-    uint32_t sink_bf16;    // its weight type
-    float out_scale;       // the result is multiplied by it
-    uint32_t dst_rs;       // row stride of dst (its first column is folded into the pointer)
-    const float* kp; const float* vp;   // POOL: pooled rows [slots, pool_rows, kw] (laid out like the cache's), their key and value columns
-    uint32_t pool, pool_rows;
-    uint32_t unslotted;    // the caches belong to the step (rows recomputed by the program), not to a state slot
-};
-__device__ __forceinline__ uint32_t ca_slot(const CaArgs& a) { return a.unslotted ? 0u : (uint32_t)ctl_word(a.ctl, ZG_CTL_SLOT); }
-__device__ __forceinline__ float ca_score(const CaArgs& a, float dot) {
-    const float s = dot * a.scale;
-    return a.cap > 0.0f ? a.cap * tanhf(s / a.cap) : s;
-}
-__device__ __forceinline__ float ca_sink(const CaArgs& a, uint32_t hm) {
-    return a.sink_bf16 ? __bfloat162float(reinterpret_cast<const bf16*>(a.sink)[hm]) : reinterpret_cast<const float*>(a.sink)[hm];
-}
-// 1 / (sum + exp(sink - max)): the sink's share of the denominator, in the frame of the running maximum
-__device__ __forceinline__ float ca_inv_sum(const CaArgs& a, uint32_t hm, float mx, float l) {
-    if (a.sink) l += expf(ca_sink(a, hm) - mx);
-    return 1.0f / l;
-}
-// weight of a visible key under the unnormalised kind
-__device__ __forceinline__ float ca_sigmoid(float s) { return __frcp_rn(1.0f + expf(-s)); }
-constexpr int kCaMaxDv = 1024;   // 32 channels per lane in the per-query kernel
-// Keys as a kernel counts them: positions of the cache, or (POOL) the pooled blocks some row of the tile can see, followed by the
-// positions from k_lo on.  One softmax runs over both.
-template <bool POOL>
-struct CaKeys {
-    const float* cache; const float* pooled;
-    uint32_t R, width, k_lo, n_pool;
-    __device__ __forceinline__ uint32_t first() const { return POOL ? 0u : k_lo; }
-    __device__ __forceinline__ uint32_t count(uint32_t p_max) const { return p_max - k_lo + 1 + (POOL ? n_pool : 0u); }
-    __device__ __forceinline__ bool is_pooled(uint32_t u) const { return POOL && u < n_pool; }
-    __device__ __forceinline__ uint32_t position(uint32_t u) const { return POOL ? u - n_pool + k_lo : u; }
-    __device__ __forceinline__ const float* row(uint32_t u) const { return is_pooled(u) ? pooled + (size_t)u * width : cache + (size_t)(position(u) % R) * width; }
-    // whether a row at position p, whose window starts at lo and that sees nb blocks, sees key u
-    __device__ __forceinline__ bool seen(uint32_t u, uint32_t p, uint32_t lo, uint32_t nb) const {
-        if (is_pooled(u)) return u < nb;
-        const uint32_t j = position(u);
-        return j <= p && j >= lo;
-    }
-};
-template <bool POOL>
-__device__ __forceinline__ CaKeys<POOL> ca_keys(const float* cache, const float* pooled, uint32_t R, uint32_t width, uint32_t k_lo, uint32_t n_pool) {
-    CaKeys<POOL> k;
-    k.cache = cache; k.pooled = pooled; k.R = R; k.width = width; k.k_lo = k_lo; k.n_pool = POOL ? n_pool : 0u;
-    return k;
-}
 // Any shape: one warp per (token, head, map); 32 keys at a time, lane = key for the scores, lane = channel for the sum.
 template <bool POOL>
 __global__ void k_cached_attention(CaArgs a) {
@@ -766,6 +703,15 @@ static uint32_t ca_reach(const ZgSeqOp& s) {
     const uint32_t tokens = s.off[3] ? min(s.n[9], s.off[4] + s.n[0]) : s.n[9];
     return s.off[3] == 3 ? tokens + s.off[6] : tokens;
 }
+static int sm_count() {
+    static const int n = [] { int dev = 0, v = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); return v > 0 ? v : 148; }();
+    return n;
+}
+static ZgAtcShape ca_shape(const ZgSeqOp& s) {
+    const uint32_t reach = ca_reach(s), keys = s.off[3] ? s.off[4] + (s.off[3] == 3 ? s.off[6] : 0) : reach;
+    return {s.n[0], s.n[1], s.n[2], s.n[3], s.n[4], s.n[5], reach, min(keys, reach)};
+}
+static bool ca_tensor(const ZgSeqOp& s) { return ca_aligned(s) && !ca_few(s) && zg_attention_tc_usable(ca_shape(s)); }
 // key shares per row tile: few CTAs and a long cache (decoding) spread over more of them
 static uint32_t ca_splits(const ZgSeqOp& s) {
     if (!ca_aligned(s)) return 1;
@@ -1128,6 +1074,7 @@ size_t zg_mix_op_scratch_elems(const ZgOp& op) {
     if (op.tag == ZG_OP_HEAD_LINEAR) return hl_tensor(op.u.seq) ? zg_dense_gemm_batched_scratch_elems(op.u.seq.n[1], op.u.seq.n[0], op.u.seq.n[3]) : 0;
     if (op.tag != ZG_OP_CACHED_ATTENTION) return 0;
     const ZgSeqOp& s = op.u.seq;
+    if (ca_tensor(s)) return zg_attention_tc_scratch_elems(ca_shape(s), sm_count());
     const uint32_t S = ca_splits(s);
     return S > 1 ? (size_t)s.n[0] * s.n[1] * s.n[3] * S * (4 + s.n[5]) : 0;
 }
@@ -1204,13 +1151,18 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
                     ZG_SEQ_CHECK();
                     launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + 127) / 128), dim3(128 * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
                 }
+            } else if (aligned && scratch && ca_tensor(s)) {
+                uint32_t S = 1;
+                float* part = nullptr;
+                if (!zg_attention_tc_launch(ca_shape(s), &a, scratch, sm_count(), st, &S, &part)) return false;
+                if (S == 1) return true;
+                launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + 127) / 128), dim3(128 * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
             } else if (aligned) {
-                const uint32_t S = scratch ? ca_splits(s) : 1;
+                const uint32_t S = scratch && !ca_tensor(s) ? ca_splits(s) : 1;
                 float* part = S > 1 ? scratch : nullptr;
                 // A latent of rank <= 512 in ONE value slice takes its scores once instead of once per 256 columns, but halves the
                 // number of CTAs: worth it only while they still fill the GPU one and a half times.
-                static int n_sm = 0;
-                if (!n_sm) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev); if (n_sm <= 0) n_sm = 1; }
+                const int n_sm = sm_count();
                 const uint32_t row_ctas = ((a.T * (a.H / a.G) + kCtBQ - 1) / kCtBQ) * a.G * a.maps * S * ((a.dv + 511) / 512);
                 if (a.dv > 256 && 2 * row_ctas >= 3 * (uint32_t)n_sm) launch_cached_attention_tiled<32>(a, S, part, st);
                 else if (a.dv > 128) launch_cached_attention_tiled<16>(a, S, part, st);
