@@ -96,3 +96,38 @@ def test_rows_that_see_nothing_non_finite_are_exact(cuda_backend, what):
     sees = seen[:, j == 150][:, 0]
     assert close(clean, want) and close(got[~sees], want[~sees])
     assert not np.isfinite(got[sees]).any()
+
+
+def test_batched_heads_with_their_own_masks_and_a_refreshed_length(cuda_backend):
+    """DeviceOp.attention of a prompt: five heads over two key / value slabs and three masks — zeros and -inf, additive values, one laid out query-contiguous — and
+    none; then the same compiled program over fewer keys."""
+    import ctypes as C
+    from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO
+    r = np.random.default_rng(5)
+    T, S, dh, H = 141, 300, 64, 5
+    q, k, v = r.standard_normal((H, T, dh)).astype(np.float32), r.standard_normal((2, S, dh)).astype(np.float32), r.standard_normal((2, S, dh)).astype(np.float32)
+    m0 = np.where(r.random((T, S)) < 0.4, -np.inf, 0.0).astype(np.float32)
+    m0[:, 128:256] = -np.inf                                          # a whole tile nobody sees, beside tiles that every row sees in part
+    m1 = np.where(r.random((T, S)) < 0.2, -np.inf, r.standard_normal((T, S))).astype(np.float32)
+    m0[7], m1[7] = -np.inf, -np.inf                                   # a row that sees nothing: zeros
+    masks = [m0, m1, m1, m0, None]
+    mask_buf = np.concatenate([m0.ravel(), m1.ravel(), m1.T.ravel()]).astype(np.float32)
+    geom = [(0, 1, S), (T * S, 1, S), (2 * T * S, T, 1), (0, 1, S), (0, 1, S)]                 # offset, stride between keys, between queries
+    ops = [DeviceOp.attention(4, 0, 1, 2, 3, masks[h] is not None, dh, T, 270, 0.3, h * T * dh, h % 2 * S * dh, h % 2 * S * dh, geom[h][0], h * T * dh, 1, dh, 1, dh, 1, dh, geom[h][1],
+                              geom[h][2], 1, dh) for h in range(H)]
+    prog = DeviceProgram(ops, [q.size, k.size, v.size, mask_buf.size, q.size], [], [])
+    handle = cuda_backend.compile_program(prog)
+    ins = [ProgramIO(i, a.ravel()) for i, a in enumerate((q, k, v, mask_buf))]
+    for n in (270, 129, 300):
+        for o in ops:
+            o.u.attention.seq_kv = n
+        cuda_backend.refresh_program(handle, ops)
+        got = np.zeros((H, T, dh), np.float32)
+        cuda_backend.execute_program(handle, ins, [ProgramIO(4, got)])
+        for h in range(H):
+            s = q[h].astype(np.float64) @ k[h % 2, :n].astype(np.float64).T * 0.3 + (0.0 if masks[h] is None else masks[h][:, :n].astype(np.float64))
+            top = s.max(1, keepdims=True)
+            e = np.exp(s - np.where(np.isfinite(top), top, 0.0))
+            want = e @ v[h % 2, :n].astype(np.float64) / np.maximum(e.sum(1, keepdims=True), 1e-300)
+            assert close(got[h], want), (n, h)
+    cuda_backend.free_program(handle)

@@ -27,7 +27,10 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <map>
 #include <type_traits>
+#include <vector>
 
 namespace {
 
@@ -36,6 +39,7 @@ constexpr uint32_t kAtcShare = 2 * 4 * 128 * 4;                   // row maxima 
 constexpr uint32_t kAtcTiles = 512;                               // key tiles whose class and scales a CTA keeps at hand
 constexpr uint32_t kAtcSmem = kAtcRing * kAtcPiece + kAtcShare + kAtcTiles * 12 + 1024 + 256;
 constexpr uint32_t kAtcSpin = 1u << 22;
+constexpr size_t kAtcProgramKeys = 1u << 20;                      // the most keys that a DeviceOp.attention batch lays out planes for
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr float kPScale = 16384.0f, kPInv = 1.0f / 16384.0f;      // probabilities are held times 2^14
 
@@ -186,7 +190,7 @@ struct AtcCached {
         if (j0 > c.p_max || j1 < c.lo_min) return 0;
         return j1 <= c.p_min && j0 >= c.lo_max && u1 < c.s.n_keys ? 1 : 2;
     }
-    struct Row { bool on; uint32_t r, p, lo, nb, hm; const float* q; const float* tab; };
+    struct Row { bool on; uint32_t r, p, lo, nb, hm; const float* tab; };
     __device__ __forceinline__ Row query(const Cta& c, uint32_t i) const {
         Row w;
         w.on = i < c.nq;
@@ -195,10 +199,10 @@ struct AtcCached {
         w.hm = h * a.maps + c.m;
         w.p = c.s.pos0 + t; w.lo = mask_low(w.p, a.kind, a.size);
         w.nb = EXTRA && a.pool ? pooled_seen(w.p, a.size, a.pool) : 0u;
-        w.q = a.q + (size_t)t * a.q_rs + a.q_off + (size_t)w.hm * a.dk;
         w.tab = EXTRA && a.tab ? a.tab + (size_t)w.hm * a.tab_rs : nullptr;
         return w;
     }
+    __device__ __forceinline__ const float* q_row(const Cta& c, const Row& w) const { return a.q + (size_t)(w.r / rh) * a.q_rs + a.q_off + (size_t)w.hm * a.dk; }
     __device__ __forceinline__ uint32_t dk() const { return a.dk; }
     __device__ __forceinline__ uint32_t dv(const Cta& c) const { return min(vslice, a.dv - c.vs * vslice); }
     __device__ __forceinline__ float scale(const Cta&) const { return a.scale; }
@@ -206,7 +210,7 @@ struct AtcCached {
     __device__ __forceinline__ bool plain_tile() const { return !EXTRA; }
     // scores in units of log2 of keys u0 .. u0 + N - 1, from the scaled products times log2(e); -inf where the row does not see the key
     template <int N>
-    __device__ __forceinline__ void scores(const Cta& c, const Row& w, uint32_t u0, float (&x)[N]) const {
+    __device__ __forceinline__ void scores(const Cta& c, const Row& w, uint32_t, uint32_t u0, uint32_t, float (&x)[N]) const {
         if (EXTRA && a.cap > 0.0f) {
 #pragma unroll
             for (int i = 0; i < N; i++) x[i] = a.cap * tanhf(x[i] * kLn2 / a.cap) * kLog2e;
@@ -233,31 +237,122 @@ struct AtcCached {
         if (EXTRA && w.tab && !pooled) s += w.tab[w.p - j];
         return s;
     }
-    // columns col .. col + N - 1 of the CTA's value slice; `m` in natural or log2 units as m2 says; sums and outputs carry the factor 1 / unit
+    // What a row's outputs are multiplied by; sums and outputs carry the factor 1 / unit, `m` is in natural or (m2) log2 units.  A share of the keys
+    // leaves its maximum and sum for the merge (`first`: one of the row's threads).
+    __device__ __forceinline__ float finish(const Cta& c, const Row& w, bool first, float m, bool m2, float l, float unit) const {
+        if (splits > 1) {
+            if (first && c.vs == 0) {
+                float* mine = part + (((size_t)(w.r / rh) * a.H * a.maps + w.hm) * splits + c.split) * (4 + a.dv);
+                mine[0] = m2 ? m * kLn2 : m; mine[1] = l * unit;
+            }
+            return unit;
+        }
+        if (sigmoid()) return unit * a.out_scale;
+        float sum = l * unit;
+        if (a.sink) sum += m2 ? exp2f(fmaf(ca_sink(a, w.hm), kLog2e, -m)) : expf(ca_sink(a, w.hm) - m);
+        return unit * a.out_scale / sum;
+    }
+    // four finished output columns from col on
+    __device__ __forceinline__ void put(const Cta& c, const Row& w, uint32_t col, float4 v) const {
+        if (col >= dv(c)) return;                                     // a multiple of four, as col is
+        const size_t t = w.r / rh, at = (size_t)c.vs * vslice + col;
+        float* out = splits == 1 ? a.dst + t * a.dst_rs + (size_t)w.hm * a.dv + at : part + ((t * a.H * a.maps + w.hm) * splits + c.split) * (4 + a.dv) + 4 + at;
+        if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) *reinterpret_cast<float4*>(out) = v;
+        else { out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w; }
+    }
+};
+
+// DeviceOp.attention of a prompt (reference src/backend/reference.zig:599-671): one table entry per head, an additive mask in memory.  Entries
+// that read the same keys and values share their planes, entries with the same mask its tile classes.
+struct AtcProgram {
+    const ZgBatchEntry* tab;
+    const uint32_t* dyn;
+    const uint32_t* map;        // [count] planes of an entry, [count] its mask, [kv items] and [mask items] an entry that stands for the item
+    uint32_t count, kv_items, mask_items, seq_q, head, row_tiles, tiles;
+    uint8_t* classes;           // [mask items][row tiles][tiles]: what k_atc_masks found
+    uint32_t* bits;             // [mask items][row tiles][tiles][128 rows][4]: which keys of a tile a row sees
+    __device__ __forceinline__ const ZgBatchEntry& kv_entry(uint32_t item) const { return tab[map[2 * count + item]]; }
+    // keys that any entry of the item (offset 0: planes, `count`: masks) attends over; whole warps call it together
+    __device__ __forceinline__ uint32_t item_keys(uint32_t item, uint32_t offset) const {
+        uint32_t n = 0;
+        for (uint32_t i = threadIdx.x & 31; i < count; i += 32) if (map[offset + i] == item) n = max(n, dyn[tab[i].dyn]);
+        return min(__reduce_max_sync(0xffffffffu, n), tiles * 128);
+    }
+    __device__ __forceinline__ uint32_t prep_keys(uint32_t item) const { return item_keys(item, 0); }
+    struct Cta { const ZgBatchEntry* e; const uint8_t* cls; const uint32_t* bits; uint32_t r0, nq, n_keys, kv, t0, t1; bool masked; };
+    __device__ __forceinline__ Cta cta(uint32_t bk) const {
+        Cta c;
+        const uint32_t item = blockIdx.x % count, tile = row_tiles - 1 - blockIdx.x / count;      // under a causal mask later rows meet more keys
+        c.e = tab + item;
+        c.kv = map[item];
+        c.masked = c.e->u[0] != 0;
+        const size_t m = ((size_t)map[count + item] * row_tiles + tile) * tiles;
+        c.cls = classes + m; c.bits = bits + m * 512;
+        c.r0 = tile * 128; c.nq = min(128u, seq_q - c.r0);
+        c.n_keys = min(dyn[c.e->dyn], tiles * 128);
+        c.t0 = 0; c.t1 = (c.n_keys + bk - 1) / bk;
+        return c;
+    }
+    __device__ __forceinline__ uint32_t k_item(const Cta& c) const { return c.kv; }
+    __device__ __forceinline__ uint32_t v_item(const Cta& c) const { return c.kv; }
+    __device__ __forceinline__ uint32_t classify(const Cta& c, uint32_t t, uint32_t bk) const {
+        const uint32_t k = c.masked ? c.cls[t * bk / 128] : 1u;
+        return k == 1 && (t + 1) * bk > c.n_keys ? 2u : k;
+    }
+    struct Row { bool on; uint32_t r; };
+    __device__ __forceinline__ Row query(const Cta& c, uint32_t i) const {
+        Row w;
+        w.on = i < c.nq;
+        w.r = c.r0 + (w.on ? i : 0);
+        return w;
+    }
+    __device__ __forceinline__ const float* q_row(const Cta& c, const Row& w) const { return c.e->s0 + c.e->u[3] + (size_t)w.r * c.e->u[9]; }
+    __device__ __forceinline__ const float* mask_row(const Cta& c, const Row& w) const { return c.masked ? c.e->s3 + c.e->u[6] + (size_t)w.r * c.e->u[15] : nullptr; }
+    __device__ __forceinline__ uint32_t dk() const { return head; }
+    __device__ __forceinline__ uint32_t dv(const Cta&) const { return head; }
+    __device__ __forceinline__ float scale(const Cta& c) const { return c.e->f; }
+    __device__ __forceinline__ bool sigmoid() const { return false; }
+    __device__ __forceinline__ bool plain_tile() const { return true; }
+    // tile 2: keys seen or not, as the bits say; tile 3: the mask's values are added, four at a time (all at once they would not fit the registers)
     template <int N>
-    __device__ __forceinline__ void store(const Cta& c, const Row& w, uint32_t col, const float (&o)[N], float m, bool m2, float l, float unit) const {
-        const uint32_t n = dv(c) > col ? dv(c) - col : 0u, t = w.r / rh;
-        float* out;
-        float f;
-        if (splits == 1) {
-            out = a.dst + (size_t)t * a.dst_rs + (size_t)w.hm * a.dv + (size_t)c.vs * vslice + col;
-            float sum = l * unit;
-            if (!sigmoid() && a.sink) sum += m2 ? exp2f(fmaf(ca_sink(a, w.hm), kLog2e, -m)) : expf(ca_sink(a, w.hm) - m);
-            f = unit * a.out_scale * (sigmoid() ? 1.0f : 1.0f / sum);
-        } else {
-            float* mine = part + (((size_t)t * a.H * a.maps + w.hm) * splits + c.split) * (4 + a.dv);
-            if (c.vs == 0 && col == 0) { mine[0] = m2 ? m * kLn2 : m; mine[1] = l * unit; }
-            out = mine + 4 + (size_t)c.vs * vslice + col;
-            f = unit;
-        }
-        if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    __device__ __forceinline__ void scores(const Cta& c, const Row& w, uint32_t t, uint32_t u0, uint32_t cls, float (&x)[N]) const {
+        uint32_t seen = 0xffffffffu;                                  // of the 32 keys that hold u0 .. u0 + N - 1
+        if (c.masked) seen = c.bits[(size_t)(u0 >> 7) * 512 + (w.r - c.r0) * 4 + ((u0 >> 5) & 3)] >> (u0 & 31);
 #pragma unroll
-            for (int i = 0; i < N; i += 4)
-                if ((uint32_t)i + 4 <= n) *reinterpret_cast<float4*>(out + i) = make_float4(o[i] * f, o[i + 1] * f, o[i + 2] * f, o[i + 3] * f);
-        } else {
+        for (int i = 0; i < N; i++) if (!((seen >> i) & 1) || u0 + i >= c.n_keys) x[i] = -INFINITY;
+        if (cls < 3) return;
+        const float* mask = mask_row(c, w) + (size_t)u0 * c.e->u[14];
+        const uint32_t rs = c.e->u[14];
 #pragma unroll
-            for (int i = 0; i < N; i++) if ((uint32_t)i < n) out[i] = o[i] * f;
+        for (int i = 0; i < N; i += 4) {
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) { v[j] = u0 + i + j < c.n_keys ? *mask : 0.0f; mask += rs; }
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[i + j] = x[i + j] == -INFINITY ? -INFINITY : fmaf(v[j], kLog2e, x[i + j]);
+            asm volatile("" ::: "memory");
         }
+    }
+    __device__ __forceinline__ float slow_score(const Cta& c, const Row& w, uint32_t u, float dot) const {
+        if (u >= c.n_keys) return -INFINITY;
+        float s = dot * c.e->f;
+        if (c.masked) {
+            const float mv = mask_row(c, w)[(size_t)u * c.e->u[14]];
+            if (!isfinite(mv)) return -INFINITY;
+            s += mv;
+        }
+        return isfinite(s) ? s : -INFINITY;      // a non-finite score counts as masked, as in the reference
+    }
+    __device__ __forceinline__ float finish(const Cta&, const Row&, bool, float, bool, float l, float) const { return l > 0.0f ? 1.0f / l : 0.0f; }
+    __device__ __forceinline__ void put(const Cta& c, const Row& w, uint32_t col, float4 v) const {
+        float* out = c.e->dst + c.e->u[7] + (size_t)w.r * c.e->u[17] + col;
+        if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) *reinterpret_cast<float4*>(out) = v;
+        else { out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w; }
+        if (!c.e->dst2) return;
+        const size_t rs = c.e->d2_rs;
+        out = c.e->dst2 + c.e->d2_off + (size_t)w.r * c.e->d2_cs + col * rs;
+        if (rs == 1 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) *reinterpret_cast<float4*>(out) = v;
+        else { out[0] = v.x; out[rs] = v.y; out[2 * rs] = v.z; out[3 * rs] = v.w; }
     }
 };
 template <bool EXTRA>
@@ -266,6 +361,13 @@ template <bool EXTRA>
 __device__ __forceinline__ const float* src_key(const AtcCached<EXTRA>& s, const typename AtcCached<EXTRA>::Cta& c, uint32_t u) { return s.row(c.s, false, c.gm, u); }
 template <bool EXTRA>
 __device__ __forceinline__ const float* src_value(const AtcCached<EXTRA>& s, const typename AtcCached<EXTRA>::Cta& c, uint32_t u) { return s.row(c.s, true, c.g, u) + c.vs * s.vslice; }
+
+__device__ __forceinline__ const float* src_row(const AtcProgram& s, bool value, uint32_t item, uint32_t u) {
+    const ZgBatchEntry& e = s.kv_entry(item);
+    return value ? e.s2 + e.u[5] + (size_t)u * e.u[13] : e.s1 + e.u[4] + (size_t)u * e.u[11];
+}
+__device__ __forceinline__ const float* src_key(const AtcProgram&, const AtcProgram::Cta& c, uint32_t u) { return c.e->s1 + c.e->u[4] + (size_t)u * c.e->u[11]; }
+__device__ __forceinline__ const float* src_value(const AtcProgram&, const AtcProgram::Cta& c, uint32_t u) { return c.e->s2 + c.e->u[5] + (size_t)u * c.e->u[13]; }
 
 struct AtcPlanes {
     __half* k;           // [key items][tiles * 128][2 dkp]: hi | lo of a key
@@ -343,11 +445,49 @@ __global__ void __launch_bounds__(kPrepThreads) k_atc_prep(const Src src, const 
     }
 }
 
-// one row in plain f32 over the keys of the CTA's tiles, output columns col .. col + N - 1
+// A mask's 128 x 128 tiles: which entries are finite (bits), and the tile's class: 0 none, 1 all, and zero, 2 those that are are zero, 3 anything
+// else.  CTA (key tile, row tile, mask item); a warp takes eight rows, lane l of it keys l, l + 32, l + 64, l + 96, all loads in flight at once.
+__global__ void __launch_bounds__(512) k_atc_masks(const AtcProgram src) {
+    pdl_enter();
+    const ZgBatchEntry& e = src.tab[src.map[2 * src.count + src.kv_items + blockIdx.z]];
+    const uint32_t u0 = blockIdx.x * 128, r0 = blockIdx.y * 128, n_keys = src.item_keys(blockIdx.z, src.count), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (u0 >= n_keys) return;
+    const float* mask = e.s3 + e.u[6];
+    const size_t tile = ((size_t)blockIdx.z * src.row_tiles + blockIdx.y) * src.tiles + blockIdx.x;
+    float v[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t u = u0 + 32 * k + lane, r = r0 + 8 * warp + i;
+            v[i][k] = u < n_keys && r < src.seq_q ? mask[(size_t)u * e.u[14] + (size_t)r * e.u[15]] : 0.0f;      // what lies outside changes no class
+        }
+    bool any = false, all = true, zero = true;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        uint32_t word = 0;
+        const bool row = r0 + 8 * warp + i < src.seq_q;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const bool fin = isfinite(v[i][k]);
+            const uint32_t b = __ballot_sync(0xffffffffu, fin);
+            if (lane == k) word = b;
+            any = any || (fin && row && u0 + 32 * k + lane < n_keys);
+            all = all && fin;
+            zero = zero && (!fin || v[i][k] == 0.0f);
+        }
+        if (lane < 4) src.bits[tile * 512 + (8 * warp + i) * 4 + lane] = word;
+    }
+    const int a = __syncthreads_or(any), f = __syncthreads_and(all), z = __syncthreads_and(zero);
+    if (threadIdx.x == 0) src.classes[tile] = !a ? 0 : !z ? 3 : f ? 1 : 2;
+}
+
+// One row in plain f32 over the keys of the CTA's tiles: output columns col .. col + N - 1, and the factor they are to be multiplied by.
 template <int N, class Src>
-__device__ __noinline__ void atc_slow_row(const Src& src, const typename Src::Cta& c, const typename Src::Row& w, uint32_t col, uint32_t bk) {
-    float acc[N], m = -INFINITY, l = 0.0f;
+__device__ __noinline__ float atc_slow_row(const Src& src, const typename Src::Cta& c, const typename Src::Row& w, uint32_t col, uint32_t bk, bool first, float* acc) {
+    float m = -INFINITY, l = 0.0f;
     for (int i = 0; i < N; i++) acc[i] = 0.0f;
+    const float* q = src.q_row(c, w);
     const uint32_t dk = src.dk(), n = src.dv(c) > col ? min((uint32_t)N, src.dv(c) - col) : 0u;
     for (uint32_t t = c.t0; t < c.t1; t++) {
         if (!src.classify(c, t, bk)) continue;
@@ -355,7 +495,7 @@ __device__ __noinline__ void atc_slow_row(const Src& src, const typename Src::Ct
             if (src.slow_score(c, w, u, 0.0f) == -INFINITY) continue;          // not seen
             const float* k = src_key(src, c, u);
             float d = 0.0f;
-            for (uint32_t i = 0; i < dk; i++) d = fmaf(w.q[i], k[i], d);
+            for (uint32_t i = 0; i < dk; i++) d = fmaf(q[i], k[i], d);
             const float s = src.slow_score(c, w, u, d);
             float e;
             if (src.sigmoid()) e = s == -INFINITY ? 0.0f : ca_sigmoid(s);
@@ -371,7 +511,7 @@ __device__ __noinline__ void atc_slow_row(const Src& src, const typename Src::Ct
             for (uint32_t i = 0; i < n; i++) acc[i] = fmaf(e, v[i], acc[i]);
         }
     }
-    src.template store<N>(c, w, col, acc, m, false, l, 1.0f);
+    return src.finish(c, w, first, m, false, l, 1.0f);
 }
 
 // NC: 64-wide chunks of the key dimension; DV: value columns of the CTA (64 or 128)
@@ -381,7 +521,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     constexpr uint32_t BK = NC <= 2 ? 128 : 64, KC = BK / 64;       // keys per tile: scores twice, outputs and queries share the 512 columns of TMEM
     constexpr uint32_t kS = 0, kO = 2 * BK, kQ = kO + DV;           // TMEM columns; the CTA owns all 512, so their addresses are constants
     static_assert(kQ + 64 * NC <= 512, "TMEM columns");
-    constexpr uint32_t kPieceK = BK * 128, kPieceV = DV * 128;
+    constexpr uint32_t kPieceK = BK * 128, kPieceV = DV * 128, kQPieces = 2 * NC;       // 128 rows of 64 NC f32 queries
     extern __shared__ uint8_t dsm_raw[];
     const uint32_t base = (smem_u32(dsm_raw) + 1023u) & ~1023u, bars = base + kAtcRing * kAtcPiece + kAtcShare + kAtcTiles * 12;
     const uint32_t full = bars, empty = full + 8 * kAtcRing, s_full = empty + 8 * kAtcRing, p_full = s_full + 16, o_full = p_full + 8, q_full = o_full + 8, tmem_slot = q_full + 8;
@@ -399,6 +539,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     const typename Src::Cta c = src.cta(BK);
     // class and scales of the first tiles: read from global memory inside the loop they cost every tile an L2 round trip
     float* const share = reinterpret_cast<float*>(dsm_raw + (base - smem_u32(dsm_raw)) + kAtcRing * kAtcPiece);
+    float4* const ring = reinterpret_cast<float4*>(dsm_raw + (base - smem_u32(dsm_raw)));
     float2* const tile_inv = reinterpret_cast<float2*>(share + kAtcShare / 4);
     uint32_t* const tile_class = reinterpret_cast<uint32_t*>(tile_inv + kAtcTiles);
     const float* k_inv = pl.k_inv + (size_t)src.k_item(c) * pl.tiles;
@@ -419,6 +560,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             bool ok = true;
             auto piece = [&](const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bytes) {
                 if (ok) ok = mbar_wait(empty + 8 * slot, phase);
+                if (ok && phase && slot == kAtcRing - kQPieces) ok = mbar_wait(q_full, 0);       // first time round: the queries are staged there
                 if (!ok) return;
                 mbar_expect_tx(full + 8 * slot, bytes);
                 tma_2d(base + slot * kAtcPiece, map, x, y, full + 8 * slot);
@@ -520,16 +662,25 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             bar_sync(1 + (warp & 3), 128);
             return fmaxf(fmaxf(s[row], s[128 + row]), fmaxf(s[256 + row], s[384 + row]));
         };
+        // The queries come by whole rows (32 lanes, 512 contiguous bytes) into the ring's last pieces, which the loading warp leaves alone until
+        // q_full, and a thread takes its quarter row from there: read from global memory row by thread they took 9000 clocks.
+        float* const stage = share - (size_t)kQPieces * (kAtcPiece / 4);
+        constexpr uint32_t Q4 = 16 * NC;                             // float4s of a row; float4 j of row r lies at place j ^ (r & 7)
+        for (uint32_t i = threadIdx.x; i < 128 * Q4; i += 512) {
+            const uint32_t r = i / Q4, j = i % Q4;
+            const bool on = 4 * j < src.dk();
+            const float* from = src.q_row(c, src.query(c, r)) + 4 * j;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(stage + 4 * (r * Q4 + (j ^ (r & 7))))), "l"(on ? from : from - 4 * j), "r"(on ? 16 : 0) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        bar_sync(5, 512);
         float q_inv, q_scale;
         {
-            const uint32_t dk = src.dk();
             float4 x[4 * NC];                                        // 16 NC dims from 16 NC part on
             float mx = 0.0f;
 #pragma unroll
-            for (int i = 0; i < 4 * NC; i++) {
-                const uint32_t d = 16 * NC * part + 4 * i;
-                x[i] = d < dk ? *reinterpret_cast<const float4*>(w.q + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
+            for (int i = 0; i < 4 * NC; i++) x[i] = *reinterpret_cast<const float4*>(stage + 4 * (row * Q4 + ((4 * NC * part + i) ^ (row & 7))));
 #pragma unroll
             for (int i = 0; i < 4 * NC; i++) mx = abs_or_inf(abs_or_inf(abs_or_inf(abs_or_inf(mx, x[i].x), x[i].y), x[i].z), x[i].w);
             split_scale(row_max(mx), q_scale, q_inv);
@@ -546,6 +697,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             }
             tmem_wait_st();
             fence_before();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the ring's last pieces are read: TMA may write them
             __syncwarp();
             if (lane == 0) mbar_arrive(q_full);
         }
@@ -586,7 +738,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             float x[KW], alpha = 1.0f, shift = 14.0f;                // scores in units of log2; probabilities times 2^14
 #pragma unroll
             for (int j = 0; j < KW; j++) x[j] = __uint_as_float(v[j]) * f;
-            if (!plain) src.scores(c, w, u0, x);
+            if (!plain) src.scores(c, w, t, u0, cls, x);
             if (!sigmoid) {
                 float m0 = x[0], m1 = x[1];
 #pragma unroll
@@ -625,9 +777,22 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             bar_sync(1 + (warp & 3), 128);
             l = (s[row] + s[128 + row]) + (s[256 + row] + s[384 + row]);
         }
-        if (ok && w.on) {
-            if (slow) atc_slow_row<OW>(src, c, w, OW * part, BK);
-            else src.template store<OW>(c, w, OW * part, o, m, true, l, kPInv);
+        // Outputs leave by whole rows too, through the idle ring.
+        auto place = [&](int j) { return row * (DV / 4) + (((OW * part + j) / 4) ^ (row & 7)); };
+        if (slow && w.on) {
+            float acc[OW];
+            const float f = atc_slow_row<OW>(src, c, w, OW * part, BK, part == 0, acc);
+#pragma unroll 1
+            for (int j = 0; j < OW; j += 4) ring[place(j)] = make_float4(acc[j] * f, acc[j + 1] * f, acc[j + 2] * f, acc[j + 3] * f);
+        } else {
+            const float f = w.on && ok ? src.finish(c, w, part == 0, m, true, l, kPInv) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < OW; j += 4) ring[place(j)] = make_float4(o[j] * f, o[j + 1] * f, o[j + 2] * f, o[j + 3] * f);
+        }
+        bar_sync(5, 512);
+        for (uint32_t i = threadIdx.x; ok && i < c.nq * (DV / 4); i += 512) {
+            const uint32_t r = i / (DV / 4), j = i % (DV / 4);
+            src.put(c, src.query(c, r), 4 * j, ring[r * (DV / 4) + (j ^ (r & 7))]);
         }
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -737,4 +902,60 @@ bool zg_attention_tc_launch(const ZgAtcShape& s, const void* args, float* scratc
     }
     AtcCached<false> src = {a, P.rh, P.row_tiles, P.pl.n_vs, P.pl.vslice, P.splits, P.pl.tiles, *part};
     return launch_dims(src, P.pl, grid, st);
+}
+
+// ── DeviceOp.attention batches ──
+// Keys an op can ever attend over: the last row of its key, value and mask operands that lies inside their buffers (what refresh checks).
+static size_t attention_key_bound(const ZgOp& op, const size_t* elems) {
+    const auto& a = op.u.attention;
+    auto rows = [](size_t n, size_t off, size_t width, size_t stride) { return n < off + width ? (size_t)0 : stride ? (n - off - width) / stride + 1 : (size_t)UINT32_MAX; };
+    size_t n = std::min(rows(elems[a.k], a.k_off, a.d_head, a.k_cs), rows(elems[a.v], a.v_off, a.d_head, a.v_cs));
+    if (a.has_mask) n = std::min(n, rows(elems[a.mask], (size_t)a.mask_off + (size_t)(a.seq_q - 1) * a.mask_cs, 1, a.mask_rs));
+    return n;
+}
+bool zg_atc_program_plan(const ZgOp* const* ops, uint32_t count, const size_t* buffer_elems, ZgAtcPlan* plan) {
+    const auto& first = ops[0]->u.attention;
+    size_t keys = 0;
+    std::map<std::vector<uint32_t>, uint32_t> kv, masks;
+    std::vector<uint32_t> kv_rep, mask_rep;
+    plan->map.assign(2 * (size_t)count, 0);
+    for (uint32_t i = 0; i < count; i++) {
+        const auto& a = ops[i]->u.attention;
+        keys = std::max(keys, attention_key_bound(*ops[i], buffer_elems));
+        const auto k = kv.emplace(std::vector<uint32_t>{a.k, a.k_off, a.k_cs, a.v, a.v_off, a.v_cs}, (uint32_t)kv.size());
+        if (k.second) kv_rep.push_back(i);
+        plan->map[i] = k.first->second;
+        if (!a.has_mask) continue;
+        const auto m = masks.emplace(std::vector<uint32_t>{a.mask, a.mask_off, a.mask_rs, a.mask_cs}, (uint32_t)masks.size());
+        if (m.second) mask_rep.push_back(i);
+        plan->map[count + i] = m.first->second;
+    }
+    if (keys == 0 || keys > kAtcProgramKeys) return false;
+    plan->map.insert(plan->map.end(), kv_rep.begin(), kv_rep.end());
+    plan->map.insert(plan->map.end(), mask_rep.begin(), mask_rep.end());
+    plan->count = count; plan->kv_items = (uint32_t)kv_rep.size(); plan->mask_items = (uint32_t)mask_rep.size();
+    plan->seq_q = first.seq_q; plan->head = first.d_head; plan->tiles = (uint32_t)((keys + 127) / 128);
+    return true;
+}
+static AtcPlanes program_planes(const ZgAtcPlan& p) {
+    AtcPlanes pl = {};
+    pl.dkp = pl.vslice = pl.dk = pl.dv = p.head;
+    pl.k_items = pl.v_items = p.kv_items; pl.n_vs = 1; pl.tiles = p.tiles;
+    return pl;
+}
+static size_t mask_tiles(const ZgAtcPlan& p) { return (size_t)p.mask_items * ((p.seq_q + 127) / 128) * p.tiles; }
+size_t zg_atc_program_scratch_elems(const ZgAtcPlan& p) { return layout(program_planes(p)).total + mask_tiles(p) * 512 + (mask_tiles(p) + 3) / 4; }
+bool zg_atc_program_launch(const ZgAtcPlan& p, const ZgBatchEntry* d_entries, const uint32_t* d_map, const uint32_t* d_dyn, float* scratch, cudaStream_t st) {
+    AtcPlanes pl = program_planes(p);
+    place(pl, scratch);
+    const uint32_t row_tiles = (p.seq_q + 127) / 128;
+    AtcProgram src = {d_entries, d_dyn, d_map, p.count, p.kv_items, p.mask_items, p.seq_q, p.head, row_tiles, p.tiles, nullptr, nullptr};
+    src.bits = reinterpret_cast<uint32_t*>(scratch + layout(pl).total);
+    src.classes = reinterpret_cast<uint8_t*>(src.bits + mask_tiles(p) * 512);
+    if (p.mask_items) {
+        launch_pdl(k_atc_masks, dim3(p.tiles, row_tiles, p.mask_items), dim3(512), 0, st, src);
+        ZG_COUNT_LAUNCH();
+    }
+    const dim3 grid(row_tiles * p.count);
+    return p.head == 64 ? launch<AtcProgram, 1, 64>(src, pl, grid, st) : launch<AtcProgram, 2, 128>(src, pl, grid, st);
 }

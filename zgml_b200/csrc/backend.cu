@@ -95,6 +95,7 @@ struct ZgCudaProgram {
         ZgNormMacro nm = {};
         uint32_t attn_splits = 1; size_t attn_part_off = 0, attn_cnt_off = 0;   // split-KV decode attention scratch (per unit)
         ZgEwMulMacro em = {};
+        bool atc = false; ZgAtcPlan atc_plan;   // a batch of prompt attentions on the tensor cores, its planes in the shared GEMM scratch
     };
     std::vector<Unit> units;
     std::vector<uint32_t> entry_of_op;   // index into d_batch for batched op kinds
@@ -109,6 +110,7 @@ struct ZgCudaProgram {
     std::vector<InSeg> in_tab_host;   // what d_in_tab holds
     float* d_attn_part = nullptr;      // split-KV partial states, one slice per attention unit
     uint32_t* d_attn_cnt = nullptr;    // arrival counters (self re-arming)
+    uint32_t* d_atc_map = nullptr;     // which planes and mask classes the entries of the tensor-core attention units use
     bool uniform_pos = true;   // every patched slice_assign sits at the same position (checked per refresh)
     // quantized KV cache mode (zg_cuda_program_quantize_kv; LlamaInferenceSession.quantizeKV, src/llama_inference.zig:648-679):
     // Q8 caches stand in for the f32 cache buffers; the patched slice_assigns into them run storeColumn, the attention ops
@@ -258,7 +260,7 @@ static void free_program(ZgCudaProgram* p) {
         if (i >= p->buffer_extern.size() || !p->buffer_extern[i]) cudaFree(p->buffers[i]);
     for (size_t i = 0; i < p->qweights.size(); i++)
         if (p->qweight_owned[i]) zg_cuda_qweight_free(p->ctx, p->qweights[i]);
-    cudaFree(p->d_steps); cudaFree(p->d_dyn); cudaFree(p->d_batch); cudaFree(p->d_chain); cudaFree(p->d_attn_part); cudaFree(p->d_attn_cnt);
+    cudaFree(p->d_steps); cudaFree(p->d_dyn); cudaFree(p->d_batch); cudaFree(p->d_chain); cudaFree(p->d_attn_part); cudaFree(p->d_attn_cnt); cudaFree(p->d_atc_map);
     cudaFree(p->d_in_stage); cudaFree(p->d_in_tab);
     if (p->h_in_stage) cudaFreeHost(p->h_in_stage);
     if (p->h_dyn) cudaFreeHost(p->h_dyn);
@@ -1667,6 +1669,28 @@ static bool build_schedule(ZgCudaProgram* p) {
         ZG_CUDA_OK(cudaMalloc(&p->d_attn_cnt, cnt_total * sizeof(uint32_t)));
         ZG_CUDA_OK(cudaMemset(p->d_attn_cnt, 0, cnt_total * sizeof(uint32_t)));
     }
+    // prompt attentions on the tensor cores: their planes lie in the shared GEMM scratch, whose virtual buffer orders them with its other users
+    cudaFree(p->d_atc_map); p->d_atc_map = nullptr;
+    std::vector<uint32_t> atc_map;
+    size_t atc_scratch = 0;
+    for (auto& u : p->units) {
+        if (!u.batched || u.entry_ops.empty() || p->ops[u.entry_ops[0]].tag != ZG_OP_ATTENTION || !zg_attention_prefill_ok(p->ops[u.entry_ops[0]])) continue;
+        std::vector<const ZgOp*> ops;
+        for (uint32_t i : u.entry_ops) ops.push_back(&p->ops[i]);
+        if (!zg_atc_program_plan(ops.data(), (uint32_t)ops.size(), p->buffer_elems.data(), &u.atc_plan)) continue;
+        u.atc = true;
+        u.atc_plan.map_off = atc_map.size();
+        atc_map.insert(atc_map.end(), u.atc_plan.map.begin(), u.atc_plan.map.end());
+        atc_scratch = std::max(atc_scratch, zg_atc_program_scratch_elems(u.atc_plan));
+        std::vector<ZgRange> tmp;
+        for (uint32_t i : u.ops) { op_ranges(p, p->ops[i], tmp); u.ranges.insert(u.ranges.end(), tmp.begin(), tmp.end()); }
+        u.ranges.push_back({(uint32_t)p->buffers.size(), 0, 1, true, 0});
+    }
+    if (!atc_map.empty()) {
+        ZG_CUDA_OK(cudaMalloc(&p->d_atc_map, atc_map.size() * sizeof(uint32_t)));
+        ZG_CUDA_OK(cudaMemcpy(p->d_atc_map, atc_map.data(), atc_map.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+        if (!zg_gemv_ws_reserve(&p->ws, 0, 0, p->ctx->stream, atc_scratch)) return false;
+    }
     // single-op launches (profiling / eager per-op mode) of batched kinds need their own plain entries
     p->single_entry.assign(n, 0);
     for (size_t i = 0; i < n; i++) {
@@ -1767,6 +1791,7 @@ static bool launch_unit(ZgCudaProgram* p, const ZgCudaProgram::Unit& u, cudaStre
         return zg_qgemv_launch_batch(p->ctx, cnt, w, xin, xout, p->ops[u.entry_ops[0]].u.qmatmul.M, irs, ors, view, st, u.pros.data());
     }
     if (!u.batched) return launch_one(p, u.ops[0], st);
+    if (u.atc) return zg_atc_program_launch(u.atc_plan, p->d_batch + u.first_entry, p->d_atc_map + u.atc_plan.map_off, p->d_dyn, p->ws.gemm_scratch, st);
     if (u.attn_splits > 1)
         return zg_launch_batch(p->ops[u.entry_ops[0]], p->d_batch + u.first_entry, u.n_entries, p->d_dyn, st,
                                p->d_attn_part + u.attn_part_off, p->d_attn_cnt + u.attn_cnt_off, u.attn_splits);

@@ -2037,6 +2037,7 @@ bool zg_launch_attention_layer(const ZgAttnBlock* d_blk, uint32_t n_heads, uint3
 
 // `first` = any op of the batch (all share the work shape); `d_entries` = `count` consecutive table entries.
 // Decode attention: how many CTAs share one head's kv range (1 = no split).  `count` ops x seq_q rows are in the launch.
+bool zg_attention_prefill_ok(const ZgOp& op) { return attn_prefill_ok(op); }
 uint32_t zg_attention_splits(const ZgOp& op, size_t k_buffer_elems, uint32_t count, int sm_count) {
     const auto& a = op.u.attention;
     if (!attn_fast_ok(op) || a.seq_q == 0 || a.seq_q > 8 || a.k_cs == 0) return 1;

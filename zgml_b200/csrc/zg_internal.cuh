@@ -252,6 +252,12 @@ uint64_t zg_batch_signature(const ZgOp& op);
 bool zg_fill_batch_entry(const ZgOp& op, float* const* bufs, uint32_t op_index, ZgBatchEntry* e);
 bool zg_launch_batch(const ZgOp& first, const ZgBatchEntry* d_entries, uint32_t count, const uint32_t* d_dyn, cudaStream_t st,
                      float* attn_part = nullptr, uint32_t* attn_cnt = nullptr, uint32_t attn_splits = 1);
+// attention_tc.cu: the same batch of prompt attentions on the tensor cores.  A plan belongs to one launch unit; its map goes to device memory.
+struct ZgAtcPlan { uint32_t count = 0, kv_items = 0, mask_items = 0, seq_q = 0, head = 0, tiles = 0; std::vector<uint32_t> map; size_t map_off = 0; };
+bool zg_attention_prefill_ok(const ZgOp& op);   // ops.cu: the layouts the prompt kernels take
+bool zg_atc_program_plan(const ZgOp* const* ops, uint32_t count, const size_t* buffer_elems, ZgAtcPlan* plan);   // false: keep the SIMT kernel
+size_t zg_atc_program_scratch_elems(const ZgAtcPlan& plan);
+bool zg_atc_program_launch(const ZgAtcPlan& plan, const ZgBatchEntry* d_entries, const uint32_t* d_map, const uint32_t* d_dyn, float* scratch, cudaStream_t st);
 uint32_t zg_attention_splits(const ZgOp& op, size_t k_buffer_elems, uint32_t count, int sm_count);
 size_t zg_attention_part_elems(const ZgOp& op, uint32_t count, uint32_t splits);
 bool zg_launch_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, const uint32_t* d_dyn,
