@@ -561,6 +561,16 @@ __global__ void k_slice_assign(const ZgBatchEntry* __restrict__ tab, const uint3
     const uint32_t doff = d_dyn[e.dyn];
     float* __restrict__ dst = e.dst;
     const float* __restrict__ src = e.s0;
+    // rows that lie together on both sides at 16-byte boundaries: four at a time
+    if (drs == 1 && srs == 1 && ((rows | doff | soff | dcs | scs) & 3) == 0 && ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0) {
+        const uint32_t r4 = rows >> 2, total = r4 * cols;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+            const uint32_t col = i / r4, row = 4 * (i - col * r4);
+            *reinterpret_cast<float4*>(dst + (size_t)doff + row + (size_t)col * dcs) = *reinterpret_cast<const float4*>(src + (size_t)soff + row + (size_t)col * scs);
+        }
+        ZG_TRACE_MARK(2)
+        return;
+    }
     uint32_t total = rows * cols;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         uint32_t row = i % rows, col = i / rows;
@@ -578,6 +588,23 @@ __global__ void k_rope(const ZgBatchEntry* __restrict__ tab) {
     float* __restrict__ dst = e.dst;
     const float* __restrict__ src = e.s0;
     const float* __restrict__ cs = e.s1;
+    if (s_rs == 1 && ((hd | s_off | c_off | d_off | s_cs | c_cs) & 3) == 0 &&
+        ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(cs)) & 15) == 0) {      // four pairs at a time
+        const uint32_t h4 = hd >> 2, total = h4 * seq_len;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+            const uint32_t col = i / h4, pair = 4 * (i - col * h4);
+            const float* x = src + (size_t)s_off + pair + (size_t)col * s_cs;
+            const float* t = cs + (size_t)c_off + pair + (size_t)col * c_cs;
+            const float4 lo = *reinterpret_cast<const float4*>(x), hi = *reinterpret_cast<const float4*>(x + hd), c = *reinterpret_cast<const float4*>(t), sn = *reinterpret_cast<const float4*>(t + hd);
+            float* y = dst + (size_t)d_off + pair + (size_t)col * 2 * hd;
+            *reinterpret_cast<float4*>(y) = make_float4(__fsub_rn(__fmul_rn(lo.x, c.x), __fmul_rn(hi.x, sn.x)), __fsub_rn(__fmul_rn(lo.y, c.y), __fmul_rn(hi.y, sn.y)),
+                                                        __fsub_rn(__fmul_rn(lo.z, c.z), __fmul_rn(hi.z, sn.z)), __fsub_rn(__fmul_rn(lo.w, c.w), __fmul_rn(hi.w, sn.w)));
+            *reinterpret_cast<float4*>(y + hd) = make_float4(__fadd_rn(__fmul_rn(hi.x, c.x), __fmul_rn(lo.x, sn.x)), __fadd_rn(__fmul_rn(hi.y, c.y), __fmul_rn(lo.y, sn.y)),
+                                                             __fadd_rn(__fmul_rn(hi.z, c.z), __fmul_rn(lo.z, sn.z)), __fadd_rn(__fmul_rn(hi.w, c.w), __fmul_rn(lo.w, sn.w)));
+        }
+        ZG_TRACE_MARK(2)
+        return;
+    }
     uint32_t total = hd * seq_len;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         uint32_t pair = i % hd, col = i / hd;
@@ -2059,13 +2086,13 @@ bool zg_launch_batch(const ZgOp& first, const ZgBatchEntry* d_entries, uint32_t 
         case ZG_OP_SLICE_ASSIGN: {
             const auto& sa = first.u.slice_assign;
             if (sa.rows == 0 || sa.cols == 0) return true;
-            launch_k(k_slice_assign, dim3(dim3(blocks_for(sa.rows * sa.cols, 256), count)), dim3(256), st, d_entries, d_dyn);
+            launch_k(k_slice_assign, dim3(blocks_for(sa.rows % 4 ? sa.rows * sa.cols : sa.rows * sa.cols / 4, 256), count), dim3(256), st, d_entries, d_dyn);
             break;
         }
         case ZG_OP_ROPE: {
             const auto& r = first.u.rope;
             if (r.half_d == 0 || r.seq_len == 0) return true;
-            launch_k(k_rope, dim3(dim3(blocks_for(r.half_d * r.seq_len, 128), count)), dim3(128), st, d_entries);
+            launch_k(k_rope, dim3(blocks_for(r.half_d % 4 ? r.half_d * r.seq_len : r.half_d * r.seq_len / 4, 128), count), dim3(128), st, d_entries);
             break;
         }
         case ZG_OP_ATTENTION: {
