@@ -1677,6 +1677,9 @@ static uint32_t attention_splits(const ZgSeqOp& s) {
     if (S > window / 32) S = window / 32;
     return S < 2 ? 1 : (S > 16 ? 16 : S);
 }
+static bool linear_split(const ZgSeqOp& s, float* const* bufs) {     // f32 weights, many rows: split operands on the tensor cores
+    return zg_split_gemm_usable(wptr<float>(bufs, s.buf[2], s.off[0]), bufs[s.buf[1]] + s.off[2], s.n[0], s.n[10] ? 2 * s.n[1] : s.n[1], s.n[2], s.n[3], s.n[7]);
+}
 size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs) {
     if (op.tag >= ZG_OP_STREAM_STEP) return 0;
     if (op.tag >= ZG_OP_SSM_SCAN) return zg_rec_op_scratch_elems(op);
@@ -1689,8 +1692,9 @@ size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs) {
         const ZgSeqOp& d = op.u.seq;
         return d.n[0] >= (uint32_t)kDeltaPrepMinTokens && d.n[3] <= (uint32_t)kWalkMaxDim ? (size_t)d.n[0] * d.n[1] * ((d.n[10] & kDeltaHeadDecay ? 2 : 3) * delta_walk_slices(d.n[3]) * kWalkRows + 4) : 0;
     }
-    if (!dense_gemm_enabled() || op.tag != ZG_OP_LINEAR || op.u.seq.n[5] != ZG_W_BF16) return 0;
+    if (!dense_gemm_enabled() || op.tag != ZG_OP_LINEAR) return 0;
     const ZgSeqOp& s = op.u.seq;
+    if (s.n[5] == ZG_W_F32) return linear_split(s, bufs) ? zg_split_gemm_scratch_elems(s.n[0], s.n[10] ? 2 * s.n[1] : s.n[1], s.n[2]) : 0;
     if (!zg_dense_gemm_usable(wptr<bf16>(bufs, s.buf[2], s.off[0]), s.n[0], s.n[10] ? 2 * s.n[1] : s.n[1], s.n[2])) return 0;
     return zg_dense_gemm_scratch_elems(s.n[0], s.n[2]);
 }
@@ -1713,6 +1717,9 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             const bool pairs = s.n[10] != 0;
             const SeqAct act = {s.n[6], s.f[0], s.n[8], s.n[9] ? s.n[9] : N};
             const float* slot_ctl = s.n[7] ? (const float*)bufs[s.buf[4]] : (const float*)nullptr;      // the source is the slot's part of a state buffer
+            if (scratch && s.n[5] == ZG_W_F32 && zg_seq_op_scratch_elems(op, bufs))
+                return zg_split_gemm_launch(wptr<float>(bufs, s.buf[2], s.off[0]), has_bias ? wptr<float>(bufs, s.buf[3], s.off[1]) : nullptr, src, dst, M, pairs ? 2 * N : N, K,
+                                            s.n[3], s.n[4], scratch, st, s.n[6], s.f[0], act.lo, act.hi, slot_ctl, s.n[7], pairs, s.n[11]);
             if (scratch && zg_seq_op_scratch_elems(op, bufs))
                 return zg_dense_gemm_launch(wptr<bf16>(bufs, s.buf[2], s.off[0]), has_bias ? wptr<bf16>(bufs, s.buf[3], s.off[1]) : nullptr, src, dst, M, N, K,
                                             s.n[3], s.n[4], scratch, st, s.n[6], s.f[0], act.lo, act.hi, slot_ctl, s.n[7], pairs, s.n[11]);

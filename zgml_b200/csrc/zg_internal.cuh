@@ -385,6 +385,11 @@ size_t zg_dense_gemm_scratch_elems(uint32_t M, uint32_t K);
 unsigned int zg_dense_gemm_timeouts();
 bool zg_dense_gemm_grouped_launch(const void* w_bf16, uint32_t groups, const void* xb, uint32_t rows, uint32_t Kp, const int* d_tile_group, float* dst,
                                   uint32_t N, uint32_t K, uint32_t dst_rs, cudaStream_t st);
+// split_gemm.cu : f32 x f32 -> f32 LINEAR of many rows, operands split into half-precision pairs (arguments as zg_dense_gemm_launch's; N counts weight rows)
+bool zg_split_gemm_usable(const float* w, const float* src, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t slot_stride);
+size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K);
+bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, cudaStream_t st,
+                          uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from);
 // mixops.cu : ZG_OP_TOKEN_SHIFT .. ZG_OP_POLY_NORM, reached through the functions above
 bool zg_mix_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* why, size_t why_n);
 uint32_t zg_mix_op_writes(uint32_t tag);
