@@ -1046,165 +1046,264 @@ __global__ void __launch_bounds__(kDeltaThreads) k_delta_rule(
         if (live && row < dim) S_g[(size_t)row * vdim + col] = S[i];
     }
 }
-// Prefill form of DELTA_RULE (kDeltaPrepMinTokens or more tokens): the per-token vectors are prepared for ALL tokens at
-// once by k_delta_prepare (one warp per (token, head); the walk's critical path then holds no transcendental and no global
-// read), into rows [unit k | scaled unit q | decay | beta, k . q, 0, 0] of 3 dpad + 4 floats laid out [head][token], so
-// that a tile of tokens is one contiguous, 16-byte aligned block.  k_delta_walk streams those tiles into shared memory with
-// cp.async, double buffered, and walks the tokens.  Per token a thread scales its rows by the decay and takes BOTH dot
-// products, with k and with q, in the same pass; one shuffle round reduces them together.  The read-out after the write
-// follows from  o = (g S)^T q + u (k . q), so the state update S <- g S + k u^T leaves the output's critical path.
-// A thread's kWalkRows rows are groups of four consecutive rows, group c of slice r at row (c RS + r) 4: the RS slices
-// of a column read consecutive float4s of a prepared vector (no bank conflict; the columns of a warp read the same words).
+// Prefill form of DELTA_RULE (kDeltaPrepMinTokens or more tokens): four tokens at a time.  With D_l the decay of token l of a block (a diagonal) and S the
+// state before it, every token's two products follow from products with S itself:
+//   S_j^T x = S^T (D_1 .. D_j x) + sum_{i <= j} (x^T D_{i+1} .. D_j k_i) u_i,
+// so the eight products of a block with the state are independent, are reduced together, and what remains between the tokens of a block is a
+// triangular solve of four scalars per value column:
+//   u_j = beta_j (v_j - A_j^T S - sum_{i < j} ckk_ij u_i),   o_j = Q_j^T S + sum_{i <= j} cqk_ij u_i,   S <- Gamma S + sum_j B_j u_j^T.
+// Only products of decays occur (nothing is divided by one), so the form is as sound as token by token for any decay.  k_delta_prepare (one warp per
+// (block, head)) leaves per block the vectors [A_1 .. A_4 | Q_1 .. Q_4 | B_1 .. B_4 | Gamma] and the scalars [beta (4) | ckk (4 x 4) | cqk (4 x 4)], zero
+// where i does not precede j, laid out [head][block]; a plain accumulation (u = v) has no A and no solve.  k_delta_walk streams them into shared memory
+// with cp.async, double buffered.
+// A warp owns two value columns; a lane holds R key rows of both.  What a thread reads of the prepared vectors per column it owns bounds the kernel
+// where a column has few threads (one thread per 16 rows of one column: 832 clocks of shared-memory reads per block and SM), the latency of a block
+// where a warp has many columns (four: 1280 clocks per block, 29 % of the issue slots).  The 16 sums (8 products, 2 columns) are reduced over the
+// lanes by halving what is left each time, and end one per lane: lane (column, k or q, token).
 constexpr int kDeltaPrepMinTokens = 16;
-// The walk keeps 16 rows per thread (four groups of four) and 128 threads per CTA.  (8 rows and 256 threads, two warps per
-// scheduler, was measured slower: 388 against 354 us at 16 heads of 128 x 128 — the per-token dependency chain, which a
-// fourth shuffle step lengthens, is what bounds the kernel, not the empty issue slots.)
-constexpr int kWalkRows = 16, kWalkThreads = 128, kWalkMaxDim = 32 * kWalkRows;
-static uint32_t delta_walk_slices(uint32_t dim) {
-    uint32_t rs = 1;
-    while (rs * kWalkRows < dim) rs <<= 1;
-    return rs;
+constexpr int kWalkThreads = 256, kWalkMaxDim = 512, kWalkBlock = 4, kWalkScalars = 36, kWalkCols = 2;
+static uint32_t delta_walk_rows(uint32_t dim) { return dim <= 64 ? 2 : dim <= 128 ? 4 : dim <= 256 ? 8 : 16; }      // key rows per lane
+__host__ __device__ constexpr uint32_t delta_block_elems(uint32_t dpad, bool plain) { return ((plain ? 2 : 3) * kWalkBlock + 1) * dpad + kWalkScalars; }
+// N values in every lane -> the total of value lane % N
+template <int N>
+__device__ __forceinline__ float reduce_scatter(float (&v)[N], uint32_t lane) {
+#pragma unroll
+    for (int o = N / 2; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (int o = N; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
 }
-__device__ __forceinline__ uint32_t delta_row(uint32_t RS, uint32_t r, int i) { return (((uint32_t)i >> 2) * RS + r) * 4 + ((uint32_t)i & 3); }
-template <typename WT>
+template <typename WT, int R>
 __global__ void k_delta_prepare(float* __restrict__ prep, const float* __restrict__ qkv, const float* __restrict__ betab, const float* __restrict__ ab,
-                                const WT* __restrict__ wts, uint32_t T, uint32_t H, uint32_t G, uint32_t dim, uint32_t dpad, uint32_t q_off,
+                                const WT* __restrict__ wts, uint32_t T, uint32_t H, uint32_t G, uint32_t dim, uint32_t q_off,
                                 uint32_t k_off, uint32_t beta_off, uint32_t A_off, uint32_t dt_off, uint32_t qkv_rs, uint32_t beta_rs, uint32_t a_rs,
                                 float unit_eps, float q_scale, uint32_t form, float inv_tau, uint32_t u_off) {
     pdl_enter();
-    const bool plain = form & kDeltaPlain, head_decay = form & kDeltaHeadDecay;
-    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (w >= T * H) return;
-    const uint32_t t = w / H, h = w % H, kv = h / (H / G);
-    const float* qr = qkv + (size_t)t * qkv_rs + q_off + (size_t)kv * dim;
-    const float* kr = qkv + (size_t)t * qkv_rs + k_off + (size_t)kv * dim;
-    const float* ar = ab + (size_t)t * a_rs + (head_decay ? (size_t)h : (size_t)h * dim);
-    float qq = 0.0f, kk = 0.0f, qk = 0.0f;
-    for (uint32_t c = lane; c < dim; c += 32) { const float a = qr[c], b = kr[c]; qq = fmaf(a, a, qq); kk = fmaf(b, b, kk);
-        qk = fmaf(a, (form & kDeltaBonus) ? b * wld(wts, (size_t)u_off + (size_t)h * dim + c) : b, qk); }
-    const float qn = plain ? q_scale : q_scale / sqrtf(warp_sum(qq) + unit_eps), kn = plain ? 1.0f : 1.0f / sqrtf(warp_sum(kk) + unit_eps);
-    qk = warp_sum(qk) * qn * kn;
-    const float Ah = (form & (kDeltaSigmoidDecay | kDeltaExpDecay)) ? 0.0f : expf(wld(wts, (size_t)A_off + h));
-    float* row = prep + ((size_t)h * T + t) * ((head_decay ? 2 : 3) * dpad + 4);
-    const float gh = head_decay ? delta_decay(ar[0] + wld(wts, (size_t)dt_off + h), Ah, form, inv_tau) : 0.0f;
-    for (uint32_t c = lane; c < dpad; c += 32) {
-        const bool in = c < dim;
-        row[c] = in ? kr[c] * kn : 0.0f;
-        row[dpad + c] = in ? qr[c] * qn : 0.0f;
-        if (!head_decay) row[2 * dpad + c] = in ? delta_decay(ar[c] + wld(wts, (size_t)dt_off + (size_t)h * dim + c), Ah, form, inv_tau) : 1.0f;
+    constexpr int B = kWalkBlock;
+    constexpr uint32_t dpad = 32 * R;
+    const bool plain = form & kDeltaPlain, head_decay = form & kDeltaHeadDecay, bonus = form & kDeltaBonus;
+    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31, blocks = (T + B - 1) / B;
+    if (w >= blocks * H) return;
+    const uint32_t b = w / H, h = w % H, kv = h / (H / G), n = min((uint32_t)B, T - b * B);
+    const float* qr = qkv + (size_t)b * B * qkv_rs + q_off + (size_t)kv * dim;
+    const float* kr = qkv + (size_t)b * B * qkv_rs + k_off + (size_t)kv * dim;
+    const float* ar = ab + (size_t)b * B * a_rs + (head_decay ? (size_t)h : (size_t)h * dim);
+    float k[B][R], q[B][R], D[B][R];                                 // every load in flight at once
+#pragma unroll
+    for (int j = 0; j < B; j++)
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const uint32_t c = lane + 32 * i;
+            const bool on = c < dim && (uint32_t)j < n;              // tokens past the step's end: nothing is written, nothing decays
+            k[j][i] = on ? kr[(size_t)j * qkv_rs + c] : 0.0f;
+            q[j][i] = on ? qr[(size_t)j * qkv_rs + c] : 0.0f;
+            D[j][i] = on ? ar[(size_t)j * a_rs + (head_decay ? 0 : c)] : 0.0f;
+        }
+    float bias[R], own[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const uint32_t c = lane + 32 * i;
+        bias[i] = c < dim ? wld(wts, (size_t)dt_off + (head_decay ? (size_t)h : (size_t)h * dim + c)) : 0.0f;
+        own[i] = bonus && c < dim ? wld(wts, (size_t)u_off + (size_t)h * dim + c) : 1.0f;
     }
-    if (lane < 4) row[(head_decay ? 2 : 3) * dpad + lane] = lane == 0 ? (plain ? 1.0f : sigmoidf_(betab[(size_t)t * beta_rs + beta_off + h])) : (lane == 1 ? qk : (lane == 2 ? gh : 0.0f));
+    const float Ah = (form & (kDeltaSigmoidDecay | kDeltaExpDecay)) ? 0.0f : expf(wld(wts, (size_t)A_off + h));
+    const float beta = plain || lane >= n ? 0.0f : betab[((size_t)b * B + lane) * beta_rs + beta_off + h];
+    float scale = (lane & 4) ? 1.0f : q_scale;                       // lane j: of q_j, lane 4 + j: of k_j
+    if (!plain) {
+        float sq[2 * B];
+#pragma unroll
+        for (int j = 0; j < B; j++) {
+            float qq = 0.0f, kk = 0.0f;
+#pragma unroll
+            for (int i = 0; i < R; i++) { qq = fmaf(q[j][i], q[j][i], qq); kk = fmaf(k[j][i], k[j][i], kk); }
+            sq[j] = qq; sq[B + j] = kk;
+        }
+        scale /= sqrtf(reduce_scatter<2 * B>(sq, lane) + unit_eps);
+    }
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+        const float qn = __shfl_sync(0xffffffffu, scale, j), kn = __shfl_sync(0xffffffffu, scale, B + j);
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            k[j][i] *= kn; q[j][i] *= qn;
+            if (i && head_decay) D[j][i] = D[j][0];                  // one decay for all rows (what lies past `dim` is zero, whatever its decay)
+            else D[j][i] = lane + 32 * i < dim && (uint32_t)j < n ? delta_decay(D[j][i] + bias[i], Ah, form, inv_tau) : 1.0f;
+        }
+    }
+    float* P = prep + ((size_t)h * blocks + b) * delta_block_elems(dpad, plain);
+    float* PQ = P + (plain ? 0 : B) * dpad;
+    float* PB = PQ + B * dpad;
+    float c[16] = {};                                                // cqk_ij at j (j + 1) / 2 + i, ckk_ij at 10 + j (j - 1) / 2 + i
+#pragma unroll
+    for (int e = 0; e < R; e++) {
+        const uint32_t at = lane + 32 * e;
+        float g = 1.0f;
+#pragma unroll
+        for (int j = 0; j < B; j++) {
+            const float before = g;
+            g *= D[j][e];
+            if (!plain) P[j * dpad + at] = g * k[j][e];
+            PQ[j * dpad + at] = (bonus ? before : g) * q[j][e];       // the bonus form reads the state before the token decays it
+        }
+        PB[B * dpad + at] = g;
+        float s = 1.0f;
+#pragma unroll
+        for (int j = B - 1; j >= 0; j--) { PB[j * dpad + at] = s * k[j][e]; s *= D[j][e]; }
+#pragma unroll
+        for (int i = 0; i < B; i++) {
+            float& self = c[i * (i + 1) / 2 + i];
+            self = fmaf(q[i][e] * own[e], k[i][e], self);
+            float d = k[i][e];                                       // what token i wrote, as the later tokens find it
+#pragma unroll
+            for (int j = i + 1; j < B; j++) {
+                float& qk = c[j * (j + 1) / 2 + i];
+                if (bonus) qk = fmaf(q[j][e], d, qk);
+                d *= D[j][e];
+                if (!bonus) qk = fmaf(q[j][e], d, qk);
+                if (!plain) { float& kk = c[10 + j * (j - 1) / 2 + i]; kk = fmaf(k[j][e], d, kk); }
+            }
+        }
+    }
+    float* sc = PB + (B + 1) * dpad;
+    if (lane < (uint32_t)B) sc[lane] = plain || lane >= n ? 0.0f : sigmoidf_(beta);
+    const uint32_t cj = (lane >> 2) & 3, ci = lane & 3;               // lane 4 j + i: ckk_ij, lane 16 + 4 j + i: cqk_ij
+    const float total = reduce_scatter<16>(c, lane);
+    const float mine = __shfl_sync(0xffffffffu, total, lane < 16 ? 10 + cj * (cj - 1) / 2 + ci : cj * (cj + 1) / 2 + ci);
+    sc[B + lane] = (lane < 16 ? ci < cj : ci <= cj) ? mine : 0.0f;
 }
 __device__ __forceinline__ void cp_async16(float* smem_dst, const float* gmem_src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gmem_src) : "memory");
 }
-// PLAIN: the accumulation without correction (u = v), which needs no product with k and only one reduction per token
-// HEADG: one decay per head and token.  It commutes with the sums over the key rows, so both dot products run on the state as
-// the token finds it and the decay joins the two results: u = beta (v - g S^T k), o = g S^T q + u (k . q), S <- g S + k u^T.
-// BONUS (PLAIN): the state as the token finds it, not yet decayed, is what is read; k . q of the prepared row carries the bonus
-template <uint32_t RS, bool PLAIN, bool HEADG, bool BONUS>         // row slices of a column: compile-time, so the shuffle steps unroll
+template <int R, bool PLAIN>                       // key rows per lane
 __global__ void __launch_bounds__(kWalkThreads) k_delta_walk(float* __restrict__ dst, const float* __restrict__ qkv, const float* __restrict__ prep,
                                                                float* __restrict__ state, const float* __restrict__ ctl, uint32_t T, uint32_t H,
                                                                uint32_t dim, uint32_t vdim, uint32_t v_off, uint32_t qkv_rs, uint32_t dst_rs) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
-    const uint32_t dpad = RS * kWalkRows, tail = (HEADG ? 2 : 3) * dpad, stride = tail + 4, tile_elems = kDeltaTile * stride;
-    const uint32_t h = blockIdx.y;
-    const uint32_t cols_per_cta = kWalkThreads / RS;
-    const uint32_t r = threadIdx.x % RS, col = blockIdx.x * cols_per_cta + threadIdx.x / RS;
-    const bool live = col < vdim;
+    constexpr int B = kWalkBlock, C = kWalkCols, VR = R < 4 ? R : 4, NG = R / VR, Q = PLAIN ? 0 : B, W = Q + B;      // vectors before Q's and before B's
+    constexpr uint32_t dpad = 32 * R, block_elems = delta_block_elems(dpad, PLAIN), tile_blocks = kDeltaTile / B, tile_elems = tile_blocks * block_elems;
+    const uint32_t h = blockIdx.y, blocks = (T + B - 1) / B, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t col0 = (blockIdx.x * (kWalkThreads / 32) + warp) * C;                     // the warp's first column
     const uint32_t slot = (uint32_t)ctl_word(ctl, ZG_CTL_SLOT);
     float* S_g = state + (((size_t)slot * H + h) * dim) * vdim;
-    float S[kWalkRows];
+    auto row_of = [&](int i) { return ((uint32_t)(i / VR) * 32 + lane) * VR + (uint32_t)(i % VR); };
+    float2 S[C][R / 2];
 #pragma unroll
-    for (int i = 0; i < kWalkRows; i++) {
-        const uint32_t row = delta_row(RS, r, i);
-        S[i] = (live && row < dim) ? S_g[(size_t)row * vdim + col] : 0.0f;
-    }
-    const float* P = prep + (size_t)h * T * stride;
-    const float* vbase = qkv + v_off + (size_t)h * vdim + col;
-    auto stage = [&](uint32_t t0, float* buf) {       // rows of tokens [t0, min(t0 + tile, T)): one contiguous block
-        const uint32_t n4 = min((uint32_t)kDeltaTile, T - t0) * stride / 4;
-        const float* src = P + (size_t)t0 * stride;
+    for (int i = 0; i < R; i++)
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const float x = row_of(i) < dim && col0 + c < vdim ? S_g[(size_t)row_of(i) * vdim + col0 + c] : 0.0f;
+            if (i & 1) S[c][i / 2].y = x; else S[c][i / 2].x = x;
+        }
+    const float* P = prep + (size_t)h * blocks * block_elems;
+    auto stage = [&](uint32_t b0, float* buf) {        // blocks [b0, min(b0 + tile, blocks)): one contiguous run
+        const uint32_t n4 = min(tile_blocks, blocks - b0) * block_elems / 4;
+        const float* src = P + (size_t)b0 * block_elems;
         for (uint32_t i = threadIdx.x; i < n4; i += kWalkThreads) cp_async16(buf + 4 * i, src + 4 * i);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     stage(0, sm);
-    float vt[kDeltaTile];
+    // lane (column, k or q, token), twice: its value of a block, its place in the outputs
+    const uint32_t lc = (lane >> 3) & 1, lj = lane & 3;
+    const bool live = col0 + lc < vdim;
+    const float* vbase = qkv + (size_t)lj * qkv_rs + v_off + (size_t)h * vdim + col0 + lc;
+    float vt[tile_blocks], vn[tile_blocks];
 #pragma unroll
-    for (int tt = 0; tt < kDeltaTile; tt++) vt[tt] = (live && (uint32_t)tt < T) ? vbase[(size_t)tt * qkv_rs] : 0.0f;
+    for (int i = 0; i < (int)tile_blocks; i++) vt[i] = live && i * B + lj < T ? vbase[(size_t)i * B * qkv_rs] : 0.0f;
+    // R / 2 pairs of a prepared vector
+    auto vec = [&](const float* v, float2 (&x)[R / 2]) {
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+            if (VR == 4) {
+                const float4 y = *reinterpret_cast<const float4*>(v + (g * 32 + lane) * 4);
+                x[2 * g] = make_float2(y.x, y.y); x[(2 * g + 1) % (R / 2)] = make_float2(y.z, y.w);
+            } else x[0] = *reinterpret_cast<const float2*>(v + lane * 2);
+        }
+    };
     uint32_t cur = 0;
     for (uint32_t t0 = 0; t0 < T; t0 += kDeltaTile, cur ^= 1) {
-        const uint32_t nt = min((uint32_t)kDeltaTile, T - t0);
         const bool more = t0 + kDeltaTile < T;
-        if (more) stage(t0 + kDeltaTile, sm + (cur ^ 1) * tile_elems);   // its last readers passed the barrier that ended the tile before
-        float vn[kDeltaTile];                                             // the next tile's values of this column, in flight during the walk
+        if (more) stage((t0 + kDeltaTile) / B, sm + (cur ^ 1) * tile_elems);   // its last readers passed the barrier that ended the tile before
 #pragma unroll
-        for (int tt = 0; tt < kDeltaTile; tt++)
-            vn[tt] = (live && more && t0 + kDeltaTile + tt < T) ? vbase[(size_t)(t0 + kDeltaTile + tt) * qkv_rs] : 0.0f;
+        for (int i = 0; i < (int)tile_blocks; i++) vn[i] = live && t0 + kDeltaTile + i * B + lj < T ? vbase[(size_t)(t0 + kDeltaTile + i * B) * qkv_rs] : 0.0f;
         if (more) asm volatile("cp.async.wait_group 1;" ::: "memory"); else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         const float* tile = sm + cur * tile_elems;
-        auto token = [&](int tti, float v) {
-            const float* row = tile + tti * stride;
-            const float4 tl = *reinterpret_cast<const float4*>(row + tail);   // beta, k . q, the head's decay: read with the vectors, before the shuffles
-            const float beta = tl.x, kq = tl.y, gh = tl.z;
-            float4 k4[kWalkRows / 4], g4[kWalkRows / 4];
-            float ks0 = 0.0f, ks1 = 0.0f, qs0 = 0.0f, qs1 = 0.0f;
 #pragma unroll
-            for (int c = 0; c < kWalkRows / 4; c++) {
-                const uint32_t at = (c * RS + r) * 4;
-                k4[c] = *reinterpret_cast<const float4*>(row + at);
-                const float4 q4 = *reinterpret_cast<const float4*>(row + dpad + at);
-                if (BONUS) {
-                    qs0 = fmaf(S[4 * c + 0], q4.x, qs0); qs1 = fmaf(S[4 * c + 1], q4.y, qs1);
-                    qs0 = fmaf(S[4 * c + 2], q4.z, qs0); qs1 = fmaf(S[4 * c + 3], q4.w, qs1);
-                }
-                if (!HEADG) {
-                    g4[c] = *reinterpret_cast<const float4*>(row + 2 * dpad + at);
-                    S[4 * c + 0] *= g4[c].x; S[4 * c + 1] *= g4[c].y; S[4 * c + 2] *= g4[c].z; S[4 * c + 3] *= g4[c].w;
-                }
-                if (!PLAIN) {
-                    ks0 = fmaf(S[4 * c + 0], k4[c].x, ks0); ks1 = fmaf(S[4 * c + 1], k4[c].y, ks1);
-                    ks0 = fmaf(S[4 * c + 2], k4[c].z, ks0); ks1 = fmaf(S[4 * c + 3], k4[c].w, ks1);
-                }
-                if (!BONUS) {
-                    qs0 = fmaf(S[4 * c + 0], q4.x, qs0); qs1 = fmaf(S[4 * c + 1], q4.y, qs1);
-                    qs0 = fmaf(S[4 * c + 2], q4.z, qs0); qs1 = fmaf(S[4 * c + 3], q4.w, qs1);
+        for (int bi = 0; bi < (int)tile_blocks; bi++) {
+            const uint32_t tb = t0 + bi * B;
+            if (bi && tb >= T) break;
+            const float* row = tile + bi * block_elems;
+            const float* sc = row + (W + B + 1) * dpad;
+            float sums[W * C];                                        // [column][product]
+#pragma unroll
+            for (int d = 0; d < W; d++) {
+                float2 x[R / 2], acc[C];
+                vec(row + d * dpad, x);
+#pragma unroll
+                for (int c = 0; c < C; c++) acc[c] = __fmul2_rn(S[c][0], x[0]);
+#pragma unroll
+                for (int i = 1; i < R / 2; i++)
+#pragma unroll
+                    for (int c = 0; c < C; c++) acc[c] = __ffma2_rn(S[c][i], x[i], acc[c]);
+#pragma unroll
+                for (int c = 0; c < C; c++) sums[c * W + d] = acc[c].x + acc[c].y;
+            }
+            float total = reduce_scatter<W * C>(sums, lane);
+            if (PLAIN) total = __shfl_sync(0xffffffffu, total, lc * B + lj);
+            float u[B], uc[C][B];
+#pragma unroll
+            for (int j = 0; j < B; j++) u[j] = __shfl_sync(0xffffffffu, PLAIN ? vt[bi] : vt[bi] - total, (lane & 8) + j);
+            if (!PLAIN) {
+                const float4 beta = *reinterpret_cast<const float4*>(sc);
+                const float4 c1 = *reinterpret_cast<const float4*>(sc + B + 4), c2 = *reinterpret_cast<const float4*>(sc + B + 8), c3 = *reinterpret_cast<const float4*>(sc + B + 12);
+                u[0] *= beta.x;
+                u[1] = fmaf(-c1.x, u[0], u[1]) * beta.y;
+                u[2] = fmaf(-c2.y, u[1], fmaf(-c2.x, u[0], u[2])) * beta.z;
+                u[3] = fmaf(-c3.z, u[2], fmaf(-c3.y, u[1], fmaf(-c3.x, u[0], u[3]))) * beta.w;
+            }
+#pragma unroll
+            for (int j = 0; j < B; j++) {
+                const float other = __shfl_xor_sync(0xffffffffu, u[j], 8);
+                uc[0][j] = lc ? other : u[j];
+                uc[1][j] = lc ? u[j] : other;
+            }
+            {
+                float2 x[R / 2];
+                vec(row + (W + B) * dpad, x);
+#pragma unroll
+                for (int i = 0; i < R / 2; i++)
+#pragma unroll
+                    for (int c = 0; c < C; c++) S[c][i] = __fmul2_rn(S[c][i], x[i]);
+#pragma unroll
+                for (int j = 0; j < B; j++) {
+                    vec(row + (W + j) * dpad, x);
+#pragma unroll
+                    for (int i = 0; i < R / 2; i++)
+#pragma unroll
+                        for (int c = 0; c < C; c++) S[c][i] = __ffma2_rn(x[i], make_float2(uc[c][j], uc[c][j]), S[c][i]);
                 }
             }
-            float ks = ks0 + ks1, qs = qs0 + qs1;
-#pragma unroll
-            for (uint32_t o = 1; o < RS; o <<= 1) { if (!PLAIN) ks += __shfl_xor_sync(0xffffffffu, ks, o); qs += __shfl_xor_sync(0xffffffffu, qs, o); }
-            if (HEADG) { ks *= gh; if (!BONUS) qs *= gh; }
-            const float u = PLAIN ? v : beta * (v - ks);
-#pragma unroll
-            for (int c = 0; c < kWalkRows / 4; c++) {
-                if (HEADG) { S[4 * c + 0] *= gh; S[4 * c + 1] *= gh; S[4 * c + 2] *= gh; S[4 * c + 3] *= gh; }
-                S[4 * c + 0] = fmaf(k4[c].x, u, S[4 * c + 0]); S[4 * c + 1] = fmaf(k4[c].y, u, S[4 * c + 1]);
-                S[4 * c + 2] = fmaf(k4[c].z, u, S[4 * c + 2]); S[4 * c + 3] = fmaf(k4[c].w, u, S[4 * c + 3]);
-            }
-            if (live && r == 0) dst[(size_t)(t0 + tti) * dst_rs + (size_t)h * vdim + col] = fmaf(u, kq, qs);
-        };
-        if (nt == (uint32_t)kDeltaTile) {                  // a full tile: straight-line code, nothing between the tokens
-#pragma unroll
-            for (int tti = 0; tti < kDeltaTile; tti++) token(tti, vt[tti]);
-        } else {
-#pragma unroll
-            for (int tti = 0; tti < kDeltaTile; tti++) {
-                if ((uint32_t)tti >= nt) break;
-                token(tti, vt[tti]);
-            }
+            const float4 cq = *reinterpret_cast<const float4*>(sc + B + 16 + 4 * lj);
+            total = fmaf(cq.w, u[3], fmaf(cq.z, u[2], fmaf(cq.y, u[1], fmaf(cq.x, u[0], total))));
+            if (live && (lane & 20) == 4 && tb + lj < T) dst[(size_t)(tb + lj) * dst_rs + (size_t)h * vdim + col0 + lc] = total;
         }
 #pragma unroll
-        for (int tt = 0; tt < kDeltaTile; tt++) vt[tt] = vn[tt];
+        for (int i = 0; i < (int)tile_blocks; i++) vt[i] = vn[i];
         __syncthreads();                                   // everyone is done with this buffer: the next iteration refills it
     }
 #pragma unroll
-    for (int i = 0; i < kWalkRows; i++) {
-        const uint32_t row = delta_row(RS, r, i);
-        if (live && row < dim) S_g[(size_t)row * vdim + col] = S[i];
-    }
+    for (int i = 0; i < R; i++)
+#pragma unroll
+        for (int c = 0; c < C; c++)
+            if (row_of(i) < dim && col0 + c < vdim) S_g[(size_t)row_of(i) * vdim + col0 + c] = i & 1 ? S[c][i / 2].y : S[c][i / 2].x;
 }
 // o / rms(o) * norm_w * sigmoid(gate) (or silu(gate)) * out_scale, one warp per (token, head), in place
 template <typename WT>
@@ -1690,7 +1789,7 @@ size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs) {
     }
     if (op.tag == ZG_OP_DELTA_RULE) {                  // the prepared per-token rows of the prefill form
         const ZgSeqOp& d = op.u.seq;
-        return d.n[0] >= (uint32_t)kDeltaPrepMinTokens && d.n[3] <= (uint32_t)kWalkMaxDim ? (size_t)d.n[0] * d.n[1] * ((d.n[10] & kDeltaHeadDecay ? 2 : 3) * delta_walk_slices(d.n[3]) * kWalkRows + 4) : 0;
+        return d.n[0] >= (uint32_t)kDeltaPrepMinTokens && d.n[3] <= (uint32_t)kWalkMaxDim ? (size_t)((d.n[0] + kWalkBlock - 1) / kWalkBlock) * d.n[1] * delta_block_elems(32 * delta_walk_rows(d.n[3]), d.n[10] & kDeltaPlain) : 0;
     }
     if (!dense_gemm_enabled() || op.tag != ZG_OP_LINEAR) return 0;
     const ZgSeqOp& s = op.u.seq;
@@ -1852,26 +1951,26 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             const size_t smem = ((size_t)3 * kDeltaTile * RS * kDeltaRows + kDeltaTile) * sizeof(float);
             const dim3 grid((vdim + cols - 1) / cols, H);
             if (scratch && T >= (uint32_t)kDeltaPrepMinTokens && dim <= (uint32_t)kWalkMaxDim) {
-                const uint32_t WS = delta_walk_slices(dim), dpad = WS * kWalkRows, wcols = kWalkThreads / WS;
-                const size_t walk_smem = (size_t)2 * kDeltaTile * ((form & kDeltaHeadDecay ? 2 : 3) * dpad + 4) * sizeof(float);
-                ZG_SEQ_WDT(s.n[9], launch_pdl(k_delta_prepare<WT>, dim3((T * H + 3) / 4), dim3(128), 0, st, scratch, bufs[s.buf[1]], betab, bufs[s.buf[3]] + s.n[13],
-                                              wptr<WT>(bufs, s.buf[5], 0), T, H, G, dim, dpad, s.off[0], s.off[1], s.off[3], s.off[4], s.off[5], s.n[5], s.n[6], s.n[7], s.f[1], s.f[2],
-                                              form, inv_tau, s.n[14]));
-                ZG_SEQ_CHECK();
-#define ZG_WALK_FORM(RS_, PLAIN_, HEADG_, BONUS_)                                                                                               \
+                const bool plain = form & kDeltaPlain;
+                const uint32_t R = delta_walk_rows(dim), warps = (T + kWalkBlock - 1) / kWalkBlock * H, wcols = kWalkThreads / 32 * kWalkCols, n_prep = (warps + 3) / 4;
+                const size_t walk_smem = ((size_t)2 * (kDeltaTile / kWalkBlock) * delta_block_elems(32 * R, plain)) * sizeof(float);
+                // Long steps: a plain launch.  CTAs placed while the predecessor still fills the GPU shared SMs two by two (128 CTAs: 430 us instead of 250).
+                const bool early = n_prep + (vdim + wcols - 1) / wcols * H <= 100;
+#define ZG_WALK_FORM(R_, PLAIN_)                                                                                                                \
     do {                                                                                                                                        \
-        if (walk_smem > 48 * 1024) cudaFuncSetAttribute(k_delta_walk<RS_, PLAIN_, HEADG_, BONUS_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem); \
-        launch_pdl(k_delta_walk<RS_, PLAIN_, HEADG_, BONUS_>, dim3((vdim + wcols - 1) / wcols, H), dim3(kWalkThreads), walk_smem, st, dst, bufs[s.buf[1]], \
-                   scratch, bufs[s.buf[6]], bufs[s.buf[7]], T, H, dim, vdim, s.off[2], s.n[5], dst_rs);                                         \
+        if (walk_smem > 48 * 1024) cudaFuncSetAttribute(k_delta_walk<R_, PLAIN_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem); \
+        launch_pdl_if(early, k_delta_walk<R_, PLAIN_>, dim3((vdim + wcols - 1) / wcols, H), dim3(kWalkThreads), walk_smem, st, dst, bufs[s.buf[1]], \
+                      scratch, bufs[s.buf[6]], bufs[s.buf[7]], T, H, dim, vdim, s.off[2], s.n[5], dst_rs);                                      \
     } while (0)
-#define ZG_WALK(RS_)                                                                                                                            \
-    case RS_:                                                                                                                                   \
-        if (form & kDeltaBonus) { if (form & kDeltaHeadDecay) ZG_WALK_FORM(RS_, true, true, true); else ZG_WALK_FORM(RS_, true, false, true); } \
-        else if (form & kDeltaPlain) { if (form & kDeltaHeadDecay) ZG_WALK_FORM(RS_, true, true, false); else ZG_WALK_FORM(RS_, true, false, false); } \
-        else if (form & kDeltaHeadDecay) ZG_WALK_FORM(RS_, false, true, false);                                                                 \
-        else ZG_WALK_FORM(RS_, false, false, false);                                                                                            \
-        break;
-                switch (WS) { ZG_WALK(1) ZG_WALK(2) ZG_WALK(4) ZG_WALK(8) ZG_WALK(16) default: ZG_WALK(32) }
+#define ZG_WALK(R_)                                                                                                                             \
+    do {                                                                                                                                        \
+        ZG_SEQ_WDT(s.n[9], launch_pdl(k_delta_prepare<WT, R_>, dim3(n_prep), dim3(128), 0, st, scratch, bufs[s.buf[1]], betab, bufs[s.buf[3]] + s.n[13], \
+                                      wptr<WT>(bufs, s.buf[5], 0), T, H, G, dim, s.off[0], s.off[1], s.off[3], s.off[4], s.off[5], s.n[5], s.n[6], s.n[7], s.f[1], s.f[2], \
+                                      form, inv_tau, s.n[14]));                                                                                 \
+        ZG_SEQ_CHECK();                                                                                                                         \
+        if (plain) ZG_WALK_FORM(R_, true); else ZG_WALK_FORM(R_, false);                                                                        \
+    } while (0)
+                if (R == 2) ZG_WALK(2); else if (R == 4) ZG_WALK(4); else if (R == 8) ZG_WALK(8); else ZG_WALK(16);
 #undef ZG_WALK
 #undef ZG_WALK_FORM
             } else ZG_SEQ_WDT(s.n[9], {
