@@ -1,8 +1,8 @@
 // Dense prefill matmul for the sequence-model LINEAR op on the 5th-generation tensor cores:
 //   dst[M, N] = bf16(src)[M, K] * W[N, K]^T (+ bias), W stored bfloat16 row-major (the checkpoint's [out, in]).
 //
-//   * tcgen05.mma.cta_group::1.kind::f16 on BF16 operands, one 128 x 128 fp32 accumulator per CTA in TMEM, issued by one
-//     thread; K advances 64 (one 128-byte swizzle row) per pipeline stage.
+//   * tcgen05.mma.cta_group::1.kind::f16 on BF16 operands, one 128 x 128 fp32 accumulator per CTA in TMEM, issued by the
+//     elected lane of a warp; K advances 64 (one 128-byte swizzle row) per pipeline stage.
 //   * BOTH operands arrive by TMA (cp.async.bulk.tensor.2d, 128B swizzle) straight into the canonical K-major layout: the
 //     weight matrix as it lies in the arena (out-of-range rows / k are zero-filled by the copy engine), the activations
 //     from a bf16 scratch that a small conversion kernel fills (one rounding per activation; accumulation stays fp32).
@@ -14,7 +14,7 @@
 //
 // Used when the session keeps bfloat16 weights and M > 8 (decode rows stream the weights through the row kernels of
 // seqops.cu); float32 sessions keep the exact SIMT tile.
-#include "zg_internal.cuh"
+#include "seq_common.cuh"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -70,6 +70,32 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
     return d;
 }
 
+// One lane of a converged warp.  The issuing warp walks its loop whole and lets the elected lane issue: addresses stay warp-uniform that way (inside a
+// single lane's branch an MMA of 128 x 128 x 16 took 130 clocks to issue; it executes in 64).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// D[tmem] (+)= A[shared] B[shared], bf16
+__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(addr));
+}
+// every loaded register passes through the wait, so that nothing that reads them moves above it
+__device__ __forceinline__ void tmem_wait_ld16(uint32_t (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
+}
 // f32 rows -> dense bf16 [Mp][Kp] (zero padding), two k per thread
 // (ctl: the rows are those of a per-sequence state buffer, `slot_stride` elements per slot; the slot is the control word's)
 // (rows_from > 0: rows from position + rows_from on are not wanted, up to the end of their 128-row tile)
@@ -118,31 +144,22 @@ struct GemmParams {
     uint32_t act;            // applied after the bias: 0 none, 1 relu^2, 2 silu, 3 gelu (tanh form), 4 relu, 5 smooth cap act_p * tanh(z / act_p), 6 gelu (erf form)
     float act_p;
     uint32_t act_lo, act_hi; // the columns it applies to
-    const int* tile_group;   // kGrouped: weight matrix (third TMA coordinate) of every 128-row tile, -1: tile unused
     const int* ctl;          // kPlain with rows_from: tiles from row position + rows_from on are skipped
     uint32_t rows_from;
     uint32_t heads, n_last, a_rows, out_hs;   // kBatched: heads, rows of the last head's matrix, padded source rows per head, columns between the heads' outputs
 };
 
-// kGrouped: the rows are sorted by weight matrix (expert) in whole 128-row tiles; tile t multiplies with matrix tile_group[t]
-// of the stacked [groups][N][K] weight tensor.
 // kBatched: blockIdx.z names a head with source rows, weight rows and output columns of its own (all in one tensor each).  A tile at the
 // end of a head reads on into the next head's weight rows; those columns are not written.
 // PAIRS: weight rows 2n and 2n + 1 are a gate and what it multiplies: out[., n] = act(gate) * up.
-enum { kPlain = 0, kGrouped = 1, kBatched = 2 };
+enum { kPlain = 0, kBatched = 1 };
 template <int MODE, int ACT, bool PAIRS>        // ACT: the activation of the epilogue (GemmParams::act; one instantiation each)
 __global__ void __launch_bounds__(kThreads, 1)
 dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
-    constexpr bool GROUPED = MODE == kGrouped;
-    int group = 0;
     const uint32_t head = MODE == kBatched ? blockIdx.z : 0, N = MODE == kBatched && head + 1 == p.heads ? p.n_last : p.N;
     if (MODE == kBatched && blockIdx.x * BN >= N) return;
     if (MODE == kPlain && p.rows_from && blockIdx.y * BM >= (uint32_t)p.ctl[ZG_CTL_POS] + p.rows_from) return;
     float* const outp = p.out + (MODE == kBatched ? (size_t)head * p.out_hs : 0);
-    if (GROUPED) {
-        group = p.tile_group[blockIdx.y];
-        if (group < 0) return;   // uniform over the CTA, before any barrier or TMEM allocation
-    }
     extern __shared__ uint8_t dsm_raw[];
     const uint32_t base = (smem_u32(dsm_raw) + 1023u) & ~1023u;
     const uint32_t bars = base + kStages * kStage;
@@ -173,32 +190,22 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 if (!mbar_wait(empty + 8 * s, ph ^ 1)) break;
                 mbar_expect_tx(full + 8 * s, kStage);
                 tma_load_2d(base + s * kStage, &tmap_a, kt * BK, head * p.a_rows + tile_m * BM, full + 8 * s);
-                if (GROUPED) tma_load_3d(base + s * kStage + kTileA, &tmap_b, kt * BK, tile_n * BN, (uint32_t)group, full + 8 * s);
-                else tma_load_2d(base + s * kStage + kTileA, &tmap_b, kt * BK, head * p.N + tile_n * BN, full + 8 * s);
+                tma_load_2d(base + s * kStage + kTileA, &tmap_b, kt * BK, head * p.N + tile_n * BN, full + 8 * s);
             }
         }
     } else if (warp == 1) {
         // instruction descriptor (kind::f16): D = F32, A = B = BF16, both K-major, N = BN, M = 128
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((BN >> 3) << 17) | ((128u >> 4) << 24);
-        if (lane == 0) {
-            for (uint32_t kt = 0; kt < n_k; kt++) {
-                const uint32_t s = kt % kStages, ph = (kt / kStages) & 1;
-                if (!mbar_wait(full + 8 * s, ph)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const bool leader = elect_one();
+        for (uint32_t kt = 0; kt < n_k; kt++) {
+            const uint32_t s = kt % kStages, ph = (kt / kStages) & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, ph))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                for (uint32_t k = 0; k < BK / 16; k++) {
-                    const uint64_t da = make_desc(base + s * kStage + k * 32), db = make_desc(base + s * kStage + kTileA + k * 32);
-                    const uint32_t accumulate = (kt | k) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                        ::"r"(tmem_base), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-                }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty + 8 * s) : "memory");
-                if (kt + 1 == n_k)
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tmem_full) : "memory");
-            }
+            for (uint32_t k = 0; k < BK / 16; k++)
+                if (leader) mma_bf16(tmem_base, make_desc(base + s * kStage + k * 32), make_desc(base + s * kStage + kTileA + k * 32), idesc, (kt | k) ? 1u : 0u);
+            if (leader) mma_commit(empty + 8 * s);
+            if (leader && kt + 1 == n_k) mma_commit(tmem_full);
         }
         __syncwarp();
     } else {
@@ -286,6 +293,115 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(kTmemCols) : "memory");
 }
 
+// Expert products of MOE_FFN: out[row, n] = sum_k x[row, k] W_e[n, k] for rows sorted by expert, one run of at most 256 rows of one expert per blockIdx.y.
+//
+// The weights are the 128-row operand and the run's rows the N operand, of as many columns as the run has rows (rounded up to 16): every weight is read
+// once per run, and what is computed for padding is less than 16 rows (whole 128-row tiles of tokens were a third padding at 16 experts of 128 rows each,
+// and read the weights again for it).  DUAL: two weight matrices against the same rows, gate and up, and out = bf16(act(gate) up), so that neither
+// product goes through memory.
+// Bound by the stream of weights.  1024 tokens, two of 16 experts, 2048 x 2048, cold: gate, up and activation 68 us (98 as two products and a pass of
+// their own over whole tiles), down 40 us (42); the op 129 us (171), 44 tokens on one of 4 experts of 1696 x 1088 31 us (60).
+constexpr uint32_t kExpertThreads = 320;          // warp 0: TMA, warp 1: MMA + TMEM, warps 2-9: epilogue
+constexpr uint32_t kExpertRows = 32;              // rows of x per copy
+constexpr uint32_t kExpertRing = 216 * 1024, kExpertSmem = kExpertRing + 1024 + 256, kExpertStages = 8;
+struct ExpertParams {
+    void* out; const ZgExpertSegment* segments;
+    uint32_t N, K;
+    float limit, alpha, up_offset;
+};
+template <bool DUAL>
+__global__ void __launch_bounds__(kExpertThreads, 1)
+k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2, const ExpertParams p) {
+    pdl_enter();
+    const ZgExpertSegment seg = p.segments[blockIdx.y];
+    if (seg.rows <= 0) return;                     // uniform over the CTA, before any barrier or TMEM allocation
+    extern __shared__ uint8_t dsm_raw[];
+    const uint32_t base = (smem_u32(dsm_raw) + 1023u) & ~1023u, bars = base + kExpertRing;
+    const uint32_t full = bars, empty = bars + 8 * kExpertStages, tmem_full = bars + 16 * kExpertStages, tmem_slot = tmem_full + 8;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t n = (uint32_t)seg.rows, copies = (n + kExpertRows - 1) / kExpertRows, n_k = (p.K + BK - 1) / BK;
+    constexpr uint32_t kWeights = (DUAL ? 2 : 1) * kTileA, kAccCols = 256;
+    const uint32_t stage_bytes = kWeights + copies * (kExpertRows * BK * 2), stages = min(kExpertStages, kExpertRing / stage_bytes);
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < stages; s++) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 1); }
+        mbar_init(tmem_full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "n"(DUAL ? 2 * kAccCols : kAccCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    uint32_t tmem;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+    const uint32_t f0 = blockIdx.x * BM;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t s = 0, ph = 1;
+            for (uint32_t kt = 0; kt < n_k; kt++) {
+                if (!mbar_wait(empty + 8 * s, ph)) break;
+                const uint32_t at = base + s * stage_bytes;
+                mbar_expect_tx(full + 8 * s, stage_bytes);
+                tma_load_3d(at, &tmap_w, kt * BK, f0, (uint32_t)seg.expert, full + 8 * s);
+                if (DUAL) tma_load_3d(at + kTileA, &tmap_w2, kt * BK, f0, (uint32_t)seg.expert, full + 8 * s);
+                for (uint32_t c = 0; c < copies; c++) tma_load_2d(at + kWeights + c * (kExpertRows * BK * 2), &tmap_x, kt * BK, (uint32_t)seg.start + c * kExpertRows, full + 8 * s);
+                if (++s == stages) { s = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // instruction descriptor (kind::f16): D = F32, A = B = BF16, both K-major, N = the run's rows, M = 128
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((n + 15) / 16 * 2) << 17) | ((128u >> 4) << 24);
+        const bool leader = elect_one();
+        uint32_t s = 0, ph = 0;
+        for (uint32_t kt = 0; kt < n_k; kt++) {
+            if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, ph))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t at = base + s * stage_bytes;
+#pragma unroll
+            for (uint32_t k = 0; k < BK / 16; k++)
+                if (leader) {
+                    const uint64_t x = make_desc(at + kWeights + k * 32);
+                    mma_bf16(tmem, make_desc(at + k * 32), x, idesc, (kt | k) ? 1u : 0u);
+                    if (DUAL) mma_bf16(tmem + kAccCols, make_desc(at + kTileA + k * 32), x, idesc, (kt | k) ? 1u : 0u);
+                }
+            if (leader) mma_commit(empty + 8 * s);
+            if (leader && kt + 1 == n_k) mma_commit(tmem_full);
+            if (++s == stages) { s = 0; ph ^= 1; }
+        }
+        __syncwarp();
+    } else {
+        // TMEM lane = output column of the CTA's 128, TMEM column = row of the run; the two warps of a quarter take 16 rows each in turn
+        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2, f = f0 + quarter * 32 + lane;
+        const bool ok = mbar_wait(tmem_full, 0);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (uint32_t c0 = 16 * half; __all_sync(0xffffffffu, ok) && c0 < n; c0 += 32) {
+            uint32_t g[16], u[16];
+            const uint32_t addr = tmem + ((quarter * 32) << 16) + c0;
+            tmem_ld16(addr, g);
+            if (DUAL) tmem_ld16(addr + kAccCols, u);
+            tmem_wait_ld16(g);
+            if (DUAL) tmem_wait_ld16(u);
+#pragma unroll
+            for (uint32_t j = 0; j < 16; j++) {
+                if (c0 + j >= n || f >= p.N) continue;
+                const size_t at = ((size_t)seg.start + c0 + j) * p.N + f;
+                if (DUAL) {
+                    const float gv = fminf(__uint_as_float(g[j]), p.limit), uv = fminf(fmaxf(__uint_as_float(u[j]), -p.limit), p.limit);
+                    reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(gv * sigmoidf_(p.alpha * gv) * (uv + p.up_offset));
+                } else reinterpret_cast<float*>(p.out)[at] = __uint_as_float(g[j]);
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(DUAL ? 2 * kAccCols : kAccCols) : "memory");
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -313,7 +429,8 @@ bool prepare() {
         g_encode = (EncodeTiledFn)fn;
     }
     if (!g_attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(dense_gemm_kernel<kGrouped, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+        cudaError_t e = cudaFuncSetAttribute(k_expert_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExpertSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_expert_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExpertSmem);
         for (int k = 0; k < 2 * kActs && e == cudaSuccess; k++) e = cudaFuncSetAttribute(g_kernel[k / kActs][k % kActs], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
         for (uint32_t k = 0; k < 6 && e == cudaSuccess; k += 5) e = cudaFuncSetAttribute(batched_kernel(k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
         if (e != cudaSuccess) { zg_set_error("cudaFuncSetAttribute(dense_gemm) failed: %s", cudaGetErrorString(e)); return false; }
@@ -369,7 +486,6 @@ bool zg_dense_gemm_launch(const void* w_bf16, const void* bias_bf16, const float
     p.ctl = reinterpret_cast<const int*>(ctl); p.rows_from = rows_from;
     p.out = dst; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias_bf16); p.M = M; p.N = N; p.K = K; p.out_rs = dst_rs; p.act = act; p.act_p = act_p; p.act_lo = act_lo; p.act_hi = act_hi;
     p.out_vec4 = ((reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (dst_rs & 3) == 0) ? 1u : 0u;
-    p.tile_group = nullptr;
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (act >= (uint32_t)kActs) { zg_set_error("dense gemm: unknown activation %u", act); return false; }
     g_kernel[pairs ? 1 : 0][act]<<<grid, kThreads, kSmem, st>>>(map_a, map_b, p);
@@ -379,37 +495,33 @@ bool zg_dense_gemm_launch(const void* w_bf16, const void* bias_bf16, const float
     return true;
 }
 
-// Grouped form: xb = bf16 rows [rows][Kp] already sorted by group in whole 128-row tiles (rows % 128 == 0, Kp % 64 == 0, zero
-// padding), W = [groups][N][K] bfloat16, dst[rows][N] f32.  d_tile_group[rows / 128] selects the matrix of every tile (< 0: skip).
-bool zg_dense_gemm_grouped_launch(const void* w_bf16, uint32_t groups, const void* xb, uint32_t rows, uint32_t Kp, const int* d_tile_group, float* dst,
-                                  uint32_t N, uint32_t K, uint32_t dst_rs, cudaStream_t st) {
+static bool expert_weights_map(CUtensorMap* map, const void* w, uint32_t E, uint32_t N, uint32_t K) {
+    const cuuint64_t gdim[3] = {K, N, E}, gstride[2] = {(cuuint64_t)K * 2, (cuuint64_t)N * K * 2};
+    const cuuint32_t box[3] = {BK, BM, 1}, estr[3] = {1, 1, 1};
+    const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) zg_set_error("cuTensorMapEncodeTiled(expert weights) failed (%d)", (int)r);
+    return r == CUDA_SUCCESS;
+}
+// xb: bf16 rows [rows][K] sorted by expert; w, w2: [E][N][K] bfloat16 (w2 null: out = f32 [rows][N]; otherwise out = bf16 [rows][N] of gate and up).
+// d_segments: `segments` runs of rows on the device (ZgExpertSegment).
+bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void* xb, uint32_t rows, const ZgExpertSegment* d_segments, uint32_t segments, void* out, uint32_t N, uint32_t K,
+                           float limit, float alpha, float up_offset, cudaStream_t st) {
     if (!prepare()) return false;
-    CUtensorMap map_a, map_b;
-    {
-        const cuuint64_t gdim[2] = {Kp, rows};
-        const cuuint64_t gstride[1] = {(cuuint64_t)Kp * 2};
-        const cuuint32_t box[2] = {BK, BM}, estr[2] = {1, 1};
-        CUresult r = g_encode(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(xb), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) { zg_set_error("cuTensorMapEncodeTiled(grouped rows) failed (%d)", (int)r); return false; }
-    }
-    {
-        const cuuint64_t gdim[3] = {K, N, groups};
-        const cuuint64_t gstride[2] = {(cuuint64_t)K * 2, (cuuint64_t)N * K * 2};
-        const cuuint32_t box[3] = {BK, BN, 1}, estr[3] = {1, 1, 1};
-        CUresult r = g_encode(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w_bf16), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) { zg_set_error("cuTensorMapEncodeTiled(stacked weights) failed (%d)", (int)r); return false; }
-    }
-    GemmParams p = {};
-    p.out = dst; p.bias = nullptr; p.M = rows; p.N = N; p.K = K; p.out_rs = dst_rs; p.act = 0; p.act_p = 0.0f; p.act_lo = p.act_hi = 0;
-    p.out_vec4 = ((reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (dst_rs & 3) == 0) ? 1u : 0u;
-    p.tile_group = d_tile_group;
-    dim3 grid((N + BN - 1) / BN, rows / BM);
-    dense_gemm_kernel<kGrouped, 0, false><<<grid, kThreads, kSmem, st>>>(map_a, map_b, p);
+    CUtensorMap map_x, map_w, map_w2;
+    const cuuint64_t gdim[2] = {K, rows}, gstride[1] = {(cuuint64_t)K * 2};
+    const cuuint32_t box[2] = {BK, kExpertRows}, estr[2] = {1, 1};
+    const CUresult r = g_encode(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(xb), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { zg_set_error("cuTensorMapEncodeTiled(expert rows) failed (%d)", (int)r); return false; }
+    if (!expert_weights_map(&map_w, w, E, N, K) || !expert_weights_map(&map_w2, w2 ? w2 : w, E, N, K)) return false;
+    const ExpertParams p = {out, d_segments, N, K, limit, alpha, up_offset};
+    const dim3 grid((N + BM - 1) / BM, segments);
+    if (w2) launch_pdl(k_expert_gemm<true>, grid, dim3(kExpertThreads), kExpertSmem, st, map_x, map_w, map_w2, p);
+    else launch_pdl(k_expert_gemm<false>, grid, dim3(kExpertThreads), kExpertSmem, st, map_x, map_w, map_w2, p);
     ZG_COUNT_LAUNCH();
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) { zg_set_error("grouped dense gemm launch failed: %s", cudaGetErrorString(e)); return false; }
+    if (e != cudaSuccess) { zg_set_error("expert gemm launch failed: %s", cudaGetErrorString(e)); return false; }
     return true;
 }
 

@@ -1507,36 +1507,35 @@ __global__ void k_moe_down(float* __restrict__ dst, const float* __restrict__ sr
     if (lane == 0) dst[(size_t)t * D + d] = acc;
 }
 
-// ── MOE_FFN, grouped form (prefill on bfloat16 sessions): the step's (token, choice) pairs are sorted by expert into whole
-// 128-row tiles, the rows are gathered as bf16, and every expert's gate / up / down products run as tiles of ONE grouped
-// tensor-core matmul each (dense_gemm.cu), so an expert's weights are read once per 128 rows instead of once per token ──
+// ── MOE_FFN, grouped form (prefill on bfloat16 sessions): the step's (token, choice) pairs are sorted by expert, the rows are gathered as bf16, and the
+// experts' products run as tiles of ONE tensor-core matmul for gate, up and activation and one for down (dense_gemm.cu), so an expert's weights are read
+// once per 256 rows instead of once per token ──
 struct MoeLayout {          // offsets in f32 slots inside the op's scratch operand
-    uint32_t R, Dp, Fp;     // rows incl. per-expert padding, padded widths of the bf16 copies
-    size_t tile_group, row_pair, pos_of_pair, xs, g, u, yb, z, total;
+    uint32_t R, segments;   // (token, choice) pairs; runs of rows of one expert, at most
+    size_t seg, row_pair, pos_of_pair, xs, yb, z, total;
 };
 __host__ __device__ inline size_t up4(size_t n) { return (n + 3) & ~(size_t)3; }
 MoeLayout moe_layout(uint32_t T, uint32_t D, uint32_t ff, uint32_t E, uint32_t top) {
     MoeLayout L;
-    L.R = (T * top + 127) / 128 * 128 + E * 128;
-    L.Dp = (D + 63) / 64 * 64; L.Fp = (ff + 63) / 64 * 64;
+    L.R = T * top;
+    L.segments = (E < L.R ? E : L.R) + L.R / kExpertSegmentRows;
     size_t o = 0;
-    L.tile_group = o; o = up4(o + L.R / 128);
+    L.seg = o; o = up4(o + (size_t)L.segments * (sizeof(ZgExpertSegment) / 4));
     L.row_pair = o; o = up4(o + L.R);
-    L.pos_of_pair = o; o = up4(o + (size_t)T * top);
-    L.xs = o; o = up4(o + (size_t)L.R * L.Dp / 2);
-    L.g = o; o = up4(o + (size_t)L.R * ff);
-    L.u = o; o = up4(o + (size_t)L.R * ff);
-    L.yb = o; o = up4(o + (size_t)L.R * L.Fp / 2);
+    L.pos_of_pair = o; o = up4(o + L.R);
+    L.xs = o; o = up4(o + (size_t)L.R * D / 2);
+    L.yb = o; o = up4(o + (size_t)L.R * ff / 2);
     L.z = o; o = up4(o + (size_t)L.R * D);
     L.total = o;
     return L;
 }
 constexpr uint32_t kMoeMaxExperts = 1024;
-__global__ void __launch_bounds__(1024) k_moe_sort(const float* __restrict__ route, int* __restrict__ tile_group, int* __restrict__ row_pair,
-                                                   int* __restrict__ pos_of_pair, uint32_t pairs, uint32_t E, uint32_t R) {
-    __shared__ int cnt[kMoeMaxExperts], off[kMoeMaxExperts + 1];
+__global__ void __launch_bounds__(1024) k_moe_sort(const float* __restrict__ route, ZgExpertSegment* __restrict__ seg, int* __restrict__ row_pair,
+                                                   int* __restrict__ pos_of_pair, uint32_t pairs, uint32_t E, uint32_t segments) {
+    pdl_enter();
+    __shared__ int cnt[kMoeMaxExperts], off[kMoeMaxExperts];
     for (uint32_t e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
-    for (uint32_t r = threadIdx.x; r < R; r += blockDim.x) row_pair[r] = -1;
+    for (uint32_t r = threadIdx.x; r < pairs; r += blockDim.x) row_pair[r] = -1;
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) {
         const uint32_t e = (uint32_t)reinterpret_cast<const int*>(route)[2 * (size_t)i];
@@ -1545,14 +1544,16 @@ __global__ void __launch_bounds__(1024) k_moe_sort(const float* __restrict__ rou
     __syncthreads();
     if (threadIdx.x == 0) {
         int o = 0;
+        uint32_t n = 0;
         for (uint32_t e = 0; e < E; e++) {
             off[e] = o;
-            const int tiles = (cnt[e] + 127) / 128;
-            for (int t = 0; t < tiles; t++) tile_group[o / 128 + t] = (int)e;
-            o += tiles * 128;
+            const int c = cnt[e], runs = (c + (int)kExpertSegmentRows - 1) / (int)kExpertSegmentRows;
+            const int rows = runs ? ((c + runs - 1) / runs + 15) / 16 * 16 : 0;      // equal shares, of whole multiples of 16
+            for (int r = 0; r < c; r += rows) seg[n++] = ZgExpertSegment{(int)e, o + r, min(rows, c - r)};
+            o += c;
             cnt[e] = 0;                                  // becomes the expert's fill cursor
         }
-        for (uint32_t t = (uint32_t)o / 128; t < R / 128; t++) tile_group[t] = -1;
+        for (; n < segments; n++) seg[n] = ZgExpertSegment{0, 0, 0};
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) {
@@ -1562,39 +1563,21 @@ __global__ void __launch_bounds__(1024) k_moe_sort(const float* __restrict__ rou
         pos_of_pair[i] = pos;                            // which row a pair landed in does not change its result
     }
 }
-__global__ void k_moe_gather(uint32_t* __restrict__ xs, const float* __restrict__ src, const int* __restrict__ row_pair, uint32_t D, uint32_t dp2,
-                             uint32_t top) {
+__global__ void k_moe_gather(uint32_t* __restrict__ xs, const float* __restrict__ src, const int* __restrict__ row_pair, uint32_t D, uint32_t top) {
+    pdl_enter();
     const uint32_t r = blockIdx.x;
     const int pair = row_pair[r];
-    const float* x = pair >= 0 ? src + (size_t)((uint32_t)pair / top) * D : nullptr;
-    for (uint32_t k2 = threadIdx.x; k2 < dp2; k2 += blockDim.x) {
-        const uint32_t k = 2 * k2;
-        const float a = (x && k < D) ? x[k] : 0.0f, b = (x && k + 1 < D) ? x[k + 1] : 0.0f;
+    if (pair < 0) return;                                // rows that no expert takes
+    const float* x = src + (size_t)((uint32_t)pair / top) * D;
+    for (uint32_t k = 2 * threadIdx.x; k < D; k += 2 * blockDim.x) {
         uint32_t v;
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(b), "f"(a));
-        xs[(size_t)r * dp2 + k2] = v;
-    }
-}
-__global__ void k_moe_act(uint32_t* __restrict__ yb, const float* __restrict__ g, const float* __restrict__ u, const int* __restrict__ row_pair,
-                          uint32_t ff, uint32_t fp2, float limit, float alpha, float uoff) {
-    const uint32_t r = blockIdx.x;
-    const bool live = row_pair[r] >= 0;
-    for (uint32_t f2 = threadIdx.x; f2 < fp2; f2 += blockDim.x) {
-        float y[2] = {0.0f, 0.0f};
-        for (int i = 0; i < 2; i++) {
-            const uint32_t f = 2 * f2 + i;
-            if (live && f < ff) {
-                const float gv = fminf(g[(size_t)r * ff + f], limit), uv = fminf(fmaxf(u[(size_t)r * ff + f], -limit), limit);
-                y[i] = gv * sigmoidf_(alpha * gv) * (uv + uoff);
-            }
-        }
-        uint32_t v;
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(y[1]), "f"(y[0]));
-        yb[(size_t)r * fp2 + f2] = v;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(x[k + 1]), "f"(x[k]));
+        xs[((size_t)r * D + k) / 2] = v;
     }
 }
 __global__ void k_moe_combine(float* __restrict__ dst, const float* __restrict__ src, const float* __restrict__ z, const float* __restrict__ route,
                               const int* __restrict__ pos_of_pair, uint32_t D, uint32_t top) {
+    pdl_enter();
     const uint32_t t = blockIdx.x;
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         float acc = 0.0f;
@@ -1998,19 +1981,16 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             if (moe_grouped(s, bufs)) {
                 const MoeLayout L = moe_layout(T, D, ff, E, top);
                 float* sc = bufs[s.buf[4]];
-                int* tile_group = reinterpret_cast<int*>(sc + L.tile_group);
+                ZgExpertSegment* seg = reinterpret_cast<ZgExpertSegment*>(sc + L.seg);
                 int* row_pair = reinterpret_cast<int*>(sc + L.row_pair);
                 int* pos_of_pair = reinterpret_cast<int*>(sc + L.pos_of_pair);
-                k_moe_sort<<<1, 1024, 0, st>>>(bufs[s.buf[2]], tile_group, row_pair, pos_of_pair, T * top, E, L.R);
+                launch_pdl(k_moe_sort, dim3(1), dim3(1024), 0, st, bufs[s.buf[2]], seg, row_pair, pos_of_pair, L.R, E, L.segments);
                 ZG_SEQ_CHECK();
-                k_moe_gather<<<L.R, 256, 0, st>>>(reinterpret_cast<uint32_t*>(sc + L.xs), bufs[s.buf[1]], row_pair, D, L.Dp / 2, top);
+                launch_pdl(k_moe_gather, dim3(L.R), dim3(256), 0, st, reinterpret_cast<uint32_t*>(sc + L.xs), bufs[s.buf[1]], row_pair, D, top);
                 ZG_SEQ_CHECK();
-                if (!zg_dense_gemm_grouped_launch(wptr<bf16>(bufs, s.buf[3], s.off[0]), E, sc + L.xs, L.R, L.Dp, tile_group, sc + L.g, ff, D, ff, st) ||
-                    !zg_dense_gemm_grouped_launch(wptr<bf16>(bufs, s.buf[3], s.off[1]), E, sc + L.xs, L.R, L.Dp, tile_group, sc + L.u, ff, D, ff, st)) return false;
-                k_moe_act<<<L.R, 256, 0, st>>>(reinterpret_cast<uint32_t*>(sc + L.yb), sc + L.g, sc + L.u, row_pair, ff, L.Fp / 2, s.f[0], s.f[1], s.f[2]);
-                ZG_SEQ_CHECK();
-                if (!zg_dense_gemm_grouped_launch(wptr<bf16>(bufs, s.buf[3], s.off[2]), E, sc + L.yb, L.R, L.Fp, tile_group, sc + L.z, D, ff, D, st)) return false;
-                k_moe_combine<<<T, 256, 0, st>>>(bufs[s.buf[0]], bufs[s.buf[1]], sc + L.z, bufs[s.buf[2]], pos_of_pair, D, top);
+                if (!zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[0]), wptr<bf16>(bufs, s.buf[3], s.off[1]), E, sc + L.xs, L.R, seg, L.segments, sc + L.yb, ff, D, s.f[0], s.f[1], s.f[2], st) ||
+                    !zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[2]), nullptr, E, sc + L.yb, L.R, seg, L.segments, sc + L.z, D, ff, 0.0f, 0.0f, 0.0f, st)) return false;
+                launch_pdl(k_moe_combine, dim3(T), dim3(256), 0, st, bufs[s.buf[0]], bufs[s.buf[1]], sc + L.z, bufs[s.buf[2]], pos_of_pair, D, top);
                 ZG_SEQ_CHECK();
                 return true;
             }
