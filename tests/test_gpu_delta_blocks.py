@@ -45,3 +45,23 @@ def test_delta_rule_in_blocks_of_four(cuda_backend, plain, T, dim, vdim, decay):
         assert np.abs(S_got - S_want).max() < 2e-5 * max(1.0, np.abs(S_want).max()), rep
     w.free()
     state.free()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_value_that_is_no_number_spares_the_tokens_before_it(cuda_backend, bad):
+    """The value of token 18 (the third of its block) is not finite: the tokens before it come out as without it."""
+    from zgml_b200 import DeviceBuffer, DeviceOp, ExternBuffer, abi
+    r = np.random.default_rng(5)
+    T, H, dim, vdim = 20, 1, 32, 16
+    w, (oA, odt, onw) = weights(cuda_backend, r.standard_normal(H), r.standard_normal((H, dim)), 1 + 0.2 * r.standard_normal(vdim))
+    qrs = 2 * dim + 2 * vdim + H
+    proj, a = r.standard_normal((T, qrs)).astype(np.float32), r.standard_normal((T, dim)).astype(np.float32)
+    outs = []
+    for value in (0.5, bad):
+        proj[18, 2 * dim:2 * dim + vdim] = value
+        state = DeviceBuffer(cuda_backend, 4 * dim * vdim)
+        op = DeviceOp.delta_rule(0, 1, 1, 2, 1, 3, 4, 5, 0, dim, 2 * dim, 2 * dim + 2 * vdim, oA, odt, onw, T, H, H, dim, vdim, qrs, qrs, dim, qrs, abi.W_F32, 1e-5, 1e-6, 0.4, gate_off=2 * dim + vdim)
+        outs.append(run(cuda_backend, [op], [T * vdim, proj.size, a.size, w.elems, state.elems, 8], [(1, proj), (2, a), (5, ctl_words(0, 0))], 0, (T, vdim), [ExternBuffer(3, w), ExternBuffer(4, state)]))
+        state.free()
+    w.free()
+    assert np.array_equal(outs[0][:18], outs[1][:18]) and not np.isfinite(outs[1][18]).any()

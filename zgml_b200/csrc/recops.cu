@@ -249,6 +249,409 @@ static uint32_t ssm_segments(uint32_t T, uint32_t H, uint32_t N, uint32_t P, uin
     return (T + len - 1) / len;
 }
 
+// ── SSM_SCAN over many tokens: chunks of 64 ──────────────────────────────────────────────────────────────────────
+// A walk token by token reads every B and C value from shared memory for two columns only and waits for its own sums (1024 tokens of 64 heads of
+// 128 x 64: two walks of segments, 78 and 131 us; by chunks 38 + 16 + 56 us, of which the products' packed instructions are 15 + 25.  165 tokens of
+// 4 heads of 64 x 64 and one token after them: 41 -> 25 us).  By chunks of 64 tokens the step is three products with reuse in both directions, all in f32:
+//   S_{c+1} = Gamma_c S_c + sum_s B_s (w_s x_s)^T                   w_s: the step size and the chunk's decays after s
+//   y_t     = P_t C_t^T S_c + sum_{s <= t} (C_t . B_s) W_st x_s      P_t: the chunk's decays up to t, W_st: the step size of s and the decays after s up to t
+// with only products of decays throughout (nothing is divided by one).  C . B is per group, not per head.
+//   k_ssm_chunks:  the sum of the first line per (head, chunk), all chunks side by side; beside them C transposed and C . B per (group, chunk).
+//   k_ssm_chain:   the first line's recurrence from chunk to chunk, one thread per four state elements.
+//   k_ssm_outputs: the second line, every (chunk, head, 64 columns) a CTA of its own: K = N + 64.
+// Products: 8 x 4 outputs per thread as packed pairs, three 16-byte shared loads per 32 of them, sums of 16 terms added to the running ones (a chain of
+// 192 would lose a digit to rounding).  Shared-memory wavefronts and the packed instructions share the time about evenly; an 8 x 8 tile per thread would
+// halve the former but leave too few registers for the sums of 16.
+// From kChunkMinTokens tokens on, where rows can be copied 16 bytes at a time; below two chunks' worth the walk has as little to wait for.
+constexpr uint32_t kChunk = 64, kChunkMinTokens = 128, kChunkK = 32, kChunkStages = 3;
+constexpr size_t kChunkScratch = (size_t)16 << 20;     // f32 slots of states that one pass over the tokens keeps, half of what the L2 holds (longer steps take several passes)
+struct ChunkArgs {
+    SsmArgs a;
+    uint32_t t0, chunks;                              // this pass: tokens from t0 on
+    float4* steps;                                    // [H][chunks * 64]: P_t, decay, step size, w_t
+    float* skip;                                      // [H]
+    float *ct, *cb, *states;                          // [G][chunks][N][64], [G][chunks][64 s][64 t], [chunks][H][N][P]
+};
+__host__ __device__ inline uint32_t chunk_count(uint32_t T, uint32_t H, uint32_t N, uint32_t P) {     // per pass
+    const size_t fit = kChunkScratch / ((size_t)H * N * P);
+    const uint32_t all = (T + kChunk - 1) / kChunk, most = fit < 4 ? 4 : (fit > all ? all : (uint32_t)fit), passes = (all + most - 1) / most;
+    return (all + passes - 1) / passes;
+}
+static size_t chunk_scratch_elems(uint32_t T, uint32_t H, uint32_t G, uint32_t N, uint32_t P) {
+    const size_t c = chunk_count(T, H, N, P);
+    return (size_t)H * c * kChunk * 4 + (H + 3) / 4 * 4 + (size_t)G * c * (N + kChunk) * kChunk + c * H * N * P;
+}
+// element of a head's state in the layout of k_ssm_scan
+__device__ __forceinline__ size_t ssm_state_at(uint32_t h, uint32_t n, uint32_t p, uint32_t N, uint32_t P, uint32_t NS) {
+    const uint32_t RQ = ssm_rq(N), CPB = kSsmThreads / NS * 2, n_cb = (P + CPB - 1) / CPB, i = 4 * (n / 4 / NS) + 2 * ((n / 2) % 2) + p % 2;
+    return (((size_t)h * n_cb + p / CPB) * 32 * RQ + 2 * i + n % 2) * kSsmThreads + p % CPB / 2 * NS + (n / 4) % NS;
+}
+// acc[pair of rows][column] += rows x columns of 16 k; A [k][LDA] at the thread's first row (its other four lie HALF further), B [k][LDB] at its first column.
+// FIRST 2: the other four only.
+template <uint32_t LDA, uint32_t HALF, uint32_t LDB, int FIRST = 0>
+__device__ __forceinline__ void chunk_mma16(float2 (&acc)[4][4], const float* A, const float* B) {
+    float2 t[4][4];
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        float2 av[4];
+#pragma unroll
+        for (int i = FIRST; i < 4; i += 2) {
+            const float4 x = *reinterpret_cast<const float4*>(A + k * LDA + (i / 2) * HALF);
+            av[i] = make_float2(x.x, x.y); av[i + 1] = make_float2(x.z, x.w);
+        }
+        const float4 b = *reinterpret_cast<const float4*>(B + k * LDB);
+        const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = FIRST; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float2 bb = make_float2(bv[j], bv[j]);
+                t[i][j] = k ? __ffma2_rn(av[i], bb, t[i][j]) : __fmul2_rn(av[i], bb);
+            }
+    }
+#pragma unroll
+    for (int i = FIRST; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = __fadd2_rn(acc[i][j], t[i][j]);
+}
+// a thread's place among TR x TC (of its 128 threads): a warp covers 4 x 8, so that its loads of either operand are few distinct, adjacent float4s
+template <uint32_t TR>
+__device__ __forceinline__ void chunk_place(uint32_t& tr, uint32_t& tc) {
+    const uint32_t warp = (threadIdx.x >> 5) % 4, lane = threadIdx.x & 31;
+    tr = warp % (TR / 4) * 4 + lane / 8;
+    tc = warp / (TR / 4) * 8 + lane % 8;
+}
+// A CTA of 256 threads: its halves take every other 16 k; the sums of the second join those of the first (buf: 4096 floats that nobody reads any more).
+__device__ __forceinline__ void chunk_join(float2 (&acc)[4][4], float* buf) {
+    float4* to = reinterpret_cast<float4*>(buf) + threadIdx.x % 128;
+    __syncthreads();
+    if (threadIdx.x >= 128)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) to[(2 * i + j / 2) * 128] = make_float4(acc[i][j].x, acc[i][j].y, acc[i][j + 1].x, acc[i][j + 1].y);
+    __syncthreads();
+    if (threadIdx.x < 128)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+                const float4 x = to[(2 * i + j / 2) * 128];
+                acc[i][j] = make_float2(acc[i][j].x + x.x, acc[i][j].y + x.y);
+                acc[i][j + 1] = make_float2(acc[i][j + 1].x + x.z, acc[i][j + 1].y + x.w);
+            }
+}
+// decays and step sizes of a head over a chunk, two tokens per lane: (P_t, decay, step size, w_t)
+template <typename WT>
+__device__ __forceinline__ void chunk_steps(const ChunkArgs& q, uint32_t h, uint32_t c, const WT* a_log, const WT* dt_bias, float4 (&to)[2]) {
+    const SsmArgs& a = q.a;
+    const uint32_t lane = threadIdx.x & 31;
+    const bool fixed = a.constant != 0;
+    const float neg_a = fixed ? 0.0f : -expf(wld(a_log, h)), bias = fixed ? 0.0f : wld(dt_bias, h);
+    float dt[2], d[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const uint32_t t = q.t0 + c * kChunk + 2 * lane + j;
+        dt[j] = t >= a.T ? 0.0f : fixed ? 1.0f : softplusf_(a.dtl[(size_t)t * a.dt_rs + a.dt_off + h] + bias);
+        d[j] = t >= a.T ? 1.0f : fixed ? a.dtl[h] : expf(neg_a * dt[j]);
+    }
+    // in 64 bits, rounded once: equal decays would all round the same way, and 64 of those in a row were 1e-6
+    double up = (double)d[0] * d[1], down = up;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, up, o), v = __shfl_down_sync(0xffffffffu, down, o);
+        if (lane >= (uint32_t)o) up *= u;
+        if (lane + o < 32) down *= v;
+    }
+    double before = __shfl_up_sync(0xffffffffu, up, 1), after = __shfl_down_sync(0xffffffffu, down, 1);
+    if (lane == 0) before = 1.0;
+    if (lane == 31) after = 1.0;
+    to[0] = make_float4((float)(before * d[0]), d[0], dt[0], (float)(after * d[1] * dt[0]));
+    to[1] = make_float4((float)up, d[1], dt[1], (float)(after * dt[1]));
+}
+constexpr uint32_t kProductK = 128, kProductPitch = kProductK + 4;       // n at a time
+template <uint32_t NT> constexpr uint32_t chunk_smem() {
+    const uint32_t products = (kChunk + 8) * kProductPitch, states = kChunk * (NT + 4096 / NT + 1);      // (at least the 4096 floats of chunk_join)
+    return (products > states ? products : states) * (uint32_t)sizeof(float);
+}
+// First 8 CTAs per (group, chunk): C transposed and C . B, 8 tokens t each.  Then per (head, chunk) and tile of NT state rows x 4096 / NT columns: the state
+// that the chunk reaches from an empty one; the first tile leaves the chunk's decays and step sizes.
+template <typename WT, uint32_t NT, uint32_t HALVES>
+__global__ void __launch_bounds__(128 * HALVES, 4 / HALVES) k_ssm_chunks(ChunkArgs q, const WT* __restrict__ a_log, const WT* __restrict__ dt_bias, const WT* __restrict__ dskip, uint32_t n_tiles, uint32_t p_tiles) {
+    pdl_enter();
+    constexpr uint32_t kThreads = 128 * HALVES;
+    extern __shared__ __align__(16) float sm[];
+    const SsmArgs& a = q.a;
+    const uint32_t tid = threadIdx.x, products = a.G * q.chunks * 8;
+    if (blockIdx.x < products) {
+        float* Bs = sm;
+        float* Cs = sm + kChunk * kProductPitch;
+        const uint32_t part = blockIdx.x % 8, gc = blockIdx.x / 8, g = gc / q.chunks, c = gc % q.chunks, t0 = q.t0 + c * kChunk;
+        const uint32_t s = tid % kChunk, tq = tid / kChunk;
+        constexpr int kPer = 4 / HALVES;               // tokens t per thread
+        float4 acc[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; j++) acc[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (uint32_t n0 = 0; n0 < a.N; n0 += kProductK) {
+            __syncthreads();
+#pragma unroll 6
+            for (uint32_t e = tid; e < (kChunk + 8) * (kProductK / 4); e += kThreads) {
+                const uint32_t r = e / (kProductK / 4), n = 4 * (e % (kProductK / 4)), t = t0 + (r < kChunk ? r : part * 8 + r - kChunk);
+                const bool on = t < a.T && n0 + n < a.N;
+                ssm_copy16(Bs + r * kProductPitch + n, on ? a.xbc + (size_t)t * a.xbc_rs + (r < kChunk ? a.b_off : a.c_off) + (size_t)g * a.N + n0 + n : a.xbc, on);
+            }
+            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (tid < kProductK && n0 + tid < a.N) {
+                float* to = q.ct + ((size_t)gc * a.N + n0 + tid) * kChunk + part * 8;
+#pragma unroll
+                for (int j = 0; j < 8; j += 4)
+                    *reinterpret_cast<float4*>(to + j) = make_float4(Cs[j * kProductPitch + tid], Cs[(j + 1) * kProductPitch + tid], Cs[(j + 2) * kProductPitch + tid], Cs[(j + 3) * kProductPitch + tid]);
+            }
+#pragma unroll 8
+            for (uint32_t n = 0; n < kProductK; n += 4) {
+                const float4 b = *reinterpret_cast<const float4*>(Bs + s * kProductPitch + n);
+#pragma unroll
+                for (int j = 0; j < kPer; j++) {
+                    const float4 x = *reinterpret_cast<const float4*>(Cs + (kPer * tq + j) * kProductPitch + n);
+                    acc[j] = make_float4(fmaf(b.x, x.x, acc[j].x), fmaf(b.y, x.y, acc[j].y), fmaf(b.z, x.z, acc[j].z), fmaf(b.w, x.w, acc[j].w));
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; j += 2)
+            *reinterpret_cast<float2*>(q.cb + ((size_t)gc * kChunk + s) * kChunk + part * 8 + kPer * tq + j) =
+                make_float2((acc[j].x + acc[j].y) + (acc[j].z + acc[j].w), (acc[j + 1].x + acc[j + 1].y) + (acc[j + 1].z + acc[j + 1].w));
+        return;
+    }
+    constexpr uint32_t PT = 4096 / NT;
+    uint32_t item = blockIdx.x - products;
+    const uint32_t nt = item % n_tiles; item /= n_tiles;
+    const uint32_t pt = item % p_tiles; item /= p_tiles;
+    const uint32_t h = item % a.H, c = item / a.H, g = h / (a.H / a.G), n0 = nt * NT, p0 = pt * PT, t0 = q.t0 + c * kChunk;
+    float* Bs = sm;
+    float* Xs = Bs + kChunk * NT;
+    float* Ws = Xs + kChunk * PT;
+#pragma unroll 8
+    for (uint32_t e = tid; e < kChunk * NT / 4; e += kThreads) {
+        const uint32_t tt = e / (NT / 4), col = n0 + 4 * (e % (NT / 4));
+        const bool on = t0 + tt < a.T && col < a.N;
+        ssm_copy16(Bs + 4 * e, on ? a.xbc + (size_t)(t0 + tt) * a.xbc_rs + a.b_off + (size_t)g * a.N + col : a.xbc, on);
+    }
+#pragma unroll 8
+    for (uint32_t e = tid; e < kChunk * PT / 4; e += kThreads) {
+        const uint32_t tt = e / (PT / 4), col = p0 + 4 * (e % (PT / 4));
+        const bool on = t0 + tt < a.T && col < a.P;
+        ssm_copy16(Xs + 4 * e, on ? a.xbc + (size_t)(t0 + tt) * a.xbc_rs + a.x_off + (size_t)h * a.P + col : a.xbc, on);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (tid < 32) {
+        float4 st[2];
+        chunk_steps(q, h, c, a_log, dt_bias, st);
+        Ws[2 * tid] = st[0].w;
+        Ws[2 * tid + 1] = st[1].w;
+        if (nt == 0 && pt == 0) {
+            float4* to = q.steps + ((size_t)h * q.chunks + c) * kChunk + 2 * tid;
+            to[0] = st[0];
+            to[1] = st[1];
+            if (c == 0 && tid == 0) q.skip[h] = a.constant ? 0.0f : wld(dskip, h);
+        }
+    }
+    uint32_t tr, tc;
+    chunk_place<NT / 8>(tr, tc);
+    float2 S[4][4];                                    // [pair of rows][column]
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) S[i][j] = make_float2(0.0f, 0.0f);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (uint32_t e = tid; e < kChunk * PT / 4; e += kThreads) {
+        const float w = Ws[e / (PT / 4)];
+        float4& x = reinterpret_cast<float4*>(Xs)[e];
+        x = make_float4(x.x * w, x.y * w, x.z * w, x.w * w);
+    }
+    __syncthreads();
+    const uint32_t half = tid / 128;
+    if (p0 + 32 * (tc / 8) < a.P)                      // uniform over the warp
+#pragma unroll 1
+        for (uint32_t k = 16 * half; k < kChunk; k += 16 * HALVES) chunk_mma16<NT, NT / 2, PT>(S, Bs + k * NT + 4 * tr, Xs + k * PT + 4 * tc);
+    if (HALVES == 2) {
+        chunk_join(S, Bs);
+        if (half) return;
+    }
+    const uint32_t p = p0 + 4 * tc;
+    float* to = q.states + ((size_t)c * a.H + h) * a.N * a.P + p;
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        const uint32_t n = n0 + (r / 4) * (NT / 2) + 4 * tr + r % 4;
+        if (n < a.N && p < a.P)
+            *reinterpret_cast<float4*>(to + (size_t)n * a.P) = r % 2 ? make_float4(S[r / 2][0].y, S[r / 2][1].y, S[r / 2][2].y, S[r / 2][3].y)
+                                                                      : make_float4(S[r / 2][0].x, S[r / 2][1].x, S[r / 2][2].x, S[r / 2][3].x);
+    }
+}
+// The states the chunks reached from empty ones become the states before them; four columns per thread, eight chunks' loads in flight.
+__global__ void __launch_bounds__(128) k_ssm_chain(ChunkArgs q, uint32_t NS) {
+    pdl_enter();
+    const SsmArgs& a = q.a;
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)a.H * a.N * a.P;
+    if (4 * e >= per) return;
+    const uint32_t p = (uint32_t)(4 * e % a.P), n = (uint32_t)(4 * e / a.P % a.N), h = (uint32_t)(4 * e / a.P / a.N), n_cb = (a.P + kSsmThreads / NS * 2 - 1) / (kSsmThreads / NS * 2);
+    float* state = a.state + (size_t)ctl_word(a.ctl, ZG_CTL_SLOT) * a.H * n_cb * 32 * ssm_rq(a.N) * kSsmThreads;
+    size_t at[4];
+    float s[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) { at[j] = ssm_state_at(h, n, p + j, a.N, a.P, NS); s[j] = state[at[j]]; }
+    float4* z = reinterpret_cast<float4*>(q.states) + e;
+    const float4* steps = q.steps + (size_t)h * q.chunks * kChunk;
+    for (uint32_t c0 = 0; c0 < q.chunks; c0 += 8) {
+        float4 v[8];
+        float gamma[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (c0 + i < q.chunks) { v[i] = z[(c0 + i) * (per / 4)]; gamma[i] = steps[(c0 + i + 1) * kChunk - 1].x; }
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (c0 + i < q.chunks) {
+                z[(c0 + i) * (per / 4)] = make_float4(s[0], s[1], s[2], s[3]);
+                s[0] = fmaf(gamma[i], s[0], v[i].x); s[1] = fmaf(gamma[i], s[1], v[i].y); s[2] = fmaf(gamma[i], s[2], v[i].z); s[3] = fmaf(gamma[i], s[3], v[i].w);
+            }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) state[at[j]] = s[j];
+}
+constexpr uint32_t kChunkOutSmem = (kChunkStages * 2 * kChunkK * kChunk + 5 * kChunk) * sizeof(float);
+template <uint32_t HALVES>
+__global__ void __launch_bounds__(128 * HALVES, 4 / HALVES) k_ssm_outputs(ChunkArgs q) {
+    constexpr uint32_t kThreads = 128 * HALVES;
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    const SsmArgs& a = q.a;
+    constexpr uint32_t stage_elems = 2 * kChunkK * kChunk, PT = 64;
+    float4* step = reinterpret_cast<float4*>(sm + kChunkStages * stage_elems);        // [64]
+    float* head = reinterpret_cast<float*>(step + kChunk);                             // [64]: decays from the start of the token's 16 up to it
+    const uint32_t tid = threadIdx.x, c = blockIdx.x, h = blockIdx.y, g = h / (a.H / a.G), p0 = blockIdx.z * PT;
+    uint32_t tr, tc;                                    // rows 4 tr .. + 3 and 32 more, columns 4 tc .. + 3
+    chunk_place<8>(tr, tc);
+    const uint32_t p = p0 + 4 * tc, half = tid / 128;
+    const uint32_t t0 = q.t0 + c * kChunk, n_n = (a.N + kChunkK - 1) / kChunkK, n_stage = n_n + kChunk / kChunkK;
+    const float* ct = q.ct + ((size_t)g * q.chunks + c) * a.N * kChunk;
+    const float* cb = q.cb + ((size_t)g * q.chunks + c) * kChunk * kChunk;
+    const float* st = q.states + ((size_t)c * a.H + h) * a.N * a.P;
+    auto fetch = [&](uint32_t i) {
+        float* As = sm + i % kChunkStages * stage_elems;
+        float* Bs = As + kChunkK * kChunk;
+#pragma unroll
+        for (uint32_t e = tid; e < kChunkK * kChunk / 4; e += kThreads) {
+            const uint32_t r = e / (kChunk / 4), col = p0 + 4 * (e % (kChunk / 4));
+            if (i < n_n) {
+                const uint32_t n = i * kChunkK + r;
+                ssm_copy16(As + 4 * e, n < a.N ? ct + (size_t)i * kChunkK * kChunk + 4 * e : ct, n < a.N);
+                const bool on = n < a.N && col < a.P;
+                ssm_copy16(Bs + 4 * e, on ? st + (size_t)n * a.P + col : st, on);
+            } else {
+                const uint32_t s = (i - n_n) * kChunkK + r;
+                ssm_copy16(As + 4 * e, cb + (size_t)(i - n_n) * kChunkK * kChunk + 4 * e, true);
+                const bool on = t0 + s < a.T && col < a.P;
+                ssm_copy16(Bs + 4 * e, on ? a.xbc + (size_t)(t0 + s) * a.xbc_rs + a.x_off + (size_t)h * a.P + col : a.xbc, on);
+            }
+        }
+    };
+#pragma unroll
+    for (uint32_t i = 0; i < kChunkStages - 1; i++) {
+        fetch(i);                                      // n_stage is at least 3
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const float4* steps = q.steps + ((size_t)h * q.chunks + c) * kChunk;
+    if (tid < kChunk) {
+        step[tid] = steps[tid];
+        double r = 1.0;
+        for (uint32_t s = tid / 16 * 16; s <= tid; s++) r *= steps[s].y;
+        head[tid] = (float)r;
+    }
+    float2 acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
+    for (uint32_t i = 0; i < n_stage; i++) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        if (i + kChunkStages - 1 < n_stage) fetch(i + kChunkStages - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        float* As = sm + i % kChunkStages * stage_elems;
+        const float* Bs = As + kChunkK * kChunk;
+        bool skip = false;
+        if (i >= n_n) {
+            if (i == n_n) {                            // the products with the state are complete
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const uint32_t t = (r / 2) * 32 + 4 * tr + 2 * (r % 2);
+                    const float2 f = make_float2(step[t].x, step[t + 1].x);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[r][j] = __fmul2_rn(acc[r][j], f);
+                }
+            }
+            // C . B times W, in place: a thread takes one t and 16 (8) s, from its last to its first
+            constexpr uint32_t kRun = 16 / HALVES;
+            const uint32_t t = tid % kChunk, s0 = 32 * (i - n_n) + kRun * (tid / kChunk), bs = s0 / 16, bt = t / 16;       // s0 .. + kRun - 1, all of one 16
+            float r = 1.0f;
+            if (bs < bt) {
+                r = head[t];
+                for (uint32_t b = bs + 1; b < bt; b++) r *= head[16 * b + 15];
+            }
+            for (uint32_t s = s0 + kRun; s < 16 * bs + 16; s++)
+                if (s <= t) r *= step[s].y;
+            bool finite = true;
+#pragma unroll
+            for (int k = kRun - 1; k >= 0; k--) {
+                const uint32_t s = s0 + k, at = (s % kChunkK) * kChunk + t;
+                const float4 f = step[s];
+                const bool seen = s <= t;
+                As[at] = seen ? As[at] * (r * f.z) : 0.0f;
+                if (seen) r *= f.y;
+                finite &= fabsf(Bs[at]) <= 3.4028234e38f;
+            }
+            skip = __syncthreads_or(!finite);
+        }
+        if (!skip) {
+#pragma unroll 1
+            for (uint32_t k = 16 * half; k < kChunkK; k += 16 * HALVES)
+                if (i == n_n + 1) chunk_mma16<kChunk, 32, kChunk, 2>(acc, As + k * kChunk + 4 * tr, Bs + k * kChunk + 4 * tc);      // tokens from 32 on: the first 32 rows have not seen them
+                else chunk_mma16<kChunk, 32, kChunk>(acc, As + k * kChunk + 4 * tr, Bs + k * kChunk + 4 * tc);
+        } else {                                       // an x that is not finite must not meet the zeros of earlier tokens
+#pragma unroll 1
+            for (uint32_t kk = 16 * half; kk < kChunkK; kk += kk % 16 == 15 ? 16 * HALVES - 15 : 1) {
+                const uint32_t s = (i - n_n) * kChunkK + kk;
+                for (uint32_t r = 0; r < 8; r++)
+                    for (uint32_t j = 0; j < 4; j++) {
+                        const uint32_t row = (r / 4) * 32 + 4 * tr + r % 4;
+                        const float v = As[kk * kChunk + row] * Bs[kk * kChunk + 4 * tc + j];
+#pragma unroll
+                        for (uint32_t rr = 0; rr < 4; rr++)
+#pragma unroll
+                            for (uint32_t jj = 0; jj < 4; jj++)
+                                if (r / 2 == rr && j == jj && s <= row) { if (r % 2) acc[rr][jj].y += v; else acc[rr][jj].x += v; }
+                    }
+            }
+        }
+    }
+    if (HALVES == 2) {
+        chunk_join(acc, sm);
+        if (half) return;
+    }
+    const float dsk = q.skip[h];
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        const uint32_t t = t0 + (r / 4) * 32 + 4 * tr + r % 4;
+        if (t >= a.T || p >= a.P) continue;
+        const float4 x = *reinterpret_cast<const float4*>(a.xbc + (size_t)t * a.xbc_rs + a.x_off + (size_t)h * a.P + p);
+        const float y[4] = {r % 2 ? acc[r / 2][0].y : acc[r / 2][0].x, r % 2 ? acc[r / 2][1].y : acc[r / 2][1].x, r % 2 ? acc[r / 2][2].y : acc[r / 2][2].x, r % 2 ? acc[r / 2][3].y : acc[r / 2][3].x};
+        *reinterpret_cast<float4*>(a.dst + ((size_t)t * a.H + h) * a.P + p) = make_float4(fmaf(dsk, x.x, y[0]), fmaf(dsk, x.y, y[1]), fmaf(dsk, x.z, y[2]), fmaf(dsk, x.w, y[3]));
+    }
+}
+
 // ── MIN_GRU, RG_LRU: gated recurrences per channel ───────────────────────────────────────────────────────────────
 // S_t = a_t S_{t-1} + b_t is a linear recurrence per channel whose coefficients do not depend on the state, so the step's
 // tokens are cut into up to 64 segments that are walked side by side: thread (channel, segment) first walks its segment
@@ -449,7 +852,9 @@ size_t zg_rec_op_scratch_elems(const ZgOp& op) {
     if (!s.n[1] || !s.n[3] || !s.n[4] || s.n[3] > (uint32_t)kSsmMaxN) return 0;
     uint32_t len;
     const uint32_t n = ssm_segments(s.n[0], s.n[1], s.n[3], s.n[4], &len);
-    return n > 1 ? (size_t)(n - 1) * (ssm_state_elems(s.n[1], s.n[3], s.n[4]) + s.n[1]) : 0;
+    const size_t walks = n > 1 ? (size_t)(n - 1) * (ssm_state_elems(s.n[1], s.n[3], s.n[4]) + s.n[1]) : 0;
+    const size_t chunks = s.n[0] >= kChunkMinTokens && s.n[2] ? chunk_scratch_elems(s.n[0], s.n[1], s.n[2], s.n[3], s.n[4]) : 0;
+    return walks > chunks ? walks : chunks;
 }
 
 // f32 slots per state slot of an op whose state layout is its own (SSM_SCAN); 0 for every other op
@@ -543,6 +948,46 @@ bool zg_launch_rec_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
                      (reinterpret_cast<uintptr_t>(a.xbc) & 15) == 0) ? 1u : 0u;
             const size_t smem = ((size_t)2 * kSsmTile * (2 * NS * 16 * RQ + CPB) + 2 * kSsmSpan) * sizeof(float);
             const size_t slot_elems = ssm_state_elems(a.H, a.N, a.P);
+            if (scratch && a.T >= kChunkMinTokens && a.vec && (reinterpret_cast<uintptr_t>(a.dst) & 15) == 0) {
+                ChunkArgs q;
+                q.a = a;
+                const uint32_t most = chunk_count(a.T, a.H, a.N, a.P);
+                q.steps = reinterpret_cast<float4*>(scratch);
+                q.skip = scratch + (size_t)a.H * most * kChunk * 4;
+                q.ct = q.skip + (a.H + 3) / 4 * 4;
+                q.cb = q.ct + (size_t)a.G * most * a.N * kChunk;
+                q.states = q.cb + (size_t)a.G * most * kChunk * kChunk;
+                for (q.t0 = 0; q.t0 < a.T; q.t0 += most * kChunk) {
+                    const uint32_t left = (a.T - q.t0 + kChunk - 1) / kChunk;
+                    q.chunks = left < most ? left : most;
+                    const uint32_t NT = a.N <= 32 ? 32 : a.N <= 64 ? 64 : 128, n_tiles = (a.N + NT - 1) / NT, p_tiles = (a.P + 4096 / NT - 1) / (4096 / NT);
+                    const dim3 cgrid(a.G * q.chunks * 8 + a.H * q.chunks * n_tiles * p_tiles);
+                    // The GPU holds about four CTAs of 128 threads per SM; a grid of fewer than two per SM is bound by the latency of each, and takes
+                    // twice the threads for it (224 tokens, 64 heads of 64 x 64: 39 us instead of 45; at 384 CTAs, 349 tokens of 32 heads of 64 x 128,
+                    // 47 us with 128 threads and 55 with 256).
+                    const dim3 ogrid(q.chunks, a.H, (a.P + 63) / 64);
+                    const bool few = ogrid.x * ogrid.y * ogrid.z <= 296;
+#define ZG_SSM_CHUNKS(NT_, HALVES_)                                                                                                           \
+    ZG_SEQ_WDT(s.n[7], launch_pdl(k_ssm_chunks<WT, NT_, HALVES_>, cgrid, dim3(128 * HALVES_), chunk_smem<NT_>(), st, q, a.constant ? (const WT*)nullptr : (const WT*)wptr<WT>(bufs, s.buf[3], s.off[4]), \
+                                  a.constant ? (const WT*)nullptr : (const WT*)wptr<WT>(bufs, s.buf[3], s.off[5]), a.constant ? (const WT*)nullptr : (const WT*)wptr<WT>(bufs, s.buf[3], s.off[6]), n_tiles, p_tiles))
+                    if (few) {
+                        if (NT == 32) ZG_SSM_CHUNKS(32, 2); else if (NT == 64) ZG_SSM_CHUNKS(64, 2); else ZG_SSM_CHUNKS(128, 2);
+                    } else if (NT == 32) ZG_SSM_CHUNKS(32, 1); else if (NT == 64) ZG_SSM_CHUNKS(64, 1); else ZG_SSM_CHUNKS(128, 1);
+#undef ZG_SSM_CHUNKS
+                    ZG_SEQ_CHECK();
+                    launch_pdl(k_ssm_chain, dim3((unsigned)(((size_t)a.H * a.N * a.P / 4 + 127) / 128)), dim3(128), 0, st, q, NS);
+                    ZG_SEQ_CHECK();
+                    if (few) {
+                        cudaFuncSetAttribute(k_ssm_outputs<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkOutSmem);
+                        launch_pdl(k_ssm_outputs<2>, ogrid, dim3(256), kChunkOutSmem, st, q);
+                    } else {
+                        cudaFuncSetAttribute(k_ssm_outputs<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkOutSmem);
+                        launch_pdl(k_ssm_outputs<1>, ogrid, dim3(128), kChunkOutSmem, st, q);
+                    }
+                    ZG_SEQ_CHECK();
+                }
+                return true;
+            }
             uint32_t seg_len = a.T;
             const uint32_t n_seg = scratch ? ssm_segments(a.T, a.H, a.N, a.P, &seg_len) : 1;
             a.seg_len = seg_len;

@@ -1292,7 +1292,10 @@ __global__ void __launch_bounds__(kWalkThreads) k_delta_walk(float* __restrict__
                 }
             }
             const float4 cq = *reinterpret_cast<const float4*>(sc + B + 16 + 4 * lj);
-            total = fmaf(cq.w, u[3], fmaf(cq.z, u[2], fmaf(cq.y, u[1], fmaf(cq.x, u[0], total))));
+            total = fmaf(cq.x, u[0], total);                          // a later token's u is left out, not multiplied by zero: it need not be finite
+            if (lj >= 1) total = fmaf(cq.y, u[1], total);
+            if (lj >= 2) total = fmaf(cq.z, u[2], total);
+            if (lj == 3) total = fmaf(cq.w, u[3], total);
             if (live && (lane & 20) == 4 && tb + lj < T) dst[(size_t)(tb + lj) * dst_rs + (size_t)h * vdim + col0 + lc] = total;
         }
 #pragma unroll
