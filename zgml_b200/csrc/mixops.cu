@@ -284,7 +284,7 @@ __global__ void k_cached_attention(CaArgs a) {
 // > 1 (few rows, long caches: decoding) the keys are dealt in contiguous ranges to gridDim.z CTAs, each leaving (max, sum,
 // unnormalised output) per row for k_cached_attention_merge; a range may be shorter than a tile (its other keys are neither
 // loaded nor counted), since what bounds such a step is how many SMs pull on the cache, not the arithmetic.
-constexpr int kCtBQ = 64, kCtBK = 64, kCtDS = 64, kCtThreads = 256, kCtMaxSplits = 64, kCtMinShare = 32;
+constexpr int kCtBQ = 64, kCtBK = 64, kCtDS = 64, kCtThreads = 256, kCtMaxSplits = 64, kCtMinShare = 32, kCaMaxShares = 160;
 // 16 bytes global -> shared without passing through registers; `on` false writes zeros (nothing is read)
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool on) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -482,24 +482,32 @@ __global__ void __launch_bounds__(kCtThreads) k_cached_attention_tiled(CaArgs a,
 // merge of the key shares: CTA (x, y) = 128 value columns y of (token, head, map) x; a share that saw no key carries
 // max = -inf and weighs nothing (its output is zero)
 // (a: for the sink, the output scale and the row layout of dst; HM = H * maps)
-constexpr int kMergeGroups = 4;        // groups of 128 threads that each add up a quarter of the shares
-__global__ void __launch_bounds__(128 * kMergeGroups) k_cached_attention_merge(CaArgs a, const float* __restrict__ part, uint32_t dv, uint32_t splits,
+constexpr int kMergeCols = 64, kMergeGroups = 8;        // groups of 64 threads that each add up an eighth of the shares
+__global__ void __launch_bounds__(kMergeCols * kMergeGroups) k_cached_attention_merge(CaArgs a, const float* __restrict__ part, uint32_t dv, uint32_t splits,
                                                                 uint32_t wkind) {
     pdl_enter();
-    __shared__ float w[kCtMaxSplits], sums[kMergeGroups][128];
-    const uint32_t group = threadIdx.x >> 7, c = blockIdx.y * 128 + (threadIdx.x & 127);
+    __shared__ float w[kCaMaxShares], sums[kMergeGroups][kMergeCols];
+    const uint32_t group = threadIdx.x / kMergeCols, c = blockIdx.y * kMergeCols + threadIdx.x % kMergeCols;
     const float* P = part + (size_t)blockIdx.x * splits * (4 + dv);
     const uint32_t HM = a.H * a.maps, hm = blockIdx.x % HM;
     if (wkind) {                                       // unnormalised weights: the shares just add up
         if (threadIdx.x < splits) w[threadIdx.x] = a.out_scale;
     } else if (threadIdx.x < 32) {                            // warp 0: the shares' weights exp(m_i - M) / L
-        float m0 = threadIdx.x < splits ? P[threadIdx.x * (4 + dv)] : -INFINITY, m1 = threadIdx.x + 32 < splits ? P[(threadIdx.x + 32) * (4 + dv)] : -INFINITY;
-        float l0 = threadIdx.x < splits ? P[threadIdx.x * (4 + dv) + 1] : 0.0f, l1 = threadIdx.x + 32 < splits ? P[(threadIdx.x + 32) * (4 + dv) + 1] : 0.0f;
-        const float M = warp_max(fmaxf(m0, m1));
-        const float e0 = m0 == -INFINITY ? 0.0f : expf(m0 - M), e1 = m1 == -INFINITY ? 0.0f : expf(m1 - M);
-        const float inv = ca_inv_sum(a, hm, M, warp_sum(l0 * e0 + l1 * e1)) * a.out_scale;
-        if (threadIdx.x < splits) w[threadIdx.x] = e0 * inv;
-        if (threadIdx.x + 32 < splits) w[threadIdx.x + 32] = e1 * inv;
+        constexpr int kPer = kCaMaxShares / 32;
+        float m[kPer], l[kPer], M = -INFINITY, L = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+            const uint32_t j = threadIdx.x + 32 * i;
+            m[i] = j < splits ? P[j * (4 + dv)] : -INFINITY;
+            l[i] = j < splits ? P[j * (4 + dv) + 1] : 0.0f;
+            M = fmaxf(M, m[i]);
+        }
+        M = warp_max(M);
+#pragma unroll
+        for (int i = 0; i < kPer; i++) { m[i] = m[i] == -INFINITY ? 0.0f : expf(m[i] - M); L = fmaf(l[i], m[i], L); }
+        const float inv = ca_inv_sum(a, hm, M, warp_sum(L)) * a.out_scale;
+#pragma unroll
+        for (int i = 0; i < kPer; i++) if (threadIdx.x + 32 * i < splits) w[threadIdx.x + 32 * i] = m[i] * inv;
     }
     __syncthreads();
     float acc = 0.0f;
@@ -507,7 +515,7 @@ __global__ void __launch_bounds__(128 * kMergeGroups) k_cached_attention_merge(C
 #pragma unroll 16
         for (uint32_t i = group; i < splits; i += kMergeGroups) acc = fmaf(P[i * (4 + dv) + 4 + c], w[i], acc);
     }
-    sums[group][threadIdx.x & 127] = acc;
+    sums[group][threadIdx.x % kMergeCols] = acc;
     __syncthreads();
     if (group || c >= dv) return;
 #pragma unroll
@@ -523,15 +531,19 @@ __global__ void __launch_bounds__(128 * kMergeGroups) k_cached_attention_merge(C
 // keys kq and kq + 16 of its row, and the 16 threads of a row keep the row's running (max, sum) in step through half-warp
 // shuffles; for the weighted sum thread t owns value columns t + 256 i of all rows.  Where the value row is the head of the
 // key row itself (a latent that serves as both), it is not loaded twice.
-constexpr int kCfRows = 16, kCfKeys = 32, kCfThreads = 256, kCfParts = kCfThreads / 32;
-template <int CI, bool POOL>
+// Wide rows leave room for one CTA per SM, whose eight warps waited for their shared-memory reads most of the time: it has sixteen then (the slices
+// of the key dimension and the columns per thread halve).  One token, 16 heads, 8192 latents of 576: with 148 shares instead of 64 and sixteen warps
+// 45 -> 24 us, the op with its merge and the append 54 -> 33.
+constexpr int kCfRows = 16, kCfKeys = 32;
+template <int kCfThreads, int CI, bool POOL>
 __global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, uint32_t rh, uint32_t splits, float* __restrict__ part, uint32_t alias) {
     pdl_enter();
+    constexpr int kCfParts = kCfThreads / 32;
     extern __shared__ __align__(16) float sm[];
     const uint32_t KP = a.dk + 4, VP = alias ? KP : a.dv;
     float* Qs = sm;                                    // [16][dk + 4]
     float* Ks = Qs + kCfRows * KP;                     // [32][dk + 4]
-    float* Sp = Ks + kCfKeys * KP;                     // [8][16][32] partial scores of the eight slices of the key dimension
+    float* Sp = Ks + kCfKeys * KP;                     // [warps][16][32] partial scores of the warps' slices of the key dimension
     float* Ss = Sp + kCfParts * kCfRows * kCfKeys;     // [16][32] probabilities
     float* Al = Ss + kCfRows * kCfKeys;                // [16] rescale of the running sums (at the end: 1 / sum)
     float* Vs = alias ? Ks : Al + kCfRows;             // [32][dv]
@@ -549,7 +561,7 @@ __global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, u
     const CaKeys<POOL> vals = ca_keys<POOL>(vbase, POOL ? a.vp + pool_slot + (size_t)g * a.dv : nullptr, a.R, a.vw, k_lo, n_pool);
     const uint32_t n_keys = keys.count(p_max), per = (n_keys + splits - 1) / splits;
     const uint32_t k_begin = keys.first() + blockIdx.y * per, k_end = min(keys.first() + n_keys, k_begin + per);
-    const bool ok = row < total;
+    const bool ok = row < total, owner = tid < 16 * kCfRows;        // owner: of a row's running (max, sum)
     const uint32_t p_r = pos0 + (ok ? row / rh : 0), lo_r = mask_low(p_r, a.kind, a.size), nb_r = POOL ? pooled_seen(p_r, a.size, a.pool) : 0u;
     const float* tab_r = a.tab ? a.tab + (size_t)((g * rh + (ok ? row % rh : 0)) * a.maps + m) * a.tab_rs : nullptr;
     const uint32_t dk4 = a.dk / 4, dv4 = a.dv / 4;
@@ -605,34 +617,36 @@ __global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, u
                 for (int c = 0; c < 4; c++) Sp[(warp * kCfRows + rg + 4 * r) * kCfKeys + kg + 8 * c] = sc[r][c];
         }
         __syncthreads();
-        float sv[2];
+        if (owner) {
+            float sv[2];
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const uint32_t kk = kq + 16 * u, j = s0 + kk;
-            float d = 0.0f;
+            for (int u = 0; u < 2; u++) {
+                const uint32_t kk = kq + 16 * u, j = s0 + kk;
+                float d = 0.0f;
 #pragma unroll
-            for (int w = 0; w < kCfParts; w++) d += Sp[(w * kCfRows + row) * kCfKeys + kk];
-            const bool seen = ok && kk < nk && keys.seen(j, p_r, lo_r, nb_r);
-            sv[u] = seen ? ca_score(a, d) : -INFINITY;
-            if (!POOL && seen && tab_r) sv[u] += tab_r[p_r - j];
+                for (int w = 0; w < kCfParts; w++) d += Sp[(w * kCfRows + row) * kCfKeys + kk];
+                const bool seen = ok && kk < nk && keys.seen(j, p_r, lo_r, nb_r);
+                sv[u] = seen ? ca_score(a, d) : -INFINITY;
+                if (!POOL && seen && tab_r) sv[u] += tab_r[p_r - j];
+            }
+            float rmax = fmaxf(sv[0], sv[1]);
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
+            const float new_m = a.wkind ? 0.0f : fmaxf(m_run, rmax);
+            const float alpha = a.wkind ? 1.0f : (m_run == -INFINITY ? (new_m == -INFINITY ? 1.0f : 0.0f) : expf(m_run - new_m));
+            float rsum = 0.0f;
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const float pv = sv[u] == -INFINITY ? 0.0f : (a.wkind ? ca_sigmoid(sv[u]) : expf(sv[u] - new_m));
+                Ss[row * kCfKeys + kq + 16 * u] = pv;
+                rsum += pv;
+            }
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1) rsum += __shfl_xor_sync(0xffffffffu, rsum, off);
+            l_run = l_run * alpha + rsum;
+            m_run = new_m;
+            if (kq == 0) Al[row] = alpha;
         }
-        float rmax = fmaxf(sv[0], sv[1]);
-#pragma unroll
-        for (int off = 8; off > 0; off >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
-        const float new_m = a.wkind ? 0.0f : fmaxf(m_run, rmax);
-        const float alpha = a.wkind ? 1.0f : (m_run == -INFINITY ? (new_m == -INFINITY ? 1.0f : 0.0f) : expf(m_run - new_m));
-        float rsum = 0.0f;
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const float pv = sv[u] == -INFINITY ? 0.0f : (a.wkind ? ca_sigmoid(sv[u]) : expf(sv[u] - new_m));
-            Ss[row * kCfKeys + kq + 16 * u] = pv;
-            rsum += pv;
-        }
-#pragma unroll
-        for (int off = 8; off > 0; off >>= 1) rsum += __shfl_xor_sync(0xffffffffu, rsum, off);
-        l_run = l_run * alpha + rsum;
-        m_run = new_m;
-        if (kq == 0) Al[row] = alpha;
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kCfRows; r++) {
@@ -656,7 +670,7 @@ __global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, u
         }
     }
     __syncthreads();
-    if (kq == 0) Al[row] = (a.wkind ? 1.0f : (l_run > 0.0f ? ca_inv_sum(a, (g * rh + (ok ? row % rh : 0)) * a.maps + m, m_run, l_run) : 0.0f)) * a.out_scale;
+    if (owner && kq == 0) Al[row] = (a.wkind ? 1.0f : (l_run > 0.0f ? ca_inv_sum(a, (g * rh + (ok ? row % rh : 0)) * a.maps + m, m_run, l_run) : 0.0f)) * a.out_scale;
     if (splits > 1 && kq == 0 && ok) {
         float* mine = part + (((size_t)(row / rh) * a.H * a.maps + (g * rh + row % rh) * a.maps + m) * splits + blockIdx.y) * (4 + a.dv);
         mine[0] = m_run; mine[1] = l_run;
@@ -676,8 +690,8 @@ __global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, u
         }
     }
 }
-static size_t cf_smem(uint32_t dk, uint32_t dv, bool alias) {
-    return ((size_t)(kCfRows + kCfKeys) * (dk + 4) + (size_t)(kCfParts + 1) * kCfRows * kCfKeys + kCfRows + (alias ? 0 : (size_t)kCfKeys * dv)) * sizeof(float);
+static size_t cf_smem(uint32_t dk, uint32_t dv, bool alias, uint32_t warps) {
+    return ((size_t)(kCfRows + kCfKeys) * (dk + 4) + (size_t)(warps + 1) * kCfRows * kCfKeys + kCfRows + (alias ? 0 : (size_t)kCfKeys * dv)) * sizeof(float);
 }
 static bool cf_alias(const ZgSeqOp& s) {   // the value row is the head of the key row (one key head, one map, same cache and column)
     return s.buf[2] == s.buf[3] && s.off[1] == s.off[2] && s.n[2] == 1 && s.n[3] == 1 && s.n[5] <= s.n[4] && s.n[7] == s.n[8];
@@ -696,7 +710,7 @@ static bool ca_aligned(const ZgSeqOp& s) {
     return s.n[4] % 4 == 0 && s.n[5] % 4 == 0 && s.n[6] % 4 == 0 && s.n[7] % 4 == 0 && s.n[8] % 4 == 0 && s.off[0] % 4 == 0 && s.off[1] % 4 == 0 && s.off[2] % 4 == 0;
 }
 static bool ca_few(const ZgSeqOp& s) {
-    return ca_aligned(s) && s.n[0] * (s.n[1] / s.n[2]) <= (uint32_t)kCfRows && cf_smem(s.n[4], s.n[5], cf_alias(s)) <= 200 * 1024;
+    return ca_aligned(s) && s.n[0] * (s.n[1] / s.n[2]) <= (uint32_t)kCfRows && cf_smem(s.n[4], s.n[5], cf_alias(s), 8) <= 200 * 1024;
 }
 // keys a step's rows can see at most
 static uint32_t ca_reach(const ZgSeqOp& s) {
@@ -718,7 +732,8 @@ static uint32_t ca_splits(const ZgSeqOp& s) {
     if (ca_few(s)) {
         const uint32_t reach = ca_reach(s);
         const uint32_t S = (reach + kCfKeys - 1) / kCfKeys;
-        return S < 2 ? 1 : (S > (uint32_t)kCtMaxSplits ? (uint32_t)kCtMaxSplits : S);
+        const uint32_t sms = (uint32_t)sm_count() / (s.n[2] * s.n[3]), most = min(max(sms, (uint32_t)kCtMaxSplits), (uint32_t)kCaMaxShares);      // one key head: a share per SM
+        return S < 2 ? 1 : (S > most ? most : S);
     }
     const uint32_t rh = s.n[1] / s.n[2], n_tiles = (s.n[0] * rh + kCtBQ - 1) / kCtBQ, dvs = s.n[5] > 256 ? 512 : (s.n[5] > 128 ? 256 : 128);
     const uint32_t ctas = n_tiles * s.n[2] * s.n[3] * ((s.n[5] + dvs - 1) / dvs);
@@ -1136,27 +1151,30 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
             if (aligned && ca_few(s)) {
                 const uint32_t S = scratch ? ca_splits(s) : 1, alias = cf_alias(s) ? 1u : 0u;
                 float* part = S > 1 ? scratch : nullptr;
-                const size_t smem = cf_smem(a.dk, a.dv, alias != 0);
+                // sixteen warps where the rows are wide enough to keep a second CTA off the SM
+                const bool wide = cf_smem(a.dk, a.dv, alias != 0, 8) > 112 * 1024 && cf_smem(a.dk, a.dv, alias != 0, 16) <= 200 * 1024;
+                const size_t smem = cf_smem(a.dk, a.dv, alias != 0, wide ? 16 : 8);
                 const dim3 grid(a.G * a.maps, S);
-#define ZG_CF(CI_)                                                                                                                         \
+#define ZG_CF(THREADS_, CI_)                                                                                                               \
     do {                                                                                                                                   \
         static size_t most[2] = {48 * 1024, 48 * 1024};                                                                                    \
-        auto kernel = a.pool ? k_cached_attention_few<CI_, true> : k_cached_attention_few<CI_, false>;                                     \
+        auto kernel = a.pool ? k_cached_attention_few<THREADS_, CI_, true> : k_cached_attention_few<THREADS_, CI_, false>;                 \
         if (smem > most[a.pool != 0]) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); most[a.pool != 0] = smem; } \
-        launch_pdl(kernel, grid, dim3(kCfThreads), smem, st, a, a.H / a.G, S, part, alias);                            \
+        launch_pdl(kernel, grid, dim3(THREADS_), smem, st, a, a.H / a.G, S, part, alias);                              \
     } while (0)
-                if (a.dv <= 256) ZG_CF(1); else if (a.dv <= 512) ZG_CF(2); else ZG_CF(4);
+                if (wide) { if (a.dv <= 512) ZG_CF(512, 1); else ZG_CF(512, 2); }
+                else if (a.dv <= 256) ZG_CF(256, 1); else if (a.dv <= 512) ZG_CF(256, 2); else ZG_CF(256, 4);
 #undef ZG_CF
                 if (S > 1) {
                     ZG_SEQ_CHECK();
-                    launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + 127) / 128), dim3(128 * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
+                    launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
                 }
             } else if (aligned && scratch && ca_tensor(s)) {
                 uint32_t S = 1;
                 float* part = nullptr;
                 if (!zg_attention_tc_launch(ca_shape(s), &a, scratch, sm_count(), st, &S, &part)) return false;
                 if (S == 1) return true;
-                launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + 127) / 128), dim3(128 * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
+                launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
             } else if (aligned) {
                 const uint32_t S = scratch && !ca_tensor(s) ? ca_splits(s) : 1;
                 float* part = S > 1 ? scratch : nullptr;
@@ -1175,7 +1193,7 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
                 }
                 if (S > 1) {
                     ZG_SEQ_CHECK();
-                    launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + 127) / 128), dim3(128 * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
+                    launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
                 }
             } else {
                 const uint32_t warps = 4, items = a.T * a.H * a.maps;
