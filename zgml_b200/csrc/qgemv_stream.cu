@@ -9,7 +9,8 @@
 //
 //  * the launch is ONE linear space: (matvec of the batch, block of 8 column groups, k) measured in chunks of G
 //    records; CTA c takes chunks [c per, (c + 1) per) — every CTA the same amount whatever the shape, one round of
-//    CTAs, `per` snapped to a divisor / multiple of a column group's chunk count so that cuts fall on few, aligned places;
+//    CTAs, `per` snapped to a divisor / multiple of a column group's chunk count (padded to one where none is near) so that
+//    cuts fall on few, aligned places;
 //  * inside a CTA each warp owns ONE column group of the block and walks the CTA's whole k-range for it (a contiguous
 //    run of records -> one TMA bulk copy per chunk into the warp's ring): no cross-warp reduction, no CTA barrier in
 //    the streaming loop, one flush per (column group, segment) instead of one per 16 records;
@@ -43,7 +44,7 @@ struct QGemvSParams {
     QGemvSOp op[kZgGemvBatch];
     uint32_t n_kc, n_nb, K, N;
     uint32_t GB;       // blocks of 8 column groups per matvec
-    uint32_t nq;       // chunks per column group = ceil(n_kc / G)
+    uint32_t nq;       // chunks per column group = ceil(n_kc / G), or a little more: chunks past n_kc hold nothing
     uint32_t TQ;       // chunks of the whole launch = count * GB * nq
     uint32_t per;      // chunks per CTA: CTA c takes [c * per, (c + 1) * per)
     uint32_t Lq;       // chunks per segment at most
@@ -447,6 +448,20 @@ bool zg_qgemv_stream_init(ZgCudaCtx* ctx) {
     return set_stream_attr<ZG_QFMT_I8_F32>() && set_stream_attr<ZG_QFMT_I8_F16>() && set_stream_attr<ZG_QFMT_I4_F16>();
 }
 
+// No divisor of a column group's chunk count near `per`: the group is cut into nq / per pieces of one size, the last of which holds a few chunks less
+// (they count as chunks past the end of K).  Every segment of every piece keeps at least one real chunk.
+// (nq = 181: whole groups were 38 CTAs, two 11552 x 4704 q8_0 matvecs took 66 us; in 7 pieces 27.)
+static void pad_group(ZgGemvStreamPlan& pl, uint32_t count, uint32_t& per) {
+    const uint32_t n = pl.nq / per;
+    for (per = (pl.nq + n - 1) / n; per < pl.nq; per++) {
+        const uint32_t pieces = (pl.nq + per - 1) / per, last = pl.nq - (pieces - 1) * per;
+        if ((last + pl.Lq - 1) / pl.Lq != (per + pl.Lq - 1) / pl.Lq) continue;
+        pl.nq = pieces * per;
+        pl.TQ = count * pl.GB * pl.nq;
+        return;
+    }
+    per = pl.nq;
+}
 // Plan of the streamed form for `count` matvecs of w's shape in one launch; use == false: the k-split kernel of qgemv.cu
 // takes the launch (little work per CTA: its finer split keeps more warps busy).
 ZgGemvStreamPlan zg_qgemv_stream_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t count) {
@@ -475,7 +490,12 @@ ZgGemvStreamPlan zg_qgemv_stream_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight*
     uint32_t per = std::max(per_min, (pl.TQ + slots_max - 1) / slots_max);
     if (ctx->stream_align == 1 || (ctx->stream_align == 0 && per < 2 * pl.nq)) {
         if (per < pl.nq && pl.TQ / pl.nq >= 128) per = pl.nq;       // whole column groups still give >= 128 CTAs: no cuts, no partials
-        else if (per < pl.nq) { while (pl.nq % per) per++; }          // smallest divisor of nq that is >= per (nq itself at the latest)
+        else if (per < pl.nq) {
+            uint32_t d = per;
+            while (pl.nq % d) d++;                                    // smallest divisor of nq that is >= per (nq itself at the latest)
+            if (4 * (pl.nq / d) >= 3 * (pl.nq / per)) per = d;
+            else pad_group(pl, count, per);
+        }
         else per = ((per + pl.nq - 1) / pl.nq) * pl.nq;
     }
     pl.per = per;
