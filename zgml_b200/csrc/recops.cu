@@ -237,7 +237,7 @@ static size_t ssm_state_elems(uint32_t H, uint32_t N, uint32_t P) {
 // issue slots), one CTA per (head, column block), so a long step of a model with few of those is cut while the GPU still holds
 // no more than about three CTAs per SM — beyond that the second walk of every token costs more than the segments gain
 // (measured at 1024 tokens: 32 heads 252 -> 115 us, 64 heads 252 -> 211 us with five segments, 128 heads 308 -> 373 us with
-// three).  A segment has at least 64 tokens.
+// three).  A segment has at least 64 tokens.  (Steps of kChunkMinTokens tokens whose rows can be copied 16 bytes at a time go by chunks instead.)
 static uint32_t ssm_segments(uint32_t T, uint32_t H, uint32_t N, uint32_t P, uint32_t* seg_len) {
     const uint32_t CPB = kSsmThreads / ssm_slices(N) * 2, ctas = H * ((P + CPB - 1) / CPB);
     uint32_t n = 448 / (ctas ? ctas : 1);
@@ -845,7 +845,8 @@ __global__ void k_activation(float* dst, const float* src, uint32_t n, uint32_t 
 
 }  // namespace
 
-// shared scratch of a long SSM_SCAN step: per segment but the last, a state (reached, then starting) and the product of its decays per head
+// shared scratch of a long SSM_SCAN step: by chunks (whether its rows are aligned for that is known at the launch), or per segment but the last a state
+// (reached, then starting) and the product of its decays per head
 size_t zg_rec_op_scratch_elems(const ZgOp& op) {
     if (op.tag != ZG_OP_SSM_SCAN) return 0;
     const ZgSeqOp& s = op.u.seq;
