@@ -1,5 +1,5 @@
 """MOE_FFN over bfloat16 weights with more than 16 (token, choice) pairs (experts' products on the tensor cores) against float64: runs of one row, of whole
-and partial multiples of 16, at and past the 256 rows of a run, experts without a row, pairs that no expert takes, widths that end within the 64-wide
+and partial multiples of 16, at and past the most rows of a run (64 where tiles are few, 256 in the last case), experts without a row, pairs that no expert takes, widths that end within the 64-wide
 steps and the 128-wide tiles.
 
 The reference rounds what the kernels round (inputs and the activated products to bfloat16) and is float64 otherwise.  Where an f32 sum falls on the other
@@ -20,7 +20,7 @@ def bf16(x):
 
 
 @pytest.mark.parametrize("counts,top,D,ff", [([17], 1, 64, 64), ([0, 1, 16, 0, 40], 1, 72, 136), ([31, 32, 33], 1, 128, 200), ([256, 0, 257], 1, 200, 64), ([513, 15], 1, 64, 128),
-                                             ([300, 20, 270], 2, 136, 264), ([5, 6, 7], 1, 1032, 72), ([100, 28], 2, 64, 1000)])
+                                             ([300, 20, 270], 2, 136, 264), ([5, 6, 7], 1, 1032, 72), ([100, 28], 2, 64, 1000), ([300, 0, 257, 256, 1, 16, 17, 49], 1, 64, 2432)])
 def test_expert_products(cuda_backend, counts, top, D, ff):
     from zgml_b200 import DeviceBuffer, DeviceOp, ExternBuffer, abi
     from zgml_b200.backend import seq_scratch_elems

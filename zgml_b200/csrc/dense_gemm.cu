@@ -300,7 +300,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 // and read the weights again for it).  DUAL: two weight matrices against the same rows, gate and up, and out = bf16(act(gate) up), so that neither
 // product goes through memory.
 // Bound by the stream of weights.  1024 tokens, two of 16 experts, 2048 x 2048, cold: gate, up and activation 68 us (98 as two products and a pass of
-// their own over whole tiles), down 40 us (42); the op 129 us (171), 44 tokens on one of 4 experts of 1696 x 1088 31 us (60).
+// their own over whole tiles), down 40 us (42); the op 124 us (171), 44 tokens on one of 4 experts of 1696 x 1088 29 us (60).
 constexpr uint32_t kExpertThreads = 320;          // warp 0: TMA, warp 1: MMA + TMEM, warps 2-9: epilogue
 constexpr uint32_t kExpertRows = 32;              // rows of x per copy
 constexpr uint32_t kExpertRing = 216 * 1024, kExpertSmem = kExpertRing + 1024 + 256, kExpertStages = 8;
