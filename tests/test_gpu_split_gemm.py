@@ -1,9 +1,9 @@
-"""LINEAR of many rows over f32 weights (operands split into half-precision pairs on the tensor cores) against float64: edges of the 128 x 128 tiles and of
-the 64-k steps, one and several shares of K, strided rows, bias, activation on part of the columns, gated pairs, rows of very different magnitude, and
-rows that hold an infinity or a NaN.
+"""LINEAR of many rows over f32 weights (operands cut into three bfloat16 parts on the tensor cores) against float64: edges of the 128 x 128 tiles and of
+the 64-k steps, one and several shares of K, strided rows, bias, activation on part of the columns, gated pairs, magnitudes that differ between rows and
+within a row, sums near the largest float, and rows that hold an infinity or a NaN.
 
-Tolerance: a split operand keeps 2^-23 of itself (2^-39 of its row's largest of 64), a 64-k step adds four truncated f32 sums and up to 100 steps add in f32: 3e-6 of
-sqrt(K) |x| |w| is over three times what that makes; the plain f32 sum shows about 1e-6."""
+Tolerance: three parts hold every operand whole, the products left out are below 2^-25 of one product, a 64-k step adds four truncated f32 sums and up to
+100 steps add in f32: 3e-6 of sqrt(K) |x| |w| is over three times what that makes; the plain f32 sum shows about 1e-6."""
 import numpy as np
 import pytest
 
@@ -64,3 +64,61 @@ def test_non_finite_rows(cuda_backend):
     assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[~fin & ~np.isnan(want)], want[~fin & ~np.isnan(want)].astype(np.float32))
     assert np.abs(got[fin] - want[fin]).max() < 1e-4
     buf.free()
+
+
+def waits_given_up(be):
+    from zgml_b200 import DeviceOp, DeviceProgram
+    h = be.compile_program(DeviceProgram([DeviceOp.rmsnorm(1, 0, 1, 32, 1e-5)], [32, 32], [], []))
+    n = be.program_stats(h)["dense_gemm_timeouts"]
+    be.free_program(h)
+    return n
+
+
+def linear(be, x, W, **kwargs):
+    from zgml_b200 import DeviceOp, ExternBuffer, abi
+    (M, K), N = x.shape, len(W)
+    buf, (ow,) = weights(be, W)
+    got = run(be, [DeviceOp.linear(0, 1, 2, ow, M, N, K, abi.W_F32, **kwargs)], [M * N, x.size, buf.elems], [(1, x)], 0, (M, N), [ExternBuffer(2, buf)])
+    buf.free()
+    return got
+
+
+def test_one_hot_weights_return_the_inputs(cuda_backend):
+    """Every output is one input, whatever else its row holds: magnitudes from 2^-60 to 2^60 in each row, all 24 bits."""
+    r = np.random.default_rng(4)
+    M, N, K = 140, 132, 200
+    x = (r.standard_normal((M, K)) * 2.0 ** r.integers(-60, 61, (M, K))).astype(np.float32)
+    pick = r.integers(0, K, N)
+    W = np.zeros((N, K), np.float32)
+    W[np.arange(N), pick] = 1.0
+    assert np.array_equal(linear(cuda_backend, x, W), x[:, pick])
+
+
+@pytest.mark.parametrize("where", ["source", "weights"])
+def test_large_elements_that_meet_zeros(cuda_backend, where):
+    """2^20 to 2^40 beside values around 1, against zeros: the bound is that of the sum without them."""
+    r = np.random.default_rng(6)
+    M, N, K = 130, 140, 320
+    x, W = r.standard_normal((M, K)).astype(np.float32), r.standard_normal((N, K)).astype(np.float32)
+    a, b = (x, W) if where == "source" else (W, x)
+    rest = np.arange(K) % 16 != 5
+    b[:, ~rest] = 0.0
+    a[:, ~rest] = 2.0 ** r.integers(20, 41, (len(a), K // 16))
+    check(linear(cuda_backend, x, W), x[:, rest], W[:, rest], x.astype(np.float64) @ W.astype(np.float64).T)
+
+
+@pytest.mark.parametrize("big,small", [(1e33, 1e-3), (1e38, 1e-30), (3e38, 1e-3), (1e-30, 1e28)])
+@pytest.mark.parametrize("where", ["source", "weights"])
+def test_finite_sums_of_extreme_operands(cuda_backend, big, small, where):
+    r = np.random.default_rng(7)
+    M, N, K = 20, 130, 192
+    x, W = r.uniform(-1, 1, (M, K)), r.uniform(-1, 1, (N, K))
+    x, W = (x * (big if where == "source" else small)).astype(np.float32), (W * (small if where == "source" else big)).astype(np.float32)
+    want = x.astype(np.float64) @ W.astype(np.float64).T
+    assert np.abs(want).max() < 1e37
+    check(linear(cuda_backend, x, W), x, W, want)
+
+
+def test_no_wait_ran_out(cuda_backend):
+    """Statistic 5 of a program counts the waits that its tensor-core kernels gave up on: none, after everything above."""
+    assert waits_given_up(cuda_backend) == 0

@@ -25,6 +25,10 @@ void zg_set_error(const char* fmt, ...) {
 extern "C" const char* zg_cuda_last_error(void) { return g_err; }
 extern "C" uint64_t zg_cuda_launch_count(void) { return g_zg_launches.load(); }
 
+uint32_t zg_sm_count() {
+    static const uint32_t n = [] { int dev = 0, v = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); return (uint32_t)(v > 0 ? v : 148); }();
+    return n;
+}
 bool zg_gemv_ws_reserve(ZgGemvWs* ws, size_t partial_elems, size_t counters, cudaStream_t st, size_t gemm_scratch_elems) {
     if (gemm_scratch_elems > ws->gemm_scratch_elems) {
         if (ws->gemm_scratch) { cudaStreamSynchronize(st); cudaFree(ws->gemm_scratch); ws->gemm_scratch = nullptr; }
@@ -2138,7 +2142,7 @@ extern "C" int zg_cuda_program_promote_dense(ZgCudaCtx* ctx, ZgCudaProgram* p, i
 extern "C" uint64_t zg_cuda_program_stats(const ZgCudaProgram* p, int what) {
     if (!p) return 0;
     switch (what) {
-        case 5: return zg_dense_gemm_timeouts();
+        case 5: return zg_dense_gemm_timeouts() + zg_split_gemm_timeouts();
         case 6: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && op.u.seq.n[5] == ZG_W_BF16 && zg_seq_op_scratch_elems(op, p->buffers.data())) n++; return n; }
         case 0: return p->graph_kernels;
         case 1: return p->dec.valid ? p->dec_count : 0;

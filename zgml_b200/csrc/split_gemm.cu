@@ -1,36 +1,47 @@
 // LINEAR of many rows over f32 weights on the tensor cores, with f32 accuracy:  part[m, n] = sum_k src[m, k] W[n, k].
 //
-// Both operands are split into half-precision pairs (split_tc.cuh) inside the kernel, 64 k at a time, each row of the 64 with a scale of its own; a product
-// is three MMAs, hi lo + lo hi + hi hi.  The tensor core's f32 accumulator truncates, which over a long sum would cost more than an f32 chain
-// rounds, so it holds the products of ONE 64-k step (four additions of hi hi) and the steps are added in registers in f32, with the two rows' scales
-// undone on the way.
+// Both operands are cut into three bfloat16 parts inside the kernel, 64 k at a time: b0 = bf16(x), b1 = bf16(x - b0), b2 = x - b0 - b1.  Three 8-bit
+// significands hold all 24 bits of x, and every part has an f32's range of exponents: nothing is scaled, and what one element of a row keeps does not
+// depend on the others (pairs of half precision with a scale per row and 64 k, three MMAs a product, lost the small elements beside a large one and
+// left f32's range before the scales were undone).  Below 2^-109 the last part runs out of exponents: such an element is held to 2^-134.
+// A product is the six MMAs b1 b1 + b0 b2 + b2 b0 + b0 b1 + b1 b0 + b0 b0, the smallest first; what is left out (b1 b2 and smaller) is at most 2^-23 of it,
+// 2^-26 on average.
+// The tensor core's f32 accumulator truncates, which over a long sum would cost more than an f32 chain rounds, so it holds the products of ONE 64-k step
+// (four additions of b0 b0) and the steps are added in registers in f32.  Error against 64 bits at 256 tokens, 2048 / 4096: 1.7e-7 (pairs 2.1e-7, the f32
+// tile 8.7e-7).
 //
-//   * 128 x 128 tile per CTA, grid (n tiles, m tiles, shares of K).  Sixteen worker warps load f32 rows (16 lanes per row of 64), find the row's maximum by
-//     shuffles, split, and store swizzled K-major tiles into a 3-stage ring; the same warps drain the accumulators of the step before (two TMEM
-//     buffers), each a quarter of the columns of its 32 rows.  Warp 16 issues the MMAs.
-//   * Per step the MMAs take 768 clocks, their operand reads and the workers' stores 1280 clocks of shared-memory bandwidth, the workers' instructions
-//     about 1500 issue slots per scheduler: the workers bound it.
-//   * Tiles leave as partial sums; k_split_finish adds the shares in order and applies bias and activation.  A result that is not a number is evaluated
-//     again there as a plain f32 sum: a row whose maximum is not finite has no scale, and what an infinity makes of a sum is the plain kernel's.
-//   * Every wait is bounded; a CTA whose wait ran out writes NaN, so that its outputs are evaluated again the plain way.
+//   * 128 x 128 tile per CTA, grid (n tiles, m tiles, shares of K).  Sixteen worker warps load f32 rows (16 lanes per row of 64), cut them, and store
+//     swizzled K-major tiles into a 2-stage ring; the same warps drain the accumulators of the step before (two TMEM buffers), each a quarter of the
+//     columns of its 32 rows.  Warp 16 issues the MMAs.
+//   * Per step the MMAs take 1536 clocks, their operand reads and the workers' stores 2300 clocks of shared-memory bandwidth; the f32 rows of the next step
+//     are in flight for one step only, and their latency bounds the kernel.
+//   * Tiles leave as partial sums; k_split_finish adds the shares in order and applies bias and activation.  A sum that is not finite is evaluated again
+//     there as a plain f32 sum: what an infinity makes of a sum is the plain kernel's.
+//   * Every wait is bounded; a CTA whose wait ran out counts it and writes NaN, so that its outputs are evaluated again the plain way.
 #include "split_tc.cuh"
 
 namespace {
 
 constexpr uint32_t kBM = 128, kBN = 128, kBK = 64;
-constexpr uint32_t kTile = kBM * kBK * 2, kSgStage = 4 * kTile, kSgStages = 3, kSgWorkers = 512, kSgThreads = kSgWorkers + 32;
-constexpr uint32_t kSgScales = 4 * (kBM + kBN) * 4;               // of four steps: a warp may be two ahead of another's drain
-constexpr uint32_t kSgSmem = kSgStages * kSgStage + kSgScales + 1024 + 128;
+constexpr uint32_t kTile = kBM * kBK * 2, kSgStage = 6 * kTile, kSgStages = 2, kSgWorkers = 512, kSgThreads = kSgWorkers + 32;
+constexpr uint32_t kSgSmem = kSgStages * kSgStage + 1024 + 128;
 
 struct SgArgs {
     const float* src; const float* W; float* part;
     uint32_t M, N, K, src_rs, part_rs, splits;       // N: weight rows
     const float* ctl; uint32_t slot_stride, rows_from;
 };
+__device__ __forceinline__ const float* sg_src(const SgArgs& a) { return a.src + (a.ctl && a.slot_stride ? (size_t)ctl_word(a.ctl, ZG_CTL_SLOT) * a.slot_stride : 0); }
+__device__ __forceinline__ float plain_sum(const float* x, const float* w, uint32_t K) {
+    float acc = 0.0f;
+#pragma unroll 1
+    for (uint32_t k = 0; k < K; k++) acc = fmaf(x[k], w[k], acc);
+    return acc;
+}
 
 __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
     extern __shared__ uint8_t dsm_raw[];
-    const uint32_t base = (smem_u32(dsm_raw) + 1023u) & ~1023u, bars = base + kSgStages * kSgStage + kSgScales;
+    const uint32_t base = (smem_u32(dsm_raw) + 1023u) & ~1023u, bars = base + kSgStages * kSgStage;
     const uint32_t full = bars, empty = full + 8 * kSgStages, d_full = empty + 8 * kSgStages, d_empty = d_full + 16, tmem_slot = d_empty + 16;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -55,7 +66,7 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
     const uint32_t n_steps = live ? s1 - s0 : 0;
 
     if (warp == 16) {
-        constexpr uint32_t idesc = (1u << 4) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24);       // f16 x f16 -> f32
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24);       // bf16 x bf16 -> f32
         const bool leader = elect_one();
         const uint32_t b0 = desc_low(base);
         bool ok = true;
@@ -65,14 +76,15 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
             if (ok && i >= 2) ok = mbar_wait(d_empty + 8 * (i & 1), ((i >> 1) - 1) & 1);
             fence_after();
             if (leader && ok) {
-                const uint32_t d = tmem + (i & 1) * kBN, ah = b0 + stage * (kSgStage >> 4), al = ah + (kTile >> 4), bh = al + (kTile >> 4), bl = bh + (kTile >> 4);
-                mma_ss<false>(d, ah, bl, idesc);
+                const uint32_t d = tmem + (i & 1) * kBN, x0 = b0 + stage * (kSgStage >> 4);
+                constexpr uint32_t kPart[6][2] = {{1, 1}, {0, 2}, {2, 0}, {0, 1}, {1, 0}, {0, 0}};       // parts of the source, of the weights
 #pragma unroll
-                for (uint32_t k = 1; k < 4; k++) mma_ss<true>(d, ah + 2 * k, bl + 2 * k, idesc);
+                for (uint32_t p = 0; p < 6; p++)
 #pragma unroll
-                for (uint32_t k = 0; k < 4; k++) mma_ss<true>(d, al + 2 * k, bh + 2 * k, idesc);
-#pragma unroll
-                for (uint32_t k = 0; k < 4; k++) mma_ss<true>(d, ah + 2 * k, bh + 2 * k, idesc);
+                    for (uint32_t k = 0; k < 4; k++) {
+                        const uint32_t x = x0 + kPart[p][0] * (kTile >> 4) + 2 * k, w = x0 + (3 + kPart[p][1]) * (kTile >> 4) + 2 * k;
+                        if (p == 0 && k == 0) mma_ss<false>(d, x, w, idesc); else mma_ss<true>(d, x, w, idesc);
+                    }
                 mma_commit(empty + 8 * stage);
                 mma_commit(d_full + 8 * (i & 1));
             }
@@ -83,8 +95,7 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
         // loading: lane group of 16 takes rows r + 32 i, columns 4 c .. + 3 of a step; draining: rows of the warp's quarter, 32 columns
         const uint32_t c = threadIdx.x & 15, r = threadIdx.x >> 4, quarter = warp & 3, part = warp >> 2;
         uint8_t* const ring = dsm_raw + (base - smem_u32(dsm_raw));
-        float* const scales = reinterpret_cast<float*>(ring + kSgStages * kSgStage);
-        const float* src = a.src + (a.ctl && a.slot_stride ? (size_t)ctl_word(a.ctl, ZG_CTL_SLOT) * a.slot_stride : 0);
+        const float* src = sg_src(a);
         float4 x[8];                                                 // four rows of the source, four of the weights
         auto load = [&](uint32_t step) {
             const uint32_t k = step * kBK + 4 * c;
@@ -108,44 +119,28 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(d_empty + 8 * (i & 1));
-            const float* sc = scales + (i & 3) * (kBM + kBN);
-            const float sa = sc[quarter * 32 + lane];
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-                const float4 sb = *reinterpret_cast<const float4*>(sc + kBM + 32 * part + j);
-                acc[j] = fmaf(__uint_as_float(v[j]) * sb.x, sa, acc[j]); acc[j + 1] = fmaf(__uint_as_float(v[j + 1]) * sb.y, sa, acc[j + 1]);
-                acc[j + 2] = fmaf(__uint_as_float(v[j + 2]) * sb.z, sa, acc[j + 2]); acc[j + 3] = fmaf(__uint_as_float(v[j + 3]) * sb.w, sa, acc[j + 3]);
+            for (int j = 0; j < 32; j += 2) {
+                const float2 r = __fadd2_rn(make_float2(acc[j], acc[j + 1]), make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])));
+                acc[j] = r.x; acc[j + 1] = r.y;
             }
         };
         if (n_steps) load(s0);
         uint32_t stage = 0, phase = 1;
         for (uint32_t i = 0; i < n_steps; i++) {
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * stage, phase));
-            float* const sc = scales + (i & 3) * (kBM + kBN);
             uint8_t* const to = ring + stage * kSgStage;
 #pragma unroll
-            for (int side = 0; side < 2; side++) {                   // the source's rows, the weights'
-                float mx[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) { const float4 y = x[4 * side + j]; mx[j] = abs_or_inf(abs_or_inf(abs_or_inf(abs_or_inf(0.0f, y.x), y.y), y.z), y.w); }
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) mx[j] = fmaxf(mx[j], __shfl_xor_sync(0xffffffffu, mx[j], o));
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float4 y = x[4 * side + j];
-                    const uint32_t row = r + 32 * j;
-                    float scale, inv;
-                    split_scale(mx[j], scale, inv);
-                    if (c == 0) sc[side * kBM + row] = inv;
-                    uint32_t h[2], l[2];
-                    split2(y.x * scale, y.y * scale, h[0], l[0]);
-                    split2(y.z * scale, y.w * scale, h[1], l[1]);
-                    uint8_t* const at = to + side * 2 * kTile + row * 128 + (((c >> 1) ^ (row & 7)) * 16 + (c & 1) * 8);
-                    *reinterpret_cast<uint2*>(at) = make_uint2(h[0], h[1]);
-                    *reinterpret_cast<uint2*>(at + kTile) = make_uint2(l[0], l[1]);
-                }
+            for (int j = 0; j < 8; j++) {                            // the source's rows, the weights'
+                const float4 y = x[j];
+                const uint32_t row = r + 32 * (j & 3);
+                uint2 p0, p1, p2;
+                split3(y.x, y.y, p0.x, p1.x, p2.x);
+                split3(y.z, y.w, p0.y, p1.y, p2.y);
+                uint8_t* const at = to + (j >> 2) * 3 * kTile + row * 128 + (((c >> 1) ^ (row & 7)) * 16 + (c & 1) * 8);
+                *reinterpret_cast<uint2*>(at) = p0;
+                *reinterpret_cast<uint2*>(at + kTile) = p1;
+                *reinterpret_cast<uint2*>(at + 2 * kTile) = p2;
             }
             if (i + 1 < n_steps) load(s0 + i + 1);                   // in flight while the step before is drained
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -190,14 +185,10 @@ __global__ void __launch_bounds__(256) k_split_finish(const SgArgs a, float* __r
         v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
     }
     float z[4] = {v.x, v.y, v.z, v.w};
-    const float* src = a.src + (a.ctl && a.slot_stride ? (size_t)ctl_word(a.ctl, ZG_CTL_SLOT) * a.slot_stride : 0) + (size_t)m * a.src_rs;
+    const float* src = sg_src(a) + (size_t)m * a.src_rs;
 #pragma unroll
     for (int j = 0; j < 4; j++)
-        if (!(z[j] == z[j]) && n + j < a.N) {                        // not a number: as a plain f32 sum
-            float acc = 0.0f;
-            for (uint32_t k = 0; k < a.K; k++) acc = fmaf(src[k], a.W[(size_t)(n + j) * a.K + k], acc);
-            z[j] = acc;
-        }
+        if (!(fabsf(z[j]) <= 3.4028234e38f) && n + j < a.N) z[j] = plain_sum(src, a.W + (size_t)(n + j) * a.K, a.K);      // not finite
     float* out = dst + (size_t)m * dst_rs;
     if (pairs) {
 #pragma unroll
@@ -222,10 +213,6 @@ uint32_t shares(uint32_t M, uint32_t N, uint32_t K, uint32_t n_sm) {
     }
     return best;
 }
-uint32_t sm_count() {
-    static const uint32_t n = [] { int dev = 0, v = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); return (uint32_t)(v > 0 ? v : 148); }();
-    return n;
-}
 uint32_t up4(uint32_t n) { return (n + 3) / 4 * 4; }
 
 }  // namespace
@@ -234,12 +221,12 @@ uint32_t up4(uint32_t n) { return (n + 3) / 4 * 4; }
 bool zg_split_gemm_usable(const float* w, const float* src, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t slot_stride) {
     return M > 8 && N >= 32 && K >= 64 && K % 4 == 0 && src_rs % 4 == 0 && slot_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
 }
-size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K) { return (size_t)shares(M, N, K, sm_count()) * M * up4(N); }
+size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K) { return (size_t)shares(M, N, K, zg_sm_count()) * M * up4(N); }
+unsigned int zg_split_gemm_timeouts() { return tc_timeouts(); }
 bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, cudaStream_t st,
                           uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from) {
-    static const cudaError_t set = cudaFuncSetAttribute(k_split_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSgSmem);
-    if (set != cudaSuccess) { zg_set_error("cudaFuncSetAttribute(split gemm) failed: %s", cudaGetErrorString(set)); return false; }
-    const SgArgs a = {src, w, scratch, M, N, K, src_rs, up4(N), shares(M, N, K, sm_count()), ctl, slot_stride, rows_from};
+    if (!zg_smem_limit<k_split_gemm>(kSgSmem)) return false;
+    const SgArgs a = {src, w, scratch, M, N, K, src_rs, up4(N), shares(M, N, K, zg_sm_count()), ctl, slot_stride, rows_from};
     launch_pdl(k_split_gemm, dim3((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, a.splits), dim3(kSgThreads), kSgSmem, st, a);
     ZG_COUNT_LAUNCH();
     launch_pdl(k_split_finish, dim3((N + 1023) / 1024, M), dim3(256), 0, st, a, dst, dst_rs, bias, SeqAct{act, act_p, act_lo, act_hi}, (uint32_t)pairs);

@@ -1,8 +1,8 @@
-// What the kernels that split f32 operands into half-precision pairs for tcgen05 share: barriers, TMA, descriptors, MMA issue, TMEM access, and
-// the split itself.
+// What the kernels that split f32 operands into 16-bit parts for tcgen05 share: barriers, TMA, descriptors, MMA issue, TMEM access, and the splits.
 //
-// x = hi + lo: hi = f16(x s), lo = f16(x s - hi), with s a power of two that brings the largest magnitude of a row or tile to [2^14, 2^15).  hi and lo
-// together keep 22 to 24 significant bits of everything within 2^-17 of that maximum; what is smaller loses bits below 2^-39 of it.
+// Pairs of half precision: x = hi + lo: hi = f16(x s), lo = f16(x s - hi), with s a power of two that brings the largest magnitude of a row or tile to
+// [2^14, 2^15).  hi and lo together keep 22 to 24 significant bits of everything within 2^-17 of that maximum; what is smaller loses bits below 2^-39 of it.
+// Three parts of bfloat16: x = b0 + b1 + b2, all 24 bits of every x by itself.
 #pragma once
 #include "seq_common.cuh"
 
@@ -12,7 +12,12 @@
 namespace {
 
 constexpr uint32_t kTcSpin = 1u << 22;       // polls after which a wait gives up
-
+__device__ unsigned int g_tc_timeouts = 0;    // threads of this file's kernels whose wait gave up
+[[maybe_unused]] unsigned int tc_timeouts() {
+    unsigned int v = 0;
+    cudaMemcpyFromSymbol(&v, g_tc_timeouts, sizeof(v));
+    return v;
+}
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
@@ -25,6 +30,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
         if (ok) return true;
     }
+    atomicAdd(&g_tc_timeouts, 1u);
     return false;
 }
 __device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap* map, uint32_t c0, uint32_t c1, uint32_t bar) {
@@ -107,6 +113,17 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
     const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// two values -> their three bfloat16 parts, packed
+__device__ __forceinline__ void split3(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    uint32_t* const to[3] = {&p0, &p1, &p2};
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+        const float2 f = __bfloat1622float2(h);
+        a -= f.x; b -= f.y;
+        *to[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
 }
 __device__ __forceinline__ float abs_or_inf(float m, float x) { const float a = fabsf(x); return a <= 3.4028234e38f ? fmaxf(m, a) : INFINITY; }   // NaN counts as infinite
 

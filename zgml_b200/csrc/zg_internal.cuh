@@ -18,6 +18,20 @@ extern std::atomic<uint64_t> g_zg_launches;
 extern std::atomic<uint64_t> g_zg_stream_launches;
 #define ZG_COUNT_LAUNCH() (g_zg_launches.fetch_add(1, std::memory_order_relaxed))
 
+uint32_t zg_sm_count();   // of the device that was current at the first call
+// Dynamic shared memory beyond the default, once per kernel and device.
+template <auto KERNEL>
+inline bool zg_smem_limit(size_t bytes) {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64 && (done.load() >> dev & 1)) return true;
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) { zg_set_error("cudaFuncSetAttribute(%zu bytes of shared memory) failed: %s", bytes, cudaGetErrorString(e)); return false; }
+    if (dev < 64) done.fetch_or(1ull << dev);
+    return true;
+}
+
 #define ZG_CUDA_OK(expr)                                                                     \
     do {                                                                                     \
         cudaError_t _e = (expr);                                                             \
@@ -387,9 +401,10 @@ struct ZgExpertSegment { int expert, start, rows; };          // rows start .. s
 constexpr uint32_t kExpertSegmentRows = 256;
 bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void* xb, uint32_t rows, const ZgExpertSegment* d_segments, uint32_t segments, void* out, uint32_t N, uint32_t K,
                            float limit, float alpha, float up_offset, cudaStream_t st);
-// split_gemm.cu : f32 x f32 -> f32 LINEAR of many rows, operands split into half-precision pairs (arguments as zg_dense_gemm_launch's; N counts weight rows)
+// split_gemm.cu : f32 x f32 -> f32 LINEAR of many rows, operands cut into three bfloat16 parts (arguments as zg_dense_gemm_launch's; N counts weight rows)
 bool zg_split_gemm_usable(const float* w, const float* src, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t slot_stride);
 size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K);
+unsigned int zg_split_gemm_timeouts();
 bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, cudaStream_t st,
                           uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from);
 // mixops.cu : ZG_OP_TOKEN_SHIFT .. ZG_OP_POLY_NORM, reached through the functions above
