@@ -1,6 +1,6 @@
 """LINEAR of many rows over f32 weights (operands cut into three bfloat16 parts on the tensor cores) against float64: edges of the 128 x 128 tiles and of
 the 64-k steps, one and several shares of K, strided rows, bias, activation on part of the columns, gated pairs, magnitudes that differ between rows and
-within a row, sums near the largest float, and rows that hold an infinity or a NaN.
+within a row, sums near the largest float, more rows than a grid has in y, and rows that hold an infinity or a NaN.
 
 Tolerance: three parts hold every operand whole, the products left out are below 2^-25 of one product, a 64-k step adds four truncated f32 sums and up to
 100 steps add in f32: 3e-6 of sqrt(K) |x| |w| is over three times what that makes; the plain f32 sum shows about 1e-6."""
@@ -117,6 +117,13 @@ def test_finite_sums_of_extreme_operands(cuda_backend, big, small, where):
     want = x.astype(np.float64) @ W.astype(np.float64).T
     assert np.abs(want).max() < 1e37
     check(linear(cuda_backend, x, W), x, W, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(65535 + 129, 32, 64), (70000, 40, 256)])
+def test_more_rows_than_a_grid_has_in_y(cuda_backend, M, N, K):
+    r = np.random.default_rng(8)
+    x, W = r.standard_normal((M, K)).astype(np.float32), r.standard_normal((N, K)).astype(np.float32)
+    check(linear(cuda_backend, x, W), x, W, x.astype(np.float64) @ W.astype(np.float64).T)
 
 
 def test_no_wait_ran_out(cuda_backend):

@@ -14,10 +14,11 @@
 //     swizzled K-major tiles into a 2-stage ring; the same warps drain the accumulators of the step before (two TMEM buffers), each a quarter of the
 //     columns of its 32 rows.  Warp 16 issues the MMAs.
 //   * Per step the MMAs take 1536 clocks, their operand reads and the workers' stores 2300 clocks of shared-memory bandwidth; the f32 rows of the next step
-//     are in flight for one step only, and their latency bounds the kernel.
-//   * Tiles leave as partial sums; k_split_finish adds the shares in order and applies bias and activation.  A sum that is not finite is evaluated again
-//     there as a plain f32 sum: what an infinity makes of a sum is the plain kernel's.
-//   * Every wait is bounded; a CTA whose wait ran out counts it and writes NaN, so that its outputs are evaluated again the plain way.
+//     are in flight for one step only, and their latency bounds the kernel (256 tokens through gate, up and down of 2048 / 4096:
+//     166 us; as pairs with partial sums in scratch 169, as the f32 tile 1034).
+//   * One share of K: the tile is finished here (bias, activation) and leaves by whole rows.  Several: partial sums go to scratch and k_split_finish adds them in
+//     order.  A sum that is not finite is evaluated again as a plain f32 sum: what an infinity makes of a sum is the plain kernel's.
+//   * Every wait is bounded; a CTA whose wait ran out counts it and treats its sums as not finite, so that they are evaluated again the plain way.
 #include "split_tc.cuh"
 
 namespace {
@@ -30,6 +31,7 @@ struct SgArgs {
     const float* src; const float* W; float* part;
     uint32_t M, N, K, src_rs, part_rs, splits;       // N: weight rows
     const float* ctl; uint32_t slot_stride, rows_from;
+    float* dst; const float* bias; uint32_t dst_rs, pairs; SeqAct act;
 };
 __device__ __forceinline__ const float* sg_src(const SgArgs& a) { return a.src + (a.ctl && a.slot_stride ? (size_t)ctl_word(a.ctl, ZG_CTL_SLOT) * a.slot_stride : 0); }
 __device__ __forceinline__ float plain_sum(const float* x, const float* w, uint32_t K) {
@@ -37,6 +39,25 @@ __device__ __forceinline__ float plain_sum(const float* x, const float* w, uint3
 #pragma unroll 1
     for (uint32_t k = 0; k < K; k++) acc = fmaf(x[k], w[k], acc);
     return acc;
+}
+// sums of four weight rows n .. n + 3 of source row m -> bias, activation, dst (pairs: two outputs)
+__device__ __forceinline__ void sg_finish(const SgArgs& a, uint32_t m, uint32_t n, float4 v) {
+    float z[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (!(fabsf(z[j]) <= 3.4028234e38f) && n + j < a.N) z[j] = plain_sum(sg_src(a) + (size_t)m * a.src_rs, a.W + (size_t)(n + j) * a.K, a.K);
+    float* out = a.dst + (size_t)m * a.dst_rs;
+    if (a.pairs) {
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) if (n + j + 1 < a.N) out[(n + j) / 2] = seq_epilogue(z[j], a.act.kind, a.act.p) * z[j + 1];
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (n + j < a.N) z[j] = seq_epilogue(z[j] + (a.bias ? a.bias[n + j] : 0.0f), a.act, n + j);
+    if (n + 4 <= a.N && (reinterpret_cast<uintptr_t>(out + n) & 15) == 0) *reinterpret_cast<float4*>(out + n) = make_float4(z[0], z[1], z[2], z[3]);
+    else
+        for (int j = 0; j < 4; j++) if (n + j < a.N) out[n + j] = z[j];
 }
 
 __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
@@ -163,7 +184,10 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
         float* const p = a.part + (size_t)blockIdx.z * a.M * a.part_rs;
         for (uint32_t i = threadIdx.x; live && i < kBM * 32; i += kSgWorkers) {
             const uint32_t rr = i >> 5, j = i & 31, m = m0 + rr, n = n0 + 4 * j;
-            if (m < a.M && n < a.part_rs) *reinterpret_cast<float4*>(p + (size_t)m * a.part_rs + n) = out[rr * 32 + (j ^ (rr & 7))];
+            if (m >= a.M || n >= a.N) continue;
+            const float4 v = out[rr * 32 + (j ^ (rr & 7))];
+            if (a.splits == 1) sg_finish(a, m, n, v);
+            else *reinterpret_cast<float4*>(p + (size_t)m * a.part_rs + n) = v;
         }
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -173,42 +197,31 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
     if (warp == 16) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
 }
 
-// the shares' sums, bias, activation; four weight rows (pairs: two outputs) per thread
-__global__ void __launch_bounds__(256) k_split_finish(const SgArgs a, float* __restrict__ dst, uint32_t dst_rs, const float* __restrict__ bias, SeqAct act, uint32_t pairs) {
+// the shares' sums, bias, activation; four weight rows per thread
+__global__ void __launch_bounds__(256) k_split_finish(const SgArgs a) {
     pdl_enter();
-    const uint32_t n = 4 * (blockIdx.x * 256 + threadIdx.x), m = blockIdx.y;
+    const uint32_t n = 4 * (blockIdx.x * 256 + threadIdx.x);
     if (n >= a.N) return;
-    if (a.rows_from && m / kBM * kBM >= (uint32_t)ctl_word(a.ctl, ZG_CTL_POS) + a.rows_from) return;
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (uint32_t s = 0; s < a.splits; s++) {
-        const float4 p = *reinterpret_cast<const float4*>(a.part + ((size_t)s * a.M + m) * a.part_rs + n);
-        v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+    for (uint32_t m = blockIdx.y; m < a.M; m += gridDim.y) {
+        if (a.rows_from && m / kBM * kBM >= (uint32_t)ctl_word(a.ctl, ZG_CTL_POS) + a.rows_from) return;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (uint32_t s = 0; s < a.splits; s++) {
+            const float4 p = *reinterpret_cast<const float4*>(a.part + ((size_t)s * a.M + m) * a.part_rs + n);
+            v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+        }
+        sg_finish(a, m, n, v);
     }
-    float z[4] = {v.x, v.y, v.z, v.w};
-    const float* src = sg_src(a) + (size_t)m * a.src_rs;
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-        if (!(fabsf(z[j]) <= 3.4028234e38f) && n + j < a.N) z[j] = plain_sum(src, a.W + (size_t)(n + j) * a.K, a.K);      // not finite
-    float* out = dst + (size_t)m * dst_rs;
-    if (pairs) {
-#pragma unroll
-        for (int j = 0; j < 4; j += 2) if (n + j + 1 < a.N) out[(n + j) / 2] = seq_epilogue(z[j], act.kind, act.p) * z[j + 1];
-        return;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-        if (n + j < a.N) z[j] = seq_epilogue(z[j] + (bias ? bias[n + j] : 0.0f), act, n + j);
-    if (n + 4 <= a.N && (reinterpret_cast<uintptr_t>(out + n) & 15) == 0) *reinterpret_cast<float4*>(out + n) = make_float4(z[0], z[1], z[2], z[3]);
-    else
-        for (int j = 0; j < 4; j++) if (n + j < a.N) out[n + j] = z[j];
 }
 
-// shares of K: the fewest rounds of CTAs times steps per CTA, a step of overhead for each round's start and end
+// shares of K: the fewest rounds of CTAs times steps per CTA, a step of overhead for each round's start and end.  Several shares only where they make
+// no more than four CTAs per SM, so that their partial sums stay within some 40 MB whatever the shape.
 uint32_t shares(uint32_t M, uint32_t N, uint32_t K, uint32_t n_sm) {
-    const uint32_t tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN), steps = (K + kBK - 1) / kBK;
-    uint32_t best = 1, best_cost = ~0u;
-    for (uint32_t s = 1; s <= 16 && s <= (steps + 3) / 4; s++) {
-        const uint32_t cost = ((tiles * s + n_sm - 1) / n_sm) * ((steps + s - 1) / s + 4) + s / 2;
+    const uint64_t tiles = (uint64_t)((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN);
+    const uint32_t steps = (K + kBK - 1) / kBK;
+    uint32_t best = 1;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t s = 1; s <= 16 && s <= (steps + 3) / 4 && (s == 1 || (uint64_t)tiles * s <= 4ull * n_sm); s++) {
+        const uint64_t cost = ((tiles * s + n_sm - 1) / n_sm) * ((steps + s - 1) / s + 4) + s / 2;
         if (cost < best_cost) { best_cost = cost; best = s; }
     }
     return best;
@@ -221,17 +234,22 @@ uint32_t up4(uint32_t n) { return (n + 3) / 4 * 4; }
 bool zg_split_gemm_usable(const float* w, const float* src, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t slot_stride) {
     return M > 8 && N >= 32 && K >= 64 && K % 4 == 0 && src_rs % 4 == 0 && slot_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
 }
-size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K) { return (size_t)shares(M, N, K, zg_sm_count()) * M * up4(N); }
+size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K) {      // never 0, which stands for the plain kernel
+    const uint32_t s = shares(M, N, K, zg_sm_count());
+    return s > 1 ? (size_t)s * M * up4(N) : 4;
+}
 unsigned int zg_split_gemm_timeouts() { return tc_timeouts(); }
 bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, cudaStream_t st,
                           uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from) {
     if (!zg_smem_limit<k_split_gemm>(kSgSmem)) return false;
-    const SgArgs a = {src, w, scratch, M, N, K, src_rs, up4(N), shares(M, N, K, zg_sm_count()), ctl, slot_stride, rows_from};
+    const SgArgs a = {src, w, scratch, M, N, K, src_rs, up4(N), shares(M, N, K, zg_sm_count()), ctl, slot_stride, rows_from, dst, bias, dst_rs, (uint32_t)pairs, SeqAct{act, act_p, act_lo, act_hi}};
     launch_pdl(k_split_gemm, dim3((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, a.splits), dim3(kSgThreads), kSgSmem, st, a);
     ZG_COUNT_LAUNCH();
-    launch_pdl(k_split_finish, dim3((N + 1023) / 1024, M), dim3(256), 0, st, a, dst, dst_rs, bias, SeqAct{act, act_p, act_lo, act_hi}, (uint32_t)pairs);
+    if (a.splits > 1) {
+        launch_pdl(k_split_finish, dim3((N + 1023) / 1024, M < 65535 ? M : 65535), dim3(256), 0, st, a);
+        ZG_COUNT_LAUNCH();
+    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { zg_set_error("split gemm launch failed: %s", cudaGetErrorString(e)); return false; }
-    ZG_COUNT_LAUNCH();
     return true;
 }
