@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from test_gpu_recops import ctl_words, run
+from test_gpu_split_gemm import waits_given_up
 
 pytestmark = pytest.mark.gpu
 
@@ -131,3 +132,8 @@ def test_batched_heads_with_their_own_masks_and_a_refreshed_length(cuda_backend)
             want = e @ v[h % 2, :n].astype(np.float64) / np.maximum(e.sum(1, keepdims=True), 1e-300)
             assert close(got[h], want), (n, h)
     cuda_backend.free_program(handle)
+
+
+def test_no_wait_ran_out(cuda_backend):
+    """After everything above: a wait that gives up is counted (and its rows are no numbers)."""
+    assert waits_given_up(cuda_backend) == 0

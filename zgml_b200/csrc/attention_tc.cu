@@ -18,7 +18,7 @@
 //     scores of tile i + 1 before values of tile i, so the softmax of one tile runs beside the products of its neighbours.
 //   * Measured per 128 x 128 tile of 128 dims (its 48 MMAs execute in 3072 clocks): 9400 clocks with one thread per query row and the MMAs issued
 //     inside a single lane's branch, 9100 with four threads per row, 4700 once the whole MMA warp walks the tiles (below).
-//   * Every wait is bounded; a CTA whose wait ran out stops issuing, leaves its rows and frees its TMEM.
+//   * Every wait is bounded; a CTA whose wait ran out counts it (zg_attention_tc_timeouts), stops issuing, makes NaN of its rows and frees its TMEM.
 //
 // Non-finite inputs: a key or value tile that holds one is marked by a NaN scale; the rows of a CTA that met such a tile are evaluated one
 // by one in plain f32 (atc_slow_row), as the SIMT kernels would.
@@ -36,6 +36,7 @@ constexpr uint32_t kAtcThreads = 576, kAtcRing = 12, kAtcPiece = 16384;
 constexpr uint32_t kAtcShare = 2 * 4 * 128 * 4;                   // row maxima of the four quarters, two tiles
 constexpr uint32_t kAtcTiles = 512;                               // key tiles whose class and scales a CTA keeps at hand
 constexpr uint32_t kAtcSmem = kAtcRing * kAtcPiece + kAtcShare + kAtcTiles * 12 + 1024 + 256;
+constexpr float kNotANumber = __builtin_nanf("");
 constexpr size_t kAtcProgramKeys = 1u << 20;                      // the most keys that a DeviceOp.attention batch lays out planes for
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr float kPScale = 16384.0f, kPInv = 1.0f / 16384.0f;      // probabilities are held times 2^14
@@ -443,6 +444,8 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tmem_slot) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    uint32_t* const trouble = reinterpret_cast<uint32_t*>(dsm_raw + (tmem_slot + 4 - smem_u32(dsm_raw)));      // a wait of the CTA ran out
+    if (threadIdx.x == 0) *trouble = 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const typename Src::Cta c = src.cta(BK);
     // class and scales of the first tiles: read from global memory inside the loop they cost every tile an L2 round trip
@@ -693,14 +696,16 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
 #pragma unroll 1
             for (int j = 0; j < OW; j += 4) ring[place(j)] = make_float4(acc[j] * f, acc[j + 1] * f, acc[j + 2] * f, acc[j + 3] * f);
         } else {
-            const float f = w.on && ok ? src.finish(c, w, part == 0, m, true, l, kPInv) : 0.0f;
+            const float f = w.on ? src.finish(c, w, part == 0, m, true, l, kPInv) : 0.0f;
 #pragma unroll
             for (int j = 0; j < OW; j += 4) ring[place(j)] = make_float4(o[j] * f, o[j + 1] * f, o[j + 2] * f, o[j + 3] * f);
         }
+        if (!ok) { *trouble = 1; if (lane == 0) count_timeout(); }
         bar_sync(5, 512);
-        for (uint32_t i = threadIdx.x; ok && i < c.nq * (DV / 4); i += 512) {
+        const bool lost = *trouble != 0;                             // (what still arrives in the ring is not looked at)
+        for (uint32_t i = threadIdx.x; i < c.nq * (DV / 4); i += 512) {
             const uint32_t r = i / (DV / 4), j = i % (DV / 4);
-            src.put(c, src.query(c, r), 4 * j, ring[r * (DV / 4) + (j ^ (r & 7))]);
+            src.put(c, src.query(c, r), 4 * j, lost ? make_float4(kNotANumber, kNotANumber, kNotANumber, kNotANumber) : ring[r * (DV / 4) + (j ^ (r & 7))]);
         }
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -754,8 +759,7 @@ bool launch(const Src& src, const AtcPlanes& pl, dim3 grid, cudaStream_t st) {
     constexpr int C = NC > DV / 64 ? NC : DV / 64;
     CUtensorMap mk, mv;
     if (!encode_plane(&mk, pl.k, 2 * pl.dkp, (uint64_t)pl.k_items * pl.tiles * 128, BK) || !encode_plane(&mv, pl.v, (uint64_t)2 * pl.tiles * 128, (uint64_t)pl.v_items * pl.vslice, DV)) return false;
-    static const cudaError_t set = cudaFuncSetAttribute(k_attention_tc<Src, NC, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAtcSmem);
-    if (set != cudaSuccess) { zg_set_error("cudaFuncSetAttribute(attention) failed: %s", cudaGetErrorString(set)); return false; }
+    if (!zg_smem_limit<k_attention_tc<Src, NC, DV>>(kAtcSmem)) return false;
     launch_pdl(k_atc_prep<Src, C>, dim3(pl.tiles, pl.k_items + pl.v_items), dim3(kPrepThreads), 0, st, src, pl);
     ZG_COUNT_LAUNCH();
     launch_pdl(k_attention_tc<Src, NC, DV>, grid, dim3(kAtcThreads), kAtcSmem, st, mk, mv, src, pl);
@@ -867,3 +871,4 @@ bool zg_atc_program_launch(const ZgAtcPlan& p, const ZgBatchEntry* d_entries, co
     const dim3 grid(row_tiles * p.count);
     return p.head == 64 ? launch<AtcProgram, 1, 64>(src, pl, grid, st) : launch<AtcProgram, 2, 128>(src, pl, grid, st);
 }
+unsigned int zg_attention_tc_timeouts() { return tc_timeouts(); }

@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
             if (i) drain(i - 1);
         }
         if (n_steps) drain(n_steps - 1);
+        if (!ok && lane == 0) count_timeout();
         // out by whole rows, through the idle ring (every MMA that reads it is done)
         float4* const out = reinterpret_cast<float4*>(ring);
         const uint32_t row = quarter * 32 + lane;
