@@ -87,6 +87,44 @@ def test_many_rows(cuda_backend, shape):
     assert close(got, want)
 
 
+def direct(be, q, k, v, pos, H, G, d):
+    """Causal CACHED_ATTENTION of rows q [T, H d] over the cache rows k, v [pos + T, G d]."""
+    from zgml_b200 import DeviceBuffer, DeviceOp, ExternBuffer
+    T = len(q)
+    q, k, v = (np.ascontiguousarray(a, np.float32) for a in (q, k, v))
+    bk, bv = DeviceBuffer(be, k.nbytes, zero=False), DeviceBuffer(be, v.nbytes, zero=False)
+    bk.upload(k)
+    bv.upload(v)
+    op = DeviceOp.cached_attention(0, 1, 2, 3, 4, 0, 0, 0, T, H, G, 1, d, d, H * d, G * d, G * d, pos + T, d ** -0.5, mask="causal")
+    got = run(be, [op], [T * H * d, q.size, bk.elems, bv.elems, 8 + T], [(1, q), (4, ctl_words(pos, 0))], 0, (T, H, d), [ExternBuffer(2, bk), ExternBuffer(3, bv)])
+    bk.free()
+    bv.free()
+    seen = np.arange(pos + T) <= np.arange(pos, pos + T)[:, None]
+    part = lambda a, i: a[:, i * d:(i + 1) * d].astype(np.float64)
+    return got, np.stack([reference(part(q, h), part(k, h * G // H), part(v, h * G // H), seen, d ** -0.5) for h in range(H)], 1)
+
+
+@pytest.mark.parametrize("what", ["key", "value", "column", "dims"])
+def test_magnitudes_far_apart_within_a_tile(cuda_backend, what):
+    """A large key or value that only the last rows see, a value column far below the others, and queries and keys whose large dims meet zeros: what is small keeps
+    its bits, column by column."""
+    r = np.random.default_rng(12)
+    T, pos, H, G, d = 200, 120, 8, 4, 128
+    k, v, q = r.standard_normal((pos + T, G * d)), r.standard_normal((pos + T, G * d)), r.standard_normal((T, H * d))
+    if what == "key":
+        k[300] *= 2.0 ** 24
+    elif what == "value":
+        v[300] *= 2.0 ** 24
+    elif what == "column":
+        v[:, 5::d] *= 2.0 ** -24
+    else:
+        k[:, 0::d], k[:, 1::d], q[:, 0::d], q[:, 1::d] = 2.0 ** 22, 0.0, 0.0, 2.0 ** 22
+    got, want = direct(cuda_backend, q, k, v, pos, H, G, d)
+    rows = slice(0, 300 - pos)                                         # those that do not see position 300
+    assert (np.abs(got - want)[rows].max((0, 1)) <= 1e-5 * np.abs(want)[rows].max((0, 1))).all()
+    assert np.isfinite(got).all()
+
+
 @pytest.mark.parametrize("what", ["nan key", "nan value", "infinite value"])
 def test_rows_that_see_nothing_non_finite_are_exact(cuda_backend, what):
     """Position 150 of every key head or value head is poisoned: the queries before it are as they were, and those that see it are not finite."""
@@ -132,6 +170,33 @@ def test_batched_heads_with_their_own_masks_and_a_refreshed_length(cuda_backend)
             want = e @ v[h % 2, :n].astype(np.float64) / np.maximum(e.sum(1, keepdims=True), 1e-300)
             assert close(got[h], want), (n, h)
     cuda_backend.free_program(handle)
+
+
+@pytest.mark.parametrize("what", ["nan key", "nan value", "infinite value"])
+def test_batched_rows_that_see_nothing_non_finite_are_exact(cuda_backend, what):
+    """DeviceOp.attention: position 70 of the first of two key / value slabs holds no number; the rows whose mask leaves it out, and the heads of the other
+    slab, are as they were."""
+    from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO
+    r = np.random.default_rng(9)
+    T, S, dh, H = 150, 200, 64, 4
+    q, k, v = r.standard_normal((H, T, dh)).astype(np.float32), r.standard_normal((2, S, dh)).astype(np.float32), r.standard_normal((2, S, dh)).astype(np.float32)
+    (k if what == "nan key" else v)[0, 70] = np.inf if what == "infinite value" else np.nan
+    mask = np.where(r.random((T, S)) < 0.5, -np.inf, 0.0).astype(np.float32)
+    ops = [DeviceOp.attention(4, 0, 1, 2, 3, True, dh, T, S, 0.3, h * T * dh, h % 2 * S * dh, h % 2 * S * dh, 0, h * T * dh, 1, dh, 1, dh, 1, dh, 1, S, 1, dh) for h in range(H)]
+    handle = cuda_backend.compile_program(DeviceProgram(ops, [q.size, k.size, v.size, mask.size, q.size], [], []))
+    got = np.zeros((H, T, dh), np.float32)
+    cuda_backend.execute_program(handle, [ProgramIO(i, a.ravel()) for i, a in enumerate((q, k, v, mask))], [ProgramIO(4, got)])
+    cuda_backend.free_program(handle)
+    sees = mask[:, 70] == 0.0
+    for h in range(H):
+        rows = ~sees if h % 2 == 0 else np.ones(T, bool)
+        kk, vv = np.where(np.isfinite(k[h % 2]), k[h % 2], 0.0).astype(np.float64), np.where(np.isfinite(v[h % 2]), v[h % 2], 0.0).astype(np.float64)
+        s = q[h].astype(np.float64) @ kk.T * 0.3 + mask
+        e = np.exp(s - s.max(1, keepdims=True))
+        want = e @ vv / e.sum(1, keepdims=True)
+        assert close(got[h][rows], want[rows])
+        # a NaN score counts as masked there, a value that is no number does not
+        assert what == "nan key" or h % 2 or not np.isfinite(got[h][sees]).any()
 
 
 def test_no_wait_ran_out(cuda_backend):

@@ -20,8 +20,9 @@
 //     inside a single lane's branch, 9100 with four threads per row, 4700 once the whole MMA warp walks the tiles (below).
 //   * Every wait is bounded; a CTA whose wait ran out counts it (zg_attention_tc_timeouts), stops issuing, makes NaN of its rows and frees its TMEM.
 //
-// Non-finite inputs: a key or value tile that holds one is marked by a NaN scale; the rows of a CTA that met such a tile are evaluated one
-// by one in plain f32 (atc_slow_row), as the SIMT kernels would.
+// What pairs cannot hold is evaluated in plain f32 (atc_plain: the CTA's 512 softmax threads over f32 tiles, as the SIMT kernels do it; 1.3 times their
+// time): all rows of a CTA that met a key or value tile, or a query row, that holds something non-finite or whose magnitudes lie too far apart for one
+// scale (is_small).  Such a tile is marked by a NaN scale.
 #include "attention_tc.cuh"
 #include "split_tc.cuh"
 
@@ -42,6 +43,11 @@ constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr float kPScale = 16384.0f, kPInv = 1.0f / 16384.0f;      // probabilities are held times 2^14
 
 __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+// A scaled element that is not zero but below 2^-18 of the largest magnitude its scale is made for (which is brought to [2^14, 2^15)).  A pair keeps it to
+// 2^-40 of that magnitude, fewer than 22 bits of its own: where that many are small, it is their own size that counts (values of a column that is small
+// as a whole, a key beside one that no row sees), not what they add to the large ones.  Normally distributed tiles of 128 x 128 have 0.1 to 0.3 of them.
+constexpr uint32_t kAtcSmallTile = 24, kAtcSmallQuery = 3;          // of 128 keys or values, of a quarter row
+__device__ __forceinline__ uint32_t is_small(float x, float scale) { const float a = fabsf(x * scale); return a < 0.0625f && a > 0.0f ? 1u : 0u; }
 // ── where keys, values and queries come from ─────────────────────────────────────────────────────────────────────
 // A SOURCE names the keys of a step (for k_atc_prep) and, for the attention kernel, a CTA's items and range of key tiles, the class of a tile
 // (0: no row sees it, 1: every row sees all of it, 2: some), a row's query and what becomes of its scores.  Keys are counted from the first one
@@ -87,6 +93,7 @@ struct AtcCached {
         c.t0 = min(end, first + c.split * per); c.t1 = min(end, c.t0 + per);
         return c;
     }
+    __device__ __forceinline__ uint32_t plain_end(const Cta& c, uint32_t bk) const { return c.t1 * bk; }
     __device__ __forceinline__ uint32_t k_item(const Cta& c) const { return c.gm; }
     __device__ __forceinline__ uint32_t v_item(const Cta& c) const { return c.g * n_vs + c.vs; }
     __device__ __forceinline__ uint32_t classify(const Cta& c, uint32_t t, uint32_t bk) const {
@@ -202,6 +209,7 @@ struct AtcProgram {
         c.t0 = 0; c.t1 = (c.n_keys + bk - 1) / bk;
         return c;
     }
+    __device__ __forceinline__ uint32_t plain_end(const Cta& c, uint32_t) const { return c.n_keys; }
     __device__ __forceinline__ uint32_t k_item(const Cta& c) const { return c.kv; }
     __device__ __forceinline__ uint32_t v_item(const Cta& c) const { return c.kv; }
     __device__ __forceinline__ uint32_t classify(const Cta& c, uint32_t t, uint32_t bk) const {
@@ -291,9 +299,10 @@ struct AtcPlanes {
 // 4 heads of 128, cold.)
 constexpr uint32_t kPrepThreads = 512;
 template <class Src, int C>
-__global__ void __launch_bounds__(kPrepThreads) k_atc_prep(const Src src, const AtcPlanes pl) {
+__global__ void __launch_bounds__(kPrepThreads, C == 1 ? 3 : C == 2 ? 2 : 1) k_atc_prep(const Src src, const AtcPlanes pl) {
     pdl_enter();
     __shared__ float red[kPrepThreads / 32];
+    __shared__ uint32_t n_small[kPrepThreads / 32];
     __shared__ uint32_t t_hi[64][65], t_lo[64][65];      // a 64-column chunk of 128 values, transposed: pairs of keys per word
     const bool value = blockIdx.y >= pl.k_items;
     const uint32_t item = value ? blockIdx.y - pl.k_items : blockIdx.y, head = value ? item / pl.n_vs : item, u0 = blockIdx.x * 128, n_keys = src.prep_keys(head);
@@ -319,7 +328,20 @@ __global__ void __launch_bounds__(kPrepThreads) k_atc_prep(const Src src, const 
     mx = warp_max(red[tid & 15]);
     float scale, inv;
     split_scale(mx, scale, inv);
-    if (tid == 0) (value ? pl.v_inv : pl.k_inv)[(size_t)item * pl.tiles + blockIdx.x] = inv;
+    uint32_t small = 0;
+#pragma unroll
+    for (int c = 0; c < C; c++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) small += is_small(x[c][k].x, scale) + is_small(x[c][k].y, scale) + is_small(x[c][k].z, scale) + is_small(x[c][k].w, scale);
+    small = __reduce_add_sync(0xffffffffu, small);
+    if ((tid & 31) == 0) n_small[tid >> 5] = small;
+    __syncthreads();
+    if (tid == 0) {
+        small = 0;
+        for (uint32_t i = 0; i < kPrepThreads / 32; i++) small += n_small[i];
+        if (small >= min(kAtcSmallTile, max(4u, min(128u, n_keys - u0)))) inv = __uint_as_float(0x7fffffffu);
+        (value ? pl.v_inv : pl.k_inv)[(size_t)item * pl.tiles + blockIdx.x] = inv;
+    }
 #pragma unroll
     for (int c = 0; c < C; c++) {
         if (64 * c >= padded) break;
@@ -391,36 +413,119 @@ __global__ void __launch_bounds__(512) k_atc_masks(const AtcProgram src) {
     if (threadIdx.x == 0) src.classes[tile] = !a ? 0 : !z ? 3 : f ? 1 : 2;
 }
 
-// One row in plain f32 over the keys of the CTA's tiles: output columns col .. col + N - 1, and the factor they are to be multiplied by.
-template <int N, class Src>
-__device__ __noinline__ float atc_slow_row(const Src& src, const typename Src::Cta& c, const typename Src::Row& w, uint32_t col, uint32_t bk, bool first, float* acc) {
-    float m = -INFINITY, l = 0.0f;
-    for (int i = 0; i < N; i++) acc[i] = 0.0f;
-    const float* q = src.q_row(c, w);
-    const uint32_t dk = src.dk(), n = src.dv(c) > col ? min((uint32_t)N, src.dv(c) - col) : 0u;
-    for (uint32_t t = c.t0; t < c.t1; t++) {
-        if (!src.classify(c, t, bk)) continue;
-        for (uint32_t u = t * bk; u < (t + 1) * bk; u++) {
-            if (src.slow_score(c, w, u, 0.0f) == -INFINITY) continue;          // not seen
-            const float* k = src_key(src, c, u);
-            float d = 0.0f;
-            for (uint32_t i = 0; i < dk; i++) d = fmaf(q[i], k[i], d);
-            const float s = src.slow_score(c, w, u, d);
-            float e;
-            if (src.sigmoid()) e = s == -INFINITY ? 0.0f : ca_sigmoid(s);
-            else {
-                if (s == -INFINITY) continue;
-                const float mn = fmaxf(m, s), al = m == -INFINITY ? 0.0f : expf(m - mn);
-                e = expf(s - mn);
-                l = fmaf(l, al, e);
-                m = mn;
-                for (uint32_t i = 0; i < n; i++) acc[i] *= al;
+// The CTA's rows in plain f32, by its 512 softmax threads once the ring is idle: thread (ty, tx) of 32 x 16 holds rows 4 ty .. + 3 against keys tx + 16 c of 64, and value
+// columns tx + 16 c.  Keys that a row does not see are left out of its sums (what they hold need not be finite).
+template <int DV, class Src>
+__device__ __noinline__ void atc_plain(const Src& src, const typename Src::Cta& c, uint32_t bk, float* sm) {
+    constexpr int OC = DV / 16, KP = 68;
+    float* const Qs = sm;                              // [128][64]: 64 dims of the queries, of the keys
+    float* const Ks = Qs + 128 * 64;                   // [64][68]
+    float* const Ps = Ks + 64 * KP;                    // [128][68]: probabilities
+    float* const Vs = Ps + 128 * KP;                   // [64][DV]
+    const uint32_t tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, dk = src.dk(), dv = src.dv(c);
+    float o[4][OC], m[4], l[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        m[r] = -INFINITY; l[r] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < OC; k++) o[r][k] = 0.0f;
+    }
+#pragma unroll 1
+    for (uint32_t u0 = c.t0 * bk; u0 < src.plain_end(c, bk); u0 += 64) {
+        if (u0 / bk < c.t1 && !src.classify(c, u0 / bk, bk)) continue;
+        float sc[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) sc[r][k] = 0.0f;
+#pragma unroll 1
+        for (uint32_t d0 = 0; d0 < dk; d0 += 64) {
+            bar_sync(5, 512);                          // the readers of the slice, the probabilities and the values before are done
+            for (uint32_t i = tid; i < 128 * 16; i += 512) {
+                const uint32_t r = i >> 4, d = 4 * (i & 15);
+                *reinterpret_cast<float4*>(Qs + r * 64 + d) = r < c.nq && d0 + d < dk ? *reinterpret_cast<const float4*>(src.q_row(c, src.query(c, r)) + d0 + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-            const float* v = src_value(src, c, u) + col;
-            for (uint32_t i = 0; i < n; i++) acc[i] = fmaf(e, v[i], acc[i]);
+            for (uint32_t i = tid; i < 64 * 16; i += 512) {
+                const uint32_t r = i >> 4, d = 4 * (i & 15);
+                *reinterpret_cast<float4*>(Ks + r * KP + d) = u0 + r < src.plain_end(c, bk) && d0 + d < dk ? *reinterpret_cast<const float4*>(src_key(src, c, u0 + r) + d0 + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+            if (d0 == 0)
+                for (uint32_t i = tid; i < 64 * (DV / 4); i += 512) {
+                    const uint32_t r = i / (DV / 4), col = 4 * (i % (DV / 4));
+                    *reinterpret_cast<float4*>(Vs + r * DV + col) = u0 + r < src.plain_end(c, bk) && col < dv ? *reinterpret_cast<const float4*>(src_value(src, c, u0 + r) + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+            bar_sync(5, 512);
+#pragma unroll 1
+            for (uint32_t d = 0; d < 64; d += 4) {
+                float4 q[4], k[4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) q[r] = *reinterpret_cast<const float4*>(Qs + (4 * ty + r) * 64 + d);
+#pragma unroll
+                for (int i = 0; i < 4; i++) k[i] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * i) * KP + d);
+#pragma unroll
+                for (int r = 0; r < 4; r++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) sc[r][i] = fmaf(q[r].w, k[i].w, fmaf(q[r].z, k[i].z, fmaf(q[r].y, k[i].y, fmaf(q[r].x, k[i].x, sc[r][i]))));
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const typename Src::Row w = src.query(c, 4 * ty + r);
+            float mx = -INFINITY, sum = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                sc[r][i] = w.on ? src.slow_score(c, w, u0 + tx + 16 * i, sc[r][i]) : -INFINITY;
+                mx = fmaxf(mx, sc[r][i]);
+            }
+            if (src.sigmoid()) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) Ps[(4 * ty + r) * KP + tx + 16 * i] = sc[r][i] == -INFINITY ? 0.0f : ca_sigmoid(sc[r][i]);
+                continue;
+            }
+#pragma unroll
+            for (int x = 8; x > 0; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+            const float mn = fmaxf(m[r], mx), al = m[r] == -INFINITY ? (mn == -INFINITY ? 1.0f : 0.0f) : expf(m[r] - mn);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float p = sc[r][i] == -INFINITY ? 0.0f : expf(sc[r][i] - mn);
+                Ps[(4 * ty + r) * KP + tx + 16 * i] = p;
+                sum += p;
+            }
+#pragma unroll
+            for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+            l[r] = fmaf(l[r], al, sum);
+            m[r] = mn;
+#pragma unroll
+            for (int k = 0; k < OC; k++) o[r][k] *= al;
+        }
+        bar_sync(5, 512);
+#pragma unroll 1
+        for (int j = 0; j < 64; j++) {
+            float v[OC];
+#pragma unroll
+            for (int k = 0; k < OC; k++) v[k] = Vs[j * DV + tx + 16 * k];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float p = Ps[(4 * ty + r) * KP + j];
+#pragma unroll
+                for (int k = 0; k < OC; k++) if (p != 0.0f) o[r][k] = fmaf(p, v[k], o[r][k]);
+            }
         }
     }
-    return src.finish(c, w, first, m, false, l, 1.0f);
+    bar_sync(5, 512);
+    float* const out = sm;                             // [128][DV]
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const typename Src::Row w = src.query(c, 4 * ty + r);
+        const float f = w.on ? src.finish(c, w, tx == 0, m[r], false, l[r], 1.0f) : 0.0f;
+#pragma unroll
+        for (int k = 0; k < OC; k++) out[(4 * ty + r) * DV + tx + 16 * k] = o[r][k] * f;
+    }
+    bar_sync(5, 512);
+    for (uint32_t i = tid; i < c.nq * (DV / 4); i += 512) {
+        const uint32_t r = i / (DV / 4), col = 4 * (i % (DV / 4));
+        src.put(c, src.query(c, r), col, *reinterpret_cast<const float4*>(out + r * DV + col));
+    }
 }
 
 // NC: 64-wide chunks of the key dimension; DV: value columns of the CTA (64 or 128)
@@ -444,7 +549,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tmem_slot) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    uint32_t* const trouble = reinterpret_cast<uint32_t*>(dsm_raw + (tmem_slot + 4 - smem_u32(dsm_raw)));      // a wait of the CTA ran out
+    uint32_t* const trouble = reinterpret_cast<uint32_t*>(dsm_raw + (tmem_slot + 4 - smem_u32(dsm_raw)));      // of the CTA: 1 rows that pairs cannot hold, 2 a wait that ran out
     if (threadIdx.x == 0) *trouble = 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const typename Src::Cta c = src.cta(BK);
@@ -587,6 +692,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         bar_sync(5, 512);
         float q_inv, q_scale;
+        bool wide;                                                    // the row's magnitudes lie too far apart
         {
             float4 x[4 * NC];                                        // 16 NC dims from 16 NC part on
             float mx = 0.0f;
@@ -595,6 +701,10 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
 #pragma unroll
             for (int i = 0; i < 4 * NC; i++) mx = abs_or_inf(abs_or_inf(abs_or_inf(abs_or_inf(mx, x[i].x), x[i].y), x[i].z), x[i].w);
             split_scale(row_max(mx), q_scale, q_inv);
+            uint32_t small = 0;
+#pragma unroll
+            for (int i = 0; i < 4 * NC; i++) small += is_small(x[i].x, q_scale) + is_small(x[i].y, q_scale) + is_small(x[i].z, q_scale) + is_small(x[i].w, q_scale);
+            wide = small >= kAtcSmallQuery;
 #pragma unroll
             for (int i = 0; i < NC; i++) {                           // 16 dims: 8 columns of pairs
                 uint32_t hi[8], lo[8];
@@ -618,7 +728,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < OW; i++) o[i] = 0.0f;
         float m = -INFINITY, l = 0.0f, alpha_prev = 1.0f, f_prev = 0.0f;
-        bool ok = true, slow = !(q_inv == q_inv);
+        bool ok = true, slow = wide || !(q_inv == q_inv);
         uint32_t it = 0;
         auto add_output = [&](uint32_t i) {                          // outputs of tile i join the running ones
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(o_full, i & 1));
@@ -690,19 +800,16 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         }
         // Outputs leave by whole rows too, through the idle ring.
         auto place = [&](int j) { return row * (DV / 4) + (((OW * part + j) / 4) ^ (row & 7)); };
-        if (slow && w.on) {
-            float acc[OW];
-            const float f = atc_slow_row<OW>(src, c, w, OW * part, BK, part == 0, acc);
-#pragma unroll 1
-            for (int j = 0; j < OW; j += 4) ring[place(j)] = make_float4(acc[j] * f, acc[j + 1] * f, acc[j + 2] * f, acc[j + 3] * f);
-        } else {
-            const float f = w.on ? src.finish(c, w, part == 0, m, true, l, kPInv) : 0.0f;
+        const float f = w.on ? src.finish(c, w, part == 0, m, true, l, kPInv) : 0.0f;
 #pragma unroll
-            for (int j = 0; j < OW; j += 4) ring[place(j)] = make_float4(o[j] * f, o[j + 1] * f, o[j + 2] * f, o[j + 3] * f);
-        }
-        if (!ok) { *trouble = 1; if (lane == 0) count_timeout(); }
+        for (int j = 0; j < OW; j += 4) ring[place(j)] = make_float4(o[j] * f, o[j + 1] * f, o[j + 2] * f, o[j + 3] * f);
+        if (slow) atomicOr(trouble, 1u);
+        if (!ok) { atomicOr(trouble, 2u); if (lane == 0) count_timeout(); }
         bar_sync(5, 512);
-        const bool lost = *trouble != 0;                             // (what still arrives in the ring is not looked at)
+        const uint32_t what = *trouble;
+        const bool lost = what & 2;                                  // (what still arrives in the ring is not looked at)
+        if (what == 1) atc_plain<DV>(src, c, BK, reinterpret_cast<float*>(ring));
+        else
         for (uint32_t i = threadIdx.x; i < c.nq * (DV / 4); i += 512) {
             const uint32_t r = i / (DV / 4), j = i % (DV / 4);
             src.put(c, src.query(c, r), 4 * j, lost ? make_float4(kNotANumber, kNotANumber, kNotANumber, kNotANumber) : ring[r * (DV / 4) + (j ^ (r & 7))]);
