@@ -125,6 +125,22 @@ def test_magnitudes_far_apart_within_a_tile(cuda_backend, what):
     assert np.isfinite(got).all()
 
 
+@pytest.mark.parametrize("what", ["values", "orthogonal"])
+def test_magnitudes_near_the_largest_float(cuda_backend, what):
+    """Values of 1e35 are averaged; queries of 1e24 meet keys of 1e24 in other dims (every score is a plain 0) and ordinary ones in none."""
+    r = np.random.default_rng(11)
+    T, pos, H, G, d = 200, 100, 8, 4, 128
+    k, v, q = r.standard_normal((pos + T, G * d)), r.standard_normal((pos + T, G * d)), r.standard_normal((T, H * d))
+    if what == "values":
+        v *= 1e35
+    else:
+        k.reshape(pos + T, G, d)[:, :, :64] = 0.0
+        q.reshape(T, H, d)[:, :, 64:] = 0.0
+        k, q = k * 1e24, q * 1e24
+    got, want = direct(cuda_backend, q, k, v, pos, H, G, d)
+    assert close(got, want)
+
+
 @pytest.mark.parametrize("what", ["nan key", "nan value", "infinite value"])
 def test_rows_that_see_nothing_non_finite_are_exact(cuda_backend, what):
     """Position 150 of every key head or value head is poisoned: the queries before it are as they were, and those that see it are not finite."""

@@ -22,7 +22,8 @@
 //
 // What pairs cannot hold is evaluated in plain f32 (atc_plain: the CTA's 512 softmax threads over f32 tiles, as the SIMT kernels do it; 1.3 times their
 // time): all rows of a CTA that met a key or value tile, or a query row, that holds something non-finite or whose magnitudes lie too far apart for one
-// scale (is_small).  Such a tile is marked by a NaN scale.
+// scale (is_small; such a tile is marked by a NaN scale), or whose scaled products or outputs could leave f32's range before the scales are undone
+// (queries times keys beyond 2^108, values beyond 2^94).
 #include "attention_tc.cuh"
 #include "split_tc.cuh"
 
@@ -39,6 +40,7 @@ constexpr uint32_t kAtcTiles = 512;                               // key tiles w
 constexpr uint32_t kAtcSmem = kAtcRing * kAtcPiece + kAtcShare + kAtcTiles * 12 + 1024 + 256;
 constexpr float kNotANumber = __builtin_nanf("");
 constexpr size_t kAtcProgramKeys = 1u << 20;                      // the most keys that a DeviceOp.attention batch lays out planes for
+constexpr float kAtcBig = 1.2e24f;                                // 2^80: scores are at most 2^38 times f, outputs 2^33 times v_inv, and stay finite below it
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr float kPScale = 16384.0f, kPInv = 1.0f / 16384.0f;      // probabilities are held times 2^14
 
@@ -747,8 +749,8 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             const uint32_t cls = class_of(t);
             if (!cls) continue;
             const float2 inv = t - c.t0 < kAtcTiles ? tile_inv[t - c.t0] : make_float2(k_inv[t * BK / 128], v_inv[t * BK / 128]);
-            slow = slow || !(inv.x + inv.y == inv.x + inv.y);
             const float f = q_inv * inv.x * unit;
+            slow = slow || !(fabsf(f) < kAtcBig) || !(inv.y < kAtcBig);
             const bool plain = src.plain_tile() && cls == 1;
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(s_full + 8 * (it & 1), (it >> 1) & 1));
             fence_after();
