@@ -188,6 +188,27 @@ def test_batched_heads_with_their_own_masks_and_a_refreshed_length(cuda_backend)
     cuda_backend.free_program(handle)
 
 
+def test_masks_of_the_lowest_float(cuda_backend):
+    """An additive mask that holds the type's lowest value where others hold -inf: beside other scores it weighs nothing; a row that holds nothing else is the
+    plain mean of the values (every sum rounds to the lowest value)."""
+    from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO
+    r = np.random.default_rng(10)
+    T, S, dh, H, low = 140, 190, 128, 2, np.finfo(np.float32).min
+    q, k, v = r.standard_normal((H, T, dh)).astype(np.float32), r.standard_normal((S, dh)).astype(np.float32), r.standard_normal((S, dh)).astype(np.float32)
+    mask = np.where(r.random((T, S)) < 0.5, low, 0.0).astype(np.float32)
+    mask[[3, 77, 139]] = low
+    ops = [DeviceOp.attention(4, 0, 1, 2, 3, True, dh, T, S, 0.1, h * T * dh, 0, 0, 0, h * T * dh, 1, dh, 1, dh, 1, dh, 1, S, 1, dh) for h in range(H)]
+    handle = cuda_backend.compile_program(DeviceProgram(ops, [q.size, k.size, v.size, mask.size, q.size], [], []))
+    got = np.zeros((H, T, dh), np.float32)
+    cuda_backend.execute_program(handle, [ProgramIO(i, a.ravel()) for i, a in enumerate((q, k, v, mask))], [ProgramIO(4, got)])
+    cuda_backend.free_program(handle)
+    for h in range(H):
+        s = q[h].astype(np.float64) @ k.astype(np.float64).T * 0.1 + mask
+        s[[3, 77, 139]] = 0.0
+        e = np.exp(s - s.max(1, keepdims=True))
+        assert close(got[h], e @ v.astype(np.float64) / e.sum(1, keepdims=True))
+
+
 @pytest.mark.parametrize("what", ["nan key", "nan value", "infinite value"])
 def test_batched_rows_that_see_nothing_non_finite_are_exact(cuda_backend, what):
     """DeviceOp.attention: position 70 of the first of two key / value slabs holds no number; the rows whose mask leaves it out, and the heads of the other

@@ -20,10 +20,10 @@
 //     inside a single lane's branch, 9100 with four threads per row, 4700 once the whole MMA warp walks the tiles (below).
 //   * Every wait is bounded; a CTA whose wait ran out counts it (zg_attention_tc_timeouts), stops issuing, makes NaN of its rows and frees its TMEM.
 //
-// What pairs cannot hold is evaluated in plain f32 (atc_plain: the CTA's 512 softmax threads over f32 tiles, as the SIMT kernels do it; 1.3 times their
-// time): all rows of a CTA that met a key or value tile, or a query row, that holds something non-finite or whose magnitudes lie too far apart for one
-// scale (is_small; such a tile is marked by a NaN scale), or whose scaled products or outputs could leave f32's range before the scales are undone
-// (queries times keys beyond 2^108, values beyond 2^94).
+// What pairs cannot hold is evaluated in plain f32 (atc_plain: the CTA's 512 softmax threads over f32 tiles, as the SIMT kernels do it; 1.3 times
+// their time): all rows of a CTA that met a key or value tile, or a query row, that holds something non-finite or whose magnitudes lie too far apart
+// for one scale (is_small; such a tile is marked by a NaN scale), whose scores all lie near the lowest float (a mask of such values), or whose scaled
+// products or outputs could leave f32's range before the scales are undone (queries times keys beyond 2^108, values beyond 2^94).
 #include "attention_tc.cuh"
 #include "split_tc.cuh"
 
@@ -40,6 +40,7 @@ constexpr uint32_t kAtcTiles = 512;                               // key tiles w
 constexpr uint32_t kAtcSmem = kAtcRing * kAtcPiece + kAtcShare + kAtcTiles * 12 + 1024 + 256;
 constexpr float kNotANumber = __builtin_nanf("");
 constexpr size_t kAtcProgramKeys = 1u << 20;                      // the most keys that a DeviceOp.attention batch lays out planes for
+constexpr float kFltMax = 3.4028234e38f, kAtcLow = -1e36f;          // a row whose largest score is below kAtcLow is evaluated in plain f32
 constexpr float kAtcBig = 1.2e24f;                                // 2^80: scores are at most 2^38 times f, outputs 2^33 times v_inv, and stay finite below it
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr float kPScale = 16384.0f, kPInv = 1.0f / 16384.0f;      // probabilities are held times 2^14
@@ -50,6 +51,12 @@ __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32
 // as a whole, a key beside one that no row sees), not what they add to the large ones.  Normally distributed tiles of 128 x 128 have 0.1 to 0.3 of them.
 constexpr uint32_t kAtcSmallTile = 24, kAtcSmallQuery = 3;          // of 128 keys or values, of a quarter row
 __device__ __forceinline__ uint32_t is_small(float x, float scale) { const float a = fabsf(x * scale); return a < 0.0625f && a > 0.0f ? 1u : 0u; }
+// a score in units of log2 and what is added to it in natural units.  A finite term does not mask: near the lowest float, where times log2(e) it would be
+// -inf, the result stays finite, and a row without any higher score is evaluated in plain f32.
+__device__ __forceinline__ float plus_natural(float x, float v) {
+    const float y = fmaf(v, kLog2e, x);
+    return y < -kFltMax && v >= -kFltMax ? -kFltMax : y;
+}
 // ── where keys, values and queries come from ─────────────────────────────────────────────────────────────────────
 // A SOURCE names the keys of a step (for k_atc_prep) and, for the attention kernel, a CTA's items and range of key tiles, the class of a tile
 // (0: no row sees it, 1: every row sees all of it, 2: some), a row's query and what becomes of its scores.  Keys are counted from the first one
@@ -136,7 +143,7 @@ struct AtcCached {
         if (EXTRA && w.tab) {                                         // no pooled blocks here: positions ascend with u
             const uint32_t j0 = c.s.k_lo + u0;
 #pragma unroll
-            for (int i = 0; i < N; i++) if (j0 + i <= w.p && j0 + i >= w.lo) x[i] = fmaf(w.tab[w.p - j0 - i], kLog2e, x[i]);
+            for (int i = 0; i < N; i++) if (j0 + i <= w.p && j0 + i >= w.lo) x[i] = plus_natural(x[i], w.tab[w.p - j0 - i]);
         }
         const uint32_t base = c.s.k_lo - c.s.n_pool;
 #pragma unroll
@@ -248,7 +255,7 @@ struct AtcProgram {
 #pragma unroll
             for (int j = 0; j < 4; j++) { v[j] = u0 + i + j < c.n_keys ? *mask : 0.0f; mask += rs; }
 #pragma unroll
-            for (int j = 0; j < 4; j++) x[i + j] = x[i + j] == -INFINITY ? -INFINITY : fmaf(v[j], kLog2e, x[i + j]);
+            for (int j = 0; j < 4; j++) x[i + j] = x[i + j] == -INFINITY ? -INFINITY : plus_natural(x[i + j], v[j]);
             asm volatile("" ::: "memory");
         }
     }
@@ -805,7 +812,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         const float f = w.on ? src.finish(c, w, part == 0, m, true, l, kPInv) : 0.0f;
 #pragma unroll
         for (int j = 0; j < OW; j += 4) ring[place(j)] = make_float4(o[j] * f, o[j + 1] * f, o[j + 2] * f, o[j + 3] * f);
-        if (slow) atomicOr(trouble, 1u);
+        if (slow || (m < kAtcLow && m != -INFINITY)) atomicOr(trouble, 1u);
         if (!ok) { atomicOr(trouble, 2u); if (lane == 0) count_timeout(); }
         bar_sync(5, 512);
         const uint32_t what = *trouble;
