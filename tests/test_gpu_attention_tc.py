@@ -87,6 +87,18 @@ def test_many_rows(cuda_backend, shape):
     assert close(got, want)
 
 
+@pytest.mark.parametrize("shape", [
+    dict(T=16, pos=0, H=8, G=8, dk=64, dv=64, R=8192), dict(T=16, pos=300, H=8, G=8, dk=64, dv=128, R=8192, sink=True), dict(T=17, pos=2000, H=8, G=4, dk=160, dv=64, R=8000, sigmoid=True),
+    dict(T=300, pos=0, H=8, G=2, dk=64, dv=64, R=20000), dict(T=1, pos=0, H=16, G=1, dk=64, dv=64, R=6000), dict(T=1, pos=30, H=16, G=1, dk=320, dv=256, R=6000, sink=True),
+    dict(T=1, pos=2047, H=8, G=1, dk=128, dv=128, R=6000), dict(T=2, pos=2048, H=8, G=1, dk=128, dv=64, R=6000, sigmoid=True), dict(T=1, pos=4735, H=4, G=1, dk=64, dv=64, R=6000, out_scale=0.5),
+    dict(T=1, pos=5999, H=16, G=1, dk=64, dv=64, R=6000), dict(T=1, pos=900, H=4, G=1, dk=64, dv=64, R=6000, mask="block", size=1000, slot=1)],
+    ids=lambda d: " ".join(f"{k}{v}" for k, v in d.items() if k in ("T", "pos", "dk", "R")))
+def test_steps_shorter_than_their_cache(cuda_backend, shape):
+    """Key shares are planned for the cache's capacity and dealt by what a step sees: records of shares that are not used hold anything."""
+    got, want, _, _ = case(cuda_backend, **shape)
+    assert close(got, want)
+
+
 def direct(be, q, k, v, pos, H, G, d):
     """Causal CACHED_ATTENTION of rows q [T, H d] over the cache rows k, v [pos + T, G d]."""
     from zgml_b200 import DeviceBuffer, DeviceOp, ExternBuffer

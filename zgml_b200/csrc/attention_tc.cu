@@ -85,7 +85,7 @@ struct AtcCached {
         return (value ? a.vc + a.v_off : a.kc + a.k_off) + ((size_t)s.slot * a.R + (s.k_lo + u - s.n_pool) % a.R) * w + col;
     }
     __device__ __forceinline__ uint32_t prep_keys(uint32_t) const { return step().n_keys; }
-    struct Cta { Step s; uint32_t r0, nq, p_min, p_max, lo_min, lo_max, nb_min, nb_max, gm, g, m, vs, split, t0, t1; };
+    struct Cta { Step s; uint32_t r0, nq, p_min, p_max, lo_min, lo_max, nb_min, nb_max, gm, g, m, vs, split, used, t0, t1; };
     __device__ __forceinline__ Cta cta(uint32_t bk) const {
         Cta c;
         c.s = step();
@@ -98,11 +98,15 @@ struct AtcCached {
         c.nb_min = c.nb_max = 0;
         if (EXTRA && a.pool) { c.nb_min = pooled_seen(c.p_min, a.size, a.pool); c.nb_max = pooled_seen(c.p_max, a.size, a.pool); }
         const uint32_t first = c.s.n_pool ? 0u : (c.lo_min - c.s.k_lo) / bk, end = (min(c.s.n_keys, c.s.n_pool + c.p_max - c.s.k_lo + 1) + bk - 1) / bk;
-        const uint32_t per = (end - min(end, first) + splits - 1) / splits;
+        // at most a share per key tile, whatever the capacity asks for: the merge reads a record per share
+        const uint32_t n = end - min(end, first);
+        c.used = max(1u, min(splits, n));
+        const uint32_t per = (n + c.used - 1) / c.used;
         c.t0 = min(end, first + c.split * per); c.t1 = min(end, c.t0 + per);
         return c;
     }
     __device__ __forceinline__ uint32_t plain_end(const Cta& c, uint32_t bk) const { return c.t1 * bk; }
+    __device__ __forceinline__ bool idle(const Cta& c) const { return c.split >= c.used; }       // a share that the step has no keys for
     __device__ __forceinline__ uint32_t k_item(const Cta& c) const { return c.gm; }
     __device__ __forceinline__ uint32_t v_item(const Cta& c) const { return c.g * n_vs + c.vs; }
     __device__ __forceinline__ uint32_t classify(const Cta& c, uint32_t t, uint32_t bk) const {
@@ -168,7 +172,7 @@ struct AtcCached {
         if (splits > 1) {
             if (first && c.vs == 0) {
                 float* mine = part + (((size_t)(w.r / rh) * a.H * a.maps + w.hm) * splits + c.split) * (4 + a.dv);
-                mine[0] = m2 ? m * kLn2 : m; mine[1] = l * unit;
+                mine[0] = sigmoid() ? 0.0f : m2 ? m * kLn2 : m; mine[1] = l * unit;
             }
             return unit;
         }
@@ -176,6 +180,13 @@ struct AtcCached {
         float sum = l * unit;
         if (a.sink) sum += m2 ? exp2f(fmaf(ca_sink(a, w.hm), kLog2e, -m)) : expf(ca_sink(a, w.hm) - m);
         return unit * a.out_scale / sum;
+    }
+    // the record of a share without keys weighs nothing
+    __device__ __forceinline__ void leave_empty(const Cta& c, uint32_t i) const {
+        const Row w = query(c, i);
+        if (!w.on || c.vs) return;
+        float* mine = part + (((size_t)(w.r / rh) * a.H * a.maps + w.hm) * splits + c.split) * (4 + a.dv);
+        mine[0] = -INFINITY; mine[1] = 0.0f;
     }
     // four finished output columns from col on
     __device__ __forceinline__ void put(const Cta& c, const Row& w, uint32_t col, float4 v) const {
@@ -219,6 +230,8 @@ struct AtcProgram {
         return c;
     }
     __device__ __forceinline__ uint32_t plain_end(const Cta& c, uint32_t) const { return c.n_keys; }
+    __device__ __forceinline__ bool idle(const Cta&) const { return false; }
+    __device__ __forceinline__ void leave_empty(const Cta&, uint32_t) const {}
     __device__ __forceinline__ uint32_t k_item(const Cta& c) const { return c.kv; }
     __device__ __forceinline__ uint32_t v_item(const Cta& c) const { return c.kv; }
     __device__ __forceinline__ uint32_t classify(const Cta& c, uint32_t t, uint32_t bk) const {
@@ -303,7 +316,7 @@ struct AtcPlanes {
     uint32_t dkp, vslice, dk, dv, k_items, v_items, n_vs, tiles;
 };
 
-// CTA (tile, item): 128 keys of key item y, or 128 values of value item y - k_items.  C: 64-wide chunks of the widest item, all of which lie in
+// CTA (x, item): 128 keys of key item y at a time, or 128 values of value item y - k_items.  C: 64-wide chunks of the widest item, all of which lie in
 // registers: every load is in flight at once.  (Reading twice, once for the maximum, took 17.5 us where this takes 9.5: 2048 keys and values of
 // 4 heads of 128, cold.)
 constexpr uint32_t kPrepThreads = 512;
@@ -314,73 +327,78 @@ __global__ void __launch_bounds__(kPrepThreads, C == 1 ? 3 : C == 2 ? 2 : 1) k_a
     __shared__ uint32_t n_small[kPrepThreads / 32];
     __shared__ uint32_t t_hi[64][65], t_lo[64][65];      // a 64-column chunk of 128 values, transposed: pairs of keys per word
     const bool value = blockIdx.y >= pl.k_items;
-    const uint32_t item = value ? blockIdx.y - pl.k_items : blockIdx.y, head = value ? item / pl.n_vs : item, u0 = blockIdx.x * 128, n_keys = src.prep_keys(head);
-    if (u0 >= n_keys) return;
+    const uint32_t item = value ? blockIdx.y - pl.k_items : blockIdx.y, head = value ? item / pl.n_vs : item, n_keys = src.prep_keys(head);
     const uint32_t first = value ? item % pl.n_vs * pl.vslice : 0, dim = value ? min(pl.vslice, pl.dv - first) : pl.dk, padded = value ? pl.vslice : pl.dkp;
     const uint32_t tid = threadIdx.x, c4 = 4 * (tid & 15), k0 = 4 * (tid >> 4);      // columns c4 .. + 3 of every chunk, keys k0 .. + 3
-    float4 x[C][4];
-    float mx = 0.0f;
+    // CTAs for four per SM; they take the tiles that hold keys in turn (a step's capacity may be many times its length)
+#pragma unroll 1
+    for (uint32_t tile = blockIdx.x; tile * 128 < n_keys; tile += gridDim.x) {
+        const uint32_t u0 = tile * 128;
+        if (tile != blockIdx.x) __syncthreads();         // the tile before is done with the shared memory
+        float4 x[C][4];
+        float mx = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const uint32_t u = u0 + k0 + k;
-        const float* row = u < n_keys ? src_row(src, value, head, u) + first : nullptr;
+        for (int k = 0; k < 4; k++) {
+            const uint32_t u = u0 + k0 + k;
+            const float* row = u < n_keys ? src_row(src, value, head, u) + first : nullptr;
 #pragma unroll
-        for (int c = 0; c < C; c++) x[c][k] = row && 64 * c + c4 < dim ? *reinterpret_cast<const float4*>(row + 64 * c + c4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-#pragma unroll
-    for (int c = 0; c < C; c++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) mx = abs_or_inf(abs_or_inf(abs_or_inf(abs_or_inf(mx, x[c][k].x), x[c][k].y), x[c][k].z), x[c][k].w);
-    mx = warp_max(mx);
-    if ((tid & 31) == 0) red[tid >> 5] = mx;
-    __syncthreads();
-    mx = warp_max(red[tid & 15]);
-    float scale, inv;
-    split_scale(mx, scale, inv);
-    uint32_t small = 0;
-#pragma unroll
-    for (int c = 0; c < C; c++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) small += is_small(x[c][k].x, scale) + is_small(x[c][k].y, scale) + is_small(x[c][k].z, scale) + is_small(x[c][k].w, scale);
-    small = __reduce_add_sync(0xffffffffu, small);
-    if ((tid & 31) == 0) n_small[tid >> 5] = small;
-    __syncthreads();
-    if (tid == 0) {
-        small = 0;
-        for (uint32_t i = 0; i < kPrepThreads / 32; i++) small += n_small[i];
-        if (small >= min(kAtcSmallTile, max(4u, min(128u, n_keys - u0)))) inv = __uint_as_float(0x7fffffffu);
-        (value ? pl.v_inv : pl.k_inv)[(size_t)item * pl.tiles + blockIdx.x] = inv;
-    }
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-        if (64 * c >= padded) break;
-        if (!value) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                uint32_t h[2], l[2];
-                split2(x[c][k].x * scale, x[c][k].y * scale, h[0], l[0]);
-                split2(x[c][k].z * scale, x[c][k].w * scale, h[1], l[1]);
-                __half* out = pl.k + ((size_t)item * pl.tiles * 128 + u0 + k0 + k) * 2 * pl.dkp + 64 * c + c4;
-                *reinterpret_cast<uint2*>(out) = make_uint2(h[0], h[1]);
-                *reinterpret_cast<uint2*>(out + pl.dkp) = make_uint2(l[0], l[1]);
-            }
-            continue;
+            for (int c = 0; c < C; c++) x[c][k] = row && 64 * c + c4 < dim ? *reinterpret_cast<const float4*>(row + 64 * c + c4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-        if (c) __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 4; k += 2) {
-            const float* a = &x[c][k].x;
-            const float* b = &x[c][k + 1].x;
+        for (int c = 0; c < C; c++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) split2(a[e] * scale, b[e] * scale, t_hi[c4 + e][(k0 + k) / 2], t_lo[c4 + e][(k0 + k) / 2]);
-        }
+            for (int k = 0; k < 4; k++) mx = abs_or_inf(abs_or_inf(abs_or_inf(abs_or_inf(mx, x[c][k].x), x[c][k].y), x[c][k].z), x[c][k].w);
+        mx = warp_max(mx);
+        if ((tid & 31) == 0) red[tid >> 5] = mx;
         __syncthreads();
+        mx = warp_max(red[tid & 15]);
+        float scale, inv;
+        split_scale(mx, scale, inv);
+        uint32_t small = 0;
 #pragma unroll
-        for (uint32_t i = tid; i < 64 * 64; i += kPrepThreads) {
-            const uint32_t col = i >> 6, w = i & 63;
-            uint32_t* out = reinterpret_cast<uint32_t*>(pl.v + ((size_t)item * pl.vslice + 64 * c + col) * 2 * pl.tiles * 128 + u0);
-            out[w] = t_hi[col][w];
-            out[pl.tiles * 64 + w] = t_lo[col][w];
+        for (int c = 0; c < C; c++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) small += is_small(x[c][k].x, scale) + is_small(x[c][k].y, scale) + is_small(x[c][k].z, scale) + is_small(x[c][k].w, scale);
+        small = __reduce_add_sync(0xffffffffu, small);
+        if ((tid & 31) == 0) n_small[tid >> 5] = small;
+        __syncthreads();
+        if (tid == 0) {
+            small = 0;
+            for (uint32_t i = 0; i < kPrepThreads / 32; i++) small += n_small[i];
+            if (small >= min(kAtcSmallTile, max(4u, min(128u, n_keys - u0)))) inv = __uint_as_float(0x7fffffffu);
+            (value ? pl.v_inv : pl.k_inv)[(size_t)item * pl.tiles + tile] = inv;
+        }
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            if (64 * c >= padded) break;
+            if (!value) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    uint32_t h[2], l[2];
+                    split2(x[c][k].x * scale, x[c][k].y * scale, h[0], l[0]);
+                    split2(x[c][k].z * scale, x[c][k].w * scale, h[1], l[1]);
+                    __half* out = pl.k + ((size_t)item * pl.tiles * 128 + u0 + k0 + k) * 2 * pl.dkp + 64 * c + c4;
+                    *reinterpret_cast<uint2*>(out) = make_uint2(h[0], h[1]);
+                    *reinterpret_cast<uint2*>(out + pl.dkp) = make_uint2(l[0], l[1]);
+                }
+                continue;
+            }
+            if (c) __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {
+                const float* a = &x[c][k].x;
+                const float* b = &x[c][k + 1].x;
+#pragma unroll
+                for (int e = 0; e < 4; e++) split2(a[e] * scale, b[e] * scale, t_hi[c4 + e][(k0 + k) / 2], t_lo[c4 + e][(k0 + k) / 2]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (uint32_t i = tid; i < 64 * 64; i += kPrepThreads) {
+                const uint32_t col = i >> 6, w = i & 63;
+                uint32_t* out = reinterpret_cast<uint32_t*>(pl.v + ((size_t)item * pl.vslice + 64 * c + col) * 2 * pl.tiles * 128 + u0);
+                out[w] = t_hi[col][w];
+                out[pl.tiles * 64 + w] = t_lo[col][w];
+            }
         }
     }
 }
@@ -579,7 +597,9 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     fence_after();
     auto class_of = [&](uint32_t t) { return t - c.t0 < kAtcTiles ? tile_class[t - c.t0] : src.classify(c, t, BK); };
 
-    if (warp == 16) {
+    if (src.idle(c)) {                                               // uniform over the CTA
+        if (threadIdx.x < 128) src.leave_empty(c, threadIdx.x);
+    } else if (warp == 16) {
         if (lane == 0) {
             uint32_t slot = 0, phase = 1;                            // ring position
             bool ok = true;
@@ -876,7 +896,8 @@ bool launch(const Src& src, const AtcPlanes& pl, dim3 grid, cudaStream_t st) {
     CUtensorMap mk, mv;
     if (!encode_plane(&mk, pl.k, 2 * pl.dkp, (uint64_t)pl.k_items * pl.tiles * 128, BK) || !encode_plane(&mv, pl.v, (uint64_t)2 * pl.tiles * 128, (uint64_t)pl.v_items * pl.vslice, DV)) return false;
     if (!zg_smem_limit<k_attention_tc<Src, NC, DV>>(kAtcSmem)) return false;
-    launch_pdl(k_atc_prep<Src, C>, dim3(pl.tiles, pl.k_items + pl.v_items), dim3(kPrepThreads), 0, st, src, pl);
+    const uint32_t items = pl.k_items + pl.v_items, per_item = (4 * zg_sm_count() + items - 1) / items;
+    launch_pdl(k_atc_prep<Src, C>, dim3(pl.tiles < per_item ? pl.tiles : per_item, items), dim3(kPrepThreads), 0, st, src, pl);
     ZG_COUNT_LAUNCH();
     launch_pdl(k_attention_tc<Src, NC, DV>, grid, dim3(kAtcThreads), kAtcSmem, st, mk, mv, src, pl);
     const cudaError_t e = cudaGetLastError();

@@ -473,17 +473,17 @@ __global__ void __launch_bounds__(kCtThreads) k_cached_attention_tiled(CaArgs a,
             for (int c = 0; c < OC; c++) if (tx + 16 * c < v_cols) out[tx + 16 * c] = o[r][c] * inv;
         } else {
             float* mine = part + (((size_t)(row / rh) * a.H * a.maps + hm) * splits + blockIdx.z) * (4 + a.dv);
-            if (tx == 0 && vs == 0) { mine[0] = m_run[r]; mine[1] = l_run[r]; }
+            if (tx == 0 && vs == 0) { mine[0] = a.wkind ? 0.0f : m_run[r]; mine[1] = l_run[r]; }
 #pragma unroll
             for (int c = 0; c < OC; c++) if (tx + 16 * c < v_cols) mine[4 + (size_t)vs * DV + tx + 16 * c] = o[r][c];
         }
     }
 }
-// merge of the key shares: CTA (x, y) = 128 value columns y of (token, head, map) x; a share that saw no key carries
-// max = -inf and weighs nothing (its output is zero)
+// merge of the key shares: CTA (x, y) = 64 value columns y of (token, head, map) x; a share that saw no key (or that the step has no keys for) carries
+// max = -inf and weighs nothing (its output may be anything)
 // (a: for the sink, the output scale and the row layout of dst; HM = H * maps)
 constexpr int kMergeCols = 64, kMergeGroups = 8;        // groups of 64 threads that each add up an eighth of the shares
-__global__ void __launch_bounds__(kMergeCols * kMergeGroups) k_cached_attention_merge(CaArgs a, const float* __restrict__ part, uint32_t dv, uint32_t splits,
+__global__ void __launch_bounds__(kMergeCols * kMergeGroups, 4) k_cached_attention_merge(CaArgs a, const float* __restrict__ part, uint32_t dv, uint32_t splits,
                                                                 uint32_t wkind) {
     pdl_enter();
     __shared__ float w[kCaMaxShares], sums[kMergeGroups][kMergeCols];
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kMergeCols * kMergeGroups) k_cached_attention_
     const float* P = part + (size_t)blockIdx.x * splits * (4 + dv);
     const uint32_t HM = a.H * a.maps, hm = blockIdx.x % HM;
     if (wkind) {                                       // unnormalised weights: the shares just add up
-        if (threadIdx.x < splits) w[threadIdx.x] = a.out_scale;
+        if (threadIdx.x < splits) w[threadIdx.x] = P[threadIdx.x * (4 + dv)] == -INFINITY ? 0.0f : a.out_scale;
     } else if (threadIdx.x < 32) {                            // warp 0: the shares' weights exp(m_i - M) / L
         constexpr int kPer = kCaMaxShares / 32;
         float m[kPer], l[kPer], M = -INFINITY, L = 0.0f;
@@ -513,7 +513,10 @@ __global__ void __launch_bounds__(kMergeCols * kMergeGroups) k_cached_attention_
     float acc = 0.0f;
     if (c < dv) {
 #pragma unroll 16
-        for (uint32_t i = group; i < splits; i += kMergeGroups) acc = fmaf(P[i * (4 + dv) + 4 + c], w[i], acc);
+        for (uint32_t i = group; i < splits; i += kMergeGroups) {
+            const float x = P[i * (4 + dv) + 4 + c];               // (of a share without keys: anything)
+            if (w[i] != 0.0f) acc = fmaf(x, w[i], acc);
+        }
     }
     sums[group][threadIdx.x % kMergeCols] = acc;
     __syncthreads();
@@ -535,6 +538,10 @@ __global__ void __launch_bounds__(kMergeCols * kMergeGroups) k_cached_attention_
 // of the key dimension and the columns per thread halve).  One token, 16 heads, 8192 latents of 576: with 148 shares instead of 64 and sixteen warps
 // 45 -> 24 us, the op with its merge and the append 54 -> 33.
 constexpr int kCfRows = 16, kCfKeys = 32;
+// How many of a step's shares (as many as the cache's capacity asks for) its keys are dealt to: beyond 64 only where each gets sixteen keys.  What the step
+// reads is its keys, and the merge reads a record per share: with 148 shares whatever the position, a token at position 500 of a cache of 8192 latents
+// of 576 took 22.6 us instead of 20.6; with 32 keys a share one at position 4000 26.7 instead of 24.8.
+__device__ __forceinline__ uint32_t few_shares(uint32_t n_keys, uint32_t splits) { return min(splits, max((uint32_t)kCtMaxSplits, (n_keys + 15) / 16)); }
 template <int kCfThreads, int CI, bool POOL>
 __global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, uint32_t rh, uint32_t splits, float* __restrict__ part, uint32_t alias) {
     pdl_enter();
@@ -559,9 +566,16 @@ __global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, u
     const size_t pool_slot = POOL ? (size_t)slot * a.pool_rows * a.kw : 0;
     const CaKeys<POOL> keys = ca_keys<POOL>(kbase, POOL ? a.kp + pool_slot + (size_t)gm * a.dk : nullptr, a.R, a.kw, k_lo, n_pool);
     const CaKeys<POOL> vals = ca_keys<POOL>(vbase, POOL ? a.vp + pool_slot + (size_t)g * a.dv : nullptr, a.R, a.vw, k_lo, n_pool);
-    const uint32_t n_keys = keys.count(p_max), per = (n_keys + splits - 1) / splits;
+    const uint32_t n_keys = keys.count(p_max), used = few_shares(n_keys, splits), per = (n_keys + used - 1) / used;
     const uint32_t k_begin = keys.first() + blockIdx.y * per, k_end = min(keys.first() + n_keys, k_begin + per);
     const bool ok = row < total, owner = tid < 16 * kCfRows;        // owner: of a row's running (max, sum)
+    if (blockIdx.y >= used) {                                       // no keys: a record that weighs nothing
+        if (kq == 0 && ok) {
+            float* mine = part + (((size_t)(row / rh) * a.H * a.maps + (g * rh + row % rh) * a.maps + m) * splits + blockIdx.y) * (4 + a.dv);
+            mine[0] = -INFINITY; mine[1] = 0.0f;
+        }
+        return;
+    }
     const uint32_t p_r = pos0 + (ok ? row / rh : 0), lo_r = mask_low(p_r, a.kind, a.size), nb_r = POOL ? pooled_seen(p_r, a.size, a.pool) : 0u;
     const float* tab_r = a.tab ? a.tab + (size_t)((g * rh + (ok ? row % rh : 0)) * a.maps + m) * a.tab_rs : nullptr;
     const uint32_t dk4 = a.dk / 4, dv4 = a.dv / 4;

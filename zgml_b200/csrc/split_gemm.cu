@@ -18,7 +18,8 @@
 //     166 us; as pairs with partial sums in scratch 169, as the f32 tile 1034).
 //   * One share of K: the tile is finished here (bias, activation) and leaves by whole rows.  Several: partial sums go to scratch and k_split_finish adds them in
 //     order.  A sum that is not finite is evaluated again as a plain f32 sum: what an infinity makes of a sum is the plain kernel's.
-//   * Every wait is bounded; a CTA whose wait ran out counts it and treats its sums as not finite, so that they are evaluated again the plain way.
+//   * Every wait is bounded and counts itself (with the count after the loops the case above took 178 us); a CTA whose wait ran out treats its sums as
+//     not finite, so that they are evaluated again the plain way.
 #include "split_tc.cuh"
 
 namespace {
@@ -93,8 +94,8 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
         bool ok = true;
         uint32_t stage = 0, phase = 0;
         for (uint32_t i = 0; i < n_steps; i++) {
-            if (ok) ok = mbar_wait(full + 8 * stage, phase);
-            if (ok && i >= 2) ok = mbar_wait(d_empty + 8 * (i & 1), ((i >> 1) - 1) & 1);
+            if (ok) ok = mbar_wait_counted(full + 8 * stage, phase);
+            if (ok && i >= 2) ok = mbar_wait_counted(d_empty + 8 * (i & 1), ((i >> 1) - 1) & 1);
             fence_after();
             if (leader && ok) {
                 const uint32_t d = tmem + (i & 1) * kBN, x0 = b0 + stage * (kSgStage >> 4);
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
         for (int j = 0; j < 32; j++) acc[j] = 0.0f;
         bool ok = true;
         auto drain = [&](uint32_t i) {
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(d_full + 8 * (i & 1), (i >> 1) & 1));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_counted(d_full + 8 * (i & 1), (i >> 1) & 1));
             fence_after();
             uint32_t v[32];
             tmem_ld(tmem + ((quarter * 32) << 16) + (i & 1) * kBN + 32 * part, v);
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
         if (n_steps) load(s0);
         uint32_t stage = 0, phase = 1;
         for (uint32_t i = 0; i < n_steps; i++) {
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * stage, phase));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_counted(empty + 8 * stage, phase));
             uint8_t* const to = ring + stage * kSgStage;
 #pragma unroll
             for (int j = 0; j < 8; j++) {                            // the source's rows, the weights'
@@ -171,7 +172,6 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
             if (i) drain(i - 1);
         }
         if (n_steps) drain(n_steps - 1);
-        if (!ok && lane == 0) count_timeout();
         // out by whole rows, through the idle ring (every MMA that reads it is done)
         float4* const out = reinterpret_cast<float4*>(ring);
         const uint32_t row = quarter * 32 + lane;

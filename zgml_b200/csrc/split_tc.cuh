@@ -34,6 +34,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 }
 // at the end of a role, once, rather than in each wait (a counter in the waits of an attention loop made it 7 % slower)
 __device__ __forceinline__ void count_timeout() { atomicAdd(&g_tc_timeouts, 1u); }
+// a wait that counts itself
+__device__ __forceinline__ bool mbar_wait_counted(uint32_t bar, uint32_t parity) {
+    const bool ok = mbar_wait(bar, parity);
+    if (!ok) count_timeout();
+    return ok;
+}
 __device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap* map, uint32_t c0, uint32_t c1, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
