@@ -200,6 +200,48 @@ def test_batched_heads_with_their_own_masks_and_a_refreshed_length(cuda_backend)
     cuda_backend.free_program(handle)
 
 
+def heads_in_a_slab(be, r, T, S, dh, G, H, offs, kv, compile_kv=None):
+    """H heads over G slabs of S rows (head h: those that start at row offs[h]) in one buffer, kv[h] keys each -> (got, want, handle, refresh)."""
+    from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO
+    q, k, v = (r.standard_normal(n).astype(np.float32) for n in ((H, T, dh), (G * S, dh), (G * S, dh)))
+    ops = [DeviceOp.attention(3, 0, 1, 2, 0, False, dh, T, (compile_kv or kv)[h], 0.2, h * T * dh, offs[h] * dh, offs[h] * dh, 0, h * T * dh, 1, dh, 1, dh, 1, dh, 0, 0, 1, dh) for h in range(H)]
+    handle = be.compile_program(DeviceProgram(ops, [q.size, k.size, v.size, q.size], [], []))
+    if compile_kv:
+        for o, n in zip(ops, kv):
+            o.u.attention.seq_kv = n
+        be.refresh_program(handle, ops)
+    got = np.zeros((H, T, dh), np.float32)
+    be.execute_program(handle, [ProgramIO(i, a.ravel()) for i, a in enumerate((q, k, v))], [ProgramIO(3, got)])
+    want = np.empty((H, T, dh))
+    for h in range(H):
+        kk, vv = (a[offs[h]:offs[h] + kv[h]].astype(np.float64) for a in (k, v))
+        want[h] = reference(q[h].astype(np.float64), kk, vv, np.ones((T, kv[h]), bool), 0.2)
+    return got, want, handle
+
+
+def test_scratch_follows_the_slabs(cuda_backend):
+    """Eight heads of one buffer: planes for what the operands hold, not for the rest of the buffer behind each head."""
+    G, S, dh, T = 8, 640, 64, 40
+    got, want, handle = heads_in_a_slab(cuda_backend, np.random.default_rng(13), T, S, dh, G, G, [g * S for g in range(G)], [500] * G)
+    assert close(got, want)
+    assert 0 < cuda_backend.program_stats(handle)["shared_scratch_elems"] <= 1.1 * 2 * G * S * dh
+    cuda_backend.free_program(handle)
+
+
+def test_more_keys_than_planes(cuda_backend):
+    """Head 1 starts at row 128 of head 0's rows when the program is compiled for 100 keys; head 0 is then refreshed past it."""
+    got, want, handle = heads_in_a_slab(cuda_backend, np.random.default_rng(14), 70, 400, 64, 1, 2, [0, 128], [390, 150], compile_kv=[100, 100])
+    assert close(got, want)
+    cuda_backend.free_program(handle)
+
+
+def test_no_room_for_planes(cuda_backend, monkeypatch):
+    monkeypatch.setenv("ZG_CUDA_SCRATCH_MB", "0")
+    got, want, handle = heads_in_a_slab(cuda_backend, np.random.default_rng(15), 70, 300, 128, 2, 4, [0, 0, 300, 300], [300, 200, 300, 10])
+    assert close(got, want) and cuda_backend.program_stats(handle)["shared_scratch_elems"] == 0
+    cuda_backend.free_program(handle)
+
+
 def test_masks_of_the_lowest_float(cuda_backend):
     """An additive mask that holds the type's lowest value where others hold -inf: beside other scores it weighs nothing; a row that holds nothing else is the
     plain mean of the values (every sum rounds to the lowest value)."""

@@ -21,9 +21,10 @@
 //   * Every wait is bounded; a CTA whose wait ran out counts it (zg_attention_tc_timeouts), stops issuing, makes NaN of its rows and frees its TMEM.
 //
 // What pairs cannot hold is evaluated in plain f32 (atc_plain: the CTA's 512 softmax threads over f32 tiles, as the SIMT kernels do it; 1.3 times
-// their time): all rows of a CTA that met a key or value tile, or a query row, that holds something non-finite or whose magnitudes lie too far apart
-// for one scale (is_small; such a tile is marked by a NaN scale), whose scores all lie near the lowest float (a mask of such values), or whose scaled
-// products or outputs could leave f32's range before the scales are undone (queries times keys beyond 2^108, values beyond 2^94).
+// their time): all rows of an op with more keys than there are planes for, and of a CTA that met a key or value tile, or a query row, that holds
+// something non-finite or whose magnitudes lie too far apart for one scale (is_small; such a tile is marked by a NaN scale), whose scores all lie
+// near the lowest float (a mask of such values), or whose scaled products or outputs could leave f32's range before the scales are undone (queries
+// times keys beyond 2^108, values beyond 2^94).
 #include "attention_tc.cuh"
 #include "split_tc.cuh"
 
@@ -107,6 +108,7 @@ struct AtcCached {
     }
     __device__ __forceinline__ uint32_t plain_end(const Cta& c, uint32_t bk) const { return c.t1 * bk; }
     __device__ __forceinline__ bool idle(const Cta& c) const { return c.split >= c.used; }       // a share that the step has no keys for
+    __device__ __forceinline__ bool over(const Cta&) const { return false; }
     __device__ __forceinline__ uint32_t k_item(const Cta& c) const { return c.gm; }
     __device__ __forceinline__ uint32_t v_item(const Cta& c) const { return c.g * n_vs + c.vs; }
     __device__ __forceinline__ uint32_t classify(const Cta& c, uint32_t t, uint32_t bk) const {
@@ -215,7 +217,7 @@ struct AtcProgram {
         return min(__reduce_max_sync(0xffffffffu, n), tiles * 128);
     }
     __device__ __forceinline__ uint32_t prep_keys(uint32_t item) const { return item_keys(item, 0); }
-    struct Cta { const ZgBatchEntry* e; const uint8_t* cls; const uint32_t* bits; uint32_t r0, nq, n_keys, kv, t0, t1; bool masked; };
+    struct Cta { const ZgBatchEntry* e; const uint8_t* cls; const uint32_t* bits; uint32_t r0, nq, n_keys, n_all, kv, t0, t1; bool masked; };
     __device__ __forceinline__ Cta cta(uint32_t bk) const {
         Cta c;
         const uint32_t item = blockIdx.x % count, tile = row_tiles - 1 - blockIdx.x / count;      // under a causal mask later rows meet more keys
@@ -226,12 +228,14 @@ struct AtcProgram {
         c.cls = classes + m; c.bits = bits + m * 512;
         c.r0 = tile * 128; c.nq = min(128u, seq_q - c.r0);
         c.n_keys = min(dyn[c.e->dyn], tiles * 128);
+        c.n_all = dyn[c.e->dyn];
         c.t0 = 0; c.t1 = (c.n_keys + bk - 1) / bk;
         return c;
     }
-    __device__ __forceinline__ uint32_t plain_end(const Cta& c, uint32_t) const { return c.n_keys; }
+    __device__ __forceinline__ uint32_t plain_end(const Cta& c, uint32_t) const { return c.n_all; }
     __device__ __forceinline__ bool idle(const Cta&) const { return false; }
     __device__ __forceinline__ void leave_empty(const Cta&, uint32_t) const {}
+    __device__ __forceinline__ bool over(const Cta& c) const { return c.n_all > c.n_keys; }          // more keys than there are planes for
     __device__ __forceinline__ uint32_t k_item(const Cta& c) const { return c.kv; }
     __device__ __forceinline__ uint32_t v_item(const Cta& c) const { return c.kv; }
     __device__ __forceinline__ uint32_t classify(const Cta& c, uint32_t t, uint32_t bk) const {
@@ -273,7 +277,7 @@ struct AtcProgram {
         }
     }
     __device__ __forceinline__ float slow_score(const Cta& c, const Row& w, uint32_t u, float dot) const {
-        if (u >= c.n_keys) return -INFINITY;
+        if (u >= c.n_all) return -INFINITY;
         float s = dot * c.e->f;
         if (c.masked) {
             const float mv = mask_row(c, w)[(size_t)u * c.e->u[14]];
@@ -757,7 +761,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < OW; i++) o[i] = 0.0f;
         float m = -INFINITY, l = 0.0f, alpha_prev = 1.0f, f_prev = 0.0f;
-        bool ok = true, slow = wide || !(q_inv == q_inv);
+        bool ok = true, slow = wide || src.over(c) || !(q_inv == q_inv);
         uint32_t it = 0;
         auto add_output = [&](uint32_t i) {                          // outputs of tile i join the running ones
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(o_full, i & 1));
@@ -954,23 +958,37 @@ bool zg_attention_tc_launch(const ZgAtcShape& s, const void* args, float* scratc
 }
 
 // ── DeviceOp.attention batches ──
-// Keys an op can ever attend over: the last row of its key, value and mask operands that lies inside their buffers (what refresh checks).
-static size_t attention_key_bound(const ZgOp& op, const size_t* elems) {
+// Keys that planes are laid out for: those up to the next head, layer or operand in the same buffer (a head's rows may lie between other heads' rows; what
+// starts past the rows it attends over now ends them), and inside its key, value and mask operands.  An op that is refreshed to more is evaluated in plain f32.
+static size_t attention_key_bound(const ZgOp& op, const size_t* elems, const std::map<uint32_t, std::vector<size_t>>& starts) {
     const auto& a = op.u.attention;
+    const size_t now = std::max(a.seq_kv, a.seq_q);
     auto rows = [](size_t n, size_t off, size_t width, size_t stride) { return n < off + width ? (size_t)0 : stride ? (n - off - width) / stride + 1 : (size_t)UINT32_MAX; };
-    size_t n = std::min(rows(elems[a.k], a.k_off, a.d_head, a.k_cs), rows(elems[a.v], a.v_off, a.d_head, a.v_cs));
+    auto slab = [&](uint32_t buf, size_t off, size_t stride) {
+        const std::vector<size_t>& at = starts.at(buf);
+        const auto next = std::lower_bound(at.begin(), at.end(), off + (now ? now - 1 : 0) * stride + a.d_head);
+        return rows(next == at.end() ? elems[buf] : std::min(elems[buf], *next), off, a.d_head, stride);
+    };
+    size_t n = std::min(slab(a.k, a.k_off, a.k_cs), slab(a.v, a.v_off, a.v_cs));
     if (a.has_mask) n = std::min(n, rows(elems[a.mask], (size_t)a.mask_off + (size_t)(a.seq_q - 1) * a.mask_cs, 1, a.mask_rs));
     return n;
 }
-bool zg_atc_program_plan(const ZgOp* const* ops, uint32_t count, const size_t* buffer_elems, ZgAtcPlan* plan) {
+bool zg_atc_program_plan(const std::vector<ZgOp>& all, const ZgOp* const* ops, uint32_t count, const size_t* buffer_elems, ZgAtcPlan* plan) {
     const auto& first = ops[0]->u.attention;
-    size_t keys = 0;
+    size_t keys = 0, now = 0;
+    std::map<uint32_t, std::vector<size_t>> starts;                   // where keys and values of the program's attentions start in a buffer
+    for (const ZgOp& op : all)
+        if (op.tag == ZG_OP_ATTENTION) { starts[op.u.attention.k].push_back(op.u.attention.k_off); starts[op.u.attention.v].push_back(op.u.attention.v_off); }
+    for (auto& b : starts) std::sort(b.second.begin(), b.second.end());
+    std::map<uint32_t, size_t> operands;
     std::map<std::vector<uint32_t>, uint32_t> kv, masks;
     std::vector<uint32_t> kv_rep, mask_rep;
     plan->map.assign(2 * (size_t)count, 0);
     for (uint32_t i = 0; i < count; i++) {
         const auto& a = ops[i]->u.attention;
-        keys = std::max(keys, attention_key_bound(*ops[i], buffer_elems));
+        keys = std::max(keys, attention_key_bound(*ops[i], buffer_elems, starts));
+        now = std::max(now, (size_t)a.seq_kv);
+        operands[a.k] = buffer_elems[a.k]; operands[a.v] = buffer_elems[a.v];
         const auto k = kv.emplace(std::vector<uint32_t>{a.k, a.k_off, a.k_cs, a.v, a.v_off, a.v_cs}, (uint32_t)kv.size());
         if (k.second) kv_rep.push_back(i);
         plan->map[i] = k.first->second;
@@ -979,7 +997,12 @@ bool zg_atc_program_plan(const ZgOp* const* ops, uint32_t count, const size_t* b
         if (m.second) mask_rep.push_back(i);
         plan->map[count + i] = m.first->second;
     }
-    if (keys == 0 || keys > kAtcProgramKeys) return false;
+    // a head that reads on into something else's rows: no more than twice what the operands hold
+    size_t most = 0;
+    for (const auto& b : operands) most += 2 * b.second;
+    most = most / (2 * (size_t)first.d_head * 128 * kv.size()) * 128;
+    keys = std::min(keys, std::max(most, (size_t)128));
+    if (keys == 0 || keys < now || keys > kAtcProgramKeys) return false;
     plan->map.insert(plan->map.end(), kv_rep.begin(), kv_rep.end());
     plan->map.insert(plan->map.end(), mask_rep.begin(), mask_rep.end());
     plan->count = count; plan->kv_items = (uint32_t)kv_rep.size(); plan->mask_items = (uint32_t)mask_rep.size();

@@ -29,23 +29,31 @@ uint32_t zg_sm_count() {
     static const uint32_t n = [] { int dev = 0, v = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); return (uint32_t)(v > 0 ? v : 148); }();
     return n;
 }
+// ZG_CUDA_SCRATCH_MB: workspaces beyond that many megabytes count as out of memory (tests)
+static bool zg_scratch_refused(size_t bytes) {
+    const char* e = getenv("ZG_CUDA_SCRATCH_MB");
+    return e && bytes > (size_t)atol(e) << 20;
+}
+// false: out of memory; what was there before is there again, without its contents
+template <typename T>
+static bool grow(T** p, size_t* have, size_t want, cudaStream_t st) {
+    if (want <= *have) return true;
+    const size_t before = *have;
+    if (*p) { cudaStreamSynchronize(st); cudaFree(*p); *p = nullptr; }
+    *have = 0;
+    const cudaError_t e = zg_scratch_refused(want * sizeof(T)) ? cudaErrorMemoryAllocation : cudaMalloc(p, want * sizeof(T));
+    if (e == cudaSuccess) { *have = want; return true; }
+    cudaGetLastError();
+    zg_set_error("workspace of %zu bytes: %s", want * sizeof(T), cudaGetErrorString(e));
+    if (before && cudaMalloc(p, before * sizeof(T)) == cudaSuccess) *have = before;
+    return false;
+}
 bool zg_gemv_ws_reserve(ZgGemvWs* ws, size_t partial_elems, size_t counters, cudaStream_t st, size_t gemm_scratch_elems) {
-    if (gemm_scratch_elems > ws->gemm_scratch_elems) {
-        if (ws->gemm_scratch) { cudaStreamSynchronize(st); cudaFree(ws->gemm_scratch); ws->gemm_scratch = nullptr; }
-        ZG_CUDA_OK(cudaMalloc(&ws->gemm_scratch, gemm_scratch_elems * sizeof(float)));
-        ws->gemm_scratch_elems = gemm_scratch_elems;
-    }
-    if (partial_elems > ws->partials_elems) {
-        if (ws->partials) { cudaStreamSynchronize(st); cudaFree(ws->partials); ws->partials = nullptr; }
-        ZG_CUDA_OK(cudaMalloc(&ws->partials, partial_elems * sizeof(float)));
-        ws->partials_elems = partial_elems;
-    }
+    if (!grow(&ws->gemm_scratch, &ws->gemm_scratch_elems, gemm_scratch_elems, st) || !grow(&ws->partials, &ws->partials_elems, partial_elems, st)) return false;
     if (counters > ws->counters_n) {
-        if (ws->counters) { cudaStreamSynchronize(st); cudaFree(ws->counters); ws->counters = nullptr; }
-        ZG_CUDA_OK(cudaMalloc(&ws->counters, counters * sizeof(uint32_t)));
+        if (!grow(&ws->counters, &ws->counters_n, counters, st)) return false;
         ZG_CUDA_OK(cudaMemsetAsync(ws->counters, 0, counters * sizeof(uint32_t), st));
         ZG_CUDA_OK(cudaStreamSynchronize(st));
-        ws->counters_n = counters;
     }
     return true;
 }
@@ -1681,7 +1689,7 @@ static bool build_schedule(ZgCudaProgram* p) {
         if (!u.batched || u.entry_ops.empty() || p->ops[u.entry_ops[0]].tag != ZG_OP_ATTENTION || !zg_attention_prefill_ok(p->ops[u.entry_ops[0]])) continue;
         std::vector<const ZgOp*> ops;
         for (uint32_t i : u.entry_ops) ops.push_back(&p->ops[i]);
-        if (!zg_atc_program_plan(ops.data(), (uint32_t)ops.size(), p->buffer_elems.data(), &u.atc_plan)) continue;
+        if (!zg_atc_program_plan(p->ops, ops.data(), (uint32_t)ops.size(), p->buffer_elems.data(), &u.atc_plan)) continue;
         u.atc = true;
         u.atc_plan.map_off = atc_map.size();
         atc_map.insert(atc_map.end(), u.atc_plan.map.begin(), u.atc_plan.map.end());
@@ -1693,7 +1701,8 @@ static bool build_schedule(ZgCudaProgram* p) {
     if (!atc_map.empty()) {
         ZG_CUDA_OK(cudaMalloc(&p->d_atc_map, atc_map.size() * sizeof(uint32_t)));
         ZG_CUDA_OK(cudaMemcpy(p->d_atc_map, atc_map.data(), atc_map.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-        if (!zg_gemv_ws_reserve(&p->ws, 0, 0, p->ctx->stream, atc_scratch)) return false;
+        if (!zg_gemv_ws_reserve(&p->ws, 0, 0, p->ctx->stream, atc_scratch))       // no room for planes: the SIMT kernel needs none
+            for (auto& u : p->units) u.atc = false;
     }
     // single-op launches (profiling / eager per-op mode) of batched kinds need their own plain entries
     p->single_entry.assign(n, 0);
@@ -2144,6 +2153,7 @@ extern "C" uint64_t zg_cuda_program_stats(const ZgCudaProgram* p, int what) {
     switch (what) {
         case 5: return zg_dense_gemm_timeouts() + zg_split_gemm_timeouts() + zg_attention_tc_timeouts();
         case 6: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && op.u.seq.n[5] == ZG_W_BF16 && zg_seq_op_scratch_elems(op, p->buffers.data())) n++; return n; }
+        case 7: return p->ws.gemm_scratch_elems;
         case 0: return p->graph_kernels;
         case 1: return p->dec.valid ? p->dec_count : 0;
         case 2: return p->dec.valid ? p->dec.plan.n_layers : 0;

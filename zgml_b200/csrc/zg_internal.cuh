@@ -270,7 +270,7 @@ bool zg_launch_batch(const ZgOp& first, const ZgBatchEntry* d_entries, uint32_t 
 struct ZgAtcPlan { uint32_t count = 0, kv_items = 0, mask_items = 0, seq_q = 0, head = 0, tiles = 0; std::vector<uint32_t> map; size_t map_off = 0; };
 bool zg_attention_prefill_ok(const ZgOp& op);   // ops.cu: the layouts the prompt kernels take
 unsigned int zg_attention_tc_timeouts();
-bool zg_atc_program_plan(const ZgOp* const* ops, uint32_t count, const size_t* buffer_elems, ZgAtcPlan* plan);   // false: keep the SIMT kernel
+bool zg_atc_program_plan(const std::vector<ZgOp>& all, const ZgOp* const* ops, uint32_t count, const size_t* buffer_elems, ZgAtcPlan* plan);   // all: the program's ops.  false: keep the SIMT kernel
 size_t zg_atc_program_scratch_elems(const ZgAtcPlan& plan);
 bool zg_atc_program_launch(const ZgAtcPlan& plan, const ZgBatchEntry* d_entries, const uint32_t* d_map, const uint32_t* d_dyn, float* scratch, cudaStream_t st);
 uint32_t zg_attention_splits(const ZgOp& op, size_t k_buffer_elems, uint32_t count, int sm_count);
