@@ -1513,22 +1513,18 @@ __global__ void k_moe_down(float* __restrict__ dst, const float* __restrict__ sr
 // ── MOE_FFN, grouped form (prefill on bfloat16 sessions): the step's (token, choice) pairs are sorted by expert, the rows are gathered as bf16, and the
 // experts' products run as tiles of ONE tensor-core matmul for gate, up and activation and one for down (dense_gemm.cu), so an expert's weights are read
 // once per run of up to 256 rows instead of once per token ──
+constexpr uint32_t kMoeMinRun = 64;
 struct MoeLayout {          // offsets in f32 slots inside the op's scratch operand
-    uint32_t R, run, segments;   // (token, choice) pairs; rows of a run at most; runs of rows of one expert, at most
+    uint32_t R, experts;         // (token, choice) pairs; experts that can have any
     size_t seg, row_pair, pos_of_pair, xs, yb, z, total;
 };
 __host__ __device__ inline size_t up4(size_t n) { return (n + 3) & ~(size_t)3; }
 MoeLayout moe_layout(uint32_t T, uint32_t D, uint32_t ff, uint32_t E, uint32_t top) {
     MoeLayout L;
     L.R = T * top;
-    // Long runs read the weights least often; where they leave the GPU without a tile per SM, what counts is the time of a tile, and the runs are shorter
-    // (395 tokens, two of 4 experts of 368 x 392, 28 tiles: 41 us with runs of 256 rows, 27 with 64).
-    const uint32_t tiles = (ff + 127) / 128, experts = E < L.R ? E : L.R;
-    L.run = kExpertSegmentRows;
-    while (L.run > 64 && tiles * (experts + L.R / L.run) < 148) L.run /= 2;
-    L.segments = experts + L.R / L.run;
+    L.experts = E < L.R ? E : L.R;
     size_t o = 0;
-    L.seg = o; o = up4(o + (size_t)L.segments * (sizeof(ZgExpertSegment) / 4));
+    L.seg = o; o = up4(o + (size_t)(L.experts + L.R / kMoeMinRun) * (sizeof(ZgExpertSegment) / 4));
     L.row_pair = o; o = up4(o + L.R);
     L.pos_of_pair = o; o = up4(o + L.R);
     L.xs = o; o = up4(o + (size_t)L.R * D / 2);
@@ -1536,6 +1532,15 @@ MoeLayout moe_layout(uint32_t T, uint32_t D, uint32_t ff, uint32_t E, uint32_t t
     L.z = o; o = up4(o + (size_t)L.R * D);
     L.total = o;
     return L;
+}
+// Rows of a run at most.  Long runs read the weights least often; where they leave the GPU without a tile of gate and up per SM, what counts is the time of a
+// tile, and the runs are shorter (395 tokens, two of 4 experts of 368 x 392, 28 tiles: 41 us with runs of 256 rows, 27 with 64).  The down product takes the
+// same runs: chosen by the fewer tiles of the two, 1024 tokens of 4 experts of 256 x 2048 took 55 us instead of 70, but 300 tokens of 8 of 512 x 2048 41 instead of 35.
+// (A launch's choice: the layout has room for the shortest runs, whatever machine sizes the scratch.)
+uint32_t moe_run(const MoeLayout& L, uint32_t ff, uint32_t n_sm) {
+    uint32_t run = kExpertSegmentRows;
+    while (run > kMoeMinRun && (ff + 127) / 128 * (L.experts + L.R / run) < n_sm) run /= 2;
+    return run;
 }
 constexpr uint32_t kMoeMaxExperts = 1024;
 __global__ void __launch_bounds__(1024) k_moe_sort(const float* __restrict__ route, ZgExpertSegment* __restrict__ seg, int* __restrict__ row_pair,
@@ -2014,15 +2019,16 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             if (moe_grouped(s, bufs)) {
                 const MoeLayout L = moe_layout(T, D, ff, E, top);
                 float* sc = bufs[s.buf[4]];
+                const uint32_t run = moe_run(L, ff, zg_sm_count()), segments = L.experts + L.R / run;
                 ZgExpertSegment* seg = reinterpret_cast<ZgExpertSegment*>(sc + L.seg);
                 int* row_pair = reinterpret_cast<int*>(sc + L.row_pair);
                 int* pos_of_pair = reinterpret_cast<int*>(sc + L.pos_of_pair);
-                launch_pdl(k_moe_sort, dim3(1), dim3(1024), 0, st, bufs[s.buf[2]], seg, row_pair, pos_of_pair, L.R, E, L.segments, L.run);
+                launch_pdl(k_moe_sort, dim3(1), dim3(1024), 0, st, bufs[s.buf[2]], seg, row_pair, pos_of_pair, L.R, E, segments, run);
                 ZG_SEQ_CHECK();
                 launch_pdl(k_moe_gather, dim3(L.R), dim3(256), 0, st, reinterpret_cast<uint32_t*>(sc + L.xs), bufs[s.buf[1]], row_pair, D, top);
                 ZG_SEQ_CHECK();
-                if (!zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[0]), wptr<bf16>(bufs, s.buf[3], s.off[1]), E, sc + L.xs, L.R, seg, L.segments, sc + L.yb, ff, D, s.f[0], s.f[1], s.f[2], st) ||
-                    !zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[2]), nullptr, E, sc + L.yb, L.R, seg, L.segments, sc + L.z, D, ff, 0.0f, 0.0f, 0.0f, st)) return false;
+                if (!zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[0]), wptr<bf16>(bufs, s.buf[3], s.off[1]), E, sc + L.xs, L.R, seg, segments, sc + L.yb, ff, D, s.f[0], s.f[1], s.f[2], st) ||
+                    !zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[2]), nullptr, E, sc + L.yb, L.R, seg, segments, sc + L.z, D, ff, 0.0f, 0.0f, 0.0f, st)) return false;
                 launch_pdl(k_moe_combine, dim3(T), dim3(256), 0, st, bufs[s.buf[0]], bufs[s.buf[1]], sc + L.z, bufs[s.buf[2]], pos_of_pair, D, top);
                 ZG_SEQ_CHECK();
                 return true;
