@@ -855,16 +855,6 @@ k_attention_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     if (warp == 17) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(0u) : "memory");
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled() {
-    static const EncodeTiledFn fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess ? (EncodeTiledFn)f : (EncodeTiledFn)nullptr;
-    }();
-    return fn;
-}
 bool encode_plane(CUtensorMap* map, void* p, uint64_t width, uint64_t rows, uint32_t box_rows) {
     const cuuint64_t dims[2] = {width, rows}, stride[1] = {width * 2};
     const cuuint32_t box[2] = {64, box_rows}, one[2] = {1, 1};

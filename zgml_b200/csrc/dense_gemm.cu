@@ -9,15 +9,12 @@
 //   * 6-stage mbarrier ring (32 KB per stage): TMA warp -> MMA warp -> (tcgen05.commit) -> stage free.  Four epilogue warps
 //     read the accumulator (tcgen05.ld 32x32b), transpose 32 x 32 blocks through the idle stage memory, add the bias and
 //     write 128-byte row segments.
-//   * Every wait is bounded: a barrier that does not flip within ~1 s of polling raises a sticky device flag
+//   * Every wait is bounded: a barrier that does not flip within ~1 s of polling is counted
 //     (zg_dense_gemm_timeouts) and the CTA drains — its roles all give up the same way — frees its TMEM and returns.
 //
 // Used when the session keeps bfloat16 weights and M > 8 (decode rows stream the weights through the row kernels of
-// seqops.cu); float32 sessions keep the exact SIMT tile.
-#include "seq_common.cuh"
-
-#include <cuda.h>
-#include <cuda_bf16.h>
+// seqops.cu); float32 sessions' products of many rows are split_gemm.cu's.
+#include "split_tc.cuh"
 
 namespace {
 
@@ -27,34 +24,7 @@ constexpr uint32_t kStages = 6;
 constexpr uint32_t kThreads = 192;   // warp 0: TMA, warp 1: MMA + TMEM, warps 2-5: epilogue
 constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kSmem = kStages * kStage + 1024 + 256;
-constexpr uint32_t kSpinLimit = 1u << 22;
 
-__device__ unsigned int g_timeouts = 0;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// false: gave up (the flag is raised; the caller stops issuing work and falls through to the common exit)
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kSpinLimit; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    atomicAdd(&g_timeouts, 1u);
-    return false;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t c0, uint32_t c1, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
-}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t c0, uint32_t c1, uint32_t c2, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
@@ -70,31 +40,10 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
     return d;
 }
 
-// One lane of a converged warp.  The issuing warp walks its loop whole and lets the elected lane issue: addresses stay warp-uniform that way (inside a
-// single lane's branch an MMA of 128 x 128 x 16 took 130 clocks to issue; it executes in 64).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(p));
-    return p != 0;
-}
 // D[tmem] (+)= A[shared] B[shared], bf16
 __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(addr));
-}
-// every loaded register passes through the wait, so that nothing that reads them moves above it
-__device__ __forceinline__ void tmem_wait_ld16(uint32_t (&v)[16]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
 }
 // f32 rows -> dense bf16 [Mp][Kp] (zero padding), two k per thread
 // (ctl: the rows are those of a per-sequence state buffer, `slot_stride` elements per slot; the slot is the control word's)
@@ -189,8 +138,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 const uint32_t s = kt % kStages, ph = (kt / kStages) & 1;
                 if (!mbar_wait(empty + 8 * s, ph ^ 1)) break;
                 mbar_expect_tx(full + 8 * s, kStage);
-                tma_load_2d(base + s * kStage, &tmap_a, kt * BK, head * p.a_rows + tile_m * BM, full + 8 * s);
-                tma_load_2d(base + s * kStage + kTileA, &tmap_b, kt * BK, head * p.N + tile_n * BN, full + 8 * s);
+                tma_2d(base + s * kStage, &tmap_a, kt * BK, head * p.a_rows + tile_m * BM, full + 8 * s);
+                tma_2d(base + s * kStage + kTileA, &tmap_b, kt * BK, head * p.N + tile_n * BN, full + 8 * s);
             }
         }
     } else if (warp == 1) {
@@ -211,7 +160,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     } else {
         // ── epilogue: warp w may touch TMEM lanes 32 (w % 4) .. + 31 ──
         const uint32_t ew = warp - 2, quarter = warp & 3;
-        const bool ok = mbar_wait(tmem_full, 0);
+        const bool ok = mbar_wait(tmem_full, 0);       // (what the other roles gave up on does not arrive here either)
+        if (!ok && lane == 0) count_timeout();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t m_base = tile_m * BM + quarter * 32;
         uint4* tb = reinterpret_cast<uint4*>(dsm_raw + (base - smem_u32(dsm_raw)) + ew * (32 * 36 * 4));   // the stages are idle now
@@ -299,7 +249,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 // once per run, and what is computed for padding is less than 16 rows (whole 128-row tiles of tokens were a third padding at 16 experts of 128 rows each,
 // and read the weights again for it).  DUAL: two weight matrices against the same rows, gate and up, and out = bf16(act(gate) up), so that neither
 // product goes through memory.
-// Bound by the stream of weights.  1024 tokens, two of 16 experts, 2048 x 2048, cold: gate, up and activation 68 us (98 as two products and a pass of
+// The stream of weights sets its floor (4.1 of 6.5 TB/s at 1024 tokens: 256 tiles on 148 SMs are two uneven rounds, each tile's ends exposed).  1024 tokens, two of 16 experts, 2048 x 2048, cold: gate, up and activation 68 us (98 as two products and a pass of
 // their own over whole tiles), down 40 us (42); the op 124 us (171), 44 tokens on one of 4 experts of 1696 x 1088 29 us (60).
 constexpr uint32_t kExpertThreads = 320;          // warp 0: TMA, warp 1: MMA + TMEM, warps 2-9: epilogue
 constexpr uint32_t kExpertRows = 32;              // rows of x per copy
@@ -348,7 +298,7 @@ k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
                 mbar_expect_tx(full + 8 * s, stage_bytes);
                 tma_load_3d(at, &tmap_w, kt * BK, f0, (uint32_t)seg.expert, full + 8 * s);
                 if (DUAL) tma_load_3d(at + kTileA, &tmap_w2, kt * BK, f0, (uint32_t)seg.expert, full + 8 * s);
-                for (uint32_t c = 0; c < copies; c++) tma_load_2d(at + kWeights + c * (kExpertRows * BK * 2), &tmap_x, kt * BK, (uint32_t)seg.start + c * kExpertRows, full + 8 * s);
+                for (uint32_t c = 0; c < copies; c++) tma_2d(at + kWeights + c * (kExpertRows * BK * 2), &tmap_x, kt * BK, (uint32_t)seg.start + c * kExpertRows, full + 8 * s);
                 if (++s == stages) { s = 0; ph ^= 1; }
             }
         }
@@ -376,15 +326,16 @@ k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
     } else {
         // TMEM lane = output column of the CTA's 128, TMEM column = row of the run; the two warps of a quarter take 16 rows each in turn
         const uint32_t quarter = warp & 3, half = (warp - 2) >> 2, f = f0 + quarter * 32 + lane;
-        const bool ok = mbar_wait(tmem_full, 0);
+        const bool ok = mbar_wait(tmem_full, 0);       // (what the other roles gave up on does not arrive here either)
+        if (!ok && lane == 0) count_timeout();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (uint32_t c0 = 16 * half; __all_sync(0xffffffffu, ok) && c0 < n; c0 += 32) {
             uint32_t g[16], u[16];
             const uint32_t addr = tmem + ((quarter * 32) << 16) + c0;
-            tmem_ld16(addr, g);
-            if (DUAL) tmem_ld16(addr + kAccCols, u);
-            tmem_wait_ld16(g);
-            if (DUAL) tmem_wait_ld16(u);
+            tmem_ld(addr, g);
+            if (DUAL) tmem_ld(addr + kAccCols, u);
+            tmem_wait_ld(g);
+            if (DUAL) tmem_wait_ld(u);
 #pragma unroll
             for (uint32_t j = 0; j < 16; j++) {
                 if (c0 + j >= n || f >= p.N) continue;
@@ -402,9 +353,6 @@ k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(DUAL ? 2 * kAccCols : kAccCols) : "memory");
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn g_encode = nullptr;
 bool g_attr_set = false;
 constexpr int kActs = 7;
@@ -420,13 +368,8 @@ GemmKernel batched_kernel(uint32_t act) {      // the activations a batched prod
 
 bool prepare() {
     if (!g_encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn) {
-            zg_set_error("cuTensorMapEncodeTiled entry point not available");
-            return false;
-        }
-        g_encode = (EncodeTiledFn)fn;
+        g_encode = encode_tiled();
+        if (!g_encode) { zg_set_error("cuTensorMapEncodeTiled entry point not available"); return false; }
     }
     if (!g_attr_set) {
         cudaError_t e = cudaFuncSetAttribute(k_expert_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExpertSmem);
@@ -449,11 +392,7 @@ bool zg_dense_gemm_usable(const void* w_bf16, uint32_t M, uint32_t N, uint32_t K
 size_t zg_dense_gemm_scratch_elems(uint32_t M, uint32_t K) {
     return (size_t)((M + BM - 1) / BM * BM) * ((K + BK - 1) / BK * BK) / 2;
 }
-unsigned int zg_dense_gemm_timeouts() {
-    unsigned int v = 0;
-    cudaMemcpyFromSymbol(&v, g_timeouts, sizeof(v));
-    return v;
-}
+unsigned int zg_dense_gemm_timeouts() { return tc_timeouts(); }
 
 bool zg_dense_gemm_launch(const void* w_bf16, const void* bias_bf16, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K,
                           uint32_t src_rs, uint32_t dst_rs, float* scratch, cudaStream_t st, uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs,

@@ -379,16 +379,11 @@ qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
                                 asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(slot_u32 + sc_off + r * RB));
                                 sc = __half2float(__ushort_as_half(h));
                             }
-#pragma unroll
-                            for (int m = 0; m < XR; m++) {
-                                if (XR == 1 || (uint32_t)m < p.M) {
-                                    const uint32_t F = __float_as_uint(fmaf(sc, __uint_as_float(lds32(xa + r * ZG_KR * 4 + m * xs_row_bytes)), 1.5f));
-                                    const uint32_t pa = planes + lane + (r * XR + m) * kPlaneRow;
-                                    sts8(pa, F);
-                                    sts8(pa + 32, F >> 8);
-                                    sts8(pa + 64, F >> 16);
-                                }
-                            }
+                            const uint32_t F = __float_as_uint(fmaf(sc, __uint_as_float(lds32(xa + r * ZG_KR * 4)), 1.5f));
+                            const uint32_t pa = planes + lane + r * kPlaneRow;
+                            sts8(pa, F);
+                            sts8(pa + 32, F >> 8);
+                            sts8(pa + 64, F >> 16);
                         }
                     }
                 } else {

@@ -1,4 +1,4 @@
-// What the kernels that split f32 operands into 16-bit parts for tcgen05 share: barriers, TMA, descriptors, MMA issue, TMEM access, and the splits.
+// What the tcgen05 kernels share: barriers, TMA, descriptors, MMA issue, TMEM access, and for those over f32 operands their splits into 16-bit parts.
 //
 // Pairs of half precision: x = hi + lo: hi = f16(x s), lo = f16(x s - hi), with s a power of two that brings the largest magnitude of a row or tile to
 // [2^14, 2^15).  hi and lo together keep 22 to 24 significant bits of everything within 2^-17 of that maximum; what is smaller loses bits below 2^-39 of it.
@@ -17,6 +17,16 @@ __device__ unsigned int g_tc_timeouts = 0;    // waits of this file's kernels th
     unsigned int v = 0;
     cudaMemcpyFromSymbol(&v, g_tc_timeouts, sizeof(v));
     return v;
+}
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+[[maybe_unused]] EncodeTiledFn encode_tiled() {      // null: not available
+    static const EncodeTiledFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess ? (EncodeTiledFn)f : (EncodeTiledFn)nullptr;
+    }();
+    return fn;
 }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
