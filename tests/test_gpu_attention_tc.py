@@ -200,6 +200,52 @@ def test_batched_heads_with_their_own_masks_and_a_refreshed_length(cuda_backend)
     cuda_backend.free_program(handle)
 
 
+@pytest.mark.parametrize("shape", [
+    dict(T=200, pos=1500, H=8, G=4, dk=128, dv=128, size=300, pool=7), dict(T=64, pos=3000, H=8, G=2, dk=192, dv=64, size=100, pool=3, cap=4.0),
+    dict(T=16, pos=6000, H=8, G=8, dk=128, dv=128, size=200, pool=4, sink=True), dict(T=130, pos=0, H=16, G=4, dk=64, dv=100, size=64, pool=1, sink=True, cap=3.0),
+    dict(T=150, pos=1024, H=8, G=8, dk=96, dv=64, size=513, pool=5), dict(T=200, pos=1500, H=8, G=4, dk=128, dv=128, size=300, pool=7, bad="key"),
+    dict(T=200, pos=1500, H=8, G=4, dk=128, dv=128, size=300, pool=7, bad="value")], ids=lambda d: " ".join(f"{k}{v}" for k, v in d.items() if k in ("T", "pos", "dk", "pool", "bad")))
+def test_pooled_blocks_of_many_rows(cuda_backend, shape):
+    """Mask "pooled": block means and window positions that share a key tile, a ring that wraps, the second slot, key shares, 64-key tiles; a block that holds no
+    number leaves the rows that do not see it exact."""
+    from zgml_b200 import DeviceBuffer, DeviceOp, ExternBuffer, abi
+    T, pos, H, G, dk, dv, size, pool = (shape[k] for k in ("T", "pos", "H", "G", "dk", "dv", "size", "pool"))
+    cap, bad = shape.get("cap", 0.0), shape.get("bad")
+    r = np.random.default_rng(T + pos)
+    n, width, R = pos + T, G * (dk + dv), size - 1 + T + 5
+    NB = n // pool
+    kv = r.standard_normal((n, width)).astype(np.float32)
+    means = kv[:NB * pool].astype(np.float64).reshape(NB, pool, width).mean(1).astype(np.float32) * np.float32(pool ** 0.5)
+    broken = (pos + T // 2 - size) // pool                             # seen from the middle of the step on
+    sees = np.arange(pos, n) + 1 - size >= (broken + 1) * pool
+    if bad:
+        means[broken, slice(0, G * dk) if bad == "key" else slice(G * dk, width)] = np.nan
+    cache, pooled = np.zeros((2, R, width), np.float32), np.zeros((2, NB, width), np.float32)
+    last = np.arange(max(0, n - R), n)
+    cache[1][last % R] = kv[last]
+    pooled[1] = means
+    bc, bp = DeviceBuffer(cuda_backend, cache.nbytes, zero=False), DeviceBuffer(cuda_backend, pooled.nbytes, zero=False)
+    bc.upload(cache)
+    bp.upload(pooled)
+    q = r.standard_normal((T, H * dk)).astype(np.float32)
+    sk = r.standard_normal(H).astype(np.float32)
+    op = DeviceOp.cached_attention(0, 1, 2, 2, 3, 0, 0, G * dk, T, H, G, 1, dk, dv, H * dk, width, width, R, dk ** -0.5, mask="pooled", mask_size=size, pooled=4, pool=pool, pool_rows=NB, softcap=cap,
+                                   **(dict(sink=5, sink_wdt=abi.W_F32) if shape.get("sink") else {}))
+    got = run(cuda_backend, [op], [T * H * dv, q.size, bc.elems, 8 + T, bp.elems, H], [(1, q), (3, ctl_words(pos, 1)), (5, sk)], 0, (T, H, dv), [ExternBuffer(2, bc), ExternBuffer(4, bp)])
+    bc.free()
+    bp.free()
+    p = np.arange(pos, n)[:, None]
+    first = max(0, pos + 1 - size)
+    j, b = np.arange(first, n), np.arange(NB)
+    seen = np.concatenate([(b + 1) * pool <= p + 1 - size, (j <= p) & (j > p - size)], 1)
+    rows = np.concatenate([np.nan_to_num(means, nan=0.0), kv[j]]).astype(np.float64)
+    want = np.stack([reference(q[:, h * dk:(h + 1) * dk].astype(np.float64), rows[:, h * G // H * dk:(h * G // H + 1) * dk], rows[:, G * dk + h * G // H * dv:G * dk + (h * G // H + 1) * dv], seen,
+                               dk ** -0.5, cap, sink=sk[h] if shape.get("sink") else None) for h in range(H)], 1)
+    clean = ~sees if bad else np.ones(T, bool)
+    assert 0 < clean.sum() and close(got[clean], want[clean])
+    assert not bad or not np.isfinite(got[~clean]).any()
+
+
 def heads_in_a_slab(be, r, T, S, dh, G, H, offs, kv, compile_kv=None):
     """H heads over G slabs of S rows (head h: those that start at row offs[h]) in one buffer, kv[h] keys each -> (got, want, handle, refresh)."""
     from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO
