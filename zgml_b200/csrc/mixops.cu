@@ -483,7 +483,10 @@ __global__ void __launch_bounds__(kCtThreads) k_cached_attention_tiled(CaArgs a,
 // max = -inf and weighs nothing (its output may be anything)
 // (a: for the sink, the output scale and the row layout of dst; HM = H * maps)
 constexpr int kMergeCols = 64, kMergeGroups = 8;        // groups of 64 threads that each add up an eighth of the shares
-__global__ void __launch_bounds__(kMergeCols * kMergeGroups, 4) k_cached_attention_merge(CaArgs a, const float* __restrict__ part, uint32_t dv, uint32_t splits,
+// BLOCKS: CTAs that an SM is to hold.  Four where there are many rows of few shares (256 tokens of 16 heads after 2000: the op 68 us, with three 75); where there are few
+// rows of up to 160 shares the loads in flight count, which three leave the registers for (one token over 8192 latents: the op 33 us, with four 35).
+template <int BLOCKS>
+__global__ void __launch_bounds__(kMergeCols * kMergeGroups, BLOCKS) k_cached_attention_merge(CaArgs a, const float* __restrict__ part, uint32_t dv, uint32_t splits,
                                                                 uint32_t wkind) {
     pdl_enter();
     __shared__ float w[kCaMaxShares], sums[kMergeGroups][kMergeCols];
@@ -1181,14 +1184,14 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
 #undef ZG_CF
                 if (S > 1) {
                     ZG_SEQ_CHECK();
-                    launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
+                    launch_pdl(k_cached_attention_merge<3>, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
                 }
             } else if (aligned && scratch && ca_tensor(s)) {
                 uint32_t S = 1;
                 float* part = nullptr;
                 if (!zg_attention_tc_launch(ca_shape(s), &a, scratch, sm_count(), st, &S, &part)) return false;
                 if (S == 1) return true;
-                launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
+                launch_pdl(k_cached_attention_merge<4>, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
             } else if (aligned) {
                 const uint32_t S = scratch && !ca_tensor(s) ? ca_splits(s) : 1;
                 float* part = S > 1 ? scratch : nullptr;
@@ -1207,7 +1210,7 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
                 }
                 if (S > 1) {
                     ZG_SEQ_CHECK();
-                    launch_pdl(k_cached_attention_merge, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
+                    launch_pdl(k_cached_attention_merge<4>, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);
                 }
             } else {
                 const uint32_t warps = 4, items = a.T * a.H * a.maps;
