@@ -106,6 +106,17 @@ template <> __device__ __forceinline__ void wld_vec<float>(const float* p, float
     const float4 v = *reinterpret_cast<const float4*>(p);
     out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
 }
+// two values -> their three bfloat16 parts, packed
+__device__ __forceinline__ void split3(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    uint32_t* const to[3] = {&p0, &p1, &p2};
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+        const float2 f = __bfloat1622float2(h);
+        a -= f.x; b -= f.y;
+        *to[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+}
 template <typename WT> const WT* wptr(float* const* bufs, uint32_t b, uint32_t off) { return reinterpret_cast<const WT*>(bufs[b]) + off; }
 
 

@@ -6,7 +6,7 @@
 //
 // Per-sequence state lives in external program buffers indexed by the state slot of the control buffer; the position of
 // the step's first token comes from the same place, so a captured graph replays unchanged from step to step.
-#include "seq_common.cuh"
+#include "split_tc.cuh"
 
 #include <stdlib.h>
 
@@ -1046,24 +1046,31 @@ __global__ void __launch_bounds__(kDeltaThreads) k_delta_rule(
         if (live && row < dim) S_g[(size_t)row * vdim + col] = S[i];
     }
 }
-// Prefill form of DELTA_RULE (kDeltaPrepMinTokens or more tokens): four tokens at a time.  With D_l the decay of token l of a block (a diagonal) and S the
+// Prefill form of DELTA_RULE (kDeltaPrepMinTokens or more tokens): chunks of 16 tokens.  With D_l the decay of token l of a chunk (a diagonal) and S the
 // state before it, every token's two products follow from products with S itself:
-//   S_j^T x = S^T (D_1 .. D_j x) + sum_{i <= j} (x^T D_{i+1} .. D_j k_i) u_i,
-// so the eight products of a block with the state are independent, are reduced together, and what remains between the tokens of a block is a
-// triangular solve of four scalars per value column:
-//   u_j = beta_j (v_j - A_j^T S - sum_{i < j} ckk_ij u_i),   o_j = Q_j^T S + sum_{i <= j} cqk_ij u_i,   S <- Gamma S + sum_j B_j u_j^T.
-// Only products of decays occur (nothing is divided by one), so the form is as sound as token by token for any decay.  k_delta_prepare (one warp per
-// (block, head)) leaves per block the vectors [A_1 .. A_4 | Q_1 .. Q_4 | B_1 .. B_4 | Gamma] and the scalars [beta (4) | ckk (4 x 4) | cqk (4 x 4)], zero
-// where i does not precede j, laid out [head][block]; a plain accumulation (u = v) has no A and no solve.  k_delta_walk streams them into shared memory
-// with cp.async, double buffered.
-// A warp owns two value columns; a lane holds R key rows of both.  What a thread reads of the prepared vectors per column it owns bounds the kernel
-// where a column has few threads (one thread per 16 rows of one column: 832 clocks of shared-memory reads per block and SM), the latency of a block
-// where a warp has many columns (four: 1280 clocks per block, 29 % of the issue slots).  The 16 sums (8 products, 2 columns) are reduced over the
-// lanes by halving what is left each time, and end one per lane: lane (column, k or q, token).
+//   S_j^T x = S^T (D_1 .. D_j x) + sum_{i <= j} (x^T D_{i+1} .. D_j k_i) u_i,   u_j = beta_j (v_j - A_j^T S - sum_{i < j} ckk_ij u_i).
+// Both are affine in S, so the triangular solve is done ahead, on the vectors instead of on the state's columns:
+//   u_j = Vt_j - W_j^T S,   W_j = beta_j (A_j - sum_{i < j} ckk_ij W_i),   Vt_j = beta_j (v_j - sum_{i < j} ckk_ij Vt_i),
+//   o_j = Vo_j + Q'_j^T S,  Q'_j = Q_j - sum_{i <= j} cqk_ij W_i,          Vo_j = sum_{i <= j} cqk_ij Vt_i,   S <- Gamma S + sum_j B_j u_j^T.
+// k_delta_prepare does that for all chunks at once; what is left in sequence, k_delta_walk, is two small products per chunk.  Only products of decays
+// occur (nothing is divided by one), so the form is as sound as token by token for any decay, and a token's row of any term depends on the tokens up to
+// it alone.  A plain accumulation (u = v) has no W.
+// Steps are walked in passes of at most kDeltaScratch bytes of prepared vectors: they stay in the L2 between the two kernels.
 constexpr int kDeltaPrepMinTokens = 16;
-constexpr int kWalkThreads = 256, kWalkMaxDim = 512, kWalkBlock = 4, kWalkScalars = 36, kWalkCols = 2;
-static uint32_t delta_walk_rows(uint32_t dim) { return dim <= 64 ? 2 : dim <= 128 ? 4 : dim <= 256 ? 8 : 16; }      // key rows per lane
-__host__ __device__ constexpr uint32_t delta_block_elems(uint32_t dpad, bool plain) { return ((plain ? 2 : 3) * kWalkBlock + 1) * dpad + kWalkScalars; }
+constexpr uint32_t kWalkChunk = 16, kWalkMaxDim = 512, kWalkCols = 16;
+constexpr size_t kDeltaScratch = 64u << 20;
+// key rows a chunk's vectors are padded to: sixteen per warp and slice of the walk
+__host__ __device__ constexpr uint32_t delta_rows(uint32_t dim) { return dim <= 64 ? 64 : dim <= 128 ? 128 : dim <= 256 ? 256 : 512; }
+// a chunk's vectors as the walk stages them: [W | Q'] of dpad + 8 rows each (the lanes of a read lie in different banks), B as [row][16 tokens], Gamma ...
+__host__ __device__ constexpr uint32_t delta_vec_elems(uint32_t dpad, bool plain) { return (plain ? 1 : 2) * kWalkChunk * (dpad + 8) + (kWalkChunk + 1) * dpad; }
+// ... and with [Vt | Vo] of 16 tokens and 16 value columns at a time behind them, in the order of the accumulators that hold such a square
+__host__ __device__ constexpr size_t delta_chunk_elems(uint32_t dpad, bool plain, uint32_t vdim) { return delta_vec_elems(dpad, plain) + (size_t)(vdim + kWalkCols - 1) / kWalkCols * 512; }
+__host__ __device__ constexpr uint32_t delta_square(uint32_t tok, uint32_t col) { return (tok >> 3) * 128 + ((col & 7) * 4 + ((tok >> 1) & 3)) * 4 + (col >> 3) * 2 + (tok & 1); }
+static uint32_t delta_pass_chunks(uint32_t T, uint32_t H, uint32_t dim, uint32_t vdim, bool plain) {
+    const size_t one = delta_chunk_elems(delta_rows(dim), plain, vdim) * H * sizeof(float), most = kDeltaScratch / one;
+    const uint32_t chunks = (T + kWalkChunk - 1) / kWalkChunk;
+    return (uint32_t)(most < 4 ? chunks < 4 ? chunks : 4 : most < chunks ? most : chunks);
+}
 // N values in every lane -> the total of value lane % N
 template <int N>
 __device__ __forceinline__ float reduce_scatter(float (&v)[N], uint32_t lane) {
@@ -1080,233 +1087,417 @@ __device__ __forceinline__ float reduce_scatter(float (&v)[N], uint32_t lane) {
     for (int o = N; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
     return v[0];
 }
-template <typename WT, int R>
-__global__ void k_delta_prepare(float* __restrict__ prep, const float* __restrict__ qkv, const float* __restrict__ betab, const float* __restrict__ ab,
-                                const WT* __restrict__ wts, uint32_t T, uint32_t H, uint32_t G, uint32_t dim, uint32_t q_off,
-                                uint32_t k_off, uint32_t beta_off, uint32_t A_off, uint32_t dt_off, uint32_t qkv_rs, uint32_t beta_rs, uint32_t a_rs,
-                                float unit_eps, float q_scale, uint32_t form, float inv_tau, uint32_t u_off) {
-    pdl_enter();
-    constexpr int B = kWalkBlock;
-    constexpr uint32_t dpad = 32 * R;
+// One CTA per (chunk, head): units, scales and decays into shared memory; the 256 products between the tokens (136 q k, 120 k k), a warp for two of the
+// tokens that wrote, four later tokens at a time; then a thread for a column of [A | V], whose solves are alike.  Loops are kept rolled where the data
+// allows it: a straight line of 5000 instructions took 88 us where this takes 43 (1024 tokens, 16 heads of 128 x 128, launches alone): every CTA fetched it anew.
+constexpr uint32_t kDeltaPrepThreads = 256;
+constexpr uint32_t delta_prep_smem(uint32_t dpad) { return (3 * kWalkChunk + 2) * (dpad + 4) * 4; }
+template <typename WT>
+__global__ void __launch_bounds__(kDeltaPrepThreads, 2) k_delta_prepare(float* __restrict__ prep, const float* __restrict__ qkv, const float* __restrict__ betab, const float* __restrict__ ab,
+                                const WT* __restrict__ wts, uint32_t T, uint32_t H, uint32_t G, uint32_t dim, uint32_t vdim, uint32_t dpad, uint32_t q_off,
+                                uint32_t k_off, uint32_t v_off, uint32_t beta_off, uint32_t A_off, uint32_t dt_off, uint32_t qkv_rs, uint32_t beta_rs, uint32_t a_rs,
+                                float unit_eps, float q_scale, uint32_t form, float inv_tau, uint32_t u_off, uint32_t early) {
+    if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr uint32_t C = kWalkChunk;
+    const uint32_t NT = blockDim.x, warps = NT >> 5;                 // 4 or 8 warps
+    extern __shared__ __align__(16) float sm[];
+    __shared__ __align__(16) float qk[C][C], kk[C][C], scale[2 * C], beta[C];      // [j][i]
     const bool plain = form & kDeltaPlain, head_decay = form & kDeltaHeadDecay, bonus = form & kDeltaBonus;
-    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31, blocks = (T + B - 1) / B;
-    if (w >= blocks * H) return;
-    const uint32_t b = w / H, h = w % H, kv = h / (H / G), n = min((uint32_t)B, T - b * B);
-    const float* qr = qkv + (size_t)b * B * qkv_rs + q_off + (size_t)kv * dim;
-    const float* kr = qkv + (size_t)b * B * qkv_rs + k_off + (size_t)kv * dim;
-    const float* ar = ab + (size_t)b * B * a_rs + (head_decay ? (size_t)h : (size_t)h * dim);
-    float k[B][R], q[B][R], D[B][R];                                 // every load in flight at once
-#pragma unroll
-    for (int j = 0; j < B; j++)
-#pragma unroll
-        for (int i = 0; i < R; i++) {
-            const uint32_t c = lane + 32 * i;
-            const bool on = c < dim && (uint32_t)j < n;              // tokens past the step's end: nothing is written, nothing decays
-            k[j][i] = on ? kr[(size_t)j * qkv_rs + c] : 0.0f;
-            q[j][i] = on ? qr[(size_t)j * qkv_rs + c] : 0.0f;
-            D[j][i] = on ? ar[(size_t)j * a_rs + (head_decay ? 0 : c)] : 0.0f;
-        }
-    float bias[R], own[R];
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-        const uint32_t c = lane + 32 * i;
-        bias[i] = c < dim ? wld(wts, (size_t)dt_off + (head_decay ? (size_t)h : (size_t)h * dim + c)) : 0.0f;
-        own[i] = bonus && c < dim ? wld(wts, (size_t)u_off + (size_t)h * dim + c) : 1.0f;
+    const uint32_t h = blockIdx.x, b = blockIdx.y, kv = h / (H / G), n = min(C, T - b * C), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, dp = dpad + 4;
+    float* sk = sm;                                                  // [token][dp]
+    float* sq = sk + C * dp;
+    float* sd = sq + C * dp;
+    float* sbias = sd + C * dp;
+    float* sown = sbias + dp;
+    const float* row0 = qkv + (size_t)b * C * qkv_rs;
+    const float* ar = ab + (size_t)b * C * a_rs + (head_decay ? (size_t)h : (size_t)h * dim);
+    for (uint32_t c = tid; c < dpad; c += NT) {
+        sbias[c] = c < dim ? wld(wts, (size_t)dt_off + (head_decay ? (size_t)h : (size_t)h * dim + c)) : 0.0f;
+        sown[c] = bonus && c < dim ? wld(wts, (size_t)u_off + (size_t)h * dim + c) : 1.0f;
     }
     const float Ah = (form & (kDeltaSigmoidDecay | kDeltaExpDecay)) ? 0.0f : expf(wld(wts, (size_t)A_off + h));
-    const float beta = plain || lane >= n ? 0.0f : betab[((size_t)b * B + lane) * beta_rs + beta_off + h];
-    float scale = (lane & 4) ? 1.0f : q_scale;                       // lane j: of q_j, lane 4 + j: of k_j
-    if (!plain) {
-        float sq[2 * B];
+    if (tid < C) beta[tid] = plain || tid >= n ? 0.0f : sigmoidf_(betab[((size_t)b * C + tid) * beta_rs + beta_off + h]);
+    // tokens past the step's end: nothing is written, nothing decays
+    for (uint32_t j0 = warp; j0 < C; j0 += 2 * warps) {              // tokens j0 and j0 + warps
+        float sums[4] = {};                                          // q q of the two, k k
+        for (uint32_t c0 = 0; c0 < dpad; c0 += 128) {
+            float x[2][3][4];
 #pragma unroll
-        for (int j = 0; j < B; j++) {
-            float qq = 0.0f, kk = 0.0f;
+            for (int l = 0; l < 2; l++)
 #pragma unroll
-            for (int i = 0; i < R; i++) { qq = fmaf(q[j][i], q[j][i], qq); kk = fmaf(k[j][i], k[j][i], kk); }
-            sq[j] = qq; sq[B + j] = kk;
+                for (int i = 0; i < 4; i++) {
+                    const uint32_t c = c0 + lane + 32 * i, j = j0 + l * warps;
+                    const bool on = c < dim && j < n;
+                    const float* r = row0 + (size_t)j * qkv_rs + (size_t)kv * dim + c;
+                    x[l][0][i] = on ? r[q_off] : 0.0f;
+                    x[l][1][i] = on ? r[k_off] : 0.0f;
+                    x[l][2][i] = on ? ar[(size_t)j * a_rs + (head_decay ? 0 : c)] : 0.0f;
+                }
+#pragma unroll
+            for (int l = 0; l < 2; l++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const uint32_t c = c0 + lane + 32 * i, at = (j0 + l * warps) * dp + c;
+                    sums[l] = fmaf(x[l][0][i], x[l][0][i], sums[l]);
+                    sums[2 + l] = fmaf(x[l][1][i], x[l][1][i], sums[2 + l]);
+                    if (c < dpad) { sq[at] = x[l][0][i]; sk[at] = x[l][1][i]; sd[at] = x[l][2][i]; }
+                }
         }
-        scale /= sqrtf(reduce_scatter<2 * B>(sq, lane) + unit_eps);
-    }
-#pragma unroll
-    for (int j = 0; j < B; j++) {
-        const float qn = __shfl_sync(0xffffffffu, scale, j), kn = __shfl_sync(0xffffffffu, scale, B + j);
-#pragma unroll
-        for (int i = 0; i < R; i++) {
-            k[j][i] *= kn; q[j][i] *= qn;
-            if (i && head_decay) D[j][i] = D[j][0];                  // one decay for all rows (what lies past `dim` is zero, whatever its decay)
-            else D[j][i] = lane + 32 * i < dim && (uint32_t)j < n ? delta_decay(D[j][i] + bias[i], Ah, form, inv_tau) : 1.0f;
-        }
-    }
-    float* P = prep + ((size_t)h * blocks + b) * delta_block_elems(dpad, plain);
-    float* PQ = P + (plain ? 0 : B) * dpad;
-    float* PB = PQ + B * dpad;
-    float c[16] = {};                                                // cqk_ij at j (j + 1) / 2 + i, ckk_ij at 10 + j (j - 1) / 2 + i
-#pragma unroll
-    for (int e = 0; e < R; e++) {
-        const uint32_t at = lane + 32 * e;
-        float g = 1.0f;
-#pragma unroll
-        for (int j = 0; j < B; j++) {
-            const float before = g;
-            g *= D[j][e];
-            if (!plain) P[j * dpad + at] = g * k[j][e];
-            PQ[j * dpad + at] = (bonus ? before : g) * q[j][e];       // the bonus form reads the state before the token decays it
-        }
-        PB[B * dpad + at] = g;
-        float s = 1.0f;
-#pragma unroll
-        for (int j = B - 1; j >= 0; j--) { PB[j * dpad + at] = s * k[j][e]; s *= D[j][e]; }
-#pragma unroll
-        for (int i = 0; i < B; i++) {
-            float& self = c[i * (i + 1) / 2 + i];
-            self = fmaf(q[i][e] * own[e], k[i][e], self);
-            float d = k[i][e];                                       // what token i wrote, as the later tokens find it
-#pragma unroll
-            for (int j = i + 1; j < B; j++) {
-                float& qk = c[j * (j + 1) / 2 + i];
-                if (bonus) qk = fmaf(q[j][e], d, qk);
-                d *= D[j][e];
-                if (!bonus) qk = fmaf(q[j][e], d, qk);
-                if (!plain) { float& kk = c[10 + j * (j - 1) / 2 + i]; kk = fmaf(k[j][e], d, kk); }
-            }
+        const float total = reduce_scatter<4>(sums, lane);           // lane l: q of token j0 + l warps, lane 2 + l: k
+        if (lane < 4) {
+            const float own = lane < 2 ? q_scale : 1.0f;
+            scale[(lane & 2) * 8 + j0 + (lane & 1) * warps] = plain ? own : own / sqrtf(total + unit_eps);
         }
     }
-    float* sc = PB + (B + 1) * dpad;
-    if (lane < (uint32_t)B) sc[lane] = plain || lane >= n ? 0.0f : sigmoidf_(beta);
-    const uint32_t cj = (lane >> 2) & 3, ci = lane & 3;               // lane 4 j + i: ckk_ij, lane 16 + 4 j + i: cqk_ij
-    const float total = reduce_scatter<16>(c, lane);
-    const float mine = __shfl_sync(0xffffffffu, total, lane < 16 ? 10 + cj * (cj - 1) / 2 + ci : cj * (cj + 1) / 2 + ci);
-    sc[B + lane] = (lane < 16 ? ci < cj : ci <= cj) ? mine : 0.0f;
-}
-__device__ __forceinline__ void cp_async16(float* smem_dst, const float* gmem_src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gmem_src) : "memory");
-}
-template <int R, bool PLAIN>                       // key rows per lane
-__global__ void __launch_bounds__(kWalkThreads) k_delta_walk(float* __restrict__ dst, const float* __restrict__ qkv, const float* __restrict__ prep,
-                                                               float* __restrict__ state, const float* __restrict__ ctl, uint32_t T, uint32_t H,
-                                                               uint32_t dim, uint32_t vdim, uint32_t v_off, uint32_t qkv_rs, uint32_t dst_rs) {
-    pdl_enter();
-    extern __shared__ __align__(16) float sm[];
-    constexpr int B = kWalkBlock, C = kWalkCols, VR = R < 4 ? R : 4, NG = R / VR, Q = PLAIN ? 0 : B, W = Q + B;      // vectors before Q's and before B's
-    constexpr uint32_t dpad = 32 * R, block_elems = delta_block_elems(dpad, PLAIN), tile_blocks = kDeltaTile / B, tile_elems = tile_blocks * block_elems;
-    const uint32_t h = blockIdx.y, blocks = (T + B - 1) / B, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t col0 = (blockIdx.x * (kWalkThreads / 32) + warp) * C;                     // the warp's first column
-    const uint32_t slot = (uint32_t)ctl_word(ctl, ZG_CTL_SLOT);
-    float* S_g = state + (((size_t)slot * H + h) * dim) * vdim;
-    auto row_of = [&](int i) { return ((uint32_t)(i / VR) * 32 + lane) * VR + (uint32_t)(i % VR); };
-    float2 S[C][R / 2];
-#pragma unroll
-    for (int i = 0; i < R; i++)
-#pragma unroll
-        for (int c = 0; c < C; c++) {
-            const float x = row_of(i) < dim && col0 + c < vdim ? S_g[(size_t)row_of(i) * vdim + col0 + c] : 0.0f;
-            if (i & 1) S[c][i / 2].y = x; else S[c][i / 2].x = x;
+    __syncthreads();
+    const uint32_t width = min(dpad, NT), at_once = NT / width;      // fewer rows than threads: several tokens at a time
+    for (uint32_t c = tid & (width - 1); c < dpad; c += width) {
+        const float bias = sbias[c];
+#pragma unroll 2
+        for (uint32_t j = tid / width; j < C; j += at_once) {
+            const uint32_t at = j * dp + c;
+            sq[at] *= scale[j];
+            sk[at] *= scale[C + j];
+            sd[at] = c < dim && j < n ? delta_decay(sd[at] + bias, Ah, form, inv_tau) : 1.0f;
         }
-    const float* P = prep + (size_t)h * blocks * block_elems;
-    auto stage = [&](uint32_t b0, float* buf) {        // blocks [b0, min(b0 + tile, blocks)): one contiguous run
-        const uint32_t n4 = min(tile_blocks, blocks - b0) * block_elems / 4;
-        const float* src = P + (size_t)b0 * block_elems;
-        for (uint32_t i = threadIdx.x; i < n4; i += kWalkThreads) cp_async16(buf + 4 * i, src + 4 * i);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    stage(0, sm);
-    // lane (column, k or q, token), twice: its value of a block, its place in the outputs
-    const uint32_t lc = (lane >> 3) & 1, lj = lane & 3;
-    const bool live = col0 + lc < vdim;
-    const float* vbase = qkv + (size_t)lj * qkv_rs + v_off + (size_t)h * vdim + col0 + lc;
-    float vt[tile_blocks], vn[tile_blocks];
+    }
+    __syncthreads();
+    auto dot = [](float4 a, float4 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w))); };
+#pragma unroll 1
+    for (uint32_t m = 2 * warp; m < C; m += m & 1 ? 2 * warps - 1 : 1) {      // tokens m / 2 and 15 - m / 2 have 17 later ones and themselves together
+        const uint32_t i = m & 1 ? C - 1 - (m >> 1) : m >> 1;
+#pragma unroll 1
+        for (uint32_t c0 = 4 * lane; c0 < max(dpad, 128u); c0 += 128) {
+            const bool on = c0 < dpad;
+            const uint32_t c = on ? c0 : 0;                          // 64 rows: the upper lanes hold zeros
+            float4 d = *reinterpret_cast<const float4*>(sk + i * dp + c);      // what token i wrote, as the later tokens find it
+            if (!on) d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 own = *reinterpret_cast<const float4*>(sown + c), q = *reinterpret_cast<const float4*>(sq + i * dp + c);
+            const float self = warp_sum(dot(make_float4(q.x * own.x, q.y * own.y, q.z * own.z, q.w * own.w), d));
+            if (lane == 0) qk[i][i] = c0 < 128 ? self : qk[i][i] + self;
+#pragma unroll 1
+            for (uint32_t j0 = i + 1; j0 < C; j0 += 4) {
+                float v[8];                                          // q k of four tokens, k k of them
 #pragma unroll
-    for (int i = 0; i < (int)tile_blocks; i++) vt[i] = live && i * B + lj < T ? vbase[(size_t)i * B * qkv_rs] : 0.0f;
-    // R / 2 pairs of a prepared vector
-    auto vec = [&](const float* v, float2 (&x)[R / 2]) {
-#pragma unroll
-        for (int g = 0; g < NG; g++) {
-            if (VR == 4) {
-                const float4 y = *reinterpret_cast<const float4*>(v + (g * 32 + lane) * 4);
-                x[2 * g] = make_float2(y.x, y.y); x[(2 * g + 1) % (R / 2)] = make_float2(y.z, y.w);
-            } else x[0] = *reinterpret_cast<const float2*>(v + lane * 2);
-        }
-    };
-    uint32_t cur = 0;
-    for (uint32_t t0 = 0; t0 < T; t0 += kDeltaTile, cur ^= 1) {
-        const bool more = t0 + kDeltaTile < T;
-        if (more) stage((t0 + kDeltaTile) / B, sm + (cur ^ 1) * tile_elems);   // its last readers passed the barrier that ended the tile before
-#pragma unroll
-        for (int i = 0; i < (int)tile_blocks; i++) vn[i] = live && t0 + kDeltaTile + i * B + lj < T ? vbase[(size_t)(t0 + kDeltaTile + i * B) * qkv_rs] : 0.0f;
-        if (more) asm volatile("cp.async.wait_group 1;" ::: "memory"); else asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        const float* tile = sm + cur * tile_elems;
-#pragma unroll
-        for (int bi = 0; bi < (int)tile_blocks; bi++) {
-            const uint32_t tb = t0 + bi * B;
-            if (bi && tb >= T) break;
-            const float* row = tile + bi * block_elems;
-            const float* sc = row + (W + B + 1) * dpad;
-            float sums[W * C];                                        // [column][product]
-#pragma unroll
-            for (int d = 0; d < W; d++) {
-                float2 x[R / 2], acc[C];
-                vec(row + d * dpad, x);
-#pragma unroll
-                for (int c = 0; c < C; c++) acc[c] = __fmul2_rn(S[c][0], x[0]);
-#pragma unroll
-                for (int i = 1; i < R / 2; i++)
-#pragma unroll
-                    for (int c = 0; c < C; c++) acc[c] = __ffma2_rn(S[c][i], x[i], acc[c]);
-#pragma unroll
-                for (int c = 0; c < C; c++) sums[c * W + d] = acc[c].x + acc[c].y;
-            }
-            float total = reduce_scatter<W * C>(sums, lane);
-            if (PLAIN) total = __shfl_sync(0xffffffffu, total, lc * B + lj);
-            float u[B], uc[C][B];
-#pragma unroll
-            for (int j = 0; j < B; j++) u[j] = __shfl_sync(0xffffffffu, PLAIN ? vt[bi] : vt[bi] - total, (lane & 8) + j);
-            if (!PLAIN) {
-                const float4 beta = *reinterpret_cast<const float4*>(sc);
-                const float4 c1 = *reinterpret_cast<const float4*>(sc + B + 4), c2 = *reinterpret_cast<const float4*>(sc + B + 8), c3 = *reinterpret_cast<const float4*>(sc + B + 12);
-                u[0] *= beta.x;
-                u[1] = fmaf(-c1.x, u[0], u[1]) * beta.y;
-                u[2] = fmaf(-c2.y, u[1], fmaf(-c2.x, u[0], u[2])) * beta.z;
-                u[3] = fmaf(-c3.z, u[2], fmaf(-c3.y, u[1], fmaf(-c3.x, u[0], u[3]))) * beta.w;
-            }
-#pragma unroll
-            for (int j = 0; j < B; j++) {
-                const float other = __shfl_xor_sync(0xffffffffu, u[j], 8);
-                uc[0][j] = lc ? other : u[j];
-                uc[1][j] = lc ? u[j] : other;
-            }
-            {
-                float2 x[R / 2];
-                vec(row + (W + B) * dpad, x);
-#pragma unroll
-                for (int i = 0; i < R / 2; i++)
-#pragma unroll
-                    for (int c = 0; c < C; c++) S[c][i] = __fmul2_rn(S[c][i], x[i]);
-#pragma unroll
-                for (int j = 0; j < B; j++) {
-                    vec(row + (W + j) * dpad, x);
-#pragma unroll
-                    for (int i = 0; i < R / 2; i++)
-#pragma unroll
-                        for (int c = 0; c < C; c++) S[c][i] = __ffma2_rn(x[i], make_float2(uc[c][j], uc[c][j]), S[c][i]);
+                for (int l = 0; l < 4; l++) {
+                    const uint32_t at = min(j0 + l, C - 1) * dp + c;
+                    const float4 g = *reinterpret_cast<const float4*>(sd + at), qj = *reinterpret_cast<const float4*>(sq + at), kj = *reinterpret_cast<const float4*>(sk + at);
+                    if (bonus) v[l] = dot(qj, d);
+                    d.x *= g.x; d.y *= g.y; d.z *= g.z; d.w *= g.w;
+                    if (!bonus) v[l] = dot(qj, d);
+                    v[4 + l] = dot(kj, d);
+                }
+                const float total = reduce_scatter<8>(v, lane);
+                const uint32_t j = j0 + (lane & 3);
+                if (lane < 8 && j < C) {
+                    float& to = lane < 4 ? qk[j][i] : kk[j][i];
+                    to = c0 < 128 ? total : to + total;
                 }
             }
-            const float4 cq = *reinterpret_cast<const float4*>(sc + B + 16 + 4 * lj);
-            total = fmaf(cq.x, u[0], total);                          // a later token's u is left out, not multiplied by zero: it need not be finite
-            if (lj >= 1) total = fmaf(cq.y, u[1], total);
-            if (lj >= 2) total = fmaf(cq.z, u[2], total);
-            if (lj == 3) total = fmaf(cq.w, u[3], total);
-            if (live && (lane & 20) == 4 && tb + lj < T) dst[(size_t)(tb + lj) * dst_rs + (size_t)h * vdim + col0 + lc] = total;
+        }
+    }
+    __syncthreads();
+    float* P = prep + ((size_t)h * gridDim.y + b) * delta_chunk_elems(dpad, plain, vdim);
+    float* PQ = P + (plain ? 0 : C) * (dpad + 8);
+    float* PB = P + (plain ? 1 : 2) * C * (dpad + 8);
+    float* PV = P + delta_vec_elems(dpad, plain);
+    const uint32_t vpad = (vdim + kWalkCols - 1) / kWalkCols * kWalkCols;
+#pragma unroll 1
+    for (uint32_t c = tid; c < dpad + vpad; c += NT) {
+        const bool key = c < dpad;
+        const uint32_t col = c - dpad;
+        float y[C], z[C];                                            // key row: A then W, Q then Q'; value column: v then Vt, 0 then -Vo
+        if (key) {
+            float g = 1.0f, s = 1.0f, B[4];
+#pragma unroll
+            for (int j = 0; j < (int)C; j++) {
+                const float before = g;
+                g *= sd[j * dp + c];
+                y[j] = sk[j * dp + c] * g;
+                z[j] = sq[j * dp + c] * (bonus ? before : g);        // the bonus form reads the state before the token decays it
+            }
+            PB[(size_t)C * dpad + c] = g;
+            // the upper and lower eight tokens change places in every other pair of rows (banks of the walk's reads)
+            float* to = PB + (size_t)c * C;
+            const uint32_t turn = ((c >> 1) & 1) << 3;
+#pragma unroll
+            for (int j = C - 1; j >= 0; j--) {
+                B[j & 3] = s * sk[j * dp + c];
+                s *= sd[j * dp + c];
+                if ((j & 3) == 0) *reinterpret_cast<float4*>(to + ((uint32_t)j ^ turn)) = make_float4(B[0], B[1], B[2], B[3]);
+            }
+        } else {
+            const float* vr = row0 + v_off + (size_t)h * vdim + col;
+#pragma unroll
+            for (int j = 0; j < (int)C; j++) { y[j] = col < vdim && (uint32_t)j < n ? vr[(size_t)j * qkv_rs] : 0.0f; z[j] = 0.0f; }
+        }
+        // what lies past the diagonal of a row is read but not used
+#pragma unroll
+        for (int j = 0; j < (int)C; j++) {
+            if (!plain) {
+#pragma unroll
+                for (int i = 0; i < j; i += 4) {
+                    const float4 r = *reinterpret_cast<const float4*>(&kk[j][i]);
+                    const float c4[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+                    for (int l = 0; l < 4 && i + l < j; l++) y[j] = fmaf(-c4[l], y[i + l], y[j]);
+                }
+                y[j] *= beta[j];
+            }
+            if (!plain || !key) {
+#pragma unroll
+                for (int i = 0; i <= j; i += 4) {
+                    const float4 r = *reinterpret_cast<const float4*>(&qk[j][i]);
+                    const float c4[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+                    for (int l = 0; l < 4 && i + l <= j; l++) z[j] = fmaf(-c4[l], y[i + l], z[j]);
+                }
+            }
+            asm volatile("" ::: "memory");                           // the coefficients of all rows at once would not fit the registers
+        }
+        if (key) {
+#pragma unroll
+            for (int j = 0; j < (int)C; j++) {
+                if (!plain) P[(size_t)j * (dpad + 8) + c] = y[j];
+                PQ[(size_t)j * (dpad + 8) + c] = z[j];
+            }
+        } else {
+            float* to = PV + (size_t)(col / kWalkCols) * 512 + delta_square(0, col % kWalkCols);
+#pragma unroll
+            for (int j = 0; j < (int)C; j += 2) {
+                *reinterpret_cast<float2*>(to + delta_square(j, 0)) = make_float2(y[j], y[j + 1]);
+                *reinterpret_cast<float2*>(to + delta_square(j, 0) + 256) = make_float2(-z[j], -z[j + 1]);
+            }
+        }
+    }
+    if (!early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the walk's CTAs are placed when the GPU is theirs
+}
+__device__ __forceinline__ void bulk_load(float* to, const float* from, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(to)), "l"(from), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ void mma_bf16_first(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {      // d = a b
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.0f));
+}
+// two pairs of values as an operand of three bfloat16 parts (24 bits)
+__device__ __forceinline__ void split3_operand(const float* x, const float* y, uint32_t (&b)[3][2]) {
+    const float2 u = *reinterpret_cast<const float2*>(x), v = *reinterpret_cast<const float2*>(y);
+    split3(u.x, u.y, b[0][0], b[1][0], b[2][0]);
+    split3(v.x, v.y, b[0][1], b[1][1], b[2][1]);
+}
+// acc[0] + acc[1] + acc[2] (first: =, else +=) a b: six products in chains of one, two and three
+__device__ __forceinline__ void mma_split3(bool first, float (&acc)[3][4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+    if (first) { mma_bf16_first(acc[2], a[2], b[0]); mma_bf16_first(acc[1], a[1], b[0]); mma_bf16_first(acc[0], a[0], b[0]); }
+    else { mma_bf16(acc[2], a[2], b[0]); mma_bf16(acc[1], a[1], b[0]); mma_bf16(acc[0], a[0], b[0]); }
+    mma_bf16(acc[2], a[0], b[2]);
+    mma_bf16(acc[1], a[0], b[1]);
+    mma_bf16(acc[2], a[1], b[1]);
+}
+// A CTA owns 16 value columns of a head.  WARPS warps hold SL slices of 16 key rows of S^T each, in registers, as f32 accumulators of mma.sync: the same
+// registers, split into three bfloat16 parts, are the A operand of the next chunk's products.  Per chunk they form their shares of W S, sum those over
+// the warps, and update S <- Gamma S + B u; as many warps beside them read the parts of S from shared memory and form the outputs Q' S + Vo, off the chain from
+// chunk to chunk.  The products are far too small for tcgen05 (16 x 32 x 128 and 128 x 16 x 16, each waiting for the one before).  Measured at 1024
+// tokens, 16 heads of 128 x 128: 75 us; with the outputs formed by the warps that hold S 84 us, with f32 FMAs 128 us (bound by what shared memory
+// delivers to registers, 128 bytes a clock: 2500 clocks a chunk), four tokens at a time on one solve each 176 us.
+constexpr uint32_t kWalkStages = 3;
+constexpr uint32_t delta_walk_smem(uint32_t dpad, bool plain, uint32_t warps, uint32_t stages) {
+    return (stages * (delta_vec_elems(dpad, plain) + 512) + 2 * dpad / 16 * 384 + warps * 512) * 4 + 3 * 256 * 2 + 8 * kWalkStages;
+}
+template <int SL, int WARPS, bool PLAIN>
+__global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ dst, const float* __restrict__ prep, float* __restrict__ state, const float* __restrict__ ctl,
+                                                           uint32_t T, uint32_t H, uint32_t dim, uint32_t vdim, uint32_t dst_rs, uint32_t stages) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr uint32_t C = kWalkChunk, QR = PLAIN ? 0 : C, dpad = 16 * SL * WARPS, xs = dpad + 8, vec_elems = delta_vec_elems(dpad, PLAIN), NT = 32 * WARPS, PER = 256 / NT;
+    constexpr uint32_t stage_elems = vec_elems + 512, slices = SL * WARPS;      // of a stage: the chunk's vectors, [Vt | Vo] of the CTA's columns
+    const uint32_t h = blockIdx.y, col0 = blockIdx.x * kWalkCols, chunks = (T + C - 1) / C, tid = threadIdx.x % NT, lane = tid & 31, warp = tid >> 5;
+    const bool outputs = threadIdx.x >= NT;                           // a warp's role
+    float* parts = sm + stages * stage_elems;                         // parts of S^T: [chunk parity][slice][part][lane][4]
+    float* part_u = parts + 2 * slices * 384;                         // [warp][256]
+    float* part_o = part_u + WARPS * 256;                             // [warp][256]
+    bf16* U = reinterpret_cast<bf16*>(part_o + WARPS * 256);          // [part][256]
+    const uint32_t bars = smem_u32(U + 3 * 256);
+    const size_t stride = delta_chunk_elems(dpad, PLAIN, vdim);
+    const float* P = prep + (size_t)h * chunks * stride;
+    if (threadIdx.x == NT) {
+        for (uint32_t i = 0; i < stages; i++) mbar_init(bars + 8 * i, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    auto stage = [&](uint32_t b, uint32_t i) {                        // one thread; nobody reads stage i any more
+        if (b >= chunks) return;
+        const float* src = P + (size_t)b * stride;
+        float* to = sm + i * stage_elems;
+        mbar_expect_tx(bars + 8 * i, stage_elems * 4);
+        bulk_load(to, src, vec_elems * 4, bars + 8 * i);
+        bulk_load(to + vec_elems, src + vec_elems + blockIdx.x * 512, 2048, bars + 8 * i);
+    };
+    if (threadIdx.x == NT) for (uint32_t b = 0; b + 1 < stages || b == 0; b++) stage(b, b);
+    bool ok = true;                                                   // a wait that gave up: the outputs and the state are not numbers
+    const uint32_t g = lane >> 2, t = lane & 3;
+    // element e of a chunk's 16 x 16 u or o, in the order of the accumulators that hold them
+    auto tok_of = [](uint32_t e) { return (e >> 7) * 8 + 2 * ((e >> 2) & 3) + (e & 1); };
+    auto col_of = [](uint32_t e) { return ((e >> 4) & 7) + 8 * ((e >> 1) & 1); };
+    auto products = [&](const uint32_t (&b)[SL][2][3][2], auto part_of, float* out) {      // of 16 vectors with this warp's rows
+        float acc[2][3][4];
+#pragma unroll
+        for (int s = 0; s < SL; s++) {
+            uint32_t a[3][4];
+            part_of(s, a);
+#pragma unroll
+            for (int i = 0; i < 2; i++) mma_split3(s == 0, acc[i], a, b[s][i]);
         }
 #pragma unroll
-        for (int i = 0; i < (int)tile_blocks; i++) vt[i] = vn[i];
-        __syncthreads();                                   // everyone is done with this buffer: the next iteration refills it
+        for (int i = 0; i < 2; i++) {
+            float x[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) x[r] = acc[i][0][r] + (acc[i][1][r] + acc[i][2][r]);
+            *reinterpret_cast<float4*>(out + i * 128 + lane * 4) = make_float4(x[0], x[1], x[2], x[3]);
+        }
+    };
+    auto vectors = [&](const float* X, uint32_t (&b)[SL][2][3][2]) {
+#pragma unroll
+        for (int s = 0; s < SL; s++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float* x = X + (8 * i + g) * xs + (s * WARPS + warp) * 16 + 2 * t;
+                split3_operand(x, x + 8, b[s][i]);
+            }
+    };
+    auto total = [&](const float* part) {                             // over the warps
+        float x[4] = {};
+#pragma unroll
+        for (uint32_t w = 0; w < WARPS; w++) x[w & 3] += part[w * 256];
+        return (x[0] + x[1]) + (x[2] + x[3]);
+    };
+    __syncthreads();                                                  // the barriers are there
+    uint32_t cur = 0, parity = 0;
+    auto turn_stage = [&](uint32_t b) {
+        if (stages == 1) {                                            // no room for the next chunk's vectors beside this one's
+            __syncthreads();
+            if (threadIdx.x == NT) stage(b + 1, 0);
+        }
+        if (++cur == stages) { cur = 0; parity ^= 1; }
+    };
+    if (outputs) {
+        float* to[PER];
+#pragma unroll
+        for (uint32_t p = 0; p < PER; p++) to[p] = dst + (size_t)tok_of(tid + p * NT) * dst_rs + (size_t)h * vdim + col0 + col_of(tid + p * NT);
+        const size_t chunk_rs = (size_t)C * dst_rs;
+#pragma unroll 1
+        for (uint32_t b = 0; b < chunks; b++) {
+            const float* X = sm + cur * stage_elems;
+            if (!mbar_wait(bars + 8 * cur, parity)) ok = false;
+            uint32_t q[SL][2][3][2];
+            vectors(X + QR * xs, q);
+            __syncthreads();                                          // the parts of S are there, and the chunk before is done with
+            if (stages > 1 && tid == 0) stage(b + stages - 1, cur == 0 ? stages - 1 : cur - 1);
+            products(q, [&](int s, uint32_t (&a)[3][4]) {
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(parts + (((b & 1) * slices + s * WARPS + warp) * 3 + i) * 128 + lane * 4);
+                    a[i][0] = x.x; a[i][1] = x.y; a[i][2] = x.z; a[i][3] = x.w;
+                }
+            }, part_o + warp * 256);
+            bar_sync(2, NT);
+#pragma unroll
+            for (uint32_t p = 0; p < PER; p++) {
+                const uint32_t e = tid + p * NT;
+                const float o = X[vec_elems + 256 + e] + total(part_o + e);
+                if (b * C + tok_of(e) < T && col0 + col_of(e) < vdim) *to[p] = ok ? o : __uint_as_float(0x7fffffffu);
+                to[p] += chunk_rs;
+            }
+            turn_stage(b);
+        }
+        if (!ok && lane == 0) count_timeout();
+        return;
     }
+    // accumulator r of tile i of slice s: column g + 8 (r / 2), row 8 i + 2 t + r % 2 of the slice
+    float* S_g = state + (((size_t)(uint32_t)ctl_word(ctl, ZG_CTL_SLOT) * H + h) * dim) * vdim + col0;
+    float S[SL][2][4];
+    auto each_state = [&](auto f) {
 #pragma unroll
-    for (int i = 0; i < R; i++)
+        for (int s = 0; s < SL; s++)
 #pragma unroll
-        for (int c = 0; c < C; c++)
-            if (row_of(i) < dim && col0 + c < vdim) S_g[(size_t)row_of(i) * vdim + col0 + c] = i & 1 ? S[c][i / 2].y : S[c][i / 2].x;
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const uint32_t row = (s * WARPS + warp) * 16 + 8 * i + 2 * t + (r & 1), col = g + 8 * (r >> 1);
+                    f(S[s][i][r], row < dim && col0 + col < vdim, (size_t)row * vdim + col);
+                }
+    };
+    each_state([&](float& x, bool on, size_t at) { x = on ? S_g[at] : 0.0f; });
+#pragma unroll 1
+    for (uint32_t b = 0; b < chunks; b++) {
+        const float* X = sm + cur * stage_elems;
+        const float* B = X + (QR + C) * xs;
+        uint32_t A[SL][3][4];
+#pragma unroll
+        for (int s = 0; s < SL; s++) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) split3(S[s][i >> 1][2 * (i & 1)], S[s][i >> 1][2 * (i & 1) + 1], A[s][0][i], A[s][1][i], A[s][2][i]);
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+                *reinterpret_cast<uint4*>(parts + (((b & 1) * slices + s * WARPS + warp) * 3 + i) * 128 + lane * 4) = make_uint4(A[s][i][0], A[s][i][1], A[s][i][2], A[s][i][3]);
+        }
+        if (!mbar_wait(bars + 8 * cur, parity)) ok = false;
+        if (!PLAIN) {
+            uint32_t w[SL][2][3][2];
+            vectors(X, w);
+            products(w, [&](int s, uint32_t (&a)[3][4]) {
+#pragma unroll
+                for (int i = 0; i < 12; i++) a[i >> 2][i & 3] = A[s][i >> 2][i & 3];
+            }, part_u + warp * 256);
+        }
+        __syncthreads();                                              // the shares of u are there
+#pragma unroll
+        for (uint32_t p = 0; p < PER; p++) {
+            const uint32_t e = tid + p * NT;
+            float u = X[vec_elems + e];
+            if (!PLAIN) u -= total(part_u + e);
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const bf16 part = __float2bfloat16_rn(u);
+                U[i * 256 + e] = part;
+                u -= __bfloat162float(part);
+            }
+        }
+        uint32_t rows[SL][2][3][2];
+        float2 decay[SL][2];
+#pragma unroll
+        for (int s = 0; s < SL; s++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const uint32_t row0 = (s * WARPS + warp) * 16 + 8 * i, turn = ((g >> 1) & 1) << 3;
+                const float* row = B + (row0 + g) * C;
+                split3_operand(row + ((2 * t) ^ turn), row + ((2 * t + 8) ^ turn), rows[s][i]);
+                decay[s][i] = *reinterpret_cast<const float2*>(B + C * dpad + row0 + 2 * t);
+            }
+        bar_sync(1, NT);                                              // u
+        uint32_t UA[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const uint2 lo = *reinterpret_cast<const uint2*>(U + i * 256 + lane * 4), hi = *reinterpret_cast<const uint2*>(U + i * 256 + 128 + lane * 4);
+            UA[i][0] = lo.x; UA[i][1] = lo.y; UA[i][2] = hi.x; UA[i][3] = hi.y;
+        }
+#pragma unroll
+        for (int s = 0; s < SL; s++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                float acc[3][4];
+                mma_split3(true, acc, UA, rows[s][i]);
+#pragma unroll
+                for (int r = 0; r < 4; r++) S[s][i][r] = fmaf(S[s][i][r], r & 1 ? decay[s][i].y : decay[s][i].x, acc[0][r] + (acc[1][r] + acc[2][r]));
+            }
+        turn_stage(b);
+    }
+    each_state([&](float& x, bool on, size_t at) { if (on) S_g[at] = ok ? x : __uint_as_float(0x7fffffffu); });
+    if (!ok && lane == 0) count_timeout();
 }
 // o / rms(o) * norm_w * sigmoid(gate) (or silu(gate)) * out_scale, one warp per (token, head), in place
 template <typename WT>
@@ -1800,6 +1991,7 @@ static uint32_t attention_splits(const ZgSeqOp& s) {
 static bool linear_split(const ZgSeqOp& s, float* const* bufs) {     // f32 weights, many rows: split operands on the tensor cores
     return zg_split_gemm_usable(wptr<float>(bufs, s.buf[2], s.off[0]), bufs[s.buf[1]] + s.off[2], s.n[0], s.n[10] ? 2 * s.n[1] : s.n[1], s.n[2], s.n[3], s.n[7]);
 }
+unsigned int zg_seq_timeouts() { return tc_timeouts(); }
 size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs) {
     if (op.tag >= ZG_OP_STREAM_STEP) return 0;
     if (op.tag >= ZG_OP_SSM_SCAN) return zg_rec_op_scratch_elems(op);
@@ -1810,7 +2002,9 @@ size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs) {
     }
     if (op.tag == ZG_OP_DELTA_RULE) {                  // the prepared per-token rows of the prefill form
         const ZgSeqOp& d = op.u.seq;
-        return d.n[0] >= (uint32_t)kDeltaPrepMinTokens && d.n[3] <= (uint32_t)kWalkMaxDim ? (size_t)((d.n[0] + kWalkBlock - 1) / kWalkBlock) * d.n[1] * delta_block_elems(32 * delta_walk_rows(d.n[3]), d.n[10] & kDeltaPlain) : 0;
+        if (d.n[0] < (uint32_t)kDeltaPrepMinTokens || d.n[3] > kWalkMaxDim) return 0;
+        const bool plain = d.n[10] & kDeltaPlain;
+        return delta_chunk_elems(delta_rows(d.n[3]), plain, d.n[4]) * d.n[1] * delta_pass_chunks(d.n[0], d.n[1], d.n[3], d.n[4], plain);
     }
     if (!dense_gemm_enabled() || op.tag != ZG_OP_LINEAR) return 0;
     const ZgSeqOp& s = op.u.seq;
@@ -1971,29 +2165,35 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             const uint32_t RS = zg_delta_row_slices(dim), cols = kDeltaThreads / RS;
             const size_t smem = ((size_t)3 * kDeltaTile * RS * kDeltaRows + kDeltaTile) * sizeof(float);
             const dim3 grid((vdim + cols - 1) / cols, H);
-            if (scratch && T >= (uint32_t)kDeltaPrepMinTokens && dim <= (uint32_t)kWalkMaxDim) {
+            if (scratch && T >= (uint32_t)kDeltaPrepMinTokens && dim <= kWalkMaxDim) {
                 const bool plain = form & kDeltaPlain;
-                const uint32_t R = delta_walk_rows(dim), warps = (T + kWalkBlock - 1) / kWalkBlock * H, wcols = kWalkThreads / 32 * kWalkCols, n_prep = (warps + 3) / 4;
-                const size_t walk_smem = ((size_t)2 * (kDeltaTile / kWalkBlock) * delta_block_elems(32 * R, plain)) * sizeof(float);
-                // Long steps: a plain launch.  CTAs placed while the predecessor still fills the GPU shared SMs two by two (128 CTAs: 430 us instead of 250).
-                const bool early = n_prep + (vdim + wcols - 1) / wcols * H <= 100;
-#define ZG_WALK_FORM(R_, PLAIN_)                                                                                                                \
-    do {                                                                                                                                        \
-        if (walk_smem > 48 * 1024) cudaFuncSetAttribute(k_delta_walk<R_, PLAIN_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem); \
-        launch_pdl_if(early, k_delta_walk<R_, PLAIN_>, dim3((vdim + wcols - 1) / wcols, H), dim3(kWalkThreads), walk_smem, st, dst, bufs[s.buf[1]], \
-                      scratch, bufs[s.buf[6]], bufs[s.buf[7]], T, H, dim, vdim, s.off[2], s.n[5], dst_rs);                                      \
+                const uint32_t dpad = delta_rows(dim), warps = dpad == 64 ? 4 : 8, pass = delta_pass_chunks(T, H, dim, vdim, plain) * kWalkChunk;
+                // Where every CTA has an SM to itself: three stages, a chunk's vectors are asked for two chunks ahead, and more than half of the SM's shared
+                // memory (two CTAs on one SM share what bounds them while other SMs stand idle).  Two stages and several CTAs per SM where there are more.
+                const bool alone = (vdim + kWalkCols - 1) / kWalkCols * H <= zg_sm_count();
+                const uint32_t stages = dpad == 512 ? 1 : alone ? kWalkStages : 2;
+                const size_t walk_smem = std::max(delta_walk_smem(dpad, plain, warps, stages), alone ? 116u * 1024 : 0u);
+                if (delta_prep_smem(dpad) > 48 * 1024)
+                    ZG_SEQ_WDT(s.n[9], cudaFuncSetAttribute(k_delta_prepare<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)delta_prep_smem(dpad)));
+                for (uint32_t t = 0; t < T; t += pass) {
+                    const uint32_t n = std::min(pass, T - t);
+                    // One CTA per SM: eight warps each, and the walk may be placed beside them.  More: four warps (1024 CTAs 41 us, with eight 47).
+                    const bool few = (n + kWalkChunk - 1) / kWalkChunk * H <= zg_sm_count();
+                    ZG_SEQ_WDT(s.n[9], launch_pdl(k_delta_prepare<WT>, dim3(H, (n + kWalkChunk - 1) / kWalkChunk), dim3(few ? kDeltaPrepThreads : kDeltaPrepThreads / 2), delta_prep_smem(dpad), st, scratch, bufs[s.buf[1]] + (size_t)t * s.n[5],
+                                                  betab ? betab + (size_t)t * s.n[6] : nullptr, bufs[s.buf[3]] + s.n[13] + (size_t)t * s.n[7], wptr<WT>(bufs, s.buf[5], 0), n, H, G, dim, vdim, dpad,
+                                                  s.off[0], s.off[1], s.off[2], s.off[3], s.off[4], s.off[5], s.n[5], s.n[6], s.n[7], s.f[1], s.f[2], form, inv_tau, s.n[14], few ? 1u : 0u));
+                    ZG_SEQ_CHECK();
+#define ZG_WALK(SL_, WARPS_)                                                                                                                                   \
+    do {                                                                                                                                                      \
+        auto kern = plain ? k_delta_walk<SL_, WARPS_, true> : k_delta_walk<SL_, WARPS_, false>;                                                                  \
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem);                                                              \
+        launch_pdl(kern, dim3((vdim + kWalkCols - 1) / kWalkCols, H), dim3(64 * warps), walk_smem, st, dst + (size_t)t * dst_rs, scratch, bufs[s.buf[6]],      \
+                   bufs[s.buf[7]], n, H, dim, vdim, dst_rs, stages);                                                                                          \
     } while (0)
-#define ZG_WALK(R_)                                                                                                                             \
-    do {                                                                                                                                        \
-        ZG_SEQ_WDT(s.n[9], launch_pdl(k_delta_prepare<WT, R_>, dim3(n_prep), dim3(128), 0, st, scratch, bufs[s.buf[1]], betab, bufs[s.buf[3]] + s.n[13], \
-                                      wptr<WT>(bufs, s.buf[5], 0), T, H, G, dim, s.off[0], s.off[1], s.off[3], s.off[4], s.off[5], s.n[5], s.n[6], s.n[7], s.f[1], s.f[2], \
-                                      form, inv_tau, s.n[14]));                                                                                 \
-        ZG_SEQ_CHECK();                                                                                                                         \
-        if (plain) ZG_WALK_FORM(R_, true); else ZG_WALK_FORM(R_, false);                                                                        \
-    } while (0)
-                if (R == 2) ZG_WALK(2); else if (R == 4) ZG_WALK(4); else if (R == 8) ZG_WALK(8); else ZG_WALK(16);
+                    if (dpad == 512) ZG_WALK(4, 8); else if (dpad == 256) ZG_WALK(2, 8); else if (dpad == 128) ZG_WALK(1, 8); else ZG_WALK(1, 4);
 #undef ZG_WALK
-#undef ZG_WALK_FORM
+                    if (t + n < T) ZG_SEQ_CHECK();
+                }
             } else ZG_SEQ_WDT(s.n[9], {
                 if (smem > 48 * 1024) cudaFuncSetAttribute(k_delta_rule<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 launch_pdl(k_delta_rule<WT>, dim3(grid), dim3(kDeltaThreads), smem, st, dst, bufs[s.buf[1]], betab, bufs[s.buf[3]] + s.n[13], wptr<WT>(bufs, s.buf[5], 0), bufs[s.buf[6]],

@@ -131,17 +131,6 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
-// two values -> their three bfloat16 parts, packed
-__device__ __forceinline__ void split3(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-    uint32_t* const to[3] = {&p0, &p1, &p2};
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-        const float2 f = __bfloat1622float2(h);
-        a -= f.x; b -= f.y;
-        *to[i] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-}
 __device__ __forceinline__ float abs_or_inf(float m, float x) { const float a = fabsf(x); return a <= 3.4028234e38f ? fmaxf(m, a) : INFINITY; }   // NaN counts as infinite
 
 }  // namespace

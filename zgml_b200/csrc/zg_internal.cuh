@@ -392,6 +392,7 @@ bool zg_comm_allgather(ZgCudaCtx* ctx, const float* src, float* dst, size_t n_pe
 inline bool zg_is_seq_op(uint32_t tag) { return tag >= ZG_OP_EMBED && tag < ZG_OP_END; }
 bool zg_seq_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* why, size_t why_n);
 uint32_t zg_seq_op_writes(uint32_t tag);
+unsigned int zg_seq_timeouts();       // waits that gave up (DELTA_RULE's walk)
 size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs);   // shared activation scratch the op stages through (0: none)
 bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st);
 // dense_gemm.cu : bf16 x bf16 -> f32 prefill matmul on tcgen05 (TMA-fed, TMEM accumulator)
