@@ -124,6 +124,7 @@ struct ZgCudaProgram {
     float* d_attn_part = nullptr;      // split-KV partial states, one slice per attention unit
     uint32_t* d_attn_cnt = nullptr;    // arrival counters (self re-arming)
     uint32_t* d_atc_map = nullptr;     // which planes and mask classes the entries of the tensor-core attention units use
+    std::vector<char> written;         // per buffer: some op of the program writes its memory (as this or as another buffer over it)
     bool uniform_pos = true;   // every patched slice_assign sits at the same position (checked per refresh)
     // quantized KV cache mode (zg_cuda_program_quantize_kv; LlamaInferenceSession.quantizeKV, src/llama_inference.zig:648-679):
     // Q8 caches stand in for the f32 cache buffers; the patched slice_assigns into them run storeColumn, the attention ops
@@ -1179,8 +1180,37 @@ static bool build_decode_plan(ZgCudaProgram* p, std::vector<DecHostLayer>& layer
 
 // Dependency levels over ITEMS (level = 1 + max level of every earlier item it conflicts with), then units in (level,
 // program order); any such order is a valid topological order of the program's dependency DAG.
+// Buffers whose memory some op writes, by address: two buffers of a program may lie over the same memory.
+static void find_written(ZgCudaProgram* p) {
+    std::vector<std::pair<const float*, const float*>> spans;
+    std::vector<ZgRange> r;
+    for (const ZgOp& op : p->ops) {
+        op_ranges(p, op, r);
+        for (const ZgRange& x : r)
+            if (x.write && x.buf < p->buffers.size()) spans.push_back({p->buffers[x.buf], p->buffers[x.buf] + p->buffer_elems[x.buf]});
+    }
+    std::sort(spans.begin(), spans.end());
+    size_t n = 0;
+    for (const auto& x : spans) {                       // merged: apart and ascending
+        if (n && x.first <= spans[n - 1].second) spans[n - 1].second = std::max(spans[n - 1].second, x.second);
+        else spans[n++] = x;
+    }
+    p->written.assign(p->buffers.size(), 0);
+    for (size_t b = 0; b < p->buffers.size(); b++) {    // the last span that starts before the buffer's end
+        const auto at = std::lower_bound(spans.begin(), spans.begin() + n, p->buffers[b] + p->buffer_elems[b], [](const auto& x, const float* end) { return x.first < end; });
+        p->written[b] = at != spans.begin() && (at - 1)->second > p->buffers[b];
+    }
+}
+// Whether a sequence op's weight may be read before the launch's predecessor has completed: nothing in the program writes it, and what was enqueued before
+// the program has completed when its graph starts (launches outside a graph may overlap the end of the program before).
+static bool const_weights(const ZgCudaProgram* p, const ZgOp& op) {
+    const uint32_t b = op.u.seq.buf[2];
+    return p->ctx->graph_mode && !p->ctx->profiling && b < p->written.size() && !p->written[b];
+}
+
 static bool build_schedule(ZgCudaProgram* p) {
     const size_t n = p->ops.size();
+    find_written(p);
     const size_t chain_max = p->ctx->chain_max;
     std::vector<ZgItem> items;
     std::vector<ZgNormMacro> norm_of;     // per item (kind ITEM_NORM)
@@ -1760,7 +1790,7 @@ static bool launch_one(ZgCudaProgram* p, size_t i, cudaStream_t st) {
         }
     }
     if (zg_op_is_batched(op.tag)) return zg_launch_batch(op, p->d_batch + p->single_entry[i], 1, p->d_dyn, st);
-    if (zg_is_seq_op(op.tag)) return zg_launch_seq_op(ctx, op, p->buffers.data(), p->lean ? nullptr : p->ws.gemm_scratch, st);
+    if (zg_is_seq_op(op.tag)) return zg_launch_seq_op(ctx, op, p->buffers.data(), p->lean ? nullptr : p->ws.gemm_scratch, st, const_weights(p, op));
     return zg_launch_op(ctx, op, p->buffers.data(), p->d_dyn, (uint32_t)i, p->d_steps + p->step_off[i], st);
 }
 

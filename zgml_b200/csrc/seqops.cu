@@ -170,6 +170,214 @@ __global__ void k_linear_rows_vec(float* __restrict__ dst, const float* __restri
     }
 }
 
+// N values in every lane -> the total of value lane % N
+template <int N>
+__device__ __forceinline__ float reduce_scatter(float (&v)[N], uint32_t lane) {
+#pragma unroll
+    for (int o = N / 2; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (int o = N; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+__device__ __forceinline__ void bulk_load(float* to, const float* from, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(to)), "l"(from), "r"(bytes), "r"(bar) : "memory");
+}
+
+// ── LINEAR, few rows, weights through a ring ─────────────────────────────────────────────────────────────────────────
+// One CTA per SM with a contiguous run of the weight's rows, which it brings by bulk copies through three 32 KB slots.  The first three are asked for before
+// the wait on the predecessor (`early`: nothing in the program writes the weight): with two such kernels of a chain resident per SM, the HBM streams the
+// next one's rows while this one's chain of norm, launch and reduction is under way.  A slot holds eight rows (of up to 4 KB pieces) per 256 threads, or
+// where a row is shorter, eight rows per 32, 64 or 128 of them; a thread multiplies one 16-byte unit of each of its eight rows with the same activations.
+// Shares of a row meet by shuffles and, once per 64 rows, in shared memory.
+// Four gated feed-forwards of 2048 / 4096, bfloat16: one row 137 us with a warp per row and weights drawn to the L2 early, 86 now; eight rows of 1024 / 2048
+// 444 us (activations that do not fit 48 KB: no staging at all) and 102.
+// Activations of all rows lie in shared memory where they fit (kRingX bytes, for one and two rows whatever there is), else a segment of whole pieces of K at a
+// time: then every weight row passes through once per segment, a piece of it each time, and its shares are added up in shared memory.
+constexpr uint32_t kRingSlots = 3, kRingSlot = 32768, kRingPiece = 4096, kRingFlush = 64, kRingX = 65536;
+struct RingPlan { uint32_t ctas, lanes, segment, rows, smem; bool split; };      // segment: pieces of K whose activations are there at once; rows: whose shares are there at once
+static RingPlan ring_plan(uint32_t M, uint32_t N, uint32_t K, bool pairs, uint32_t elem, uint32_t sms) {
+    RingPlan r;
+    const uint32_t units = K * elem / 16, pieces = (K * elem + kRingPiece - 1) / kRingPiece;
+    r.ctas = std::min(sms, N);
+    r.lanes = units <= 32 ? 32 : units <= 64 ? 64 : units <= 128 ? 128 : 256;
+    r.split = M > 2 && (size_t)M * K * 4 > kRingX;
+    r.segment = r.split ? std::min(pieces, std::max(1u, kRingX / (M * (kRingPiece / elem) * 4))) : pieces;
+    r.rows = r.split ? ((N + r.ctas - 1) / r.ctas * (pairs ? 2 : 1) + 7) / 8 * 8 : 2 * kRingFlush;
+    const size_t x = r.split ? (size_t)M * r.segment * (kRingPiece / elem) : (size_t)M * K, smem = kRingSlots * kRingSlot + ((size_t)r.rows * 8 * M + x) * 4 + 16 * kRingSlots;
+    r.smem = smem <= 227 * 1024 ? (uint32_t)smem : 0;                 // 0: it does not fit
+    return r;
+}
+template <typename WT, int MR, bool PAIRS, bool SPLIT>      // SPLIT: several segments of K
+__global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float* __restrict__ dst, const float* __restrict__ src, const WT* __restrict__ W, const WT* __restrict__ bias,
+                                                             uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, SeqAct act, const float* __restrict__ ctl,
+                                                             uint32_t slot_stride, uint32_t lanes, uint32_t segment, uint32_t part_rows, uint32_t early) {
+    constexpr int V = WVec<WT>::n;
+    constexpr uint32_t piece_k = kRingPiece / (uint32_t)sizeof(WT);
+    extern __shared__ __align__(128) unsigned char ring[];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row_bytes = K * (uint32_t)sizeof(WT);
+    // `lanes` threads (32, 64, 128, 256) share a row
+    const uint32_t pieces = (row_bytes + kRingPiece - 1) / kRingPiece, group = 8 * (256 / lanes), shares = lanes >> 5, unit = tid % lanes, sub = tid / lanes;
+    const uint32_t per = N / gridDim.x, more = N % gridDim.x, n0 = blockIdx.x * per + min(blockIdx.x, more), n1 = n0 + per + (blockIdx.x < more ? 1 : 0);
+    const uint32_t r0 = PAIRS ? 2 * n0 : n0, rows = (PAIRS ? 2 : 1) * (n1 - n0);
+    const char* w0 = reinterpret_cast<const char*>(W) + (size_t)r0 * row_bytes;
+    float* part = reinterpret_cast<float*>(ring + kRingSlots * kRingSlot);      // [row][m][share], twice 64 rows or all of them
+    float* xs = part + part_rows * 8 * M;                                       // [m][a segment of K]
+    const uint32_t xw = SPLIT ? segment * piece_k : K;
+    const uint32_t bars = smem_u32(xs + M * xw), pitch = pieces == 1 ? row_bytes : kRingPiece;
+    if (tid == 0) {
+        for (uint32_t i = 0; i < kRingSlots; i++) { mbar_init(bars + 8 * i, 1); mbar_init(bars + 8 * (kRingSlots + i), 8); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __syncthreads();
+    if (warp == 8) {                                   // segment by segment of K, in a segment group by group of rows, of a group piece by piece
+        if (!early) asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint32_t slot = 0, parity = 0, p = 0;
+        bool again = false;                            // every slot has been filled once
+        for (uint32_t s0 = 0; s0 < pieces; s0 = p) {
+            const uint32_t s1 = SPLIT ? min(pieces, s0 + segment) : pieces;
+            for (uint32_t first = 0; first < rows; first += group)
+                for (p = s0; p < s1; p++) {
+                    if (again && !mbar_wait(bars + 8 * (kRingSlots + slot), parity)) { if (lane == 0) count_timeout(); return; }
+                    const uint32_t n = min(group, rows - first), bytes = min(kRingPiece, row_bytes - p * kRingPiece), bar = bars + 8 * slot;
+                    unsigned char* to = ring + slot * kRingSlot;
+                    const char* from = w0 + (size_t)first * row_bytes + p * kRingPiece;
+                    if (lane == 0) mbar_expect_tx(bar, n * bytes);
+                    __syncwarp();
+                    if (pieces == 1) {
+                        if (lane == 0) bulk_load(reinterpret_cast<float*>(to), reinterpret_cast<const float*>(from), n * bytes, bar);
+                    } else if (lane < n) {
+                        bulk_load(reinterpret_cast<float*>(to + lane * kRingPiece), reinterpret_cast<const float*>(from + (size_t)lane * row_bytes), bytes, bar);
+                    }
+                    if (++slot == kRingSlots) { slot = 0; if (again) parity ^= 1; again = true; }
+                }
+        }
+        return;
+    }
+    // The first step is run through before the wait as well, over whatever the activations' place holds, its results dropped: the instructions are there
+    // when the activations are (94.6 -> 91.7 us over four feed-forwards of 2048 / 4096).
+    bool warm = early && MR <= 4;
+    if (!warm) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (ctl && !warm) src += (size_t)ctl_word(ctl, ZG_CTL_SLOT) * slot_stride;
+    const bool vec = ((reinterpret_cast<uintptr_t>(src) & 15) | (src_rs & 3)) == 0;
+    auto load_x = [&](uint32_t k0) {                    // K is a multiple of four
+        const uint32_t n = min(xw, K - k0);
+        for (uint32_t m = 0; m < M; m++) {
+            const float* from = src + (size_t)m * src_rs + k0;
+            if (vec) for (uint32_t k = 4 * tid; k < n; k += 1024) *reinterpret_cast<float4*>(xs + m * xw + k) = *reinterpret_cast<const float4*>(from + k);
+            else for (uint32_t k = tid; k < n; k += 256) xs[m * xw + k] = from[k];
+        }
+        bar_sync(1, 256);
+    };
+    if (!warm) load_x(0);
+    bool ok = true;
+    constexpr bool TWO = MR <= 2;                       // sums of even and of odd elements, by packed FMAs, where the registers allow it
+    float2 acc[8][MR];
+    uint32_t slot = 0, parity = 0, done = 0, half = 0;       // done: rows whose outputs are written; half: of `part`, where a flush of 64 rows reads one and the next fills the other
+    auto flush = [&](uint32_t have) {
+        for (uint32_t e = tid; e < (PAIRS ? have / 2 : have) * M; e += 256) {
+            const uint32_t o = MR == 1 ? e : e / M, m = MR == 1 ? 0 : e % M, n = (r0 + done) / (PAIRS ? 2 : 1) + o;
+            auto sum = [&](uint32_t row) {
+                const float* s = part + ((size_t)(half * kRingFlush + row) * M + m) * 8;
+                float t = s[0];
+                for (uint32_t i = 1; i < shares; i++) t += s[i];
+                return ok ? t : __uint_as_float(0x7fffffffu);
+            };
+            if (PAIRS) dst[(size_t)m * dst_rs + n] = seq_epilogue(sum(2 * o), act.kind, act.p) * sum(2 * o + 1);
+            else dst[(size_t)m * dst_rs + n] = seq_epilogue(sum(o) + (bias ? wld(bias, n) : 0.0f), act, n);
+        }
+        done += have;
+    };
+    uint32_t s0 = 0, s1 = SPLIT ? segment : pieces, p = 0, first = 0;      // the segment, the piece, the group's first row
+#pragma unroll 1
+    while (true) {
+        if (p == s0) {
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+#pragma unroll
+                for (int m = 0; m < MR; m++) acc[r][m] = make_float2(0.0f, 0.0f);
+        }
+        if (!mbar_wait(bars + 8 * slot, parity)) ok = false;
+        const uint32_t k = p * piece_k + unit * V;
+        if (k < K) {
+            const unsigned char* w = ring + slot * kRingSlot + (size_t)sub * 8 * pitch + unit * 16;
+            const float* xk = xs + (SPLIT ? k - s0 * piece_k : k);
+            float x[MR][V];
+#pragma unroll
+            for (int m = 0; m < MR; m++)
+#pragma unroll
+                for (int i = 0; i < V; i += 4) {
+                    const float4 y = MR <= 2 || m < (int)M ? *reinterpret_cast<const float4*>(xk + m * xw + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    x[m][i] = y.x; x[m][i + 1] = y.y; x[m][i + 2] = y.z; x[m][i + 3] = y.w;
+                }
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                float wv[V];
+                wld_vec<WT>(reinterpret_cast<const WT*>(w + r * pitch), wv);
+#pragma unroll
+                for (int m = 0; m < MR; m++)
+#pragma unroll
+                    for (int i = 0; i < V; i += 2) {
+                        if (TWO) acc[r][m] = __ffma2_rn(make_float2(wv[i], wv[i + 1]), make_float2(x[m][i], x[m][i + 1]), acc[r][m]);
+                        else acc[r][m].x = fmaf(wv[i + 1], x[m][i + 1], fmaf(wv[i], x[m][i], acc[r][m].x));
+                    }
+            }
+        }
+        __syncwarp();
+        if (!warm && lane == 0) mbar_arrive(bars + 8 * (kRingSlots + slot));      // the slot is free
+        const bool last = ++p == s1;                    // of the group's pieces in this segment
+        if (last) {
+            const uint32_t row = (SPLIT ? first : half * kRingFlush + first - done) + sub * 8 + (lane & 7);
+#pragma unroll
+            for (int m = 0; m < MR; m++) {
+                if (MR > 2 && m >= (int)M) break;
+                float v[8];
+#pragma unroll
+                for (int r = 0; r < 8; r++) v[r] = TWO ? acc[r][m].x + acc[r][m].y : acc[r][m].x;
+                const float total = reduce_scatter<8>(v, lane);
+                if (lane < 8) {
+                    float& to = part[(row * (MR <= 2 ? MR : M) + m) * 8 + warp % shares];
+                    to = SPLIT && s0 ? to + total : total;
+                }
+            }
+        }
+        if (warm) {
+            warm = false;
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (ctl) src += (size_t)ctl_word(ctl, ZG_CTL_SLOT) * slot_stride;
+            load_x(0);
+            p = s0;
+            continue;
+        }
+        if (++slot == kRingSlots) { slot = 0; parity ^= 1; }
+        if (!last) continue;
+        first += group; p = s0;
+        const bool end = first >= rows;
+        if (!SPLIT) {
+            if (first - done >= kRingFlush || end) {
+                bar_sync(1, 256);                       // the shares are there; until the next time here, nobody writes this half
+                flush(min(first, rows) - done);
+                half ^= 1;
+            }
+            if (end) break;
+        } else if (end) {
+            first = 0; s0 = s1; p = s1; s1 = min(pieces, s1 + segment);
+            bar_sync(1, 256);                           // everyone is done with the segment's activations, or the last shares are there
+            if (s0 == pieces) break;
+            load_x(s0 * piece_k);
+        }
+    }
+    if (SPLIT) flush(rows);
+    if (!ok && lane == 0) count_timeout();
+}
+
 // ── LINEAR, many rows (prefill), exact f32: 64 x 64 tile, 16-deep k slices, 4 x 4 outputs per thread ──────────────────
 constexpr int kTM = 64, kTN = 64, kTK = 16;
 // rows_from > 0: only the rows of positions the sequence holds after this step matter (rows < position + rows_from)
@@ -1071,22 +1279,6 @@ static uint32_t delta_pass_chunks(uint32_t T, uint32_t H, uint32_t dim, uint32_t
     const uint32_t chunks = (T + kWalkChunk - 1) / kWalkChunk;
     return (uint32_t)(most < 4 ? chunks < 4 ? chunks : 4 : most < chunks ? most : chunks);
 }
-// N values in every lane -> the total of value lane % N
-template <int N>
-__device__ __forceinline__ float reduce_scatter(float (&v)[N], uint32_t lane) {
-#pragma unroll
-    for (int o = N / 2; o > 0; o >>= 1) {
-        const bool up = lane & o;
-#pragma unroll
-        for (int i = 0; i < o; i++) {
-            const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-#pragma unroll
-    for (int o = N; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-    return v[0];
-}
 // One CTA per (chunk, head): units, scales and decays into shared memory; the 256 products between the tokens (136 q k, 120 k k), a warp for two of the
 // tokens that wrote, four later tokens at a time; then a thread for a column of [A | V], whose solves are alike.  Loops are kept rolled where the data
 // allows it: a straight line of 5000 instructions took 88 us where this takes 43 (1024 tokens, 16 heads of 128 x 128, launches alone): every CTA fetched it anew.
@@ -1272,9 +1464,6 @@ __global__ void __launch_bounds__(kDeltaPrepThreads, 2) k_delta_prepare(float* _
         }
     }
     if (!early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the walk's CTAs are placed when the GPU is theirs
-}
-__device__ __forceinline__ void bulk_load(float* to, const float* from, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(to)), "l"(from), "r"(bytes), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -2013,7 +2202,22 @@ size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs) {
     return zg_dense_gemm_scratch_elems(s.n[0], s.n[2]);
 }
 
-bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st) {
+// Below that, a warp per output row and no staging is faster (four gated feed-forwards, one row: 256 / 512 27 us against 33, 512 / 1024 35 both ways,
+// 1024 / 2048 68 against 41; two rows: 256 / 512 35 against 39, 256 / 1024 44 against 39).
+static bool linear_ring(uint32_t M, size_t weight_bytes) { return weight_bytes >= (M == 1 ? 3u << 19 : 3u << 18); }
+template <typename WT>
+static void launch_linear_ring(bool pairs, float* dst, const float* src, const WT* W, const WT* bias, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, SeqAct act,
+                               const float* ctl, uint32_t slot_stride, bool early, const RingPlan& r, cudaStream_t st) {
+    auto kern = k_linear_rows_ring<WT, 1, false, false>;
+#define ZG_RING(MR_, SPLIT_) kern = pairs ? k_linear_rows_ring<WT, MR_, true, SPLIT_> : k_linear_rows_ring<WT, MR_, false, SPLIT_>
+    if (M == 1) ZG_RING(1, false); else if (M == 2) ZG_RING(2, false);
+    else if (r.split) { if (M <= 4) ZG_RING(4, true); else ZG_RING(8, true); }
+    else if (M <= 4) ZG_RING(4, false); else ZG_RING(8, false);
+#undef ZG_RING
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem);
+    launch_pdl(kern, dim3(r.ctas), dim3(288), r.smem, st, dst, src, W, bias, M, N, K, src_rs, dst_rs, act, ctl, slot_stride, r.lanes, r.segment, r.rows, early ? 1u : 0u);
+}
+bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st, bool const_weights) {
     (void)ctx;
     const ZgSeqOp& s = op.u.seq;
     switch (op.tag) {
@@ -2050,8 +2254,14 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                 constexpr uint32_t V = WVec<WT>::n;
                 if (M <= kGemvRows) {
                     const size_t xs_bytes = (size_t)M * K * sizeof(float);
-                    const bool vec = K % V == 0 && (reinterpret_cast<size_t>(W) & 15) == 0 && xs_bytes <= 48 * 1024;
+                    const bool aligned = K % V == 0 && (reinterpret_cast<size_t>(W) & 15) == 0, vec = aligned && xs_bytes <= 48 * 1024;
                     const dim3 grid((N + 7) / 8);
+                    const RingPlan ring = ring_plan(M, N, K, pairs, sizeof(WT), zg_sm_count());
+                    if (aligned && ring.smem && linear_ring(M, (size_t)(pairs ? 2 : 1) * N * K * sizeof(WT))) {
+                        launch_linear_ring<WT>(pairs, dst, src, W, b, M, N, K, s.n[3], s.n[4], act, slot_ctl, s.n[7], const_weights, ring, st);
+                        ZG_SEQ_CHECK();
+                        return true;
+                    }
                     if (pairs) ZG_ROWS(true); else ZG_ROWS(false);
                 } else {
                     const uint32_t NW = pairs ? 2 * N : N;

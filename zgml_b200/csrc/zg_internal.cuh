@@ -394,7 +394,8 @@ bool zg_seq_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* w
 uint32_t zg_seq_op_writes(uint32_t tag);
 unsigned int zg_seq_timeouts();       // waits that gave up (DELTA_RULE's walk)
 size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs);   // shared activation scratch the op stages through (0: none)
-bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st);
+// const_weights: nothing writes the op's weight (buf 2) while the program runs, so that it may be read before the launch's predecessor has completed
+bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st, bool const_weights);
 // dense_gemm.cu : bf16 x bf16 -> f32 prefill matmul on tcgen05 (TMA-fed, TMEM accumulator)
 bool zg_dense_gemm_usable(const void* w_bf16, uint32_t M, uint32_t N, uint32_t K);
 size_t zg_dense_gemm_scratch_elems(uint32_t M, uint32_t K);
