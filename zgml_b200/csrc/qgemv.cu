@@ -1,4 +1,4 @@
-// Decode-path quantized matvec / small-batch matmul for sm_100a.
+// Decode-path quantized matvec of one or two rows for sm_100a (three to eight: qgemv_rows.cu).
 //
 //   dst[m, n] = sum_k ( x[m, k] * s[(k*N + n) / 32] ) * q[k, n]
 //
@@ -127,16 +127,15 @@ __device__ __forceinline__ void sts8(uint32_t addr, uint32_t v) {
 
 constexpr uint32_t kPlaneRow = 144;   // bytes per (record, activation row) digit planes: 4 x 32 B + 16 B bank skew
 
-// FMT: ZG_QFMT_I8_F32 / ZG_QFMT_I8_F16 / ZG_QFMT_I4_F16.  MP: pairs of activation rows (M <= 2*MP).
-// XR: activation rows staged per warp (1 for the decode matvec M == 1, else 2*MP).
+// FMT: ZG_QFMT_I8_F32 / ZG_QFMT_I8_F16 / ZG_QFMT_I4_F16.  XR: activation rows, one or two.
 // PRO: 0 = activations are read; 1 / 2 = produced in the prologue (ZgGemvPrologue; M <= 2 only)
-template <int FMT, int MP, int XR, int PRO = 0>
-__global__ void __launch_bounds__(kThreads, MP == 1 ? 3 : (MP == 2 ? 2 : 1))
+template <int FMT, int XR, int PRO = 0>
+__global__ void __launch_bounds__(kThreads, 3)
 qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
     const auto& p = bt.p[blockIdx.y];
     constexpr bool kI4 = (FMT == ZG_QFMT_I4_F16);
     constexpr bool kF32 = (FMT == ZG_QFMT_I8_F32);
-    constexpr int MR = 2 * MP;
+    constexpr int MR = 2;
     constexpr uint32_t QB = kI4 ? 512u : 1024u;
     constexpr uint32_t SB = kF32 ? 32u : 16u;  // scale bytes per t
     constexpr uint32_t RB = QB + 4 * SB;       // record bytes
@@ -322,17 +321,14 @@ qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
         __syncwarp();
     }
 
-    // MMA role of this lane: B column g = digit j (j == 3: the ones plane) of activation row 2*mp + (g >> 2)
-    uint32_t brow[MP];
-#pragma unroll
-    for (int mp = 0; mp < MP; mp++)
-        brow[mp] = planes + (XR == 1 ? 0u : min((uint32_t)(2 * mp) + (g >> 2), p.M - 1)) * kPlaneRow + j * 32 + 4 * t;
+    // MMA role of this lane: B column g = digit j (j == 3: the ones plane) of activation row g >> 2
+    const uint32_t brow = planes + (XR == 1 ? 0u : min(g >> 2, p.M - 1)) * kPlaneRow + j * 32 + 4 * t;
     const uint32_t q_off = lane * 16;
     // digit-generation role of this lane: k row `lane` of each record
     const uint32_t sc_off = QB + (kF32 ? 4u : 2u) * (8 * ((lane & 15) >> 2) + 4 * (lane >> 4) + (lane & 3));  // zg_scale_row_slot(lane)
 
-    int acc[MP][2][4];
-    uint32_t dsum[MP];
+    int acc[2][4];
+    uint32_t dsum;
     uint32_t buf = 0, slot = 0, parity = 0, slot_u32 = ring, bar_u32 = bars;
     const uint32_t xs_row_bytes = p.xs_stride * 4;
     float sm_prev = sm_next;
@@ -350,14 +346,11 @@ qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
             __syncwarp();
             sm_prev = sm;
         }
+        dsum = 0;
 #pragma unroll
-        for (int mp = 0; mp < MP; mp++) {
-            dsum[mp] = 0;
+        for (int ct = 0; ct < 2; ct++)
 #pragma unroll
-            for (int ct = 0; ct < 2; ct++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) acc[mp][ct][i] = 0;
-        }
+            for (int i = 0; i < 4; i++) acc[ct][i] = 0;
 
         uint32_t xa = xs_u32 + lane * 4;   // this lane's (k = lane) staged activation of the chunk's first record
         for (uint32_t c = 0; c < n_chunk; c++, xa += G * ZG_KR * 4) {
@@ -433,17 +426,14 @@ qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
                             a[0][0] = q0.x; a[0][1] = q0.x & 0x0F0F0F0Fu; a[0][2] = q0.y; a[0][3] = q0.y & 0x0F0F0F0Fu;
                             a[1][0] = q0.z; a[1][1] = q0.z & 0x0F0F0F0Fu; a[1][2] = q0.w; a[1][3] = q0.w & 0x0F0F0F0Fu;
                         }
-#pragma unroll
-                        for (int mp = 0; mp < MP; mp++) {
-                            const uint32_t b0 = lds32(brow[mp] + r * XR * kPlaneRow), b1 = lds32(brow[mp] + r * XR * kPlaneRow + 16);
-                            if constexpr (kI4) {
-                                dsum[mp] = __dp4a(b0, 0x01010101u, __dp4a(b1, 0x01010101u, dsum[mp]));
-                                imma_u8u8(acc[mp][0], a[0][0], a[0][1], a[0][2], a[0][3], b0, b1);
-                                imma_u8u8(acc[mp][1], a[1][0], a[1][1], a[1][2], a[1][3], b0, b1);
-                            } else {
-                                imma_s8u8(acc[mp][0], a[0][0], a[0][1], a[0][2], a[0][3], b0, b1);
-                                imma_s8u8(acc[mp][1], a[1][0], a[1][1], a[1][2], a[1][3], b0, b1);
-                            }
+                        const uint32_t b0 = lds32(brow + r * XR * kPlaneRow), b1 = lds32(brow + r * XR * kPlaneRow + 16);
+                        if constexpr (kI4) {
+                            dsum = __dp4a(b0, 0x01010101u, __dp4a(b1, 0x01010101u, dsum));
+                            imma_u8u8(acc[0], a[0][0], a[0][1], a[0][2], a[0][3], b0, b1);
+                            imma_u8u8(acc[1], a[1][0], a[1][1], a[1][2], a[1][3], b0, b1);
+                        } else {
+                            imma_s8u8(acc[0], a[0][0], a[0][1], a[0][2], a[0][3], b0, b1);
+                            imma_s8u8(acc[1], a[1][0], a[1][1], a[1][2], a[1][3], b0, b1);
                         }
                     }
                 }
@@ -459,48 +449,45 @@ qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
         {
             const uint32_t kcnt = L * ZG_KR;   // rows fed to the MMA
             float* dstp = &part[buf][warp][0][0];
+            const float xw = (t >> 1) ? xm[1] : xm[0];   // row this lane writes
+            // 2^-23 * E2, E2 = max|x| * smax / 0.499
+            const float esc = (xw <= 3.0e38f) ? ((xw >= 1.0e-30f) ? (xw * (2.004008016f * 1.1920928955078125e-07f)) * sm : 0.0f)
+                                              : __int_as_float(0x7fc00000);
+            long long dS = 0;
+            if constexpr (kI4) {
+                uint32_t ds = dsum;
+                ds += __shfl_xor_sync(0xffffffffu, ds, 1);
+                ds += __shfl_xor_sync(0xffffffffu, ds, 2);
+                const uint32_t gsrc = 4 * (t >> 1);   // digit columns of the row this lane writes
+                const uint32_t D0 = __shfl_sync(0xffffffffu, ds, 4 * (gsrc + 0));
+                const uint32_t D1 = __shfl_sync(0xffffffffu, ds, 4 * (gsrc + 1));
+                const uint32_t D2 = __shfl_sync(0xffffffffu, ds, 4 * (gsrc + 2));
+                dS = (long long)D0 + ((long long)D1 << 8) + ((long long)D2 << 16);
+            }
 #pragma unroll
-            for (int mp = 0; mp < MP; mp++) {
-                const float xw = (t >> 1) ? xm[2 * mp + 1] : xm[2 * mp];   // row this lane writes
-                // 2^-23 * E2, E2 = max|x| * smax / 0.499
-                const float esc = (xw <= 3.0e38f) ? ((xw >= 1.0e-30f) ? (xw * (2.004008016f * 1.1920928955078125e-07f)) * sm : 0.0f)
-                                                  : __int_as_float(0x7fc00000);
-                long long dS = 0;
-                if constexpr (kI4) {
-                    uint32_t ds = dsum[mp];
-                    ds += __shfl_xor_sync(0xffffffffu, ds, 1);
-                    ds += __shfl_xor_sync(0xffffffffu, ds, 2);
-                    const uint32_t gsrc = 4 * (t >> 1);   // digit columns of the row this lane writes
-                    const uint32_t D0 = __shfl_sync(0xffffffffu, ds, 4 * (gsrc + 0));
-                    const uint32_t D1 = __shfl_sync(0xffffffffu, ds, 4 * (gsrc + 1));
-                    const uint32_t D2 = __shfl_sync(0xffffffffu, ds, 4 * (gsrc + 2));
-                    dS = (long long)D0 + ((long long)D1 << 8) + ((long long)D2 << 16);
-                }
+            for (int ct = 0; ct < 2; ct++) {
+                int pz[4];
 #pragma unroll
-                for (int ct = 0; ct < 2; ct++) {
-                    int pz[4];
+                for (int i = 0; i < 4; i++) pz[i] = __shfl_xor_sync(0xffffffffu, acc[ct][i], 1);
+                if ((t & 1) == 0) {
+                    const int m = (int)(t >> 1);
+                    const int* o = acc[ct];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) pz[i] = __shfl_xor_sync(0xffffffffu, acc[mp][ct][i], 1);
-                    if ((t & 1) == 0) {
-                        const int m = 2 * mp + (int)(t >> 1);
-                        const int* o = acc[mp][ct];
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            long long T;
-                            if constexpr (!kI4) {
-                                // own columns 2t, 2t+1 = digits 0, 1; partner's = digit 2 and sum_k q; row g + 8h
-                                T = (long long)o[2 * h] + ((long long)o[2 * h + 1] << 8) + ((long long)pz[2 * h] << 16) -
-                                    12582912LL * (long long)pz[2 * h + 1];
-                            } else {
-                                // Y (row g + 8) = sum u[n] d ; X (row g) = sum (16 u[n+8] + u[n]) d
-                                long long u0, u1, u2, us;
-                                if (h == 0) { u0 = o[2]; u1 = o[3]; u2 = pz[2]; us = pz[3]; }
-                                else { u0 = (o[0] - o[2]) >> 4; u1 = (o[1] - o[3]) >> 4; u2 = (pz[0] - pz[2]) >> 4; us = (pz[1] - pz[3]) >> 4; }
-                                // sum (u - 8)(Mk - 3*2^22) = sum u Mk - 8 sum Mk - 3*2^22 (sum u - 8 kcnt)
-                                T = u0 + (u1 << 8) + (u2 << 16) - 8 * dS - 12582912LL * (us - 8LL * (long long)kcnt);
-                            }
-                            dstp[m * ZG_TN + ct * 16 + g + 8 * h] = __ll2float_rn(T) * esc;
+                    for (int h = 0; h < 2; h++) {
+                        long long T;
+                        if constexpr (!kI4) {
+                            // own columns 2t, 2t+1 = digits 0, 1; partner's = digit 2 and sum_k q; row g + 8h
+                            T = (long long)o[2 * h] + ((long long)o[2 * h + 1] << 8) + ((long long)pz[2 * h] << 16) -
+                                12582912LL * (long long)pz[2 * h + 1];
+                        } else {
+                            // Y (row g + 8) = sum u[n] d ; X (row g) = sum (16 u[n+8] + u[n]) d
+                            long long u0, u1, u2, us;
+                            if (h == 0) { u0 = o[2]; u1 = o[3]; u2 = pz[2]; us = pz[3]; }
+                            else { u0 = (o[0] - o[2]) >> 4; u1 = (o[1] - o[3]) >> 4; u2 = (pz[0] - pz[2]) >> 4; us = (pz[1] - pz[3]) >> 4; }
+                            // sum (u - 8)(Mk - 3*2^22) = sum u Mk - 8 sum Mk - 3*2^22 (sum u - 8 kcnt)
+                            T = u0 + (u1 << 8) + (u2 << 16) - 8 * dS - 12582912LL * (us - 8LL * (long long)kcnt);
                         }
+                        dstp[m * ZG_TN + ct * 16 + g + 8 * h] = __ll2float_rn(T) * esc;
                     }
                 }
             }
@@ -856,7 +843,7 @@ __global__ void qmatmul_generic_kernel(const int8_t* __restrict__ data, const fl
     out[(size_t)m * out_rs + n] = acc;
 }
 
-template <int FMT, int MP, int XR, int PRO = 0>
+template <int FMT, int XR, int PRO = 0>
 bool launch_fast(const ZgGemvPlan& plan, const QGemvBatch& p, uint32_t count, cudaStream_t st, bool pdl) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(plan.grid, count);
@@ -874,11 +861,11 @@ bool launch_fast(const ZgGemvPlan& plan, const QGemvBatch& p, uint32_t count, cu
     cfg.numAttrs = na;
     cudaError_t e;
     if constexpr (PRO != 0) {
-        e = cudaLaunchKernelEx(&cfg, qgemv_kernel<FMT, MP, XR, PRO>, p);
+        e = cudaLaunchKernelEx(&cfg, qgemv_kernel<FMT, XR, PRO>, p);
     } else {
         QGemvBatchT<false> plain;
         for (uint32_t i = 0; i < kZgGemvBatch; i++) plain.p[i] = static_cast<const QGemvParams&>(p.p[i]);
-        e = cudaLaunchKernelEx(&cfg, qgemv_kernel<FMT, MP, XR, 0>, plain);
+        e = cudaLaunchKernelEx(&cfg, qgemv_kernel<FMT, XR, 0>, plain);
     }
     ZG_COUNT_LAUNCH();
     if (e != cudaSuccess) {
@@ -891,35 +878,26 @@ bool launch_fast(const ZgGemvPlan& plan, const QGemvBatch& p, uint32_t count, cu
 template <int FMT>
 bool launch_fmt(const ZgGemvPlan& plan, const QGemvBatch& p, uint32_t count, cudaStream_t st, bool pdl) {
     const uint32_t pk = p.p[0].pro.kind;
-    if (pk != 0) {   // prologue recipes exist for the decode variants only (M <= 2)
-        if (plan.mp != 1) { zg_set_error("internal: matvec prologue with more than 2 rows"); return false; }
-        if (pk == 1) return p.p[0].M == 1 ? launch_fast<FMT, 1, 1, 1>(plan, p, count, st, pdl) : launch_fast<FMT, 1, 2, 1>(plan, p, count, st, pdl);
-        return p.p[0].M == 1 ? launch_fast<FMT, 1, 1, 2>(plan, p, count, st, pdl) : launch_fast<FMT, 1, 2, 2>(plan, p, count, st, pdl);
-    }
-    switch (plan.mp) {
-        case 1: return p.p[0].M == 1 ? launch_fast<FMT, 1, 1>(plan, p, count, st, pdl) : launch_fast<FMT, 1, 2>(plan, p, count, st, pdl);
-        case 2: return launch_fast<FMT, 2, 4>(plan, p, count, st, pdl);
-        case 4: return launch_fast<FMT, 4, 8>(plan, p, count, st, pdl);
-        default: zg_set_error("qmatmul: bad plan (row pairs %u)", plan.mp); return false;
-    }
+    const bool one = p.p[0].M == 1;
+    if (pk == 1) return one ? launch_fast<FMT, 1, 1>(plan, p, count, st, pdl) : launch_fast<FMT, 2, 1>(plan, p, count, st, pdl);
+    if (pk) return one ? launch_fast<FMT, 1, 2>(plan, p, count, st, pdl) : launch_fast<FMT, 2, 2>(plan, p, count, st, pdl);
+    return one ? launch_fast<FMT, 1>(plan, p, count, st, pdl) : launch_fast<FMT, 2>(plan, p, count, st, pdl);
 }
 
 } // namespace
 
-// Work split for one launch of up to 8 activation rows.
+// Work split for one launch of one or two activation rows.
 ZgGemvPlan zg_qgemv_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t M, uint32_t count) {
     ZgGemvPlan pl;
-    const uint32_t rows = M > 8 ? 8 : M;
-    pl.mp = rows <= 2 ? 1 : (rows <= 4 ? 2 : 4);
+    const uint32_t rows = M > 2 ? 2 : M;
     pl.threads = kThreads;
-    const uint32_t occ = pl.mp == 1 ? 3 : (pl.mp == 2 ? 2 : 1);
-    const uint32_t target = (uint32_t)ctx->sm_count * occ;   // CTAs resident at once
+    const uint32_t target = (uint32_t)ctx->sm_count * 3;   // CTAs resident at once
     const uint32_t warps = kThreads / 32;
     // k-splits: each warp stages its k-range of the activations in shared memory -> at most lcap_max records per
     // warp.  Beyond that K is split across CTAs only until there is one CTA per SM (>= 4 records per warp): CTAs
     // that live long amortise their fixed latencies (activation staging, flush, reduction) and leave room for the
     // next kernel's CTAs, which is what keeps HBM busy across kernel boundaries.
-    const uint32_t lcap_max = kLcap / pl.mp;   // staged activations stay <= 32 KB per CTA
+    const uint32_t lcap_max = kLcap;           // staged activations stay <= 32 KB per CTA
     uint32_t S = (w->n_kc + warps * lcap_max - 1) / (warps * lcap_max);
     if (w->n_nb * S * 2 <= (uint32_t)ctx->sm_count) {
         uint32_t fill = (uint32_t)ctx->sm_count / w->n_nb;
@@ -963,7 +941,7 @@ ZgGemvPlan zg_qgemv_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t 
     // allow), which is worth more than a deeper ring - short-lived CTAs are latency-bound, bytes in flight come from CTA count
     pl.NS = ctx->tune_u ? (uint32_t)ctx->tune_u : 2;
     pl.xs_stride = pl.lcap * ZG_KR;
-    const uint32_t xrows = rows == 1 ? 1 : 2 * pl.mp;
+    const uint32_t xrows = rows;
     const uint32_t chunks = ((pl.lcap + pl.G - 1) / pl.G) * P;   // chunks a warp ever requests
     if (pl.NS > chunks) pl.NS = chunks < 1 ? 1 : chunks;
     auto smem_of = [&]() {
@@ -975,16 +953,15 @@ ZgGemvPlan zg_qgemv_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t 
     return pl;
 }
 
-template <int FMT, int MP, int XR, int PRO = 0>
+template <int FMT, int XR, int PRO = 0>
 bool set_smem_attr() {
-    cudaError_t e = cudaFuncSetAttribute(qgemv_kernel<FMT, MP, XR, PRO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(qgemv_kernel<FMT, XR, PRO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) { zg_set_error("cudaFuncSetAttribute(qgemv) failed: %s", cudaGetErrorString(e)); return false; }
     return true;
 }
 template <int FMT>
 bool set_smem_attrs() {
-    return set_smem_attr<FMT, 1, 1>() && set_smem_attr<FMT, 1, 2>() && set_smem_attr<FMT, 2, 4>() && set_smem_attr<FMT, 4, 8>() &&
-           set_smem_attr<FMT, 1, 1, 1>() && set_smem_attr<FMT, 1, 2, 1>() && set_smem_attr<FMT, 1, 1, 2>() && set_smem_attr<FMT, 1, 2, 2>();
+    return set_smem_attr<FMT, 1>() && set_smem_attr<FMT, 2>() && set_smem_attr<FMT, 1, 1>() && set_smem_attr<FMT, 2, 1>() && set_smem_attr<FMT, 1, 2>() && set_smem_attr<FMT, 2, 2>();
 }
 
 bool zg_qgemv_init(ZgCudaCtx* ctx) {
@@ -994,7 +971,6 @@ bool zg_qgemv_init(ZgCudaCtx* ctx) {
     if (const char* e = getenv("ZG_GEMV_NS")) ctx->tune_u = atoi(e);
     if (const char* e = getenv("ZG_GEMV_CLUSTER")) ctx->gemv_cluster = (e[0] != '0');   // 0: split-K through global scratch + arrival counters
     if (const char* e = getenv("ZG_GEMV_G")) ctx->tune_g = atoi(e);
-    if (const char* e = getenv("ZG_GEMV_ROWS")) { ctx->tune_rows = atoi(e); if (ctx->tune_rows < 1 || ctx->tune_rows > 8) ctx->tune_rows = 0; }
     if (ctx->tune_u < 2 || ctx->tune_u > 16) ctx->tune_u = 0;
     if (ctx->tune_g < 1 || ctx->tune_g > 16) ctx->tune_g = 0;
     // opt every instantiation into its dynamic shared memory once per context, outside any stream capture
@@ -1005,14 +981,10 @@ void zg_qgemv_ws_need(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t M, 
                       size_t* counters) {
     *partial_elems = 0; *counters = 0;
     if (w->fmt == ZG_QFMT_GENERIC || M == 0 || M > 8) return;
-    uint32_t S = 1, mp = 1;
-    for (uint32_t count = 1; count <= kZgGemvBatch; count++) {   // the split count depends on how many matvecs share the launch: size for the largest
-        const ZgGemvPlan plan = zg_qgemv_plan(ctx, w, M, count);
-        if (plan.S > S) S = plan.S;
-        mp = plan.mp;
-    }
+    uint32_t S = 1;                        // the split count depends on how many matvecs share the launch: size for the largest
+    for (uint32_t count = 1; count <= kZgGemvBatch; count++) S = std::max(S, M > 2 ? zg_qgemv_rows_plan(ctx, w, M, count).S : zg_qgemv_plan(ctx, w, M, count).S);
     if (S > 1) {
-        *partial_elems = (size_t)w->n_nb * S * (2 * mp) * ZG_TN;
+        *partial_elems = (size_t)w->n_nb * S * (M > 2 ? 8 : 2) * ZG_TN;
         *counters = w->n_nb;
     }
     if (M == 1)   // the streamed form cuts column groups at CTA boundaries: one partial slot per piece
@@ -1041,20 +1013,10 @@ bool zg_qmatmul_launch(ZgCudaCtx* ctx, const ZgCudaQWeight* w, const float* d_in
         if (!ws || ws->gemm_scratch_elems < need) { zg_set_error("internal: GEMM scratch too small (%zu needed)", need); return false; }
         return zg_qgemm_launch(ctx, w, d_in, d_out, M, in_rs, out_rs, ws->gemm_scratch, st);
     }
-    if (M <= 8) return zg_qgemv_launch_batch(ctx, 1, &w, &d_in, &d_out, M, &in_rs, &out_rs, ws, st);
-    // M > 8 in the generic-format-free matvec path never happens (the GEMM takes it); kept for direct callers
-    for (uint32_t m0 = 0; m0 < M; m0 += 8) {
-        const uint32_t rows = (M - m0) > 8 ? 8 : (M - m0);
-        const float* xin = d_in + (size_t)m0 * in_rs;
-        float* xout = d_out + (size_t)m0 * out_rs;
-        if (!zg_qgemv_launch_batch(ctx, 1, &w, &xin, &xout, rows, &in_rs, &out_rs, ws, st)) return false;
-    }
-    return true;
+    return zg_qgemv_launch_batch(ctx, 1, &w, &d_in, &d_out, M, &in_rs, &out_rs, ws, st);
 }
 
-// `count` (<= kZgGemvBatch) matvecs with identical weight shape, format and row count M <= 8 in one launch per pass of
-// `rows_per_pass` activation rows (ZG_GEMV_ROWS: the wide 8-row variant keeps one CTA per SM and short k-ranges; fewer
-// rows per pass re-stream the weights but run the well-occupied narrow variants).
+// `count` (<= kZgGemvBatch) matvecs with identical weight shape, format and row count, one or two, in one launch.
 static bool launch_batch_rows(ZgCudaCtx* ctx, uint32_t count, const ZgCudaQWeight* const* ws_w, const float* const* d_in,
                               float* const* d_out, uint32_t M, const uint32_t* in_rs, const uint32_t* out_rs,
                               const ZgGemvWs* ws, cudaStream_t st, const ZgGemvPrologue* pro) {
@@ -1105,18 +1067,11 @@ bool zg_qgemv_launch_batch(ZgCudaCtx* ctx, uint32_t count, const ZgCudaQWeight* 
     if (count > kZgGemvBatch || M > 8) { zg_set_error("internal: bad matvec batch (%u ops, %u rows)", count, M); return false; }
     const ZgGemvWs none[kZgGemvBatch] = {};
     if (!ws) ws = none;
-    const uint32_t rpp = ctx->tune_rows ? (uint32_t)ctx->tune_rows : 4u;   // measured: two 4-row passes beat one 8-row pass (ZG_GEMV_ROWS)
-    if (M <= rpp) return launch_batch_rows(ctx, count, ws_w, d_in, d_out, M, in_rs, out_rs, ws, st, pro);
-    if (pro && pro[0].kind) { zg_set_error("internal: matvec prologue on a multi-pass launch"); return false; }
-    for (uint32_t m0 = 0; m0 < M; m0 += rpp) {
-        const float* xin[kZgGemvBatch]; float* xout[kZgGemvBatch];
-        for (uint32_t i = 0; i < count; i++) {
-            xin[i] = d_in[i] + (size_t)m0 * (in_rs[i] ? in_rs[i] : (uint32_t)ws_w[i]->K);
-            xout[i] = d_out[i] + (size_t)m0 * (out_rs[i] ? out_rs[i] : (uint32_t)ws_w[i]->N);
-        }
-        if (!launch_batch_rows(ctx, count, ws_w, xin, xout, std::min(rpp, M - m0), in_rs, out_rs, ws, st, nullptr)) return false;
-    }
-    return true;
+    // Two rows: digit planes are cheap enough, and three CTAs of an SM overlap their prologues (14336 x 4096, Q8_0: 14.5 us against 18.6 in qgemv_rows.cu; 4096 x 1024
+    // 3.1 a matvec against 2.6).
+    if (M <= 2) return launch_batch_rows(ctx, count, ws_w, d_in, d_out, M, in_rs, out_rs, ws, st, pro);
+    if (pro && pro[0].kind) { zg_set_error("internal: matvec prologue on a launch of more than two rows"); return false; }
+    return zg_qgemv_rows_launch(ctx, count, ws_w, d_in, d_out, M, in_rs, out_rs, ws, st);
 }
 
 

@@ -122,7 +122,7 @@ struct ZgCudaCtx {
     bool graph_mode = true;
     bool profiling = false;
     bool pdl = true; // programmatic dependent launch between consecutive qgemv kernels (ZG_CUDA_PDL=0 disables)
-    int tune_s = 0, tune_p = 0, tune_u = 0, tune_g = 0, tune_smax = 0, tune_rows = 0; // ZG_GEMV_S / _P / _NS / _G overrides (kernel tuning only)
+    int tune_s = 0, tune_p = 0, tune_u = 0, tune_g = 0, tune_smax = 0; // ZG_GEMV_S / _P / _NS / _G overrides (kernel tuning only)
     ZgGemvWs ws; // split-K workspace for the direct zg_cuda_qmatmul_* calls
     int gemv_batch = 8;          // independent same-shape matvecs of a dependency level per launch (ZG_CUDA_GEMV_BATCH, 1 = off)
     int gemv_fuse = 0;           // evaluate norm (bit 0) / SiLU*up (bit 1) blocks inside the consuming matvecs' prologues (ZG_CUDA_GEMV_FUSE).
@@ -157,7 +157,7 @@ ZgCudaQWeight* zg_qweight_from_device_flat(ZgCudaCtx* ctx, const int8_t* d_data,
 // qgemv.cu
 // Work split of one launch (<= 8 activation rows): P column groups per CTA, S k-splits per column group.
 struct ZgGemvPlan {
-    uint32_t grid = 0, threads = 256, P = 1, S = 1, mp = 1, G = 2, NS = 3, lcap = 1, xs_stride = 32, smem_bytes = 0;
+    uint32_t grid = 0, threads = 256, P = 1, S = 1, G = 2, NS = 3, lcap = 1, xs_stride = 32, smem_bytes = 0;
 };
 ZgGemvPlan zg_qgemv_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t M, uint32_t count = 1);
 // dense_head.cu: bf16 copy of a dense matmul B operand (the tied LM head) with the argmax-safe exact recompute
@@ -173,6 +173,11 @@ ZgGemvStreamPlan zg_qgemv_stream_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight*
 bool zg_qgemv_stream_init(ZgCudaCtx* ctx);
 bool zg_qgemv_stream_launch(ZgCudaCtx* ctx, const ZgGemvStreamPlan& pl, uint32_t count, const ZgCudaQWeight* const* w, const float* const* d_in,
                             float* const* d_out, const ZgGemvWs* ws, cudaStream_t st);
+// qgemv_rows.cu: three to eight activation rows in one pass over the weights
+struct ZgGemvRowsPlan { uint32_t grid = 0, P = 1, S = 1, L = 1, NS = 2, teams = 1, smem_bytes = 0; };
+ZgGemvRowsPlan zg_qgemv_rows_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t M, uint32_t count);
+bool zg_qgemv_rows_launch(ZgCudaCtx* ctx, uint32_t count, const ZgCudaQWeight* const* w, const float* const* d_in, float* const* d_out, uint32_t M, const uint32_t* in_rs,
+                          const uint32_t* out_rs, const ZgGemvWs* ws, cudaStream_t st);
 void zg_trace_set_gemv_stream(unsigned long long* d_buf);   // count: matvecs sharing the launch
 void zg_qgemv_ws_need(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t M, size_t* partial_elems,
                       size_t* counters);
