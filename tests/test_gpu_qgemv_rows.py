@@ -41,3 +41,21 @@ def test_column_groups_of_different_scales(cuda_backend):
     for n in range(0, N, 32):
         assert rel_err(got[:, n:n + 32], want[:, n:n + 32]) < 2e-5, n
     w.free()
+
+
+@pytest.mark.parametrize("M", [1, 2, 5])
+def test_matvecs_of_unequal_widths_share_a_launch(cuda_backend, M):
+    """q, k and v of grouped heads: one K, two widths, one launch; the outputs are those of the matvecs alone."""
+    from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO, ResidentQuantizedWeight
+    K, widths = 576, (192, 576, 192, 64)
+    ws = [_weights("q8_0", K, N, N + 1)[1](cuda_backend) for N in widths]
+    x = rng(M).standard_normal((M, K)).astype(np.float32)
+    ops = [DeviceOp.qmatmul(1 + i, 0, i, M, N, K) for i, N in enumerate(widths)]
+    h = cuda_backend.compile_program(DeviceProgram(ops, [M * K] + [M * N for N in widths], [], [ResidentQuantizedWeight(w) for w in ws]))
+    got = [np.zeros((M, N), np.float32) for N in widths]
+    cuda_backend.execute_program(h, [ProgramIO(0, x.ravel())], [ProgramIO(1 + i, g) for i, g in enumerate(got)])
+    for w, g in zip(ws, got):
+        assert np.array_equal(g, w.matmul(x, M))
+    cuda_backend.free_program(h)
+    for w in ws:
+        w.free()

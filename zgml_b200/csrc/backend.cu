@@ -1510,14 +1510,16 @@ static bool build_schedule(ZgCudaProgram* p) {
             }
             if (it.kind == ITEM_OP && op.tag == ZG_OP_QMATMUL && op.u.qmatmul.M >= 1 && op.u.qmatmul.M <= 8 &&
                 (p->ctx->gemv_batch > 1 || pro_of[order[k]].kind != 0) && p->qweights[op.u.qmatmul.weight_idx]->fmt != ZG_QFMT_GENERIC) {
-                // independent matvecs of one shape / format / row count (and prologue kind) share a launch (q|k|v, gate|up)
+                // independent matvecs of one K / format / row count (and prologue kind) share a launch (q|k|v, gate|up).  q apart from k|v, on a branch of its own, tied
+                // the attention to two predecessors: an edge across branches is a full one, without programmatic launch (30 layers of 576: 1094 us a token, in one launch 974).
                 const ZgCudaQWeight* w = p->qweights[op.u.qmatmul.weight_idx];
                 const uint32_t pk = pro_of[order[k]].kind;
                 size_t ui = (size_t)-1;
                 for (auto& o : open_mv) {
                     const ZgCudaQWeight* r = o.first;
                     const ZgCudaProgram::Unit& u = p->units[o.second];
-                    if (r->fmt == w->fmt && r->K == w->K && r->N == w->N && p->ops[u.entry_ops[0]].u.qmatmul.M == op.u.qmatmul.M &&
+                    if (r->fmt == w->fmt && r->K == w->K && p->ops[u.entry_ops[0]].u.qmatmul.M == op.u.qmatmul.M &&
+                        (r->N == w->N || (!pk && zg_qgemv_mixes(p->ctx, r, op.u.qmatmul.M) && zg_qgemv_mixes(p->ctx, w, op.u.qmatmul.M))) &&
                         u.pros[0].kind == pk && u.entry_ops.size() < (size_t)std::max(p->ctx->gemv_batch, 1)) { ui = o.second; break; }
                 }
                 if (ui == (size_t)-1) {

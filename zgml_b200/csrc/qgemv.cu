@@ -151,6 +151,7 @@ qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
     const uint32_t g = lane >> 2, t = lane & 3, j = g & 3;
     const uint32_t split = blockIdx.x % p.S, grp = blockIdx.x / p.S;
     const uint32_t nb_begin = grp * p.P;
+    if (nb_begin >= p.n_nb) return;                // a narrower matvec of a launch of unequal widths (no k-splits there)
     const uint32_t nb_end = min(nb_begin + p.P, p.n_nb);
     const uint32_t ks = (uint32_t)(((uint64_t)split * p.n_kc) / p.S);
     const uint32_t ke = (uint32_t)(((uint64_t)(split + 1) * p.n_kc) / p.S);
@@ -1016,11 +1017,24 @@ bool zg_qmatmul_launch(ZgCudaCtx* ctx, const ZgCudaQWeight* w, const float* d_in
     return zg_qgemv_launch_batch(ctx, 1, &w, &d_in, &d_out, M, &in_rs, &out_rs, ws, st);
 }
 
-// `count` (<= kZgGemvBatch) matvecs with identical weight shape, format and row count, one or two, in one launch.
+// Whether a matvec may share a launch with narrower or wider ones over the same K: no k-splits (their number follows the width), not the streamed form.
+bool zg_qgemv_mixes(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t M) {
+    if (M > 2) return zg_qgemv_rows_plan(ctx, w, M, 1).S == 1;
+    for (uint32_t count = 1; count <= kZgGemvBatch; count++)
+        if (zg_qgemv_plan(ctx, w, M, count).S > 1 || (M == 1 && zg_qgemv_stream_plan(ctx, w, count).use)) return false;
+    return true;
+}
+static const ZgCudaQWeight* widest(const ZgCudaQWeight* const* w, uint32_t count) {
+    const ZgCudaQWeight* r = w[0];
+    for (uint32_t i = 1; i < count; i++) if (w[i]->N > r->N) r = w[i];
+    return r;
+}
+
+// `count` (<= kZgGemvBatch) matvecs with identical K, format and row count, one or two, in one launch (of unequal widths where zg_qgemv_mixes says so).
 static bool launch_batch_rows(ZgCudaCtx* ctx, uint32_t count, const ZgCudaQWeight* const* ws_w, const float* const* d_in,
                               float* const* d_out, uint32_t M, const uint32_t* in_rs, const uint32_t* out_rs,
                               const ZgGemvWs* ws, cudaStream_t st, const ZgGemvPrologue* pro) {
-    const ZgCudaQWeight* w0 = ws_w[0];
+    const ZgCudaQWeight* w0 = widest(ws_w, count);
     if (M == 1 && !(pro && pro[0].kind)) {
         const ZgGemvStreamPlan sp = zg_qgemv_stream_plan(ctx, w0, count);
         if (sp.use) return zg_qgemv_stream_launch(ctx, sp, count, ws_w, d_in, d_out, ws, st);
@@ -1030,7 +1044,7 @@ static bool launch_batch_rows(ZgCudaCtx* ctx, uint32_t count, const ZgCudaQWeigh
     memset(&bt, 0, sizeof(bt));
     for (uint32_t i = 0; i < count; i++) {
         const ZgCudaQWeight* w = ws_w[i];
-        if (w->fmt != w0->fmt || w->K != w0->K || w->N != w0->N || w->fmt == ZG_QFMT_GENERIC) { zg_set_error("internal: mixed matvec batch"); return false; }
+        if (w->fmt != w0->fmt || w->K != w0->K || (w->N != w0->N && (plan.S > 1 || !zg_qgemv_mixes(ctx, w, M))) || w->fmt == ZG_QFMT_GENERIC) { zg_set_error("internal: mixed matvec batch"); return false; }
         size_t pe = 0, nc = 0;
         zg_qgemv_ws_need(ctx, w, M, &pe, &nc);
         if (pe && (ws[i].partials_elems < pe || ws[i].counters_n < nc)) {

@@ -344,12 +344,14 @@ ZgGemvRowsPlan zg_qgemv_rows_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, 
 
 bool zg_qgemv_rows_launch(ZgCudaCtx* ctx, uint32_t count, const ZgCudaQWeight* const* w, const float* const* d_in, float* const* d_out, uint32_t M, const uint32_t* in_rs,
                           const uint32_t* out_rs, const ZgGemvWs* ws, cudaStream_t st) {
-    const ZgGemvRowsPlan pl = zg_qgemv_rows_plan(ctx, w[0], M, count);
+    const ZgCudaQWeight* w0 = w[0];
+    for (uint32_t i = 1; i < count; i++) if (w[i]->N > w0->N) w0 = w[i];
+    const ZgGemvRowsPlan pl = zg_qgemv_rows_plan(ctx, w0, M, count);
     const bool cluster = ctx->gemv_cluster && (pl.S == 2 || pl.S == 4 || pl.S == 8);
     RowsBatch bt;
     memset(&bt, 0, sizeof(bt));
     for (uint32_t i = 0; i < count; i++) {
-        if (w[i]->fmt != w[0]->fmt || w[i]->K != w[0]->K || w[i]->N != w[0]->N || w[i]->fmt == ZG_QFMT_GENERIC) { zg_set_error("internal: mixed matvec batch"); return false; }
+        if (w[i]->fmt != w0->fmt || w[i]->K != w0->K || (w[i]->N != w0->N && pl.S > 1) || w[i]->fmt == ZG_QFMT_GENERIC) { zg_set_error("internal: mixed matvec batch"); return false; }
         size_t pe = 0, nc = 0;
         zg_qgemv_ws_need(ctx, w[i], M, &pe, &nc);
         if (pe && (ws[i].partials_elems < pe || ws[i].counters_n < nc)) { zg_set_error("internal: split workspace too small (%zu/%zu needed)", pe, nc); return false; }
