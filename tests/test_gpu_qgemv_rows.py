@@ -46,7 +46,8 @@ def test_column_groups_of_different_scales(cuda_backend):
 @pytest.mark.parametrize("M", [1, 2, 5])
 def test_matvecs_of_unequal_widths_share_a_launch(cuda_backend, M):
     """q, k and v of grouped heads: one K, two widths, one launch; the outputs are those of the matvecs alone."""
-    from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO, ResidentQuantizedWeight
+    from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO
+    from zgml_b200.backend import ResidentQuantizedWeight
     K, widths = 576, (192, 576, 192, 64)
     ws = [_weights("q8_0", K, N, N + 1)[1](cuda_backend) for N in widths]
     x = rng(M).standard_normal((M, K)).astype(np.float32)
