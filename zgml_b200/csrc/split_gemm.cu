@@ -10,22 +10,25 @@
 // (four additions of b0 b0) and the steps are added in registers in f32.  Error against 64 bits at 256 tokens, 2048 / 4096: 1.7e-7 (pairs 2.1e-7, the f32
 // tile 8.7e-7).
 //
-//   * 128 x 128 tile per CTA, grid (n tiles, m tiles, shares of K).  Sixteen worker warps load f32 rows (16 lanes per row of 64), cut them, and store
-//     swizzled K-major tiles into a 2-stage ring; the same warps drain the accumulators of the step before (two TMEM buffers), each a quarter of the
-//     columns of its 32 rows.  Warp 16 issues the MMAs.
-//   * Per step the MMAs take 1536 clocks, their operand reads and the workers' stores 2300 clocks of shared-memory bandwidth; the f32 rows of the next step
-//     are in flight for one step only, and their latency bounds the kernel (256 tokens through gate, up and down of 2048 / 4096:
-//     166 us; as pairs with partial sums in scratch 169, as the f32 tile 1034).
+//   * 128 x 128 tile per CTA, grid (n tiles, m tiles, shares of K).  Sixteen worker warps load f32 rows of the weights (16 lanes per row of 64), two steps ahead, cut
+//     them, and store swizzled K-major tiles into a 2-stage ring; the same warps drain the accumulators of the step before (two TMEM buffers), each a quarter of
+//     the columns of its 32 rows.  Warp 16 issues the MMAs, warp 17 brings the source's parts, which k_split_source has cut once for all tiles of weight rows.
+//   * Per step the MMAs take 1536 clocks, their operand reads, the copies and the stores 2300 clocks of shared-memory bandwidth.  Where the workers cut the source
+//     too, every CTA its 128 rows of it, a step was 555 instructions of each worker warp, 2200 clocks of issue and 5000 in all, with its loads in flight for one step
+//     only: 256 tokens through gate, up and down of 2048 / 4096 took 166 us, now 95 (as the f32 tile 1034).
 //   * One share of K: the tile is finished here (bias, activation) and leaves by whole rows.  Several: partial sums go to scratch and k_split_finish adds them in
 //     order.  A sum that is not finite is evaluated again as a plain f32 sum: what an infinity makes of a sum is the plain kernel's.
 //   * Every wait is bounded and counts itself (with the count after the loops the case above took 178 us); a CTA whose wait ran out treats its sums as
 //     not finite, so that they are evaluated again the plain way.
 #include "split_tc.cuh"
 
+#include <algorithm>
+#include <string.h>
+
 namespace {
 
 constexpr uint32_t kBM = 128, kBN = 128, kBK = 64;
-constexpr uint32_t kTile = kBM * kBK * 2, kSgStage = 6 * kTile, kSgStages = 2, kSgWorkers = 512, kSgThreads = kSgWorkers + 32;
+constexpr uint32_t kTile = kBM * kBK * 2, kSgStage = 6 * kTile, kSgStages = 2, kSgWorkers = 512;
 constexpr uint32_t kSgSmem = kSgStages * kSgStage + 1024 + 128;
 
 struct SgArgs {
@@ -33,6 +36,7 @@ struct SgArgs {
     uint32_t M, N, K, src_rs, part_rs, splits;       // N: weight rows
     const float* ctl; uint32_t slot_stride, rows_from;
     float* dst; const float* bias; uint32_t dst_rs, pairs; SeqAct act;
+    uint16_t* planes; uint32_t pitch;                // PRE: [part][M][pitch] bfloat16 of the source
 };
 __device__ __forceinline__ const float* sg_src(const SgArgs& a) { return a.src + (a.ctl && a.slot_stride ? (size_t)ctl_word(a.ctl, ZG_CTL_SLOT) * a.slot_stride : 0); }
 __device__ __forceinline__ float plain_sum(const float* x, const float* w, uint32_t K) {
@@ -61,13 +65,34 @@ __device__ __forceinline__ void sg_finish(const SgArgs& a, uint32_t m, uint32_t 
         for (int j = 0; j < 4; j++) if (n + j < a.N) out[n + j] = z[j];
 }
 
-__global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
+// The source's parts, once per linear instead of once per tile of weight rows: eight elements a thread.
+__global__ void __launch_bounds__(256) k_split_source(const SgArgs a) {
+    pdl_enter();
+    const float* src = sg_src(a);
+    const uint32_t per_row = a.pitch / 8;
+    for (size_t e = blockIdx.x * 256 + threadIdx.x; e < (size_t)a.M * per_row; e += (size_t)gridDim.x * 256) {
+        const uint32_t m = (uint32_t)(e / per_row), k = (uint32_t)(e % per_row) * 8;
+        const float* x = src + (size_t)m * a.src_rs + k;      // K is a multiple of four
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f), u = *reinterpret_cast<const float4*>(x), v = k + 4 < a.K ? *reinterpret_cast<const float4*>(x + 4) : zero;
+        uint4 p[3];
+        split3(u.x, u.y, p[0].x, p[1].x, p[2].x);
+        split3(u.z, u.w, p[0].y, p[1].y, p[2].y);
+        split3(v.x, v.y, p[0].z, p[1].z, p[2].z);
+        split3(v.z, v.w, p[0].w, p[1].w, p[2].w);
+#pragma unroll
+        for (int i = 0; i < 3; i++) *reinterpret_cast<uint4*>(a.planes + ((size_t)i * a.M + m) * a.pitch + k) = p[i];
+    }
+}
+
+// PRE: the source's parts come by TMA from k_split_source's planes (warp 17), the workers cut the weights alone and load them two steps ahead
+template <bool PRE>
+__global__ void __launch_bounds__(kSgWorkers + (PRE ? 64 : 32), 1) k_split_gemm(const SgArgs a, const __grid_constant__ CUtensorMap planes) {
     extern __shared__ uint8_t dsm_raw[];
     const uint32_t base = (smem_u32(dsm_raw) + 1023u) & ~1023u, bars = base + kSgStages * kSgStage;
     const uint32_t full = bars, empty = full + 8 * kSgStages, d_full = empty + 8 * kSgStages, d_empty = d_full + 16, tmem_slot = d_empty + 16;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (uint32_t i = 0; i < kSgStages; i++) { mbar_init(full + 8 * i, 16); mbar_init(empty + 8 * i, 1); }
+        for (uint32_t i = 0; i < kSgStages; i++) { mbar_init(full + 8 * i, PRE ? 17 : 16); mbar_init(empty + 8 * i, 1); }
         for (uint32_t i = 0; i < 2; i++) { mbar_init(d_full + 8 * i, 1); mbar_init(d_empty + 8 * i, 16); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -113,18 +138,33 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
             __syncwarp();
             if (++stage == kSgStages) { stage = 0; phase ^= 1; }
         }
+    } else if (PRE && warp == 17) {
+        bool ok = true;
+        uint32_t stage = 0, phase = 1;
+        for (uint32_t i = 0; i < n_steps && ok; i++) {
+            ok = mbar_wait_counted(empty + 8 * stage, phase);
+            if (lane == 0 && ok) {
+                mbar_expect_tx(full + 8 * stage, 3 * kTile);
+                const int32_t k = (int32_t)((s0 + i) * kBK), m = (int32_t)m0;
+                asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                             ::"r"(base + stage * kSgStage), "l"(&planes), "r"(k), "r"(m), "r"(0), "r"(full + 8 * stage) : "memory");
+            }
+            __syncwarp();
+            if (++stage == kSgStages) { stage = 0; phase ^= 1; }
+        }
     } else {
         // loading: lane group of 16 takes rows r + 32 i, columns 4 c .. + 3 of a step; draining: rows of the warp's quarter, 32 columns
         const uint32_t c = threadIdx.x & 15, r = threadIdx.x >> 4, quarter = warp & 3, part = warp >> 2;
         uint8_t* const ring = dsm_raw + (base - smem_u32(dsm_raw));
         const float* src = sg_src(a);
-        float4 x[8];                                                 // four rows of the source, four of the weights
-        auto load = [&](uint32_t step) {
+        constexpr int FIRST = PRE ? 4 : 0, AHEAD = PRE ? 2 : 1;
+        float4 x[AHEAD][8];                                          // four rows of the source, four of the weights
+        auto load = [&](uint32_t step, float4 (&x)[8]) {
             const uint32_t k = step * kBK + 4 * c;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const uint32_t m = m0 + r + 32 * i, n = n0 + r + 32 * i;
-                x[i] = m < a.M && k < a.K ? *reinterpret_cast<const float4*>(src + (size_t)m * a.src_rs + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (!PRE) x[i] = m < a.M && k < a.K ? *reinterpret_cast<const float4*>(src + (size_t)m * a.src_rs + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 x[4 + i] = n < a.N && k < a.K ? *reinterpret_cast<const float4*>(a.W + (size_t)n * a.K + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
         };
@@ -135,25 +175,31 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
         auto drain = [&](uint32_t i) {
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait_counted(d_full + 8 * (i & 1), (i >> 1) & 1));
             fence_after();
-            uint32_t v[32];
-            tmem_ld(tmem + ((quarter * 32) << 16) + (i & 1) * kBN + 32 * part, v);
-            tmem_wait_ld(v);
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(d_empty + 8 * (i & 1));
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-                const float2 r = __fadd2_rn(make_float2(acc[j], acc[j + 1]), make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])));
-                acc[j] = r.x; acc[j + 1] = r.y;
+            for (int h = 0; h < 32; h += 16) {                       // half at a time: the registers of the other half hold rows on their way
+                uint32_t v[16];
+                tmem_ld(tmem + ((quarter * 32) << 16) + (i & 1) * kBN + 32 * part + h, v);
+                tmem_wait_ld(v);
+                if (h) {
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(d_empty + 8 * (i & 1));
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {
+                    const float2 r = __fadd2_rn(make_float2(acc[h + j], acc[h + j + 1]), make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])));
+                    acc[h + j] = r.x; acc[h + j + 1] = r.y;
+                }
             }
         };
-        if (n_steps) load(s0);
+        if (n_steps) load(s0, x[0]);
+        if (PRE && n_steps > 1) load(s0 + 1, x[AHEAD - 1]);
         uint32_t stage = 0, phase = 1;
-        for (uint32_t i = 0; i < n_steps; i++) {
+        auto step = [&](uint32_t i, float4 (&x)[8]) {
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait_counted(empty + 8 * stage, phase));
             uint8_t* const to = ring + stage * kSgStage;
 #pragma unroll
-            for (int j = 0; j < 8; j++) {                            // the source's rows, the weights'
+            for (int j = FIRST; j < 8; j++) {                        // the source's rows, the weights'
                 const float4 y = x[j];
                 const uint32_t row = r + 32 * (j & 3);
                 uint2 p0, p1, p2;
@@ -164,12 +210,16 @@ __global__ void __launch_bounds__(kSgThreads, 1) k_split_gemm(const SgArgs a) {
                 *reinterpret_cast<uint2*>(at + kTile) = p1;
                 *reinterpret_cast<uint2*>(at + 2 * kTile) = p2;
             }
-            if (i + 1 < n_steps) load(s0 + i + 1);                   // in flight while the step before is drained
+            if (i + AHEAD < n_steps) load(s0 + i + AHEAD, x);        // in flight while the step before is drained, and with PRE the next one is cut
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * stage);
             if (++stage == kSgStages) { stage = 0; phase ^= 1; }
             if (i) drain(i - 1);
+        };
+        for (uint32_t i = 0; i < n_steps; i += AHEAD) {
+            step(i, x[0]);
+            if (PRE && i + 1 < n_steps) step(i + 1, x[AHEAD - 1]);
         }
         if (n_steps) drain(n_steps - 1);
         // out by whole rows, through the idle ring (every MMA that reads it is done)
@@ -228,6 +278,16 @@ uint32_t shares(uint32_t M, uint32_t N, uint32_t K, uint32_t n_sm) {
     return best;
 }
 uint32_t up4(uint32_t n) { return (n + 3) / 4 * 4; }
+uint32_t up8(uint32_t n) { return (n + 7) / 8 * 8; }
+// Whether the source is cut ahead, by a launch of its own (some 3 us): where a CTA takes four steps or more, each about 1 us shorter for it (up and down of 1000 / 3000
+// with 100 tokens 58.7 us without, 43.2 from four steps on, 47.0 from eight, 51.4 always).
+constexpr size_t kSgPlanes = 40u << 20;              // elements: 240 MB of planes at most
+bool split_first(uint32_t M, uint32_t N, uint32_t K) {
+    const uint64_t tiles = (uint64_t)((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN), n_sm = zg_sm_count();
+    const uint32_t s = shares(M, N, K, (uint32_t)n_sm), steps = ((K + kBK - 1) / kBK + s - 1) / s;
+    return (tiles * s + n_sm - 1) / n_sm * steps >= 4 && (size_t)M * K <= kSgPlanes && encode_tiled();
+}
+size_t plane_elems(uint32_t M, uint32_t N, uint32_t K) { return split_first(M, N, K) ? ((size_t)3 * M * up8(K) / 2 + 3) / 4 * 4 : 0; }
 
 }  // namespace
 
@@ -237,14 +297,29 @@ bool zg_split_gemm_usable(const float* w, const float* src, uint32_t M, uint32_t
 }
 size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K) {      // never 0, which stands for the plain kernel
     const uint32_t s = shares(M, N, K, zg_sm_count());
-    return s > 1 ? (size_t)s * M * up4(N) : 4;
+    return (s > 1 ? (size_t)s * M * up4(N) : 4) + plane_elems(M, N, K);
 }
 unsigned int zg_split_gemm_timeouts() { return tc_timeouts(); }
 bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, cudaStream_t st,
                           uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from) {
-    if (!zg_smem_limit<k_split_gemm>(kSgSmem)) return false;
-    const SgArgs a = {src, w, scratch, M, N, K, src_rs, up4(N), shares(M, N, K, zg_sm_count()), ctl, slot_stride, rows_from, dst, bias, dst_rs, (uint32_t)pairs, SeqAct{act, act_p, act_lo, act_hi}};
-    launch_pdl(k_split_gemm, dim3((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, a.splits), dim3(kSgThreads), kSgSmem, st, a);
+    if (!zg_smem_limit<k_split_gemm<false>>(kSgSmem) || !zg_smem_limit<k_split_gemm<true>>(kSgSmem)) return false;
+    SgArgs a = {src, w, scratch, M, N, K, src_rs, up4(N), shares(M, N, K, zg_sm_count()), ctl, slot_stride, rows_from, dst, bias, dst_rs, (uint32_t)pairs, SeqAct{act, act_p, act_lo, act_hi}, nullptr, 0};
+    const dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, a.splits);
+    CUtensorMap map;
+    memset(&map, 0, sizeof(map));
+    if (split_first(M, N, K)) {
+        a.planes = reinterpret_cast<uint16_t*>(scratch);
+        a.pitch = up8(K);
+        a.part = scratch + plane_elems(M, N, K);
+        const cuuint64_t dims[3] = {a.pitch, M, 3}, strides[2] = {(cuuint64_t)a.pitch * 2, (cuuint64_t)a.pitch * 2 * M};
+        const cuuint32_t box[3] = {kBK, kBM, 3}, ones[3] = {1, 1, 1};
+        const CUresult r = encode_tiled()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a.planes, dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) { zg_set_error("split gemm: tensor map failed (%d)", (int)r); return false; }
+        launch_pdl(k_split_source, dim3(std::min<uint32_t>(4 * zg_sm_count(), (uint32_t)(((size_t)M * a.pitch / 8 + 255) / 256))), dim3(256), 0, st, a);
+        ZG_COUNT_LAUNCH();
+        launch_pdl(k_split_gemm<true>, grid, dim3(kSgWorkers + 64), kSgSmem, st, a, map);
+    } else launch_pdl(k_split_gemm<false>, grid, dim3(kSgWorkers + 32), kSgSmem, st, a, map);
     ZG_COUNT_LAUNCH();
     if (a.splits > 1) {
         launch_pdl(k_split_finish, dim3((N + 1023) / 1024, M < 65535 ? M : 65535), dim3(256), 0, st, a);
