@@ -531,34 +531,50 @@ __global__ void __launch_bounds__(kMergeCols * kMergeGroups, BLOCKS) k_cached_at
 
 // Few query rows (decoding: tokens x heads of a key group <= 16): what bounds the step is the latency of pulling the cache,
 // so a CTA takes one share of the keys, 32 at a time with WHOLE rows in shared memory — one round of loads per 32 keys instead
-// of one per 64-wide slice — and the shares are merged afterwards.  Scores: the 16 x 32 (row, key) pairs are covered by 32
-// threads holding 4 x 4 pairs each (rows rg + 4 r, keys kg + 8 c: conflict-free 16-byte reads of padded rows), and the eight
-// warps split the key dimension; their partial dot products meet in shared memory.  Then thread (row, kq) of 16 x 16 owns
-// keys kq and kq + 16 of its row, and the 16 threads of a row keep the row's running (max, sum) in step through half-warp
-// shuffles; for the weighted sum thread t owns value columns t + 256 i of all rows.  Where the value row is the head of the
-// key row itself (a latent that serves as both), it is not loaded twice.
-// Wide rows leave room for one CTA per SM, whose eight warps waited for their shared-memory reads most of the time: it has sixteen then (the slices
-// of the key dimension and the columns per thread halve).  One token, 16 heads, 8192 latents of 576: with 148 shares instead of 64 and sixteen warps
-// 45 -> 24 us, the op with its merge and the append 54 -> 33.
+// of one per 64-wide slice — and the shares are merged afterwards; the next 32 keys are on their way while these are worked on, where a share has more.
+// The 16 rows are the M of mma.sync.m16n8k16.  Scores and weighted sums are products of operands in three bfloat16 parts each, all 24 bits of
+// them, with the six products that matter (as in split_gemm.cu): cut where they are read, so a key's or a value's element is read from shared memory once
+// and not once per four rows.  Scores: pairs of warps take every n-th 16 of the key dimension, each half of the keys; the partial sums meet in shared memory, a warp adds up
+// a row's 32 and keeps the row's running (max, sum), and leaves the probabilities cut and in the order of an A operand.  Weighted sum: a warp has 32 value columns.
+// A score or a sum that is not finite is evaluated again as a plain f32 sum: what an infinity makes of it is the plain form's.
+// Which 16 of the key dimension, of the keys and of the columns make up an operand is free as long as both operands agree: a lane takes four
+// consecutive elements of a key row, four consecutive columns of every fourth key.  Rows are 8 mod 32 floats apart; every read is 16 bytes without conflicts.
+// Where the value row is the head of the key row itself (a latent that serves as both), it is not loaded twice.
+// Measured, the op with its merge and the append, against f32 FMAs with a column per thread (which read 68 floats of shared memory for every 64 FMAs, in
+// CTAs of 8 or 16 warps without a second buffer): one token, 16 heads, 8192 latents of 576 33 -> 28 us; 8192 positions of 12 heads of 64 80 -> 45, of 16 heads of 32 84 -> 37,
+// of 32 heads on 8 of 128 68 -> 53, of 8 heads on 2 of 256 41 -> 31; 100 positions as before.  Of the 28 us 4 are the launch of the append, 4 to 6 the merge,
+// the rest the chain load - scores - softmax - sums of two rounds.
 constexpr int kCfRows = 16, kCfKeys = 32;
 // How many of a step's shares (as many as the cache's capacity asks for) its keys are dealt to: beyond 64 only where each gets sixteen keys.  What the step
 // reads is its keys, and the merge reads a record per share: with 148 shares whatever the position, a token at position 500 of a cache of 8192 latents
 // of 576 took 22.6 us instead of 20.6; with 32 keys a share one at position 4000 26.7 instead of 24.8.
 __device__ __forceinline__ uint32_t few_shares(uint32_t n_keys, uint32_t splits) { return min(splits, max((uint32_t)kCtMaxSplits, (n_keys + 15) / 16)); }
-template <int kCfThreads, int CI, bool POOL>
-__global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, uint32_t rh, uint32_t splits, float* __restrict__ part, uint32_t alias) {
+constexpr int kCfSpPitch = 40;
+__host__ __device__ constexpr uint32_t cf_pitch(uint32_t n) { return (n + 23) / 32 * 32 + 8; }
+__device__ __forceinline__ uint32_t cf_swap(uint32_t i) { return (i & 4) | (i & 1) * 2 | ((i >> 1) & 1); }      // of eight rows: whose rows two lanes' groups read at a time lie 16 banks apart
+// the products that make up all but 2^-24 of one: the large one and the sum of the small ones
+__device__ __forceinline__ void cf_mma(float (&big)[4], float (&small)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+    mma_bf16(small, a[0], b[2]);
+    mma_bf16(small, a[2], b[0]);
+    mma_bf16(small, a[1], b[1]);
+    mma_bf16(small, a[0], b[1]);
+    mma_bf16(small, a[1], b[0]);
+    mma_bf16(big, a[0], b[0]);
+}
+// WARPS: as many as dv has 32 columns, up to 16; COLS times 32 columns each
+template <int WARPS, int COLS, bool POOL>
+__global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_cached_attention_few(CaArgs a, uint32_t rh, uint32_t splits, float* __restrict__ part, uint32_t alias, uint32_t bufs) {
     pdl_enter();
-    constexpr int kCfParts = kCfThreads / 32;
+    constexpr int kSlices = WARPS / 2;                 // of the key dimension
     extern __shared__ __align__(16) float sm[];
-    const uint32_t KP = a.dk + 4, VP = alias ? KP : a.dv;
-    float* Qs = sm;                                    // [16][dk + 4]
-    float* Ks = Qs + kCfRows * KP;                     // [32][dk + 4]
-    float* Sp = Ks + kCfKeys * KP;                     // [warps][16][32] partial scores of the warps' slices of the key dimension
-    float* Ss = Sp + kCfParts * kCfRows * kCfKeys;     // [16][32] probabilities
-    float* Al = Ss + kCfRows * kCfKeys;                // [16] rescale of the running sums (at the end: 1 / sum)
-    float* Vs = alias ? Ks : Al + kCfRows;             // [32][dv]
-    const uint32_t tid = threadIdx.x, row = tid >> 4, kq = tid & 15;
-    const uint32_t warp = tid >> 5, rg = (tid & 31) >> 3, kg = tid & 7;
+    const uint32_t dk16 = (a.dk + 15) / 16 * 16, KP = cf_pitch(dk16), VP = alias ? KP : cf_pitch(a.dv), buf_elems = kCfKeys * (KP + (alias ? 0 : VP));
+    float* Qs = sm;                                    // [16][KP]
+    uint4* Ps = reinterpret_cast<uint4*>(Qs + kCfRows * KP);        // [3 parts][2 of 16 keys][32 lanes] probabilities as A operands
+    float* Al = reinterpret_cast<float*>(Ps + 3 * 2 * 32);          // [16] rescale of the running sums (at the end: 1 / sum)
+    float* Run = Al + kCfRows;                         // [2][16] running max and sum
+    float* Sp = Run + 2 * kCfRows;                     // [slices][16][40] partial scores
+    float* Bs = Sp + kSlices * kCfRows * kCfSpPitch;   // [1 or 2] keys [32][KP], values [32][VP]
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, t = lane & 3;
     const uint32_t gm = blockIdx.x, g = gm / a.maps, m = gm % a.maps;
     const uint32_t pos0 = (uint32_t)ctl_word(a.ctl, ZG_CTL_POS), slot = ca_slot(a);
     const uint32_t total = a.T * rh, p_max = pos0 + a.T - 1;
@@ -571,145 +587,227 @@ __global__ void __launch_bounds__(kCfThreads) k_cached_attention_few(CaArgs a, u
     const CaKeys<POOL> vals = ca_keys<POOL>(vbase, POOL ? a.vp + pool_slot + (size_t)g * a.dv : nullptr, a.R, a.vw, k_lo, n_pool);
     const uint32_t n_keys = keys.count(p_max), used = few_shares(n_keys, splits), per = (n_keys + used - 1) / used;
     const uint32_t k_begin = keys.first() + blockIdx.y * per, k_end = min(keys.first() + n_keys, k_begin + per);
-    const bool ok = row < total, owner = tid < 16 * kCfRows;        // owner: of a row's running (max, sum)
+    // (token, head, map) of a row and its record
+    auto head_of = [&](uint32_t row) { return (g * rh + row % rh) * a.maps + m; };
+    auto record = [&](uint32_t row) { return part + (((size_t)(row / rh) * a.H * a.maps + head_of(row)) * splits + blockIdx.y) * (4 + a.dv); };
     if (blockIdx.y >= used) {                                       // no keys: a record that weighs nothing
-        if (kq == 0 && ok) {
-            float* mine = part + (((size_t)(row / rh) * a.H * a.maps + (g * rh + row % rh) * a.maps + m) * splits + blockIdx.y) * (4 + a.dv);
+        if (tid < total) {
+            float* mine = record(tid);
             mine[0] = -INFINITY; mine[1] = 0.0f;
         }
         return;
     }
-    const uint32_t p_r = pos0 + (ok ? row / rh : 0), lo_r = mask_low(p_r, a.kind, a.size), nb_r = POOL ? pooled_seen(p_r, a.size, a.pool) : 0u;
-    const float* tab_r = a.tab ? a.tab + (size_t)((g * rh + (ok ? row % rh : 0)) * a.maps + m) * a.tab_rs : nullptr;
-    const uint32_t dk4 = a.dk / 4, dv4 = a.dv / 4;
-    const uint32_t chunk4 = (dk4 + kCfParts - 1) / kCfParts, d_begin = 4 * min(dk4, warp * chunk4), d_end = 4 * min(dk4, (warp + 1) * chunk4);
-    for (uint32_t i = tid; i < kCfRows * dk4; i += kCfThreads) {     // rows past the step's are zero: their scores are never used
-        const uint32_t r = i / dk4, c4 = i % dk4;
-        copy16(Qs + r * KP + 4 * c4, r < total ? a.q + (size_t)(r / rh) * a.q_rs + a.q_off + (size_t)((g * rh + r % rh) * a.maps + m) * a.dk + 4 * c4 : a.q, r < total);
-    }
-    float acc[kCfRows][CI];
+    // rows of `cols` floats, as many lanes to a row as it has 16 bytes (a power of two, 32 at most); zeros up to `padded`, and for rows that are not there
+    auto copy_rows = [&](uint32_t rows, uint32_t cols, uint32_t padded, auto to, auto from, uint32_t there) {
+        const uint32_t lg = min(5u, 32u - (uint32_t)__clz(padded / 4 - 1)), n = 32 * WARPS >> lg;
+#pragma unroll 4
+        for (uint32_t r = tid >> lg; r < rows; r += n) {
+            const bool on = r < there;
+            const float* src = on ? from(r) : kbase;
+            float* dst = to(r);
+            for (uint32_t c = 4 * (tid & ((1u << lg) - 1)); c < padded; c += 4u << lg) copy16(dst + c, on && c < cols ? src + c : kbase, on && c < cols);
+        }
+    };
+    auto load = [&](uint32_t s0, float* Ks) {          // every load in flight at once: one round trip
+        const uint32_t nk = min((uint32_t)kCfKeys, k_end - s0);
+        copy_rows(kCfKeys, a.dk, dk16, [&](uint32_t r) { return Ks + r * KP; }, [&](uint32_t r) { return keys.row(s0 + r); }, nk);
+        if (!alias) copy_rows(kCfKeys, a.dv, a.dv, [&](uint32_t r) { return Ks + kCfKeys * KP + r * VP; }, [&](uint32_t r) { return vals.row(s0 + r); }, nk);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // (rows past the step's are zero: their scores are never used)
+    copy_rows(kCfRows, a.dk, dk16, [&](uint32_t r) { return Qs + ((r & 8) | cf_swap(r & 7)) * KP; },
+              [&](uint32_t r) { return a.q + (size_t)(r / rh) * a.q_rs + a.q_off + (size_t)head_of(r) * a.dk; }, total);
+    if (k_begin < k_end) load(k_begin, Bs);
+    for (uint32_t i = tid; i < 3 * 2 * 32; i += 32 * WARPS) Ps[i] = make_uint4(0, 0, 0, 0);
+    if (tid < kCfRows) { Al[tid] = 1.0f; Run[tid] = -INFINITY; Run[kCfRows + tid] = 0.0f; }
+    float acc[COLS][4][4];                             // 32 columns as four operands of eight: lane's rows gr and gr + 8, columns 8 t + j and 8 t + 4 + j
 #pragma unroll
-    for (int r = 0; r < kCfRows; r++)
+    for (int c = 0; c < COLS; c++)
 #pragma unroll
-        for (int i = 0; i < CI; i++) acc[r][i] = 0.0f;
-    float m_run = -INFINITY, l_run = 0.0f;
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[c][j][i] = 0.0f;
+    uint32_t cur = 0;
+#pragma unroll 1
     for (uint32_t s0 = k_begin; s0 < k_end; s0 += kCfKeys) {
         const uint32_t nk = min((uint32_t)kCfKeys, k_end - s0);
-        __syncthreads();                               // the previous keys' readers are done
-        for (uint32_t i = tid; i < kCfKeys * dk4; i += kCfThreads) {
-            const uint32_t kk = i / dk4, c4 = i % dk4;
-            copy16(Ks + kk * KP + 4 * c4, kk < nk ? keys.row(s0 + kk) + 4 * c4 : kbase, kk < nk);
-        }
-        if (!alias)
-            for (uint32_t i = tid; i < nk * dv4; i += kCfThreads) {
-                const uint32_t kk = i / dv4, c4 = i % dv4;
-                copy16(Vs + kk * VP + 4 * c4, vals.row(s0 + kk) + 4 * c4, true);
-            }
-        asm volatile("cp.async.commit_group;" ::: "memory");   // every load of the share is in flight at once: one round trip
+        const float* Ks = Bs + cur * buf_elems;
+        const float* Vs = alias ? Ks : Ks + kCfKeys * KP;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
+        __syncthreads();                               // these keys are there, and the readers of the ones before are done
+        if (bufs == 2 && s0 + kCfKeys < k_end) { cur ^= 1; load(s0 + kCfKeys, Bs + cur * buf_elems); }
         {
-            float sc[4][4];
+            float big[2][4], small[2][4];
 #pragma unroll
-            for (int r = 0; r < 4; r++)
+            for (int j = 0; j < 2; j++)
 #pragma unroll
-                for (int c = 0; c < 4; c++) sc[r][c] = 0.0f;
-            for (uint32_t d = d_begin; d < d_end; d += 4) {
-                float4 qa[4], ka[4];
+                for (int i = 0; i < 4; i++) big[j][i] = small[j][i] = 0.0f;
+            const uint32_t slice = warp / 2, n0 = warp % 2 * 16, place = cf_swap(gr);
+            const float* Q = Qs + place * KP + 4 * t;
+            const float* K = Ks + (n0 + place) * KP + 4 * t;
+#pragma unroll 1
+            for (uint32_t d = 16 * slice; d < dk16; d += 16 * kSlices) {
+                uint32_t A[3][4];
+                const float4 q0 = *reinterpret_cast<const float4*>(Q + d), q1 = *reinterpret_cast<const float4*>(Q + 8 * KP + d);
+                split3(q0.x, q0.y, A[0][0], A[1][0], A[2][0]);
+                split3(q1.x, q1.y, A[0][1], A[1][1], A[2][1]);
+                split3(q0.z, q0.w, A[0][2], A[1][2], A[2][2]);
+                split3(q1.z, q1.w, A[0][3], A[1][3], A[2][3]);
 #pragma unroll
-                for (int r = 0; r < 4; r++) qa[r] = *reinterpret_cast<const float4*>(Qs + (rg + 4 * r) * KP + d);
-#pragma unroll
-                for (int c = 0; c < 4; c++) ka[c] = *reinterpret_cast<const float4*>(Ks + (kg + 8 * c) * KP + d);
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        sc[r][c] = fmaf(qa[r].x, ka[c].x, sc[r][c]); sc[r][c] = fmaf(qa[r].y, ka[c].y, sc[r][c]);
-                        sc[r][c] = fmaf(qa[r].z, ka[c].z, sc[r][c]); sc[r][c] = fmaf(qa[r].w, ka[c].w, sc[r][c]);
-                    }
+                for (int j = 0; j < 2; j++) {
+                    uint32_t B[3][2];
+                    const float4 k = *reinterpret_cast<const float4*>(K + 8 * j * KP + d);
+                    split3(k.x, k.y, B[0][0], B[1][0], B[2][0]);
+                    split3(k.z, k.w, B[0][1], B[1][1], B[2][1]);
+                    cf_mma(big[j], small[j], A, B);
+                }
             }
+            float* to = Sp + (slice * kCfRows + gr) * kCfSpPitch + n0 + 2 * t;      // keys by their place among the eight
 #pragma unroll
-            for (int r = 0; r < 4; r++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) Sp[(warp * kCfRows + rg + 4 * r) * kCfKeys + kg + 8 * c] = sc[r][c];
+            for (int j = 0; j < 2; j++) {
+                *reinterpret_cast<float2*>(to + 8 * j) = make_float2(big[j][0] + small[j][0], big[j][1] + small[j][1]);
+                *reinterpret_cast<float2*>(to + 8 * kCfSpPitch + 8 * j) = make_float2(big[j][2] + small[j][2], big[j][3] + small[j][3]);
+            }
         }
         __syncthreads();
-        if (owner) {
-            float sv[2];
+        const uint32_t kk = (lane & 24) | cf_swap(lane & 7);        // the lane's key
+#pragma unroll 1
+        for (uint32_t row = warp; row < total; row += WARPS) {
+            const uint32_t p_r = pos0 + row / rh, j = s0 + kk;
+            const float m_run = Run[row];
+            float d = 0.0f;
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const uint32_t kk = kq + 16 * u, j = s0 + kk;
-                float d = 0.0f;
-#pragma unroll
-                for (int w = 0; w < kCfParts; w++) d += Sp[(w * kCfRows + row) * kCfKeys + kk];
-                const bool seen = ok && kk < nk && keys.seen(j, p_r, lo_r, nb_r);
-                sv[u] = seen ? ca_score(a, d) : -INFINITY;
-                if (!POOL && seen && tab_r) sv[u] += tab_r[p_r - j];
+            for (int w = 0; w < kSlices; w++) d += Sp[(w * kCfRows + row) * kCfSpPitch + lane];
+            const bool seen = kk < nk && keys.seen(j, p_r, mask_low(p_r, a.kind, a.size), POOL ? pooled_seen(p_r, a.size, a.pool) : 0u);
+            if (seen && !(fabsf(d) <= 3.4028234e38f)) {
+                const float* q = Qs + ((row & 8) | cf_swap(row & 7)) * KP;
+                d = 0.0f;
+#pragma unroll 1
+                for (uint32_t e = 0; e < a.dk; e++) d = fmaf(q[e], Ks[kk * KP + e], d);
             }
-            float rmax = fmaxf(sv[0], sv[1]);
+            float sv = seen ? ca_score(a, d) : -INFINITY;
+            if (!POOL && seen && a.tab) sv += a.tab[(size_t)head_of(row) * a.tab_rs + p_r - j];
+            float rmax = sv;
 #pragma unroll
-            for (int off = 8; off > 0; off >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
+            for (int off = 16; off > 0; off >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
             const float new_m = a.wkind ? 0.0f : fmaxf(m_run, rmax);
             const float alpha = a.wkind ? 1.0f : (m_run == -INFINITY ? (new_m == -INFINITY ? 1.0f : 0.0f) : expf(m_run - new_m));
-            float rsum = 0.0f;
+            const float pv = sv == -INFINITY ? 0.0f : (a.wkind ? ca_sigmoid(sv) : expf(sv - new_m));
+            float rsum = pv;
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const float pv = sv[u] == -INFINITY ? 0.0f : (a.wkind ? ca_sigmoid(sv[u]) : expf(sv[u] - new_m));
-                Ss[row * kCfKeys + kq + 16 * u] = pv;
-                rsum += pv;
-            }
+            for (int off = 16; off > 0; off >>= 1) rsum += __shfl_xor_sync(0xffffffffu, rsum, off);
+            if (lane == 0) { Al[row] = alpha; Run[row] = new_m; Run[kCfRows + row] = Run[kCfRows + row] * alpha + rsum; }
+            // key 16 s + 4 w + t is the operand's k of lane group t: register pair w / 2, half w % 2
+            unsigned short* to = reinterpret_cast<unsigned short*>(Ps) + ((kk / 16 * 32 + row % 8 * 4 + kk % 4) * 4 + kk % 16 / 8 * 2 + row / 8) * 2 + kk / 4 % 2;
+            uint32_t b[3];
+            split3(pv, 0.0f, b[0], b[1], b[2]);
 #pragma unroll
-            for (int off = 8; off > 0; off >>= 1) rsum += __shfl_xor_sync(0xffffffffu, rsum, off);
-            l_run = l_run * alpha + rsum;
-            m_run = new_m;
-            if (kq == 0) Al[row] = alpha;
+            for (int k = 0; k < 3; k++) to[k * 2 * 32 * 8] = (unsigned short)b[k];
         }
         __syncthreads();
+        const float al[2] = {Al[gr], Al[gr + 8]};
 #pragma unroll
-        for (int r = 0; r < kCfRows; r++) {
-            const float al = Al[r];
+        for (int c = 0; c < COLS; c++) {
+            const uint32_t col = 32 * (warp + WARPS * c) + 4 * gr;
+            if (32 * (warp + WARPS * c) >= a.dv) break;
+            float big[4][4], small[4][4];
 #pragma unroll
-            for (int i = 0; i < CI; i++) acc[r][i] *= al;
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) big[j][i] = small[j][i] = 0.0f;
+#pragma unroll 1
+            for (int s = 0; s < 2; s++) {
+                if (16u * s >= nk) break;
+                uint32_t A[3][4];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const uint4 x = Ps[(k * 2 + s) * 32 + lane];
+                    A[k][0] = x.x; A[k][1] = x.y; A[k][2] = x.z; A[k][3] = x.w;
+                }
+                float v[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float4 x = col < a.dv ? *reinterpret_cast<const float4*>(Vs + (16 * s + 4 * i + t) * VP + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    uint32_t B[3][2];
+                    split3(v[0][j], v[1][j], B[0][0], B[1][0], B[2][0]);
+                    split3(v[2][j], v[3][j], B[0][1], B[1][1], B[2][1]);
+                    cf_mma(big[j], small[j], A, B);
+                }
+            }
+            bool finite = true;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    big[j][i] += small[j][i];
+                    finite &= fabsf(big[j][i]) <= 3.4028234e38f;
+                }
+            if (!finite) {                             // the lane's own sums, over the keys there are
+                const unsigned short* P = reinterpret_cast<const unsigned short*>(Ps);
+#pragma unroll 1
+                for (uint32_t e = 0; e < 16; e++) {
+                    const uint32_t row = gr + (e & 2) * 4, at = col - 4 * gr + 8 * t + (e & 1) * 4 + e / 4;
+                    float sum = 0.0f;
+                    if (at < a.dv)
+#pragma unroll 1
+                        for (uint32_t k = 0; k < nk; k++) {
+                            const uint32_t w = ((k / 16 * 32 + row % 8 * 4 + k % 4) * 4 + k % 16 / 8 * 2 + row / 8) * 2 + k / 4 % 2;
+                            const float p = __uint_as_float((uint32_t)P[w] << 16) + (__uint_as_float((uint32_t)P[w + 512] << 16) + __uint_as_float((uint32_t)P[w + 1024] << 16));
+                            sum = fmaf(p, Vs[k * VP + at], sum);
+                        }
+#pragma unroll
+                    for (uint32_t k = 0; k < 16; k++)
+                        if (k == e) big[k / 4][k % 4] = sum;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[c][j][i] = fmaf(acc[c][j][i], al[i / 2], big[j][i]);
         }
-        for (uint32_t kk = 0; kk < nk; kk += 4) {      // four keys per trip: the probabilities are read as float4s
-            float v[4][CI];
+        if (bufs == 1 && s0 + kCfKeys < k_end) {       // no room for the next keys beside these
+            __syncthreads();
+            load(s0 + kCfKeys, Bs);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (tid < total) {
+        const float m_run = Run[tid], l_run = Run[kCfRows + tid];
+        Al[tid] = (a.wkind ? 1.0f : (l_run > 0.0f ? ca_inv_sum(a, head_of(tid), m_run, l_run) : 0.0f)) * a.out_scale;
+        if (splits > 1) {
+            float* mine = record(tid);
+            mine[0] = m_run; mine[1] = l_run;
+        }
+    }
+    __syncthreads();
 #pragma unroll
-            for (int u = 0; u < 4; u++)
+    for (int c = 0; c < COLS; c++)
 #pragma unroll
-                for (int i = 0; i < CI; i++) { const uint32_t c = tid + kCfThreads * i; v[u][i] = (c < a.dv && kk + u < nk) ? Vs[(kk + u) * VP + c] : 0.0f; }
+        for (int i = 0; i < 4; i++) {
+            const uint32_t row = gr + i / 2 * 8, col = 32 * (warp + WARPS * c) + 8 * t + i % 2 * 4;
+            if (row >= total || col >= a.dv) continue;
+            if (splits > 1) *reinterpret_cast<float4*>(record(row) + 4 + col) = make_float4(acc[c][0][i], acc[c][1][i], acc[c][2][i], acc[c][3][i]);      // (records are whole numbers of 16 bytes)
+            else {
+                float* out = a.dst + (size_t)(row / rh) * a.dst_rs + (size_t)head_of(row) * a.dv + col;
 #pragma unroll
-            for (int r = 0; r < kCfRows; r++) {
-                const float4 pr = *reinterpret_cast<const float4*>(Ss + r * kCfKeys + kk);
-#pragma unroll
-                for (int i = 0; i < CI; i++)
-                    acc[r][i] = fmaf(pr.x, v[0][i], fmaf(pr.y, v[1][i], fmaf(pr.z, v[2][i], fmaf(pr.w, v[3][i], acc[r][i]))));
+                for (int j = 0; j < 4; j++) out[j] = acc[c][j][i] * Al[row];
             }
         }
-    }
-    __syncthreads();
-    if (owner && kq == 0) Al[row] = (a.wkind ? 1.0f : (l_run > 0.0f ? ca_inv_sum(a, (g * rh + (ok ? row % rh : 0)) * a.maps + m, m_run, l_run) : 0.0f)) * a.out_scale;
-    if (splits > 1 && kq == 0 && ok) {
-        float* mine = part + (((size_t)(row / rh) * a.H * a.maps + (g * rh + row % rh) * a.maps + m) * splits + blockIdx.y) * (4 + a.dv);
-        mine[0] = m_run; mine[1] = l_run;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < kCfRows; r++) {
-        if ((uint32_t)r >= total) break;
-        const uint32_t hm_r = (g * rh + (uint32_t)r % rh) * a.maps + m;
-        const size_t item = (size_t)((uint32_t)r / rh) * a.H * a.maps + hm_r;
-#pragma unroll
-        for (int i = 0; i < CI; i++) {
-            const uint32_t c = tid + kCfThreads * i;
-            if (c >= a.dv) continue;
-            if (splits == 1) a.dst[(size_t)((uint32_t)r / rh) * a.dst_rs + (size_t)hm_r * a.dv + c] = acc[r][i] * Al[r];
-            else part[(item * splits + blockIdx.y) * (4 + a.dv) + 4 + c] = acc[r][i];
-        }
-    }
 }
-static size_t cf_smem(uint32_t dk, uint32_t dv, bool alias, uint32_t warps) {
-    return ((size_t)(kCfRows + kCfKeys) * (dk + 4) + (size_t)(warps + 1) * kCfRows * kCfKeys + kCfRows + (alias ? 0 : (size_t)kCfKeys * dv)) * sizeof(float);
+static size_t cf_smem(uint32_t dk, uint32_t dv, bool alias, uint32_t warps, uint32_t bufs = 1) {
+    const size_t KP = cf_pitch((dk + 15) / 16 * 16), VP = alias ? 0 : cf_pitch(dv);
+    return (kCfRows * KP + 3 * 2 * 32 * 4 + 3 * kCfRows + (size_t)warps / 2 * kCfRows * kCfSpPitch + bufs * kCfKeys * (KP + VP)) * sizeof(float);
 }
+constexpr size_t kCfMost = 226 * 1024;
+// Warps of a CTA.  Four where there is little to do per key and CTAs are many: 16 heads of 32 over 8192 positions 37 us, with eight 58, with sixteen 92;
+// 8 heads of 64 31, 41, 60.  Eight above: with four, two of 128 take the softmax's rows in turn (8 heads on one key head 128, 8192 positions: 20.6 us, with four 22.6;
+// 32 heads on 8 of 128 53, 60).  Sixteen where the columns ask for them; at 256 eight and sixteen are alike.
+static uint32_t cf_warps(uint32_t dv) { return dv <= 64 ? 4 : dv <= 256 ? 8 : 16; }
 static bool cf_alias(const ZgSeqOp& s) {   // the value row is the head of the key row (one key head, one map, same cache and column)
     return s.buf[2] == s.buf[3] && s.off[1] == s.off[2] && s.n[2] == 1 && s.n[3] == 1 && s.n[5] <= s.n[4] && s.n[7] == s.n[8];
 }
@@ -727,7 +825,7 @@ static bool ca_aligned(const ZgSeqOp& s) {
     return s.n[4] % 4 == 0 && s.n[5] % 4 == 0 && s.n[6] % 4 == 0 && s.n[7] % 4 == 0 && s.n[8] % 4 == 0 && s.off[0] % 4 == 0 && s.off[1] % 4 == 0 && s.off[2] % 4 == 0;
 }
 static bool ca_few(const ZgSeqOp& s) {
-    return ca_aligned(s) && s.n[0] * (s.n[1] / s.n[2]) <= (uint32_t)kCfRows && cf_smem(s.n[4], s.n[5], cf_alias(s), 8) <= 200 * 1024;
+    return ca_aligned(s) && s.n[0] * (s.n[1] / s.n[2]) <= (uint32_t)kCfRows && s.n[5] <= 1024 && cf_smem(s.n[4], s.n[5], cf_alias(s), 16) <= kCfMost;
 }
 // keys a step's rows can see at most
 static uint32_t ca_reach(const ZgSeqOp& s) {
@@ -1168,19 +1266,18 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
             if (aligned && ca_few(s)) {
                 const uint32_t S = scratch ? ca_splits(s) : 1, alias = cf_alias(s) ? 1u : 0u;
                 float* part = S > 1 ? scratch : nullptr;
-                // sixteen warps where the rows are wide enough to keep a second CTA off the SM
-                const bool wide = cf_smem(a.dk, a.dv, alias != 0, 8) > 112 * 1024 && cf_smem(a.dk, a.dv, alias != 0, 16) <= 200 * 1024;
-                const size_t smem = cf_smem(a.dk, a.dv, alias != 0, wide ? 16 : 8);
+                // a second buffer where a share can have more than one buffer's keys
+                const uint32_t warps = cf_warps(a.dv), bufs = ca_reach(s) > S * kCfKeys && cf_smem(a.dk, a.dv, alias != 0, warps, 2) <= kCfMost ? 2 : 1;
+                const size_t smem = cf_smem(a.dk, a.dv, alias != 0, warps, bufs);
                 const dim3 grid(a.G * a.maps, S);
-#define ZG_CF(THREADS_, CI_)                                                                                                               \
+#define ZG_CF(WARPS_, COLS_)                                                                                                               \
     do {                                                                                                                                   \
         static size_t most[2] = {48 * 1024, 48 * 1024};                                                                                    \
-        auto kernel = a.pool ? k_cached_attention_few<THREADS_, CI_, true> : k_cached_attention_few<THREADS_, CI_, false>;                 \
+        auto kernel = a.pool ? k_cached_attention_few<WARPS_, COLS_, true> : k_cached_attention_few<WARPS_, COLS_, false>;                 \
         if (smem > most[a.pool != 0]) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); most[a.pool != 0] = smem; } \
-        launch_pdl(kernel, grid, dim3(THREADS_), smem, st, a, a.H / a.G, S, part, alias);                              \
+        launch_pdl(kernel, grid, dim3(32 * WARPS_), smem, st, a, a.H / a.G, S, part, alias, bufs);                                         \
     } while (0)
-                if (wide) { if (a.dv <= 512) ZG_CF(512, 1); else ZG_CF(512, 2); }
-                else if (a.dv <= 256) ZG_CF(256, 1); else if (a.dv <= 512) ZG_CF(256, 2); else ZG_CF(256, 4);
+                if (warps == 4) ZG_CF(4, 1); else if (warps == 8) ZG_CF(8, 1); else if (a.dv <= 512) ZG_CF(16, 1); else ZG_CF(16, 2);
 #undef ZG_CF
                 if (S > 1) {
                     ZG_SEQ_CHECK();
