@@ -2289,7 +2289,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                                                   s.n[7] ? (const float*)bufs[s.buf[6]] : (const float*)nullptr, s.n[7] ? wptr<WT>(bufs, s.buf[2], s.off[2]) : (const WT*)nullptr,
                                                   s.n[8] ? s.n[8] - 1 : 0u, s.n[8] ? wptr<WT>(bufs, s.buf[2], s.off[5]) : (const WT*)nullptr));
                 // Four values a thread: with eight the unrolled code is twice as long and each launch fetches it anew (four feed-forwards of one token, 2048 / 4096,
-                // whose 2048 columns had 256 threads: 88 us, with 512 threads 76).
+                // whose 2048 columns had 256 threads: 88 us, with 512 threads 76, with 1024 of two values 80).
                 else if (s.n[1] <= 1024) ZG_NORM_ANY(4, 256);
                 else if (s.n[1] <= 2048) ZG_NORM_ANY(4, 512);
                 else ZG_NORM_ANY(4, 1024);                          // up to 4096 columns in registers; wider rows are walked from memory
