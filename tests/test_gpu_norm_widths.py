@@ -1,11 +1,12 @@
-"""NORM of few rows that closes a sublayer and opens the next (dst = res + src, then = rms(dst) w) at the widths where the threads per row change.
+"""NORM of few rows at the widths where the threads per row change: the step that closes a sublayer and opens the next (dst = res + src, then = rms(dst) w), and
+two sources, each normed on its own (dst = res + outer(rms(src) w + rms(src2) w2), then = rms(dst) w3).
 
 Tolerance: a sum of 4097 squares in f32, four to a thread and then over lanes and warps, is off by less than 2^-20 of itself, its root by half of that: 1e-5 of the
-largest output leaves room for the division and two products."""
+largest output leaves room for the division and two products.  With two sources two or three such norms follow one another: 2e-5."""
 import numpy as np
 import pytest
 
-from test_gpu_recops import run
+from test_gpu_recops import run, weights
 
 pytestmark = pytest.mark.gpu
 
@@ -24,4 +25,30 @@ def test_residual_then_rms(cuda_backend, rows, cols):
     for out, want in ((0, total), (4, total / np.sqrt((total ** 2).mean(1, keepdims=True) + 1e-5) * w)):
         got = run(cuda_backend, [op], sizes, io, out, x.shape, [ExternBuffer(2, buf)])
         assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+    buf.free()
+
+
+@pytest.mark.parametrize("cols", [1024, 1025, 2048, 2049, 3000, 4095, 4096, 4097])
+@pytest.mark.parametrize("outer", [False, True], ids=["plain", "outer"])
+@pytest.mark.parametrize("kind", ["rms", "layer"])
+def test_two_sources(cuda_backend, kind, outer, cols):
+    """The sources' sizes differ by 30, so that sums that were mixed up would show."""
+    from zgml_b200 import DeviceOp, ExternBuffer, abi
+    r = np.random.default_rng(cols)
+    rows = 2
+    x, y, res = (s * r.standard_normal((rows, cols)).astype(np.float32) for s in (np.float32(1), np.float32(30), np.float32(1)))
+    w = (1 + 0.3 * r.standard_normal((4, cols))).astype(np.float32)
+    buf, offs = weights(cuda_backend, *w)
+    op = DeviceOp.norm(0, 1, 2, offs[0], rows, cols, 1e-5, abi.W_F32, kind=kind, res=3, src2=5, src2_w_off=offs[1], outer=kind if outer else None, outer_w_off=offs[2], then=4, then_w=2,
+                       then_w_off=offs[3], then_kind="rms")
+
+    def normed(v, i, mean=kind == "layer"):
+        v = v - v.mean(1, keepdims=True) if mean else v
+        return v / np.sqrt((v ** 2).mean(1, keepdims=True) + 1e-5) * w[i].astype(np.float64)
+    total = normed(x.astype(np.float64), 0) + normed(y.astype(np.float64), 1)
+    total = res + (normed(total, 2) if outer else total)
+    sizes, io = [x.size, x.size, buf.elems, x.size, x.size, x.size], [(1, x), (3, res), (5, y)]
+    for out, want in ((0, total), (4, normed(total, 3, False))):
+        got = run(cuda_backend, [op], sizes, io, out, x.shape, [ExternBuffer(2, buf)])
+        assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
     buf.free()

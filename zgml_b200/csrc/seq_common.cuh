@@ -34,9 +34,11 @@ __device__ float block_sum(float v, float* sh) {
     for (int i = 0; i < nw; i++) r += sh[i];
     return r;
 }
-// two sums at once
-__device__ __forceinline__ float2 block_sum2(float a, float b, float* sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;   // at most 16 warps: sh holds 32 floats
+// two sums at once, of blocks of at most THREADS threads
+template <int THREADS, int N>
+__device__ __forceinline__ float2 block_sum2(float a, float b, float (&sh)[N]) {
+    static_assert(N >= THREADS / 16, "two floats a warp");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     a = warp_sum(a);
     b = warp_sum(b);
     __syncthreads();

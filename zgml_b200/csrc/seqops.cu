@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(kThreads) k_norm_any(float* dst, const float* 
                                                   float* dst2, const WT* __restrict__ w2, uint32_t kind2, float gain, const float* src_b, const WT* __restrict__ w_b,
                                                        uint32_t kind_o, const WT* __restrict__ w_o) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __shared__ float sh[32];
+    __shared__ float sh[kThreads > 512 ? kThreads / 16 : 32];      // of a warp: one sum, or the two sources'
     const size_t row = (size_t)blockIdx.x * cols;
     if (cols > kKeep * kThreads) {                  // rows too wide for the registers
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -688,7 +688,7 @@ __global__ void __launch_bounds__(kThreads) k_norm_any(float* dst, const float* 
         float q = 0.0f, qb = 0.0f;
 #pragma unroll
         for (int i = 0; i < kKeep; i++) { q = fmaf(v[i], v[i], q); qb = fmaf(vb[i], vb[i], qb); }
-        const float2 s2 = block_sum2(q, qb, sh);
+        const float2 s2 = block_sum2<kThreads>(q, qb, sh);
         inv = 1.0f / sqrtf(s2.x / (float)cols + eps); inv_b = 1.0f / sqrtf(s2.y / (float)cols + eps);
         mean = 0.0f;
     } else {
