@@ -1,13 +1,13 @@
 """LINEAR of up to eight rows over enough weight for the ring of slots: K within one piece of a row, of several and with a short last one, where 32, 64, 128 and
 256 threads share a row, fewer outputs than SMs and counts that do not divide among them, activations that fit shared memory and those that pass through
-in segments of K, strided and unaligned rows, and a weight that the program itself writes.
+in segments of K, strided and unaligned rows, rows of a state buffer's slot, and a weight that the program itself writes.
 
 Tolerance: a sum is added up in chains of at most 16 elements per 4 KB piece of a row (64 for K = 16384), then over 256 threads in a tree: below 100 roundings
 of 2^-24 of the sum of magnitudes."""
 import numpy as np
 import pytest
 
-from test_gpu_recops import run
+from test_gpu_recops import ctl_words, run
 
 pytestmark = pytest.mark.gpu
 
@@ -51,6 +51,31 @@ def test_linear_rows_through_the_ring(cuda_backend, M, N, K, fmt, pairs):
         got = run(cuda_backend, [op], [M * drs, src.size, buf.elems], [(1, src)], 0, (M, drs), [ExternBuffer(2, buf)])[:, :N]
         assert (np.abs(got - want) <= room).all(), unaligned
     buf.free()
+
+
+@pytest.mark.parametrize("M,K", [(1, 2056), (2, 2056), (3, 1032), (4, 4104), (8, 1032), (8, 6144)])
+@pytest.mark.parametrize("extra", [0, 1, 2, 3])
+@pytest.mark.parametrize("fmt", ["bfloat16", "float32"])
+def test_rows_of_a_slot(cuda_backend, fmt, extra, M, K):
+    """The source is the second slot of a state buffer whose slots lie any number of elements apart."""
+    from zgml_b200 import DeviceBuffer, DeviceOp, ExternBuffer, abi
+    from zgml_b200.host.weights import WeightArena
+    wdt = abi.W_F32 if fmt == "float32" else abi.W_BF16
+    r = np.random.default_rng(K + extra)
+    N, stride = 777, M * K + extra
+    W = _bf16(r.standard_normal((N, K)) / np.sqrt(K))
+    A = WeightArena(wdt)
+    ow = A.add("w", W)
+    buf = A.upload(cuda_backend)
+    slots = r.standard_normal(2 * stride).astype(np.float32)
+    state = DeviceBuffer(cuda_backend, slots.nbytes, zero=False)
+    state.upload(slots)
+    x, ww = slots[stride:stride + M * K].reshape(M, K).astype(np.float64), W.astype(np.float64)
+    op = DeviceOp.linear(0, 1, 2, ow, M, N, K, wdt, ctl=3, src_slot_stride=stride)
+    got = run(cuda_backend, [op], [M * N, state.elems, buf.elems, 8], [(3, ctl_words(0, 1))], 0, (M, N), [ExternBuffer(2, buf), ExternBuffer(1, state)])
+    assert (np.abs(got - x @ ww.T) <= 100 * 2.0 ** -24 * (np.abs(x) @ np.abs(ww).T)).all()
+    buf.free()
+    state.free()
 
 
 def test_a_weight_that_the_program_writes_is_read_after_it(cuda_backend):

@@ -266,9 +266,9 @@ __global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float
     bool warm = early && MR <= 4;
     if (!warm) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (ctl && !warm) src += (size_t)ctl_word(ctl, ZG_CTL_SLOT) * slot_stride;
-    const bool vec = ((reinterpret_cast<uintptr_t>(src) & 15) | (src_rs & 3)) == 0;
-    auto load_x = [&](uint32_t k0) {                    // K is a multiple of four
+    auto load_x = [&](uint32_t k0) {                    // K is a multiple of four; the rows of a state buffer's slot start anywhere
         const uint32_t n = min(xw, K - k0);
+        const bool vec = ((reinterpret_cast<uintptr_t>(src) & 15) | (src_rs & 3)) == 0;
         for (uint32_t m = 0; m < M; m++) {
             const float* from = src + (size_t)m * src_rs + k0;
             if (vec) for (uint32_t k = 4 * tid; k < n; k += 1024) *reinterpret_cast<float4*>(xs + m * xw + k) = *reinterpret_cast<const float4*>(from + k);
