@@ -256,7 +256,12 @@ __global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float
                     } else if (lane < n) {
                         bulk_load(reinterpret_cast<float*>(to + lane * kRingPiece), reinterpret_cast<const float*>(from + (size_t)lane * row_bytes), bytes, bar);
                     }
-                    if (++slot == kRingSlots) { slot = 0; if (again) parity ^= 1; again = true; }
+                    if (++slot == kRingSlots) {
+                        slot = 0;
+                        if (again) parity ^= 1;
+                        else asm volatile("griddepcontrol.wait;" ::: "memory");      // slots come free when the predecessor has completed, however long that takes: no bounded wait before
+                        again = true;
+                    }
                 }
         }
         return;
