@@ -1,6 +1,8 @@
 """Sequence ops where the scratch that their faster forms stage in cannot be had (ZG_CUDA_SCRATCH_MB refuses every allocation): the program compiles all the same
 and the forms without scratch answer as the others do.
 
+Where only the LINEAR's cut source has no room, the form that cuts it as it goes gives the same sums, bit for bit.
+
 Tolerance: two f32 evaluations of the same sums, each within 1e-5 of the result's largest value of the true one (the bars of the ops' own tests)."""
 import numpy as np
 import pytest
@@ -68,3 +70,19 @@ def test_without_scratch(cuda_backend, monkeypatch, make):
         for b in owned:
             b.free()
     assert np.abs(outs[0] - outs[1]).max() <= 2e-5 * np.abs(outs[0]).max()
+
+
+def test_without_room_for_the_cut_source(cuda_backend, monkeypatch):
+    """150 tiles of one share each: the parts of the source are all that it stages (1.8 MB)."""
+    from zgml_b200 import DeviceOp, ExternBuffer, abi
+    r = np.random.default_rng(3)
+    M, N, K = 600, 3800, 512
+    w, (ow,) = weights(cuda_backend, r.standard_normal((N, K)))
+    x = r.standard_normal((M, K)).astype(np.float32)
+    outs = []
+    for limit in (None, "1"):
+        if limit:
+            monkeypatch.setenv("ZG_CUDA_SCRATCH_MB", limit)
+        outs.append(run(cuda_backend, [DeviceOp.linear(0, 1, 2, ow, M, N, K, abi.W_F32)], [M * N, x.size, w.elems], [(1, x)], 0, (M, N), [ExternBuffer(2, w)]))
+    assert np.array_equal(outs[0], outs[1])
+    w.free()

@@ -345,12 +345,16 @@ static bool validate_ops(const ZgCudaProgram* p, const ZgOp* ops, size_t n_ops) 
 static bool build_schedule(ZgCudaProgram* p);
 
 static bool reserve_workspace(ZgCudaProgram* p) {
-    size_t pe = 0, nc = 0, gs = 0, seq = 0;
+    size_t pe = 0, nc = 0, gs = 0, seq = 0, least = 0;
     p->ws_part_off.assign(p->ops.size(), 0);
     p->ws_cnt_off.assign(p->ops.size(), 0);
     for (size_t i = 0; i < p->ops.size(); i++) {
         const ZgOp& op = p->ops[i];
-        if (zg_is_seq_op(op.tag)) { const size_t g = zg_seq_op_scratch_elems(op, p->buffers.data()); if (g > seq) seq = g; continue; }
+        if (zg_is_seq_op(op.tag)) {
+            seq = std::max(seq, zg_seq_op_scratch_elems(op, p->buffers.data()));
+            least = std::max(least, zg_seq_op_scratch_elems(op, p->buffers.data(), true));
+            continue;
+        }
         if (op.tag != ZG_OP_QMATMUL) continue;
         size_t a = 0, b = 0;
         zg_qgemv_ws_need(p->ctx, p->qweights[op.u.qmatmul.weight_idx], op.u.qmatmul.M, &a, &b);
@@ -359,7 +363,8 @@ static bool reserve_workspace(ZgCudaProgram* p) {
         const size_t g = zg_qgemm_scratch_elems(p->qweights[op.u.qmatmul.weight_idx], op.u.qmatmul.M);
         if (g > gs) gs = g;
     }
-    if (zg_gemv_ws_reserve(&p->ws, pe, nc, p->ctx->stream, gs > seq ? gs : seq)) return true;
+    if (zg_gemv_ws_reserve(&p->ws, pe, nc, p->ctx->stream, std::max(gs, seq))) return true;
+    if (least < seq && zg_gemv_ws_reserve(&p->ws, pe, nc, p->ctx->stream, std::max(gs, least))) return true;
     p->lean = true;                                                  // no room for what the sequence ops stage: they have kernels that need none
     return seq > gs && zg_gemv_ws_reserve(&p->ws, pe, nc, p->ctx->stream, gs);
 }
@@ -1792,7 +1797,7 @@ static bool launch_one(ZgCudaProgram* p, size_t i, cudaStream_t st) {
         }
     }
     if (zg_op_is_batched(op.tag)) return zg_launch_batch(op, p->d_batch + p->single_entry[i], 1, p->d_dyn, st);
-    if (zg_is_seq_op(op.tag)) return zg_launch_seq_op(ctx, op, p->buffers.data(), p->lean ? nullptr : p->ws.gemm_scratch, st, const_weights(p, op));
+    if (zg_is_seq_op(op.tag)) return zg_launch_seq_op(ctx, op, p->buffers.data(), p->lean ? nullptr : p->ws.gemm_scratch, p->ws.gemm_scratch_elems, st, const_weights(p, op));
     return zg_launch_op(ctx, op, p->buffers.data(), p->d_dyn, (uint32_t)i, p->d_steps + p->step_off[i], st);
 }
 

@@ -2182,7 +2182,7 @@ static bool linear_split(const ZgSeqOp& s, float* const* bufs) {     // f32 weig
     return zg_split_gemm_usable(wptr<float>(bufs, s.buf[2], s.off[0]), bufs[s.buf[1]] + s.off[2], s.n[0], s.n[10] ? 2 * s.n[1] : s.n[1], s.n[2], s.n[3], s.n[7]);
 }
 unsigned int zg_seq_timeouts() { return tc_timeouts(); }
-size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs) {
+size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs, bool least) {
     if (op.tag >= ZG_OP_STREAM_STEP) return 0;
     if (op.tag >= ZG_OP_SSM_SCAN) return zg_rec_op_scratch_elems(op);
     if (op.tag >= ZG_OP_TOKEN_SHIFT) return zg_mix_op_scratch_elems(op);
@@ -2198,7 +2198,7 @@ size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs) {
     }
     if (!dense_gemm_enabled() || op.tag != ZG_OP_LINEAR) return 0;
     const ZgSeqOp& s = op.u.seq;
-    if (s.n[5] == ZG_W_F32) return linear_split(s, bufs) ? zg_split_gemm_scratch_elems(s.n[0], s.n[10] ? 2 * s.n[1] : s.n[1], s.n[2]) : 0;
+    if (s.n[5] == ZG_W_F32) return linear_split(s, bufs) ? zg_split_gemm_scratch_elems(s.n[0], s.n[10] ? 2 * s.n[1] : s.n[1], s.n[2], least) : 0;
     if (!zg_dense_gemm_usable(wptr<bf16>(bufs, s.buf[2], s.off[0]), s.n[0], s.n[10] ? 2 * s.n[1] : s.n[1], s.n[2])) return 0;
     return zg_dense_gemm_scratch_elems(s.n[0], s.n[2]);
 }
@@ -2218,7 +2218,7 @@ static void launch_linear_ring(bool pairs, float* dst, const float* src, const W
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem);
     launch_pdl(kern, dim3(r.ctas), dim3(288), r.smem, st, dst, src, W, bias, M, N, K, src_rs, dst_rs, act, ctl, slot_stride, r.lanes, r.segment, r.rows, early ? 1u : 0u);
 }
-bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st, bool const_weights) {
+bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool const_weights) {
     (void)ctx;
     const ZgSeqOp& s = op.u.seq;
     switch (op.tag) {
@@ -2238,7 +2238,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             const float* slot_ctl = s.n[7] ? (const float*)bufs[s.buf[4]] : (const float*)nullptr;      // the source is the slot's part of a state buffer
             if (scratch && s.n[5] == ZG_W_F32 && zg_seq_op_scratch_elems(op, bufs))
                 return zg_split_gemm_launch(wptr<float>(bufs, s.buf[2], s.off[0]), has_bias ? wptr<float>(bufs, s.buf[3], s.off[1]) : nullptr, src, dst, M, pairs ? 2 * N : N, K,
-                                            s.n[3], s.n[4], scratch, st, s.n[6], s.f[0], act.lo, act.hi, slot_ctl, s.n[7], pairs, s.n[11]);
+                                            s.n[3], s.n[4], scratch, scratch_elems, st, s.n[6], s.f[0], act.lo, act.hi, slot_ctl, s.n[7], pairs, s.n[11]);
             if (scratch && zg_seq_op_scratch_elems(op, bufs))
                 return zg_dense_gemm_launch(wptr<bf16>(bufs, s.buf[2], s.off[0]), has_bias ? wptr<bf16>(bufs, s.buf[3], s.off[1]) : nullptr, src, dst, M, N, K,
                                             s.n[3], s.n[4], scratch, st, s.n[6], s.f[0], act.lo, act.hi, slot_ctl, s.n[7], pairs, s.n[11]);

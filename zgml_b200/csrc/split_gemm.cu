@@ -296,19 +296,19 @@ size_t plane_elems(uint32_t M, uint32_t N, uint32_t K) { return split_first(M, N
 bool zg_split_gemm_usable(const float* w, const float* src, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t slot_stride) {
     return M > 8 && N >= 32 && K >= 64 && K % 4 == 0 && src_rs % 4 == 0 && slot_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
 }
-size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K) {      // never 0, which stands for the plain kernel
+size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K, bool least) {      // never 0, which stands for the plain kernel
     const uint32_t s = shares(M, N, K, zg_sm_count());
-    return (s > 1 ? (size_t)s * M * up4(N) : 4) + plane_elems(M, N, K);
+    return (s > 1 ? (size_t)s * M * up4(N) : 4) + (least ? 0 : plane_elems(M, N, K));
 }
 unsigned int zg_split_gemm_timeouts() { return tc_timeouts(); }
-bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, cudaStream_t st,
-                          uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from) {
+bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, size_t scratch_elems,
+                          cudaStream_t st, uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from) {
     if (!zg_smem_limit<k_split_gemm<false>>(kSgSmem) || !zg_smem_limit<k_split_gemm<true>>(kSgSmem)) return false;
     SgArgs a = {src, w, scratch, M, N, K, src_rs, up4(N), shares(M, N, K, zg_sm_count()), ctl, slot_stride, rows_from, dst, bias, dst_rs, (uint32_t)pairs, SeqAct{act, act_p, act_lo, act_hi}, nullptr, 0};
     const dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, a.splits);
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
-    if (split_first(M, N, K)) {
+    if (split_first(M, N, K) && scratch_elems >= zg_split_gemm_scratch_elems(M, N, K, false)) {      // where the planes found no room, the workers cut the source as they go
         a.planes = reinterpret_cast<uint16_t*>(scratch);
         a.pitch = up8(K);
         a.part = scratch + plane_elems(M, N, K);

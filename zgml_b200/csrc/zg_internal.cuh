@@ -399,9 +399,10 @@ inline bool zg_is_seq_op(uint32_t tag) { return tag >= ZG_OP_EMBED && tag < ZG_O
 bool zg_seq_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* why, size_t why_n);
 uint32_t zg_seq_op_writes(uint32_t tag);
 unsigned int zg_seq_timeouts();       // waits that gave up (DELTA_RULE's walk)
-size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs);   // shared activation scratch the op stages through (0: none)
+// shared activation scratch the op stages through (0: none); least: what that form does not work without
+size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs, bool least = false);
 // const_weights: nothing writes the op's weight (buf 2) while the program runs, so that it may be read before the launch's predecessor has completed
-bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st, bool const_weights);
+bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool const_weights);
 // dense_gemm.cu : bf16 x bf16 -> f32 prefill matmul on tcgen05 (TMA-fed, TMEM accumulator)
 bool zg_dense_gemm_usable(const void* w_bf16, uint32_t M, uint32_t N, uint32_t K);
 size_t zg_dense_gemm_scratch_elems(uint32_t M, uint32_t K);
@@ -412,10 +413,10 @@ bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void
                            float limit, float alpha, float up_offset, cudaStream_t st);
 // split_gemm.cu : f32 x f32 -> f32 LINEAR of many rows, operands cut into three bfloat16 parts (arguments as zg_dense_gemm_launch's; N counts weight rows)
 bool zg_split_gemm_usable(const float* w, const float* src, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t slot_stride);
-size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K);
+size_t zg_split_gemm_scratch_elems(uint32_t M, uint32_t N, uint32_t K, bool least);      // least: it does with so much, and is slower for it
 unsigned int zg_split_gemm_timeouts();
-bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, cudaStream_t st,
-                          uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from);
+bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, float* dst, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, float* scratch, size_t scratch_elems,
+                          cudaStream_t st, uint32_t act, float act_p, uint32_t act_lo, uint32_t act_hi, const float* ctl, uint32_t slot_stride, bool pairs, uint32_t rows_from);
 // mixops.cu : ZG_OP_TOKEN_SHIFT .. ZG_OP_POLY_NORM, reached through the functions above
 bool zg_mix_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* why, size_t why_n);
 uint32_t zg_mix_op_writes(uint32_t tag);
