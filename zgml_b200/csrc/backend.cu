@@ -2191,7 +2191,7 @@ extern "C" int zg_cuda_program_promote_dense(ZgCudaCtx* ctx, ZgCudaProgram* p, i
 extern "C" uint64_t zg_cuda_program_stats(const ZgCudaProgram* p, int what) {
     if (!p) return 0;
     switch (what) {
-        case 5: return zg_dense_gemm_timeouts() + zg_split_gemm_timeouts() + zg_attention_tc_timeouts() + zg_seq_timeouts();
+        case 5: return zg_dense_gemm_timeouts() + zg_split_gemm_timeouts() + zg_attention_tc_timeouts() + zg_seq_timeouts() + zg_qgemv_rows_timeouts();
         case 6: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && op.u.seq.n[5] == ZG_W_BF16 && zg_seq_op_scratch_elems(op, p->buffers.data())) n++; return n; }
         case 7: return p->ws.gemm_scratch_elems;
         case 0: return p->graph_kernels;

@@ -13,7 +13,7 @@
 // in fixed order.  With S > 1 the CTAs of a column group are a cluster (S = 2, 4, 8) and add their sums over distributed shared memory, several column groups at a
 // time, or meet in global scratch.
 // The C operand leaves all three digits of (column g, rows 2 t and 2 t + 1) in one lane: they are put together without shuffles.
-#include "zg_internal.cuh"
+#include "split_tc.cuh"
 
 #include <algorithm>
 #include <string.h>
@@ -44,16 +44,6 @@ __device__ __forceinline__ void imma_u8u8(int (&d)[4], const uint32_t (&a)[4], u
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t rows_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-constexpr uint32_t kRowsSpin = 1u << 22;       // polls after which a wait gives up
-__device__ __forceinline__ bool rows_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kRowsSpin; i++) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
 __device__ __forceinline__ uint4 rows_lds128(uint32_t addr) {
     uint4 r;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(addr));
@@ -83,14 +73,14 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qgemv_rows_kernel(const __gri
     extern __shared__ __align__(128) uint8_t dsm[];      // [warp][slot][G records] | [warp][row][L records of 32] | [warp][slot] mbarriers
     constexpr uint32_t W = kRowsWarps / TEAMS;           // warps of a team
     const uint32_t tid = threadIdx.x % (32 * W), lane = tid & 31, warp = threadIdx.x >> 5, team = TEAMS == 1 ? 0 : threadIdx.x / (32 * W), g = lane >> 2, t = lane & 3, of_team = warp % W;
-    auto sync = [&] { if (TEAMS == 1) __syncthreads(); else asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(32 * W) : "memory"); };
+    auto sync = [&] { if (TEAMS == 1) __syncthreads(); else bar_sync(1 + team, 32 * W); };
     const uint32_t split = blockIdx.x % p.S, grp = blockIdx.x / p.S, nb_begin = grp * p.P, nb_end = min(nb_begin + p.P, p.n_nb);
     const uint32_t ks = (uint32_t)(((uint64_t)split * p.n_kc) / p.S), ke = (uint32_t)(((uint64_t)(split + 1) * p.n_kc) / p.S);
     const uint32_t k0 = ks + of_team * (ke - ks) / W, L = ks + (of_team + 1) * (ke - ks) / W - k0;      // this warp's records of a column group
     const uint32_t NS = p.NS, n_chunk = (L + G - 1) / G, row_elems = p.L * ZG_KR;
-    const uint32_t ring = rows_smem(dsm) + warp * NS * G * RB;
+    const uint32_t ring = smem_u32(dsm) + warp * NS * G * RB;
     float* xs = reinterpret_cast<float*>(dsm + kRowsWarps * NS * G * RB) + (size_t)warp * p.M * row_elems;
-    const uint32_t bars = rows_smem(dsm) + kRowsWarps * (NS * G * RB + p.M * row_elems * 4) + warp * NS * 8;
+    const uint32_t bars = smem_u32(dsm) + kRowsWarps * (NS * G * RB + p.M * row_elems * 4) + warp * NS * 8;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // weights are immutable: the first NS slots are asked for before the wait on the predecessor
     const uint32_t nb0 = nb_begin + team;
@@ -98,7 +88,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qgemv_rows_kernel(const __gri
     const uint8_t* ask_src = p.recs + ((size_t)nb0 * p.n_kc + k0) * RB;
     auto ask = [&] {                                     // lane 0
         const uint32_t bytes = min(G, L - ask_c * G) * RB, bar = bars + ask_slot * 8;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        mbar_expect_tx(bar, bytes);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                      ::"r"(ring + ask_slot * G * RB), "l"(ask_src + (size_t)ask_c * G * RB), "r"(bytes), "r"(bar) : "memory");
         ask_left--;
@@ -106,7 +96,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qgemv_rows_kernel(const __gri
         if (++ask_slot == NS) ask_slot = 0;
     };
     if (lane == 0) {
-        for (uint32_t s = 0; s < NS; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + s * 8), "r"(1) : "memory");
+        for (uint32_t s = 0; s < NS; s++) mbar_init(bars + s * 8, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         for (uint32_t i = 0; i < NS && ask_left; i++) ask();
     }
@@ -148,8 +138,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qgemv_rows_kernel(const __gri
         __syncwarp();
     }
     const uint32_t row = min(g, p.M - 1);                // columns past the last row repeat it
-    const uint32_t x_lo = rows_smem(xs + row * row_elems) + 16 * (t ^ ((row & 1) << 2)), x_hi = rows_smem(xs + row * row_elems) + 16 * ((4 + t) ^ ((row & 1) << 2));
-    bool ok = true;                                      // a wait that gave up: the sums are not numbers
+    const uint32_t x_lo = smem_u32(xs + row * row_elems) + 16 * (t ^ ((row & 1) << 2)), x_hi = smem_u32(xs + row * row_elems) + 16 * ((4 + t) ^ ((row & 1) << 2));
+    bool ok = true;                                      // a wait that gave up: the warp's sums are not numbers (one lane's operands enter them all)
     uint32_t slot = 0, parity = 0, held = 0, half = 0;   // cluster: column groups whose sums wait, in the half of xpart at `half`
     const uint32_t hold = nb_end - nb_begin <= kRowsHeld ? kRowsHeld : kRowsHeld / 2;
     for (uint32_t nb = nb0; nb < nb_end; nb += TEAMS) {
@@ -164,7 +154,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qgemv_rows_kernel(const __gri
         uint32_t dsum[3] = {};
         for (uint32_t c = 0; c < n_chunk; c++) {
             const uint32_t cnt = min(G, L - c * G), base = ring + slot * G * RB;
-            if (!rows_wait(bars + slot * 8, parity)) ok = false;
+            if (!__all_sync(0xffffffffu, mbar_wait(bars + slot * 8, parity))) ok = false;
 #pragma unroll
             for (uint32_t r = 0; r < G; r++) {
                 if (r >= cnt) break;
@@ -272,7 +262,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qgemv_rows_kernel(const __gri
                 v = 0.0f;
                 for (uint32_t s2 = 0; s2 < p.S; s2++) {
                     uint32_t remote; float x;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(rows_smem(&xpart[half + i][m][col])), "r"(s2));
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&xpart[half + i][m][col])), "r"(s2));
                     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote) : "memory");
                     v += x;
                 }
@@ -295,6 +285,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qgemv_rows_kernel(const __gri
             }
         }
     }
+    if (!ok && lane == 0) count_timeout();
     if (TEAMS == 1 && p.S > 1 && p.cl) rows_cluster_sync();      // nobody leaves while another may still read its partials
 }
 
@@ -365,3 +356,4 @@ bool zg_qgemv_rows_launch(ZgCudaCtx* ctx, uint32_t count, const ZgCudaQWeight* c
         default: zg_set_error("qmatmul: unknown weight format %d", w[0]->fmt); return false;
     }
 }
+unsigned int zg_qgemv_rows_timeouts() { return tc_timeouts(); }

@@ -210,7 +210,7 @@ static RingPlan ring_plan(uint32_t M, uint32_t N, uint32_t K, bool pairs, uint32
     r.split = M > 2 && (size_t)M * K * 4 > kRingX;
     r.segment = r.split ? std::min(pieces, std::max(1u, kRingX / (M * (kRingPiece / elem) * 4))) : pieces;
     r.rows = r.split ? ((N + r.ctas - 1) / r.ctas * (pairs ? 2 : 1) + 7) / 8 * 8 : 2 * kRingFlush;
-    const size_t x = r.split ? (size_t)M * r.segment * (kRingPiece / elem) : (size_t)M * K, smem = kRingSlots * kRingSlot + ((size_t)r.rows * 8 * M + x) * 4 + 16 * kRingSlots;
+    const size_t x = r.split ? (size_t)M * r.segment * (kRingPiece / elem) : (size_t)M * K, smem = kRingSlots * kRingSlot + ((size_t)r.rows * 8 * M + x) * 4 + 16 * kRingSlots + 16;
     r.smem = smem <= 227 * 1024 ? (uint32_t)smem : 0;                 // 0: it does not fit
     return r;
 }
@@ -230,8 +230,9 @@ __global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float
     float* part = reinterpret_cast<float*>(ring + kRingSlots * kRingSlot);      // [row][m][share], twice 64 rows or all of them
     float* xs = part + part_rows * 8 * M;                                       // [m][a segment of K]
     const uint32_t xw = SPLIT ? segment * piece_k : K;
-    const uint32_t bars = smem_u32(xs + M * xw), pitch = pieces == 1 ? row_bytes : kRingPiece;
+    const uint32_t bars = smem_u32(xs + M * xw), pitch = pieces == 1 ? row_bytes : kRingPiece, failed = bars + 16 * kRingSlots;      // failed: some thread's wait gave up: the CTA's outputs are not numbers
     if (tid == 0) {
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(failed), "r"(0) : "memory");
         for (uint32_t i = 0; i < kRingSlots; i++) { mbar_init(bars + 8 * i, 1); mbar_init(bars + 8 * (kRingSlots + i), 8); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float
             const uint32_t s1 = SPLIT ? min(pieces, s0 + segment) : pieces;
             for (uint32_t first = 0; first < rows; first += group)
                 for (p = s0; p < s1; p++) {
-                    if (again && !mbar_wait(bars + 8 * (kRingSlots + slot), parity)) { if (lane == 0) count_timeout(); return; }
+                    if (again && !__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kRingSlots + slot), parity))) { if (lane == 0) count_timeout(); return; }
                     const uint32_t n = min(group, rows - first), bytes = min(kRingPiece, row_bytes - p * kRingPiece), bar = bars + 8 * slot;
                     unsigned char* to = ring + slot * kRingSlot;
                     const char* from = w0 + (size_t)first * row_bytes + p * kRingPiece;
@@ -282,7 +283,6 @@ __global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float
         bar_sync(1, 256);
     };
     if (!warm) load_x(0);
-    bool ok = true;
     constexpr bool TWO = MR <= 2;                       // sums of even and of odd elements, by packed FMAs, where the registers allow it
     float2 acc[8][MR];
     uint32_t slot = 0, parity = 0, done = 0, half = 0;       // done: rows whose outputs are written; half: of `part`, where a flush of 64 rows reads one and the next fills the other
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float
                 const float* s = part + ((size_t)(half * kRingFlush + row) * M + m) * 8;
                 float t = s[0];
                 for (uint32_t i = 1; i < shares; i++) t += s[i];
-                return ok ? t : __uint_as_float(0x7fffffffu);
+                return t;
             };
             if (PAIRS) dst[(size_t)m * dst_rs + n] = seq_epilogue(sum(2 * o), act.kind, act.p) * sum(2 * o + 1);
             else dst[(size_t)m * dst_rs + n] = seq_epilogue(sum(o) + (bias ? wld(bias, n) : 0.0f), act, n);
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float
 #pragma unroll
                 for (int m = 0; m < MR; m++) acc[r][m] = make_float2(0.0f, 0.0f);
         }
-        if (!mbar_wait(bars + 8 * slot, parity)) ok = false;
+        if (!mbar_wait(bars + 8 * slot, parity)) asm volatile("st.shared.u32 [%0], %1;" ::"r"(failed), "r"(1) : "memory");
         const uint32_t k = p * piece_k + unit * V;
         if (k < K) {
             const unsigned char* w = ring + slot * kRingSlot + (size_t)sub * 8 * pitch + unit * 16;
@@ -380,7 +380,14 @@ __global__ void __launch_bounds__(288, MR <= 2 ? 2 : 1) k_linear_rows_ring(float
         }
     }
     if (SPLIT) flush(rows);
-    if (!ok && lane == 0) count_timeout();
+    uint32_t gave_up;                                  // every wait is behind the last barrier
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(gave_up) : "r"(failed) : "memory");
+    if (gave_up) {
+        bar_sync(1, 256);
+        for (uint32_t m = 0; m < M; m++)
+            for (uint32_t n = n0 + tid; n < n1; n += 256) dst[(size_t)m * dst_rs + n] = __uint_as_float(0x7fffffffu);
+        if (tid == 0) count_timeout();
+    }
 }
 
 // ── LINEAR, many rows (prefill), exact f32: 64 x 64 tile, 16-deep k slices, 4 x 4 outputs per thread ──────────────────
@@ -1502,6 +1509,7 @@ template <int SL, int WARPS, bool PLAIN>
 __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ dst, const float* __restrict__ prep, float* __restrict__ state, const float* __restrict__ ctl,
                                                            uint32_t T, uint32_t H, uint32_t dim, uint32_t vdim, uint32_t dst_rs, uint32_t stages) {
     extern __shared__ __align__(16) float sm[];
+    __shared__ uint32_t failed;                                       // some thread's wait gave up: the CTA's outputs and its part of the state are not numbers
     constexpr uint32_t C = kWalkChunk, QR = PLAIN ? 0 : C, dpad = 16 * SL * WARPS, xs = dpad + 8, vec_elems = delta_vec_elems(dpad, PLAIN), NT = 32 * WARPS, PER = 256 / NT;
     constexpr uint32_t stage_elems = vec_elems + 512, slices = SL * WARPS;      // of a stage: the chunk's vectors, [Vt | Vo] of the CTA's columns
     const uint32_t h = blockIdx.y, col0 = blockIdx.x * kWalkCols, chunks = (T + C - 1) / C, tid = threadIdx.x % NT, lane = tid & 31, warp = tid >> 5;
@@ -1514,6 +1522,7 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
     const size_t stride = delta_chunk_elems(dpad, PLAIN, vdim);
     const float* P = prep + (size_t)h * chunks * stride;
     if (threadIdx.x == NT) {
+        failed = 0;
         for (uint32_t i = 0; i < stages; i++) mbar_init(bars + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1528,7 +1537,6 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
         bulk_load(to + vec_elems, src + vec_elems + blockIdx.x * 512, 2048, bars + 8 * i);
     };
     if (threadIdx.x == NT) for (uint32_t b = 0; b + 1 < stages || b == 0; b++) stage(b, b);
-    bool ok = true;                                                   // a wait that gave up: the outputs and the state are not numbers
     const uint32_t g = lane >> 2, t = lane & 3;
     // element e of a chunk's 16 x 16 u or o, in the order of the accumulators that hold them
     auto tok_of = [](uint32_t e) { return (e >> 7) * 8 + 2 * ((e >> 2) & 3) + (e & 1); };
@@ -1582,7 +1590,7 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
 #pragma unroll 1
         for (uint32_t b = 0; b < chunks; b++) {
             const float* X = sm + cur * stage_elems;
-            if (!mbar_wait(bars + 8 * cur, parity)) ok = false;
+            if (!mbar_wait(bars + 8 * cur, parity)) failed = 1;
             uint32_t q[SL][2][3][2];
             vectors(X + QR * xs, q);
             __syncthreads();                                          // the parts of S are there, and the chunk before is done with
@@ -1599,12 +1607,17 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
             for (uint32_t p = 0; p < PER; p++) {
                 const uint32_t e = tid + p * NT;
                 const float o = X[vec_elems + 256 + e] + total(part_o + e);
-                if (b * C + tok_of(e) < T && col0 + col_of(e) < vdim) *to[p] = ok ? o : __uint_as_float(0x7fffffffu);
+                if (b * C + tok_of(e) < T && col0 + col_of(e) < vdim) *to[p] = o;
                 to[p] += chunk_rs;
             }
             turn_stage(b);
         }
-        if (!ok && lane == 0) count_timeout();
+        __syncthreads();
+        if (failed) {
+            if (tid == 0) count_timeout();
+            for (uint32_t e = tid; e < T * kWalkCols; e += NT)
+                if (col0 + e % kWalkCols < vdim) dst[(size_t)(e / kWalkCols) * dst_rs + (size_t)h * vdim + col0 + e % kWalkCols] = __uint_as_float(0x7fffffffu);
+        }
         return;
     }
     // accumulator r of tile i of slice s: column g + 8 (r / 2), row 8 i + 2 t + r % 2 of the slice
@@ -1635,7 +1648,7 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
             for (int i = 0; i < 3; i++)
                 *reinterpret_cast<uint4*>(parts + (((b & 1) * slices + s * WARPS + warp) * 3 + i) * 128 + lane * 4) = make_uint4(A[s][i][0], A[s][i][1], A[s][i][2], A[s][i][3]);
         }
-        if (!mbar_wait(bars + 8 * cur, parity)) ok = false;
+        if (!mbar_wait(bars + 8 * cur, parity)) failed = 1;
         if (!PLAIN) {
             uint32_t w[SL][2][3][2];
             vectors(X, w);
@@ -1686,8 +1699,9 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
             }
         turn_stage(b);
     }
+    __syncthreads();
+    const bool ok = !failed;
     each_state([&](float& x, bool on, size_t at) { if (on) S_g[at] = ok ? x : __uint_as_float(0x7fffffffu); });
-    if (!ok && lane == 0) count_timeout();
 }
 // o / rms(o) * norm_w * sigmoid(gate) (or silu(gate)) * out_scale, one warp per (token, head), in place
 template <typename WT>

@@ -179,6 +179,7 @@ struct ZgGemvRowsPlan { uint32_t grid = 0, P = 1, S = 1, L = 1, NS = 2, teams = 
 ZgGemvRowsPlan zg_qgemv_rows_plan(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t M, uint32_t count);
 bool zg_qgemv_rows_launch(ZgCudaCtx* ctx, uint32_t count, const ZgCudaQWeight* const* w, const float* const* d_in, float* const* d_out, uint32_t M, const uint32_t* in_rs,
                           const uint32_t* out_rs, const ZgGemvWs* ws, cudaStream_t st);
+unsigned int zg_qgemv_rows_timeouts();       // waits that gave up
 void zg_trace_set_gemv_stream(unsigned long long* d_buf);   // count: matvecs sharing the launch
 void zg_qgemv_ws_need(const ZgCudaCtx* ctx, const ZgCudaQWeight* w, uint32_t M, size_t* partial_elems,
                       size_t* counters);
@@ -398,7 +399,7 @@ bool zg_comm_allgather(ZgCudaCtx* ctx, const float* src, float* dst, size_t n_pe
 inline bool zg_is_seq_op(uint32_t tag) { return tag >= ZG_OP_EMBED && tag < ZG_OP_END; }
 bool zg_seq_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* why, size_t why_n);
 uint32_t zg_seq_op_writes(uint32_t tag);
-unsigned int zg_seq_timeouts();       // waits that gave up (DELTA_RULE's walk)
+unsigned int zg_seq_timeouts();       // waits that gave up (LINEAR of few rows, DELTA_RULE's walk)
 // shared activation scratch the op stages through (0: none); least: what that form does not work without
 size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs, bool least = false);
 // const_weights: nothing writes the op's weight (buf 2) while the program runs, so that it may be read before the launch's predecessor has completed
