@@ -812,14 +812,15 @@ static bool cf_alias(const ZgSeqOp& s) {   // the value row is the head of the k
     return s.buf[2] == s.buf[3] && s.off[1] == s.off[2] && s.n[2] == 1 && s.n[3] == 1 && s.n[5] <= s.n[4] && s.n[7] == s.n[8];
 }
 template <int OC>
-static void launch_cached_attention_tiled(const CaArgs& a, uint32_t splits, float* part, cudaStream_t st) {
+static bool launch_cached_attention_tiled(const CaArgs& a, uint32_t splits, float* part, cudaStream_t st) {
     constexpr int DV = 16 * OC;
-    const size_t smem = ((size_t)(a.dk <= (uint32_t)kCtDS ? 1 : 2) * kCtBQ * kCtDS + (size_t)2 * kCtBK * (kCtDS + 4) + (size_t)kCtBQ * (kCtBK + 4) + (size_t)kCtBK * DV) * sizeof(float);
+    auto smem_of = [](size_t slices) { return (slices * kCtBQ * kCtDS + (size_t)2 * kCtBK * (kCtDS + 4) + (size_t)kCtBQ * (kCtBK + 4) + (size_t)kCtBK * DV) * sizeof(float); };
+    const size_t smem = smem_of(a.dk <= (uint32_t)kCtDS ? 1 : 2);
     auto kernel = a.pool ? k_cached_attention_tiled<OC, true> : k_cached_attention_tiled<OC, false>;
-    static size_t most[2] = {0, 0};
-    if (smem > most[a.pool != 0]) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); most[a.pool != 0] = smem; }
+    if (!(a.pool ? zg_smem_limit<k_cached_attention_tiled<OC, true>>(smem_of(2)) : zg_smem_limit<k_cached_attention_tiled<OC, false>>(smem_of(2)))) return false;
     const uint32_t rh = a.H / a.G, n_tiles = (a.T * rh + kCtBQ - 1) / kCtBQ, n_vs = (a.dv + DV - 1) / DV;
     launch_pdl(kernel, dim3(n_tiles, a.G * a.maps * n_vs, splits), dim3(kCtThreads), smem, st, a, rh, n_tiles, splits, part);
+    return true;
 }
 static bool ca_aligned(const ZgSeqOp& s) {
     return s.n[4] % 4 == 0 && s.n[5] % 4 == 0 && s.n[6] % 4 == 0 && s.n[7] % 4 == 0 && s.n[8] % 4 == 0 && s.off[0] % 4 == 0 && s.off[1] % 4 == 0 && s.off[2] % 4 == 0;
@@ -1272,9 +1273,8 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
                 const dim3 grid(a.G * a.maps, S);
 #define ZG_CF(WARPS_, COLS_)                                                                                                               \
     do {                                                                                                                                   \
-        static size_t most[2] = {48 * 1024, 48 * 1024};                                                                                    \
         auto kernel = a.pool ? k_cached_attention_few<WARPS_, COLS_, true> : k_cached_attention_few<WARPS_, COLS_, false>;                 \
-        if (smem > most[a.pool != 0]) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); most[a.pool != 0] = smem; } \
+        if (!(a.pool ? zg_smem_limit<k_cached_attention_few<WARPS_, COLS_, true>>(kCfMost) : zg_smem_limit<k_cached_attention_few<WARPS_, COLS_, false>>(kCfMost))) return false; \
         launch_pdl(kernel, grid, dim3(32 * WARPS_), smem, st, a, a.H / a.G, S, part, alias, bufs);                                         \
     } while (0)
                 if (warps == 4) ZG_CF(4, 1); else if (warps == 8) ZG_CF(8, 1); else if (a.dv <= 512) ZG_CF(16, 1); else ZG_CF(16, 2);
@@ -1296,15 +1296,17 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
                 // number of CTAs: worth it only while they still fill the GPU one and a half times.
                 const int n_sm = sm_count();
                 const uint32_t row_ctas = ((a.T * (a.H / a.G) + kCtBQ - 1) / kCtBQ) * a.G * a.maps * S * ((a.dv + 511) / 512);
-                if (a.dv > 256 && 2 * row_ctas >= 3 * (uint32_t)n_sm) launch_cached_attention_tiled<32>(a, S, part, st);
-                else if (a.dv > 128) launch_cached_attention_tiled<16>(a, S, part, st);
+                bool ok;
+                if (a.dv > 256 && 2 * row_ctas >= 3 * (uint32_t)n_sm) ok = launch_cached_attention_tiled<32>(a, S, part, st);
+                else if (a.dv > 128) ok = launch_cached_attention_tiled<16>(a, S, part, st);
                 else switch ((a.dv + 15) / 16) {
-                    case 1: launch_cached_attention_tiled<1>(a, S, part, st); break;
-                    case 2: launch_cached_attention_tiled<2>(a, S, part, st); break;
-                    case 3: case 4: launch_cached_attention_tiled<4>(a, S, part, st); break;
-                    case 5: case 6: launch_cached_attention_tiled<6>(a, S, part, st); break;
-                    default: launch_cached_attention_tiled<8>(a, S, part, st); break;
+                    case 1: ok = launch_cached_attention_tiled<1>(a, S, part, st); break;
+                    case 2: ok = launch_cached_attention_tiled<2>(a, S, part, st); break;
+                    case 3: case 4: ok = launch_cached_attention_tiled<4>(a, S, part, st); break;
+                    case 5: case 6: ok = launch_cached_attention_tiled<6>(a, S, part, st); break;
+                    default: ok = launch_cached_attention_tiled<8>(a, S, part, st); break;
                 }
+                if (!ok) return false;
                 if (S > 1) {
                     ZG_SEQ_CHECK();
                     launch_pdl(k_cached_attention_merge<4>, dim3(a.T * a.H * a.maps, (a.dv + kMergeCols - 1) / kMergeCols), dim3(kMergeCols * kMergeGroups), 0, st, a, (const float*)part, a.dv, S, a.wkind);

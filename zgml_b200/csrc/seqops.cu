@@ -200,7 +200,7 @@ __device__ __forceinline__ void bulk_load(float* to, const float* from, uint32_t
 // 444 us (activations that do not fit 48 KB: no staging at all) and 102.
 // Activations of all rows lie in shared memory where they fit (kRingX bytes, for one and two rows whatever there is), else a segment of whole pieces of K at a
 // time: then every weight row passes through once per segment, a piece of it each time, and its shares are added up in shared memory.
-constexpr uint32_t kRingSlots = 3, kRingSlot = 32768, kRingPiece = 4096, kRingFlush = 64, kRingX = 65536;
+constexpr uint32_t kRingSlots = 3, kRingSlot = 32768, kRingPiece = 4096, kRingFlush = 64, kRingX = 65536, kRingSmem = 227 * 1024;
 struct RingPlan { uint32_t ctas, lanes, segment, rows, smem; bool split; };      // segment: pieces of K whose activations are there at once; rows: whose shares are there at once
 static RingPlan ring_plan(uint32_t M, uint32_t N, uint32_t K, bool pairs, uint32_t elem, uint32_t sms) {
     RingPlan r;
@@ -211,7 +211,7 @@ static RingPlan ring_plan(uint32_t M, uint32_t N, uint32_t K, bool pairs, uint32
     r.segment = r.split ? std::min(pieces, std::max(1u, kRingX / (M * (kRingPiece / elem) * 4))) : pieces;
     r.rows = r.split ? ((N + r.ctas - 1) / r.ctas * (pairs ? 2 : 1) + 7) / 8 * 8 : 2 * kRingFlush;
     const size_t x = r.split ? (size_t)M * r.segment * (kRingPiece / elem) : (size_t)M * K, smem = kRingSlots * kRingSlot + ((size_t)r.rows * 8 * M + x) * 4 + 16 * kRingSlots + 16;
-    r.smem = smem <= 227 * 1024 ? (uint32_t)smem : 0;                 // 0: it does not fit
+    r.smem = smem <= kRingSmem ? (uint32_t)smem : 0;                 // 0: it does not fit
     return r;
 }
 template <typename WT, int MR, bool PAIRS, bool SPLIT>      // SPLIT: several segments of K
@@ -1501,7 +1501,7 @@ __device__ __forceinline__ void mma_split3(bool first, float (&acc)[3][4], const
 // chunk to chunk.  The products are far too small for tcgen05 (16 x 32 x 128 and 128 x 16 x 16, each waiting for the one before).  Measured at 1024
 // tokens, 16 heads of 128 x 128: 75 us; with the outputs formed by the warps that hold S 84 us, with f32 FMAs 128 us (bound by what shared memory
 // delivers to registers, 128 bytes a clock: 2500 clocks a chunk), four tokens at a time on one solve each 176 us.
-constexpr uint32_t kWalkStages = 3;
+constexpr uint32_t kWalkStages = 3, kWalkAlone = 116 * 1024;      // the latter: bytes of shared memory of a CTA that is to have an SM to itself
 constexpr uint32_t delta_walk_smem(uint32_t dpad, bool plain, uint32_t warps, uint32_t stages) {
     return (stages * (delta_vec_elems(dpad, plain) + 512) + 2 * dpad / 16 * 384 + warps * 512) * 4 + 3 * 256 * 2 + 8 * kWalkStages;
 }
@@ -2220,17 +2220,20 @@ size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs, bool least) {
 // Below that, a warp per output row and no staging is faster (four gated feed-forwards, one row: 256 / 512 27 us against 33, 512 / 1024 35 both ways,
 // 1024 / 2048 68 against 41; two rows: 256 / 512 35 against 39, 256 / 1024 44 against 39).
 static bool linear_ring(uint32_t M, size_t weight_bytes) { return weight_bytes >= (M == 1 ? 3u << 19 : 3u << 18); }
-template <typename WT>
-static void launch_linear_ring(bool pairs, float* dst, const float* src, const WT* W, const WT* bias, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, SeqAct act,
+template <typename WT, bool PAIRS>
+static bool launch_linear_ring(float* dst, const float* src, const WT* W, const WT* bias, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, SeqAct act,
                                const float* ctl, uint32_t slot_stride, bool early, const RingPlan& r, cudaStream_t st) {
-    auto kern = k_linear_rows_ring<WT, 1, false, false>;
-#define ZG_RING(MR_, SPLIT_) kern = pairs ? k_linear_rows_ring<WT, MR_, true, SPLIT_> : k_linear_rows_ring<WT, MR_, false, SPLIT_>
+#define ZG_RING(MR_, SPLIT_)                                                                                                                                  \
+    do {                                                                                                                                                      \
+        if (!zg_smem_limit<k_linear_rows_ring<WT, MR_, PAIRS, SPLIT_>>(kRingSmem)) return false;                                                              \
+        launch_pdl(k_linear_rows_ring<WT, MR_, PAIRS, SPLIT_>, dim3(r.ctas), dim3(288), r.smem, st, dst, src, W, bias, M, N, K, src_rs, dst_rs, act, ctl,     \
+                   slot_stride, r.lanes, r.segment, r.rows, early ? 1u : 0u);                                                                                 \
+    } while (0)
     if (M == 1) ZG_RING(1, false); else if (M == 2) ZG_RING(2, false);
     else if (r.split) { if (M <= 4) ZG_RING(4, true); else ZG_RING(8, true); }
     else if (M <= 4) ZG_RING(4, false); else ZG_RING(8, false);
 #undef ZG_RING
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem);
-    launch_pdl(kern, dim3(r.ctas), dim3(288), r.smem, st, dst, src, W, bias, M, N, K, src_rs, dst_rs, act, ctl, slot_stride, r.lanes, r.segment, r.rows, early ? 1u : 0u);
+    return true;
 }
 bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool const_weights) {
     (void)ctx;
@@ -2273,7 +2276,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                     const dim3 grid((N + 7) / 8);
                     const RingPlan ring = ring_plan(M, N, K, pairs, sizeof(WT), zg_sm_count());
                     if (aligned && ring.smem && linear_ring(M, (size_t)(pairs ? 2 : 1) * N * K * sizeof(WT))) {
-                        launch_linear_ring<WT>(pairs, dst, src, W, b, M, N, K, s.n[3], s.n[4], act, slot_ctl, s.n[7], const_weights, ring, st);
+                        if (!(pairs ? launch_linear_ring<WT, true> : launch_linear_ring<WT, false>)(dst, src, W, b, M, N, K, s.n[3], s.n[4], act, slot_ctl, s.n[7], const_weights, ring, st)) return false;
                         ZG_SEQ_CHECK();
                         return true;
                     }
@@ -2399,9 +2402,8 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                 // memory (two CTAs on one SM share what bounds them while other SMs stand idle).  Two stages and several CTAs per SM where there are more.
                 const bool alone = (vdim + kWalkCols - 1) / kWalkCols * H <= zg_sm_count();
                 const uint32_t stages = dpad == 512 ? 1 : alone ? kWalkStages : 2;
-                const size_t walk_smem = std::max(delta_walk_smem(dpad, plain, warps, stages), alone ? 116u * 1024 : 0u);
-                if (delta_prep_smem(dpad) > 48 * 1024)
-                    ZG_SEQ_WDT(s.n[9], cudaFuncSetAttribute(k_delta_prepare<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)delta_prep_smem(dpad)));
+                const size_t walk_smem = std::max(delta_walk_smem(dpad, plain, warps, stages), alone ? kWalkAlone : 0u);
+                ZG_SEQ_WDT(s.n[9], if (!zg_smem_limit<k_delta_prepare<WT>>(delta_prep_smem(kWalkMaxDim))) return false);
                 for (uint32_t t = 0; t < T; t += pass) {
                     const uint32_t n = std::min(pass, T - t);
                     // One CTA per SM: eight warps each, and the walk may be placed beside them.  More: four warps (1024 CTAs 41 us, with eight 47).
@@ -2410,19 +2412,24 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                                                   betab ? betab + (size_t)t * s.n[6] : nullptr, bufs[s.buf[3]] + s.n[13] + (size_t)t * s.n[7], wptr<WT>(bufs, s.buf[5], 0), n, H, G, dim, vdim, dpad,
                                                   s.off[0], s.off[1], s.off[2], s.off[3], s.off[4], s.off[5], s.n[5], s.n[6], s.n[7], s.f[1], s.f[2], form, inv_tau, s.n[14], few ? 1u : 0u));
                     ZG_SEQ_CHECK();
-#define ZG_WALK(SL_, WARPS_)                                                                                                                                   \
+#define ZG_WALK(SL_, WARPS_, PLAIN_)                                                                                                                           \
     do {                                                                                                                                                      \
-        auto kern = plain ? k_delta_walk<SL_, WARPS_, true> : k_delta_walk<SL_, WARPS_, false>;                                                                  \
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem);                                                              \
-        launch_pdl(kern, dim3((vdim + kWalkCols - 1) / kWalkCols, H), dim3(64 * warps), walk_smem, st, dst + (size_t)t * dst_rs, scratch, bufs[s.buf[6]],      \
-                   bufs[s.buf[7]], n, H, dim, vdim, dst_rs, stages);                                                                                          \
+        constexpr uint32_t rows = 16 * SL_ * WARPS_, most = delta_walk_smem(rows, PLAIN_, WARPS_, rows == 512 ? 1 : kWalkStages);                             \
+        if (!zg_smem_limit<k_delta_walk<SL_, WARPS_, PLAIN_>>(std::max(most, kWalkAlone))) return false;                                                      \
+        launch_pdl(k_delta_walk<SL_, WARPS_, PLAIN_>, dim3((vdim + kWalkCols - 1) / kWalkCols, H), dim3(64 * WARPS_), walk_smem, st, dst + (size_t)t * dst_rs, \
+                   scratch, bufs[s.buf[6]], bufs[s.buf[7]], n, H, dim, vdim, dst_rs, stages);                                                                 \
     } while (0)
-                    if (dpad == 512) ZG_WALK(4, 8); else if (dpad == 256) ZG_WALK(2, 8); else if (dpad == 128) ZG_WALK(1, 8); else ZG_WALK(1, 4);
+#define ZG_WALK_ROWS(PLAIN_)                                                                                                                                   \
+    do {                                                                                                                                                      \
+        if (dpad == 512) ZG_WALK(4, 8, PLAIN_); else if (dpad == 256) ZG_WALK(2, 8, PLAIN_); else if (dpad == 128) ZG_WALK(1, 8, PLAIN_); else ZG_WALK(1, 4, PLAIN_); \
+    } while (0)
+                    if (plain) ZG_WALK_ROWS(true); else ZG_WALK_ROWS(false);
+#undef ZG_WALK_ROWS
 #undef ZG_WALK
                     if (t + n < T) ZG_SEQ_CHECK();
                 }
             } else ZG_SEQ_WDT(s.n[9], {
-                if (smem > 48 * 1024) cudaFuncSetAttribute(k_delta_rule<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (!zg_smem_limit<k_delta_rule<WT>>(((size_t)3 * kDeltaTile * kWalkMaxDim + kDeltaTile) * sizeof(float))) return false;
                 launch_pdl(k_delta_rule<WT>, dim3(grid), dim3(kDeltaThreads), smem, st, dst, bufs[s.buf[1]], betab, bufs[s.buf[3]] + s.n[13], wptr<WT>(bufs, s.buf[5], 0), bufs[s.buf[6]],
                                                                   bufs[s.buf[7]], T, H, G, dim, vdim, RS, s.off[0], s.off[1], s.off[2], s.off[3], s.off[4], s.off[5],
                                                                   s.n[5], s.n[6], s.n[7], s.f[1], s.f[2], form, inv_tau, dst_rs, s.n[14]);
