@@ -1505,11 +1505,57 @@ constexpr uint32_t kWalkStages = 3, kWalkAlone = 116 * 1024;      // the latter:
 constexpr uint32_t delta_walk_smem(uint32_t dpad, bool plain, uint32_t warps, uint32_t stages) {
     return (stages * (delta_vec_elems(dpad, plain) + 512) + 2 * dpad / 16 * 384 + warps * 512) * 4 + 3 * 256 * 2 + 8 * kWalkStages;
 }
+// Columns of a CTA's 16 (`which`) as plain f32 sums, by all of its threads: where the state, a vector or a u rounds to infinity as bfloat16 or is not finite, its parts are no
+// numbers though the sums may be.  Outputs that are finite stay.  sm: dpad + 16 rows of 16; dst, S_g: at the first column.
+template <uint32_t dpad, bool PLAIN>
+__device__ __forceinline__ void delta_walk_plain(float* sm, const float* P, size_t stride, float* dst, uint32_t dst_rs, float* S_g, uint32_t T, uint32_t dim, uint32_t vdim, uint32_t cols,
+                                              uint32_t which) {
+    constexpr uint32_t C = kWalkChunk, QR = PLAIN ? 0 : C, xs = dpad + 8, vec_elems = delta_vec_elems(dpad, PLAIN);
+    float* S = sm;                                                    // [row][16]
+    float* u = sm + dpad * kWalkCols;                                 // [token][16]
+    const uint32_t col = threadIdx.x % kWalkCols, first = threadIdx.x / kWalkCols, step = blockDim.x / kWalkCols;
+    const bool on = col < cols && (which >> col & 1);
+    for (uint32_t row = first; row < dim; row += step) S[row * kWalkCols + col] = on ? S_g[(size_t)row * vdim + col] : 0.0f;
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t t = 0; t < T; t += C, P += stride) {
+        const float* B = P + (QR + C) * xs;
+        const uint32_t n = min(C, T - t);
+        for (uint32_t j = first; j < n; j += step) {
+            const float* V = P + vec_elems + blockIdx.x * 512 + delta_square(j, col);
+            float ws = 0.0f, qs = 0.0f;
+            for (uint32_t row = 0; row < dim; row++) {
+                const float x = S[row * kWalkCols + col];
+                if (!PLAIN) ws = fmaf(P[j * xs + row], x, ws);
+                qs = fmaf(P[(QR + j) * xs + row], x, qs);
+            }
+            u[j * kWalkCols + col] = V[0] - ws;
+            float* o = dst + (size_t)(t + j) * dst_rs + col;
+            if (on && !(fabsf(*o) <= 3.4028234e38f)) *o = V[256] + qs;
+        }
+        __syncthreads();
+        for (uint32_t row = first; row < dim; row += step) {
+            const uint32_t turn = ((row >> 1) & 1) << 3;
+            float x = S[row * kWalkCols + col] * B[C * dpad + row];
+            for (uint32_t j = 0; j < n; j++) x = fmaf(B[row * C + (j ^ turn)], u[j * kWalkCols + col], x);
+            S[row * kWalkCols + col] = x;
+        }
+        __syncthreads();
+    }
+    if (on) for (uint32_t row = first; row < dim; row += step) S_g[(size_t)row * vdim + col] = S[row * kWalkCols + col];
+}
+// as a call: inlined into the kernels of 256 and 512 rows, it costs them registers (512 rows, 1024 tokens: 304 us, inlined 320)
+template <uint32_t dpad, bool PLAIN>
+__device__ __noinline__ void delta_walk_plain_call(float* sm, const float* P, size_t stride, float* dst, uint32_t dst_rs, float* S_g, uint32_t T, uint32_t dim, uint32_t vdim, uint32_t cols,
+                                                   uint32_t which) {
+    delta_walk_plain<dpad, PLAIN>(sm, P, stride, dst, dst_rs, S_g, T, dim, vdim, cols, which);
+}
+// (the second bound: 256 rows, 8 heads, 1024 tokens 151 us with it and 157 without; the others are left to the compiler)
 template <int SL, int WARPS, bool PLAIN>
-__global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ dst, const float* __restrict__ prep, float* __restrict__ state, const float* __restrict__ ctl,
+__global__ void __launch_bounds__(64 * WARPS, SL == 2 ? 1 : 0) k_delta_walk(float* __restrict__ dst, const float* __restrict__ prep, float* __restrict__ state, const float* __restrict__ ctl,
                                                            uint32_t T, uint32_t H, uint32_t dim, uint32_t vdim, uint32_t dst_rs, uint32_t stages) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ uint32_t failed;                                       // some thread's wait gave up: the CTA's outputs and its part of the state are not numbers
+    __shared__ uint32_t failed, spoiled;                              // some thread's wait gave up: the CTA's outputs and its part of the state are not numbers; columns that are not finite
     constexpr uint32_t C = kWalkChunk, QR = PLAIN ? 0 : C, dpad = 16 * SL * WARPS, xs = dpad + 8, vec_elems = delta_vec_elems(dpad, PLAIN), NT = 32 * WARPS, PER = 256 / NT;
     constexpr uint32_t stage_elems = vec_elems + 512, slices = SL * WARPS;      // of a stage: the chunk's vectors, [Vt | Vo] of the CTA's columns
     const uint32_t h = blockIdx.y, col0 = blockIdx.x * kWalkCols, chunks = (T + C - 1) / C, tid = threadIdx.x % NT, lane = tid & 31, warp = tid >> 5;
@@ -1522,12 +1568,17 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
     const size_t stride = delta_chunk_elems(dpad, PLAIN, vdim);
     const float* P = prep + (size_t)h * chunks * stride;
     if (threadIdx.x == NT) {
-        failed = 0;
+        failed = spoiled = 0;
         for (uint32_t i = 0; i < stages; i++) mbar_init(bars + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    auto state_of = [&] { return state + (((size_t)(uint32_t)ctl_word(ctl, ZG_CTL_SLOT) * H + h) * dim) * vdim + col0; };
+    auto redo = [&] {                                                 // both roles, at the end: every copy has arrived, and of these columns the state in memory is that before the step
+        auto plain = SL == 1 ? delta_walk_plain<dpad, PLAIN> : delta_walk_plain_call<dpad, PLAIN>;
+        plain(sm, prep + (size_t)h * chunks * stride, stride, dst + (size_t)h * vdim + col0, dst_rs, state_of(), T, dim, vdim, vdim - col0, spoiled);
+    };
     auto stage = [&](uint32_t b, uint32_t i) {                        // one thread; nobody reads stage i any more
         if (b >= chunks) return;
         const float* src = P + (size_t)b * stride;
@@ -1584,6 +1635,7 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
     };
     if (outputs) {
         float* to[PER];
+        float zero[PER] = {};                                         // not zero once an output was not finite
 #pragma unroll
         for (uint32_t p = 0; p < PER; p++) to[p] = dst + (size_t)tok_of(tid + p * NT) * dst_rs + (size_t)h * vdim + col0 + col_of(tid + p * NT);
         const size_t chunk_rs = (size_t)C * dst_rs;
@@ -1607,21 +1659,25 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
             for (uint32_t p = 0; p < PER; p++) {
                 const uint32_t e = tid + p * NT;
                 const float o = X[vec_elems + 256 + e] + total(part_o + e);
+                zero[p] = fmaf(o, 0.0f, zero[p]);
                 if (b * C + tok_of(e) < T && col0 + col_of(e) < vdim) *to[p] = o;
                 to[p] += chunk_rs;
             }
             turn_stage(b);
         }
+#pragma unroll
+        for (uint32_t p = 0; p < PER; p++)
+            if (zero[p] != 0.0f) atomicOr(&spoiled, 1u << col_of(tid + p * NT));
         __syncthreads();
         if (failed) {
             if (tid == 0) count_timeout();
             for (uint32_t e = tid; e < T * kWalkCols; e += NT)
                 if (col0 + e % kWalkCols < vdim) dst[(size_t)(e / kWalkCols) * dst_rs + (size_t)h * vdim + col0 + e % kWalkCols] = __uint_as_float(0x7fffffffu);
-        }
+        } else if (spoiled) redo();
         return;
     }
     // accumulator r of tile i of slice s: column g + 8 (r / 2), row 8 i + 2 t + r % 2 of the slice
-    float* S_g = state + (((size_t)(uint32_t)ctl_word(ctl, ZG_CTL_SLOT) * H + h) * dim) * vdim + col0;
+    float* S_g = state_of();
     float S[SL][2][4];
     auto each_state = [&](auto f) {
 #pragma unroll
@@ -1631,10 +1687,10 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
                     const uint32_t row = (s * WARPS + warp) * 16 + 8 * i + 2 * t + (r & 1), col = g + 8 * (r >> 1);
-                    f(S[s][i][r], row < dim && col0 + col < vdim, (size_t)row * vdim + col);
+                    f(S[s][i][r], row < dim && col0 + col < vdim, (size_t)row * vdim + col, r >> 1);
                 }
     };
-    each_state([&](float& x, bool on, size_t at) { x = on ? S_g[at] : 0.0f; });
+    each_state([&](float& x, bool on, size_t at, int) { x = on ? S_g[at] : 0.0f; });
 #pragma unroll 1
     for (uint32_t b = 0; b < chunks; b++) {
         const float* X = sm + cur * stage_elems;
@@ -1699,9 +1755,18 @@ __global__ void __launch_bounds__(64 * WARPS) k_delta_walk(float* __restrict__ d
             }
         turn_stage(b);
     }
+    // (what is not finite on the way stays so in the state)
+    float zero[2] = {};
+    each_state([&](float& x, bool, size_t, int half) { zero[half] = fmaf(x, 0.0f, zero[half]); });
+    if (zero[0] != 0.0f) atomicOr(&spoiled, 1u << g);
+    if (zero[1] != 0.0f) atomicOr(&spoiled, 1u << (g + 8));
     __syncthreads();
     const bool ok = !failed;
-    each_state([&](float& x, bool on, size_t at) { if (on) S_g[at] = ok ? x : __uint_as_float(0x7fffffffu); });
+    const uint32_t keep = ok ? ~spoiled : ~0u;
+    each_state([&](float& x, bool on, size_t at, int half) {
+        if (on && (keep >> (g + 8 * half) & 1)) S_g[at] = ok ? x : __uint_as_float(0x7fffffffu);
+    });
+    if (ok && spoiled) redo();
 }
 // o / rms(o) * norm_w * sigmoid(gate) (or silu(gate)) * out_scale, one warp per (token, head), in place
 template <typename WT>
