@@ -1,5 +1,5 @@
 """DELTA_RULE in chunks of 16 tokens where the launches differ: steps walked in several passes of prepared vectors, more CTAs than SMs (two stages of
-shared memory instead of three), one stage (512 key rows), chunks that end one token early, on time and one late.
+shared memory instead of three), one stage (512 key rows), chunks that end one token early, on time and one late; and short steps, by blocks of four tokens.
 
 Tolerance: as for the shorter steps, sums of at most 512 f32 terms of a state that the decay keeps at the inputs' size: a few 1e-6 of the output's largest
 value, 2e-5 with room for the normalisation's division by a small root."""
@@ -12,10 +12,14 @@ from test_gpu_recops import ctl_words, run
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("T,H,dim,vdim", [(1320, 8, 512, 16), (47, 80, 64, 40), (48, 75, 128, 32), (49, 3, 256, 20), (63, 1, 512, 7)],
-                         ids=["two passes", "two stages, 64 rows", "two stages, 128 rows", "256 rows", "one stage"])
+@pytest.mark.parametrize("T,H,dim,vdim", [(1320, 8, 512, 16), (47, 80, 64, 40), (65, 80, 64, 40), (48, 75, 128, 32), (49, 3, 256, 20), (63, 1, 512, 7)],
+                         ids=["two passes", "two stages, 47 tokens by blocks", "two stages, 64 rows", "two stages, 128 rows", "256 rows", "one stage"])
 @pytest.mark.parametrize("plain", [False, True], ids=["corrected", "plain"])
 def test_delta_rule_in_chunks(cuda_backend, plain, T, H, dim, vdim):
+    step(cuda_backend, plain, T, H, dim, vdim)
+
+
+def step(cuda_backend, plain, T, H, dim, vdim):
     from zgml_b200 import DeviceBuffer, DeviceOp, ExternBuffer, abi
     r = np.random.default_rng(T)
     eps, unit_eps, q_scale = 1e-5, 1e-6, 0.4
@@ -41,6 +45,14 @@ def test_delta_rule_in_chunks(cuda_backend, plain, T, H, dim, vdim):
     assert np.abs(S_got - S_want).max() < 2e-5 * max(1.0, np.abs(S_want).max())
     w.free()
     state.free()
+
+
+@pytest.mark.parametrize("T,H,dim,vdim", [(16, 1, 5, 3), (31, 3, 64, 17), (32, 3, 64, 17), (39, 2, 32, 9), (40, 2, 32, 9), (52, 16, 33, 64), (53, 16, 33, 64), (41, 150, 20, 24),
+                                          (16, 12, 128, 128), (23, 10, 97, 128), (23, 11, 97, 128), (24, 18, 65, 120), (25, 18, 65, 120), (24, 9, 128, 128), (17, 20, 128, 128)])
+@pytest.mark.parametrize("plain", [False, True], ids=["corrected", "plain"])
+def test_short_steps_on_both_sides_of_the_rule(cuda_backend, plain, T, H, dim, vdim):
+    """Steps of blocks of four tokens, with two and four key rows per lane, and the next ones that go by chunks."""
+    step(cuda_backend, plain, T, H, dim, vdim)
 
 
 @pytest.mark.parametrize("dim,vdim", [(64, 64), (100, 20), (256, 16), (512, 7)])

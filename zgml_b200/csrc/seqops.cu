@@ -1266,7 +1266,7 @@ __global__ void __launch_bounds__(kDeltaThreads) k_delta_rule(
         if (live && row < dim) S_g[(size_t)row * vdim + col] = S[i];
     }
 }
-// Prefill form of DELTA_RULE (kDeltaPrepMinTokens or more tokens): chunks of 16 tokens.  With D_l the decay of token l of a chunk (a diagonal) and S the
+// Prefill form of DELTA_RULE (kDeltaPrepMinTokens or more tokens, but for the short steps of delta_by_blocks): chunks of 16 tokens.  With D_l the decay of token l of a chunk (a diagonal) and S the
 // state before it, every token's two products follow from products with S itself:
 //   S_j^T x = S^T (D_1 .. D_j x) + sum_{i <= j} (x^T D_{i+1} .. D_j k_i) u_i,   u_j = beta_j (v_j - A_j^T S - sum_{i < j} ckk_ij u_i).
 // Both are affine in S, so the triangular solve is done ahead, on the vectors instead of on the state's columns:
@@ -1767,6 +1767,256 @@ __global__ void __launch_bounds__(64 * WARPS, SL == 2 ? 1 : 0) k_delta_walk(floa
         if (on && (keep >> (g + 8 * half) & 1)) S_g[at] = ok ? x : __uint_as_float(0x7fffffffu);
     });
     if (ok && spoiled) redo();
+}
+// Short prefill steps (delta_by_blocks): four tokens at a time, the triangular solve of four scalars per value column in the walk itself.  Preparing is cheap
+// then (a warp per block of four tokens and head leaves [A_1 .. A_4 | Q_1 .. Q_4 | B_1 .. B_4 | Gamma] and the scalars [beta (4) | ckk (4 x 4) | cqk (4 x 4)], zero
+// where i does not precede j, laid out [head][block]), but a block waits for the one before.  k_delta_block_walk streams the vectors into shared memory with cp.async,
+// double buffered; a warp owns two value columns, a lane R key rows of both, and the 16 sums of a block (8 products, 2 columns) are reduced over the lanes by
+// halving what is left each time: they end one per lane (column, k or q, token).
+constexpr int kBlockThreads = 256, kBlockTokens = 4, kBlockScalars = 36, kBlockCols = 2;
+__host__ __device__ constexpr uint32_t delta_block_elems(uint32_t dpad, bool plain) { return ((plain ? 2 : 3) * kBlockTokens + 1) * dpad + kBlockScalars; }
+static uint32_t delta_block_rows(uint32_t dim) { return dim <= 64 ? 2 : 4; }      // key rows per lane
+// Where that is faster than chunks of 16, whose fixed costs are larger.  Up to 64 key rows: below 32 tokens (2 heads of 64 x 64, 16 tokens: 10.1 us against 11.5,
+// 24 tokens 11.7 against 12.4, 32 tokens 12.7 against 12.4), below 40 up to 32 rows (8 heads of 32 x 32: 32 tokens 11.2 against 12.0, 40 tokens equal), and up to 52 where the
+// chunks' three launches have more CTAs than SMs and no longer start side by side (16 heads of 64 x 64, 24 tokens: 11.8 against 14.8, 52 tokens equal; 64 heads, 48 tokens
+// 19.7 against 21.9; up to 40 where walk CTAs share SMs and their launch is early, or are more than two an SM: 40 heads, 48 tokens 19.5 against 17.7; 128 heads, 40 tokens
+// 27.8 against 28.5, 48 tokens 32.4 against 29.6).  Up to 128 key rows only up to 24 tokens
+// and where the chunks' walk has nearly an SM per CTA, so that the blocks' kernels do not start side by side either (16 heads of 128 x 128, 16 tokens: 15.4 against
+// 16.5, 28 tokens equal; 10 heads 17.9 against 13.8; 24 heads 18.7 against 15.1).
+constexpr uint32_t kBlockSideBySide = 100;             // CTAs of both kernels up to which the second is placed beside the first
+static uint32_t delta_block_prep_ctas(uint32_t T, uint32_t H) { return ((T + kBlockTokens - 1) / kBlockTokens * H + 3) / 4; }
+static bool delta_by_blocks(uint32_t T, uint32_t H, uint32_t dim, uint32_t vdim) {
+    const uint32_t sms = zg_sm_count(), walk = (vdim + kWalkCols - 1) / kWalkCols * H;
+    if (T > 52 || dim > 128) return false;
+    if (dim > 64) return T <= 24 && walk <= sms && walk + delta_block_prep_ctas(T, H) > kBlockSideBySide;
+    if (T < (dim <= 32 ? 40u : 32u)) return true;
+    const uint32_t prep = (T + kWalkChunk - 1) / kWalkChunk * H;
+    return prep + walk + (T * H + 3) / 4 > sms && (T <= 40 || walk <= sms || (prep > sms && walk <= 2 * sms));
+}
+template <typename WT, int R>
+__global__ void k_delta_block_prepare(float* __restrict__ prep, const float* __restrict__ qkv, const float* __restrict__ betab, const float* __restrict__ ab,
+                                const WT* __restrict__ wts, uint32_t T, uint32_t H, uint32_t G, uint32_t dim, uint32_t q_off,
+                                uint32_t k_off, uint32_t beta_off, uint32_t A_off, uint32_t dt_off, uint32_t qkv_rs, uint32_t beta_rs, uint32_t a_rs,
+                                float unit_eps, float q_scale, uint32_t form, float inv_tau, uint32_t u_off) {
+    pdl_enter();
+    constexpr int B = kBlockTokens;
+    constexpr uint32_t dpad = 32 * R;
+    const bool plain = form & kDeltaPlain, head_decay = form & kDeltaHeadDecay, bonus = form & kDeltaBonus;
+    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31, blocks = (T + B - 1) / B;
+    if (w >= blocks * H) return;
+    const uint32_t b = w / H, h = w % H, kv = h / (H / G), n = min((uint32_t)B, T - b * B);
+    const float* qr = qkv + (size_t)b * B * qkv_rs + q_off + (size_t)kv * dim;
+    const float* kr = qkv + (size_t)b * B * qkv_rs + k_off + (size_t)kv * dim;
+    const float* ar = ab + (size_t)b * B * a_rs + (head_decay ? (size_t)h : (size_t)h * dim);
+    float k[B][R], q[B][R], D[B][R];                                 // every load in flight at once
+#pragma unroll
+    for (int j = 0; j < B; j++)
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const uint32_t c = lane + 32 * i;
+            const bool on = c < dim && (uint32_t)j < n;              // tokens past the step's end: nothing is written, nothing decays
+            k[j][i] = on ? kr[(size_t)j * qkv_rs + c] : 0.0f;
+            q[j][i] = on ? qr[(size_t)j * qkv_rs + c] : 0.0f;
+            D[j][i] = on ? ar[(size_t)j * a_rs + (head_decay ? 0 : c)] : 0.0f;
+        }
+    float bias[R], own[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const uint32_t c = lane + 32 * i;
+        bias[i] = c < dim ? wld(wts, (size_t)dt_off + (head_decay ? (size_t)h : (size_t)h * dim + c)) : 0.0f;
+        own[i] = bonus && c < dim ? wld(wts, (size_t)u_off + (size_t)h * dim + c) : 1.0f;
+    }
+    const float Ah = (form & (kDeltaSigmoidDecay | kDeltaExpDecay)) ? 0.0f : expf(wld(wts, (size_t)A_off + h));
+    const float beta = plain || lane >= n ? 0.0f : betab[((size_t)b * B + lane) * beta_rs + beta_off + h];
+    float scale = (lane & 4) ? 1.0f : q_scale;                       // lane j: of q_j, lane 4 + j: of k_j
+    if (!plain) {
+        float sq[2 * B];
+#pragma unroll
+        for (int j = 0; j < B; j++) {
+            float qq = 0.0f, kk = 0.0f;
+#pragma unroll
+            for (int i = 0; i < R; i++) { qq = fmaf(q[j][i], q[j][i], qq); kk = fmaf(k[j][i], k[j][i], kk); }
+            sq[j] = qq; sq[B + j] = kk;
+        }
+        scale /= sqrtf(reduce_scatter<2 * B>(sq, lane) + unit_eps);
+    }
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+        const float qn = __shfl_sync(0xffffffffu, scale, j), kn = __shfl_sync(0xffffffffu, scale, B + j);
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            k[j][i] *= kn; q[j][i] *= qn;
+            if (i && head_decay) D[j][i] = D[j][0];                  // one decay for all rows (what lies past `dim` is zero, whatever its decay)
+            else D[j][i] = lane + 32 * i < dim && (uint32_t)j < n ? delta_decay(D[j][i] + bias[i], Ah, form, inv_tau) : 1.0f;
+        }
+    }
+    float* P = prep + ((size_t)h * blocks + b) * delta_block_elems(dpad, plain);
+    float* PQ = P + (plain ? 0 : B) * dpad;
+    float* PB = PQ + B * dpad;
+    float c[16] = {};                                                // cqk_ij at j (j + 1) / 2 + i, ckk_ij at 10 + j (j - 1) / 2 + i
+#pragma unroll
+    for (int e = 0; e < R; e++) {
+        const uint32_t at = lane + 32 * e;
+        float g = 1.0f;
+#pragma unroll
+        for (int j = 0; j < B; j++) {
+            const float before = g;
+            g *= D[j][e];
+            if (!plain) P[j * dpad + at] = g * k[j][e];
+            PQ[j * dpad + at] = (bonus ? before : g) * q[j][e];       // the bonus form reads the state before the token decays it
+        }
+        PB[B * dpad + at] = g;
+        float s = 1.0f;
+#pragma unroll
+        for (int j = B - 1; j >= 0; j--) { PB[j * dpad + at] = s * k[j][e]; s *= D[j][e]; }
+#pragma unroll
+        for (int i = 0; i < B; i++) {
+            float& self = c[i * (i + 1) / 2 + i];
+            self = fmaf(q[i][e] * own[e], k[i][e], self);
+            float d = k[i][e];                                       // what token i wrote, as the later tokens find it
+#pragma unroll
+            for (int j = i + 1; j < B; j++) {
+                float& qk = c[j * (j + 1) / 2 + i];
+                if (bonus) qk = fmaf(q[j][e], d, qk);
+                d *= D[j][e];
+                if (!bonus) qk = fmaf(q[j][e], d, qk);
+                if (!plain) { float& kk = c[10 + j * (j - 1) / 2 + i]; kk = fmaf(k[j][e], d, kk); }
+            }
+        }
+    }
+    float* sc = PB + (B + 1) * dpad;
+    if (lane < (uint32_t)B) sc[lane] = plain || lane >= n ? 0.0f : sigmoidf_(beta);
+    const uint32_t cj = (lane >> 2) & 3, ci = lane & 3;               // lane 4 j + i: ckk_ij, lane 16 + 4 j + i: cqk_ij
+    const float total = reduce_scatter<16>(c, lane);
+    const float mine = __shfl_sync(0xffffffffu, total, lane < 16 ? 10 + cj * (cj - 1) / 2 + ci : cj * (cj + 1) / 2 + ci);
+    sc[B + lane] = (lane < 16 ? ci < cj : ci <= cj) ? mine : 0.0f;
+}
+__device__ __forceinline__ void cp_async16(float* smem_dst, const float* gmem_src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gmem_src) : "memory");
+}
+template <int R, bool PLAIN>                       // key rows per lane: 2 or 4
+__global__ void __launch_bounds__(kBlockThreads) k_delta_block_walk(float* __restrict__ dst, const float* __restrict__ qkv, const float* __restrict__ prep,
+                                                               float* __restrict__ state, const float* __restrict__ ctl, uint32_t T, uint32_t H,
+                                                               uint32_t dim, uint32_t vdim, uint32_t v_off, uint32_t qkv_rs, uint32_t dst_rs) {
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    constexpr int B = kBlockTokens, C = kBlockCols, Q = PLAIN ? 0 : B, W = Q + B;      // vectors before Q's and before B's
+    constexpr uint32_t dpad = 32 * R, block_elems = delta_block_elems(dpad, PLAIN), tile_blocks = kDeltaTile / B, tile_elems = tile_blocks * block_elems;
+    const uint32_t h = blockIdx.y, blocks = (T + B - 1) / B, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t col0 = (blockIdx.x * (kBlockThreads / 32) + warp) * C;                     // the warp's first column
+    const uint32_t slot = (uint32_t)ctl_word(ctl, ZG_CTL_SLOT);
+    float* S_g = state + (((size_t)slot * H + h) * dim) * vdim;
+    auto row_of = [&](int i) { return lane * R + (uint32_t)i; };
+    float2 S[C][R / 2];
+#pragma unroll
+    for (int i = 0; i < R; i++)
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const float x = row_of(i) < dim && col0 + c < vdim ? S_g[(size_t)row_of(i) * vdim + col0 + c] : 0.0f;
+            if (i & 1) S[c][i / 2].y = x; else S[c][i / 2].x = x;
+        }
+    const float* P = prep + (size_t)h * blocks * block_elems;
+    auto stage = [&](uint32_t b0, float* buf) {        // blocks [b0, min(b0 + tile, blocks)): one contiguous run
+        const uint32_t n4 = min(tile_blocks, blocks - b0) * block_elems / 4;
+        const float* src = P + (size_t)b0 * block_elems;
+        for (uint32_t i = threadIdx.x; i < n4; i += kBlockThreads) cp_async16(buf + 4 * i, src + 4 * i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    stage(0, sm);
+    // lane (column, k or q, token), twice: its value of a block, its place in the outputs
+    const uint32_t lc = (lane >> 3) & 1, lj = lane & 3;
+    const bool live = col0 + lc < vdim;
+    const float* vbase = qkv + (size_t)lj * qkv_rs + v_off + (size_t)h * vdim + col0 + lc;
+    float vt[tile_blocks], vn[tile_blocks];
+#pragma unroll
+    for (int i = 0; i < (int)tile_blocks; i++) vt[i] = live && i * B + lj < T ? vbase[(size_t)i * B * qkv_rs] : 0.0f;
+    // R / 2 pairs of a prepared vector
+    auto vec = [&](const float* v, float2 (&x)[R / 2]) {
+        if (R == 4) {
+            const float4 y = *reinterpret_cast<const float4*>(v + lane * 4);
+            x[0] = make_float2(y.x, y.y); x[R / 2 - 1] = make_float2(y.z, y.w);
+        } else x[0] = *reinterpret_cast<const float2*>(v + lane * 2);
+    };
+    uint32_t cur = 0;
+    for (uint32_t t0 = 0; t0 < T; t0 += kDeltaTile, cur ^= 1) {
+        const bool more = t0 + kDeltaTile < T;
+        if (more) stage((t0 + kDeltaTile) / B, sm + (cur ^ 1) * tile_elems);   // its last readers passed the barrier that ended the tile before
+#pragma unroll
+        for (int i = 0; i < (int)tile_blocks; i++) vn[i] = live && t0 + kDeltaTile + i * B + lj < T ? vbase[(size_t)(t0 + kDeltaTile + i * B) * qkv_rs] : 0.0f;
+        if (more) asm volatile("cp.async.wait_group 1;" ::: "memory"); else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const float* tile = sm + cur * tile_elems;
+#pragma unroll
+        for (int bi = 0; bi < (int)tile_blocks; bi++) {
+            const uint32_t tb = t0 + bi * B;
+            if (bi && tb >= T) break;
+            const float* row = tile + bi * block_elems;
+            const float* sc = row + (W + B + 1) * dpad;
+            float sums[W * C];                                        // [column][product]
+#pragma unroll
+            for (int d = 0; d < W; d++) {
+                float2 x[R / 2], acc[C];
+                vec(row + d * dpad, x);
+#pragma unroll
+                for (int c = 0; c < C; c++) acc[c] = __fmul2_rn(S[c][0], x[0]);
+#pragma unroll
+                for (int i = 1; i < R / 2; i++)
+#pragma unroll
+                    for (int c = 0; c < C; c++) acc[c] = __ffma2_rn(S[c][i], x[i], acc[c]);
+#pragma unroll
+                for (int c = 0; c < C; c++) sums[c * W + d] = acc[c].x + acc[c].y;
+            }
+            float total = reduce_scatter<W * C>(sums, lane);
+            if (PLAIN) total = __shfl_sync(0xffffffffu, total, lc * B + lj);
+            float u[B], uc[C][B];
+#pragma unroll
+            for (int j = 0; j < B; j++) u[j] = __shfl_sync(0xffffffffu, PLAIN ? vt[bi] : vt[bi] - total, (lane & 8) + j);
+            if (!PLAIN) {
+                const float4 beta = *reinterpret_cast<const float4*>(sc);
+                const float4 c1 = *reinterpret_cast<const float4*>(sc + B + 4), c2 = *reinterpret_cast<const float4*>(sc + B + 8), c3 = *reinterpret_cast<const float4*>(sc + B + 12);
+                u[0] *= beta.x;
+                u[1] = fmaf(-c1.x, u[0], u[1]) * beta.y;
+                u[2] = fmaf(-c2.y, u[1], fmaf(-c2.x, u[0], u[2])) * beta.z;
+                u[3] = fmaf(-c3.z, u[2], fmaf(-c3.y, u[1], fmaf(-c3.x, u[0], u[3]))) * beta.w;
+            }
+#pragma unroll
+            for (int j = 0; j < B; j++) {
+                const float other = __shfl_xor_sync(0xffffffffu, u[j], 8);
+                uc[0][j] = lc ? other : u[j];
+                uc[1][j] = lc ? u[j] : other;
+            }
+            {
+                float2 x[R / 2];
+                vec(row + (W + B) * dpad, x);
+#pragma unroll
+                for (int i = 0; i < R / 2; i++)
+#pragma unroll
+                    for (int c = 0; c < C; c++) S[c][i] = __fmul2_rn(S[c][i], x[i]);
+#pragma unroll
+                for (int j = 0; j < B; j++) {
+                    vec(row + (W + j) * dpad, x);
+#pragma unroll
+                    for (int i = 0; i < R / 2; i++)
+#pragma unroll
+                        for (int c = 0; c < C; c++) S[c][i] = __ffma2_rn(x[i], make_float2(uc[c][j], uc[c][j]), S[c][i]);
+                }
+            }
+            const float4 cq = *reinterpret_cast<const float4*>(sc + B + 16 + 4 * lj);
+            total = fmaf(cq.x, u[0], total);                          // a later token's u is left out, not multiplied by zero: it need not be finite
+            if (lj >= 1) total = fmaf(cq.y, u[1], total);
+            if (lj >= 2) total = fmaf(cq.z, u[2], total);
+            if (lj == 3) total = fmaf(cq.w, u[3], total);
+            if (live && (lane & 20) == 4 && tb + lj < T) dst[(size_t)(tb + lj) * dst_rs + (size_t)h * vdim + col0 + lc] = total;
+        }
+#pragma unroll
+        for (int i = 0; i < (int)tile_blocks; i++) vt[i] = vn[i];
+        __syncthreads();                                   // everyone is done with this buffer: the next iteration refills it
+    }
+#pragma unroll
+    for (int i = 0; i < R; i++)
+#pragma unroll
+        for (int c = 0; c < C; c++)
+            if (row_of(i) < dim && col0 + c < vdim) S_g[(size_t)row_of(i) * vdim + col0 + c] = i & 1 ? S[c][i / 2].y : S[c][i / 2].x;
 }
 // o / rms(o) * norm_w * sigmoid(gate) (or silu(gate)) * out_scale, one warp per (token, head), in place
 template <typename WT>
@@ -2273,6 +2523,7 @@ size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs, bool least) {
         const ZgSeqOp& d = op.u.seq;
         if (d.n[0] < (uint32_t)kDeltaPrepMinTokens || d.n[3] > kWalkMaxDim) return 0;
         const bool plain = d.n[10] & kDeltaPlain;
+        if (delta_by_blocks(d.n[0], d.n[1], d.n[3], d.n[4])) return (size_t)((d.n[0] + kBlockTokens - 1) / kBlockTokens) * d.n[1] * delta_block_elems(32 * delta_block_rows(d.n[3]), plain);
         return delta_chunk_elems(delta_rows(d.n[3]), plain, d.n[4]) * d.n[1] * delta_pass_chunks(d.n[0], d.n[1], d.n[3], d.n[4], plain);
     }
     if (!dense_gemm_enabled() || op.tag != ZG_OP_LINEAR) return 0;
@@ -2460,7 +2711,29 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             const uint32_t RS = zg_delta_row_slices(dim), cols = kDeltaThreads / RS;
             const size_t smem = ((size_t)3 * kDeltaTile * RS * kDeltaRows + kDeltaTile) * sizeof(float);
             const dim3 grid((vdim + cols - 1) / cols, H);
-            if (scratch && T >= (uint32_t)kDeltaPrepMinTokens && dim <= kWalkMaxDim) {
+            if (scratch && T >= (uint32_t)kDeltaPrepMinTokens && delta_by_blocks(T, H, dim, vdim)) {
+                const uint32_t R = delta_block_rows(dim), wcols = kBlockThreads / 32 * kBlockCols, n_prep = delta_block_prep_ctas(T, H);
+                // Many CTAs: a plain launch.  CTAs placed while the predecessor still fills the GPU share SMs two by two.
+                const bool plain = form & kDeltaPlain, early = n_prep + (vdim + wcols - 1) / wcols * H <= kBlockSideBySide;
+#define ZG_BLOCK_FORM(R_, PLAIN_)                                                                                                                             \
+    do {                                                                                                                                                      \
+        constexpr size_t walk_smem = (size_t)2 * (kDeltaTile / kBlockTokens) * delta_block_elems(32 * R_, PLAIN_) * sizeof(float);                            \
+        if (!zg_smem_limit<k_delta_block_walk<R_, PLAIN_>>(walk_smem)) return false;                                                                          \
+        launch_pdl_if(early, k_delta_block_walk<R_, PLAIN_>, dim3((vdim + wcols - 1) / wcols, H), dim3(kBlockThreads), walk_smem, st, dst, bufs[s.buf[1]],    \
+                      scratch, bufs[s.buf[6]], bufs[s.buf[7]], T, H, dim, vdim, s.off[2], s.n[5], dst_rs);                                                    \
+    } while (0)
+#define ZG_BLOCK(R_)                                                                                                                                          \
+    do {                                                                                                                                                      \
+        ZG_SEQ_WDT(s.n[9], launch_pdl(k_delta_block_prepare<WT, R_>, dim3(n_prep), dim3(128), 0, st, scratch, bufs[s.buf[1]], betab, bufs[s.buf[3]] + s.n[13], \
+                                      wptr<WT>(bufs, s.buf[5], 0), T, H, G, dim, s.off[0], s.off[1], s.off[3], s.off[4], s.off[5], s.n[5], s.n[6], s.n[7],    \
+                                      s.f[1], s.f[2], form, inv_tau, s.n[14]));                                                                               \
+        ZG_SEQ_CHECK();                                                                                                                                       \
+        if (plain) ZG_BLOCK_FORM(R_, true); else ZG_BLOCK_FORM(R_, false);                                                                                    \
+    } while (0)
+                if (R == 2) ZG_BLOCK(2); else ZG_BLOCK(4);
+#undef ZG_BLOCK
+#undef ZG_BLOCK_FORM
+            } else if (scratch && T >= (uint32_t)kDeltaPrepMinTokens && dim <= kWalkMaxDim) {
                 const bool plain = form & kDeltaPlain;
                 const uint32_t dpad = delta_rows(dim), warps = dpad == 64 ? 4 : 8, pass = delta_pass_chunks(T, H, dim, vdim, plain) * kWalkChunk;
                 // Where every CTA has an SM to itself: three stages, a chunk's vectors are asked for two chunks ahead, and more than half of the SM's shared
@@ -2471,9 +2744,12 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                 ZG_SEQ_WDT(s.n[9], if (!zg_smem_limit<k_delta_prepare<WT>>(delta_prep_smem(kWalkMaxDim))) return false);
                 for (uint32_t t = 0; t < T; t += pass) {
                     const uint32_t n = std::min(pass, T - t);
-                    // One CTA per SM: eight warps each, and the walk may be placed beside them.  More: four warps (1024 CTAs 41 us, with eight 47).
-                    const bool few = (n + kWalkChunk - 1) / kWalkChunk * H <= zg_sm_count();
-                    ZG_SEQ_WDT(s.n[9], launch_pdl(k_delta_prepare<WT>, dim3(H, (n + kWalkChunk - 1) / kWalkChunk), dim3(few ? kDeltaPrepThreads : kDeltaPrepThreads / 2), delta_prep_smem(dpad), st, scratch, bufs[s.buf[1]] + (size_t)t * s.n[5],
+                    // Up to one CTA per SM: eight warps each, and the walk may be placed beside them; up to two where the walk has an SM per CTA or vectors are long
+                    // (16 heads of 128 x 128, 160 tokens 29 us, with four warps and no early walk 39; 32 heads of 64 x 64, 80 tokens 18.5 and 23.5; but 40 heads, 112
+                    // tokens 28.7 and 25.4).  More: four warps (1024 CTAs 41 us, with eight 47).
+                    const uint32_t n_prep = (n + kWalkChunk - 1) / kWalkChunk * H;
+                    const bool few = n_prep <= (alone || dpad > 64 ? 2 : 1) * zg_sm_count();
+                    ZG_SEQ_WDT(s.n[9], launch_pdl(k_delta_prepare<WT>, dim3(H, n_prep / H), dim3(few ? kDeltaPrepThreads : kDeltaPrepThreads / 2), delta_prep_smem(dpad), st, scratch, bufs[s.buf[1]] + (size_t)t * s.n[5],
                                                   betab ? betab + (size_t)t * s.n[6] : nullptr, bufs[s.buf[3]] + s.n[13] + (size_t)t * s.n[7], wptr<WT>(bufs, s.buf[5], 0), n, H, G, dim, vdim, dpad,
                                                   s.off[0], s.off[1], s.off[2], s.off[3], s.off[4], s.off[5], s.n[5], s.n[6], s.n[7], s.f[1], s.f[2], form, inv_tau, s.n[14], few ? 1u : 0u));
                     ZG_SEQ_CHECK();
