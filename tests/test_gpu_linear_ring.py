@@ -1,5 +1,5 @@
 """LINEAR of up to eight rows over enough weight for the ring of slots: K within one piece of a row, of several and with a short last one, where 32, 64, 128 and
-256 threads share a row, fewer outputs than SMs and counts that do not divide among them, activations that fit shared memory and those that pass through
+256 threads share a row, fewer outputs than SMs and counts that do not divide among them, pairs just below and above what asks for the ring, activations that fit shared memory and those that pass through
 in segments of K, strided and unaligned rows, rows of a state buffer's slot, and a weight that the program itself writes.
 
 Tolerance: a sum is added up in chains of at most 16 elements per 4 KB piece of a row (64 for K = 16384), then over 256 threads in a tree: below 100 roundings
@@ -23,7 +23,7 @@ def _silu(z):
 
 @pytest.mark.parametrize("M,N,K,fmt", [(1, 3100, 256, "bfloat16"), (1, 1600, 520, "bfloat16"), (2, 149, 2056, "float32"), (1, 147, 8200, "bfloat16"), (3, 1033, 1000, "bfloat16"),
                                        (4, 777, 512, "float32"), (5, 301, 4104, "bfloat16"), (8, 297, 6144, "bfloat16"), (8, 150, 3076, "float32"), (2, 64, 16384, "bfloat16"),
-                                       (7, 40, 12296, "bfloat16"), (1, 60000, 32, "bfloat16")])
+                                       (7, 40, 12296, "bfloat16"), (1, 60000, 32, "bfloat16"), (1, 1024, 568, "bfloat16"), (1, 1024, 576, "bfloat16"), (4, 1024, 144, "float32")])
 @pytest.mark.parametrize("pairs", [False, True], ids=["rows", "pairs"])
 def test_linear_rows_through_the_ring(cuda_backend, M, N, K, fmt, pairs):
     from zgml_b200 import DeviceOp, ExternBuffer, abi

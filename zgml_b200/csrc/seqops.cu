@@ -2533,9 +2533,13 @@ size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs, bool least) {
     return zg_dense_gemm_scratch_elems(s.n[0], s.n[2]);
 }
 
-// Below that, a warp per output row and no staging is faster (four gated feed-forwards, one row: 256 / 512 27 us against 33, 512 / 1024 35 both ways,
-// 1024 / 2048 68 against 41; two rows: 256 / 512 35 against 39, 256 / 1024 44 against 39).
-static bool linear_ring(uint32_t M, size_t weight_bytes) { return weight_bytes >= (M == 1 ? 3u << 19 : 3u << 18); }
+// Below that, a warp per output row and no staging is faster (four feed-forwards of 256 / 512, one row 27 us against 33; two rows 35 against 39, of 256 / 1024 44 against
+// 39).  Pairs whose outputs are one wave of such warps need half as much again (gated feed-forwards of 512 / 1024, bfloat16, one row, 2 MB: 8.7 us each against 9.6;
+// 256 / 1024, four rows, 1 MB: 17.2 against 22.0; 384 / 1024, one row 9.2 both ways, four rows, 1.5 MB: 20.0 against 14.9).
+static bool linear_ring(uint32_t M, uint32_t N, bool pairs, size_t weight_bytes) {
+    const size_t least = M == 1 ? 3u << 19 : 3u << 18;
+    return weight_bytes >= (pairs && N <= 8 * zg_sm_count() ? least * 3 / 2 : least);
+}
 template <typename WT, bool PAIRS>
 static bool launch_linear_ring(float* dst, const float* src, const WT* W, const WT* bias, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t dst_rs, SeqAct act,
                                const float* ctl, uint32_t slot_stride, bool early, const RingPlan& r, cudaStream_t st) {
@@ -2591,7 +2595,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                     const bool aligned = K % V == 0 && (reinterpret_cast<size_t>(W) & 15) == 0, vec = aligned && xs_bytes <= 48 * 1024;
                     const dim3 grid((N + 7) / 8);
                     const RingPlan ring = ring_plan(M, N, K, pairs, sizeof(WT), zg_sm_count());
-                    if (aligned && ring.smem && linear_ring(M, (size_t)(pairs ? 2 : 1) * N * K * sizeof(WT))) {
+                    if (aligned && ring.smem && linear_ring(M, N, pairs, (size_t)(pairs ? 2 : 1) * N * K * sizeof(WT))) {
                         if (!(pairs ? launch_linear_ring<WT, true> : launch_linear_ring<WT, false>)(dst, src, W, b, M, N, K, s.n[3], s.n[4], act, slot_ctl, s.n[7], const_weights, ring, st)) return false;
                         ZG_SEQ_CHECK();
                         return true;
