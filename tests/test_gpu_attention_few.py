@@ -29,6 +29,11 @@ pytestmark = pytest.mark.gpu
     (9, 3000, 4, 4, 96, 96, dict(mask="window", size=513, R=530)),
     (3, 200, 4, 2, 128, 128, dict(mask="block", size=64, gain=1e18)),
     (2, 129, 8, 2, 128, 64, dict(gain=1e-18)),
+    (1, 2100, 8, 8, 60, 64, {}),                       # more CTAs than SMs: four and eight warps; few: eight and sixteen
+    (3, 2100, 12, 4, 64, 68, {}),
+    (2, 2100, 6, 6, 36, 256, {}),
+    (2, 70, 16, 2, 36, 256, {}),
+    (5, 40, 6, 2, 68, 100, {}),
 ])
 def test_few_rows(cuda_backend, T, pos, H, G, dk, dv, kw):
     got, want, _, _ = case(cuda_backend, T, pos, H, G, dk, dv, seed=T + pos + dk, **kw)

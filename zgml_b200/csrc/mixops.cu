@@ -561,7 +561,7 @@ __device__ __forceinline__ void cf_mma(float (&big)[4], float (&small)[4], const
     mma_bf16(small, a[1], b[0]);
     mma_bf16(big, a[0], b[0]);
 }
-// WARPS: as many as dv has 32 columns, up to 16; COLS times 32 columns each
+// WARPS: cf_warps; a warp has up to COLS times 32 value columns
 template <int WARPS, int COLS, bool POOL>
 __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_cached_attention_few(CaArgs a, uint32_t rh, uint32_t splits, float* __restrict__ part, uint32_t alias, uint32_t bufs) {
     pdl_enter();
@@ -806,8 +806,10 @@ static size_t cf_smem(uint32_t dk, uint32_t dv, bool alias, uint32_t warps, uint
 constexpr size_t kCfMost = 226 * 1024;
 // Warps of a CTA.  Four where there is little to do per key and CTAs are many: 16 heads of 32 over 8192 positions 37 us, with eight 58, with sixteen 92;
 // 8 heads of 64 31, 41, 60.  Eight above: with four, two of 128 take the softmax's rows in turn (8 heads on one key head 128, 8192 positions: 20.6 us, with four 22.6;
-// 32 heads on 8 of 128 53, 60).  Sixteen where the columns ask for them; at 256 eight and sixteen are alike.
-static uint32_t cf_warps(uint32_t dv) { return dv <= 64 ? 4 : dv <= 256 ? 8 : 16; }
+// 32 heads on 8 of 128 53, 60).  Sixteen where the columns ask for them; at 256 eight and sixteen are alike.  Twice as many where the CTAs have an SM each: what
+// counts there is the latency of one (per op and merge: 16 heads of 32 on one key head, 100 of 2048 positions 8.8 us, with four warps 9.6; 16 heads on 2 of 128, 8100
+// positions 20.8, with eight 25.6; a step of 16 tokens of one head of 64, 500 positions 11.3, with four 13.8).
+static uint32_t cf_warps(uint32_t dv, uint32_t ctas) { return (dv <= 64 ? 4 : dv <= 256 ? 8 : 16) * (dv <= 256 && ctas <= zg_sm_count() ? 2 : 1); }
 static bool cf_alias(const ZgSeqOp& s) {   // the value row is the head of the key row (one key head, one map, same cache and column)
     return s.buf[2] == s.buf[3] && s.off[1] == s.off[2] && s.n[2] == 1 && s.n[3] == 1 && s.n[5] <= s.n[4] && s.n[7] == s.n[8];
 }
@@ -1268,7 +1270,7 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
                 const uint32_t S = scratch ? ca_splits(s) : 1, alias = cf_alias(s) ? 1u : 0u;
                 float* part = S > 1 ? scratch : nullptr;
                 // a second buffer where a share can have more than one buffer's keys
-                const uint32_t warps = cf_warps(a.dv), bufs = ca_reach(s) > S * kCfKeys && cf_smem(a.dk, a.dv, alias != 0, warps, 2) <= kCfMost ? 2 : 1;
+                const uint32_t warps = cf_warps(a.dv, a.G * a.maps * S), bufs = ca_reach(s) > S * kCfKeys && cf_smem(a.dk, a.dv, alias != 0, warps, 2) <= kCfMost ? 2 : 1;
                 const size_t smem = cf_smem(a.dk, a.dv, alias != 0, warps, bufs);
                 const dim3 grid(a.G * a.maps, S);
 #define ZG_CF(WARPS_, COLS_)                                                                                                               \
