@@ -1,6 +1,6 @@
 """LINEAR of up to eight rows over enough weight for the ring of slots: K within one piece of a row, of several and with a short last one, where 32, 64, 128 and
-256 threads share a row, fewer outputs than SMs and counts that do not divide among them, pairs just below and above what asks for the ring, activations that fit shared memory and those that pass through
-in segments of K, strided and unaligned rows, rows of a state buffer's slot, and a weight that the program itself writes.
+256 threads share a row, fewer outputs than SMs and counts that do not divide among them, pairs just below and above what asks for the ring, activations that fit
+shared memory and those that pass through in segments of K, strided and unaligned rows, rows of a state buffer's slot, and a weight that the program itself writes.
 
 Tolerance: a sum is added up in chains of at most 16 elements per 4 KB piece of a row (64 for K = 16384), then over 256 threads in a tree: below 100 roundings
 of 2^-24 of the sum of magnitudes."""
@@ -79,13 +79,30 @@ def test_rows_of_a_slot(cuda_backend, fmt, extra, M, K):
 
 
 def test_a_weight_that_the_program_writes_is_read_after_it(cuda_backend):
-    from zgml_b200 import DeviceOp, abi
+    """The weight is copied into its place by the op before: the same program, executed with one weight after the other, would answer with the one of the pass before."""
+    from zgml_b200 import DeviceOp, DeviceProgram, ProgramIO, abi
     r = np.random.default_rng(3)
-    N, K = 512, 1024
+    N, K = 2048, 2048
     x = r.standard_normal(K).astype(np.float32)
-    for seed in (1, 2, 3):                                 # the same program would read the weight of the pass before
-        W = np.random.default_rng(seed).standard_normal((N, K)).astype(np.float32)
-        ops = [DeviceOp.slice_assign(2, 3, K, N, 0, 0, 1, K, 0, 1, K, 0), DeviceOp.linear(0, 1, 2, 0, 1, N, K, abi.W_F32)]
-        got = run(cuda_backend, ops, [N, K, N * K, N * K], [(1, x), (3, W)], 0, (N,))
+    ops = [DeviceOp.slice_assign(2, 3, K, N, 0, 0, 1, K, 0, 1, K, 0), DeviceOp.linear(0, 1, 2, 0, 1, N, K, abi.W_F32)]
+    h = cuda_backend.compile_program(DeviceProgram(ops, [N, K, N * K, N * K]))
+    assert cuda_backend.program_stats(h)["early_weight_linears"] == 0
+    for seed in range(6):
+        W, got = np.random.default_rng(seed).standard_normal((N, K)).astype(np.float32), np.zeros(N, np.float32)
+        cuda_backend.execute_program(h, [ProgramIO(1, x), ProgramIO(3, W.ravel())], [ProgramIO(0, got)])
         want, mag = W.astype(np.float64) @ x, np.abs(W).astype(np.float64) @ np.abs(x)
-        assert (np.abs(got - want) <= 100 * 2.0 ** -24 * mag).all()
+        assert (np.abs(got - want) <= 100 * 2.0 ** -24 * mag).all(), seed
+    cuda_backend.free_program(h)
+
+
+def test_which_weights_may_be_read_early(cuda_backend):
+    """Those whose memory no op writes, as the LINEAR's buffer or as another one over it.  (Only the decision is looked at: ops on different buffers have no order of their own.)"""
+    from zgml_b200 import DeviceBuffer, DeviceOp, DeviceProgram, ExternBuffer, abi
+    N, K = 64, 512
+    place = DeviceBuffer(cuda_backend, 4 * N * K)
+    write, read = (DeviceOp.slice_assign(b, 3, K, N, 0, 0, 1, K, 0, 1, K, 0) for b in (2, 4)), DeviceOp.linear(0, 1, 2, 0, 1, N, K, abi.W_F32)
+    for ops, early in (([read], 1), ([next(write), read], 0), ([next(write), read], 0), ([read, read], 2)):
+        h = cuda_backend.compile_program(DeviceProgram(ops, [N, K, N * K, N * K, N * K], [], [], [ExternBuffer(2, place), ExternBuffer(4, place)]))
+        assert cuda_backend.program_stats(h)["early_weight_linears"] == early
+        cuda_backend.free_program(h)
+    place.free()

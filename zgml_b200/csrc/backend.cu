@@ -1183,8 +1183,6 @@ static bool build_decode_plan(ZgCudaProgram* p, std::vector<DecHostLayer>& layer
     return true;
 }
 
-// Dependency levels over ITEMS (level = 1 + max level of every earlier item it conflicts with), then units in (level,
-// program order); any such order is a valid topological order of the program's dependency DAG.
 // Buffers whose memory some op writes, by address: two buffers of a program may lie over the same memory.
 static void find_written(ZgCudaProgram* p) {
     std::vector<std::pair<const float*, const float*>> spans;
@@ -1213,6 +1211,8 @@ static bool const_weights(const ZgCudaProgram* p, const ZgOp& op) {
     return p->ctx->graph_mode && !p->ctx->profiling && b < p->written.size() && !p->written[b];
 }
 
+// Dependency levels over ITEMS (level = 1 + max level of every earlier item it conflicts with), then units in (level,
+// program order); any such order is a valid topological order of the program's dependency DAG.
 static bool build_schedule(ZgCudaProgram* p) {
     const size_t n = p->ops.size();
     find_written(p);
@@ -2194,6 +2194,7 @@ extern "C" uint64_t zg_cuda_program_stats(const ZgCudaProgram* p, int what) {
         case 5: return zg_dense_gemm_timeouts() + zg_split_gemm_timeouts() + zg_attention_tc_timeouts() + zg_seq_timeouts() + zg_qgemv_rows_timeouts();
         case 6: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && op.u.seq.n[5] == ZG_W_BF16 && zg_seq_op_scratch_elems(op, p->buffers.data())) n++; return n; }
         case 7: return p->ws.gemm_scratch_elems;
+        case 8: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && const_weights(p, op)) n++; return n; }
         case 0: return p->graph_kernels;
         case 1: return p->dec.valid ? p->dec_count : 0;
         case 2: return p->dec.valid ? p->dec.plan.n_layers : 0;
