@@ -542,7 +542,8 @@ __global__ void __launch_bounds__(kMergeCols * kMergeGroups, BLOCKS) k_cached_at
 // Where the value row is the head of the key row itself (a latent that serves as both), it is not loaded twice.
 // Measured, the op with its merge and the append, against f32 FMAs with a column per thread (which read 68 floats of shared memory for every 64 FMAs, in
 // CTAs of 8 or 16 warps without a second buffer): one token, 16 heads, 8192 latents of 576 33 -> 28 us; 8192 positions of 12 heads of 64 80 -> 45, of 16 heads of 32 84 -> 37,
-// of 32 heads on 8 of 128 68 -> 53, of 8 heads on 2 of 256 41 -> 31; 100 positions as before.  Of the 28 us 4 are the launch of the append, 4 to 6 the merge,
+// of 32 heads on 8 of 128 68 -> 53, of 8 heads on 2 of 256 41 -> 31; at 100 of 2048 positions 0.5 to 0.9 us
+// slower where CTAs share SMs (4 heads of 96 9.2 -> 9.9), the cutting of operands where a handful of FMAs did.  Of the 28 us 4 are the launch of the append, 4 to 6 the merge,
 // the rest the chain load - scores - softmax - sums of two rounds.
 constexpr int kCfRows = 16, kCfKeys = 32;
 // How many of a step's shares (as many as the cache's capacity asks for) its keys are dealt to: beyond 64 only where each gets sixteen keys.  What the step

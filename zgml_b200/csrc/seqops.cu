@@ -2634,7 +2634,9 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                 // whose 2048 columns had 256 threads: 88 us, with 512 threads 76, with 1024 of two values 80).
                 else if (s.n[1] <= 1024) ZG_NORM_ANY(4, 256);
                 else if (s.n[1] <= 2048) ZG_NORM_ANY(4, 512);
-                else ZG_NORM_ANY(4, 1024);                          // up to 4096 columns in registers; wider rows are walked from memory
+                // Up to 4096 columns in registers (eight values and 512 threads / four and 1024, per launch in a chain: 2056 columns 3.39 / 2.82 us, 4096 4.03 / 3.07, two sources
+                // of 4096 5.16 / 4.61; four feed-forwards of 2304 / 6912 136 / 121); wider rows are walked from memory.
+                else ZG_NORM_ANY(4, 1024);
 #undef ZG_NORM_ANY
                 ZG_SEQ_CHECK();
                 return true;

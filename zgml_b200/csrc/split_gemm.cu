@@ -15,7 +15,7 @@
 //     the columns of its 32 rows.  Warp 16 issues the MMAs, warp 17 brings the source's parts, which k_split_source has cut once for all tiles of weight rows.
 //   * Per step the MMAs take 1536 clocks, their operand reads, the copies and the stores 2300 clocks of shared-memory bandwidth.  Where the workers cut the source
 //     too, every CTA its 128 rows of it, a step was 555 instructions of each worker warp, 2200 clocks of issue and 5000 in all, with its loads in flight for one step
-//     only: 256 tokens through gate, up and down of 2048 / 4096 took 166 us, now 95 (as the f32 tile 1034).
+//     only: 256 tokens through gate, up and down of 2048 / 4096 took 166 us, now 105 (as the f32 tile 1034).
 //   * One share of K: the tile is finished here (bias, activation) and leaves by whole rows.  Several: partial sums go to scratch and k_split_finish adds them in
 //     order.  A sum that is not finite is evaluated again as a plain f32 sum: what an infinity makes of a sum is the plain kernel's.
 //   * Every wait is bounded and counts itself (with the count after the loops the case above took 178 us); a CTA whose wait ran out treats its sums as

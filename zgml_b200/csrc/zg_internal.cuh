@@ -155,7 +155,7 @@ bool zg_qweight_dequant_to_device(ZgCudaCtx* ctx, const ZgCudaQWeight* w, float*
 ZgCudaQWeight* zg_qweight_from_device_flat(ZgCudaCtx* ctx, const int8_t* d_data, const float* d_scales,
                                            size_t K, size_t N, size_t bs, int fmt_hint);
 // qgemv.cu
-// Work split of one launch (<= 8 activation rows): P column groups per CTA, S k-splits per column group.
+// Work split of one launch of one or two activation rows: P column groups per CTA, S k-splits per column group.
 struct ZgGemvPlan {
     uint32_t grid = 0, threads = 256, P = 1, S = 1, G = 2, NS = 3, lcap = 1, xs_stride = 32, smem_bytes = 0;
 };
