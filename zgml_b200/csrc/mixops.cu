@@ -676,9 +676,14 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_cached_attention_few
         for (uint32_t row = warp; row < total; row += WARPS) {
             const uint32_t p_r = pos0 + row / rh, j = s0 + kk;
             const float m_run = Run[row];
-            float d = 0.0f;
+            float sl[kSlices];                         // added in pairs: no more rounding than the fewer slices of fewer warps have
 #pragma unroll
-            for (int w = 0; w < kSlices; w++) d += Sp[(w * kCfRows + row) * kCfSpPitch + lane];
+            for (int w = 0; w < kSlices; w++) sl[w] = Sp[(w * kCfRows + row) * kCfSpPitch + lane];
+#pragma unroll
+            for (int n = kSlices / 2; n > 0; n /= 2)
+#pragma unroll
+                for (int w = 0; w < n; w++) sl[w] += sl[w + n];
+            float d = sl[0];
             const bool seen = kk < nk && keys.seen(j, p_r, mask_low(p_r, a.kind, a.size), POOL ? pooled_seen(p_r, a.size, a.pool) : 0u);
             if (seen && !(fabsf(d) <= 3.4028234e38f)) {
                 const float* q = Qs + ((row & 8) | cf_swap(row & 7)) * KP;
