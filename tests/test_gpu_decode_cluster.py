@@ -1,0 +1,85 @@
+"""The layers of a small single-token LLaMA on one thread-block cluster (csrc/decode_cluster.cu) against the general schedule of the same program (which the other LLaMA
+tests hold against the oracle): every program buffer, at the edges of what the kernel splits — head widths, query heads per KV head, KV heads that do not divide the CTAs,
+column groups and feed-forward pairs that do not either, positions around a stage of keys and past all of them."""
+import os
+
+import numpy as np
+import pytest
+
+from zgml_b200.host.llama import DeviceLlamaSession, LlamaConfig, synthetic_weights
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def general():
+    from zgml_b200 import CudaBackend
+    old = os.environ.get("ZG_CUDA_DECODE_CLUSTER")
+    os.environ["ZG_CUDA_DECODE_CLUSTER"] = "0"
+    try:
+        return CudaBackend(0)
+    finally:
+        if old is None:
+            os.environ.pop("ZG_CUDA_DECODE_CLUSTER")
+        else:
+            os.environ["ZG_CUDA_DECODE_CLUSTER"] = old
+
+
+#          d_head, heads, kv, ff, max_seq
+SHAPES = [(32, 1, 1, 32, 40),          # one column group, one pair: most CTAs have nothing
+          (32, 3, 3, 96, 200), (32, 16, 16, 544, 330), (64, 4, 1, 256, 1100), (64, 9, 3, 1536, 700), (64, 10, 5, 800, 420), (128, 2, 2, 288, 600), (128, 2, 1, 640, 1100)]
+
+
+@pytest.mark.parametrize("kind", ["q8_0", "q4_0", "i8_f32"])
+@pytest.mark.parametrize("dh,heads,kv,ff,seq", SHAPES)
+def test_every_buffer_as_the_general_schedule_leaves_it(cuda_backend, general, dh, heads, kv, ff, seq, kind):
+    from zgml_b200 import ProgramIO
+    cfg = LlamaConfig(vocab_size=64, d_model=dh * heads, n_layers=3, n_heads=heads, n_kv_heads=kv, d_ff=ff, max_seq_len=seq)
+    w = synthetic_weights(cfg, "q4_0" if kind == "q4_0" else "q8_0", seed=dh + heads + ff, embed_scale=1.0)
+    if kind == "i8_f32":           # scales that half precision does not hold keep their 32 bits
+        for layer in w.layers:
+            for u in layer.values():
+                u.scales[:] *= np.float32(1.0001)
+    dev, ref = DeviceLlamaSession(cuda_backend, cfg, w, 1), DeviceLlamaSession(general, cfg, w, 1)
+    assert cuda_backend.program_stats(dev.handle)["fused_decode_layers"] == 3 and general.program_stats(ref.handle)["fused_decode_layers"] == 0
+    sizes = dev.lp.program.buffer_sizes
+    got, want = ([np.zeros(n, np.float32) for n in sizes] for _ in range(2))
+    dev.outputs = [ProgramIO(i, b) for i, b in enumerate(got)]
+    ref.outputs = [ProgramIO(i, b) for i, b in enumerate(want)]
+    for pos in [0, 1, 2, 15, 16, 31, 32, 33, 63, 64, 127, 128, 129, seq - 1]:
+        if pos >= seq:
+            continue
+        dev.execute_at([(7 * pos + 1) % 64], pos)
+        ref.execute_at([(7 * pos + 1) % 64], pos)
+        for i, (g, v) in enumerate(zip(got, want)):
+            fin = np.isfinite(v)
+            assert np.array_equal(np.isfinite(g), fin), f"buffer {i} at position {pos}"
+            # a product of K terms on a grid of 2^-24 of its largest is off by some 2^-24 sqrt(K) = 1.4e-6 of its own size; seven in a row per layer, three layers, and scores
+            # of up to 10 that a softmax turns into factors: 1e-4, which is what either schedule is held to against the oracle
+            assert np.max(np.abs(g[fin] - v[fin]), initial=0.0) <= 1e-4 * np.max(np.abs(v[fin]), initial=0.0) + 1e-6, f"buffer {i} at position {pos}"
+    dev.close()
+    ref.close()
+
+
+def test_not_finite_input_comes_out_as_the_oracle_has_it(cuda_backend):
+    """Positions whose score is not finite are passed over, with whatever their values hold."""
+    from llama_reference import OracleBackend
+    cfg = LlamaConfig(vocab_size=64, d_model=192, n_layers=2, n_heads=3, n_kv_heads=1, d_ff=256, max_seq_len=64)
+    for bad in (np.nan, np.inf, 3e38, 1e-38):
+        w = synthetic_weights(cfg, "q8_0", seed=3, embed_scale=1.0)
+        w.token_embed[5, 17] = bad
+        dev, ref = DeviceLlamaSession(cuda_backend, cfg, w, 1), DeviceLlamaSession(OracleBackend(), cfg, w, 1)
+        for t in (4, 5, 6):
+            a, b = dev.step(t).copy(), ref.step(t).copy()
+            assert np.array_equal(np.isfinite(a), np.isfinite(b)), (bad, t)
+            fin = np.isfinite(b)
+            assert np.max(np.abs(a[fin] - b[fin]), initial=0.0) <= 1e-4 * np.max(np.abs(b[fin]), initial=0.0)
+        dev.close()
+        ref.close()
+
+
+def test_layers_beyond_its_size_keep_the_general_schedule(cuda_backend):
+    cfg = LlamaConfig(vocab_size=64, d_model=1024, n_layers=1, n_heads=16, n_kv_heads=4, d_ff=2048, max_seq_len=64)      # 9.5 MB of Q8_0
+    dev = DeviceLlamaSession(cuda_backend, cfg, synthetic_weights(cfg, "q8_0", seed=1), 1)
+    assert cuda_backend.program_stats(dev.handle)["fused_decode_layers"] == 0
+    dev.close()

@@ -139,6 +139,7 @@ struct ZgCudaProgram {
     std::vector<ZgAttnBlock> attn_blocks;            // single-token attention blocks fused into one launch each (ops.cu k_attention_layer)
     ZgAttnBlock* d_attn_blocks = nullptr; float* d_attn_blk_part = nullptr; uint32_t* d_attn_blk_cnt = nullptr;
     ZgDecodeHost dec;          // fused decode kernel (decode.cu) when the program's layers match the single-token LLaMA pattern
+    ZgClusterHost cl;          // or the cluster form of it (decode_cluster.cu), for layers of a few MB
     uint32_t dec_first = 0, dec_count = 0;   // the ops it covers
 };
 
@@ -171,6 +172,7 @@ extern "C" ZgCudaCtx* zg_cuda_create(int device_ordinal) {
     if (const char* e = getenv("ZG_CUDA_GEMV_PAIR")) ctx->gemv_pair = (e[0] != '0');   // 0: gate | up as a plain batch, the activation chain as its own launch
     if (const char* e = getenv("ZG_CUDA_ATTN_LAYER")) ctx->attn_layer = (e[0] != '0');   // 0: rope / cache stores / attention as separate launches
     if (const char* e = getenv("ZG_CUDA_DECODE")) ctx->decode_fused = (e[0] != '0');   // 0: never use the fused decode kernel
+    if (const char* e = getenv("ZG_CUDA_DECODE_CLUSTER")) ctx->decode_cluster = (e[0] != '0');
     if (!zg_qgemv_init(ctx) || !zg_qgemm_init(ctx) || !zg_decode_init(ctx)) { cudaStreamDestroy(ctx->stream); delete ctx; return nullptr; }
     int n_branch = 7; // capture streams for independent ops of a program (ZG_CUDA_BRANCH=0: strictly serial graphs)
     if (const char* e = getenv("ZG_CUDA_BRANCH")) n_branch = atoi(e);
@@ -280,6 +282,7 @@ static void free_program(ZgCudaProgram* p) {
     if (p->h_dyn) cudaFreeHost(p->h_dyn);
     zg_gemv_ws_free(&p->ws);
     zg_decode_free(&p->dec);
+    zg_decode_cluster_free(&p->cl);
     for (auto& kv : p->kv_caches) zg_cuda_kvcache_free(p->ctx, kv.second);
     for (auto& d : p->dense) zg_dense_head_free(d.second);
     cudaFree(p->d_kvq_store); cudaFree(p->d_kvq_attn); cudaFree(p->d_kvq_part); cudaFree(p->d_kvq_cnt);
@@ -1183,6 +1186,134 @@ static bool build_decode_plan(ZgCudaProgram* p, std::vector<DecHostLayer>& layer
     return true;
 }
 
+// The cluster form of the fused layers (decode_cluster.cu).  False: not these layers.
+//
+// Up to kZgClusterLayerBytes of weights a layer: its 16 SMs stream about 1 TB/s and a layer takes some 18 us at least, the general schedule (seven launches a layer, all
+// SMs) some 31.  Whole steps, general / cluster: 8 layers of width 128 231 / 190 us, 10 of 384 (F 1024) 325 / 270, 30 of 576 (3.8 MB of Q8_0) 980 / 808, 12 of 768 (6.7 MB)
+// 428 / 415; 8 of 1024 (F 4096): 18 MB of Q8_0 333 / 449, 9.4 MB of Q4_0 333 / 345.
+constexpr size_t kZgClusterLayerBytes = 7u << 20;
+static bool build_cluster_plan(ZgCudaProgram* p, const std::vector<DecHostLayer>& layers) {
+    ZgClusterHost& h = p->cl;
+    zg_decode_cluster_free(&h);
+    if (p->ctx->world != 1) return false;
+    const ZgDecLayer& l0 = layers[0].ly;
+    const uint32_t D = l0.D, F = l0.F, dh = l0.d_head, H = l0.n_heads, G = l0.n_kv;
+    if (!G || H % G) return false;
+    const auto aligned = [](std::initializer_list<const void*> ps) { for (const void* q : ps) if ((size_t)q & 15) return false; return true; };
+    const auto room = [&](const float* q) {      // elements of the program buffer that starts here
+        size_t n = 0;
+        for (size_t b = 0; b < p->buffers.size(); b++) if (p->buffers[b] == q) n = std::max(n, (size_t)p->buffer_elems[b]);
+        return n;
+    };
+    // What the kernel writes, with the role it has in the layer, and what it takes for constant.  Stores of one role come from the same CTA in every layer, those
+    // of the vectors of D from the owner of their column group: only these may share memory.
+    struct Span { const float* a; const float* b; int role, layer; };
+    std::vector<Span> writes, reads;
+    enum { R_SUM0, R_SUM1, R_O, R_DOWN, R_BARE, R_GREP, R_NORM, R_OWNED, R_Q = R_OWNED, R_K, R_V, R_GATE, R_UP, R_SILU, R_HIDDEN, R_CAT, R_HEADS, R_CACHES = R_HEADS + 3 * 64 };
+    for (size_t l = 0; l < layers.size(); l++) {
+        const DecHostLayer& L = layers[l];
+        const ZgDecLayer& y = L.ly;
+        if (y.D != D || y.F != F || y.d_head != dh || y.n_heads != H || y.n_kv != G || y.ar_o || y.ar_down || y.k_cs != dh || y.v_cs != dh) return false;
+        for (int ph = 0; ph < 4; ph++)
+            if (L.ph[ph].fmt != layers[0].ph[0].fmt) return false;
+        if (L.ph[0].mv[0].N != H * dh || L.ph[0].mv[1].N != G * dh || L.ph[0].mv[2].N != G * dh || L.ph[0].K != D || L.ph[1].K != H * dh || L.ph[1].mv[0].N != D ||
+            L.ph[2].mv[0].N != F || L.ph[2].mv[1].N != F || L.ph[3].K != F || L.ph[3].mv[0].N != D) return false;
+        for (uint32_t i = 0; i < H; i++)
+            if (L.heads[i].kv != i / (H / G) || L.heads[i].q_src != i * dh || L.heads[i].buf_off != i * dh) return false;
+        for (uint32_t g = 0; g < G; g++)
+            if (L.kvs[g].k_src != g * dh || L.kvs[g].v_src != g * dh || L.kvs[g].k_base % 4 || L.kvs[g].v_base % 4) return false;
+        if (!aligned({y.gamma1, y.gamma2, y.cs, y.k_cache, y.v_cache, L.ph[0].mv[0].out, L.ph[0].mv[1].out, L.ph[0].mv[2].out, L.ph[1].mv[0].out, L.ph[2].mv[0].out, L.ph[2].mv[1].out,
+                      L.ph[3].mv[0].out, y.x1_sum, y.x2_sum, y.bare1, y.bare2, y.grep1, y.grep2, y.norm1, y.norm2, y.silu, y.hidden})) return false;
+        const auto w = [&](const float* q, size_t n, int role) { if (q) writes.push_back({q, q + n, role, (int)l}); };
+        const auto r = [&](const float* q, size_t n) { if (q) reads.push_back({q, q + n, 0, (int)l}); };
+        w(y.x1_sum, D, R_SUM0); w(y.x2_sum, D, R_SUM1); w(L.ph[1].mv[0].out, D, R_O); w(L.ph[3].mv[0].out, D, R_DOWN);
+        w(y.bare1, D, R_BARE); w(y.grep1, D, R_GREP); w(y.norm1, D, R_NORM);
+        w(y.bare2, D, R_BARE); w(y.grep2, D, R_GREP); w(y.norm2, D, R_NORM);
+        w(L.ph[0].mv[0].out, H * dh, R_Q); w(L.ph[0].mv[1].out, G * dh, R_K); w(L.ph[0].mv[2].out, G * dh, R_V);
+        w(L.ph[2].mv[0].out, F, R_GATE); w(L.ph[2].mv[1].out, F, R_UP); w(y.silu, F, R_SILU); w(y.hidden, F, R_HIDDEN); w(y.attn_buf, H * dh, R_CAT);
+        for (uint32_t i = 0; i < H; i++) { w(L.heads[i].q_rot, dh, R_HEADS + i); w(L.heads[i].attn_out, dh, R_HEADS + 64 + i); }
+        for (uint32_t g = 0; g < G; g++) w(L.kvs[g].k_rot, dh, R_HEADS + 128 + g);
+        w(y.k_cache, room(y.k_cache), R_CACHES + 2 * (int)l); w(y.v_cache, room(y.v_cache), R_CACHES + 2 * (int)l + 1);
+        r(y.gamma1, D); r(y.gamma2, D); r(y.cs, dh); r(y.mask, y.has_mask ? room(y.mask) : 0);
+        if (l == 0) r(y.x1_a, D);
+        for (uint32_t s = 0; s < y.n_steps; s++) {
+            if (!aligned({y.steps[s].sec})) return false;
+            r(y.steps[s].sec, F);
+        }
+    }
+    std::sort(writes.begin(), writes.end(), [](const Span& x, const Span& y) { return x.a != y.a ? x.a < y.a : x.b != y.b ? x.b < y.b : x.layer < y.layer; });
+    const float* reach = nullptr;
+    for (size_t i = 0; i < writes.size(); i++) {
+        if (i && writes[i].a < reach) {      // overlaps the group before it: the very same vector, in a role that may share it
+            const Span &x = writes[i - 1], &y = writes[i];
+            if (x.a != y.a || x.b != y.b) return false;
+            if (x.role != y.role && (x.role >= R_OWNED || y.role >= R_OWNED || x.layer == y.layer)) return false;
+        }
+        reach = std::max(reach, writes[i].b);
+    }
+    for (const Span& x : reads) {
+        const auto at = std::lower_bound(writes.begin(), writes.end(), x.b, [](const Span& y, const float* end) { return y.a < end; });
+        if (at != writes.begin() && (at - 1)->b > x.a) return false;      // spans that overlap are equal: the last one before the end reaches furthest
+    }
+    size_t bytes = 0;
+    const ZgDecPhase* ph0 = layers[0].ph;
+    for (int ph = 0; ph < 4; ph++)
+        for (uint32_t m = 0; m < ph0[ph].n_mv; m++) bytes += (size_t)ph0[ph].mv[m].n_nb * ph0[ph].n_kc * ph0[ph].rec_bytes;
+    if (bytes > kZgClusterLayerBytes) return false;
+
+    ZgClusterPlan& P = h.plan;
+    P.n_layers = (uint32_t)layers.size(); P.D = D; P.Dq = H * dh; P.Dkv = G * dh; P.F = F; P.n_heads = H; P.n_kv = G; P.dh = dh;
+    P.blk_bytes = (uint32_t)((sizeof(ZgClusterLayer) + H * sizeof(ZgClusterHead) + G * sizeof(ZgClusterKv) + 15) & ~(size_t)15);
+    h.fmt = (int)ph0[0].fmt;
+    if (!zg_decode_cluster_layout(P, h.fmt)) return false;
+    std::vector<uint8_t> blocks((size_t)P.n_layers * P.blk_bytes, 0);
+    for (size_t l = 0; l < layers.size(); l++) {
+        const DecHostLayer& L = layers[l];
+        const ZgDecLayer& y = L.ly;
+        ZgClusterLayer c;
+        memset(&c, 0, sizeof(c));
+        const ZgDecMv* mv[7] = {&L.ph[0].mv[0], &L.ph[0].mv[1], &L.ph[0].mv[2], &L.ph[1].mv[0], &L.ph[2].mv[0], &L.ph[2].mv[1], &L.ph[3].mv[0]};
+        for (int k = 0; k < 7; k++) { c.recs[k] = mv[k]->recs; c.smax[k] = mv[k]->smax; c.out[k] = mv[k]->out; }
+        c.gamma[0] = y.gamma1; c.gamma[1] = y.gamma2; c.cs = y.cs; c.mask = y.mask; c.x_in = y.x1_a; c.k_cache = y.k_cache; c.v_cache = y.v_cache; c.attn_buf = y.attn_buf;
+        c.sum[0] = y.x1_sum; c.sum[1] = y.x2_sum; c.bare[0] = y.bare1; c.bare[1] = y.bare2; c.grep[0] = y.grep1; c.grep[1] = y.grep2; c.norm[0] = y.norm1; c.norm[1] = y.norm2;
+        c.silu = y.silu; c.hidden = y.hidden; c.eps[0] = y.eps1; c.eps[1] = y.eps2; c.scale = y.scale;
+        c.has_mask = y.has_mask; c.mask_off = y.mask_off; c.mask_rs = y.mask_rs; c.n_steps = y.n_steps; c.act_silu = y.act_silu;
+        memcpy(c.steps, y.steps, sizeof(c.steps));
+        c.first_ext = -1;
+        for (int s = (int)y.n_steps - 1; s >= 0; s--)
+            if ((y.steps[s].op == ZG_EW_ADD || y.steps[s].op == ZG_EW_MUL) && y.steps[s].sec_kind == 0) c.first_ext = s;
+        uint8_t* b = blocks.data() + l * P.blk_bytes;
+        memcpy(b, &c, sizeof(c));
+        ZgClusterHead* hd = reinterpret_cast<ZgClusterHead*>(b + sizeof(c));
+        for (uint32_t i = 0; i < H; i++) hd[i] = {L.heads[i].q_rot, L.heads[i].attn_out, L.heads[i].dyn, 0};
+        ZgClusterKv* kv = reinterpret_cast<ZgClusterKv*>(hd + H);
+        for (uint32_t g = 0; g < G; g++) kv[g] = {L.kvs[g].k_rot, L.kvs[g].k_base, L.kvs[g].v_base, L.kvs[g].k_dyn, L.kvs[g].v_dyn};
+    }
+    // the scale ceilings as the CTAs take them
+    if (cudaStreamSynchronize(p->ctx->stream) != cudaSuccess) { cudaGetLastError(); return false; }
+    constexpr size_t kPer = kZgClusterCtas * 4 * kZgClusterItems;
+    std::vector<int> weight(kPer);
+    std::vector<uint32_t> group(kPer);
+    zg_decode_cluster_items(P, weight.data(), group.data());
+    std::vector<float> smax(P.n_layers * kPer, 1.0f), one;
+    for (size_t l = 0; l < layers.size(); l++) {
+        const DecHostLayer& L = layers[l];
+        const ZgDecMv* mv[7] = {&L.ph[0].mv[0], &L.ph[0].mv[1], &L.ph[0].mv[2], &L.ph[1].mv[0], &L.ph[2].mv[0], &L.ph[2].mv[1], &L.ph[3].mv[0]};
+        for (int k = 0; k < 7; k++) {
+            one.resize(mv[k]->n_nb);
+            if (cudaMemcpy(one.data(), mv[k]->smax, one.size() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return false; }
+            for (size_t i = 0; i < kPer; i++) if (weight[i] == k) smax[l * kPer + i] = one[group[i]];
+        }
+    }
+    if (cudaMalloc(&h.d_blocks, blocks.size()) != cudaSuccess || cudaMalloc(&h.d_smax, smax.size() * sizeof(float)) != cudaSuccess || cudaMalloc(&h.d_err, sizeof(uint32_t)) != cudaSuccess ||
+        cudaMallocHost(&h.h_err, sizeof(uint32_t)) != cudaSuccess || cudaMemcpy(h.d_blocks, blocks.data(), blocks.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(h.d_smax, smax.data(), smax.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) { cudaGetLastError(); zg_decode_cluster_free(&h); return false; }
+    *h.h_err = 0;
+    P.blocks = (const uint8_t*)h.d_blocks; P.smax = h.d_smax; P.err = h.d_err;
+    h.valid = true;
+    return true;
+}
+
 // Buffers whose memory some op writes, by address: two buffers of a program may lie over the same memory.
 static void find_written(ZgCudaProgram* p) {
     std::vector<std::pair<const float*, const float*>> spans;
@@ -1226,10 +1357,13 @@ static bool build_schedule(ZgCudaProgram* p) {
     std::vector<DecHostLayer> dec_layers;
     size_t dec_end = 0;
     zg_decode_free(&p->dec);
+    zg_decode_cluster_free(&p->cl);
     p->dec_first = 0; p->dec_count = 0;
-    if (p->ctx->decode_fused && !p->kvq && p->ctx->fuse && chain_max && p->uniform_pos && match_decode_layers(p, 0, dec_layers, &dec_end)) {
-        if (!build_decode_plan(p, dec_layers)) return false;
-        p->dec_count = (uint32_t)dec_end;
+    if ((p->ctx->decode_fused || p->ctx->decode_cluster) && !p->kvq && p->ctx->fuse && chain_max && p->uniform_pos && match_decode_layers(p, 0, dec_layers, &dec_end)) {
+        if (p->ctx->decode_fused) {
+            if (!build_decode_plan(p, dec_layers)) return false;
+            p->dec_count = (uint32_t)dec_end;
+        } else if (build_cluster_plan(p, dec_layers)) p->dec_count = (uint32_t)dec_end;
     }
     for (size_t i = 0; i < n;) {
         if (p->dec_count && i == 0) {
@@ -1802,6 +1936,7 @@ static bool launch_one(ZgCudaProgram* p, size_t i, cudaStream_t st) {
 }
 
 static bool launch_unit(ZgCudaProgram* p, const ZgCudaProgram::Unit& u, cudaStream_t st) {
+    if (u.decode && p->cl.valid) { p->cl.plan.dyn = p->d_dyn; return zg_decode_cluster_launch(p->cl, st); }
     if (u.decode) { p->dec.plan.dyn = p->d_dyn; return zg_decode_launch(p->ctx, p->dec, st); }
     if (u.ar_norm) {
         const auto& ar = p->ops[u.ops[0]].u.allreduce;
@@ -2049,10 +2184,12 @@ extern "C" void zg_cuda_execute(ZgCudaCtx* ctx, ZgCudaProgram* p, const ZgIO* in
         cudaMemcpyAsync(io.host_ptr, (uint8_t*)p->buffers[io.buf_idx] + io.offset, io.size, cudaMemcpyDeviceToHost, st);
     }
     if (p->dec.valid) cudaMemcpyAsync(p->dec.h_err, p->dec.d_sync + 64, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    if (p->cl.valid) cudaMemcpyAsync(p->cl.h_err, p->cl.d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
     zg_peer_check_enqueue(ctx, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) zg_set_error("execute: %s", cudaGetErrorString(e));
     zg_peer_check_result(ctx);
+    if (p->cl.valid && *p->cl.h_err) zg_set_error("execute: a wait of the cluster decode kernel gave up; the step's outputs are invalid");
     if (p->dec.valid && *p->dec.h_err) {   // a bounded wait inside the fused decode kernel gave up: results are invalid
         static const char* what[] = {"", "grid barrier", "weight ring (TMA)", "NVLink peer all-reduce: a peer rank never arrived"};
         zg_set_error("execute: fused decode kernel timed out in its %s wait; the step's outputs are invalid", what[*p->dec.h_err & 3]);
@@ -2191,13 +2328,13 @@ extern "C" int zg_cuda_program_promote_dense(ZgCudaCtx* ctx, ZgCudaProgram* p, i
 extern "C" uint64_t zg_cuda_program_stats(const ZgCudaProgram* p, int what) {
     if (!p) return 0;
     switch (what) {
-        case 5: return zg_dense_gemm_timeouts() + zg_split_gemm_timeouts() + zg_attention_tc_timeouts() + zg_seq_timeouts() + zg_qgemv_rows_timeouts();
+        case 5: return zg_dense_gemm_timeouts() + zg_split_gemm_timeouts() + zg_attention_tc_timeouts() + zg_seq_timeouts() + zg_qgemv_rows_timeouts() + zg_decode_cluster_timeouts();
         case 6: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && op.u.seq.n[5] == ZG_W_BF16 && zg_seq_op_scratch_elems(op, p->buffers.data())) n++; return n; }
         case 7: return p->ws.gemm_scratch_elems;
         case 8: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && const_weights(p, op)) n++; return n; }
         case 0: return p->graph_kernels;
-        case 1: return p->dec.valid ? p->dec_count : 0;
-        case 2: return p->dec.valid ? p->dec.plan.n_layers : 0;
+        case 1: return p->dec.valid || p->cl.valid ? p->dec_count : 0;
+        case 2: return p->dec.valid ? p->dec.plan.n_layers : p->cl.valid ? p->cl.plan.n_layers : 0;
         case 3: return p->graph_streamed;
         case 4: { uint64_t b = 0; for (auto& d : p->dense) b += (uint64_t)d.second->N * d.second->K * 2 - (uint64_t)d.second->N * 6; return b; }   // HBM bytes per execution saved by the bf16 operands
         default: return 0;

@@ -31,6 +31,7 @@
 // No spin in this kernel is unbounded: grid barrier, mbarrier and peer waits give up after ~2 s, set the sticky error
 // word (reported by zg_cuda_execute through zg_cuda_last_error) and let the kernel drain.
 #include "zg_internal.cuh"
+#include "decode_act.cuh"
 
 #include <stdlib.h>
 #include <string.h>
@@ -583,33 +584,6 @@ __device__ __forceinline__ void prologue_attn_merge(Ctx& cx, const ZgDecodePlan&
     __syncthreads();   // wsm (the partial-sum buffers) is free again
 }
 
-__device__ __noinline__ float apply_unary(uint32_t op, float v) {
-    switch (op) {
-        case ZG_EW_NEG: return -v;
-        case ZG_EW_ABS: return fabsf(v);
-        case ZG_EW_RELU: return fmaxf(v, 0.0f);
-        case ZG_EW_SQRT: return sqrtf(v);
-        case ZG_EW_RECIP: return 1.0f / v;
-        case ZG_EW_EXP: return expf(v);
-        case ZG_EW_LOG: return logf(v);
-        case ZG_EW_GELU: { const float kk = 0.7978845608f * (v + 0.044715f * v * v * v); return 0.5f * v * (1.0f + tanhf(kk)); }
-        default: return v;
-    }
-}
-// the general activation chain of one element (fused_elementwise steps, src/backend/reference.zig:262-300); out of line
-__device__ __noinline__ float act_chain(const ZgDecLayer* ly, float gt, float up, float sec0, int first_ext, uint32_t k) {
-    float v = gt;
-    for (uint32_t s = 0; s < ly->n_steps; s++) {
-        const ZgDecStep st = ly->steps[s];
-        if (st.op == ZG_EW_ADD || st.op == ZG_EW_MUL) {
-            const float o2 = st.sec_kind == 1 ? gt : (st.sec_kind == 2 ? up : ((int)s == first_ext ? sec0 : __ldg(st.sec + k)));
-            if (st.op == ZG_EW_ADD) v = st.is_swapped ? __fadd_rn(o2, v) : __fadd_rn(v, o2);
-            else v = st.is_swapped ? __fmul_rn(o2, v) : __fmul_rn(v, o2);
-        } else v = apply_unary(st.op, v);
-    }
-    return v;
-}
-
 // ── prologue of phase 5: mid = steps(gate) ; hidden = mid * up for the CTA's k-range.  The SiLU chain of the lowering (neg,
 //    exp, + ones, recip, * gate: src/nn.zig:38-44) is evaluated inline, op by op with the same roundings; any other chain by
 //    the general interpreter. ──
@@ -656,7 +630,7 @@ __device__ __forceinline__ void prologue_act(Ctx& cx, const Desc& d, const Geo& 
                 if (k < F) {
                     float v;
                     if (ly.act_silu) v = __fmul_rn(gt[u], 1.0f / __fadd_rn(expf(-gt[u]), sec0[u]));
-                    else v = act_chain(d.ly, gt[u], up[u], sec0[u], first_ext, k);
+                    else v = act_chain(ly.steps, ly.n_steps, gt[u], up[u], sec0[u], first_ext, k);
                     hv = __fmul_rn(v, up[u]);
                     if (writer) {
                         ly.silu[k] = v; ly.hidden[k] = hv;

@@ -133,6 +133,7 @@ struct ZgCudaCtx {
     bool gemv_cluster = true;    // k-split matvec: S in {2, 4, 8} splits of a column group form one cluster, partial sums meet in DSMEM (ZG_GEMV_CLUSTER=0: global scratch)
     bool gemv_pair = true;       // single-token programs: gate | up matvecs + SiLU * up chain in ONE launch (ZG_CUDA_GEMV_PAIR=0: off)
     bool attn_layer = true;      // single-token programs: rope + KV-cache stores + attention + concat of a layer in ONE launch (ZG_CUDA_ATTN_LAYER=0: off)
+    bool decode_cluster = true;  // single-token LLaMA layers of a few MB run on one cluster (decode_cluster.cu; ZG_CUDA_DECODE_CLUSTER=0: off)
     bool decode_fused = false;   // single-token LLaMA layers run in the persistent fused decode kernel (decode.cu; ZG_CUDA_DECODE=1: on)
     bool fuse = true;            // evaluate the lowering's fixed op patterns (norm+gamma, SiLU*up, attention+store) in one pass
     size_t chain_max = 8200;     // small ops up to this many element visits join single-CTA chains (0 = off, ZG_CUDA_CHAIN)
@@ -351,6 +352,43 @@ struct ZgDecodeHost {       // owned by a compiled program
     uint32_t* h_err = nullptr;   // pinned copy of the error flag, read after every execute
     bool valid = false;
 };
+// ── decode_cluster.cu : the same layers on one cluster, for models whose layers are a few MB (one rank) ──
+constexpr uint32_t kZgClusterCtas = 16;
+constexpr uint32_t kZgClusterSmem = 227 * 1024;
+constexpr uint32_t kZgClusterItems = 64;      // column groups of a CTA in one phase
+struct ZgClusterHead { float* q_rot; float* attn_out; uint32_t dyn, _pad; };
+struct ZgClusterKv { float* k_rot; uint32_t k_off, v_off, k_dyn, v_dyn; };
+struct ZgClusterLayer {     // heads and KV heads follow it in the layer's block
+    const uint8_t* recs[7];         // q, k, v, o, gate, up, down (first: the weight stream reads these alone)
+    const float* smax[7];
+    float* out[7];
+    const float* gamma[2];
+    const float* cs; const float* mask; const float* x_in; float* k_cache; float* v_cache; float* attn_buf;
+    float* sum[2];                  // x as the first norm takes it (layers after the first), x after attention
+    float* bare[2]; float* grep[2]; float* norm[2]; float* silu; float* hidden;
+    float eps[2]; float scale;
+    uint32_t has_mask, mask_off, mask_rs, n_steps, act_silu;
+    int first_ext; uint32_t _pad;   // first step whose second operand is neither gate nor up (-1: none)
+    ZgDecStep steps[kZgDecMaxSteps];
+};
+static_assert(sizeof(ZgClusterLayer) % 8 == 0, "the heads hold pointers");
+struct ZgClusterPlan {      // passed to the kernel by value
+    const uint8_t* blocks; const float* smax; const uint32_t* dyn; uint32_t* err;      // smax: [layer][CTA][phase][kZgClusterItems] scale ceilings
+    uint32_t blk_bytes, n_layers, D, Dq, Dkv, F, n_heads, n_kv, dh, dh_log2, gs, splits;
+    uint32_t ring_slots, kv_stages, seg, own_max, hid_max, const_bytes, slot_bytes, smem_bytes;      // zg_decode_cluster_layout
+    uint32_t o_const, o_a1, o_a2, o_q, o_t, o_r, o_part, o_state, o_sq, o_ao, o_hid, o_planes, o_ptrs, o_table, o_list, list_max, o_bars, o_kv, o_ring;
+};
+struct ZgClusterHost {      // owned by a compiled program
+    ZgClusterPlan plan = {};
+    int fmt = 0;
+    void* d_blocks = nullptr; float* d_smax = nullptr; uint32_t* d_err = nullptr; uint32_t* h_err = nullptr;
+    bool valid = false;
+};
+bool zg_decode_cluster_layout(ZgClusterPlan& P, int fmt);
+void zg_decode_cluster_items(const ZgClusterPlan& P, int* weight, uint32_t* group);
+bool zg_decode_cluster_launch(const ZgClusterHost& h, cudaStream_t st);
+void zg_decode_cluster_free(ZgClusterHost* h);
+unsigned int zg_decode_cluster_timeouts();
 // ── ops.cu k_attention_layer: the whole attention block of one layer of a single-token program in ONE launch ──
 // rope(k) -> K-cache store, V-cache store, rope(q), split-KV attention, merge, copy into the concatenated buffer — 3 * (n_kv +
 // n_heads) DeviceOps (src/device_inference.zig lowering of llama_transformer.zig:192-253).  Every op's buffer is still written.
