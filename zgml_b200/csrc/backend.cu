@@ -1342,6 +1342,28 @@ static bool const_weights(const ZgCudaProgram* p, const ZgOp& op) {
     return p->ctx->graph_mode && !p->ctx->profiling && b < p->written.size() && !p->written[b];
 }
 
+// The same of the rows of earlier positions that a CACHED_ATTENTION reads: all that the program writes into the cache's memory are this step's rows, by CACHE_APPENDs
+// of as many tokens at the positions of the same control words.
+static bool const_keys(ZgCudaProgram* p, const ZgOp& op) {
+    const ZgSeqOp& s = op.u.seq;
+    if (!p->ctx->graph_mode || p->ctx->profiling || p->written.size() != p->buffers.size() || p->written[s.buf[4]]) return false;
+    std::vector<ZgRange> r;
+    for (int c = 2; c <= 3; c++) {
+        const uint32_t cache = s.buf[c], width = s.n[c == 2 ? 7 : 8];
+        const float *lo = p->buffers[cache], *hi = lo + p->buffer_elems[cache];
+        for (const ZgOp& w : p->ops) {
+            op_ranges(p, w, r);
+            for (const ZgRange& x : r) {
+                if (!x.write || x.buf >= p->buffers.size() || p->buffers[x.buf] >= hi || p->buffers[x.buf] + p->buffer_elems[x.buf] <= lo) continue;
+                const ZgSeqOp& a = w.u.seq;
+                if (w.tag != ZG_OP_CACHE_APPEND || x.buf != cache || a.buf[0] != cache || a.buf[2] != s.buf[4] || a.n[0] != s.n[0] || a.n[3] != width || a.n[4] != s.n[9] ||
+                    (size_t)a.off[1] + a.n[1] > width || a.buf[1] == cache || a.buf[5] == cache || a.buf[6] == cache) return false;
+            }
+        }
+    }
+    return true;
+}
+
 // Dependency levels over ITEMS (level = 1 + max level of every earlier item it conflicts with), then units in (level,
 // program order); any such order is a valid topological order of the program's dependency DAG.
 static bool build_schedule(ZgCudaProgram* p) {
@@ -1931,7 +1953,8 @@ static bool launch_one(ZgCudaProgram* p, size_t i, cudaStream_t st) {
         }
     }
     if (zg_op_is_batched(op.tag)) return zg_launch_batch(op, p->d_batch + p->single_entry[i], 1, p->d_dyn, st);
-    if (zg_is_seq_op(op.tag)) return zg_launch_seq_op(ctx, op, p->buffers.data(), p->lean ? nullptr : p->ws.gemm_scratch, p->ws.gemm_scratch_elems, st, const_weights(p, op));
+    if (zg_is_seq_op(op.tag)) return zg_launch_seq_op(ctx, op, p->buffers.data(), p->lean ? nullptr : p->ws.gemm_scratch, p->ws.gemm_scratch_elems, st,
+                                                      op.tag == ZG_OP_CACHED_ATTENTION ? const_keys(p, op) : const_weights(p, op));
     return zg_launch_op(ctx, op, p->buffers.data(), p->d_dyn, (uint32_t)i, p->d_steps + p->step_off[i], st);
 }
 

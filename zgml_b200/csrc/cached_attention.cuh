@@ -26,6 +26,7 @@ struct CaArgs {
     uint32_t dst_rs;       // row stride of dst (its first column is folded into the pointer)
     const float* kp; const float* vp;   // POOL: pooled rows [slots, pool_rows, kw] (laid out like the cache's), their key and value columns
     uint32_t pool, pool_rows;
+    uint32_t early;        // (few rows) the cache's rows of earlier positions may be read before the launch's predecessor has completed
     uint32_t unslotted;    // the caches belong to the step (rows recomputed by the program), not to a state slot
 };
 __device__ __forceinline__ uint32_t ca_slot(const CaArgs& a) { return a.unslotted ? 0u : (uint32_t)ctl_word(a.ctl, ZG_CTL_SLOT); }

@@ -543,8 +543,9 @@ __global__ void __launch_bounds__(kMergeCols * kMergeGroups, BLOCKS) k_cached_at
 // Measured, the op with its merge and the append, against f32 FMAs with a column per thread (which read 68 floats of shared memory for every 64 FMAs, in
 // CTAs of 8 or 16 warps without a second buffer): one token, 16 heads, 8192 latents of 576 33 -> 28 us; 8192 positions of 12 heads of 64 80 -> 45, of 16 heads of 32 84 -> 37,
 // of 32 heads on 8 of 128 68 -> 53, of 8 heads on 2 of 256 41 -> 31; at 100 of 2048 positions 0.5 to 0.9 us
-// slower where CTAs share SMs (4 heads of 96 9.2 -> 9.9), the cutting of operands where a handful of FMAs did.  Of the 28 us 4 are the launch of the append, 4 to 6 the merge,
-// the rest the chain load - scores - softmax - sums of two rounds.
+// slower where CTAs share SMs (4 heads of 96 9.2 -> 9.9), the cutting of operands where a handful of FMAs did.  Of the 28 us 4 were the launch of the append, 4 to 6 the merge,
+// the rest the chain load - scores - softmax - sums of two rounds.  The keys of earlier positions now come while the append runs, where nothing else in the program writes the
+// cache (CaArgs::early), and both buffers are filled at the start: 28.7 -> 26.7 us; 16 heads on 4 of 128, 4000 positions 22.6 -> 20.5; 4 heads, latents of 320, 8192 22.2 -> 20.8.
 constexpr int kCfRows = 16, kCfKeys = 32;
 // How many of a step's shares (as many as the cache's capacity asks for) its keys are dealt to: beyond 64 only where each gets sixteen keys.  What the step
 // reads is its keys, and the merge reads a record per share: with 148 shares whatever the position, a token at position 500 of a cache of 8192 latents
@@ -565,7 +566,8 @@ __device__ __forceinline__ void cf_mma(float (&big)[4], float (&small)[4], const
 // WARPS: cf_warps; a warp has up to COLS times 32 value columns
 template <int WARPS, int COLS, bool POOL>
 __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_cached_attention_few(CaArgs a, uint32_t rh, uint32_t splits, float* __restrict__ part, uint32_t alias, uint32_t bufs) {
-    pdl_enter();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (POOL || !a.early) asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int kSlices = WARPS / 2;                 // of the key dimension
     extern __shared__ __align__(16) float sm[];
     const uint32_t dk16 = (a.dk + 15) / 16 * 16, KP = cf_pitch(dk16), VP = alias ? KP : cf_pitch(a.dv), buf_elems = kCfKeys * (KP + (alias ? 0 : VP));
@@ -592,6 +594,7 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_cached_attention_few
     auto head_of = [&](uint32_t row) { return (g * rh + row % rh) * a.maps + m; };
     auto record = [&](uint32_t row) { return part + (((size_t)(row / rh) * a.H * a.maps + head_of(row)) * splits + blockIdx.y) * (4 + a.dv); };
     if (blockIdx.y >= used) {                                       // no keys: a record that weighs nothing
+        if (!POOL && a.early) asm volatile("griddepcontrol.wait;" ::: "memory");
         if (tid < total) {
             float* mine = record(tid);
             mine[0] = -INFINITY; mine[1] = 0.0f;
@@ -599,26 +602,38 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_cached_attention_few
         return;
     }
     // rows of `cols` floats, as many lanes to a row as it has 16 bytes (a power of two, 32 at most); zeros up to `padded`, and for rows that are not there
-    auto copy_rows = [&](uint32_t rows, uint32_t cols, uint32_t padded, auto to, auto from, uint32_t there) {
+    auto copy_rows = [&](uint32_t first, uint32_t rows, uint32_t cols, uint32_t padded, auto to, auto from, uint32_t there) {
         const uint32_t lg = min(5u, 32u - (uint32_t)__clz(padded / 4 - 1)), n = 32 * WARPS >> lg;
 #pragma unroll 4
-        for (uint32_t r = tid >> lg; r < rows; r += n) {
+        for (uint32_t r = first + (tid >> lg); r < rows; r += n) {
             const bool on = r < there;
             const float* src = on ? from(r) : kbase;
             float* dst = to(r);
             for (uint32_t c = 4 * (tid & ((1u << lg) - 1)); c < padded; c += 4u << lg) copy16(dst + c, on && c < cols ? src + c : kbase, on && c < cols);
         }
     };
-    auto load = [&](uint32_t s0, float* Ks) {          // every load in flight at once: one round trip
+    auto load = [&](uint32_t s0, float* Ks, uint32_t from = 0, uint32_t to = (uint32_t)kCfKeys) {      // every load in flight at once: one round trip
         const uint32_t nk = min((uint32_t)kCfKeys, k_end - s0);
-        copy_rows(kCfKeys, a.dk, dk16, [&](uint32_t r) { return Ks + r * KP; }, [&](uint32_t r) { return keys.row(s0 + r); }, nk);
-        if (!alias) copy_rows(kCfKeys, a.dv, a.dv, [&](uint32_t r) { return Ks + kCfKeys * KP + r * VP; }, [&](uint32_t r) { return vals.row(s0 + r); }, nk);
+        copy_rows(from, to, a.dk, dk16, [&](uint32_t r) { return Ks + r * KP; }, [&](uint32_t r) { return keys.row(s0 + r); }, nk);
+        if (!alias) copy_rows(from, to, a.dv, a.dv, [&](uint32_t r) { return Ks + kCfKeys * KP + r * VP; }, [&](uint32_t r) { return vals.row(s0 + r); }, nk);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // Keys of earlier positions do not depend on the launch before this one (which appends this step's): they are on their way while that runs, the new ones follow.
+    const uint32_t both = bufs == 2 && k_begin + kCfKeys < k_end ? 2u : 1u;        // buffers that are filled before the first is used
+    uint32_t old[2] = {0, 0};
+    if (!POOL && a.early) {
+        for (uint32_t i = 0; i < both; i++) {
+            const uint32_t s0 = k_begin + i * kCfKeys;
+            old[i] = k_begin < k_end && s0 < pos0 && n_keys <= a.R ? min((uint32_t)kCfKeys, min(k_end, pos0) - s0) : 0;      // (in a smaller ring the new rows would lie over visible ones)
+            if (old[i]) load(s0, Bs + i * buf_elems, 0, old[i]);
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
     // (rows past the step's are zero: their scores are never used)
-    copy_rows(kCfRows, a.dk, dk16, [&](uint32_t r) { return Qs + ((r & 8) | cf_swap(r & 7)) * KP; },
+    copy_rows(0, kCfRows, a.dk, dk16, [&](uint32_t r) { return Qs + ((r & 8) | cf_swap(r & 7)) * KP; },
               [&](uint32_t r) { return a.q + (size_t)(r / rh) * a.q_rs + a.q_off + (size_t)head_of(r) * a.dk; }, total);
-    if (k_begin < k_end) load(k_begin, Bs);
+    if (k_begin < k_end) load(k_begin, Bs, old[0]);
+    if (both == 2) load(k_begin + kCfKeys, Bs + buf_elems, old[1]);
     for (uint32_t i = tid; i < 3 * 2 * 32; i += 32 * WARPS) Ps[i] = make_uint4(0, 0, 0, 0);
     if (tid < kCfRows) { Al[tid] = 1.0f; Run[tid] = -INFINITY; Run[kCfRows + tid] = 0.0f; }
     float acc[COLS][4][4];                             // 32 columns as four operands of eight: lane's rows gr and gr + 8, columns 8 t + j and 8 t + 4 + j
@@ -634,9 +649,13 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_cached_attention_few
         const uint32_t nk = min((uint32_t)kCfKeys, k_end - s0);
         const float* Ks = Bs + cur * buf_elems;
         const float* Vs = alias ? Ks : Ks + kCfKeys * KP;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (s0 == k_begin && both == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                               // these keys are there, and the readers of the ones before are done
-        if (bufs == 2 && s0 + kCfKeys < k_end) { cur ^= 1; load(s0 + kCfKeys, Bs + cur * buf_elems); }
+        if (bufs == 2 && s0 + kCfKeys < k_end) {
+            cur ^= 1;
+            if (s0 != k_begin) load(s0 + kCfKeys, Bs + cur * buf_elems);
+        }
         {
             float big[2][4], small[2][4];
 #pragma unroll
@@ -1218,7 +1237,7 @@ size_t zg_mix_op_scratch_elems(const ZgOp& op) {
     return S > 1 ? (size_t)s.n[0] * s.n[1] * s.n[3] * S * (4 + s.n[5]) : 0;
 }
 
-bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st) {
+bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st, bool early_keys) {
     (void)scratch;
     const ZgSeqOp& s = op.u.seq;
     switch (op.tag) {
@@ -1268,6 +1287,7 @@ bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaSt
             a.tab = s.buf[5] != ZG_NO_BUF ? bufs[s.buf[5]] : nullptr; a.tab_rs = s.off[6]; a.wkind = s.off[5];
             a.cap = s.f[1]; a.out_scale = s.n[13] ? s.f[2] : 1.0f; a.dst_rs = s.n[10] ? s.n[10] : a.H * a.maps * a.dv; a.dst += s.n[11];
             a.sink = nullptr; a.sink_bf16 = s.n[12] == ZG_W_BF16; a.unslotted = s.n[14];
+            a.early = early_keys && !a.unslotted && a.kind != 3 ? 1u : 0u;
             a.kp = a.vp = nullptr; a.pool = a.pool_rows = 0;
             if (a.kind == 3) { a.pool = s.n[15]; a.pool_rows = s.off[6]; a.kp = bufs[s.buf[7]] + a.k_off; a.vp = bufs[s.buf[7]] + a.v_off; }
             if (s.buf[6] != ZG_NO_BUF) a.sink = a.sink_bf16 ? (const void*)wptr<bf16>(bufs, s.buf[6], s.off[7]) : (const void*)wptr<float>(bufs, s.buf[6], s.off[7]);

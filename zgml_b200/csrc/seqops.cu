@@ -2555,7 +2555,8 @@ static bool launch_linear_ring(float* dst, const float* src, const WT* W, const 
 #undef ZG_RING
     return true;
 }
-bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool const_weights) {
+bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool ahead) {
+    const bool const_weights = ahead;
     (void)ctx;
     const ZgSeqOp& s = op.u.seq;
     switch (op.tag) {
@@ -2828,6 +2829,6 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
         }
         default:
             if (op.tag >= ZG_OP_STREAM_STEP) return zg_launch_stream_op(op, bufs, st);
-            return op.tag >= ZG_OP_SSM_SCAN ? zg_launch_rec_op(op, bufs, scratch, st) : zg_launch_mix_op(op, bufs, scratch, st);
+            return op.tag >= ZG_OP_SSM_SCAN ? zg_launch_rec_op(op, bufs, scratch, st) : zg_launch_mix_op(op, bufs, scratch, st, ahead);
     }
 }

@@ -440,8 +440,9 @@ uint32_t zg_seq_op_writes(uint32_t tag);
 unsigned int zg_seq_timeouts();       // waits that gave up (LINEAR of few rows, DELTA_RULE's walk)
 // shared activation scratch the op stages through (0: none); least: what that form does not work without
 size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs, bool least = false);
-// const_weights: nothing writes the op's weight (buf 2) while the program runs, so that it may be read before the launch's predecessor has completed
-bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool const_weights);
+// ahead: nothing writes the op's weight (buf 2; CACHED_ATTENTION: the cache's rows of earlier positions) while the program runs, so that it may be read before the
+// launch's predecessor has completed
+bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool ahead);
 // dense_gemm.cu : bf16 x bf16 -> f32 prefill matmul on tcgen05 (TMA-fed, TMEM accumulator)
 bool zg_dense_gemm_usable(const void* w_bf16, uint32_t M, uint32_t N, uint32_t K);
 size_t zg_dense_gemm_scratch_elems(uint32_t M, uint32_t K);
@@ -460,7 +461,7 @@ bool zg_split_gemm_launch(const float* w, const float* bias, const float* src, f
 bool zg_mix_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* why, size_t why_n);
 uint32_t zg_mix_op_writes(uint32_t tag);
 size_t zg_mix_op_scratch_elems(const ZgOp& op);
-bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st);
+bool zg_launch_mix_op(const ZgOp& op, float* const* bufs, float* scratch, cudaStream_t st, bool early_keys);
 // recops.cu : ZG_OP_SSM_SCAN .. ZG_OP_RG_LRU, reached the same way
 bool zg_rec_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* why, size_t why_n);
 uint32_t zg_rec_op_writes(uint32_t tag);
