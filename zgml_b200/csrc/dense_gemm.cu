@@ -16,6 +16,8 @@
 // seqops.cu); float32 sessions' products of many rows are split_gemm.cu's.
 #include "split_tc.cuh"
 
+#include <algorithm>
+
 namespace {
 
 constexpr uint32_t BM = 128, BN = 128, BK = 64;
@@ -249,108 +251,156 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 // once per run, and what is computed for padding is less than 16 rows (whole 128-row tiles of tokens were a third padding at 16 experts of 128 rows each,
 // and read the weights again for it).  DUAL: two weight matrices against the same rows, gate and up, and out = bf16(act(gate) up), so that neither
 // product goes through memory.
-// The stream of weights sets its floor (4.1 of 6.5 TB/s at 1024 tokens: 256 tiles on 148 SMs are two uneven rounds, each tile's ends exposed).  1024 tokens, two of 16 experts, 2048 x 2048, cold: gate, up and activation 68 us (98 as two products and a pass of
-// their own over whole tiles), down 40 us (42); the op 124 us (171), 44 tokens on one of 4 experts of 1696 x 1088 29 us (60).
+// Where there are more tiles than SMs, a CTA per SM walks them: the next tile's operands are on their way while this one's products end, and its products run while this one
+// is written out, where two accumulators have room.  1024 tokens, two of 16 experts, 2048 x 2048: the op 125 us with a CTA per tile, 120 walked, 117 with the down product by
+// 256 rows; two of 8 experts, 1024 x 1024 61.6 -> 53.8; 700 tokens, one of 16, 1600 / 296 43.0 -> 39.8.  What bounds it is what the SMs take in: 403 MB of weights from memory and
+// 240 MB of runs' rows from the L2 (64 tokens, the same weights: 87 us, of which the two products take some 65 at 6.2 TB/s).
 constexpr uint32_t kExpertThreads = 320;          // warp 0: TMA, warp 1: MMA + TMEM, warps 2-9: epilogue
 constexpr uint32_t kExpertRows = 32;              // rows of x per copy
 constexpr uint32_t kExpertRing = 216 * 1024, kExpertSmem = kExpertRing + 1024 + 256, kExpertStages = 8;
 struct ExpertParams {
     void* out; const ZgExpertSegment* segments;
-    uint32_t N, K;
+    uint32_t N, K, runs;                           // runs: room in `segments`; those with rows come first
     float limit, alpha, up_offset;
 };
-template <bool DUAL>
+enum { kExpertDual, kExpertWide, kExpertOne };      // gate and up; 256 and 128 rows of one matrix
+// LOOP: a CTA per SM takes every gridDim.x-th tile of all runs; otherwise a CTA is (tile, run), and done after it
+template <int MODE, bool LOOP>
 __global__ void __launch_bounds__(kExpertThreads, 1)
 k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2, const ExpertParams p) {
+    constexpr bool DUAL = MODE == kExpertDual, PAIR = MODE != kExpertOne;      // PAIR: two 128-row operands
+    constexpr uint32_t ROWS = MODE == kExpertWide ? 2 * BM : BM;               // of the output's columns that a tile covers
     pdl_enter();
-    const ZgExpertSegment seg = p.segments[blockIdx.y];
-    if (seg.rows <= 0) return;                     // uniform over the CTA, before any barrier or TMEM allocation
+    const uint32_t n_k = (p.K + BK - 1) / BK, n_f = (p.N + ROWS - 1) / ROWS;
+    const ZgExpertSegment first = p.segments[LOOP ? min(blockIdx.x / n_f, p.runs - 1) : blockIdx.y];      // of the first tile: on its way with the others
+    if (!LOOP && first.rows <= 0) return;          // uniform over the CTA, before any barrier or TMEM allocation
+    auto run_of = [&](uint32_t t) { return !LOOP || t == blockIdx.x ? first : p.segments[t / n_f]; };
     extern __shared__ uint8_t dsm_raw[];
+    __shared__ uint32_t live, longest;             // runs with rows, rows of the longest
     const uint32_t base = (smem_u32(dsm_raw) + 1023u) & ~1023u, bars = base + kExpertRing;
-    const uint32_t full = bars, empty = bars + 8 * kExpertStages, tmem_full = bars + 16 * kExpertStages, tmem_slot = tmem_full + 8;
+    const uint32_t full = bars, empty = bars + 8 * kExpertStages, tmem_full = bars + 16 * kExpertStages, tmem_empty = tmem_full + 16, tmem_slot = tmem_empty + 16;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t n = (uint32_t)seg.rows, copies = (n + kExpertRows - 1) / kExpertRows, n_k = (p.K + BK - 1) / BK;
-    constexpr uint32_t kWeights = (DUAL ? 2 : 1) * kTileA, kAccCols = 256;
-    const uint32_t stage_bytes = kWeights + copies * (kExpertRows * BK * 2), stages = min(kExpertStages, kExpertRing / stage_bytes);
-
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < stages; s++) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 1); }
-        mbar_init(tmem_full, 1);
+        for (uint32_t s = 0; s < kExpertStages; s++) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 1); }
+        for (uint32_t i = 0; i < 2; i++) { mbar_init(tmem_full + 8 * i, 1); mbar_init(tmem_empty + 8 * i, 8); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "n"(DUAL ? 2 * kAccCols : kAccCols) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tmem_slot) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (LOOP && warp == 2) {
+        uint32_t n = 0, mx = 0;
+        for (uint32_t i = lane; i < p.runs; i += 32) {
+            const uint32_t rows = (uint32_t)max(p.segments[i].rows, 0);
+            n += rows > 0;
+            mx = max(mx, rows);
+        }
+        n = __reduce_add_sync(0xffffffffu, n);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (lane == 0) { live = n; longest = mx; }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
-    const uint32_t f0 = blockIdx.x * BM;
+    constexpr uint32_t kWeights = (PAIR ? 2 : 1) * kTileA;
+    const uint32_t tiles = LOOP ? live * n_f : n_f, most = LOOP ? longest : (uint32_t)first.rows;
+    const uint32_t stage_bytes = kWeights + (most + kExpertRows - 1) / kExpertRows * (kExpertRows * BK * 2), stages = min(kExpertStages, kExpertRing / stage_bytes);
+    // accumulators: two where both fit the 512 columns, so that a tile's products run while the one before is written out
+    const bool two = (PAIR ? 4 : 2) * ((most + 15) / 16 * 16) <= 512;
+    const uint32_t up_at = two && PAIR ? 128 : 256;              // the second matrix's columns; the other accumulator lies 256 columns on
 
     if (warp == 0) {
         if (lane == 0) {
             uint32_t s = 0, ph = 1;
-            for (uint32_t kt = 0; kt < n_k; kt++) {
-                if (!mbar_wait(empty + 8 * s, ph)) break;
-                const uint32_t at = base + s * stage_bytes;
-                mbar_expect_tx(full + 8 * s, stage_bytes);
-                tma_load_3d(at, &tmap_w, kt * BK, f0, (uint32_t)seg.expert, full + 8 * s);
-                if (DUAL) tma_load_3d(at + kTileA, &tmap_w2, kt * BK, f0, (uint32_t)seg.expert, full + 8 * s);
-                for (uint32_t c = 0; c < copies; c++) tma_2d(at + kWeights + c * (kExpertRows * BK * 2), &tmap_x, kt * BK, (uint32_t)seg.start + c * kExpertRows, full + 8 * s);
-                if (++s == stages) { s = 0; ph ^= 1; }
+            bool ok = true;
+            for (uint32_t t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
+                const ZgExpertSegment seg = run_of(t);
+                const uint32_t f0 = t % n_f * ROWS, copies = ((uint32_t)seg.rows + kExpertRows - 1) / kExpertRows;
+                for (uint32_t kt = 0; kt < n_k; kt++) {
+                    ok = mbar_wait(empty + 8 * s, ph);
+                    if (!ok) break;
+                    const uint32_t at = base + s * stage_bytes;
+                    mbar_expect_tx(full + 8 * s, kWeights + copies * (kExpertRows * BK * 2));
+                    tma_load_3d(at, &tmap_w, kt * BK, f0, (uint32_t)seg.expert, full + 8 * s);
+                    if (PAIR) tma_load_3d(at + kTileA, &tmap_w2, kt * BK, DUAL ? f0 : f0 + BM, (uint32_t)seg.expert, full + 8 * s);
+                    for (uint32_t c = 0; c < copies; c++) tma_2d(at + kWeights + c * (kExpertRows * BK * 2), &tmap_x, kt * BK, (uint32_t)seg.start + c * kExpertRows, full + 8 * s);
+                    if (++s == stages) { s = 0; ph ^= 1; }
+                }
             }
         }
     } else if (warp == 1) {
-        // instruction descriptor (kind::f16): D = F32, A = B = BF16, both K-major, N = the run's rows, M = 128
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((n + 15) / 16 * 2) << 17) | ((128u >> 4) << 24);
         const bool leader = elect_one();
-        uint32_t s = 0, ph = 0;
-        for (uint32_t kt = 0; kt < n_k; kt++) {
-            if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, ph))) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t at = base + s * stage_bytes;
+        uint32_t s = 0, ph = 0, i = 0;
+        bool ok = true;
+        for (uint32_t t = blockIdx.x; ok && t < tiles; t += gridDim.x, i++) {
+            // instruction descriptor (kind::f16): D = F32, A = B = BF16, both K-major, N = the run's rows, M = 128
+            const uint32_t n = (uint32_t)run_of(t).rows, idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((n + 15) / 16 * 2) << 17) | ((128u >> 4) << 24);
+            const uint32_t acc = two ? i & 1 : 0, use = two ? i >> 1 : i, d = tmem + acc * 256;
+            if (use) ok = __all_sync(0xffffffffu, mbar_wait(tmem_empty + 8 * acc, (use - 1) & 1));
+            for (uint32_t kt = 0; ok && kt < n_k; kt++) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * s, ph));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t at = base + s * stage_bytes;
 #pragma unroll
-            for (uint32_t k = 0; k < BK / 16; k++)
-                if (leader) {
-                    const uint64_t x = make_desc(at + kWeights + k * 32);
-                    mma_bf16(tmem, make_desc(at + k * 32), x, idesc, (kt | k) ? 1u : 0u);
-                    if (DUAL) mma_bf16(tmem + kAccCols, make_desc(at + kTileA + k * 32), x, idesc, (kt | k) ? 1u : 0u);
-                }
-            if (leader) mma_commit(empty + 8 * s);
-            if (leader && kt + 1 == n_k) mma_commit(tmem_full);
-            if (++s == stages) { s = 0; ph ^= 1; }
+                for (uint32_t k = 0; k < BK / 16; k++)
+                    if (leader) {
+                        const uint64_t x = make_desc(at + kWeights + k * 32);
+                        mma_bf16(d, make_desc(at + k * 32), x, idesc, (kt | k) ? 1u : 0u);
+                        if (PAIR) mma_bf16(d + up_at, make_desc(at + kTileA + k * 32), x, idesc, (kt | k) ? 1u : 0u);
+                    }
+                if (leader) mma_commit(empty + 8 * s);
+                if (leader && kt + 1 == n_k) mma_commit(tmem_full + 8 * acc);
+                if (++s == stages) { s = 0; ph ^= 1; }
+            }
         }
         __syncwarp();
     } else {
-        // TMEM lane = output column of the CTA's 128, TMEM column = row of the run; the two warps of a quarter take 16 rows each in turn
-        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2, f = f0 + quarter * 32 + lane;
-        const bool ok = mbar_wait(tmem_full, 0);       // (what the other roles gave up on does not arrive here either)
-        if (!ok && lane == 0) count_timeout();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (uint32_t c0 = 16 * half; __all_sync(0xffffffffu, ok) && c0 < n; c0 += 32) {
-            uint32_t g[16], u[16];
-            const uint32_t addr = tmem + ((quarter * 32) << 16) + c0;
-            tmem_ld(addr, g);
-            if (DUAL) tmem_ld(addr + kAccCols, u);
-            tmem_wait_ld(g);
-            if (DUAL) tmem_wait_ld(u);
-#pragma unroll
-            for (uint32_t j = 0; j < 16; j++) {
-                if (c0 + j >= n || f >= p.N) continue;
-                const size_t at = ((size_t)seg.start + c0 + j) * p.N + f;
-                if (DUAL) {
-                    const float gv = fminf(__uint_as_float(g[j]), p.limit), uv = fminf(fmaxf(__uint_as_float(u[j]), -p.limit), p.limit);
-                    reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(gv * sigmoidf_(p.alpha * gv) * (uv + p.up_offset));
-                } else reinterpret_cast<float*>(p.out)[at] = __uint_as_float(g[j]);
+        // TMEM lane = output column of the tile's 128, TMEM column = row of the run; the two warps of a quarter take 16 rows each in turn
+        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
+        uint32_t i = 0;
+        for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
+            const ZgExpertSegment seg = run_of(t);
+            const uint32_t n = (uint32_t)seg.rows, f = t % n_f * ROWS + quarter * 32 + lane, acc = two ? i & 1 : 0, use = two ? i >> 1 : i;
+            const bool ok = __all_sync(0xffffffffu, mbar_wait(tmem_full + 8 * acc, use & 1));       // (what the other roles gave up on does not arrive here either)
+            if (!ok) {
+                if (lane == 0) count_timeout();
+                break;
             }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (uint32_t c0 = 16 * half; c0 < n; c0 += 32) {
+                uint32_t g[16], u[16];
+                const uint32_t addr = tmem + acc * 256 + ((quarter * 32) << 16) + c0;
+                tmem_ld(addr, g);
+                if (PAIR) tmem_ld(addr + up_at, u);
+                tmem_wait_ld(g);
+                if (PAIR) tmem_wait_ld(u);
+#pragma unroll
+                for (uint32_t j = 0; j < 16; j++) {
+                    if (c0 + j >= n || f >= p.N) continue;
+                    const size_t at = ((size_t)seg.start + c0 + j) * p.N + f;
+                    if (DUAL) {
+                        const float gv = fminf(__uint_as_float(g[j]), p.limit), uv = fminf(fmaxf(__uint_as_float(u[j]), -p.limit), p.limit);
+                        reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(gv * sigmoidf_(p.alpha * gv) * (uv + p.up_offset));
+                    } else {
+                        reinterpret_cast<float*>(p.out)[at] = __uint_as_float(g[j]);
+                        if (PAIR && f + BM < p.N) reinterpret_cast<float*>(p.out)[at + BM] = __uint_as_float(u[j]);
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            // relaxed: what it orders are the reads of TMEM above (a releasing arrival waits for the outputs' stores)
+            if (lane == 0) asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];" ::"r"(tmem_empty + 8 * acc) : "memory");
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(DUAL ? 2 * kAccCols : kAccCols) : "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
 EncodeTiledFn g_encode = nullptr;
@@ -362,6 +412,9 @@ typedef void (*GemmKernel)(const CUtensorMap, const CUtensorMap, const GemmParam
      dense_gemm_kernel<MODE_, 4, PAIRS_>, dense_gemm_kernel<MODE_, 5, PAIRS_>, dense_gemm_kernel<MODE_, 6, PAIRS_>}
 const GemmKernel g_kernel[2][kActs] = {ZG_ACTS(kPlain, false), ZG_ACTS(kPlain, true)};   // [pairs][activation]
 #undef ZG_ACTS
+typedef void (*ExpertKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const ExpertParams);
+const ExpertKernel g_expert[3][2] = {{k_expert_gemm<kExpertDual, false>, k_expert_gemm<kExpertDual, true>}, {k_expert_gemm<kExpertWide, false>, k_expert_gemm<kExpertWide, true>},
+                                     {k_expert_gemm<kExpertOne, false>, k_expert_gemm<kExpertOne, true>}};      // [mode][loop]
 GemmKernel batched_kernel(uint32_t act) {      // the activations a batched product's last head can have
     return act == 0 ? dense_gemm_kernel<kBatched, 0, false> : act == 5 ? dense_gemm_kernel<kBatched, 5, false> : (GemmKernel)nullptr;
 }
@@ -372,8 +425,8 @@ bool prepare() {
         if (!g_encode) { zg_set_error("cuTensorMapEncodeTiled entry point not available"); return false; }
     }
     if (!g_attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(k_expert_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExpertSmem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_expert_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExpertSmem);
+        cudaError_t e = cudaSuccess;
+        for (int k = 0; k < 6 && e == cudaSuccess; k++) e = cudaFuncSetAttribute(g_expert[k / 2][k % 2], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExpertSmem);
         for (int k = 0; k < 2 * kActs && e == cudaSuccess; k++) e = cudaFuncSetAttribute(g_kernel[k / kActs][k % kActs], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
         for (uint32_t k = 0; k < 6 && e == cudaSuccess; k += 5) e = cudaFuncSetAttribute(batched_kernel(k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
         if (e != cudaSuccess) { zg_set_error("cudaFuncSetAttribute(dense_gemm) failed: %s", cudaGetErrorString(e)); return false; }
@@ -443,8 +496,13 @@ static bool expert_weights_map(CUtensorMap* map, const void* w, uint32_t E, uint
     return r == CUDA_SUCCESS;
 }
 // xb: bf16 rows [rows][K] sorted by expert; w, w2: [E][N][K] bfloat16 (w2 null: out = f32 [rows][N]; otherwise out = bf16 [rows][N] of gate and up).
-// d_segments: `segments` runs of rows on the device (ZgExpertSegment).
-bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void* xb, uint32_t rows, const ZgExpertSegment* d_segments, uint32_t segments, void* out, uint32_t N, uint32_t K,
+// d_segments: `segments` runs of rows on the device (ZgExpertSegment), those with rows first; full_runs: how many will have some at least where every expert has its share, likely_runs: with
+// half a run more per expert.
+// One matrix is taken 256 rows at a time where there are tiles of that size for three sevenths of the SMs: the runs' rows then cross the L2 half as often (1024 tokens, two of 16
+// experts, 2048 / 2048 120.3 -> 117.8 us, of 8 experts, 1024 / 1024 56.2 -> 54.4; but 20 tokens of 4 experts, 32 such tiles, 40.8 -> 43.7, 500 of 8, 800 / 800, 60 of
+// them, 34.8 -> 36.9).  More tiles than SMs are walked by one CTA per SM (k_expert_gemm); where there are fewer, the walk's preparations cost (1000 tokens, one of 8 experts,
+// 400 / 1800, 120 tiles: 47.2 us, walked 48.9).
+bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void* xb, uint32_t rows, const ZgExpertSegment* d_segments, uint32_t segments, uint32_t full_runs, uint32_t likely_runs, void* out, uint32_t N, uint32_t K,
                            float limit, float alpha, float up_offset, cudaStream_t st) {
     if (!prepare()) return false;
     CUtensorMap map_x, map_w, map_w2;
@@ -454,10 +512,11 @@ bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { zg_set_error("cuTensorMapEncodeTiled(expert rows) failed (%d)", (int)r); return false; }
     if (!expert_weights_map(&map_w, w, E, N, K) || !expert_weights_map(&map_w2, w2 ? w2 : w, E, N, K)) return false;
-    const ExpertParams p = {out, d_segments, N, K, limit, alpha, up_offset};
-    const dim3 grid((N + BM - 1) / BM, segments);
-    if (w2) launch_pdl(k_expert_gemm<true>, grid, dim3(kExpertThreads), kExpertSmem, st, map_x, map_w, map_w2, p);
-    else launch_pdl(k_expert_gemm<false>, grid, dim3(kExpertThreads), kExpertSmem, st, map_x, map_w, map_w2, p);
+    const ExpertParams p = {out, d_segments, N, K, segments, limit, alpha, up_offset};
+    const int mode = w2 ? kExpertDual : 7 * ((N + 2 * BM - 1) / (2 * BM)) * full_runs >= 3 * zg_sm_count() ? kExpertWide : kExpertOne;
+    const uint32_t n_f = (N + (mode == kExpertWide ? 2 : 1) * BM - 1) / ((mode == kExpertWide ? 2 : 1) * BM);
+    const bool loop = n_f * likely_runs > zg_sm_count();
+    launch_pdl(g_expert[mode][loop], loop ? dim3(zg_sm_count()) : dim3(n_f, segments), dim3(kExpertThreads), kExpertSmem, st, map_x, map_w, map_w2, p);
     ZG_COUNT_LAUNCH();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { zg_set_error("expert gemm launch failed: %s", cudaGetErrorString(e)); return false; }
