@@ -809,7 +809,7 @@ template <int FMT>
 __global__ void __launch_bounds__(kThreads, 1)
 k_decode_cluster(const __grid_constant__ ZgClusterPlan plan) {
     extern __shared__ __align__(128) uint8_t smem[];
-    // a copy of the plan for the functions that are calls (the workers read it as constants: 752 us a token, from shared memory 817)
+    // a copy of the plan for the functions that are calls (the workers read it as constants: 759 us a token, from shared memory 818)
     static_assert(sizeof(ZgClusterPlan) <= kDead, "the mark lies behind it");
     if (threadIdx.x < sizeof(ZgClusterPlan) / 4) reinterpret_cast<uint32_t*>(smem)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&plan)[threadIdx.x];
     __syncthreads();
