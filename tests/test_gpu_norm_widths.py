@@ -52,3 +52,23 @@ def test_two_sources(cuda_backend, kind, outer, cols):
         got = run(cuda_backend, [op], sizes, io, out, x.shape, [ExternBuffer(2, buf)])
         assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
     buf.free()
+
+
+@pytest.mark.parametrize("cols", [512, 513, 1024, 1025, 2048, 2049, 4096, 4097])
+@pytest.mark.parametrize("more", [0, 1], ids=["one-wave", "past-it"])
+def test_many_rows(cuda_backend, cols, more):
+    """The largest count of rows that is resident at once, and one row more.  The weight comes from a launch of the same program."""
+    import torch
+    from zgml_b200 import DeviceOp, abi
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = sms * (4 if cols <= 1024 else 2 if cols <= 2048 else 1) + more
+    r = np.random.default_rng(cols)
+    x, res = (r.standard_normal((rows, cols)).astype(np.float32) for _ in range(2))
+    w, ones = (1 + 0.3 * r.standard_normal((1, cols))).astype(np.float32), np.ones((2 * cols,), np.float32)
+    ops = [DeviceOp.norm(2, 5, 6, 0, 1, cols, 1e-5, abi.W_F32, kind="rms"), DeviceOp.norm(0, 1, 2, 0, rows, cols, 1e-5, abi.W_F32, kind="none", res=3, then=4, then_w=2, then_w_off=0, then_kind="rms")]
+    sizes, io = [x.size, x.size, cols, x.size, x.size, cols, ones.size], [(1, x), (3, res), (5, w), (6, ones)]
+    wn = w / np.sqrt((w.astype(np.float64) ** 2).mean() + 1e-5)
+    total = res.astype(np.float64) + x
+    for out, want in ((0, total), (4, total / np.sqrt((total ** 2).mean(1, keepdims=True) + 1e-5) * wn)):
+        got = run(cuda_backend, ops, sizes, io, out, x.shape)
+        assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()

@@ -617,7 +617,7 @@ __device__ void norm_any_sum(float* out, const float* x, const float* res, const
     norm_any_pass(out, x, w_o ? (const float*)nullptr : res, w, cols, kind, eps, gain, sh, xb, wb);
     if (w_o) norm_any_pass(out, out, res, w_o, cols, kind_o, eps, gain, sh, (const float*)nullptr, (const WT*)nullptr);
 }
-// many rows (prompts): what counts is how many rows are resident per SM, so nothing is kept in registers
+// more rows than fit at once in registers (and narrow ones): what counts is how many rows are resident per SM, so nothing is kept in registers
 template <typename WT>
 __global__ void __launch_bounds__(256) k_norm_any_rows(float* dst, const float* src, const WT* __restrict__ w, const float* res, uint32_t cols, uint32_t kind, float eps,
                                                        float* dst2, const WT* __restrict__ w2, uint32_t kind2, float gain, const float* src_b, const WT* __restrict__ w_b,
@@ -649,7 +649,7 @@ __device__ __forceinline__ void norm_any_weights(float (&out)[kKeep], const WT* 
 template <typename WT, int kKeep, int kThreads>          // a row of up to kKeep x kThreads values lives in registers (fewer kept values, more CTAs per SM)
 __global__ void __launch_bounds__(kThreads) k_norm_any(float* dst, const float* src, const WT* __restrict__ w, const float* res, uint32_t cols, uint32_t kind, float eps,
                                                   float* dst2, const WT* __restrict__ w2, uint32_t kind2, float gain, const float* src_b, const WT* __restrict__ w_b,
-                                                       uint32_t kind_o, const WT* __restrict__ w_o) {
+                                                       uint32_t kind_o, const WT* __restrict__ w_o, bool weights_first) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ float sh[kThreads > 512 ? kThreads / 16 : 32];      // of a warp: one sum, or the two sources'
     const size_t row = (size_t)blockIdx.x * cols;
@@ -662,6 +662,7 @@ __global__ void __launch_bounds__(kThreads) k_norm_any(float* dst, const float* 
         }
         return;
     }
+    if (!weights_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     float v[kKeep], wa[kKeep], aux[kKeep], wc[kKeep], bc[kKeep], wo[kKeep];   // aux: the bias of a Dynamic Tanh, or the second source's weight
     norm_any_weights<WT, kKeep>(wa, w, !(kind & 16u), cols, kind);
     norm_any_weights<WT, kKeep>(aux, (kind & 8u) ? w + cols : w_b, (kind & 8u) || src_b, cols, kind);
@@ -669,7 +670,7 @@ __global__ void __launch_bounds__(kThreads) k_norm_any(float* dst, const float* 
     norm_any_weights<WT, kKeep>(wo, w_o, w_o != nullptr, cols, kind_o);
     norm_any_weights<WT, kKeep>(bc, w2 + cols, dst2 && (kind2 & 8u), cols, kind2);
     const float alpha = (kind & 8u) ? wld(w, (size_t)2 * cols) : 0.0f, alpha2 = (dst2 && (kind2 & 8u)) ? wld(w2, (size_t)2 * cols) : 0.0f;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (weights_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     float rv[kKeep], vb[kKeep];
 #pragma unroll
     for (int i = 0; i < kKeep; i++) {
@@ -2624,8 +2625,14 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                                   (s.n[2] & 16u) ? (const WT*)nullptr : wptr<WT>(bufs, s.buf[2], s.off[0]), res, s.n[1], s.n[2], s.f[0], dst2,                \
                                   dst2 && !(s.n[4] & 16u) ? wptr<WT>(bufs, s.buf[5], s.off[1]) : (const WT*)nullptr, s.n[4], s.f[1],                         \
                                   s.n[7] ? (const float*)bufs[s.buf[6]] : (const float*)nullptr, s.n[7] ? wptr<WT>(bufs, s.buf[2], s.off[2]) : (const WT*)nullptr, \
-                                  s.n[8] ? s.n[8] - 1 : 0u, s.n[8] ? wptr<WT>(bufs, s.buf[2], s.off[5]) : (const WT*)nullptr))
-                if (s.n[0] >= 64 || s.n[1] > 4096)
+                                  s.n[8] ? s.n[8] - 1 : 0u, s.n[8] ? wptr<WT>(bufs, s.buf[2], s.off[5]) : (const WT*)nullptr, s.n[0] < 64))
+                // Many rows: the kernel that keeps a row in registers (64 each: 1024 threads an SM) as long as all rows are resident at once.  Each value is then read once
+                // and all its loads are in flight together; the other one walks a row up to four times.  Feed-forwards of f32 / bf16 weights, walked -> in registers:
+                // 64 tokens of 4096 101.4 -> 91.8 / 68.2 -> 63.6 us, 256 of 2048 97.3 -> 92.3 / 53.3 -> 52.2, 256 of 1024 46.9 -> 45.3 / 36.9 -> 34.9.  Up to 512 columns
+                // two values a thread leave nothing to overlap (300 of 512: 37.0 -> 38.6), and past one wave a second one begins where the walk has 2048 threads an SM.
+                // Their weights may come from a launch of the same program: they are read after the wait, as the walk reads them.
+                const uint32_t cols = s.n[1], resident = zg_sm_count() * (cols <= 1024 ? 4u : cols <= 2048 ? 2u : 1u);
+                if (cols > 4096 || (s.n[0] >= 64 && (cols <= 512 || s.n[0] > resident)))
                     ZG_SEQ_WDT(s.n[3], launch_pdl(k_norm_any_rows<WT>, dim3(s.n[0]), dim3(256), 0, st, bufs[s.buf[0]] + s.off[3], (const float*)bufs[s.buf[1]],
                                                   (s.n[2] & 16u) ? (const WT*)nullptr : wptr<WT>(bufs, s.buf[2], s.off[0]), res, s.n[1], s.n[2], s.f[0], dst2,
                                                   dst2 && !(s.n[4] & 16u) ? wptr<WT>(bufs, s.buf[5], s.off[1]) : (const WT*)nullptr, s.n[4], s.f[1],
