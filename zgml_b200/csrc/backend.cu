@@ -1189,8 +1189,8 @@ static bool build_decode_plan(ZgCudaProgram* p, std::vector<DecHostLayer>& layer
 // The cluster form of the fused layers (decode_cluster.cu).  False: not these layers.
 //
 // Up to kZgClusterLayerBytes of weights a layer: its 16 SMs stream about 1 TB/s and a layer takes some 18 us at least, the general schedule (seven launches a layer, all
-// SMs) some 31.  Whole steps, general / cluster: 8 layers of width 128 231 / 190 us, 10 of 384 (F 1024) 325 / 270, 30 of 576 (3.8 MB of Q8_0) 980 / 808, 12 of 768 (6.7 MB)
-// 428 / 415; 8 of 1024 (F 4096): 18 MB of Q8_0 333 / 449, 9.4 MB of Q4_0 333 / 345.
+// SMs) some 31.  Whole steps, general / cluster: 8 layers of width 128 (Q8_0) 228 / 181 us, 10 of 384 (F 1024) 327 / 236, 30 of 576 (3.8 MB) 973 / 748, 12 of 768 (6.7 MB)
+// 429 / 393; 8 of 1024 in Q4_0: 7.2 MB 332 / 316, 9.1 MB 333 / 339; in Q8_0: 13 MB 333 / 383, 16 MB 333 / 437.
 constexpr size_t kZgClusterLayerBytes = 7u << 20;
 static bool build_cluster_plan(ZgCudaProgram* p, const std::vector<DecHostLayer>& layers) {
     ZgClusterHost& h = p->cl;

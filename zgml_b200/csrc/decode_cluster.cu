@@ -2,10 +2,11 @@
 //
 // What bounds such a step is the chain of dependent launches: seven per layer, 31 us for the 3.8 MB of a layer of width 576, whose
 // bytes pass in 2 - 3 us.  Here a layer is five phases on 16 SMs without a launch between them, and what passes from one to the next
-// are vectors in shared memory.  30 layers of width 576 over 512 positions (Q8_0): 985 -> 815 us a token, head and host included, 24 us a
-// layer; 8 layers of width 128: 231 -> 190 us.  What bounds it now is not memory but the walk of the warps through a layer's code: some
-// 45 000 clocks for about 2000 instructions a warp, most of them executed once per layer, each waiting for the one before it or for its
-// own fetch (58 KB of code; attention 9000 clocks, the four products 1700 - 3500 each, reductions and exchanges between them the rest).
+// are vectors in shared memory.  30 layers of width 576 over 512 positions (Q8_0): 981 -> 758 us a token, head and host included, some
+// 22 us a layer; 8 layers of width 128: 228 -> 181 us.  What bounds it now is not memory but the walk of the warps through a layer's
+// code: about 2000 instructions a warp, most of them executed once per layer, each waiting for the one before it or for its own fetch
+// (58 KB of code).  Stamped while a layer still took 24 us, 45 000 clocks: attention 9000, the four products 1700 - 3500 each,
+// reductions and exchanges between them the rest.
 //
 //   1  x (residual stream) -> rmsnorm, gamma in the registers of the consumers -> q | k | v matvecs, whole columns per CTA
 //   2  rope, cache stores, attention: CTA = (KV head, share of the positions), all query heads of the group -> partial states
