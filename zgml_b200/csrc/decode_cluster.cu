@@ -65,9 +65,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm vo
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Relaxed: a releasing arrival waits until the thread's stores to global memory are acknowledged (some 1500 clocks here).  What these order are reads of shared memory, whose
-// values the instructions before them have used.
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// Releases the reads before it, its own and (a __syncwarp or a barrier before it) the other lanes': what they read may be overwritten then.  It also waits until the warp's
+// stores to global memory are acknowledged, some 25 us of a step of 30 layers; storing later, behind the products, made no difference (788 / 790 us) or cost more (795).
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
@@ -95,7 +95,7 @@ __device__ __forceinline__ void push1(uint32_t at, float v, uint32_t bar) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(at), "r"(__float_as_uint(v)), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void arrive_remote(uint32_t bar, uint32_t rank) {
-    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(bar, rank)) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(bar, rank)) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -165,6 +165,13 @@ __device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity) {
         if (++polls == kPolls) asm volatile("st.shared.u32 [%0], %1;" ::"r"(smem_base() + kDead), "r"(1u) : "memory");
         if (dead()) break;
     }
+}
+
+// On a barrier that other CTAs complete: what they did before is seen after it.  (Asked for once more at cluster scope, when it is there: an acquire at that scope
+// empties the L1 at every poll.)
+__device__ __forceinline__ void wait_cluster(uint32_t bar, uint32_t parity) {
+    wait_bar(bar, parity);
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n\t}" ::"r"(bar), "r"(parity) : "memory");
 }
 
 // One phase's share of a CTA: `own` column groups of `nk` records each, dealt to the warps as one list of own * nk records.
@@ -640,7 +647,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
                 }
                 const uint32_t bar = bar_of(c, ph ? kBarA2 : kBarA1);
                 if (ph | l) {
-                    wait_bar(bar, (ph ? l : l - 1) & 1);
+                    wait_cluster(bar, (ph ? l : l - 1) & 1);
                     if (tid == 0) mbar_expect_tx(bar, tx_a);
                 }
                 x = c.base + (ph ? P.o_a2 : P.o_a1); top = x + (P.D + nD) * 4; gamma = gammas + (ph ? P.D * 4 : 0);
@@ -648,7 +655,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
             } else if (ph == 1) {
                 // ── rope, cache, attention over the CTA's positions ──
                 const uint32_t kv = heads + P.n_heads * (uint32_t)sizeof(ZgClusterHead) + g * (uint32_t)sizeof(ZgClusterKv);
-                wait_bar(bar_of(c, kBarQ), l & 1);
+                wait_cluster(bar_of(c, kBarQ), l & 1);
                 if (tid == 0) mbar_expect_tx(bar_of(c, kBarQ), (P.Dq + 2 * P.Dkv) * 4);
                 if (attends) {
                     const uint32_t hd2 = dh >> 1;
@@ -674,7 +681,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
                     kv_base += (lds32(at + 28) + kKvRows - 1) / kKvRows;
                 }
                 // ── merge of the shares ──
-                wait_bar(bar_of(c, kBarT), l & 1);
+                wait_cluster(bar_of(c, kBarT), l & 1);
                 if (tid == 0) mbar_expect_tx(bar_of(c, kBarT), P.n_heads * P.splits * (dh + 4) * 4);
 #pragma unroll 1
                 for (uint32_t kg0 = warp; kg0 < nQ; kg0 += 2 * kW) {      // two groups of 32 side by side
@@ -723,6 +730,8 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
             workers_sync();
             if ((ph & 1) == 0) {
                 if (ph == 0) {
+                    // (every warp is past the layer before)
+                    if (l && warp == kW - 1 && lane == 0) mbar_arrive(bar_of(c, kBarConstEmpty + ((l - 1) & 1)));
                     // ── q | k | v to every CTA ──
 #pragma unroll 1
                     for (uint32_t i = warp; i < own; i += kW) {
@@ -762,7 +771,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
                 const bool down = ph == 3, last = l + 1 == P.n_layers;
                 const uint32_t next = c.base + P.o_const + ((l + down) & 1) * P.const_bytes;      // whose norm takes the sum
                 if (down) {
-                    wait_bar(bar_of(c, kBarGo), l & 1);
+                    wait_cluster(bar_of(c, kBarGo), l & 1);
                     // a column group's records are few here: its partials by the eight lanes of one dg
 #pragma unroll 1
                     for (uint32_t i = warp * 4 + dg; i < own; i += 4 * kW) {
@@ -777,7 +786,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
                     float4 v;
                     if (down) {
                         if (!last) wait_bar(bar_of(c, kBarConstFull + ((l + 1) & 1)), ((l + 1) >> 1) & 1);
-                        wait_bar(bar_of(c, kBarR), l & 1);
+                        wait_cluster(bar_of(c, kBarR), l & 1);
                         if (tid == 0) mbar_expect_tx(bar_of(c, kBarR), ownD * 128 * min(P.F >> 5, kC));
                         const uint32_t r_in = c.base + P.o_r + ((dg * 4 * P.own_max + warp) * 32 + c4) * 4, step = P.own_max * 128;
                         v = add4(add4(ldf4(r_in), ldf4(r_in + step)), add4(ldf4(r_in + 2 * step), ldf4(r_in + 3 * step)));
@@ -800,8 +809,6 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
                 }
             }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_of(c, kBarConstEmpty + (l & 1)));
     }
 }
 #undef LY
@@ -826,7 +833,7 @@ k_decode_cluster(const __grid_constant__ ZgClusterPlan plan) {
         const uint32_t nD = P.D >> 5, ownD = (nD + kC - 1 - c.rank) / kC;
 #pragma unroll 1
         for (uint32_t b = kBarA1; b < kBarFull + 2 * kW * P.ring_slots; b++)
-            mbar_init(bar_of(c, b), b == kBarGo ? kC : b == kBarConstEmpty || b == kBarConstEmpty + 1 ? kW + (c.rank / P.splits < P.n_kv) : b == kBarConstFull || b == kBarConstFull + 1 ? 32 : b >= kBarKvFull && b < kBarKvEmpty ? 33 :
+            mbar_init(bar_of(c, b), b == kBarGo ? kC : b == kBarConstEmpty || b == kBarConstEmpty + 1 ? 1 + (c.rank / P.splits < P.n_kv) : b == kBarConstFull || b == kBarConstFull + 1 ? 32 : b >= kBarKvFull && b < kBarKvEmpty ? 33 :
                                     b >= kBarKvEmpty && b < kBarFull ? 8 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         mbar_expect_tx(bar_of(c, kBarA1), (P.D + 2 * nD) * 4);

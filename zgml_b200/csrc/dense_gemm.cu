@@ -393,8 +393,7 @@ k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            // relaxed: what it orders are the reads of TMEM above (a releasing arrival waits for the outputs' stores)
-            if (lane == 0) asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];" ::"r"(tmem_empty + 8 * acc) : "memory");
+            if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(tmem_empty + 8 * acc) : "memory");
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
