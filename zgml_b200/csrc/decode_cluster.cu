@@ -167,6 +167,12 @@ __device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity) {
     }
 }
 
+// What a warp's bulk copies have still to bring lands before the warp ends, whatever made it end: their CTA's shared memory must not go before (some 60 ms at most).
+__device__ __forceinline__ void settle(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+    for (uint32_t polls = 0; polls < (1u << 14) && !mbar_try(bar, parity); polls++) {}
+}
+
 // On a barrier that other CTAs complete: what they did before is seen after it.  (Asked for once more at cluster scope, when it is there: an acquire at that scope
 // empties the L1 at every poll.)
 __device__ __forceinline__ void wait_cluster(uint32_t bar, uint32_t parity) {
@@ -480,7 +486,12 @@ __device__ __noinline__ void weight_stream(const ZgClusterPlan* plan) {
         }
         if (__any_sync(0xffffffffu, go)) { idle = 0; continue; }
         __nanosleep(100);
-        if (++idle > (1u << 23) || dead()) return;      // a second and more
+        if (++idle > (1u << 23) || dead()) break;      // a second and more
+    }
+#pragma unroll 1
+    for (uint32_t s = 0; s < P.ring_slots; s++) {
+        const uint32_t fills = wrapped + (s < slot);
+        if (lane < kW && fills) settle(full + 8 * s, (fills - 1) & 1);
     }
 }
 // The list of a warp's copies in one layer: entry {8 * weight | bytes << 8, offset}; counts behind the lists.  By one lane per warp, before the start.
@@ -535,7 +546,7 @@ __device__ __noinline__ void kv_stream(const ZgClusterPlan* plan, uint32_t rank)
             const uint32_t st = cum & (P.kv_stages - 1), turn = cum >> lg, bytes = min(kKvRows, len - p) * row;
             const float m = mask ? __ldcg(mask + (size_t)(lo + min(p + lane, len - 1)) * mask_rs) : 0.0f;
             if (turn) wait_bar(bars + 8 * (kBarKvEmpty + st), (turn - 1) & 1);
-            if (dead()) return;
+            if (dead()) { l = P.n_layers; break; }
             const uint32_t dst = base + P.o_kv + st * stage, bar = bars + 8 * (kBarKvFull + st);
             stf(dst + 2 * kKvRows * row + lane * 4, m);
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");      // releases the mask
@@ -546,6 +557,8 @@ __device__ __noinline__ void kv_stream(const ZgClusterPlan* plan, uint32_t rank)
             }
         }
     }
+#pragma unroll 1
+    for (uint32_t st = 0; st < min(cum, P.kv_stages); st++) settle(bars + 8 * (kBarKvFull + st), ((cum - 1 - st) >> lg) & 1);
 }
 
 // The layer's small operands, one layer ahead: [block][gamma1][gamma2][cos | sin][scale ceilings of the CTA's column groups][positions: those of the heads, the new one
@@ -555,10 +568,11 @@ __device__ __noinline__ void const_stream(const ZgClusterPlan* plan, uint32_t ra
     const uint32_t lane = threadIdx.x & 31, g = rank / P.splits, split = rank - g * P.splits, base = smem_base(), bars = base + P.o_bars;
     const ZgClusterLayer* ly = reinterpret_cast<const ZgClusterLayer*>(P.blocks);
     const float* smax = P.smax + (size_t)rank * 4 * kMaxItems;
+    uint32_t l = 0;
 #pragma unroll 1
-    for (uint32_t l = 0; l < P.n_layers; l++) {
+    for (; l < P.n_layers; l++) {
         if (l >= 2) wait_bar(bars + 8 * (kBarConstEmpty + (l & 1)), ((l >> 1) - 1) & 1);
-        if (dead()) return;
+        if (dead()) break;
         const uint32_t area = base + P.o_const + (l & 1) * P.const_bytes, at = area + P.const_bytes - 48, bar = bars + 8 * (kBarConstFull + (l & 1));
         if (lane < 5) {
             const void* src = lane == 0 ? (const void*)ly : lane == 1 ? (const void*)ly->gamma[0] : lane == 2 ? (const void*)ly->gamma[1] : lane == 3 ? (const void*)ly->cs : (const void*)smax;
@@ -582,6 +596,8 @@ __device__ __noinline__ void const_stream(const ZgClusterPlan* plan, uint32_t ra
         ly = reinterpret_cast<const ZgClusterLayer*>(reinterpret_cast<const uint8_t*>(ly) + P.blk_bytes);
         smax += kC * 4 * kMaxItems;
     }
+    if (l > 1) settle(bars + 8 * (kBarConstFull + (l & 1)), ((l - 2) >> 1) & 1);
+    if (l) settle(bars + 8 * (kBarConstFull + ((l - 1) & 1)), ((l - 1) >> 1) & 1);
 }
 
 template <int NI>
@@ -889,9 +905,11 @@ k_decode_cluster(const __grid_constant__ ZgClusterPlan plan) {
         atomicAdd(&g_timeouts, 1u);
     }
     cluster_sync();      // nobody leaves while others may still store into its shared memory
-    if (*reinterpret_cast<volatile uint32_t*>(P.err) && c.warp < kW) {      // a wait gave up: the step's results are not to be used
+    if (*reinterpret_cast<volatile uint32_t*>(P.err)) {      // a wait gave up: the step's results are not to be used, and stores to other CTAs may be under way that nobody has waited for
+        __nanosleep(100000);
+        cluster_sync();
         const ZgClusterLayer* ly = reinterpret_cast<const ZgClusterLayer*>(P.blocks + (size_t)(P.n_layers - 1) * P.blk_bytes);
-        for (uint32_t i = c.rank * kT + c.tid; i < P.D; i += kC * kT) ly->out[6][i] = __int_as_float(0x7fc00000);
+        for (uint32_t i = c.rank * kT + c.tid; c.tid < kT && i < P.D; i += kC * kT) ly->out[6][i] = __int_as_float(0x7fc00000);
     }
 }
 
