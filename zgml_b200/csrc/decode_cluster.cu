@@ -485,6 +485,7 @@ __device__ __noinline__ void weight_stream(const ZgClusterPlan* plan) {
             if (++i == n) { i = 0; left = ptrs != last; ptrs += 56; }
         }
         if (__any_sync(0xffffffffu, go)) { idle = 0; continue; }
+        if (idle == 0) asm volatile("griddepcontrol.wait;" ::: "memory");      // no slot comes free before the predecessor has completed, however long that takes: no bounded wait before
         __nanosleep(100);
         if (++idle > (1u << 23) || dead()) break;      // a second and more
     }
