@@ -314,7 +314,7 @@ k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
 
     if (warp == 0) {
         if (lane == 0) {
-            uint32_t s = 0, ph = 1;
+            uint32_t s = 0, ph = 1, fills = 0;
             bool ok = true;
             for (uint32_t t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
                 const ZgExpertSegment seg = run_of(t);
@@ -327,13 +327,16 @@ k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
                     tma_load_3d(at, &tmap_w, kt * BK, f0, (uint32_t)seg.expert, full + 8 * s);
                     if (PAIR) tma_load_3d(at + kTileA, &tmap_w2, kt * BK, DUAL ? f0 : f0 + BM, (uint32_t)seg.expert, full + 8 * s);
                     for (uint32_t c = 0; c < copies; c++) tma_2d(at + kWeights + c * (kExpertRows * BK * 2), &tmap_x, kt * BK, (uint32_t)seg.start + c * kExpertRows, full + 8 * s);
+                    fills++;
                     if (++s == stages) { s = 0; ph ^= 1; }
                 }
             }
+            // the copies that are under way land before the CTA's shared memory goes, whatever gave up
+            for (uint32_t i = 0; i < min(fills, stages); i++) mbar_wait(full + 8 * i, ((fills - 1 - i) / stages) & 1);
         }
     } else if (warp == 1) {
         const bool leader = elect_one();
-        uint32_t s = 0, ph = 0, i = 0;
+        uint32_t s = 0, ph = 0, i = 0, last = 0, last_ph = 0;
         bool ok = true;
         for (uint32_t t = blockIdx.x; ok && t < tiles; t += gridDim.x, i++) {
             // instruction descriptor (kind::f16): D = F32, A = B = BF16, both K-major, N = the run's rows, M = 128
@@ -354,21 +357,34 @@ k_expert_gemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
                     }
                 if (leader) mma_commit(empty + 8 * s);
                 if (leader && kt + 1 == n_k) mma_commit(tmem_full + 8 * acc);
+                last = empty + 8 * s; last_ph = ph;
                 if (++s == stages) { s = 0; ph ^= 1; }
             }
         }
+        if (!ok && last) mbar_wait(last, last_ph);      // products under way end before their accumulators go
         __syncwarp();
     } else {
         // TMEM lane = output column of the tile's 128, TMEM column = row of the run; the two warps of a quarter take 16 rows each in turn
         const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
         uint32_t i = 0;
+        bool ok = true;
         for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
             const ZgExpertSegment seg = run_of(t);
             const uint32_t n = (uint32_t)seg.rows, f = t % n_f * ROWS + quarter * 32 + lane, acc = two ? i & 1 : 0, use = two ? i >> 1 : i;
-            const bool ok = __all_sync(0xffffffffu, mbar_wait(tmem_full + 8 * acc, use & 1));       // (what the other roles gave up on does not arrive here either)
-            if (!ok) {
-                if (lane == 0) count_timeout();
-                break;
+            if (ok) {
+                ok = __all_sync(0xffffffffu, mbar_wait(tmem_full + 8 * acc, use & 1));       // (what the other roles gave up on does not arrive here either)
+                if (!ok && lane == 0) count_timeout();
+            }
+            if (!ok) {      // the outputs of this tile and of those after it are not numbers
+                for (uint32_t c = half; f < p.N && c < n; c += 2) {
+                    const size_t at = ((size_t)seg.start + c) * p.N + f;
+                    if (DUAL) reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(__int_as_float(0x7fc00000));
+                    else {
+                        reinterpret_cast<float*>(p.out)[at] = __int_as_float(0x7fc00000);
+                        if (PAIR && f + BM < p.N) reinterpret_cast<float*>(p.out)[at + BM] = __int_as_float(0x7fc00000);
+                    }
+                }
+                continue;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (uint32_t c0 = 16 * half; c0 < n; c0 += 32) {
