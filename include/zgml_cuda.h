@@ -516,7 +516,7 @@ void* zg_cuda_program_buffer(ZgCudaProgram* prog, uint32_t buf_idx);
  * 4: HBM bytes per execution saved by promoted dense operands (zg_cuda_program_promote_dense); 5: waits that kernels have given up on
  * since process start (dense and f32 matmuls, attention, LINEAR of few rows, quantized matmuls of three to eight, DELTA_RULE; 0 in a healthy run); 6: LINEAR ops of the program whose bfloat16 weights run on the tensor cores;
  * 7: f32 slots of the scratch that the program's tensor-core kernels and sequence ops share; 8: LINEAR ops whose weight nothing in the program writes, so that a
- * launch may read it before its predecessor has completed. */
+ * launch may read it before its predecessor has completed; 9: NORM and STREAM_STEP ops with such weights. */
 uint64_t zg_cuda_program_stats(const ZgCudaProgram* prog, int what);
 /* Run the program's ops with no host<->device copies (inputs already resident);
  * asynchronous on the ctx stream. */

@@ -783,7 +783,7 @@ class CudaBackend:
         return {"kernels": int(f(handle.ptr, 0)), "fused_decode_ops": int(f(handle.ptr, 1)), "fused_decode_layers": int(f(handle.ptr, 2)),
                 "streamed_matvec_launches": int(f(handle.ptr, 3)), "dense_bytes_saved_per_execution": int(f(handle.ptr, 4)),
                 "dense_gemm_timeouts": int(f(handle.ptr, 5)), "tensor_core_linears": int(f(handle.ptr, 6)), "shared_scratch_elems": int(f(handle.ptr, 7)),
-                "early_weight_linears": int(f(handle.ptr, 8))}
+                "early_weight_linears": int(f(handle.ptr, 8)), "early_weight_norms": int(f(handle.ptr, 9))}
 
 
 class QuantizedWeight:

@@ -1335,11 +1335,17 @@ static void find_written(ZgCudaProgram* p) {
         p->written[b] = at != spans.begin() && (at - 1)->second > p->buffers[b];
     }
 }
-// Whether a sequence op's weight may be read before the launch's predecessor has completed: nothing in the program writes it, and what was enqueued before
+// Whether a sequence op's weights may be read before the launch's predecessor has completed: nothing in the program writes them, and what was enqueued before
 // the program has completed when its graph starts (launches outside a graph may overlap the end of the program before).
 static bool const_weights(const ZgCudaProgram* p, const ZgOp& op) {
-    const uint32_t b = op.u.seq.buf[2];
-    return p->ctx->graph_mode && !p->ctx->profiling && b < p->written.size() && !p->written[b];
+    const uint32_t* buf = op.u.seq.buf;
+    const auto kept = [&](uint32_t b) { return b == ZG_NO_BUF || (b < p->written.size() && !p->written[b]); };
+    if (!p->ctx->graph_mode || p->ctx->profiling) return false;
+    switch (op.tag) {
+        case ZG_OP_NORM: return kept(buf[2]) && kept(buf[5]);             // the norm's weights and those of the one chained to it
+        case ZG_OP_STREAM_STEP: return kept(buf[3]) && kept(buf[4]);      // the closing and the opening side's
+        default: return buf[2] != ZG_NO_BUF && kept(buf[2]);
+    }
 }
 
 // The same of the rows of earlier positions that a CACHED_ATTENTION reads: all that the program writes into the cache's memory are this step's rows, by CACHE_APPENDs
@@ -2355,6 +2361,7 @@ extern "C" uint64_t zg_cuda_program_stats(const ZgCudaProgram* p, int what) {
         case 6: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && op.u.seq.n[5] == ZG_W_BF16 && zg_seq_op_scratch_elems(op, p->buffers.data())) n++; return n; }
         case 7: return p->ws.gemm_scratch_elems;
         case 8: { uint64_t n = 0; for (const ZgOp& op : p->ops) if (op.tag == ZG_OP_LINEAR && const_weights(p, op)) n++; return n; }
+        case 9: { uint64_t n = 0; for (const ZgOp& op : p->ops) if ((op.tag == ZG_OP_NORM || op.tag == ZG_OP_STREAM_STEP) && const_weights(p, op)) n++; return n; }
         case 0: return p->graph_kernels;
         case 1: return p->dec.valid || p->cl.valid ? p->dec_count : 0;
         case 2: return p->dec.valid ? p->dec.plan.n_layers : p->cl.valid ? p->cl.plan.n_layers : 0;

@@ -496,10 +496,11 @@ template <typename WT>
 __global__ void k_norm(float* __restrict__ dst, const float* __restrict__ src, const WT* __restrict__ w, const float* __restrict__ res,
                        uint32_t cols, uint32_t kind, float eps, float* __restrict__ dst2, const WT* __restrict__ w2, uint32_t kind2, float gain,
                        const WT* __restrict__ shift_mix, float* __restrict__ shift_state, const float* __restrict__ ctl,
-                       const WT* __restrict__ avg_coeff, uint32_t avg_terms, uint32_t avg_stride, float* __restrict__ avg_out) {
-    // Rows that fit the registers: the norm weights are constants of the model and are read BEFORE the wait on the predecessor;
+                       const WT* __restrict__ avg_coeff, uint32_t avg_terms, uint32_t avg_stride, float* __restrict__ avg_out, bool weights_first) {
+    // Rows that fit the registers: norm weights that nothing in the program writes (weights_first) are read BEFORE the wait on the predecessor;
     // the row and the residual are read together right after it, so the kernel has one round of global loads, not three.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!weights_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float sh[32];
     const size_t row = (size_t)blockIdx.x * cols;
     const float* x = src + row;
@@ -513,7 +514,7 @@ __global__ void k_norm(float* __restrict__ dst, const float* __restrict__ src, c
             wb[i] = (dst2 && c < cols) ? norm_weight(wld(w2, norm_col(c, kind2)), kind2, gain) : 0.0f;
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (weights_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (cached) {
         if (avg_terms) {   // the row to norm is a weighted sum of `avg_terms` streams (a depth average), kept in avg_out too
 #pragma unroll
@@ -2625,12 +2626,12 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                                   (s.n[2] & 16u) ? (const WT*)nullptr : wptr<WT>(bufs, s.buf[2], s.off[0]), res, s.n[1], s.n[2], s.f[0], dst2,                \
                                   dst2 && !(s.n[4] & 16u) ? wptr<WT>(bufs, s.buf[5], s.off[1]) : (const WT*)nullptr, s.n[4], s.f[1],                         \
                                   s.n[7] ? (const float*)bufs[s.buf[6]] : (const float*)nullptr, s.n[7] ? wptr<WT>(bufs, s.buf[2], s.off[2]) : (const WT*)nullptr, \
-                                  s.n[8] ? s.n[8] - 1 : 0u, s.n[8] ? wptr<WT>(bufs, s.buf[2], s.off[5]) : (const WT*)nullptr, s.n[0] < 64))
+                                  s.n[8] ? s.n[8] - 1 : 0u, s.n[8] ? wptr<WT>(bufs, s.buf[2], s.off[5]) : (const WT*)nullptr, const_weights && s.n[0] < 64))
                 // Many rows: the kernel that keeps a row in registers (64 each: 1024 threads an SM) as long as all rows are resident at once.  Each value is then read once
                 // and all its loads are in flight together; the other one walks a row up to four times.  Feed-forwards of f32 / bf16 weights, walked -> in registers:
                 // 64 tokens of 4096 101.4 -> 91.8 / 68.2 -> 63.6 us, 256 of 2048 97.3 -> 92.3 / 53.3 -> 52.2, 256 of 1024 46.9 -> 45.3 / 36.9 -> 34.9.  Up to 512 columns
                 // two values a thread leave nothing to overlap (300 of 512: 37.0 -> 38.6), and past one wave a second one begins where the walk has 2048 threads an SM.
-                // Their weights may come from a launch of the same program: they are read after the wait, as the walk reads them.
+                // Their weights are read after the wait, as the walk reads them.
                 const uint32_t cols = s.n[1], resident = zg_sm_count() * (cols <= 1024 ? 4u : cols <= 2048 ? 2u : 1u);
                 if (cols > 4096 || (s.n[0] >= 64 && (cols <= 512 || s.n[0] > resident)))
                     ZG_SEQ_WDT(s.n[3], launch_pdl(k_norm_any_rows<WT>, dim3(s.n[0]), dim3(256), 0, st, bufs[s.buf[0]] + s.off[3], (const float*)bufs[s.buf[1]],
@@ -2653,7 +2654,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             ZG_SEQ_WDT(s.n[3], launch_pdl(k_norm<WT>, dim3(s.n[0]), dim3(256), 0, st, bufs[s.buf[0]] + s.off[3], bufs[s.buf[1]], wptr<WT>(bufs, s.buf[2], s.off[0]), res, s.n[1], s.n[2], s.f[0],
                                           dst2, dst2 ? wptr<WT>(bufs, s.buf[5], s.off[1]) : nullptr, s.n[4], s.f[1],
                                           shift_state ? wptr<WT>(bufs, s.buf[dst2 ? 5 : 2], s.off[2]) : nullptr, shift_state, shift_state ? bufs[s.buf[7]] : nullptr,
-                                          avg_terms ? wptr<WT>(bufs, s.buf[2], s.off[4]) : nullptr, avg_terms, s.n[6], avg_terms ? bufs[s.buf[4]] : nullptr));
+                                          avg_terms ? wptr<WT>(bufs, s.buf[2], s.off[4]) : nullptr, avg_terms, s.n[6], avg_terms ? bufs[s.buf[4]] : nullptr, const_weights));
             ZG_SEQ_CHECK();
             return true;
         }
@@ -2835,7 +2836,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             return true;
         }
         default:
-            if (op.tag >= ZG_OP_STREAM_STEP) return zg_launch_stream_op(op, bufs, st);
+            if (op.tag >= ZG_OP_STREAM_STEP) return zg_launch_stream_op(op, bufs, st, const_weights);
             return op.tag >= ZG_OP_SSM_SCAN ? zg_launch_rec_op(op, bufs, scratch, st) : zg_launch_mix_op(op, bufs, scratch, st, ahead);
     }
 }

@@ -15,6 +15,7 @@ struct StArgs {
     float* dst; const float* src; const float* y; float* h; float* state; const float* ctl;
     uint32_t T, D, streams, stride, kind, shifts, rows;      // stride: between the old streams; rows: walked by one thread
     float mult, gain;
+    bool weights_first;      // nothing in the program writes the weights: they may be read before the wait on the predecessor
 };
 template <typename WT, int V>
 __device__ __forceinline__ void st_weights(float (&out)[V], const WT* __restrict__ w) {
@@ -42,8 +43,9 @@ __device__ __forceinline__ void st_store(float* __restrict__ p, const float (&v)
 template <typename WT, int S, int V, bool SHIFT>
 __global__ void __launch_bounds__(128) k_stream_step(StArgs a, const WT* __restrict__ w_out, const WT* __restrict__ w_mix, const WT* __restrict__ w_ls,
                                                       const WT* __restrict__ w_in, const WT* __restrict__ w_norm, const WT* __restrict__ w_mu) {
-    // Weights are constants of the model and are read before the wait on the predecessor.
+    // Weights that nothing in the program writes are read before the wait on the predecessor.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!a.weights_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t n = S < kStMaxStreams ? S : a.streams;
     const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     const bool on = c < a.D, close = a.y != nullptr, open = a.h != nullptr, tanh_norm = a.kind & 8u;
@@ -67,7 +69,7 @@ __global__ void __launch_bounds__(128) k_stream_step(StArgs a, const WT* __restr
         }
     }
     __syncthreads();
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (a.weights_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (!on) return;
     const size_t TD = (size_t)a.T * a.D;
     // row t: new streams (written when `write`) and the opened input of the next sublayer
@@ -174,13 +176,14 @@ bool zg_stream_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char
     return true;
 }
 
-bool zg_launch_stream_op(const ZgOp& op, float* const* bufs, cudaStream_t st) {
+bool zg_launch_stream_op(const ZgOp& op, float* const* bufs, cudaStream_t st, bool const_weights) {
     const ZgSeqOp& s = op.u.seq;
     const bool close = s.buf[2] != ZG_NO_BUF, open = s.buf[5] != ZG_NO_BUF;
     auto ptr = [&](int i) { return s.buf[i] != ZG_NO_BUF ? bufs[s.buf[i]] : (float*)nullptr; };
     StArgs a;
     a.dst = ptr(0); a.src = bufs[s.buf[1]]; a.y = ptr(2); a.h = ptr(5); a.state = ptr(6); a.ctl = ptr(7);
     a.T = s.n[0]; a.D = s.n[1]; a.streams = s.n[2]; a.stride = s.n[3]; a.kind = s.n[5]; a.shifts = s.n[6]; a.mult = s.f[0]; a.gain = s.f[1];
+    a.weights_first = const_weights;
     a.rows = a.shifts && a.T > 4 ? 4 : 1;              // a token shift computes the row before each walk once more
 #define ZG_ST(S_)                                                                                  \
     do {                                                                                           \

@@ -440,7 +440,7 @@ uint32_t zg_seq_op_writes(uint32_t tag);
 unsigned int zg_seq_timeouts();       // waits that gave up (LINEAR of few rows, DELTA_RULE's walk)
 // shared activation scratch the op stages through (0: none); least: what that form does not work without
 size_t zg_seq_op_scratch_elems(const ZgOp& op, float* const* bufs, bool least = false);
-// ahead: nothing writes the op's weight (buf 2; CACHED_ATTENTION: the cache's rows of earlier positions) while the program runs, so that it may be read before the
+// ahead: nothing writes the op's weights (CACHED_ATTENTION: the cache's rows of earlier positions) while the program runs, so that they may be read before the
 // launch's predecessor has completed
 bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool ahead);
 // dense_gemm.cu : bf16 x bf16 -> f32 prefill matmul on tcgen05 (TMA-fed, TMEM accumulator)
@@ -480,4 +480,4 @@ bool zg_dense_gemm_batched_launch(const void* w_bf16, const float* src, float* d
                                   uint32_t dst_hs, uint32_t dst_rs, float* scratch, cudaStream_t st, uint32_t act_last, float act_p);
 // streamops.cu : ZG_OP_STREAM_STEP
 bool zg_stream_op_valid(const ZgOp& op, const size_t* elems, size_t n_bufs, char* why, size_t why_n);
-bool zg_launch_stream_op(const ZgOp& op, float* const* bufs, cudaStream_t st);
+bool zg_launch_stream_op(const ZgOp& op, float* const* bufs, cudaStream_t st, bool const_weights);
