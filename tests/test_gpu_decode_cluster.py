@@ -78,6 +78,27 @@ def test_not_finite_input_comes_out_as_the_oracle_has_it(cuda_backend):
         ref.close()
 
 
+def test_op_by_op_steps_report_no_wait(cuda_backend):
+    """Profiled steps run op by op, without the kernel: what its error word held when it was allocated is not an error."""
+    from zgml_b200 import DeviceBuffer
+    from zgml_b200.backend import last_error
+    cfg = LlamaConfig(vocab_size=64, d_model=64, n_layers=1, n_heads=1, n_kv_heads=1, d_ff=64, max_seq_len=16)
+    old = [DeviceBuffer(cuda_backend, 512, zero=False) for _ in range(8192)]      # small allocations that leave their contents behind
+    for b in old:
+        b.upload(np.full(128, -1, np.int32))
+    for b in old:
+        b.free()
+    dev = DeviceLlamaSession(cuda_backend, cfg, synthetic_weights(cfg, "q8_0", seed=1), 1)
+    assert cuda_backend.program_stats(dev.handle)["fused_decode_layers"] == 1
+    cuda_backend.set_profiling(True)
+    try:
+        dev.step(3)
+    finally:
+        cuda_backend.set_profiling(False)
+    assert "gave up" not in last_error()
+    dev.close()
+
+
 def test_layers_beyond_its_size_keep_the_general_schedule(cuda_backend):
     cfg = LlamaConfig(vocab_size=64, d_model=1024, n_layers=1, n_heads=16, n_kv_heads=4, d_ff=2048, max_seq_len=64)      # 9.5 MB of Q8_0
     dev = DeviceLlamaSession(cuda_backend, cfg, synthetic_weights(cfg, "q8_0", seed=1), 1)

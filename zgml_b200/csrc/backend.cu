@@ -1306,7 +1306,7 @@ static bool build_cluster_plan(ZgCudaProgram* p, const std::vector<DecHostLayer>
         }
     }
     if (cudaMalloc(&h.d_blocks, blocks.size()) != cudaSuccess || cudaMalloc(&h.d_smax, smax.size() * sizeof(float)) != cudaSuccess || cudaMalloc(&h.d_err, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMallocHost(&h.h_err, sizeof(uint32_t)) != cudaSuccess || cudaMemcpy(h.d_blocks, blocks.data(), blocks.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMallocHost(&h.h_err, sizeof(uint32_t)) != cudaSuccess || cudaMemset(h.d_err, 0, sizeof(uint32_t)) != cudaSuccess || cudaMemcpy(h.d_blocks, blocks.data(), blocks.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(h.d_smax, smax.data(), smax.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) { cudaGetLastError(); zg_decode_cluster_free(&h); return false; }
     *h.h_err = 0;
     P.blocks = (const uint8_t*)h.d_blocks; P.smax = h.d_smax; P.err = h.d_err;
@@ -2218,7 +2218,12 @@ extern "C" void zg_cuda_execute(ZgCudaCtx* ctx, ZgCudaProgram* p, const ZgIO* in
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) zg_set_error("execute: %s", cudaGetErrorString(e));
     zg_peer_check_result(ctx);
-    if (p->cl.valid && *p->cl.h_err) zg_set_error("execute: a wait of the cluster decode kernel gave up; the step's outputs are invalid");
+    if (p->cl.valid && *p->cl.h_err) {
+        zg_set_error("execute: a wait of the cluster decode kernel gave up; the step's outputs are invalid");
+        cudaMemsetAsync(p->cl.d_err, 0, sizeof(uint32_t), st);      // (a step that runs op by op does not set it)
+        cudaStreamSynchronize(st);
+        *p->cl.h_err = 0;
+    }
     if (p->dec.valid && *p->dec.h_err) {   // a bounded wait inside the fused decode kernel gave up: results are invalid
         static const char* what[] = {"", "grid barrier", "weight ring (TMA)", "NVLink peer all-reduce: a peer rank never arrived"};
         zg_set_error("execute: fused decode kernel timed out in its %s wait; the step's outputs are invalid", what[*p->dec.h_err & 3]);
