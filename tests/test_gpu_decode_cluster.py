@@ -78,6 +78,39 @@ def test_not_finite_input_comes_out_as_the_oracle_has_it(cuda_backend):
         ref.close()
 
 
+@pytest.mark.parametrize("heads,kv,ff,kind", [(9, 3, 1536, "q8_0"), (9, 3, 1536, "q4_0"), (12, 4, 2048, "q8_0"), (6, 2, 1024, "q8_0"), (6, 2, 1024, "q4_0")])
+def test_no_coarser_beside_channels_that_stand_out(cuda_backend, general, heads, kv, ff, kind):
+    """gate and up against 64 bits where one channel of the normed row is 30 000 times the others and its weights are zero: what is left is the grid that the others are cut
+    on, 2^-24 of the largest value of their range.  The ranges are those of the general schedule, so the errors are alike over all places of the channel (a tenth for the other
+    order of sums)."""
+    from zgml_b200 import ProgramIO, abi
+    width = 64 * heads
+    cfg = LlamaConfig(vocab_size=8, d_model=width, n_layers=1, n_heads=heads, n_kv_heads=kv, d_ff=ff, max_seq_len=8)
+    err = {}
+    for record in range(width // 32):
+        w, k = synthetic_weights(cfg, kind, seed=record, embed_scale=1.0), 32 * record + 5
+        w.norm2[0][k] = 3e4
+        for name in ("w_gate", "w_up"):
+            w.layers[0][name].data.reshape(width, -1)[k] = 0
+        for be in (cuda_backend, general):
+            s = DeviceLlamaSession(be, cfg, w, 1)
+            assert be.program_stats(s.handle)["fused_decode_layers"] == (1 if be is cuda_backend else 0)
+            ops = s.lp.program.ops
+            at = [i for i, op in enumerate(ops) if op.tag == abi.OP_QMATMUL]          # q, k, v, o, gate, up, down
+            bufs = [np.zeros(n, np.float32) for n in s.lp.program.buffer_sizes]
+            s.outputs = [ProgramIO(i, b) for i, b in enumerate(bufs)]
+            s.execute_at([1], 0)
+            x = bufs[ops[at[3] + 1].u.elementwise.dst].astype(np.float64)              # x after attention
+            x = x / np.sqrt((x ** 2).mean() + cfg.rms_norm_eps) * w.norm2[0]
+            for name, i in (("w_gate", at[4]), ("w_up", at[5])):
+                u = w.layers[0][name]
+                want = x @ (u.data * np.repeat(u.scales.astype(np.float64), 32)).reshape(width, -1)
+                err.setdefault(be, []).append(np.linalg.norm(bufs[ops[i].u.qmatmul.dst] - want) / np.linalg.norm(want))
+            s.close()
+    mean = {be: np.sqrt(np.mean(np.square(e))) for be, e in err.items()}
+    assert mean[cuda_backend] <= 1.1 * mean[general]
+
+
 def test_op_by_op_steps_report_no_wait(cuda_backend):
     """Profiled steps run op by op, without the kernel: what its error word held when it was allocated is not an error."""
     from zgml_b200 import DeviceBuffer

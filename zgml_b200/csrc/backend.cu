@@ -1265,6 +1265,14 @@ static bool build_cluster_plan(ZgCudaProgram* p, const std::vector<DecHostLayer>
     P.n_layers = (uint32_t)layers.size(); P.D = D; P.Dq = H * dh; P.Dkv = G * dh; P.F = F; P.n_heads = H; P.n_kv = G; P.dh = dh;
     P.blk_bytes = (uint32_t)((sizeof(ZgClusterLayer) + H * sizeof(ZgClusterHead) + G * sizeof(ZgClusterKv) + 15) & ~(size_t)15);
     h.fmt = (int)ph0[0].fmt;
+    for (int ph = 0; ph < 4; ph++) {
+        ZgCudaQWeight w;
+        w.fmt = (int)ph0[ph].fmt; w.n_kc = ph0[ph].n_kc; w.rec_bytes = ph0[ph].rec_bytes; w.n_nb = 0;
+        for (uint32_t m = 0; m < ph0[ph].n_mv; m++) w.n_nb = std::max(w.n_nb, ph0[ph].mv[m].n_nb);
+        const ZgGemvPlan pl = zg_qgemv_plan(p->ctx, &w, 1, 1);
+        if (pl.threads != 32 * kZgClusterRanges) return false;
+        P.splits_k[ph] = pl.S;
+    }
     if (!zg_decode_cluster_layout(P, h.fmt)) return false;
     std::vector<uint8_t> blocks((size_t)P.n_layers * P.blk_bytes, 0);
     for (size_t l = 0; l < layers.size(); l++) {

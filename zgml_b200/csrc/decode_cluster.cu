@@ -111,6 +111,11 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(addr));
     return r;
 }
+__device__ __forceinline__ uint32_t lds8(uint32_t addr) {
+    uint32_t r;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(r) : "r"(addr));
+    return r;
+}
 __device__ __forceinline__ float ldf(uint32_t addr) { return __uint_as_float(lds32(addr)); }
 __device__ __forceinline__ float2 ldf2(uint32_t addr) {
     float2 r;
@@ -203,6 +208,8 @@ __host__ __device__ inline uint32_t item_of(const ZgClusterPlan& P, uint32_t ran
 }
 
 // ── a warp's records of one phase: partial sums of its stretch of every column group that it touches -> part[warp * seg + n][32] ──
+// Activations share a scale over the records that lie in one range of the general schedule (a warp's there), so that none is cut on a coarser grid than there: with a scale for
+// the whole stretch, seven records instead of two or three, gate and up of width 576 were off by 1.6 times as much beside channels that stand out (and a step of 30 layers took 788 us, with the ranges 800).
 // Addresses in shared memory: x: the K values; gamma: 0, or x * inv * gamma is what is multiplied; top: largest magnitude of 32 values of x (times gamma).
 __device__ __noinline__ float true_max(uint32_t x, uint32_t gamma, float inv, uint32_t n) {      // the bound was infinite, the products may not be
     float mx = 0.0f;
@@ -215,13 +222,14 @@ __device__ __noinline__ float true_max(uint32_t x, uint32_t gamma, float inv, ui
     return warp_max(mx);
 }
 template <int FMT>
-__device__ __forceinline__ void matvec(const Cta& c, const ZgClusterPlan& P, uint2 stretch, uint32_t nk, uint32_t x, uint32_t gamma, float inv, uint32_t top, uint32_t smax, uint32_t part,
+__device__ __forceinline__ void matvec(const Cta& c, const ZgClusterPlan& P, uint2 stretch, uint32_t nk, uint32_t lens, uint32_t x, uint32_t gamma, float inv, uint32_t top, uint32_t smax, uint32_t part,
                                        uint32_t& slot, uint32_t& parity) {
     constexpr bool kI4 = (FMT == ZG_QFMT_I4_F16), kF32 = (FMT == ZG_QFMT_I8_F32);
     constexpr uint32_t QB = kI4 ? 512u : 1024u, SB = kF32 ? 32u : 16u, RB = QB + 4 * SB, G = turn_records(FMT), kSlotBytes = G * RB;
     static_assert(RB == record_bytes(FMT), "record");
     const uint32_t lane = c.lane, warp = c.warp, gq = lane >> 2, t = lane & 3;
-    uint32_t left = stretch.x, item = stretch.y & 0xffffu, k = stretch.y >> 16;
+    lens += stretch.x >> 16;
+    uint32_t left = stretch.x & 0xffffu, item = stretch.y & 0xffffu, k = stretch.y >> 16;
     uint32_t out = part + warp * P.seg * 128 + ((t >> 1) * 16 + gq + 8 * (t & 1)) * 4;
     if (left == 0) {         // fewer records than warps: the sum over the warps of an item passes this one
         stf(out, 0.0f);
@@ -230,9 +238,10 @@ __device__ __forceinline__ void matvec(const Cta& c, const ZgClusterPlan& P, uin
     const uint32_t planes = c.base + P.o_planes + warp * kPlaneBytes, brow = planes + (gq & 3) * 32 + 4 * t;
     const uint32_t sc_off = QB + (kF32 ? 4u : 2u) * (8 * ((lane & 15) >> 2) + 4 * (lane >> 4) + (lane & 3));
     const uint32_t ring = c.base + P.o_ring + warp * P.ring_slots * kSlotBytes, full = bar_of(c, kBarFull + warp * P.ring_slots), empty = full + 8 * kW * P.ring_slots;
+    float sum = 0.0f;
 #pragma unroll 1
     while (left) {
-        const uint32_t n = min(nk - k, left);
+        const uint32_t n = lds8(lens++);
         float mx = 0.0f;
 #pragma unroll 1
         for (uint32_t j = lane; j < n; j += 32) mx = fmaxf(mx, ldf(top + (k + j) * 4));
@@ -312,10 +321,13 @@ __device__ __forceinline__ void matvec(const Cta& c, const ZgClusterPlan& P, uin
         if constexpr (kI4) T += -8 * dS - 12582912LL * (ones - 8LL * (long long)((n + G - 1) / G * G * ZG_KR));
         else T -= 12582912LL * ones;
         const float esc = (mx <= 3.0e38f) ? ((mx >= 1.0e-30f) ? (mx * (2.004008016f * 1.1920928955078125e-07f)) * sm : 0.0f) : __int_as_float(0x7fc00000);
-        const float res = __ll2float_rn(T) * esc;
-        stf(out, res);
-        out += 128;
-        left -= n; k = 0; item++;
+        sum = fmaf(__ll2float_rn(T), esc, sum);
+        left -= n; k += n;
+        if (k == nk || left == 0) {
+            stf(out, sum);
+            out += 128;
+            sum = 0.0f; k = 0; item++;
+        }
     }
 }
 // sum of an item's partials: columns c4 .. c4 + 3, by the four dg of a warp together; entry: first and last warp that hold some, and which of its pieces the first one's is
@@ -495,7 +507,8 @@ __device__ __noinline__ void weight_stream(const ZgClusterPlan* plan) {
         if (lane < kW && fills) settle(full + 8 * s, (fills - 1) & 1);
     }
 }
-// The list of a warp's copies in one layer: entry {8 * weight | bytes << 8, offset}; counts behind the lists.  By one lane per warp, before the start.
+// The list of a warp's copies in one layer: entry {8 * weight | bytes << 8, offset}; counts behind the lists.  And of its stretches: records and first of their ranges' lengths,
+// first column group and record.  By one lane per warp, before the start.
 template <int FMT>
 __device__ __noinline__ void copy_list(const ZgClusterPlan* plan, uint32_t w) {
     constexpr uint32_t RB = record_bytes(FMT), G = turn_records(FMT);
@@ -504,18 +517,29 @@ __device__ __noinline__ void copy_list(const ZgClusterPlan* plan, uint32_t w) {
     uint32_t* lists = reinterpret_cast<uint32_t*>(smem + P.o_list);
     const Share* shares = reinterpret_cast<const Share*>(smem + P.o_table);
     const uint32_t* items = reinterpret_cast<const uint32_t*>(shares + 4);
-    uint32_t n = 0;
+    const uint32_t* ranges = reinterpret_cast<const uint32_t*>(smem + P.o_ranges);
+    uint8_t* lens = smem + P.o_lens;
+    uint32_t n = 0, n_ranges = 0;
 #pragma unroll 1
     for (uint32_t ph = 0; ph < 4; ph++) {
         const Share s = shares[ph];
         const uint32_t R = s.own * s.nk, end = ((w + 1) * R) / kW;
         uint32_t pos = (w * R) / kW, item = s.nk ? pos / s.nk : 0, k = pos - item * s.nk;
         const uint32_t stretches = P.o_table + 4 * sizeof(Share) + 8 * kMaxItems * 4 + (ph * kW + w) * 8;
-        reinterpret_cast<uint32_t*>(smem + stretches)[0] = end - pos;
+        reinterpret_cast<uint32_t*>(smem + stretches)[0] = (end - pos) | (n_ranges << 16);
         reinterpret_cast<uint32_t*>(smem + stretches)[1] = item | (k << 16);
+        uint32_t range = 0;      // left of the records that share a scale
 #pragma unroll 1
         while (pos < end) {
-            const uint32_t it = items[ph * kMaxItems + item], m = min(G, min(s.nk - k, end - pos));
+            if (!range) {
+                const uint32_t at = s.k0 + k;
+                uint32_t word = at >> 5, ends = ranges[ph * P.range_words + word] & (~0u << (at & 31));
+                while (!ends) ends = ranges[ph * P.range_words + ++word];
+                range = min(word * 32 + __ffs(ends) - at, min(s.nk - k, end - pos));
+                lens[w * P.list_max + n_ranges++] = (uint8_t)range;
+            }
+            const uint32_t it = items[ph * kMaxItems + item], m = min(G, range);
+            range -= m;
             lists[(w * P.list_max + n) * 2] = (it & 255u) * 8 | (m * RB) << 8;
             lists[(w * P.list_max + n) * 2 + 1] = ((it >> 8) * s.stride + s.k0 + k) * RB;
             n++; pos += m; k += m;
@@ -743,7 +767,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
             }
             const uint32_t part = c.base + P.o_part + (ph & 1) * kW * P.seg * 128, tab = table + ph * 4 * kMaxItems;
             const uint32_t mine = stretches + (ph * kW + warp) * 8;
-            matvec<FMT>(c, P, make_uint2(lds32(mine), lds32(mine + 4)), nk, x, gamma, inv, top, smax + ph * 4 * kMaxItems, part, slot, parity);
+            matvec<FMT>(c, P, make_uint2(lds32(mine), lds32(mine + 4)), nk, c.base + P.o_lens + warp * P.list_max, x, gamma, inv, top, smax + ph * 4 * kMaxItems, part, slot, parity);
             workers_sync();
             if ((ph & 1) == 0) {
                 if (ph == 0) {
@@ -887,6 +911,19 @@ k_decode_cluster(const __grid_constant__ ZgClusterPlan plan) {
         items[i] = it < s.own ? item_of(P, c.rank, ph, it) : 0;
         items[4 * kMaxItems + i] = e;
     }
+    // where the ranges of a scale end, a bit per record of K
+    uint32_t* ranges = reinterpret_cast<uint32_t*>(smem + P.o_ranges);
+#pragma unroll 1
+    for (uint32_t i = c.tid; i < 4 * P.range_words; i += kThreads) ranges[i] = 0;
+    __syncthreads();
+    if (c.tid < 4 * kZgClusterRanges) {
+        const uint32_t ph = c.tid / kZgClusterRanges, w = c.tid % kZgClusterRanges, n = (ph == 1 ? P.Dq : ph == 3 ? P.F : P.D) >> 5, S = P.splits_k[ph];
+#pragma unroll 1
+        for (uint32_t s = 0; s < S; s++) {
+            const uint32_t ks = s * n / S, end = ks + (w + 1) * ((s + 1) * n / S - ks) / kZgClusterRanges;
+            if (end) atomicOr(ranges + ph * P.range_words + ((end - 1) >> 5), 1u << ((end - 1) & 31));
+        }
+    }
     __syncthreads();
     if (c.tid < kW) copy_list<FMT>(copy, c.tid);
     __syncthreads();
@@ -998,12 +1035,20 @@ bool zg_decode_cluster_layout(ZgClusterPlan& P, int fmt) {
     put(P.o_planes, kW * kPlaneBytes);
     put(P.o_ptrs, P.n_layers * 56);
     put(P.o_table, 4 * sizeof(Share) + 8 * kMaxItems * 4 + 4 * kW * 8);
-    // copies of a warp in one layer: a stretch of n records that starts anywhere takes at most n / G + 1 for each column group that it touches
+    // Copies of a warp in one layer: one for every G records and one more for each range; of n records n / (the shortest range) ranges, and two more for each column group.
     P.slot_bytes = turn_records(fmt) * record_bytes(fmt);
-    P.list_max = 0;
-    for (int ph = 0; ph < 4; ph++) P.list_max += up(own[ph] * nk[ph], kW) / turn_records(fmt) + P.seg;
+    P.list_max = P.range_words = 0;
+    const uint32_t stride[4] = {nD, nQ, nD, nF};
+    for (int ph = 0; ph < 4; ph++) {
+        const uint32_t n = up(own[ph] * nk[ph], kW);
+        if (stride[ph] > 255 * kZgClusterRanges || n > 0xffffu) return false;
+        P.list_max += n / turn_records(fmt) + n / std::max(1u, stride[ph] / P.splits_k[ph] / kZgClusterRanges) + 2 * P.seg;
+        P.range_words = std::max(P.range_words, (stride[ph] + 31) / 32);
+    }
+    put(P.o_ranges, 4 * P.range_words * 4);
+    put(P.o_lens, kW * P.list_max);
     put(P.o_list, kW * (P.list_max * 8 + 4));
-        put(P.o_bars, (kBarFull + 2 * kW * 8) * 8);
+    put(P.o_bars, (kBarFull + 2 * kW * 8) * 8);
     // what is left: the keys' and values' stages, then as deep a ring as fits
     const uint32_t stage = kv_stage_bytes(P.dh);
     for (P.kv_stages = 4; P.kv_stages >= 2; P.kv_stages /= 2) {

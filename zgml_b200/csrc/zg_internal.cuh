@@ -355,6 +355,7 @@ struct ZgDecodeHost {       // owned by a compiled program
 // ── decode_cluster.cu : the same layers on one cluster, for models whose layers are a few MB (one rank) ──
 constexpr uint32_t kZgClusterCtas = 16;
 constexpr uint32_t kZgClusterSmem = 227 * 1024;
+constexpr uint32_t kZgClusterRanges = 8;      // ranges of a split of K: the warps of a CTA in the general schedule's matvecs
 constexpr uint32_t kZgClusterItems = 64;      // column groups of a CTA in one phase
 struct ZgClusterHead { float* q_rot; float* attn_out; uint32_t dyn, _pad; };
 struct ZgClusterKv { float* k_rot; uint32_t k_off, v_off, k_dyn, v_dyn; };
@@ -375,8 +376,9 @@ static_assert(sizeof(ZgClusterLayer) % 8 == 0, "the heads hold pointers");
 struct ZgClusterPlan {      // passed to the kernel by value
     const uint8_t* blocks; const float* smax; const uint32_t* dyn; uint32_t* err;      // smax: [layer][CTA][phase][kZgClusterItems] scale ceilings
     uint32_t blk_bytes, n_layers, D, Dq, Dkv, F, n_heads, n_kv, dh, dh_log2, gs, splits;
+    uint32_t splits_k[4];      // of the K of a phase's products in the general schedule, whose ranges a scale may span (zg_qgemv_plan)
     uint32_t ring_slots, kv_stages, seg, own_max, hid_max, const_bytes, slot_bytes, smem_bytes;      // zg_decode_cluster_layout
-    uint32_t o_const, o_a1, o_a2, o_q, o_t, o_r, o_part, o_state, o_sq, o_ao, o_hid, o_planes, o_ptrs, o_table, o_list, list_max, o_bars, o_kv, o_ring;
+    uint32_t o_const, o_a1, o_a2, o_q, o_t, o_r, o_part, o_state, o_sq, o_ao, o_hid, o_planes, o_ptrs, o_table, o_ranges, o_lens, o_list, list_max, range_words, o_bars, o_kv, o_ring;
 };
 struct ZgClusterHost {      // owned by a compiled program
     ZgClusterPlan plan = {};
