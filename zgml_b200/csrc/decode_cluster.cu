@@ -727,7 +727,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
 #pragma unroll 1
                 for (uint32_t kg0 = warp; kg0 < nQ; kg0 += 2 * kW) {      // two groups of 32 side by side
                     uint32_t rec[2], d[2];
-                    float w[2], v[2];
+                    float w[2], v[2], inv_den[2];
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         const uint32_t kg = min(kg0 + u * kW, nQ - 1), h = (kg * 32) >> P.dh_log2;
@@ -742,7 +742,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
                         float den = in ? w[u] * got.x : 0.0f;
 #pragma unroll
                         for (int o = 1; o < 16; o <<= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-                        w[u] = den > 0.0f ? __fdividef(w[u], den) : 0.0f;
+                        inv_den[u] = den > 0.0f ? 1.0f / den : 0.0f;
                     }
 #pragma unroll 1
                     for (uint32_t sp = 0; sp < P.splits; sp++)
@@ -751,6 +751,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         const uint32_t kg = kg0 + u * kW;
+                        v[u] *= inv_den[u];
                         if (kg < nQ) {
                             stf(ao + (kg * 32 + lane) * 4, v[u]);
                             const float mx = warp_max(abs_or_inf(v[u]));
