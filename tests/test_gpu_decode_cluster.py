@@ -78,7 +78,7 @@ def test_not_finite_input_comes_out_as_the_oracle_has_it(cuda_backend):
         ref.close()
 
 
-@pytest.mark.parametrize("heads,kv,ff,kind", [(9, 3, 1536, "q8_0"), (9, 3, 1536, "q4_0"), (12, 4, 2048, "q8_0"), (6, 2, 1024, "q8_0"), (6, 2, 1024, "q4_0")])
+@pytest.mark.parametrize("heads,kv,ff,kind", [(9, 3, 1536, "q8_0"), (9, 3, 1536, "q4_0"), (12, 4, 1024, "q8_0"), (6, 2, 1024, "q8_0"), (6, 2, 1024, "q4_0")])
 def test_no_coarser_beside_channels_that_stand_out(cuda_backend, general, heads, kv, ff, kind):
     """gate and up against 64 bits where one channel of the normed row is 30 000 times the others and its weights are zero: what is left is the grid that the others are cut
     on, 2^-24 of the largest value of their range.  The ranges are those of the general schedule, so the errors are alike over all places of the channel (a tenth for the other
@@ -129,6 +129,19 @@ def test_op_by_op_steps_report_no_wait(cuda_backend):
     finally:
         cuda_backend.set_profiling(False)
     assert "gave up" not in last_error()
+    dev.close()
+
+
+@pytest.mark.parametrize("dh,heads,kv,ff,seq,kind,taken", [
+    (64, 9, 3, 1536, 4096, "q8_0", True), (64, 8, 8, 1376, 512, "q8_0", True), (64, 2, 1, 352, 8192, "q8_0", True),
+    (64, 8, 8, 1376, 8192, "q8_0", False), (32, 16, 16, 1376, 2048, "q8_0", False), (64, 6, 6, 1024, 4096, "q8_0", False), (64, 12, 4, 1024, 8192, "q4_0", False),       # the cache's share of a CTA
+    (64, 2, 1, 352, 8193, "q8_0", False),                                                                                          # beyond what the rule was measured for
+    (64, 12, 4, 2048, 64, "q8_0", False), (64, 12, 3, 2496, 64, "q4_0", False)])                                                   # the weights of a CTA
+def test_what_the_form_is_taken_for(cuda_backend, dh, heads, kv, ff, seq, kind, taken):
+    """Weights and, up to the last position of the cache, keys and values that 16 SMs stream as fast as the general schedule takes."""
+    cfg = LlamaConfig(vocab_size=8, d_model=dh * heads, n_layers=1, n_heads=heads, n_kv_heads=kv, d_ff=ff, max_seq_len=seq)
+    dev = DeviceLlamaSession(cuda_backend, cfg, synthetic_weights(cfg, kind, seed=1), 1)
+    assert cuda_backend.program_stats(dev.handle)["fused_decode_layers"] == int(taken)
     dev.close()
 
 

@@ -1186,12 +1186,21 @@ static bool build_decode_plan(ZgCudaProgram* p, std::vector<DecHostLayer>& layer
     return true;
 }
 
-// The cluster form of the fused layers (decode_cluster.cu).  False: not these layers.
-//
-// Up to kZgClusterLayerBytes of weights a layer: its 16 SMs stream about 1 TB/s and a layer takes some 18 us at least, the general schedule (seven launches a layer, all
-// SMs) some 31.  Whole steps, general / cluster: 8 layers of width 128 (Q8_0) 228 / 181 us, 10 of 384 (F 1024) 327 / 236, 30 of 576 (3.8 MB) 973 / 748, 12 of 768 (6.7 MB)
-// 429 / 393; 8 of 1024 in Q4_0: 7.2 MB 332 / 316, 9.1 MB 333 / 339; in Q8_0: 13 MB 333 / 383, 16 MB 333 / 437.
-constexpr size_t kZgClusterLayerBytes = 7u << 20;
+// Whether the layers take the cluster form (decode_cluster.cu): whether no step is slower there, up to the last position of the cache.  Its 16 SMs stream weights, keys and
+// values alone, where the general schedule (seven launches a layer) has all SMs.  What is compared, in ns a layer:
+//   - an early step takes 14.5 us here and 48 ns for every turn (zg_decode_cluster_turns), 18 us in Q4_0; in the general schedule 24 - 25 us;
+//   - the general schedule's steps get longer with the positions, by 3.1 us up to 512 and by at least 1.9 us for every 1024 more (1.2 at heads of 32);
+//   - here a CTA takes 15 ns a position of its share of a KV head's (of some 16 / KV heads), 25 where there is room for two stages of keys only or heads are 128 wide.
+// Steps of 8 layers, general / cluster, us: 9 heads on 3 of 64, F 1536 (Q8_0) at 64 193 / 168, 2048 258 / 218, 8192 377 / 379; 8 heads of 64, F 1376 at 64 186 / 149, 2048
+// 254 / 257, 8192 372 / 641; 12 heads on 4, F 2048 at 64 202 / 216.  Of 90 shapes that it takes, with the largest caches that it takes them with, none was slower at any
+// of five positions (at most 0.96 of the time of the general schedule; 30 more with scales of 32 bits 0.99).
+static bool cluster_pays(const ZgClusterPlan& P, int fmt, size_t positions) {
+    const double early = 45.0 * ((fmt == ZG_QFMT_I4_F16 ? 150.0 : 200.0) - zg_decode_cluster_turns(P, fmt));      // ns by which an early step is shorter here, at least
+    if (early < 0.0 || positions > kZgClusterPositions) return false;
+    const double longer = (double)positions / P.splits * (P.kv_stages == 2 || P.dh == 128 ? 25.0 : 15.0);
+    return longer <= early + 3100.0 + (P.dh == 32 ? 1.2 : 1.9) * std::max(0.0, (double)positions - 512.0);
+}
+// False: not these layers.
 static bool build_cluster_plan(ZgCudaProgram* p, const std::vector<DecHostLayer>& layers) {
     ZgClusterHost& h = p->cl;
     zg_decode_cluster_free(&h);
@@ -1255,12 +1264,7 @@ static bool build_cluster_plan(ZgCudaProgram* p, const std::vector<DecHostLayer>
         const auto at = std::lower_bound(writes.begin(), writes.end(), x.b, [](const Span& y, const float* end) { return y.a < end; });
         if (at != writes.begin() && (at - 1)->b > x.a) return false;      // spans that overlap are equal: the last one before the end reaches furthest
     }
-    size_t bytes = 0;
     const ZgDecPhase* ph0 = layers[0].ph;
-    for (int ph = 0; ph < 4; ph++)
-        for (uint32_t m = 0; m < ph0[ph].n_mv; m++) bytes += (size_t)ph0[ph].mv[m].n_nb * ph0[ph].n_kc * ph0[ph].rec_bytes;
-    if (bytes > kZgClusterLayerBytes) return false;
-
     ZgClusterPlan& P = h.plan;
     P.n_layers = (uint32_t)layers.size(); P.D = D; P.Dq = H * dh; P.Dkv = G * dh; P.F = F; P.n_heads = H; P.n_kv = G; P.dh = dh;
     P.blk_bytes = (uint32_t)((sizeof(ZgClusterLayer) + H * sizeof(ZgClusterHead) + G * sizeof(ZgClusterKv) + 15) & ~(size_t)15);
@@ -1273,7 +1277,7 @@ static bool build_cluster_plan(ZgCudaProgram* p, const std::vector<DecHostLayer>
         if (pl.threads != 32 * kZgClusterRanges) return false;
         P.splits_k[ph] = pl.S;
     }
-    if (!zg_decode_cluster_layout(P, h.fmt)) return false;
+    if (!zg_decode_cluster_layout(P, h.fmt) || !cluster_pays(P, h.fmt, room(layers[0].ly.k_cache) / (G * dh))) return false;
     std::vector<uint8_t> blocks((size_t)P.n_layers * P.blk_bytes, 0);
     for (size_t l = 0; l < layers.size(); l++) {
         const DecHostLayer& L = layers[l];

@@ -196,6 +196,11 @@ __host__ __device__ inline Share share_of(const ZgClusterPlan& P, uint32_t rank,
     else { s.own = hi > lo ? nD : 0; s.nk = hi - lo; s.k0 = lo; s.stride = nF; }
     return s;
 }
+// where range i of the n records of K ends: those of the warps of the general schedule's matvecs, in each of S splits
+__host__ __device__ inline uint32_t range_end(uint32_t n, uint32_t S, uint32_t i) {
+    const uint32_t s = i / kZgClusterRanges, ks = s * n / S;
+    return ks + (i % kZgClusterRanges + 1) * ((s + 1) * n / S - ks) / kZgClusterRanges;
+}
 // item i of the phase: its weight, and from bit 8 on its column group there
 __host__ __device__ inline uint32_t item_of(const ZgClusterPlan& P, uint32_t rank, uint32_t ph, uint32_t i) {
     if (ph == 0) {
@@ -921,7 +926,7 @@ k_decode_cluster(const __grid_constant__ ZgClusterPlan plan) {
         const uint32_t ph = c.tid / kZgClusterRanges, w = c.tid % kZgClusterRanges, n = (ph == 1 ? P.Dq : ph == 3 ? P.F : P.D) >> 5, S = P.splits_k[ph];
 #pragma unroll 1
         for (uint32_t s = 0; s < S; s++) {
-            const uint32_t ks = s * n / S, end = ks + (w + 1) * ((s + 1) * n / S - ks) / kZgClusterRanges;
+            const uint32_t end = range_end(n, S, s * kZgClusterRanges + w);
             if (end) atomicOr(ranges + ph * P.range_words + ((end - 1) >> 5), 1u << ((end - 1) & 31));
         }
     }
@@ -1067,6 +1072,26 @@ bool zg_decode_cluster_layout(ZgClusterPlan& P, int fmt) {
         }
     }
     return false;
+}
+
+uint32_t zg_decode_cluster_turns(const ZgClusterPlan& P, int fmt) {
+    const uint32_t n[4] = {P.D / 32, P.Dq / 32, P.D / 32, P.F / 32}, G = turn_records(fmt);
+    uint32_t most = 0;
+    for (uint32_t r = 0; r < kC; r++) {
+        uint32_t turns = 0;
+        for (uint32_t ph = 0; ph < 4; ph++) {
+            const Share s = share_of(P, r, ph);
+            uint32_t at = 0, of_group = 0;      // ranges' ends, and the turns of what lies in this CTA's part of a column group
+            for (uint32_t i = 1; i <= P.splits_k[ph] * kZgClusterRanges; i++) {
+                const uint32_t end = range_end(n[ph], P.splits_k[ph], i - 1), lo = std::max(at, s.k0), hi = std::min(end, s.k0 + s.nk);
+                if (hi > lo) of_group += (hi - lo + G - 1) / G;
+                at = end;
+            }
+            turns += s.own * of_group;
+        }
+        most = std::max(most, turns);
+    }
+    return most;
 }
 
 // Which weight (0 .. 6) and column group the items of the CTAs are, [rank][phase][kZgClusterItems], -1: none.

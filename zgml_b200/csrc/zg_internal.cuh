@@ -356,6 +356,7 @@ struct ZgDecodeHost {       // owned by a compiled program
 constexpr uint32_t kZgClusterCtas = 16;
 constexpr uint32_t kZgClusterSmem = 227 * 1024;
 constexpr uint32_t kZgClusterRanges = 8;      // ranges of a split of K: the warps of a CTA in the general schedule's matvecs
+constexpr uint32_t kZgClusterPositions = 8192;      // of the cache, at most (cluster_pays)
 constexpr uint32_t kZgClusterItems = 64;      // column groups of a CTA in one phase
 struct ZgClusterHead { float* q_rot; float* attn_out; uint32_t dyn, _pad; };
 struct ZgClusterKv { float* k_rot; uint32_t k_off, v_off, k_dyn, v_dyn; };
@@ -387,6 +388,7 @@ struct ZgClusterHost {      // owned by a compiled program
     bool valid = false;
 };
 bool zg_decode_cluster_layout(ZgClusterPlan& P, int fmt);
+uint32_t zg_decode_cluster_turns(const ZgClusterPlan& P, int fmt);      // of the warps of the CTA that has most of a layer, a ring slot of weights each
 void zg_decode_cluster_items(const ZgClusterPlan& P, int* weight, uint32_t* group);
 bool zg_decode_cluster_launch(const ZgClusterHost& h, cudaStream_t st);
 void zg_decode_cluster_free(ZgClusterHost* h);
