@@ -148,3 +148,35 @@ def test_scheduling_knobs_do_not_change_results(knobs):
         dev.close(); ref.close()
     finally:
         be.close()
+
+
+@pytest.mark.parametrize("form", ["pair", "prologue", "two rows", "cluster"])
+@pytest.mark.parametrize("op", ["gelu", "abs", "relu", "sqrt", "exp", "log", "recip", "neg", "sgn", "step"])
+def test_every_unary_activation(monkeypatch, form, op):
+    """The activation of a gated feed-forward, wherever the schedule evaluates it: with the gate | up products, before the down product (one row and two), in the cluster form.
+    (log, sqrt and recip of the magnitude.)"""
+    from llama_reference import OracleBackend
+    from zgml_b200 import CudaBackend, DeviceOp, abi
+    from zgml_b200.host import llama
+    cfg = LlamaConfig(vocab_size=64, d_model=128, n_layers=1, n_heads=2, n_kv_heads=1, d_ff=160, max_seq_len=8)
+    w = synthetic_weights(cfg, "q8_0", seed=2, embed_scale=1.0)
+    plain, T = llama.build_program, 2 if form == "two rows" else 1
+
+    def build(cfg, w, token_len=1):
+        lp = plain(cfg, w, token_len)
+        for i, o in enumerate(lp.program.ops):
+            if o.tag == abi.OP_FUSED_ELEMENTWISE:
+                f = o.u.fused_elementwise
+                steps = [("abs", 0, 0, 0), (op, 0, 0, 0)] if op in ("sqrt", "log", "recip") else [(op, 0, 0, 0)]
+                lp.program.ops[i] = DeviceOp.fused_elementwise(steps, f.n, f.dst, f.src)
+        return lp
+    monkeypatch.setattr(llama, "build_program", build)
+    if form != "cluster":
+        monkeypatch.setenv("ZG_CUDA_DECODE_CLUSTER", "0")
+    if form == "prologue":
+        monkeypatch.setenv("ZG_CUDA_GEMV_PAIR", "0")
+    dev, ref = DeviceLlamaSession(CudaBackend(0), cfg, w, T), DeviceLlamaSession(OracleBackend(), cfg, w, T)
+    a, b = (s.execute_at([3, 4][:T], 0).copy() for s in (dev, ref))
+    assert np.max(np.abs(a - b)) <= 1e-4 * np.max(np.abs(b))
+    dev.close()
+    ref.close()

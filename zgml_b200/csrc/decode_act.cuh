@@ -4,19 +4,6 @@
 
 namespace {
 
-__device__ __noinline__ float apply_unary(uint32_t op, float v) {
-    switch (op) {
-        case ZG_EW_NEG: return -v;
-        case ZG_EW_ABS: return fabsf(v);
-        case ZG_EW_RELU: return fmaxf(v, 0.0f);
-        case ZG_EW_SQRT: return sqrtf(v);
-        case ZG_EW_RECIP: return 1.0f / v;
-        case ZG_EW_EXP: return expf(v);
-        case ZG_EW_LOG: return logf(v);
-        case ZG_EW_GELU: { const float kk = 0.7978845608f * (v + 0.044715f * v * v * v); return 0.5f * v * (1.0f + tanhf(kk)); }
-        default: return v;
-    }
-}
 // the general activation chain of one element (fused_elementwise steps, src/backend/reference.zig:262-300); out of line
 __device__ __noinline__ float act_chain(const ZgDecStep* steps, uint32_t n_steps, float gt, float up, float sec0, int first_ext, uint32_t k) {
     float v = gt;

@@ -59,25 +59,6 @@ __device__ float block_reduce(float v, float* sh) {
     return r;
 }
 
-__device__ __forceinline__ float gelu_tanh(float a) { // reference.zig:265-269
-    float kk = 0.7978845608f * (a + 0.044715f * a * a * a);
-    return 0.5f * a * (1.0f + tanhf(kk));
-}
-
-__device__ __forceinline__ float apply_unary(uint32_t op, float v) {
-    switch (op) {
-        case ZG_EW_NEG: return -v;
-        case ZG_EW_ABS: return fabsf(v);
-        case ZG_EW_RELU: return fmaxf(v, 0.0f);
-        case ZG_EW_SQRT: return sqrtf(v);
-        case ZG_EW_RECIP: return 1.0f / v;
-        case ZG_EW_EXP: return expf(v);
-        case ZG_EW_LOG: return logf(v);
-        case ZG_EW_GELU: return gelu_tanh(v);
-        default: return v; // sgn/step/others: reference copies src0 / leaves v unchanged
-    }
-}
-
 __global__ void k_elementwise(uint32_t op, float* __restrict__ dst, const float* __restrict__ s0,
                               const float* __restrict__ s1, uint32_t n) {
     ZG_TRACE_BEGIN(1)

@@ -277,13 +277,7 @@ qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
                 const uint32_t sop = p.pro.steps[st].op, sw = p.pro.steps[st].is_swapped;
                 if (sop == ZG_EW_ADD) { const float t2 = p.pro.steps[st].sec[f]; v = sw ? __fadd_rn(t2, v) : __fadd_rn(v, t2); }
                 else if (sop == ZG_EW_MUL) { const float t2 = p.pro.steps[st].sec[f]; v = sw ? __fmul_rn(t2, v) : __fmul_rn(v, t2); }
-                else if (sop == ZG_EW_NEG) v = -v;
-                else if (sop == ZG_EW_EXP) v = expf(v);
-                else if (sop == ZG_EW_RECIP) v = 1.0f / v;
-                else if (sop == ZG_EW_ABS) v = fabsf(v);
-                else if (sop == ZG_EW_RELU) v = fmaxf(v, 0.0f);
-                else if (sop == ZG_EW_SQRT) v = sqrtf(v);
-                else if (sop == ZG_EW_LOG) v = logf(v);
+                else v = apply_unary(sop, v);
             }
             const float xv = __fmul_rn(v, p.pro.b[f]);
             if (pro_write) { p.pro.o_mid[f] = v; p.pro.o_x[f] = xv; }
@@ -552,18 +546,6 @@ qgemv_kernel(const __grid_constant__ QGemvBatchT<PRO != 0> bt) {
 struct QGemvPair { QGemvParams a, b; ZgGemvEpilogue epi; };
 struct QGemvPairBatch { QGemvPair p[2]; };
 
-__device__ __forceinline__ float epi_unary(uint32_t op, float v) {
-    switch (op) {
-        case ZG_EW_NEG: return -v;
-        case ZG_EW_ABS: return fabsf(v);
-        case ZG_EW_RELU: return fmaxf(v, 0.0f);
-        case ZG_EW_SQRT: return sqrtf(v);
-        case ZG_EW_RECIP: return 1.0f / v;
-        case ZG_EW_EXP: return expf(v);
-        case ZG_EW_LOG: return logf(v);
-        default: return v;
-    }
-}
 
 template <int FMT>
 __global__ void __launch_bounds__(kThreads, 3)
@@ -813,7 +795,7 @@ qgemv_pair_kernel(const __grid_constant__ QGemvPairBatch bt) {
                         const float o2 = kd == 1 ? gt : (kd == 2 ? up : pp.epi.steps[st].sec[n]);
                         if (sop == ZG_EW_ADD) v = sw ? __fadd_rn(o2, v) : __fadd_rn(v, o2);
                         else v = sw ? __fmul_rn(o2, v) : __fmul_rn(v, o2);
-                    } else v = epi_unary(sop, v);
+                    } else v = apply_unary(sop, v);
                 }
                 pp.epi.o_mid[n] = v;
                 pp.epi.o_dst[n] = __fmul_rn(v, up);

@@ -87,6 +87,21 @@ struct ZgCudaQWeight {
     size_t device_bytes = 0;
 };
 
+// One value through a unary elementwise op, wherever a chain of them is evaluated.  gelu: reference.zig:265-269; sgn, step and others: the reference copies src0 / leaves v unchanged.
+__device__ __forceinline__ float apply_unary(uint32_t op, float v) {
+    switch (op) {
+        case ZG_EW_NEG: return -v;
+        case ZG_EW_ABS: return fabsf(v);
+        case ZG_EW_RELU: return fmaxf(v, 0.0f);
+        case ZG_EW_SQRT: return sqrtf(v);
+        case ZG_EW_RECIP: return 1.0f / v;
+        case ZG_EW_EXP: return expf(v);
+        case ZG_EW_LOG: return logf(v);
+        case ZG_EW_GELU: { const float kk = 0.7978845608f * (v + 0.044715f * v * v * v); return 0.5f * v * (1.0f + tanhf(kk)); }
+        default: return v;
+    }
+}
+
 static inline uint32_t zg_rec_q_bytes(int fmt) { return fmt == ZG_QFMT_I4_F16 ? 512u : 1024u; }
 static inline uint32_t zg_rec_s_bytes(int fmt) { return fmt == ZG_QFMT_I8_F32 ? 128u : 64u; }
 
