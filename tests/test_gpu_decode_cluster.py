@@ -1,6 +1,6 @@
 """The layers of a small single-token LLaMA on one thread-block cluster (csrc/decode_cluster.cu) against the general schedule of the same program (which the other LLaMA
 tests hold against the oracle): every program buffer, at the edges of what the kernel splits — head widths, query heads per KV head, KV heads that do not divide the CTAs,
-column groups and feed-forward pairs that do not either, positions around a stage of keys and past all of them."""
+column groups and feed-forward pairs that do not either, positions around a stage of keys and past all of them, other activations; and what the form is taken for."""
 import os
 
 import numpy as np
@@ -27,7 +27,9 @@ def general():
 
 #          d_head, heads, kv, ff, max_seq
 SHAPES = [(32, 1, 1, 32, 40),          # one column group, one pair: most CTAs have nothing
-          (32, 3, 3, 96, 200), (32, 16, 16, 544, 330), (64, 4, 1, 256, 1100), (64, 9, 3, 1536, 700), (64, 10, 5, 800, 420), (128, 2, 2, 288, 600), (128, 2, 1, 640, 1100)]
+          (32, 3, 3, 96, 200), (32, 16, 16, 544, 330), (64, 4, 1, 256, 1100), (64, 9, 3, 1536, 700), (64, 10, 5, 800, 420), (128, 2, 2, 288, 600), (128, 2, 1, 640, 1100),
+          # with the eight above: every head width with every count of query heads per KV head that the kernel is compiled for
+          (32, 2, 1, 96, 300), (32, 6, 2, 160, 300), (32, 8, 2, 256, 300), (64, 3, 3, 224, 300)]
 
 
 @pytest.mark.parametrize("kind", ["q8_0", "q4_0", "i8_f32"])
@@ -57,6 +59,44 @@ def test_every_buffer_as_the_general_schedule_leaves_it(cuda_backend, general, d
             # a product of K terms on a grid of 2^-24 of its largest is off by some 2^-24 sqrt(K) = 1.4e-6 of its own size; seven in a row per layer, three layers, and scores
             # of up to 10 that a softmax turns into factors: 1e-4, which is what either schedule is held to against the oracle
             assert np.max(np.abs(g[fin] - v[fin]), initial=0.0) <= 1e-4 * np.max(np.abs(v[fin]), initial=0.0) + 1e-6, f"buffer {i} at position {pos}"
+    dev.close()
+    ref.close()
+
+
+@pytest.mark.parametrize("chain", ["gelu", "two constants", "gate and up"])
+def test_other_activations(cuda_backend, general, monkeypatch, chain):
+    """Chains other than SiLU run through the interpreter of steps: unary ops, constants (the first is read ahead, a second is not), gate and up as operands, either order."""
+    from zgml_b200 import DeviceOp, ProgramIO, abi
+    from zgml_b200.host import llama
+    cfg = LlamaConfig(vocab_size=64, d_model=192, n_layers=2, n_heads=3, n_kv_heads=1, d_ff=1120, max_seq_len=24)      # 35 pairs of column groups
+    w = synthetic_weights(cfg, "q8_0", seed=9, embed_scale=1.0)
+    plain = llama.build_program
+
+    def build(cfg, w, token_len=1):
+        lp = plain(cfg, w, token_len)
+        r, F = np.random.default_rng(4), cfg.d_ff
+        first, second = (len(lp.program.buffer_sizes) + i for i in range(2))
+        lp.program.buffer_sizes += [F + 8, F + 4]
+        lp.program.initial_uploads += [ProgramIO(first, r.standard_normal(F + 8).astype(np.float32)), ProgramIO(second, r.standard_normal(F + 4).astype(np.float32))]
+        for i, op in enumerate(lp.program.ops):
+            if op.tag != abi.OP_FUSED_ELEMENTWISE:
+                continue
+            gate, silu, up = op.u.fused_elementwise.src, op.u.fused_elementwise.dst, lp.program.ops[i + 1].u.elementwise.src1
+            steps = {"gelu": [("gelu", 0, 0, 0)], "two constants": [("abs", 0, 0, 0), ("mul", 1, first, 8), ("relu", 0, 0, 0), ("add", 0, second, 4), ("neg", 0, 0, 0)],
+                     "gate and up": [("add", 1, up, 0), ("mul", 0, gate, 0), ("abs", 0, 0, 0), ("sqrt", 0, 0, 0)]}[chain]
+            lp.program.ops[i] = DeviceOp.fused_elementwise(steps, F, silu, gate)
+        return lp
+    monkeypatch.setattr(llama, "build_program", build)
+    dev, ref = DeviceLlamaSession(cuda_backend, cfg, w, 1), DeviceLlamaSession(general, cfg, w, 1)
+    assert cuda_backend.program_stats(dev.handle)["fused_decode_layers"] == 2 and general.program_stats(ref.handle)["fused_decode_layers"] == 0
+    got, want = ([np.zeros(n, np.float32) for n in dev.lp.program.buffer_sizes] for _ in range(2))
+    dev.outputs, ref.outputs = ([ProgramIO(i, b) for i, b in enumerate(bufs)] for bufs in (got, want))
+    for pos in range(3):
+        dev.execute_at([pos + 1], pos)
+        ref.execute_at([pos + 1], pos)
+        for i, (g, v) in enumerate(zip(got, want)):
+            fin = np.isfinite(v)
+            assert np.array_equal(np.isfinite(g), fin) and np.max(np.abs(g[fin] - v[fin]), initial=0.0) <= 1e-4 * np.max(np.abs(v[fin]), initial=0.0) + 1e-6, f"buffer {i} at position {pos}"
     dev.close()
     ref.close()
 

@@ -43,7 +43,7 @@ __host__ __device__ constexpr uint32_t turn_records(int fmt) { return fmt == ZG_
 __host__ __device__ constexpr uint32_t record_bytes(int fmt) { return fmt == ZG_QFMT_I4_F16 ? 576u : fmt == ZG_QFMT_I8_F32 ? 1152u : 1088u; }
 constexpr uint32_t kPlaneRow = 144, kPlaneBytes = 4 * kPlaneRow;
 constexpr uint32_t kKvRows = 32;                      // positions of a stage of keys and values
-constexpr uint32_t kMaxGroup = 4;                     // query heads of a KV head
+__host__ __device__ constexpr uint32_t max_group(uint32_t dh) { return dh == 128 ? 2u : 4u; }      // query heads of a KV head (three of 128 leave no room for keys and weights)
 __host__ __device__ constexpr uint32_t kv_stage_bytes(uint32_t dh) { return (2 * kKvRows * dh + kKvRows) * 4; }      // keys, values, mask
 constexpr uint32_t kMaxItems = kZgClusterItems;                    // column groups of a CTA in one phase
 
@@ -635,8 +635,10 @@ __device__ __forceinline__ void attend(uint32_t gs, uint32_t kv, uint32_t bars, 
                                        float scale) {
     if (gs == 1) attention_share<NI, 1>(kv, bars, lg, sq, state, at, t_at, t_stride, base, scale);
     else if (gs == 2) attention_share<NI, 2>(kv, bars, lg, sq, state, at, t_at, t_stride, base, scale);
-    else if (gs == 3) attention_share<NI, 3>(kv, bars, lg, sq, state, at, t_at, t_stride, base, scale);
-    else attention_share<NI, 4>(kv, bars, lg, sq, state, at, t_at, t_stride, base, scale);
+    else if constexpr (max_group(32 * NI) > 2) {
+        if (gs == 3) attention_share<NI, 3>(kv, bars, lg, sq, state, at, t_at, t_stride, base, scale);
+        else attention_share<NI, 4>(kv, bars, lg, sq, state, at, t_at, t_stride, base, scale);
+    }
 }
 #define LY(field) (area + (uint32_t)offsetof(ZgClusterLayer, field))
 
@@ -1006,7 +1008,7 @@ unsigned int zg_decode_cluster_timeouts() {
 bool zg_decode_cluster_layout(ZgClusterPlan& P, int fmt) {
     const uint32_t nD = P.D / 32, nQ = P.Dq / 32, nK = P.Dkv / 32, nF = P.F / 32;
     if (P.D % 32 || P.Dq % 32 || P.Dkv % 32 || P.F % 32 || (P.dh != 32 && P.dh != 64 && P.dh != 128) || P.n_layers == 0 || P.n_layers > 128) return false;
-    if (P.n_kv == 0 || P.n_kv > kC || P.n_heads % P.n_kv || P.n_heads / P.n_kv > kMaxGroup || P.n_heads * P.dh != P.Dq || P.n_kv * P.dh != P.Dkv) return false;
+    if (P.n_kv == 0 || P.n_kv > kC || P.n_heads % P.n_kv || P.n_heads / P.n_kv > max_group(P.dh) || P.n_heads * P.dh != P.Dq || P.n_kv * P.dh != P.Dkv) return false;
     P.gs = P.n_heads / P.n_kv;
     P.dh_log2 = P.dh == 32 ? 5 : P.dh == 64 ? 6 : 7;
     P.splits = kC / P.n_kv;
