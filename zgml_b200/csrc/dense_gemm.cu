@@ -511,13 +511,13 @@ static bool expert_weights_map(CUtensorMap* map, const void* w, uint32_t E, uint
     return r == CUDA_SUCCESS;
 }
 // xb: bf16 rows [rows][K] sorted by expert; w, w2: [E][N][K] bfloat16 (w2 null: out = f32 [rows][N]; otherwise out = bf16 [rows][N] of gate and up).
-// d_segments: `segments` runs of rows on the device (ZgExpertSegment), those with rows first; full_runs: how many will have some at least where every expert has its share, likely_runs: with
-// half a run more per expert.
-// One matrix is taken 256 rows at a time where there are tiles of that size for three sevenths of the SMs: the runs' rows then cross the L2 half as often (1024 tokens, two of 16
-// experts, 2048 / 2048 120.3 -> 117.8 us, of 8 experts, 1024 / 1024 56.2 -> 54.4; but 20 tokens of 4 experts, 32 such tiles, 40.8 -> 43.7, 500 of 8, 800 / 800, 60 of
-// them, 34.8 -> 36.9).  More tiles than SMs are walked by one CTA per SM (k_expert_gemm); where there are fewer, the walk's preparations cost (1000 tokens, one of 8 experts,
-// 400 / 1800, 120 tiles: 47.2 us, walked 48.9).
-bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void* xb, uint32_t rows, const ZgExpertSegment* d_segments, uint32_t segments, uint32_t full_runs, uint32_t likely_runs, void* out, uint32_t N, uint32_t K,
+// d_segments: `segments` runs of rows on the device (ZgExpertSegment), those with rows first; likely_runs: how many will have some, with half a run more per expert than the rows fill.
+// One matrix is taken 256 rows at a time where tiles of 128 rows would be more than the SMs: half as many take one round instead of two, and the runs' rows cross the L2 half as often.
+// The op, tiles of 128 / of 256 rows: 64 tokens, two of 16 experts, ff 2048, 1024 columns (128 tiles of 128 rows) 54.9 / 55.8 us, 1280 (160) 68.7 / 63.7, 2048 87.1 / 86.4; 100
+// tokens, one of 12, ff 1536, 1536 columns (144) 49.3 / 49.4, 1792 (168) 57.4 / 53.5; 1024 tokens, two of 8, ff 2048, 1024 columns (96) 91.9 / 97.6, 1792 (168) 124.3 / 118.2.  At
+// several rounds either way the two differ by -3 to 7 %.  More tiles than SMs are walked by one CTA per SM (k_expert_gemm); where there are fewer, the walk's preparations
+// cost (1000 tokens, one of 8 experts, 400 / 1800, 120 tiles: 47.2 us, walked 48.9).
+bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void* xb, uint32_t rows, const ZgExpertSegment* d_segments, uint32_t segments, uint32_t likely_runs, void* out, uint32_t N, uint32_t K,
                            float limit, float alpha, float up_offset, cudaStream_t st) {
     if (!prepare()) return false;
     CUtensorMap map_x, map_w, map_w2;
@@ -528,7 +528,7 @@ bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void
     if (r != CUDA_SUCCESS) { zg_set_error("cuTensorMapEncodeTiled(expert rows) failed (%d)", (int)r); return false; }
     if (!expert_weights_map(&map_w, w, E, N, K) || !expert_weights_map(&map_w2, w2 ? w2 : w, E, N, K)) return false;
     const ExpertParams p = {out, d_segments, N, K, segments, limit, alpha, up_offset};
-    const int mode = w2 ? kExpertDual : 7 * ((N + 2 * BM - 1) / (2 * BM)) * full_runs >= 3 * zg_sm_count() ? kExpertWide : kExpertOne;
+    const int mode = w2 ? kExpertDual : (N + BM - 1) / BM * likely_runs > zg_sm_count() ? kExpertWide : kExpertOne;
     const uint32_t n_f = (N + (mode == kExpertWide ? 2 : 1) * BM - 1) / ((mode == kExpertWide ? 2 : 1) * BM);
     const bool loop = n_f * likely_runs > zg_sm_count();
     launch_pdl(g_expert[mode][loop], loop ? dim3(zg_sm_count()) : dim3(n_f, segments), dim3(kExpertThreads), kExpertSmem, st, map_x, map_w, map_w2, p);

@@ -2809,7 +2809,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             if (moe_grouped(s, bufs)) {
                 const MoeLayout L = moe_layout(T, D, ff, E, top);
                 float* sc = bufs[s.buf[4]];
-                const uint32_t run = moe_run(L, ff, zg_sm_count()), segments = L.experts + L.R / run, full_runs = std::max(L.experts, L.R / run), likely = std::max(full_runs, L.R / run + L.experts / 2);
+                const uint32_t run = moe_run(L, ff, zg_sm_count()), segments = L.experts + L.R / run, likely = std::max(L.experts, L.R / run + L.experts / 2);
                 ZgExpertSegment* seg = reinterpret_cast<ZgExpertSegment*>(sc + L.seg);
                 int* row_pair = reinterpret_cast<int*>(sc + L.row_pair);
                 int* pos_of_pair = reinterpret_cast<int*>(sc + L.pos_of_pair);
@@ -2817,8 +2817,8 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                 ZG_SEQ_CHECK();
                 launch_pdl(k_moe_gather, dim3(L.R), dim3(256), 0, st, reinterpret_cast<uint32_t*>(sc + L.xs), bufs[s.buf[1]], row_pair, D, top);
                 ZG_SEQ_CHECK();
-                if (!zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[0]), wptr<bf16>(bufs, s.buf[3], s.off[1]), E, sc + L.xs, L.R, seg, segments, full_runs, likely, sc + L.yb, ff, D, s.f[0], s.f[1], s.f[2], st) ||
-                    !zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[2]), nullptr, E, sc + L.yb, L.R, seg, segments, full_runs, likely, sc + L.z, D, ff, 0.0f, 0.0f, 0.0f, st)) return false;
+                if (!zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[0]), wptr<bf16>(bufs, s.buf[3], s.off[1]), E, sc + L.xs, L.R, seg, segments, likely, sc + L.yb, ff, D, s.f[0], s.f[1], s.f[2], st) ||
+                    !zg_expert_gemm_launch(wptr<bf16>(bufs, s.buf[3], s.off[2]), nullptr, E, sc + L.yb, L.R, seg, segments, likely, sc + L.z, D, ff, 0.0f, 0.0f, 0.0f, st)) return false;
                 launch_pdl(k_moe_combine, dim3(T), dim3(256), 0, st, bufs[s.buf[0]], bufs[s.buf[1]], sc + L.z, bufs[s.buf[2]], pos_of_pair, D, top);
                 ZG_SEQ_CHECK();
                 return true;

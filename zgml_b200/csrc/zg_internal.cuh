@@ -468,7 +468,7 @@ size_t zg_dense_gemm_scratch_elems(uint32_t M, uint32_t K);
 unsigned int zg_dense_gemm_timeouts();
 struct ZgExpertSegment { int expert, start, rows; };          // rows start .. start + rows - 1 (at most kExpertSegmentRows) belong to the expert; rows 0: unused
 constexpr uint32_t kExpertSegmentRows = 256;
-bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void* xb, uint32_t rows, const ZgExpertSegment* d_segments, uint32_t segments, uint32_t full_runs, uint32_t likely_runs, void* out, uint32_t N, uint32_t K,
+bool zg_expert_gemm_launch(const void* w, const void* w2, uint32_t E, const void* xb, uint32_t rows, const ZgExpertSegment* d_segments, uint32_t segments, uint32_t likely_runs, void* out, uint32_t N, uint32_t K,
                            float limit, float alpha, float up_offset, cudaStream_t st);
 // split_gemm.cu : f32 x f32 -> f32 LINEAR of many rows, operands cut into three bfloat16 parts (arguments as zg_dense_gemm_launch's; N counts weight rows)
 bool zg_split_gemm_usable(const float* w, const float* src, uint32_t M, uint32_t N, uint32_t K, uint32_t src_rs, uint32_t slot_stride);
