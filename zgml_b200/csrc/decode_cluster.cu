@@ -27,7 +27,8 @@
 // and phase 5 of layer l + 1 follows the arrival of all of that x.
 //
 // Every DeviceOp's buffer is written (the owners and producers store what they hold).  Every wait is bounded: a CTA that gives up
-// counts it, marks the launch, and no longer waits; the last layer's outputs then come out as NaN.
+// counts it, marks the launch, no longer waits and stops before a layer whose operands (addresses among them) have not come; the last
+// layer's outputs then come out as NaN.
 #include "zg_internal.cuh"
 #include "decode_act.cuh"
 
@@ -135,6 +136,7 @@ __device__ __forceinline__ T* ldp(uint32_t addr) {
 }
 __device__ __forceinline__ void stf(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 __device__ __forceinline__ void stf4(uint32_t addr, float4 v) { asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory"); }
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts8(uint32_t addr, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 __device__ __forceinline__ void stg4(float* p, float4 v) { asm volatile("st.global.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory"); }
 __device__ __forceinline__ float warp_sum(float v) {
@@ -157,19 +159,20 @@ struct Cta {
 };
 __device__ __forceinline__ uint32_t bar_of(const Cta& c, uint32_t i) { return c.bars + 8 * i; }
 // A poll holds the warp for up to 4 us.  Who has polled for some two seconds marks the CTA, and nobody in it waits any more.
-constexpr uint32_t kDead = 248, kPolls = 1u << 19;      // where the mark lies in shared memory
+constexpr uint32_t kDead = 248, kNoOperands = 252, kPolls = 1u << 19;      // where the mark lies in shared memory, and that of a layer whose operands have not come
 __device__ __forceinline__ uint32_t smem_base() {
     extern __shared__ __align__(128) uint8_t smem[];
     return smem_u32(smem);
 }
 __device__ __forceinline__ bool dead() { return lds32(smem_base() + kDead) != 0; }
-__device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity) {      // false: it is not there
     uint32_t polls = 0;
 #pragma unroll 1
     while (!mbar_try(bar, parity)) {
-        if (++polls == kPolls) asm volatile("st.shared.u32 [%0], %1;" ::"r"(smem_base() + kDead), "r"(1u) : "memory");
-        if (dead()) break;
+        if (++polls == kPolls) sts32(smem_base() + kDead, 1u);
+        if (dead()) return false;
     }
+    return true;
 }
 
 // What a warp's bulk copies have still to bring lands before the warp ends, whatever made it end: their CTA's shared memory must not go before (some 60 ms at most).
@@ -564,7 +567,7 @@ __device__ __noinline__ void kv_stream(const ZgClusterPlan* plan, uint32_t rank)
 #pragma unroll 1
     for (uint32_t l = 0; l < P.n_layers; l++) {
         const uint32_t area = base + P.o_const + (l & 1) * P.const_bytes, kv = area + (uint32_t)sizeof(ZgClusterLayer) + P.n_heads * (uint32_t)sizeof(ZgClusterHead) + g * (uint32_t)sizeof(ZgClusterKv);
-        wait_bar(bars + 8 * (kBarConstFull + (l & 1)), (l >> 1) & 1);
+        if (!__all_sync(0xffffffffu, wait_bar(bars + 8 * (kBarConstFull + (l & 1)), (l >> 1) & 1))) break;      // (what would be read there are addresses)
         const uint32_t at = area + P.const_bytes - 48, lo = lds32(at + 24), len = lds32(at + 28), mask_rs = lds32(area + (uint32_t)offsetof(ZgClusterLayer, mask_rs));
         const uint8_t* K = ldp<const uint8_t>(area + (uint32_t)offsetof(ZgClusterLayer, k_cache)) + (size_t)(lds32(kv + (uint32_t)offsetof(ZgClusterKv, k_off)) + lo * P.dh) * 4;
         const uint8_t* V = ldp<const uint8_t>(area + (uint32_t)offsetof(ZgClusterLayer, v_cache)) + (size_t)(lds32(kv + (uint32_t)offsetof(ZgClusterKv, v_off)) + lo * P.dh) * 4;
@@ -665,8 +668,11 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
     for (uint32_t l = 0; l < P.n_layers; l++) {
         const uint32_t area = c.base + P.o_const + (l & 1) * P.const_bytes, heads = area + (uint32_t)sizeof(ZgClusterLayer), gammas = area + P.blk_bytes;
         const uint32_t cs = gammas + 8 * P.D, smax = cs + dh * 4, at = smax + 16 * kMaxItems;
-        wait_bar(bar_of(c, kBarConstFull + (l & 1)), (l >> 1) & 1);
+        // a layer without its operands has no addresses either: nothing is stored there (set before a barrier, asked for behind it: the same to all)
+        if (!wait_bar(bar_of(c, kBarConstFull + (l & 1)), (l >> 1) & 1)) sts32(c.base + kNoOperands, 1u);
         if (l == 0) {      // the program's input: every CTA takes all of it
+            workers_sync();
+            if (lds32(c.base + kNoOperands)) return;
             const uint32_t a1 = c.base + P.o_a1;
             const float* x_in = ldp<const float>(LY(x_in));
 #pragma unroll 1
@@ -779,6 +785,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
             workers_sync();
             if ((ph & 1) == 0) {
                 if (ph == 0) {
+                    if (lds32(c.base + kNoOperands)) return;
                     // (every warp is past the layer before)
                     if (l && warp == kW - 1 && lane == 0) mbar_arrive(bar_of(c, kBarConstEmpty + ((l - 1) & 1)));
                     // ── q | k | v to every CTA ──
@@ -833,8 +840,9 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
                 }
                 if (warp < ownD) {
                     float4 v;
+                    bool next_there = true;
                     if (down) {
-                        if (!last) wait_bar(bar_of(c, kBarConstFull + ((l + 1) & 1)), ((l + 1) >> 1) & 1);
+                        next_there = last || wait_bar(bar_of(c, kBarConstFull + ((l + 1) & 1)), ((l + 1) >> 1) & 1);
                         wait_cluster(bar_of(c, kBarR), l & 1);
                         if (tid == 0) mbar_expect_tx(bar_of(c, kBarR), ownD * 128 * min(P.F >> 5, kC));
                         const uint32_t r_in = c.base + P.o_r + ((dg * 4 * P.own_max + warp) * 32 + c4) * 4, step = P.own_max * 128;
@@ -852,7 +860,7 @@ __device__ __forceinline__ void workers(const Cta& c, const ZgClusterPlan& P) {
 #pragma unroll
                             for (uint32_t u = 0; u < 4; u++) push1(inbox + (P.D + (lane & 1) * nD + grp) * 4 + away[u], lane & 1 ? mx : ss, bar + away[u]);
                         }
-                        if (dg == 1) stg4(ldp<float>(next + (uint32_t)offsetof(ZgClusterLayer, sum) + (down ? 0 : 8)) + own_i, xown);
+                        if (dg == 1 && next_there) stg4(ldp<float>(next + (uint32_t)offsetof(ZgClusterLayer, sum) + (down ? 0 : 8)) + own_i, xown);
                     }
                     if (dg == 0) stg4(ldp<float>(LY(out) + (down ? 48 : 24)) + own_i, v);
                 }
@@ -878,7 +886,7 @@ k_decode_cluster(const __grid_constant__ ZgClusterPlan plan) {
     c.tid = threadIdx.x; c.lane = c.tid & 31; c.warp = c.tid >> 5;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (c.tid == 0) {
-        *reinterpret_cast<uint32_t*>(smem + kDead) = 0;
+        *reinterpret_cast<uint32_t*>(smem + kDead) = *reinterpret_cast<uint32_t*>(smem + kNoOperands) = 0;
         const uint32_t nD = P.D >> 5, ownD = (nD + kC - 1 - c.rank) / kC;
 #pragma unroll 1
         for (uint32_t b = kBarA1; b < kBarFull + 2 * kW * P.ring_slots; b++)
