@@ -2558,7 +2558,6 @@ static bool launch_linear_ring(float* dst, const float* src, const WT* W, const 
     return true;
 }
 bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float* scratch, size_t scratch_elems, cudaStream_t st, bool ahead) {
-    const bool const_weights = ahead;
     (void)ctx;
     const ZgSeqOp& s = op.u.seq;
     switch (op.tag) {
@@ -2599,7 +2598,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                     const dim3 grid((N + 7) / 8);
                     const RingPlan ring = ring_plan(M, N, K, pairs, sizeof(WT), zg_sm_count());
                     if (aligned && ring.smem && linear_ring(M, N, pairs, (size_t)(pairs ? 2 : 1) * N * K * sizeof(WT))) {
-                        if (!(pairs ? launch_linear_ring<WT, true> : launch_linear_ring<WT, false>)(dst, src, W, b, M, N, K, s.n[3], s.n[4], act, slot_ctl, s.n[7], const_weights, ring, st)) return false;
+                        if (!(pairs ? launch_linear_ring<WT, true> : launch_linear_ring<WT, false>)(dst, src, W, b, M, N, K, s.n[3], s.n[4], act, slot_ctl, s.n[7], ahead, ring, st)) return false;
                         ZG_SEQ_CHECK();
                         return true;
                     }
@@ -2626,7 +2625,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
                                   (s.n[2] & 16u) ? (const WT*)nullptr : wptr<WT>(bufs, s.buf[2], s.off[0]), res, s.n[1], s.n[2], s.f[0], dst2,                \
                                   dst2 && !(s.n[4] & 16u) ? wptr<WT>(bufs, s.buf[5], s.off[1]) : (const WT*)nullptr, s.n[4], s.f[1],                         \
                                   s.n[7] ? (const float*)bufs[s.buf[6]] : (const float*)nullptr, s.n[7] ? wptr<WT>(bufs, s.buf[2], s.off[2]) : (const WT*)nullptr, \
-                                  s.n[8] ? s.n[8] - 1 : 0u, s.n[8] ? wptr<WT>(bufs, s.buf[2], s.off[5]) : (const WT*)nullptr, const_weights && s.n[0] < 64))
+                                  s.n[8] ? s.n[8] - 1 : 0u, s.n[8] ? wptr<WT>(bufs, s.buf[2], s.off[5]) : (const WT*)nullptr, ahead && s.n[0] < 64))
                 // Many rows: the kernel that keeps a row in registers (64 each: 1024 threads an SM) as long as all rows are resident at once.  Each value is then read once
                 // and all its loads are in flight together; the other one walks a row up to four times.  Feed-forwards of f32 / bf16 weights, walked -> in registers:
                 // 64 tokens of 4096 101.4 -> 91.8 / 68.2 -> 63.6 us, 256 of 2048 97.3 -> 92.3 / 53.3 -> 52.2, 256 of 1024 46.9 -> 45.3 / 36.9 -> 34.9.  Up to 512 columns
@@ -2654,7 +2653,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             ZG_SEQ_WDT(s.n[3], launch_pdl(k_norm<WT>, dim3(s.n[0]), dim3(256), 0, st, bufs[s.buf[0]] + s.off[3], bufs[s.buf[1]], wptr<WT>(bufs, s.buf[2], s.off[0]), res, s.n[1], s.n[2], s.f[0],
                                           dst2, dst2 ? wptr<WT>(bufs, s.buf[5], s.off[1]) : nullptr, s.n[4], s.f[1],
                                           shift_state ? wptr<WT>(bufs, s.buf[dst2 ? 5 : 2], s.off[2]) : nullptr, shift_state, shift_state ? bufs[s.buf[7]] : nullptr,
-                                          avg_terms ? wptr<WT>(bufs, s.buf[2], s.off[4]) : nullptr, avg_terms, s.n[6], avg_terms ? bufs[s.buf[4]] : nullptr, const_weights));
+                                          avg_terms ? wptr<WT>(bufs, s.buf[2], s.off[4]) : nullptr, avg_terms, s.n[6], avg_terms ? bufs[s.buf[4]] : nullptr, ahead));
             ZG_SEQ_CHECK();
             return true;
         }
@@ -2836,7 +2835,7 @@ bool zg_launch_seq_op(ZgCudaCtx* ctx, const ZgOp& op, float* const* bufs, float*
             return true;
         }
         default:
-            if (op.tag >= ZG_OP_STREAM_STEP) return zg_launch_stream_op(op, bufs, st, const_weights);
+            if (op.tag >= ZG_OP_STREAM_STEP) return zg_launch_stream_op(op, bufs, st, ahead);
             return op.tag >= ZG_OP_SSM_SCAN ? zg_launch_rec_op(op, bufs, scratch, st) : zg_launch_mix_op(op, bufs, scratch, st, ahead);
     }
 }
