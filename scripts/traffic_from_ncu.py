@@ -12,8 +12,7 @@ import statistics
 import sys
 
 root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-src = sys.argv[1] if len(sys.argv) > 1 else os.path.join(root, "profiles")
-prefix = sys.argv[2] if len(sys.argv) > 2 else "r02"
+src, prefix = sys.argv[1:3]                            # folder and first part of the captures' names: <prefix>_traffic_<KxN>_<fmt>.csv
 BLK = {"i8_f32": 36, "q8_0": 34, "q4_0": 18}
 out = {}
 for path in sorted(glob.glob(os.path.join(src, f"{prefix}_traffic_*.csv"))):

@@ -2,7 +2,7 @@
 
 * 1 GPU: a program built from weights streamed into HBM first (ZG_QWEIGHT_RESIDENT descriptors) equals the program
   that uploads the same weights through compile_program; collective ops at world 1 are identity / copy.
-* >= 2 GPUs (skipped otherwise; `gpurun --gpus 2`): two processes, one per GPU, NCCL all-reduce / all-gather inside
+* >= 2 GPUs (skipped otherwise): two processes, one per GPU, NCCL all-reduce / all-gather inside
   the program's CUDA graph; logits vs the unsharded oracle within 1e-3 relative, greedy tokens identical."""
 import os
 import socket
@@ -137,7 +137,7 @@ def _n_gpus():
                          ids=["untied-q4-graph", "tied-q8-graph", "untied-q8-eager", "chunk4", "chunk24-tensor-core"])
 def test_two_gpu_sharded_decode_matches_unsharded_oracle(cfg, kind, token_len, graph):
     if _n_gpus() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     import torch.multiprocessing as mp
     world = 2
     out = mp.Manager().dict()
@@ -193,7 +193,7 @@ def test_sharded_70b_width_matches_unsharded_oracle(world, path):
     """Every rank holds its slab of the same hashed synthetic model; rank-identical logits, 1e-3 against the unsharded oracle
     executor on the host form of that model, identical greedy tokens.  Self-skips below `world` GPUs."""
     if _n_gpus() < world:
-        pytest.skip(f"needs {world} GPUs (gpurun --gpus {world})")
+        pytest.skip(f"needs {world} GPUs")
     import torch.multiprocessing as mp
     from zgml_b200.host.llama import synthetic_model_host
     cfg, kind, n_tok, context = CFG_70B_WIDTH, "q4_0", 3, 20
