@@ -136,18 +136,23 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
     if (warp == 0) {
         if (lane == 0) {
+            uint32_t fills = 0;
             for (uint32_t kt = 0; kt < n_k; kt++) {
                 const uint32_t s = kt % kStages, ph = (kt / kStages) & 1;
                 if (!mbar_wait(empty + 8 * s, ph ^ 1)) break;
                 mbar_expect_tx(full + 8 * s, kStage);
                 tma_2d(base + s * kStage, &tmap_a, kt * BK, head * p.a_rows + tile_m * BM, full + 8 * s);
                 tma_2d(base + s * kStage + kTileA, &tmap_b, kt * BK, head * p.N + tile_n * BN, full + 8 * s);
+                fills++;
             }
+            // the copies that are under way land before the CTA's shared memory goes, whatever gave up
+            for (uint32_t i = 0; i < min(fills, (uint32_t)kStages); i++) mbar_wait(full + 8 * i, ((fills - 1 - i) / kStages) & 1);
         }
     } else if (warp == 1) {
         // instruction descriptor (kind::f16): D = F32, A = B = BF16, both K-major, N = BN, M = 128
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((BN >> 3) << 17) | ((128u >> 4) << 24);
         const bool leader = elect_one();
+        uint32_t issued = 0;
         for (uint32_t kt = 0; kt < n_k; kt++) {
             const uint32_t s = kt % kStages, ph = (kt / kStages) & 1;
             if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, ph))) break;
@@ -157,7 +162,10 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 if (leader) mma_bf16(tmem_base, make_desc(base + s * kStage + k * 32), make_desc(base + s * kStage + kTileA + k * 32), idesc, (kt | k) ? 1u : 0u);
             if (leader) mma_commit(empty + 8 * s);
             if (leader && kt + 1 == n_k) mma_commit(tmem_full);
+            issued = kt + 1;
         }
+        // products under way end before their accumulator goes
+        if (issued < n_k && issued) mbar_wait(empty + 8 * ((issued - 1) % kStages), ((issued - 1) / kStages) & 1);
         __syncwarp();
     } else {
         // ── epilogue: warp w may touch TMEM lanes 32 (w % 4) .. + 31 ──
@@ -166,6 +174,11 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if (!ok && lane == 0) count_timeout();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t m_base = tile_m * BM + quarter * 32;
+        if (!ok) {      // outputs that are not numbers, instead of what was there before
+            const uint32_t per = PAIRS ? 2 : 1, n1 = min(N, (tile_n + 1) * BN) / per;
+            for (uint32_t n = tile_n * BN / per + lane; n < n1; n += 32)
+                for (uint32_t m = m_base; m < min(p.M, m_base + 32); m++) outp[(size_t)m * p.out_rs + n] = __int_as_float(0x7fc00000);
+        }
         uint4* tb = reinterpret_cast<uint4*>(dsm_raw + (base - smem_u32(dsm_raw)) + ew * (32 * 36 * 4));   // the stages are idle now
 #pragma unroll 1
         for (uint32_t c0 = 0; ok && c0 < BN; c0 += 32) {
