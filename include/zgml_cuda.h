@@ -511,10 +511,10 @@ void zg_cuda_set_graph_mode(ZgCudaCtx* ctx, int enabled);
 /* Device pointer of program buffer `buf_idx` (for device-resident benches). */
 void* zg_cuda_program_buffer(ZgCudaProgram* prog, uint32_t buf_idx);
 /* Schedule introspection (tests / benches assert that the fast paths are the ones that run): what == 0: kernels one
- * execution launches (graph nodes); 1: DeviceOps covered by the fused single-token decode kernel (0: general schedule);
+ * execution launches (graph nodes); 1: DeviceOps covered by the fused single-token decode kernel or its cluster form (0: general schedule);
  * 2: layers inside that kernel; 3: launches of the streamed single-row matvec kernel (csrc/qgemv_stream.cu) among them;
  * 4: HBM bytes per execution saved by promoted dense operands (zg_cuda_program_promote_dense); 5: waits that kernels have given up on
- * since process start (dense and f32 matmuls, attention, LINEAR of few rows, quantized matmuls of three to eight, DELTA_RULE; 0 in a healthy run); 6: LINEAR ops of the program whose bfloat16 weights run on the tensor cores;
+ * since process start (dense and f32 matmuls, experts' products, attention, LINEAR of few rows, quantized matmuls of three to eight, DELTA_RULE, the cluster form of single-token steps; 0 in a healthy run); 6: LINEAR ops of the program whose bfloat16 weights run on the tensor cores;
  * 7: f32 slots of the scratch that the program's tensor-core kernels and sequence ops share; 8: LINEAR ops whose weight nothing in the program writes, so that a
  * launch may read it before its predecessor has completed; 9: NORM and STREAM_STEP ops with such weights. */
 uint64_t zg_cuda_program_stats(const ZgCudaProgram* prog, int what);

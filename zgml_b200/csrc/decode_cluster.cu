@@ -2,13 +2,13 @@
 //
 // What bounds such a step is the chain of dependent launches: seven per layer, 31 us for the 3.8 MB of a layer of width 576, whose
 // bytes pass in 2 - 3 us.  Here a layer is five phases on 16 SMs without a launch between them, and what passes from one to the next
-// are vectors in shared memory.  30 layers of width 576 over 512 positions (Q8_0): 981 -> 758 us a token, head and host included, some
-// 22 us a layer; 8 layers of width 128: 228 -> 181 us.  What bounds it now is not memory but the walk of the warps through a layer's
-// code: about 2000 instructions a warp, most of them executed once per layer, each waiting for the one before it or for its own fetch
-// (58 KB of code).  Stamped while a layer still took 24 us, 45 000 clocks: attention 9000, the four products 1700 - 3500 each,
-// reductions and exchanges between them the rest.
+// are vectors in shared memory.  30 layers of width 576 over 512 positions (Q8_0): 975 -> 797 us a token, head and host included, some
+// 23 us a layer; other shapes and where the line to the general schedule lies: cluster_pays (backend.cu).  What bounds it now is not
+// memory but the walk of the warps through a layer's code: about 2000 instructions a warp, most of them executed once per layer, each
+// waiting for the one before it or for its own fetch (some 58 KB of code).  Stamped while a layer took 24 us, 45 000 clocks: attention
+// 9000, the four products 1700 - 3500 each, reductions and exchanges between them the rest.
 //
-//   1  x (residual stream) -> rmsnorm, gamma in the registers of the consumers -> q | k | v matvecs, whole columns per CTA
+//   1  x (residual stream) -> rmsnorm, x inv gamma formed where a record's digits are cut -> q | k | v matvecs, whole columns per CTA
 //   2  rope, cache stores, attention: CTA = (KV head, share of the positions), all query heads of the group -> partial states
 //   3  merge of the partial states -> o matvec, whole columns -> the owner of a column group adds the residual
 //   4  rmsnorm -> gate | up matvecs in pairs -> activation: stays in the CTA
@@ -217,7 +217,8 @@ __host__ __device__ inline uint32_t item_of(const ZgClusterPlan& P, uint32_t ran
 
 // ── a warp's records of one phase: partial sums of its stretch of every column group that it touches -> part[warp * seg + n][32] ──
 // Activations share a scale over the records that lie in one range of the general schedule (a warp's there), so that none is cut on a coarser grid than there: with a scale for
-// the whole stretch, seven records instead of two or three, gate and up of width 576 were off by 1.6 times as much beside channels that stand out (and a step of 30 layers took 788 us, with the ranges 800).
+// the whole stretch, seven records instead of two or three, gate and up of width 576 were off by 1.6 times as much beside channels that stand out (a step of 30 layers took 788 us,
+// with the ranges 800).
 // Addresses in shared memory: x: the K values; gamma: 0, or x * inv * gamma is what is multiplied; top: largest magnitude of 32 values of x (times gamma).
 __device__ __noinline__ float true_max(uint32_t x, uint32_t gamma, float inv, uint32_t n) {      // the bound was infinite, the products may not be
     float mx = 0.0f;
@@ -874,7 +875,7 @@ template <int FMT>
 __global__ void __launch_bounds__(kThreads, 1)
 k_decode_cluster(const __grid_constant__ ZgClusterPlan plan) {
     extern __shared__ __align__(128) uint8_t smem[];
-    // a copy of the plan for the functions that are calls (the workers read it as constants: 759 us a token, from shared memory 818)
+    // a copy of the plan for the functions that are calls (the workers read it as constants: from shared memory a token takes 8 % longer)
     static_assert(sizeof(ZgClusterPlan) <= kDead, "the mark lies behind it");
     if (threadIdx.x < sizeof(ZgClusterPlan) / 4) reinterpret_cast<uint32_t*>(smem)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&plan)[threadIdx.x];
     __syncthreads();
@@ -988,7 +989,7 @@ bool launch(const ZgClusterHost& h, cudaStream_t st) {
     return true;
 }
 
-// whether the device takes a cluster of this size (asked once per format and device)
+// whether the device takes a cluster of this size (asked when a program is compiled)
 template <int FMT>
 bool fits(uint32_t smem) {
     if (!zg_smem_limit<k_decode_cluster<FMT>>(kZgClusterSmem)) return false;

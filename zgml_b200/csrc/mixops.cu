@@ -545,7 +545,8 @@ __global__ void __launch_bounds__(kMergeCols * kMergeGroups, BLOCKS) k_cached_at
 // of 32 heads on 8 of 128 68 -> 53, of 8 heads on 2 of 256 41 -> 31; at 100 of 2048 positions 0.5 to 0.9 us
 // slower where CTAs share SMs (4 heads of 96 9.2 -> 9.9), the cutting of operands where a handful of FMAs did.  Of the 28 us 4 were the launch of the append, 4 to 6 the merge,
 // the rest the chain load - scores - softmax - sums of two rounds.  The keys of earlier positions now come while the append runs, where nothing else in the program writes the
-// cache (CaArgs::early), and both buffers are filled at the start: 28.7 -> 26.7 us; 16 heads on 4 of 128, 4000 positions 22.6 -> 20.5; 4 heads, latents of 320, 8192 22.2 -> 20.8.
+// cache (CaArgs::early), and both buffers are filled at the start: 28.7 -> 26.7 .. 28.6 us by where the buffers lie (28.9 -> 28.2 on average over 32 layouts of memory);
+// 16 heads on 4 of 128, 4000 positions 22.6 -> 20.5; 4 heads, latents of 320, 8192 22.2 -> 20.8.
 constexpr int kCfRows = 16, kCfKeys = 32;
 // How many of a step's shares (as many as the cache's capacity asks for) its keys are dealt to: beyond 64 only where each gets sixteen keys.  What the step
 // reads is its keys, and the merge reads a record per share: with 148 shares whatever the position, a token at position 500 of a cache of 8192 latents
